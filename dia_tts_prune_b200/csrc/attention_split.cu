@@ -1,0 +1,689 @@
+// attention_split.cu - softmax attention of many query rows on the 5th-generation tensor cores, with fp32 operands split into
+// two fp16 terms (sm_100a).
+//
+// A CTA owns 128 (token, head) rows: up to 128 / PK consecutive tokens times PK query heads that read the same key/value head, so
+// that a tile of keys serves all of them.  It walks its keys 64 at a time:
+//   warps 8 .. 11   fetch key and value rows from the pages, scale them by a power of two, split x = hi + lo into fp16 and put both
+//                   into a ring of shared-memory slots ([key / 8][channel / 8] blocks of 8 x 16 bytes: the layout is the K-major
+//                   operand of the scores and the MN-major operand of the value product)
+//   warp 12         issues tcgen05.mma: scores S = Q K^T (M = 128, N = 64; lo hi, hi lo, then hi hi, so that the small terms are
+//                   added first) per group of at most 128 channels, and the value product of the tile before (weights as the
+//                   operand in tensor memory)
+//   warps 0 .. 7    two threads per row, 32 keys each: scores from tensor memory (the channel groups are summed here, in fp32),
+//                   cap, bias, mask, online softmax in base 2, weights split and written to tensor memory; then the value
+//                   product of the tile before is added to the row's fp32 registers
+// The accumulator of a tensor-core product loses up to one unit in the last place at every step, towards zero (measured: 2e-6
+// over K = 2048).  So no accumulator lives longer than one tile and one channel group, and sums over tiles are fp32 additions
+// in registers: measured against 64 bits the output is as close as the fp32 FMA kernels' (2.6e-7 both at 300 rows, d = 128).
+//
+// Scaling: a query tile, a group of 16 keys and a tile of values are each brought to a largest magnitude of [2^14, 2^15) before
+// the split (the largest finite one; powers of two, undone exactly), so the fp16 range costs nothing: an element down to 2^-17 of
+// its group's largest keeps its 22 bits.  Softmax weights carry 2^14.
+//
+// Bound: per 64 keys and 128 rows 3 x 128 x 64 x (dk + dv) multiply-adds on the tensor pipe (1536 cycles at 128 + 128) against
+// about as many issue slots for splitting and softmax.
+// Every wait is bounded: a wait that runs out makes the CTA write NaN and end.
+#include <algorithm>
+
+#include <cuda_fp16.h>
+#include <cuda_bf16.h>
+#include <cuda_runtime.h>
+#include <math_constants.h>
+#include <stdint.h>
+
+#include "attention_split.h"
+#include "common.cuh"
+
+namespace dia {
+
+namespace {
+
+constexpr int kRows = 128, kKeys = 64, kGroupW = 128;        // query rows of a CTA, keys of a tile, channels of a stage
+constexpr int kSplitThreadsTC = 512;
+constexpr int kMaxSlots = 6, kScaleRing = 8, kMaxKStages = 4;
+constexpr int kSmemMost = 232448;
+constexpr float kLog2e = 1.4426950408889634f;
+constexpr float kWeightScale = 16384.f;                       // on the softmax weights (at most 1) before the split
+constexpr unsigned kSpinMost = 4000000u;
+
+struct Geometry {
+    int pk_shift;                            // log2 of the heads of a CTA's rows
+    int n_kst, n_vst;                        // channel groups of a key, of a value
+    int wk0, wk_last;                        // their padded widths (multiples of 16): all but the last, the last
+    int wv0, wv_last;
+    int slot_bytes, n_slots, q_bytes;
+};
+
+__device__ __forceinline__ bool wait_for(uint64_t* bar, uint32_t parity) {
+    for (unsigned i = 0; i < kSpinMost; ++i)
+        if (mbar_try_wait(bar, parity)) return true;
+    return false;
+}
+// the same for a converged warp, with one answer for all lanes (so that what follows is uniform: see elect_one_sync)
+__device__ __forceinline__ bool wait_warp(uint64_t* bar, uint32_t parity) {
+    for (unsigned i = 0; i < kSpinMost; ++i)
+        if (__any_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+    return false;
+}
+__device__ __forceinline__ float ex2(float x) {
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+// operands without swizzle: blocks of 8 rows x 16 bytes; lead / stride: bytes between blocks along the contraction / the rows
+// (K-major) or along the contraction / the channels (MN-major)
+__device__ __forceinline__ uint64_t block_desc(uint32_t addr, uint32_t lead, uint32_t stride) {
+    const uint32_t lo = ((addr & 0x3FFFFu) >> 4) | ((lead >> 4) << 16);
+    const uint32_t hi = (stride >> 4) | (1u << 14);
+    return ((uint64_t)hi << 32) | lo;
+}
+__device__ __forceinline__ void mma_ss(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(acc)
+        : "memory");
+}
+__device__ __forceinline__ void mma_ts(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, uint32_t acc) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d), "r"(a), "l"(b), "r"(idesc), "r"(acc)
+        : "memory");
+}
+__device__ __forceinline__ void commit_to(uint64_t* bar) {
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+__device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void fence_smem_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+__device__ __forceinline__ void tmem_load8(uint32_t addr, float (&v)[8]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
+                 : "r"(addr)
+                 : "memory");
+}
+__device__ __forceinline__ void tmem_loaded() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ void tmem_store8(uint32_t addr, const uint32_t (&v)[8]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(addr), "r"(v[0]), "r"(v[1]),
+                 "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
+                 : "memory");
+}
+
+// (x, y) = hi + lo, both rounded to fp16
+__device__ __forceinline__ void split2(float x, float y, uint32_t& hi, uint32_t& lo) {
+    const __half2 h = __floats2half2_rn(x, y);
+    const float2 f = __half22float2(h);
+    const __half2 l = __floats2half2_rn(x - f.x, y - f.y);
+    hi = *reinterpret_cast<const uint32_t*>(&h);
+    lo = *reinterpret_cast<const uint32_t*>(&l);
+}
+// the power of two that brings a largest magnitude m to [2^14, 2^15), and its inverse (m = 0: 2^114; both stay normal numbers)
+__device__ __forceinline__ float scale_of(float m, float& inverse) {
+    const int e = max((int)(__float_as_uint(m) >> 23) - 127, -100);
+    inverse = __uint_as_float((uint32_t)(e + 113) << 23);
+    return __uint_as_float((uint32_t)(min(141 - e, 254)) << 23);
+}
+__device__ __forceinline__ float max_abs4(float m, const float4& v) {
+    return fmaxf(fmaxf(fmaxf(m, fabsf(v.x)), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w)));
+}
+__device__ __forceinline__ float finite_abs(float x) { const float a = fabsf(x); return a <= 3.402823466e38f ? a : 0.f; }
+__device__ __forceinline__ float warp_max_of(float v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
+    return v;
+}
+__device__ __forceinline__ int first_key_of(int i, int window, int chunk) {
+    const int w = window > 0 ? max(0, i - window + 1) : 0;
+    return chunk > 0 ? max(w, i - i % chunk) : w;
+}
+
+// The key tiles of a CTA in the order in which every role walks them.  A segment is a maximal run of the CTA's tokens with one
+// slot and consecutive positions (and, by row mode 1, on one side of n); its keys are the kept first positions in front of its
+// window range (phase 0), then the range from its first token's first key on (phase 1).
+struct Walk {
+    const int* s_slot; const int* s_pos;
+    int n, seg_a, seg_b, phase, j0, k_end, lo;
+    __device__ Walk(const int* slots, const int* pos, int n_tok)
+        : s_slot(slots), s_pos(pos), n(n_tok), seg_a(0), seg_b(0), phase(1), j0(0), k_end(0), lo(0) {}
+    // true: tile [j0, min(j0 + 64, k_end)) of the segment's sequence
+    __device__ bool next(const SplitAttention& p) {
+        if (j0 < k_end) j0 += kKeys;                          // (the tile that was walked last)
+        for (;;) {
+            if (j0 < k_end) return true;
+            if (phase == 0) {
+                phase = 1;
+                j0 = lo;
+                k_end = s_pos[seg_b - 1] + 1;
+                continue;
+            }
+            seg_a = seg_b;
+            if (seg_a >= n) return false;
+            const int slot = s_slot[seg_a];
+            const int nv = p.rows_per_slot > 0 ? p.n_valid[slot] : 0;
+            const bool split_at = p.rows_per_slot > 0 && p.mode == 1;
+            seg_b = seg_a + 1;
+            while (seg_b < n && s_slot[seg_b] == slot && s_pos[seg_b] == s_pos[seg_b - 1] + 1 && !(split_at && s_pos[seg_b] == nv)) ++seg_b;
+            if (p.rows_per_slot > 0 && p.mode != 0) {
+                const bool tail = p.mode == 1 && s_pos[seg_a] >= nv;
+                phase = 1;
+                j0 = tail ? nv : 0;
+                k_end = tail ? p.n_keys : min(nv, p.n_keys);
+                continue;
+            }
+            lo = first_key_of(s_pos[seg_a], p.window, p.chunk);
+            phase = 0;
+            j0 = 0;
+            k_end = p.window > 0 ? min(p.keep_first, lo) : 0;
+        }
+    }
+};
+
+// NVS: channel groups of a value (1: up to 128 channels, a thread of a row keeps half of them; 2: up to 256, a group each)
+template <int NVS>
+__global__ void __launch_bounds__(kSplitThreadsTC, 1)
+split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_constant__ Geometry geo) {
+    constexpr int DVH = 64 * NVS;                             // output channels of a thread
+    extern __shared__ __align__(128) unsigned char smem[];
+    __shared__ float s_red[16];
+    __shared__ uint32_t s_tmem;
+    unsigned char* ring = smem;
+    unsigned char* qs = ring + (size_t)geo.n_slots * geo.slot_bytes;
+    uint64_t* full = reinterpret_cast<uint64_t*>(qs + geo.q_bytes);
+    uint64_t* empty = full + kMaxSlots;
+    uint64_t* s_full = empty + kMaxSlots;                     // scores of a tile are there / have been read
+    uint64_t* s_empty = s_full + 1;
+    uint64_t* p_ready = s_empty + 1;                          // weights of a tile are there / its value product is done
+    uint64_t* pv_done = p_ready + 1;
+    uint64_t* v_max = pv_done + 1;                            // the four fetching warps' largest values
+    uint64_t* pair = v_max + 1;                               // [4] the two warps that share rows
+    float* k_inv = reinterpret_cast<float*>(pair + 4);        // [kScaleRing][kMaxKStages][4] inverse scales of 16 keys
+    float* v_inv = k_inv + kScaleRing * kMaxKStages * 4;      // [kScaleRing][2]
+    float* vm_s = v_inv + kScaleRing * 2;                     // [2][4]
+    float* row_x = vm_s + 8;                                  // [2][2][128] what the two threads of a row tell each other
+    int* s_slot = reinterpret_cast<int*>(row_x + 4 * kRows);  // [tokens]
+    const int TT = kRows >> geo.pk_shift;
+    int* s_pos = s_slot + TT;
+
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int PK = 1 << geo.pk_shift;
+    const int h0 = blockIdx.x * PK, rep = p.heads / p.kv_heads, g = h0 / rep;
+    const int r0 = (gridDim.y - 1 - blockIdx.y) * TT;         // later tokens see more keys: their tiles start first
+    const int n_tok = min(TT, p.M - r0);
+
+    if (tid == 0) {
+        for (int i = 0; i < kMaxSlots; ++i) { mbar_init(&full[i], 4); mbar_init(&empty[i], 1); }
+        mbar_init(s_full, 1);
+        mbar_init(s_empty, 8);
+        mbar_init(p_ready, 8);
+        mbar_init(pv_done, 1);
+        mbar_init(v_max, 4);
+        for (int i = 0; i < 4; ++i) mbar_init(&pair[i], 2);
+        fence_mbar_init();
+    }
+    if (warp == 12) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(&s_tmem)));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::);
+    }
+    for (int i = tid; i < TT; i += kSplitThreadsTC) {
+        const int r = r0 + i;
+        const bool in = i < n_tok;
+        s_slot[i] = !in ? -1 : p.rows_per_slot > 0 ? r / p.rows_per_slot : p.row_slot[r];
+        s_pos[i] = !in ? -1 : p.rows_per_slot > 0 ? r % p.rows_per_slot : p.row_pos[r];
+    }
+
+    // ---- the query tile: largest magnitude, then both terms.  Row r of the tile is head h0 + r % PK of token r / PK ----
+    const int wk_sum = (geo.n_kst - 1) * geo.wk0 + geo.wk_last, chunks = wk_sum >> 3;
+    auto q_values = [&](int row, int ch, float (&v)[8]) {     // channels 8 ch .. of the padded row
+        const int i = row >> geo.pk_shift, h = h0 + (row & (PK - 1));
+        const int cpad = 8 * ch, st = cpad / geo.wk0, c = cpad - st * geo.wk0;
+        const int width = p.talk ? p.kdim : min(kGroupW, p.kdim - st * kGroupW);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) v[e] = 0.f;
+        if (i >= n_tok || c >= width) return;
+        const float* src = p.q + (size_t)(r0 + i) * p.ldq;
+        const bool both = c + 4 < width;                      // (widths are multiples of 4)
+        if (!p.talk) {
+            src += (size_t)h * p.qdim + st * kGroupW + c;
+            const float4 a = *reinterpret_cast<const float4*>(src);
+            v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+            if (both) {
+                const float4 b = *reinterpret_cast<const float4*>(src + 4);
+                v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+            }
+            return;
+        }
+        for (int t = 0; t < rep; ++t) {                       // the mixed score is linear in the queries: mix those instead
+            const int gh = st * rep + t;
+            const float w = p.talk[h * p.heads + gh];
+            const float4 a = *reinterpret_cast<const float4*>(src + (size_t)gh * p.qdim + c);
+            v[0] = fmaf(w, a.x, v[0]); v[1] = fmaf(w, a.y, v[1]); v[2] = fmaf(w, a.z, v[2]); v[3] = fmaf(w, a.w, v[3]);
+            if (both) {
+                const float4 b = *reinterpret_cast<const float4*>(src + (size_t)gh * p.qdim + c + 4);
+                v[4] = fmaf(w, b.x, v[4]); v[5] = fmaf(w, b.y, v[5]); v[6] = fmaf(w, b.z, v[6]); v[7] = fmaf(w, b.w, v[7]);
+            }
+        }
+    };
+    float qm = 0.f;
+    for (int idx = tid; idx < kRows * chunks; idx += kSplitThreadsTC) {
+        const int rg = idx / (8 * chunks), rest = idx - rg * 8 * chunks, row = rg * 8 + (rest & 7), ch = rest >> 3;
+        float v[8];
+        q_values(row, ch, v);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) qm = fmaxf(qm, finite_abs(v[e]));
+    }
+    qm = warp_max_of(qm);
+    if (lane == 0) s_red[warp] = qm;
+    __syncthreads();
+    for (int w = 0; w < 16; ++w) qm = fmaxf(qm, s_red[w]);
+    float q_inv;
+    const float q_scale = scale_of(qm, q_inv);
+    for (int idx = tid; idx < kRows * chunks; idx += kSplitThreadsTC) {
+        const int rg = idx / (8 * chunks), rest = idx - rg * 8 * chunks, row = rg * 8 + (rest & 7), ch = rest >> 3;
+        float v[8];
+        q_values(row, ch, v);
+        uint32_t hi[4], lo[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) split2(v[2 * e] * q_scale, v[2 * e + 1] * q_scale, hi[e], lo[e]);
+        const int st = 8 * ch / geo.wk0, w = st == geo.n_kst - 1 ? geo.wk_last : geo.wk0, c8 = ch - st * (geo.wk0 >> 3);
+        unsigned char* dst = qs + (size_t)st * geo.wk0 * kRows * 4 + (size_t)((rg * (w >> 3) + c8) * 128 + (row & 7) * 16);
+        *reinterpret_cast<uint4*>(dst) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+        *reinterpret_cast<uint4*>(dst + (size_t)w * kRows * 2) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+    }
+    fence_smem_async();
+    fence_before();
+    __syncthreads();
+    fence_after();
+    const uint32_t tmem = s_tmem;
+    const uint32_t t_s = tmem, t_p = tmem + 64u * geo.n_kst, t_o = t_p + 64u;    // scores | weights (hi, lo) | value product
+
+    if (warp < 8) {
+        // ================= softmax: rows 32 (warp % 4) + lane, keys 32 (warp / 4) .. + 31 of a tile =================
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 184;");
+        const int qt = warp & 3, hf = warp >> 2, row = qt * 32 + lane, tok = row >> geo.pk_shift, h = h0 + (row & (PK - 1));
+        const uint32_t lanes = (uint32_t)(qt * 32) << 16;
+        const int my_pos = s_pos[tok];
+        const int my_lo = first_key_of(max(my_pos, 0), p.window, p.chunk), kept = p.window > 0 ? p.keep_first : 0;
+        const bool ranged = p.rows_per_slot > 0 && p.mode != 0;
+        const float mult = q_inv * p.scale * (p.temp ? p.temp[h] : 1.f), cap = p.cap, inv_cap = cap > 0.f ? 1.0f / cap : 0.f;
+        const float slope = p.slopes ? p.slopes[h] : 0.f;
+        const int half = NVS == 1 ? geo.wv0 >> 1 : 128;       // channels of this thread (NVS == 2: a whole group)
+        const uint32_t t_mine = t_o + (NVS == 1 ? hf * half : hf * 128) + lanes;
+        const int n_mine = NVS == 1 ? half : (hf ? geo.wv_last : geo.wv0);
+        float O[DVH];
+#pragma unroll
+        for (int c = 0; c < DVH; ++c) O[c] = 0.f;
+        float m_run = -CUDART_INF_F, c_run = 0.f, l_run = 0.f, corr_prev = 1.f;
+        bool ok = true;
+        auto add_values = [&](unsigned t) {                   // O <- corr O + value product of tile t
+            if (!wait_for(pv_done, t & 1u)) { ok = false; return; }
+            fence_after();
+            const float vi = v_inv[(t % kScaleRing) * 2 + (NVS == 1 ? 0 : hf)] * (1.0f / kWeightScale);
+            const bool same = __all_sync(0xffffffffu, corr_prev == 1.f);
+#pragma unroll
+            for (int c = 0; c < DVH; c += 8) {
+                if (c < n_mine) {
+                    float v[8];
+                    tmem_load8(t_mine + c, v);
+                    tmem_loaded();
+                    if (same) {
+#pragma unroll
+                        for (int e = 0; e < 8; ++e) O[c + e] = fmaf(v[e], vi, O[c + e]);
+                    } else {
+#pragma unroll
+                        for (int e = 0; e < 8; ++e) O[c + e] = fmaf(v[e], vi, O[c + e] * corr_prev);
+                    }
+                }
+            }
+        };
+        unsigned t = 0;
+        Walk w(s_slot, s_pos, n_tok);
+        for (; w.next(p); ++t) {
+            if (!wait_for(s_full, t & 1u)) { ok = false; break; }
+            fence_after();
+            float s[32];
+            const float* ki = k_inv + (t % kScaleRing) * kMaxKStages * 4 + hf * 2;
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                float v[8];
+                tmem_load8(t_s + lanes + hf * 32 + c * 8, v);
+                tmem_loaded();
+                const float a = ki[c >> 1] * mult;
+#pragma unroll
+                for (int e = 0; e < 8; ++e) s[c * 8 + e] = v[e] * a;
+                for (int st = 1; st < geo.n_kst; ++st) {
+                    tmem_load8(t_s + lanes + st * 64 + hf * 32 + c * 8, v);
+                    tmem_loaded();
+                    const float b = ki[st * 4 + (c >> 1)] * mult;
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) s[c * 8 + e] = fmaf(v[e], b, s[c * 8 + e]);
+                }
+            }
+            fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(s_empty);
+            // ---- cap, distance bias, visibility ----
+            const int k0 = w.j0 + hf * 32;
+            if (cap > 0.f) {
+#pragma unroll
+                for (int e = 0; e < 32; ++e) s[e] = cap * tanhf(s[e] * inv_cap);
+            }
+            if (p.slopes) {
+                const float base = (float)(my_pos - k0);
+#pragma unroll
+                for (int e = 0; e < 32; ++e) s[e] -= slope * (base - (float)e);
+            }
+            const bool live = tok >= w.seg_a && tok < w.seg_b;
+            const int last = live ? min(w.k_end - 1, ranged ? 0x7fffffff : my_pos) : -1, first = ranged ? 0 : my_lo;
+            if (!__all_sync(0xffffffffu, k0 + 31 <= last && (k0 >= first || k0 + 31 < kept))) {
+#pragma unroll
+                for (int e = 0; e < 32; ++e) {
+                    const int j = k0 + e;
+                    if (!(j <= last && (j >= first || j < kept))) s[e] = -CUDART_INF_F;
+                }
+            }
+            float mx = s[0];
+#pragma unroll
+            for (int e = 1; e < 32; ++e) mx = fmaxf(mx, s[e]);
+            float* xm = row_x + (t & 1u) * 2 * kRows;
+            xm[hf * kRows + row] = mx;
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&pair[qt]);
+            if (!wait_for(&pair[qt], t & 1u)) { ok = false; break; }
+            mx = fmaxf(mx, xm[(hf ^ 1) * kRows + row]);
+            const float m_new = fmaxf(m_run, mx);
+            const float c_new = m_new == -CUDART_INF_F ? 0.f : m_new * kLog2e;
+            const float corr = m_run == -CUDART_INF_F ? 0.f : ex2(c_run - c_new);
+            float sum0 = 0.f, sum1 = 0.f;
+#pragma unroll
+            for (int e = 0; e < 32; e += 2) {
+                s[e] = ex2(fmaf(s[e], kLog2e, -c_new));
+                s[e + 1] = ex2(fmaf(s[e + 1], kLog2e, -c_new));
+                sum0 += s[e];
+                sum1 += s[e + 1];
+            }
+            l_run = fmaf(l_run, corr, sum0 + sum1);
+            m_run = m_new;
+            c_run = c_new;
+            if (t > 0) add_values(t - 1);                     // (also: the weights' columns are free)
+            if (!ok) break;
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+                uint32_t hi[8], lo[8];
+#pragma unroll
+                for (int e = 0; e < 8; ++e) split2(s[c * 16 + 2 * e] * kWeightScale, s[c * 16 + 2 * e + 1] * kWeightScale, hi[e], lo[e]);
+                tmem_store8(t_p + lanes + hf * 16 + c * 8, hi);
+                tmem_store8(t_p + lanes + 32 + hf * 16 + c * 8, lo);
+            }
+            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+            fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(p_ready);
+            corr_prev = corr;
+        }
+        if (ok && t > 0) add_values(t - 1);
+        // ---- both threads' denominators, the sink's own term, normalise, store ----
+        float* xl = row_x + (t & 1u) * 2 * kRows;
+        xl[hf * kRows + row] = l_run;
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&pair[qt]);
+        ok = ok && wait_for(&pair[qt], t & 1u);
+        float l = l_run + xl[(hf ^ 1) * kRows + row];
+        if (p.sink) l += ex2(fmaf(p.sink[h], kLog2e, -c_run));
+        if (tok < n_tok) {
+            float f = l > 0.f ? p.out_scale / l : 0.f;
+            if (!ok) f = CUDART_NAN_F;
+            const int r = r0 + tok;
+            if (p.head_gate) f *= p.head_gate[(size_t)r * p.ldg + h];
+            const int c0 = NVS == 1 ? hf * half : hf * 128;
+            const size_t at = (size_t)r * p.ldo + (size_t)h * p.vdim + c0;
+            const float* gate = p.gate ? p.gate + (size_t)r * p.ldg + (size_t)h * p.vdim + c0 : nullptr;
+#pragma unroll
+            for (int c = 0; c < DVH; c += 4) {                // (vdim is a multiple of 4)
+                if (c < n_mine && c0 + c < p.vdim) {
+                    float4 o = make_float4(O[c] * f, O[c + 1] * f, O[c + 2] * f, O[c + 3] * f);
+                    if (gate) {
+                        const float4 z = *reinterpret_cast<const float4*>(gate + c);
+                        o.x *= 1.0f / (1.0f + expf(-z.x)); o.y *= 1.0f / (1.0f + expf(-z.y));
+                        o.z *= 1.0f / (1.0f + expf(-z.z)); o.w *= 1.0f / (1.0f + expf(-z.w));
+                    }
+                    if (p.out) *reinterpret_cast<float4*>(p.out + at + c) = o;
+                    if (p.out_bf16) {
+                        const __nv_bfloat162 a = __floats2bfloat162_rn(o.x, o.y), b = __floats2bfloat162_rn(o.z, o.w);
+                        *reinterpret_cast<uint2*>(reinterpret_cast<__nv_bfloat16*>(p.out_bf16) + at + c) =
+                            make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
+                    }
+                }
+            }
+        }
+    } else if (warp < 12) {
+        // ================= keys and values: warp lw takes keys 16 lw .. + 15 of a tile, a lane one key of either eight =================
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 112;");
+        const int lw = warp - 8, kin = lane & 7, cq = lane >> 3;
+        unsigned at = 0;                                      // ring position
+        unsigned v_turn = 0;
+        bool ok = true;
+        size_t cur[2] = {~(size_t)0, ~(size_t)0}, prev[2];    // row of the two keys in the pages of kv head 0 (~0: none)
+        auto stage = [&](const float* cache, int width, int c0, int w, int wp, int gg, const size_t (&rows)[2], float* inv, bool value) {
+            float4 v[16];
+#pragma unroll
+            for (int kg = 0; kg < 2; ++kg) {
+                const bool in = rows[kg] != ~(size_t)0;
+                const float* src = cache + (in ? (rows[kg] + (size_t)gg * p.page_size) * width + c0 : 0);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const int c = 8 * (cq + 4 * i);
+                    const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
+                    v[kg * 8 + 2 * i] = in && c < w ? *reinterpret_cast<const float4*>(src + c) : z;
+                    v[kg * 8 + 2 * i + 1] = in && c + 4 < w ? *reinterpret_cast<const float4*>(src + c + 4) : z;
+                }
+            }
+            const unsigned slot = at % geo.n_slots;
+            if (!wait_for(&empty[slot], ((at / geo.n_slots) & 1u) ^ 1u)) { ok = false; return; }
+            float m = 0.f;
+#pragma unroll
+            for (int i = 0; i < 16; ++i) m = max_abs4(m, v[i]);
+            m = warp_max_of(m);
+            if (!(m <= 3.402823466e38f)) {                    // an infinity among them: it stays one, the others set the scale
+                m = 0.f;
+#pragma unroll
+                for (int i = 0; i < 16; ++i) m = fmaxf(fmaxf(fmaxf(m, finite_abs(v[i].x)), finite_abs(v[i].y)), fmaxf(finite_abs(v[i].z), finite_abs(v[i].w)));
+                m = warp_max_of(m);
+            }
+            if (value) {                                      // values are summed over the tile's keys: one scale for all of them
+                float* vm = vm_s + (v_turn & 1u) * 4;
+                if (lane == 0) { vm[lw] = m; mbar_arrive(v_max); }
+                if (!wait_for(v_max, v_turn & 1u)) { ok = false; return; }
+                ++v_turn;
+                m = fmaxf(fmaxf(vm[0], vm[1]), fmaxf(vm[2], vm[3]));
+            }
+            float inverse;
+            const float sc = scale_of(m, inverse);
+            if (lane == 0 && (!value || lw == 0)) *inv = inverse;
+            unsigned char* base = ring + (size_t)slot * geo.slot_bytes;
+            const int blocks = wp >> 3;
+#pragma unroll
+            for (int kg = 0; kg < 2; ++kg)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const int c8 = cq + 4 * i;
+                    if (c8 < blocks) {
+                        const float4 a = v[kg * 8 + 2 * i], b = v[kg * 8 + 2 * i + 1];
+                        uint32_t hi[4], lo[4];
+                        split2(a.x * sc, a.y * sc, hi[0], lo[0]);
+                        split2(a.z * sc, a.w * sc, hi[1], lo[1]);
+                        split2(b.x * sc, b.y * sc, hi[2], lo[2]);
+                        split2(b.z * sc, b.w * sc, hi[3], lo[3]);
+                        unsigned char* dst = base + ((lw * 2 + kg) * blocks + c8) * 128 + kin * 16;
+                        *reinterpret_cast<uint4*>(dst) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+                        *reinterpret_cast<uint4*>(dst + kKeys * wp * 2) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+                    }
+                }
+            fence_smem_async();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&full[slot]);
+            ++at;
+        };
+        auto values = [&](unsigned t, const size_t (&rows)[2]) {
+            for (int vs = 0; vs < NVS && ok; ++vs)
+                stage(p.vcache, p.vrow, vs * kGroupW, min(kGroupW, p.vdim - vs * kGroupW), vs == geo.n_vst - 1 ? geo.wv_last : geo.wv0, g, rows,
+                      v_inv + (t % kScaleRing) * 2 + vs, true);
+        };
+        unsigned t = 0;
+        Walk w(s_slot, s_pos, n_tok);
+        for (; ok && w.next(p); ++t) {
+            const int slot = s_slot[w.seg_a];
+#pragma unroll
+            for (int kg = 0; kg < 2; ++kg) {
+                const int j = w.j0 + lw * 16 + kg * 8 + kin;
+                prev[kg] = cur[kg];
+                cur[kg] = ~(size_t)0;
+                if (j < w.k_end) {
+                    const int page = p.table ? p.table[(size_t)slot * p.max_pages + j / p.page_size] : slot;
+                    cur[kg] = (size_t)page * p.kv_heads * p.page_size + (p.table ? j % p.page_size : j);
+                }
+            }
+            for (int st = 0; st < geo.n_kst && ok; ++st)
+                stage(p.kcache, p.kdim, p.talk ? 0 : st * kGroupW, p.talk ? p.kdim : min(kGroupW, p.kdim - st * kGroupW),
+                      st == geo.n_kst - 1 ? geo.wk_last : geo.wk0, p.talk ? st : g, cur,
+                      k_inv + ((t % kScaleRing) * kMaxKStages + st) * 4 + lw, false);
+            if (t > 0 && ok) values(t - 1, prev);
+        }
+        if (t > 0 && ok) values(t - 1, cur);
+    } else {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 32;");
+        if (warp == 12) {
+            // ================= the MMA issuer: the whole warp walks, one elected lane issues =================
+            const uint32_t idesc_s = (1u << 4) | ((uint32_t)(kKeys >> 3) << 17) | ((uint32_t)(kRows >> 4) << 24);
+            const uint32_t q_addr = smem_u32(qs), ring_addr = smem_u32(ring);
+            unsigned at = 0;
+            bool ok = true;
+            auto values = [&](unsigned t) {                   // value product of tile t
+                if (!wait_warp(p_ready, t & 1u)) { ok = false; return; }
+                for (int vs = 0; vs < NVS; ++vs) {
+                    const unsigned slot = at % geo.n_slots;
+                    if (!wait_warp(&full[slot], (at / geo.n_slots) & 1u)) { ok = false; return; }
+                    fence_after();
+                    const uint32_t wp = vs == geo.n_vst - 1 ? geo.wv_last : geo.wv0;
+                    const uint32_t idesc = (1u << 4) | (1u << 16) | ((wp >> 3) << 17) | ((uint32_t)(kRows >> 4) << 24);
+                    const uint32_t va = ring_addr + slot * geo.slot_bytes;
+                    const uint64_t vh = block_desc(va, wp * 16u, 128u), vl = block_desc(va + kKeys * wp * 2u, wp * 16u, 128u);
+                    const uint32_t step = 2u * wp;            // 16 keys, in descriptor units of 16 bytes
+                    const uint32_t d = t_o + 128u * vs;
+                    if (elect_one_sync()) {
+#pragma unroll
+                        for (uint32_t k = 0; k < 4; ++k) mma_ts(d, t_p + 32u + 8u * k, vh + k * step, idesc, k != 0);
+#pragma unroll
+                        for (uint32_t k = 0; k < 4; ++k) mma_ts(d, t_p + 8u * k, vl + k * step, idesc, 1u);
+#pragma unroll
+                        for (uint32_t k = 0; k < 4; ++k) mma_ts(d, t_p + 8u * k, vh + k * step, idesc, 1u);
+                        commit_to(&empty[slot]);
+                        if (vs == NVS - 1) commit_to(pv_done);
+                    }
+                    __syncwarp();
+                    ++at;
+                }
+            };
+            unsigned t = 0;
+            Walk w(s_slot, s_pos, n_tok);
+            for (; ok && w.next(p); ++t) {
+                if (t > 0 && !wait_warp(s_empty, (t - 1) & 1u)) { ok = false; break; }
+                for (int st = 0; st < geo.n_kst; ++st) {
+                    const unsigned slot = at % geo.n_slots;
+                    if (!wait_warp(&full[slot], (at / geo.n_slots) & 1u)) { ok = false; break; }
+                    fence_after();
+                    const uint32_t wp = st == geo.n_kst - 1 ? geo.wk_last : geo.wk0;
+                    const uint32_t ka = ring_addr + slot * geo.slot_bytes, qa = q_addr + st * geo.wk0 * kRows * 4u;
+                    const uint64_t kh = block_desc(ka, 128u, wp * 16u), kl = block_desc(ka + kKeys * wp * 2u, 128u, wp * 16u);
+                    const uint64_t qh = block_desc(qa, 128u, wp * 16u), ql = block_desc(qa + kRows * wp * 2u, 128u, wp * 16u);
+                    const uint32_t d = t_s + 64u * st;
+                    if (elect_one_sync()) {
+                        const uint32_t n = wp >> 4;           // 16 channels per instruction: 2 blocks, 16 descriptor units
+                        for (uint32_t k = 0; k < n; ++k) mma_ss(d, ql + 16u * k, kh + 16u * k, idesc_s, k != 0);
+                        for (uint32_t k = 0; k < n; ++k) mma_ss(d, qh + 16u * k, kl + 16u * k, idesc_s, 1u);
+                        for (uint32_t k = 0; k < n; ++k) mma_ss(d, qh + 16u * k, kh + 16u * k, idesc_s, 1u);
+                        commit_to(&empty[slot]);
+                        if (st == geo.n_kst - 1) commit_to(s_full);
+                    }
+                    __syncwarp();
+                    ++at;
+                }
+                if (t > 0 && ok) values(t - 1);
+            }
+            if (t > 0 && ok) values(t - 1);
+        }
+    }
+    fence_before();
+    __syncthreads();
+    if (warp == 12) {
+        fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem));
+    }
+}
+
+bool geometry_of(const SplitAttention& a, Geometry& g, size_t& smem) {
+    if (a.heads <= 0 || a.kv_heads <= 0 || a.heads % a.kv_heads || a.kdim <= 0 || a.vdim <= 0) return false;
+    auto mul4 = [](int v) { return v % 4 == 0; };
+    auto aligned = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
+    if (!mul4(a.ldq) || !mul4(a.qdim) || !mul4(a.kdim) || !mul4(a.vdim) || !mul4(a.vrow) || !mul4(a.ldo) || !aligned(a.q) || !aligned(a.kcache) ||
+        !aligned(a.vcache) || !aligned(a.out) || (reinterpret_cast<uintptr_t>(a.out_bf16) & 7) || (a.gate && (!mul4(a.ldg) || !aligned(a.gate))))
+        return false;
+    if (a.qdim != a.kdim || a.vdim > 256 || (a.talk && a.kdim > kGroupW)) return false;
+    if (a.rows_per_slot > 0 && (long long)a.rows_per_slot * 16 < a.M) return false;
+    auto pad16 = [](int v) { return (v + 15) & ~15; };
+    const int rep = a.heads / a.kv_heads;
+    g.pk_shift = 0;
+    while (g.pk_shift < 7 && rep % (2 << g.pk_shift) == 0) ++g.pk_shift;
+    if (a.talk) {
+        g.n_kst = a.kv_heads;
+        g.wk0 = g.wk_last = pad16(a.kdim);
+    } else {
+        g.n_kst = (a.kdim + kGroupW - 1) / kGroupW;
+        g.wk0 = pad16(std::min(a.kdim, kGroupW));
+        g.wk_last = pad16(a.kdim - (g.n_kst - 1) * kGroupW);
+    }
+    g.n_vst = (a.vdim + kGroupW - 1) / kGroupW;
+    g.wv0 = pad16(std::min(a.vdim, kGroupW));
+    g.wv_last = pad16(a.vdim - (g.n_vst - 1) * kGroupW);
+    if (g.n_kst > kMaxKStages || 64 * g.n_kst + 64 + 128 * g.n_vst > 512) return false;      // columns of tensor memory
+    g.slot_bytes = kKeys * std::max(g.wk0, g.wv0) * 4;
+    g.q_bytes = ((g.n_kst - 1) * g.wk0 + g.wk_last) * kRows * 4;
+    const int control = (2 * kMaxSlots + 5 + 4) * 8 + (kScaleRing * kMaxKStages * 4 + kScaleRing * 2 + 8 + 4 * kRows) * 4 + 2 * (kRows >> g.pk_shift) * 4;
+    g.n_slots = (kSmemMost - 128 - g.q_bytes - control) / g.slot_bytes;      // (128: the few static words)
+    if (g.n_slots < 2) return false;
+    g.n_slots = std::min(g.n_slots, kMaxSlots);
+    smem = (size_t)g.n_slots * g.slot_bytes + g.q_bytes + control;
+    return true;
+}
+
+template <int NVS>
+cudaError_t launch_inst(const SplitAttention& a, const Geometry& g, size_t smem, cudaStream_t st) {
+    static size_t allowed[64] = {};
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    if (dev < 0 || dev >= 64 || allowed[dev] < smem) {
+        e = cudaFuncSetAttribute(split_attention_kernel<NVS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return e;
+        if (dev >= 0 && dev < 64) allowed[dev] = smem;
+    }
+    const int tt = kRows >> g.pk_shift, tiles = (a.M + tt - 1) / tt;
+    if (tiles > 65535) return cudaErrorNotSupported;
+    split_attention_kernel<NVS><<<dim3(a.heads >> g.pk_shift, tiles), kSplitThreadsTC, smem, st>>>(a, g);
+    return cudaGetLastError();
+}
+
+}  // namespace
+
+bool split_attention_ok(const SplitAttention& a) {
+    Geometry g;
+    size_t smem;
+    return geometry_of(a, g, smem);
+}
+
+cudaError_t launch_split_attention(const SplitAttention& a, cudaStream_t st) {
+    Geometry g;
+    size_t smem;
+    if (a.M <= 0 || !geometry_of(a, g, smem)) return cudaErrorNotSupported;
+    return g.n_vst == 1 ? launch_inst<1>(a, g, smem, st) : launch_inst<2>(a, g, smem, st);
+}
+
+}  // namespace dia

@@ -1,0 +1,44 @@
+// attention_split.h - softmax attention for many query rows on the tensor cores (attention_split.cu).
+//
+// Queries, keys, values and softmax weights are fp32; every product takes them as two fp16 terms of a scaled value (22
+// significand bits) and is accumulated in fp32.  Serves grouped-query attention over paged keys and values, attention over one
+// cached latent per position (the value is the head of the key row), and attention whose scores are mixed across heads.
+#pragma once
+
+#include <cuda_runtime.h>
+
+namespace dia {
+
+struct SplitAttention {
+    // query head h of row r: q + r * ldq + h * qdim, qdim channels
+    const float* q; int ldq; int qdim;
+    // key of (page, kv head, offset): kcache + ((page * kv_heads + g) * page_size + offset) * kdim; the value likewise in vcache
+    // with rows of vrow floats, of which vdim are the value.  table [slot][max_pages] -> page; null: the page is the slot
+    const float* kcache; const float* vcache;
+    const int* table; int max_pages, page_size;
+    int heads, kv_heads, kdim, vdim, vrow;
+    // score = q . k * scale * temp_h, capped (cap > 0: cap tanh(score / cap)), minus slopes_h (i - j); temp, slopes: null: none
+    float scale, cap;
+    const float* temp; const float* slopes;
+    const float* sink;                       // [heads] logits that join the denominator only; null: none
+    const float* talk;                       // [heads][heads]: score_h <- sum_g talk[h][g] score_g before the softmax; null: none
+    // row r: position row_pos[r] of sequence row_slot[r]; rows of a sequence adjacent and in order.  It sees key j <= its
+    // position inside its window (window > 0) and its chunk (chunk > 0), and with a window the first keep_first keys
+    const int* row_slot; const int* row_pos; int M;
+    int window, keep_first, chunk;
+    // rows_per_slot > 0: row r is position r % rows_per_slot of slot r / rows_per_slot (at most 16 slots), and with n = n_valid[slot]
+    // sees, by mode, 0: the keys up to its own position; 1: [0, n) if its position is below n, else [n, n_keys); 2: [0, n)
+    int rows_per_slot, mode, n_keys;
+    int n_valid[16];
+    // out[r * ldo + h * vdim + c] = softmax-weighted value * out_scale [* sigmoid(gate[r * ldg + h * vdim + c])]
+    // [* head_gate[r * ldg + h]], and its bf16 copy (either may be null)
+    float* out; int ldo; void* out_bf16;
+    float out_scale;
+    const float* gate; const float* head_gate; int ldg;
+};
+
+// whether the kernel takes the shape (head sizes, alignment); M does not matter
+bool split_attention_ok(const SplitAttention& a);
+cudaError_t launch_split_attention(const SplitAttention& a, cudaStream_t st);
+
+}  // namespace dia

@@ -179,6 +179,10 @@ bool tensor_path(const lm_b200_engine* e, int M, int N, int K) {
     return e->m.precision == LM_B200_PRECISION_BF16 && M >= kTensorRowsMin && dia::gemm_tcgen05_shape_ok(M, N, K);
 }
 
+// The attention of a prompt portion runs on the tensor cores with split fp32 operands, whatever the precision of the products: its
+// error against 64 bits is that of the fp32 FMA kernels (attention_split.cu).
+bool split_operands(int M) { return M >= kTensorRowsMin; }
+
 const dia::GemmEpilogue kPlain{nullptr, nullptr, nullptr, 0.f, nullptr};
 
 struct StepView {
@@ -475,7 +479,8 @@ int mixer(lm_b200_engine* e, const lm_b200_layer& l, const float* h, const void*
                                  v.rm, M, st));
     const lm::AttnShape a{l.heads, l.kv_heads, l.dim, l.window, l.keep_first, l.scale, l.softcap, l.temp, l.slopes, l.sink};
     const bool tc_o = tensor_path(e, M, D, nq);
-    LCK(lm::launch_sink_attention(e->qk, nq + nk, l.k_pages, l.v_pages, pm, a, v.rm, e->att, tc_o ? e->attb : nullptr, e->split_ws, e->split_arrived, M, st));
+    LCK(lm::launch_sink_attention(e->qk, nq + nk, l.k_pages, l.v_pages, pm, a, v.rm, e->att, tc_o ? e->attb : nullptr, e->split_ws, e->split_arrived, M, st,
+                                  0, 1.f, nullptr, 0, split_operands(M)));
     if (tc_o) {
         if (fuse_x) {
             const dia::GemmEpilogue ep{fuse_x, l.norm_mix_out.w, l.norm_mix_out.b, l.norm_mix_out.alpha, nullptr};
@@ -585,7 +590,7 @@ int mixer_kernels(lm_b200_engine* e, const lm_b200_layer& l, const InCols& c, fl
             LCK(lm::launch_talk_prep(proj, c.n, l.in_bias, c.q, c.k, c.v, c.gate, a, l.q_norm, l.k_norm, e->m.eps, l.k_pages,
                                      l.v_pages, pm, v.rm, M, st));
             LCK(lm::launch_talk_attention(proj, c.n, c.q, c.gate, l.k_pages, l.v_pages, pm, a, v.rm, e->outcat, ko, ob,
-                                          e->split_ws, e->split_arrived, M, st));
+                                          e->split_ws, e->split_arrived, M, st, split_operands(M)));
             break;
         }
         case LM_B200_MIXER_HGRN2: {
@@ -700,7 +705,7 @@ int stream_mixer_kernels(lm_b200_engine* e, const lm_b200_layer& l, const MixPla
             LCK(lm::launch_rot_rows(e->qk, nq, l.dim, dq, e->qlat, nl, l.kv_rank, RK, H, rd, rot, H, l.scale, l.scale, v.rm, M, st));
         if (lm::talk_attention_supported(latent_shape(l)))
             LCK(lm::launch_talk_attention(e->qlat, nl, 0, -1, l.latent_pages, l.latent_pages, pm, latent_shape(l), v.rm, e->olat, no,
-                                          nullptr, e->split_ws, e->split_arrived, M, st));
+                                          nullptr, e->split_ws, e->split_arrived, M, st, split_operands(M)));
         else
             LCK(lm::launch_latent_attention_rows(e->qlat, l.latent_pages, pm, H, l.kv_rank, l.sink, v.rm, e->olat, M, st, rd,
                                                  l.window > 0 ? l.window : 0));
@@ -732,7 +737,7 @@ int stream_mixer_kernels(lm_b200_engine* e, const lm_b200_layer& l, const MixPla
         LCK(lm::launch_talk_prep(proj, ld, nullptr, c.q, c.k, c.v, -1, a, l.q_norm, l.k_norm, e->m.eps, l.k_pages, l.v_pages, pm, v.rm, M, st));
         const lm::AttnShape s{H, l.kv_heads, l.dim, l.window > 0 ? l.window : 0, 0, 1.f, 0.f, nullptr, nullptr, l.sink, l.chunk};
         LCK(lm::launch_sink_attention(proj + c.q, ld, l.k_pages, l.v_pages, pm, s, v.rm, at.out, at.out_b, e->split_ws, e->split_arrived, M,
-                                      st, at.ldo, at.scale, gate, ld));
+                                      st, at.ldo, at.scale, gate, ld, split_operands(M)));
     } else if (l.mixer == LM_B200_MIXER_GATED_LINEAR) {
         LCK(lm::launch_decay_proj(proj + c.a1, ld, l.w_a2, l.dt_bias, l.decay_tau, e->rec, H * l.dim, l.rank_a, M, st));
         const lm::ScanInputs si{c.q, c.k, 0, c.v, 0};
@@ -1361,7 +1366,8 @@ int lm_b200_op_attention(lm_b200_engine* e, int layer, float* qk, const int32_t*
     LCK(lm::launch_qk_norm_cache(qk, nq, nk, l.q_norm, l.k_norm, e->m.eps, l.k_pages, l.v_pages, pm, l.kv_heads, l.dim, v.rm, M,
                                  S(stream)));
     const lm::AttnShape a{l.heads, l.kv_heads, l.dim, l.window, l.keep_first, l.scale, l.softcap, l.temp, l.slopes, l.sink};
-    LCK(lm::launch_sink_attention(qk, nq + nk, l.k_pages, l.v_pages, pm, a, v.rm, out, nullptr, e->split_ws, e->split_arrived, M, S(stream)));
+    LCK(lm::launch_sink_attention(qk, nq + nk, l.k_pages, l.v_pages, pm, a, v.rm, out, nullptr, e->split_ws, e->split_arrived, M, S(stream), 0, 1.f,
+                                  nullptr, 0, split_operands(M)));
     return LM_B200_OK;
 }
 

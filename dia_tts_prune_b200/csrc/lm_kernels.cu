@@ -41,6 +41,7 @@
 #include <math_constants.h>
 #include <stdint.h>
 
+#include "attention_split.h"
 #include "lm_device.cuh"
 #include "lm_internal.h"
 
@@ -1259,11 +1260,23 @@ static cudaError_t launch_attention_splits(const float* qk, int q_stride, const 
 // split_ws: kRowsKernelMax * heads * kAttnSplitsMax * (dim + 2) floats; arrived: kRowsKernelMax * heads zeroed counters
 cudaError_t launch_sink_attention(const float* qk, int q_stride, const float* kcache, const float* vcache, const PageMap& pm,
                                   const AttnShape& a, const RowMeta& rm, float* out, void* out_bf16, float* split_ws,
-                                  unsigned* arrived, int M, cudaStream_t st, int ldo, float out_scale, const float* gate, int ldg) {
+                                  unsigned* arrived, int M, cudaStream_t st, int ldo, float out_scale, const float* gate, int ldg,
+                                  bool tensor_cores) {
     if (ldo <= 0) ldo = a.heads * a.dim;
     if (a.dim > 32 * kAttnMaxDimPerLane || a.heads % a.kv_heads) return cudaErrorNotSupported;
     __nv_bfloat16* ob = reinterpret_cast<__nv_bfloat16*>(out_bf16);
     if (M > kAttnRowsKernelMax) {
+        if (tensor_cores) {
+            dia::SplitAttention s{};
+            s.q = qk; s.ldq = q_stride; s.qdim = a.dim;
+            s.kcache = kcache; s.vcache = vcache; s.table = pm.table; s.max_pages = pm.max_pages; s.page_size = pm.page_size;
+            s.heads = a.heads; s.kv_heads = a.kv_heads; s.kdim = s.vdim = s.vrow = a.dim;
+            s.scale = a.scale; s.cap = a.softcap; s.temp = a.temp; s.slopes = a.slopes; s.sink = a.sink;
+            s.row_slot = rm.slot; s.row_pos = rm.pos; s.M = M;
+            s.window = a.window; s.keep_first = a.keep_first; s.chunk = a.chunk;
+            s.out = out; s.ldo = ldo; s.out_bf16 = out_bf16; s.out_scale = out_scale; s.gate = gate; s.ldg = ldg;
+            if (dia::split_attention_ok(s)) return dia::launch_split_attention(s, st);
+        }
         switch ((a.dim + 63) / 64) {
             case 1: return launch_attention_tiles<1>(qk, q_stride, kcache, vcache, pm, a, rm, out, ob, ldo, out_scale, M, st, gate, ldg);
             case 2: return launch_attention_tiles<2>(qk, q_stride, kcache, vcache, pm, a, rm, out, ob, ldo, out_scale, M, st, gate, ldg);

@@ -33,6 +33,7 @@
 #include <math_constants.h>
 #include <stdint.h>
 
+#include "attention_split.h"
 #include "lm_device.cuh"
 #include "lm_internal.h"
 
@@ -801,9 +802,21 @@ bool talk_attention_supported(const TalkShape& a) {
 // to hide the latencies of a tile's dependent phases); a handful of rows run 8 warps per (row, share of the keys).
 cudaError_t launch_talk_attention(const float* proj, int ld, int q_off, int gate_off, const float* kcache, const float* vcache,
                                   const PageMap& pm, const TalkShape& a, const RowMeta& rm, float* out, int ldo, void* out_bf16,
-                                  float* split_ws, unsigned* arrived, int M, cudaStream_t st) {
+                                  float* split_ws, unsigned* arrived, int M, cudaStream_t st, bool tensor_cores) {
     if (!talk_attention_supported(a)) return cudaErrorNotSupported;
     __nv_bfloat16* ob = reinterpret_cast<__nv_bfloat16*>(out_bf16);
+    if (tensor_cores && M > kAttnRowsKernelMax) {
+        dia::SplitAttention s{};
+        const bool latent = kcache == vcache;                 // the value is the head of the key row
+        s.q = proj + q_off; s.ldq = ld; s.qdim = a.dim;
+        s.kcache = kcache; s.vcache = vcache; s.table = pm.table; s.max_pages = pm.max_pages; s.page_size = pm.page_size;
+        s.heads = a.heads; s.kv_heads = a.kv_heads; s.kdim = a.dim; s.vdim = a.vdim; s.vrow = latent ? a.dim : a.vdim;
+        s.scale = 1.f; s.sink = a.sink; s.talk = a.talk;
+        s.row_slot = rm.slot; s.row_pos = rm.pos; s.M = M; s.window = a.window;
+        s.out = out; s.ldo = ldo; s.out_bf16 = out_bf16; s.out_scale = 1.f;
+        if (gate_off >= 0) { s.head_gate = proj + gate_off; s.ldg = ld; }
+        if (dia::split_attention_ok(s)) return dia::launch_split_attention(s, st);
+    }
     const int vu = (a.vdim + 31) / 32;
 #define TALK_CASE(VU, NP, NW) \
     return launch_talk_inst<VU, NP, NW>(proj, ld, q_off, gate_off, kcache, vcache, pm, a, rm, out, ldo, ob, split_ws, arrived, M, TQ, S, st)

@@ -1,0 +1,108 @@
+"""The tensor-core attention with split fp32 operands (csrc/attention_split.cu) at the sizes where it can go wrong: edges of its
+tiles of 64 keys and 128 (token, head) rows, channel groups, segments of several sequences, windows, magnitudes far from one."""
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def close(got, ref, scale):
+    """fp32 arithmetic: 22-bit terms and fp32 sums.  A score is off by at most about 2^-21 |q| |k| and a weighted sum by 2^-21 of the
+    largest value, so 2e-5 of the result's largest magnitude leaves a factor of ten."""
+    assert torch.isfinite(got).all()
+    err = (got.double().cpu() - ref).abs().max().item()
+    assert err <= 2e-5 * scale, (err, scale)
+
+
+def sink_reference(x, past, H, G, d, p, window, keep, cap, eps):
+    n = x.shape[0]
+    q, raw = x[past:, :H * d], x[:, H * d:]
+    rms = lambda t: t / torch.sqrt((t * t).mean(-1, keepdim=True) + eps)      # noqa: E731
+    q, k, v = (rms(q) * p["q"]).reshape(-1, H, d), (rms(raw) * p["k"]).reshape(n, G, d), raw.reshape(n, G, d)
+    i, j = torch.arange(past, n)[:, None], torch.arange(n)[None]
+    ok = j <= i
+    if window:
+        ok = ok & ((i - j < window) | (j < keep))
+    out = []
+    for h in range(H):
+        s = q[:, h] @ k[:, h * G // H].T * (d ** -0.5 * p["temp"][h])
+        if cap:
+            s = cap * torch.tanh(s / cap)
+        s = (s - 2.0 ** (-8.0 * (h + 1) / H) * (i - j)).masked_fill(~ok, -torch.inf)
+        m = torch.maximum(s.max(-1, keepdim=True).values, p["sink"][h])
+        e = torch.exp(s - m)
+        out.append(e @ v[:, h * G // H] / (e.sum(-1, keepdim=True) + torch.exp(p["sink"][h] - m)))
+    return torch.stack(out, 1).reshape(n - past, H * d)
+
+
+@pytest.mark.parametrize("rows,past,H,G,d,window,keep,cap,amp,page", [
+    ([64], 0, 4, 1, 128, 0, 0, 0.0, 1.0, 64),           # one key tile
+    ([65], 0, 1, 1, 128, 0, 0, 30.0, 1.0, 16),          # one key more; one head per row tile
+    ([32], 33, 8, 2, 64, 0, 0, 0.0, 1e-4, 16),          # a portion behind cached keys; small values
+    ([127, 1, 2], 0, 4, 4, 16, 0, 0, 0.0, 1e4, 64),     # 128 tokens of a row tile: the last segments in the next one; large values
+    ([40, 90], 70, 6, 2, 96, 33, 3, 30.0, 1.0, 16),     # two heads per tile, a window that keeps the first keys
+    ([130], 0, 8, 1, 200, 100, 200, 0.0, 1.0, 64),      # two channel groups, more kept keys than the window starts behind
+    ([70], 0, 16, 1, 256, 0, 0, 0.0, 1.0, 64),          # the widest heads
+    ([33], 0, 3, 1, 20, 5, 1, 0.0, 1.0, 7),             # channels that are no multiple of 16, odd pages
+])
+def test_grouped_query_attention(rows, past, H, G, d, window, keep, cap, amp, page):
+    from dia_tts_prune_b200 import synthetic as SY
+    from dia_tts_prune_b200.lm_config import PubopelConfig
+    from dia_tts_prune_b200.lm_model import CausalLM
+    cfg = SY.pubopel_config(width=32, layers=1, heads=H, kv_heads=G, dim=d, experts=1, top=1, expert_ff=8, shared_ff=None, vocab=64,
+                            window=window or None, keep_first=keep, softcap=cap or None)
+    w = SY.pubopel_weights(cfg, 3)
+    model = CausalLM(PubopelConfig.model_validate(cfg), w, dtype="bfloat16", device="cuda:0", max_tokens=2048, max_sequences=4,
+                     page_size=page, max_rows=512)
+    p = {n: w[f"l0.mix.{t}"].double() for n, t in (("q", "q.norm"), ("k", "k.norm"), ("temp", "temp"), ("sink", "sink"))}
+    g = torch.Generator().manual_seed(5)
+    x = [torch.randn((past + n, (H + G) * d), generator=g) * amp for n in rows]
+    seqs = [model.state.open(str(i)) for i in range(len(rows))]
+    for s, t in zip(seqs, x):
+        model.state.reserve(s, len(t))
+        if past:
+            model.engine.op_attention(0, t[:past].cuda(), [(s, past, 0)])
+    got = model.engine.op_attention(0, torch.cat([t[past:] for t in x]).cuda(), [(s, n, past) for s, n in zip(seqs, rows)])
+    ref = torch.cat([sink_reference(t.double(), past, H, G, d, p, window, keep, cap, cfg["norm"]["eps"]) for t in x])
+    close(got, ref, ref.abs().max().item())
+
+
+@pytest.mark.parametrize("H,G,d,dv,rows", [(8, 2, 128, 128, [70, 1]), (4, 4, 64, 32, [64]), (12, 3, 40, 24, [33, 5]), (16, 1, 24, 256, [65])])
+def test_mixed_scores(H, G, d, dv, rows):
+    """Scores mixed across heads: the kernel mixes the queries instead, against the mixer's definition in 64 bits."""
+    from dia_tts_prune_b200 import synthetic as SY
+    from dia_tts_prune_b200.lm_config import KupelixConfig
+    from dia_tts_prune_b200.lm_model import CausalLM
+    cfg = SY.kupelix_config(width=32, kinds=["attention"], heads=H, kv_heads=G, dim=d, vdim=dv, ff=8, vocab=64)
+    cfg["layers"][0]["mixer"]["rot"] = None
+    w = SY.kupelix_weights(cfg, 3)
+    cfg["layers"][0]["mlp"] = None
+    model = CausalLM(KupelixConfig.model_validate(cfg), w, dtype="bfloat16", device="cuda:0", max_tokens=512, max_sequences=2, max_rows=128)
+    n_in = model.layers[0].layer.n_in
+    g = torch.Generator().manual_seed(6)
+    x = [torch.randn((n, n_in), generator=g) for n in rows]
+    seqs = [model.state.open(str(i)) for i in range(len(rows))]
+    for s, n in zip(seqs, rows):
+        model.state.reserve(s, n)
+    got = model.engine.op_mixer_kernels(0, torch.cat(x).cuda(), [(s, n, 0) for s, n in zip(seqs, rows)])
+    p = {n[len("l0.mix."):]: t.double() for n, t in w.items() if n.startswith("l0.mix.")}
+    ref = []
+    for t in x:
+        t, n = t.double(), t.shape[0]
+        nq, nk = H * d, G * d
+        rms = lambda a: a / torch.sqrt((a * a).mean(-1, keepdim=True) + cfg["norm"]["eps"])      # noqa: E731
+        q = rms((t[:, :nq] + p["q.b"]).reshape(n, H, d)) * p["q.norm"]
+        k = rms((t[:, nq:nq + nk] + p["k.b"]).reshape(n, G, d)) * p["k.norm"]
+        v = (t[:, nq + nk:nq + nk + G * dv] + p["v.b"]).reshape(n, G, dv)
+        raw = torch.stack([q[:, h] @ k[:, h * G // H].T for h in range(H)]) * cfg["layers"][0]["mixer"]["scale"]
+        mixed = torch.einsum("hg,gij->hij", p["talk"], raw).masked_fill(torch.ones(n, n).triu(1).bool(), -torch.inf)
+        gate = torch.sigmoid(t[:, nq + nk + G * dv:nq + nk + G * dv + H])
+        out = []
+        for h in range(H):
+            m = torch.maximum(mixed[h].max(-1, keepdim=True).values, p["sink"][h])
+            e = torch.exp(mixed[h] - m)
+            out.append(e @ v[:, h * G // H] / (e.sum(-1, keepdim=True) + torch.exp(p["sink"][h] - m)) * gate[:, h:h + 1])
+        ref.append(torch.stack(out, 1).reshape(n, H * dv))
+    ref = torch.cat(ref)
+    close(got, ref, ref.abs().max().item())
