@@ -44,6 +44,7 @@ constexpr int kMaxSlots = 6, kScaleRing = 8, kMaxKStages = 4;
 constexpr int kSmemMost = 232448;
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr float kWeightScale = 16384.f;                       // on the softmax weights (at most 1) before the split
+constexpr int kSplitOnceRows = 512;                           // rows of a kv head (M rep) from which the keys are split in advance
 constexpr unsigned kSpinMost = 4000000u;
 
 struct Geometry {
@@ -51,8 +52,17 @@ struct Geometry {
     int n_kst, n_vst;                        // channel groups of a key, of a value
     int wk0, wk_last;                        // their padded widths (multiples of 16): all but the last, the last
     int wv0, wv_last;
+    int v0_layout, v_last_layout;            // widths in which the value groups lie in a slot (a latent's value group is its key group)
+    int shared_kv;                           // the value is the head of the key row: value group i is key group i
     int slot_bytes, n_slots, q_bytes;
+    // the split keys and values in SplitAttention::work: SlotTiles per slot, then inverse scales [tile][part], then the tiles.  A
+    // tile's parts: key groups (per kv head where the launch reads one head at a time), then value groups
+    int parts, k_parts, cap_tiles;
+    unsigned tile_bytes, scale_off, tile_off;
 };
+// where the tiles of a slot's sequence lie: tile j / 64 of its keys is tile base + j / 64 of the room for first <= j / 64 < end; its
+// tile 0 is tile `zero` (-1: only by the range)
+struct SlotTiles { int base, first, end, zero; };
 
 __device__ __forceinline__ bool wait_for(uint64_t* bar, uint32_t parity) {
     for (unsigned i = 0; i < kSpinMost; ++i)
@@ -136,9 +146,120 @@ __device__ __forceinline__ int first_key_of(int i, int window, int chunk) {
     return chunk > 0 ? max(w, i - i % chunk) : w;
 }
 
+__device__ __forceinline__ size_t part_offset(const Geometry& geo, int part) {
+    const unsigned k_head = kKeys * 4u * ((geo.n_kst - 1) * geo.wk0 + geo.wk_last), v_head = kKeys * 4u * ((geo.n_vst - 1) * geo.wv0 + geo.wv_last);
+    if (part < geo.k_parts) return (size_t)(part / geo.n_kst) * k_head + (size_t)(part % geo.n_kst) * geo.wk0 * kKeys * 4;
+    part -= geo.k_parts;
+    return (size_t)(geo.k_parts / geo.n_kst) * k_head + (size_t)(part / geo.n_vst) * v_head + (size_t)(part % geo.n_vst) * geo.wv0 * kKeys * 4;
+}
+
+// Splits the keys and values that the step's rows see, once for all row tiles: without it each of the M rep / 128 row tiles of a
+// key/value head converts every tile it walks, and that conversion (two thirds of the instructions) bounds the kernel below.
+// One CTA per (tile of the room, part); tiles are dealt to the sequences in order.  Warp w takes keys 8 w .. of the tile.
+__global__ void __launch_bounds__(256)
+split_keys_kernel(const __grid_constant__ SplitAttention p, const __grid_constant__ Geometry geo) {
+    __shared__ int s_first, s_seq, s_run;
+    __shared__ float s_m[8];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, tile = blockIdx.x, part = blockIdx.y;
+    const bool writes_plan = tile == 0 && part == 0;
+    SlotTiles* plan = reinterpret_cast<SlotTiles*>(p.work);
+    // ---- which sequence's tile is this? ----
+    if (tid == 0) { s_seq = -1; s_run = 0; }
+    __syncthreads();
+    for (int s0 = 0; s0 < p.n_seq; s0 += 32) {                // warp 0: 32 sequences at a time, running sum of their tiles
+        if (warp == 0) {
+            const int s = s0 + lane;
+            int first = 0, n = 0, slot = 0, extra = 0, end = 0;
+            if (s < p.n_seq) {
+                slot = p.seq_slot[s];
+                const int r = p.seq_row0[s], pos = p.row_pos[r];
+                first = first_key_of(pos, p.window, p.chunk) / kKeys;
+                end = (pos + p.seq_count[s] + kKeys - 1) / kKeys;
+                extra = p.window > 0 && p.keep_first > 0 && first > 0 ? 1 : 0;    // tile 0 holds the kept keys (of at most 64)
+                n = end - first + extra;
+            }
+            int sum = n;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int v = __shfl_up_sync(0xffffffffu, sum, o);
+                if (lane >= o) sum += v;
+            }
+            const int begin = s_run + sum - n;
+            if (writes_plan && s < p.n_seq) {
+                SlotTiles t;
+                t.zero = extra && begin < geo.cap_tiles ? begin : -1;
+                t.base = begin + extra - first;
+                t.first = first;
+                t.end = min(end, geo.cap_tiles - t.base);
+                plan[slot] = t;
+            }
+            if (s < p.n_seq && tile >= begin && tile < begin + n) {
+                s_seq = s;
+                s_first = extra && tile == begin ? 0 : first + tile - begin - extra;
+            }
+            __syncwarp();
+            if (lane == 31) s_run += sum;
+            __syncwarp();
+        }
+        __syncthreads();
+        if (s_seq >= 0 && !writes_plan) break;                // (the same for all threads: read behind the barrier)
+        __syncthreads();
+    }
+    if (s_seq < 0) return;
+    const int seq = s_seq, slot = p.seq_slot[seq], pos0 = p.row_pos[p.seq_row0[seq]], k_end = pos0 + p.seq_count[seq], j0 = s_first * kKeys;
+    // ---- which rows and channels? ----
+    const bool is_v = part >= geo.k_parts;
+    const int q = is_v ? part - geo.k_parts : part, per = is_v ? geo.n_vst : geo.n_kst, gg = q / per, st = q % per;
+    const bool talk = p.talk != nullptr && !is_v;             // (a key group is a whole kv head there)
+    const int g = talk ? st : gg, c0 = talk ? 0 : st * kGroupW;
+    const int w = talk ? p.kdim : min(kGroupW, (is_v ? p.vdim : p.kdim) - c0), wp = is_v ? (st == per - 1 ? geo.wv_last : geo.wv0) : (st == per - 1 ? geo.wk_last : geo.wk0);
+    const int width = is_v ? p.vrow : p.kdim, kin = lane & 7, cq = lane >> 3, j = j0 + warp * 8 + kin, blocks = wp >> 3;
+    const bool in = j < k_end;
+    const float* src = is_v ? p.vcache : p.kcache;
+    if (in) {
+        const int page = p.table[(size_t)slot * p.max_pages + j / p.page_size];
+        src += (((size_t)page * p.kv_heads + g) * p.page_size + j % p.page_size) * width + c0;
+    }
+    float4 v[8];
+    float m = 0.f;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int c = 8 * (cq + 4 * i);
+        const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
+        v[2 * i] = in && c < w ? *reinterpret_cast<const float4*>(src + c) : z;
+        v[2 * i + 1] = in && c + 4 < w ? *reinterpret_cast<const float4*>(src + c + 4) : z;
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) m = fmaxf(fmaxf(fmaxf(m, finite_abs(v[i].x)), finite_abs(v[i].y)), fmaxf(finite_abs(v[i].z), finite_abs(v[i].w)));
+    m = warp_max_of(m);
+    if (lane == 0) s_m[warp] = m;
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 8; ++i) m = fmaxf(m, s_m[i]);
+    float inverse;
+    const float sc = scale_of(m, inverse);
+    unsigned char* work = reinterpret_cast<unsigned char*>(p.work);
+    if (tid == 0) *reinterpret_cast<float*>(work + geo.scale_off + 4 * ((size_t)tile * geo.parts + part)) = inverse;
+    unsigned char* base = work + geo.tile_off + (size_t)tile * geo.tile_bytes + part_offset(geo, part);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int c8 = cq + 4 * i;
+        if (c8 >= blocks) continue;
+        uint32_t hi[4], lo[4];
+        split2(v[2 * i].x * sc, v[2 * i].y * sc, hi[0], lo[0]);
+        split2(v[2 * i].z * sc, v[2 * i].w * sc, hi[1], lo[1]);
+        split2(v[2 * i + 1].x * sc, v[2 * i + 1].y * sc, hi[2], lo[2]);
+        split2(v[2 * i + 1].z * sc, v[2 * i + 1].w * sc, hi[3], lo[3]);
+        unsigned char* dst = base + (warp * blocks + c8) * 128 + kin * 16;
+        *reinterpret_cast<uint4*>(dst) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+        *reinterpret_cast<uint4*>(dst + kKeys * wp * 2) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+    }
+}
+
 // The key tiles of a CTA in the order in which every role walks them.  A segment is a maximal run of the CTA's tokens with one
 // slot and consecutive positions (and, by row mode 1, on one side of n); its keys are the kept first positions in front of its
-// window range (phase 0), then the range from its first token's first key on (phase 1).
+// window range (phase 0), then the range from its first token's first key on (phase 1).  Tiles start on multiples of 64 (keys in
+// front of a token's first key are masked), so that a tile split in advance serves every row tile.
 struct Walk {
     const int* s_slot; const int* s_pos;
     int n, seg_a, seg_b, phase, j0, k_end, lo;
@@ -153,6 +274,7 @@ struct Walk {
                 phase = 1;
                 j0 = lo;
                 k_end = s_pos[seg_b - 1] + 1;
+                if (p.rows_per_slot > 0) k_end = min(k_end, p.n_keys);
                 continue;
             }
             seg_a = seg_b;
@@ -165,11 +287,12 @@ struct Walk {
             if (p.rows_per_slot > 0 && p.mode != 0) {
                 const bool tail = p.mode == 1 && s_pos[seg_a] >= nv;
                 phase = 1;
-                j0 = tail ? nv : 0;
+                lo = tail ? nv : 0;
+                j0 = lo & ~(kKeys - 1);
                 k_end = tail ? p.n_keys : min(nv, p.n_keys);
                 continue;
             }
-            lo = first_key_of(s_pos[seg_a], p.window, p.chunk);
+            lo = first_key_of(s_pos[seg_a], p.window, p.chunk) & ~(kKeys - 1);
             phase = 0;
             j0 = 0;
             k_end = p.window > 0 ? min(p.keep_first, lo) : 0;
@@ -372,7 +495,7 @@ split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_co
                 for (int e = 0; e < 32; ++e) s[e] -= slope * (base - (float)e);
             }
             const bool live = tok >= w.seg_a && tok < w.seg_b;
-            const int last = live ? min(w.k_end - 1, ranged ? 0x7fffffff : my_pos) : -1, first = ranged ? 0 : my_lo;
+            const int last = live ? min(w.k_end - 1, ranged ? 0x7fffffff : my_pos) : -1, first = ranged ? w.lo : my_lo;
             if (!__all_sync(0xffffffffu, k0 + 31 <= last && (k0 >= first || k0 + 31 < kept))) {
 #pragma unroll
                 for (int e = 0; e < 32; ++e) {
@@ -462,6 +585,36 @@ split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_co
         unsigned v_turn = 0;
         bool ok = true;
         size_t cur[2] = {~(size_t)0, ~(size_t)0}, prev[2];    // row of the two keys in the pages of kv head 0 (~0: none)
+        const SlotTiles* const plan = reinterpret_cast<const SlotTiles*>(p.work);
+        auto split_tile = [&](int slot, int j0) -> int {      // the tile of the room that holds these keys (-1: none)
+            if (!plan) return -1;
+            const SlotTiles s = plan[slot];
+            const int j = j0 / kKeys;
+            return j >= s.first && j < s.end ? s.base + j : j == 0 ? s.zero : -1;
+        };
+        auto copied = [&](int tile, int part, unsigned bytes, float* inv, int n_inv) {    // a part that is split already
+            const unsigned slot = at % geo.n_slots;
+            if (lane == 0) {
+                const unsigned char* work = reinterpret_cast<const unsigned char*>(p.work);
+                float scale = 0.f;
+                if (lw == 1) scale = *reinterpret_cast<const float*>(work + geo.scale_off + 4 * ((size_t)tile * geo.parts + part));
+                ok = wait_for(&empty[slot], ((at / geo.n_slots) & 1u) ^ 1u);
+                if (ok && lw == 0) {
+                    mbar_arrive_expect_tx(&full[slot], bytes);
+                    const size_t off = (size_t)tile * geo.tile_bytes + part_offset(geo, part);
+                    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                                     smem_u32(ring + (size_t)slot * geo.slot_bytes)),
+                                 "l"(work + geo.tile_off + off), "r"(bytes), "r"(smem_u32(&full[slot]))
+                                 : "memory");
+                } else if (ok) {
+                    if (lw == 1)
+                        for (int i = 0; i < n_inv; ++i) inv[i] = scale;
+                    mbar_arrive(&full[slot]);
+                }
+            }
+            ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
+            ++at;
+        };
         auto stage = [&](const float* cache, int width, int c0, int w, int wp, int gg, const size_t (&rows)[2], float* inv, bool value) {
             float4 v[16];
 #pragma unroll
@@ -522,32 +675,45 @@ split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_co
             if (lane == 0) mbar_arrive(&full[slot]);
             ++at;
         };
-        auto values = [&](unsigned t, const size_t (&rows)[2]) {
-            for (int vs = 0; vs < NVS && ok; ++vs)
-                stage(p.vcache, p.vrow, vs * kGroupW, min(kGroupW, p.vdim - vs * kGroupW), vs == geo.n_vst - 1 ? geo.wv_last : geo.wv0, g, rows,
-                      v_inv + (t % kScaleRing) * 2 + vs, true);
+        auto values = [&](unsigned t, const size_t (&rows)[2], int tile) {
+            for (int vs = 0; vs < NVS && ok; ++vs) {
+                const int wl = vs == geo.n_vst - 1 ? geo.v_last_layout : geo.v0_layout;
+                float* inv = v_inv + (t % kScaleRing) * 2 + vs;
+                if (tile >= 0)
+                    copied(tile, geo.shared_kv ? vs : geo.k_parts + g * geo.n_vst + vs, kKeys * wl * 4, inv, 1);
+                else
+                    stage(p.vcache, p.vrow, vs * kGroupW, min(kGroupW, (geo.shared_kv ? p.kdim : p.vdim) - vs * kGroupW), wl, g, rows, inv, true);
+            }
         };
+        int tile = -1, prev_tile = -1;
         unsigned t = 0;
         Walk w(s_slot, s_pos, n_tok);
         for (; ok && w.next(p); ++t) {
             const int slot = s_slot[w.seg_a];
+            prev_tile = tile;
+            tile = split_tile(slot, w.j0);
 #pragma unroll
             for (int kg = 0; kg < 2; ++kg) {
                 const int j = w.j0 + lw * 16 + kg * 8 + kin;
                 prev[kg] = cur[kg];
                 cur[kg] = ~(size_t)0;
-                if (j < w.k_end) {
+                if (tile < 0 && j < w.k_end) {
                     const int page = p.table ? p.table[(size_t)slot * p.max_pages + j / p.page_size] : slot;
                     cur[kg] = (size_t)page * p.kv_heads * p.page_size + (p.table ? j % p.page_size : j);
                 }
             }
-            for (int st = 0; st < geo.n_kst && ok; ++st)
-                stage(p.kcache, p.kdim, p.talk ? 0 : st * kGroupW, p.talk ? p.kdim : min(kGroupW, p.kdim - st * kGroupW),
-                      st == geo.n_kst - 1 ? geo.wk_last : geo.wk0, p.talk ? st : g, cur,
-                      k_inv + ((t % kScaleRing) * kMaxKStages + st) * 4 + lw, false);
-            if (t > 0 && ok) values(t - 1, prev);
+            for (int st = 0; st < geo.n_kst && ok; ++st) {
+                const int wp = st == geo.n_kst - 1 ? geo.wk_last : geo.wk0;
+                float* inv = k_inv + ((t % kScaleRing) * kMaxKStages + st) * 4;
+                if (tile >= 0)
+                    copied(tile, p.talk ? st : g * geo.n_kst + st, kKeys * wp * 4, inv, 4);
+                else
+                    stage(p.kcache, p.kdim, p.talk ? 0 : st * kGroupW, p.talk ? p.kdim : min(kGroupW, p.kdim - st * kGroupW), wp, p.talk ? st : g, cur,
+                          inv + lw, false);
+            }
+            if (t > 0 && ok) values(t - 1, prev, prev_tile);
         }
-        if (t > 0 && ok) values(t - 1, cur);
+        if (t > 0 && ok) values(t - 1, cur, tile);
     } else {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 32;");
         if (warp == 12) {
@@ -562,8 +728,8 @@ split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_co
                     const unsigned slot = at % geo.n_slots;
                     if (!wait_warp(&full[slot], (at / geo.n_slots) & 1u)) { ok = false; return; }
                     fence_after();
-                    const uint32_t wp = vs == geo.n_vst - 1 ? geo.wv_last : geo.wv0;
-                    const uint32_t idesc = (1u << 4) | (1u << 16) | ((wp >> 3) << 17) | ((uint32_t)(kRows >> 4) << 24);
+                    const uint32_t wn = vs == geo.n_vst - 1 ? geo.wv_last : geo.wv0, wp = vs == geo.n_vst - 1 ? geo.v_last_layout : geo.v0_layout;
+                    const uint32_t idesc = (1u << 4) | (1u << 16) | ((wn >> 3) << 17) | ((uint32_t)(kRows >> 4) << 24);
                     const uint32_t va = ring_addr + slot * geo.slot_bytes;
                     const uint64_t vh = block_desc(va, wp * 16u, 128u), vl = block_desc(va + kKeys * wp * 2u, wp * 16u, 128u);
                     const uint32_t step = 2u * wp;            // 16 keys, in descriptor units of 16 bytes
@@ -644,7 +810,25 @@ bool geometry_of(const SplitAttention& a, Geometry& g, size_t& smem) {
     g.wv0 = pad16(std::min(a.vdim, kGroupW));
     g.wv_last = pad16(a.vdim - (g.n_vst - 1) * kGroupW);
     if (g.n_kst > kMaxKStages || 64 * g.n_kst + 64 + 128 * g.n_vst > 512) return false;      // columns of tensor memory
-    g.slot_bytes = kKeys * std::max(g.wk0, g.wv0) * 4;
+    g.shared_kv = a.kcache == a.vcache && a.kv_heads == 1 && !a.talk && a.vrow == a.kdim && a.vdim <= a.kdim;
+    g.v0_layout = g.wv0;
+    g.v_last_layout = g.wv_last;
+    if (g.shared_kv) {                                        // value group i lies in key group i
+        g.v0_layout = g.n_kst == 1 ? g.wk_last : g.wk0;
+        g.v_last_layout = g.n_vst == g.n_kst ? g.wk_last : g.wk0;
+    }
+    const int k_heads = a.talk ? 1 : a.kv_heads;              // (a mixed score's key groups are all kv heads)
+    g.k_parts = k_heads * g.n_kst;
+    g.parts = g.k_parts + (g.shared_kv ? 0 : a.kv_heads * g.n_vst);
+    g.tile_bytes = kKeys * 4u * (k_heads * ((g.n_kst - 1) * g.wk0 + g.wk_last) + (g.shared_kv ? 0 : a.kv_heads * ((g.n_vst - 1) * g.wv0 + g.wv_last)));
+    g.cap_tiles = 0;
+    if (a.work && a.table && a.rows_per_slot <= 0 && a.n_seq > 0 && aligned(a.work)) {
+        g.scale_off = (unsigned)a.n_slots * sizeof(SlotTiles);
+        const size_t per = g.tile_bytes + 4u * g.parts, fixed = g.scale_off + 128;
+        if (a.work_bytes > fixed) g.cap_tiles = (int)std::min<size_t>((a.work_bytes - fixed) / per, 65535);
+        g.tile_off = (unsigned)((g.scale_off + 4u * g.parts * (unsigned)g.cap_tiles + 127u) & ~127u);
+    }
+    g.slot_bytes = kKeys * std::max(g.wk0, std::max(g.wv0, g.v0_layout)) * 4;
     g.q_bytes = ((g.n_kst - 1) * g.wk0 + g.wk_last) * kRows * 4;
     const int control = (2 * kMaxSlots + 5 + 4) * 8 + (kScaleRing * kMaxKStages * 4 + kScaleRing * 2 + 8 + 4 * kRows) * 4 + 2 * (kRows >> g.pk_shift) * 4;
     g.n_slots = (kSmemMost - 128 - g.q_bytes - control) / g.slot_bytes;      // (128: the few static words)
@@ -667,6 +851,7 @@ cudaError_t launch_inst(const SplitAttention& a, const Geometry& g, size_t smem,
     }
     const int tt = kRows >> g.pk_shift, tiles = (a.M + tt - 1) / tt;
     if (tiles > 65535) return cudaErrorNotSupported;
+    if (a.work) split_keys_kernel<<<dim3(g.cap_tiles, g.parts), 256, 0, st>>>(a, g);
     split_attention_kernel<NVS><<<dim3(a.heads >> g.pk_shift, tiles), kSplitThreadsTC, smem, st>>>(a, g);
     return cudaGetLastError();
 }
@@ -679,11 +864,20 @@ bool split_attention_ok(const SplitAttention& a) {
     return geometry_of(a, g, smem);
 }
 
+size_t split_attention_work_bytes(const SplitAttention& a, int keys) {
+    Geometry g;
+    size_t smem;
+    if (!geometry_of(a, g, smem)) return 0;
+    return (size_t)a.n_slots * sizeof(SlotTiles) + 256 + (size_t)((keys + kKeys - 1) / kKeys) * (g.tile_bytes + 4u * g.parts);
+}
+
 cudaError_t launch_split_attention(const SplitAttention& a, cudaStream_t st) {
     Geometry g;
     size_t smem;
     if (a.M <= 0 || !geometry_of(a, g, smem)) return cudaErrorNotSupported;
-    return g.n_vst == 1 ? launch_inst<1>(a, g, smem, st) : launch_inst<2>(a, g, smem, st);
+    SplitAttention with = a;
+    if (g.cap_tiles <= 0 || (long long)a.M * (a.heads / a.kv_heads) < kSplitOnceRows) with.work = nullptr;
+    return g.n_vst == 1 ? launch_inst<1>(with, g, smem, st) : launch_inst<2>(with, g, smem, st);
 }
 
 }  // namespace dia

@@ -35,10 +35,17 @@ struct SplitAttention {
     float* out; int ldo; void* out_bf16;
     float out_scale;
     const float* gate; const float* head_gate; int ldg;
+    // Optional: room in which a launch in front splits the keys and values that the rows see once for all row tiles (null: every row
+    // tile splits them for itself).  seq_*: per sequence its slot, first row and row count; n_slots: slots there are.  Keys beyond
+    // the room's size are split by the row tiles.
+    void* work; size_t work_bytes; int n_slots;
+    const int* seq_slot; const int* seq_row0; const int* seq_count; int n_seq;
 };
 
 // whether the kernel takes the shape (head sizes, alignment); M does not matter
 bool split_attention_ok(const SplitAttention& a);
+// bytes of `work` for `keys` keys of this shape (0: the shape is not taken)
+size_t split_attention_work_bytes(const SplitAttention& a, int keys);
 cudaError_t launch_split_attention(const SplitAttention& a, cudaStream_t st);
 
 }  // namespace dia

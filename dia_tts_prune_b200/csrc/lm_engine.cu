@@ -90,6 +90,7 @@
 
 #include <cuda_runtime.h>
 
+#include "attention_split.h"
 #include "gemm_tcgen05.h"
 #include "lm_b200.h"
 #include "lm_internal.h"
@@ -156,6 +157,8 @@ struct lm_b200_engine {
     bool stream_form = false;
     float* split_ws;                             // partial results of the key splits of a few rows' attention
     unsigned* split_arrived;                     // ... and their arrival counters (zero between launches)
+    void* kv_split;                              // keys and values of a long step's attention, split for the tensor cores
+    size_t kv_split_bytes;
     // steps of a few rows are captured once per (rows, sequences, wanted) into a CUDA graph over these fixed buffers
     int32_t* step_static = nullptr;
     float* logits_static = nullptr;
@@ -179,16 +182,13 @@ bool tensor_path(const lm_b200_engine* e, int M, int N, int K) {
     return e->m.precision == LM_B200_PRECISION_BF16 && M >= kTensorRowsMin && dia::gemm_tcgen05_shape_ok(M, N, K);
 }
 
-// The attention of a prompt portion runs on the tensor cores with split fp32 operands, whatever the precision of the products: its
-// error against 64 bits is that of the fp32 FMA kernels (attention_split.cu).
-bool split_operands(int M) { return M >= kTensorRowsMin; }
-
 const dia::GemmEpilogue kPlain{nullptr, nullptr, nullptr, 0.f, nullptr};
 
 struct StepView {
     const int *token, *want;
     lm::RowMeta rm;
     lm::SeqMeta sm;
+    int n_seq;
 };
 StepView view(const int32_t* step, int M, int n_seq) {
     StepView v;
@@ -197,7 +197,15 @@ StepView view(const int32_t* step, int M, int n_seq) {
     const int32_t* s = step + 4 * (size_t)M;
     v.sm = lm::SeqMeta{s, s + n_seq, s + 2 * (size_t)n_seq};
     v.want = s + 3 * (size_t)n_seq;
+    v.n_seq = n_seq;
     return v;
+}
+
+// The attention of more than a few rows runs on the tensor cores with split fp32 operands, whatever the precision of the products: its
+// error against 64 bits is that of the fp32 FMA kernels (attention_split.cu).
+struct SplitUse { lm::SplitRoom room; bool use; operator const lm::SplitRoom*() const { return use ? &room : nullptr; } };
+SplitUse split_operands(const lm_b200_engine* e, const StepView& v, int M) {
+    return SplitUse{lm::SplitRoom{e->kv_split, e->kv_split_bytes, e->m.n_slots, v.sm, v.n_seq}, M > lm::kAttnRowsKernelMax};
 }
 
 // columns of the stacked projections of a parallel record
@@ -480,7 +488,7 @@ int mixer(lm_b200_engine* e, const lm_b200_layer& l, const float* h, const void*
     const lm::AttnShape a{l.heads, l.kv_heads, l.dim, l.window, l.keep_first, l.scale, l.softcap, l.temp, l.slopes, l.sink};
     const bool tc_o = tensor_path(e, M, D, nq);
     LCK(lm::launch_sink_attention(e->qk, nq + nk, l.k_pages, l.v_pages, pm, a, v.rm, e->att, tc_o ? e->attb : nullptr, e->split_ws, e->split_arrived, M, st,
-                                  0, 1.f, nullptr, 0, split_operands(M)));
+                                  0, 1.f, nullptr, 0, split_operands(e, v, M)));
     if (tc_o) {
         if (fuse_x) {
             const dia::GemmEpilogue ep{fuse_x, l.norm_mix_out.w, l.norm_mix_out.b, l.norm_mix_out.alpha, nullptr};
@@ -590,7 +598,7 @@ int mixer_kernels(lm_b200_engine* e, const lm_b200_layer& l, const InCols& c, fl
             LCK(lm::launch_talk_prep(proj, c.n, l.in_bias, c.q, c.k, c.v, c.gate, a, l.q_norm, l.k_norm, e->m.eps, l.k_pages,
                                      l.v_pages, pm, v.rm, M, st));
             LCK(lm::launch_talk_attention(proj, c.n, c.q, c.gate, l.k_pages, l.v_pages, pm, a, v.rm, e->outcat, ko, ob,
-                                          e->split_ws, e->split_arrived, M, st, split_operands(M)));
+                                          e->split_ws, e->split_arrived, M, st, split_operands(e, v, M)));
             break;
         }
         case LM_B200_MIXER_HGRN2: {
@@ -705,7 +713,7 @@ int stream_mixer_kernels(lm_b200_engine* e, const lm_b200_layer& l, const MixPla
             LCK(lm::launch_rot_rows(e->qk, nq, l.dim, dq, e->qlat, nl, l.kv_rank, RK, H, rd, rot, H, l.scale, l.scale, v.rm, M, st));
         if (lm::talk_attention_supported(latent_shape(l)))
             LCK(lm::launch_talk_attention(e->qlat, nl, 0, -1, l.latent_pages, l.latent_pages, pm, latent_shape(l), v.rm, e->olat, no,
-                                          nullptr, e->split_ws, e->split_arrived, M, st, split_operands(M)));
+                                          nullptr, e->split_ws, e->split_arrived, M, st, split_operands(e, v, M)));
         else
             LCK(lm::launch_latent_attention_rows(e->qlat, l.latent_pages, pm, H, l.kv_rank, l.sink, v.rm, e->olat, M, st, rd,
                                                  l.window > 0 ? l.window : 0));
@@ -737,7 +745,7 @@ int stream_mixer_kernels(lm_b200_engine* e, const lm_b200_layer& l, const MixPla
         LCK(lm::launch_talk_prep(proj, ld, nullptr, c.q, c.k, c.v, -1, a, l.q_norm, l.k_norm, e->m.eps, l.k_pages, l.v_pages, pm, v.rm, M, st));
         const lm::AttnShape s{H, l.kv_heads, l.dim, l.window > 0 ? l.window : 0, 0, 1.f, 0.f, nullptr, nullptr, l.sink, l.chunk};
         LCK(lm::launch_sink_attention(proj + c.q, ld, l.k_pages, l.v_pages, pm, s, v.rm, at.out, at.out_b, e->split_ws, e->split_arrived, M,
-                                      st, at.ldo, at.scale, gate, ld, split_operands(M)));
+                                      st, at.ldo, at.scale, gate, ld, split_operands(e, v, M)));
     } else if (l.mixer == LM_B200_MIXER_GATED_LINEAR) {
         LCK(lm::launch_decay_proj(proj + c.a1, ld, l.w_a2, l.dt_bias, l.decay_tau, e->rec, H * l.dim, l.rank_a, M, st));
         const lm::ScanInputs si{c.q, c.k, 0, c.v, 0};
@@ -959,7 +967,20 @@ int lm_b200_engine_create(const lm_b200_model* model, const lm_b200_layer* layer
     e->device = device;
     const size_t R = (size_t)m.max_rows, D = (size_t)m.width;
     size_t qk = 0, att = 0, E = 1, top = 1, F = 1, Sf = 1, slots = 1;
-    size_t n_in = 0, k_out = 0, n_rec = 0, split_dim = 0;
+    size_t n_in = 0, k_out = 0, n_rec = 0, split_dim = 0, kv_split = 0;
+    // room for the split keys and values of twice a step's rows and 4096 cached keys more (and a partly filled tile at either end of
+    // every sequence); what does not fit is split where it is used
+    const long long split_keys = std::min<long long>(2LL * m.max_rows + 4096 + 192LL * m.n_slots, 64LL * 65535);
+    auto split_room = [&](int heads, int kv_heads, int kdim, int vdim, bool latent, const float* talk) {
+        dia::SplitAttention s{};
+        float* const some = reinterpret_cast<float*>(256);        // (only whether keys and values are one buffer, and alignment, are looked at)
+        s.q = s.out = some;
+        s.kcache = some;
+        s.vcache = latent ? some : some + 64;
+        s.heads = heads; s.kv_heads = kv_heads; s.qdim = s.kdim = kdim; s.vdim = vdim; s.vrow = latent ? kdim : vdim; s.talk = talk;
+        s.n_slots = m.n_slots;
+        kv_split = std::max(kv_split, dia::split_attention_work_bytes(s, (int)split_keys));
+    };
     size_t n_streams = 0, n_lat = 0, q_rank = 0, n_heads = 0, n_side = 0;
     bool pre = false, any_parallel = false;
     e->stream_form = e->layers[0].form == LM_B200_FORM_STREAMS;
@@ -976,10 +997,12 @@ int lm_b200_engine_create(const lm_b200_model* model, const lm_b200_layer* layer
                     n_lat = std::max(n_lat, (size_t)p.heads * (p.kv_rank + p.rot_dim));
                     q_rank = std::max(q_rank, (size_t)p.q_rank);
                     if (lm::talk_attention_supported(latent_shape(p))) split_dim = std::max(split_dim, (size_t)p.heads * (p.kv_rank + 2));
+                    split_room(p.heads, 1, p.kv_rank + p.rot_dim, p.kv_rank, true, nullptr);
                 } else if (p.mixer == LM_B200_MIXER_MLSTM) {
                     n_lat = std::max(n_lat, (size_t)p.heads * (p.vdim + 1));
                 } else if (p.mixer == LM_B200_MIXER_ROTARY_ATTENTION) {
                     split_dim = std::max(split_dim, (size_t)p.heads * (p.dim + 2));
+                    split_room(p.heads, p.kv_heads, p.dim, p.dim, false, nullptr);
                 }
                 n_rec = std::max(n_rec, (size_t)stream_rec_cols(p));
             }
@@ -1000,12 +1023,16 @@ int lm_b200_engine_create(const lm_b200_model* model, const lm_b200_layer* layer
             k_out = std::max(k_out, (size_t)l.k_out);
             n_rec = std::max(n_rec, (size_t)rec_cols(l));
             pre = pre || l.w_pre;
-            if (l.mixer == LM_B200_MIXER_TALK_ATTENTION) split_dim = std::max(split_dim, (size_t)l.heads * (l.vdim + 2));
+            if (l.mixer == LM_B200_MIXER_TALK_ATTENTION) {
+                split_dim = std::max(split_dim, (size_t)l.heads * (l.vdim + 2));
+                split_room(l.heads, l.kv_heads, l.dim, l.vdim, false, l.talk);
+            }
             continue;
         }
         qk = std::max(qk, (size_t)(l.heads + l.kv_heads) * l.dim);
         att = std::max(att, (size_t)l.heads * l.dim);
         split_dim = std::max(split_dim, (size_t)l.heads * (l.dim + 2));
+        split_room(l.heads, l.kv_heads, l.dim, l.dim, false, nullptr);
         if (l.ff == LM_B200_FF_ROUTED_EXPERTS) {
             E = std::max(E, (size_t)l.experts);
             top = std::max(top, (size_t)l.top);
@@ -1039,6 +1066,7 @@ int lm_b200_engine_create(const lm_b200_model* model, const lm_b200_layer* layer
     const size_t o_catb = take(tcb && pre ? R * 2 * D * 2 : 0), o_outcatb = take(tcb ? R * k_out * 2 : 0);
     const size_t o_cqb = take(tcb ? R * q_rank * 2 : 0), o_h2b = take(tcb && any_parallel ? R * D * 2 : 0),
                  o_sidegb = take(tcb ? R * n_side * 2 : 0);
+    const size_t o_kvsplit = take(kv_split);
     if (cudaMalloc(&e->arena, off) != cudaSuccess) {
         (void)cudaGetLastError();
         delete e;
@@ -1061,6 +1089,8 @@ int lm_b200_engine_create(const lm_b200_model* model, const lm_b200_layer* layer
     e->ymix = (float*)(b + o_ymix); e->h2 = (float*)(b + o_h2); e->h2b = b + o_h2b;
     e->side_z = (float*)(b + o_sidez); e->side_g = (float*)(b + o_sideg); e->side_gb = b + o_sidegb;
     e->split_ws = (float*)(b + o_split);
+    e->kv_split = kv_split ? b + o_kvsplit : nullptr;
+    e->kv_split_bytes = kv_split;
     e->split_arrived = (unsigned*)(b + o_arrived);
     const float unit_host[2] = {0.f, 1.f};
     if (cudaMemset(e->split_arrived, 0, arrived_bytes) != cudaSuccess ||
@@ -1367,7 +1397,7 @@ int lm_b200_op_attention(lm_b200_engine* e, int layer, float* qk, const int32_t*
                                  S(stream)));
     const lm::AttnShape a{l.heads, l.kv_heads, l.dim, l.window, l.keep_first, l.scale, l.softcap, l.temp, l.slopes, l.sink};
     LCK(lm::launch_sink_attention(qk, nq + nk, l.k_pages, l.v_pages, pm, a, v.rm, out, nullptr, e->split_ws, e->split_arrived, M, S(stream), 0, 1.f,
-                                  nullptr, 0, split_operands(M)));
+                                  nullptr, 0, split_operands(e, v, M)));
     return LM_B200_OK;
 }
 

@@ -68,12 +68,14 @@ cudaError_t launch_router_rows(const float* h, int D, const void* Wr, int E, int
 cudaError_t launch_qk_norm_cache(float* qk, int nq, int nk, const float* qw, const float* kw, float eps, float* kcache,
                                  float* vcache, const PageMap& pm, int kv_heads, int dim, const RowMeta& rm, int M,
                                  cudaStream_t st);
+// What the tensor-core attention with split operands is given: room for keys and values split in advance, and the step's sequences
+struct SplitRoom { void* work; size_t bytes; int n_slots; SeqMeta sm; int n_seq; };
 // ldo: row stride of the output (0: heads * dim); out_scale multiplies it, and so does the sigmoid of gate[row * ldg + column],
-// if given.  tensor_cores: steps of more than kAttnRowsKernelMax rows run on the split-operand kernel where it takes the shape
+// if given.  split: steps of more than kAttnRowsKernelMax rows run on the split-operand kernel where it takes the shape
 cudaError_t launch_sink_attention(const float* qk, int q_stride, const float* kcache, const float* vcache, const PageMap& pm,
                                   const AttnShape& a, const RowMeta& rm, float* out, void* out_bf16, float* split_ws,
                                   unsigned* arrived, int M, cudaStream_t st, int ldo = 0, float out_scale = 1.f,
-                                  const float* gate = nullptr, int ldg = 0, bool tensor_cores = false);
+                                  const float* gate = nullptr, int ldg = 0, const SplitRoom* split = nullptr);
 cudaError_t launch_router_topk(const float* z, int E, int top, int M, int* sel_e, float* sel_w, cudaStream_t st,
                                const float* bias = nullptr, bool softmax_top = false, const GroupedRoute* gr = nullptr);
 cudaError_t launch_moe_group(const int* sel_e, const float* sel_w, int n_assign, int top, int E, int pad, const GroupMap& gm,
@@ -117,7 +119,7 @@ cudaError_t launch_talk_prep(float* proj, int ld, const float* bias, int q_off, 
 bool talk_attention_supported(const TalkShape& a);
 cudaError_t launch_talk_attention(const float* proj, int ld, int q_off, int gate_off, const float* kcache, const float* vcache,
                                   const PageMap& pm, const TalkShape& a, const RowMeta& rm, float* out, int ldo, void* out_bf16,
-                                  float* split_ws, unsigned* arrived, int M, cudaStream_t st, bool tensor_cores = false);
+                                  float* split_ws, unsigned* arrived, int M, cudaStream_t st, const SplitRoom* split = nullptr);
 // head_decay_off >= 0: ONE decay per head, exp(-exp(a_log_h) softplus(proj[head_decay_off + h] + dt_bias_h)); the rec row is
 // then q | k | v | decay (H) | beta (H) and the output gate is left to the caller
 cudaError_t launch_delta_prep(const float* proj, int ld, int beta_off, const DeltaShape& d, const float* tail, const RowMeta& rm,

@@ -1261,12 +1261,12 @@ static cudaError_t launch_attention_splits(const float* qk, int q_stride, const 
 cudaError_t launch_sink_attention(const float* qk, int q_stride, const float* kcache, const float* vcache, const PageMap& pm,
                                   const AttnShape& a, const RowMeta& rm, float* out, void* out_bf16, float* split_ws,
                                   unsigned* arrived, int M, cudaStream_t st, int ldo, float out_scale, const float* gate, int ldg,
-                                  bool tensor_cores) {
+                                  const SplitRoom* split) {
     if (ldo <= 0) ldo = a.heads * a.dim;
     if (a.dim > 32 * kAttnMaxDimPerLane || a.heads % a.kv_heads) return cudaErrorNotSupported;
     __nv_bfloat16* ob = reinterpret_cast<__nv_bfloat16*>(out_bf16);
     if (M > kAttnRowsKernelMax) {
-        if (tensor_cores) {
+        if (split) {
             dia::SplitAttention s{};
             s.q = qk; s.ldq = q_stride; s.qdim = a.dim;
             s.kcache = kcache; s.vcache = vcache; s.table = pm.table; s.max_pages = pm.max_pages; s.page_size = pm.page_size;
@@ -1275,6 +1275,8 @@ cudaError_t launch_sink_attention(const float* qk, int q_stride, const float* kc
             s.row_slot = rm.slot; s.row_pos = rm.pos; s.M = M;
             s.window = a.window; s.keep_first = a.keep_first; s.chunk = a.chunk;
             s.out = out; s.ldo = ldo; s.out_bf16 = out_bf16; s.out_scale = out_scale; s.gate = gate; s.ldg = ldg;
+            s.work = split->work; s.work_bytes = split->bytes; s.n_slots = split->n_slots;
+            s.seq_slot = split->sm.slot; s.seq_row0 = split->sm.row0; s.seq_count = split->sm.count; s.n_seq = split->n_seq;
             if (dia::split_attention_ok(s)) return dia::launch_split_attention(s, st);
         }
         switch ((a.dim + 63) / 64) {

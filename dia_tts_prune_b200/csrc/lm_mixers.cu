@@ -802,10 +802,10 @@ bool talk_attention_supported(const TalkShape& a) {
 // to hide the latencies of a tile's dependent phases); a handful of rows run 8 warps per (row, share of the keys).
 cudaError_t launch_talk_attention(const float* proj, int ld, int q_off, int gate_off, const float* kcache, const float* vcache,
                                   const PageMap& pm, const TalkShape& a, const RowMeta& rm, float* out, int ldo, void* out_bf16,
-                                  float* split_ws, unsigned* arrived, int M, cudaStream_t st, bool tensor_cores) {
+                                  float* split_ws, unsigned* arrived, int M, cudaStream_t st, const SplitRoom* split) {
     if (!talk_attention_supported(a)) return cudaErrorNotSupported;
     __nv_bfloat16* ob = reinterpret_cast<__nv_bfloat16*>(out_bf16);
-    if (tensor_cores && M > kAttnRowsKernelMax) {
+    if (split && M > kAttnRowsKernelMax) {
         dia::SplitAttention s{};
         const bool latent = kcache == vcache;                 // the value is the head of the key row
         s.q = proj + q_off; s.ldq = ld; s.qdim = a.dim;
@@ -815,6 +815,8 @@ cudaError_t launch_talk_attention(const float* proj, int ld, int q_off, int gate
         s.row_slot = rm.slot; s.row_pos = rm.pos; s.M = M; s.window = a.window;
         s.out = out; s.ldo = ldo; s.out_bf16 = out_bf16; s.out_scale = 1.f;
         if (gate_off >= 0) { s.head_gate = proj + gate_off; s.ldg = ld; }
+        s.work = split->work; s.work_bytes = split->bytes; s.n_slots = split->n_slots;
+        s.seq_slot = split->sm.slot; s.seq_row0 = split->sm.row0; s.seq_count = split->sm.count; s.n_seq = split->n_seq;
         if (dia::split_attention_ok(s)) return dia::launch_split_attention(s, st);
     }
     const int vu = (a.vdim + 31) / 32;

@@ -45,6 +45,11 @@ def sink_reference(x, past, H, G, d, p, window, keep, cap, eps):
     ([130], 0, 8, 1, 200, 100, 200, 0.0, 1.0, 64),      # two channel groups, more kept keys than the window starts behind
     ([70], 0, 16, 1, 256, 0, 0, 0.0, 1.0, 64),          # the widest heads
     ([33], 0, 3, 1, 20, 5, 1, 0.0, 1.0, 7),             # channels that are no multiple of 16, odd pages
+    # from here on enough rows that the keys are split in advance
+    ([128], 0, 4, 1, 128, 0, 0, 0.0, 1.0, 64),
+    ([200, 1, 63, 190], 130, 8, 2, 64, 33, 3, 30.0, 1.0, 16),    # the kept keys' tile in front of the window's
+    ([150, 90], 200, 8, 1, 40, 50, 100, 0.0, 1e3, 7),   # more kept keys than one tile holds
+    ([256], 6100, 4, 2, 64, 0, 0, 0.0, 1.0, 64),        # more cached keys than the room holds
 ])
 def test_grouped_query_attention(rows, past, H, G, d, window, keep, cap, amp, page):
     from dia_tts_prune_b200 import synthetic as SY
@@ -53,7 +58,7 @@ def test_grouped_query_attention(rows, past, H, G, d, window, keep, cap, amp, pa
     cfg = SY.pubopel_config(width=32, layers=1, heads=H, kv_heads=G, dim=d, experts=1, top=1, expert_ff=8, shared_ff=None, vocab=64,
                             window=window or None, keep_first=keep, softcap=cap or None)
     w = SY.pubopel_weights(cfg, 3)
-    model = CausalLM(PubopelConfig.model_validate(cfg), w, dtype="bfloat16", device="cuda:0", max_tokens=2048, max_sequences=4,
+    model = CausalLM(PubopelConfig.model_validate(cfg), w, dtype="bfloat16", device="cuda:0", max_tokens=8192, max_sequences=4,
                      page_size=page, max_rows=512)
     p = {n: w[f"l0.mix.{t}"].double() for n, t in (("q", "q.norm"), ("k", "k.norm"), ("temp", "temp"), ("sink", "sink"))}
     g = torch.Generator().manual_seed(5)
@@ -61,14 +66,15 @@ def test_grouped_query_attention(rows, past, H, G, d, window, keep, cap, amp, pa
     seqs = [model.state.open(str(i)) for i in range(len(rows))]
     for s, t in zip(seqs, x):
         model.state.reserve(s, len(t))
-        if past:
-            model.engine.op_attention(0, t[:past].cuda(), [(s, past, 0)])
+        for a in range(0, past, 512):
+            b = min(past, a + 512)
+            model.engine.op_attention(0, t[a:b].cuda(), [(s, b - a, a)])
     got = model.engine.op_attention(0, torch.cat([t[past:] for t in x]).cuda(), [(s, n, past) for s, n in zip(seqs, rows)])
     ref = torch.cat([sink_reference(t.double(), past, H, G, d, p, window, keep, cap, cfg["norm"]["eps"]) for t in x])
     close(got, ref, ref.abs().max().item())
 
 
-@pytest.mark.parametrize("H,G,d,dv,rows", [(8, 2, 128, 128, [70, 1]), (4, 4, 64, 32, [64]), (12, 3, 40, 24, [33, 5]), (16, 1, 24, 256, [65])])
+@pytest.mark.parametrize("H,G,d,dv,rows", [(8, 2, 128, 128, [70, 1]), (8, 2, 128, 128, [128, 40]), (4, 4, 64, 32, [64]), (12, 3, 40, 24, [33, 5]), (16, 1, 24, 256, [65])])
 def test_mixed_scores(H, G, d, dv, rows):
     """Scores mixed across heads: the kernel mixes the queries instead, against the mixer's definition in 64 bits."""
     from dia_tts_prune_b200 import synthetic as SY
@@ -78,7 +84,7 @@ def test_mixed_scores(H, G, d, dv, rows):
     cfg["layers"][0]["mixer"]["rot"] = None
     w = SY.kupelix_weights(cfg, 3)
     cfg["layers"][0]["mlp"] = None
-    model = CausalLM(KupelixConfig.model_validate(cfg), w, dtype="bfloat16", device="cuda:0", max_tokens=512, max_sequences=2, max_rows=128)
+    model = CausalLM(KupelixConfig.model_validate(cfg), w, dtype="bfloat16", device="cuda:0", max_tokens=512, max_sequences=2, max_rows=256)
     n_in = model.layers[0].layer.n_in
     g = torch.Generator().manual_seed(6)
     x = [torch.randn((n, n_in), generator=g) for n in rows]
