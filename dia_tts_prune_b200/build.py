@@ -14,8 +14,8 @@ PKG = Path(__file__).resolve().parent
 CSRC = PKG / "csrc"
 INCLUDE = PKG.parent / "include"
 LIB = CSRC / "libdia_b200.so"
-SOURCES = ["step_kernel.cu", "aux_kernels.cu", "gemm_tcgen05.cu", "prefill_kernels.cu", "batch_kernel.cu", "engine.cu"]
-HEADERS = ["common.cuh", "engine_internal.h", "sampler.cuh", "gemm_tcgen05.h"]
+SOURCES = ["step_kernel.cu", "aux_kernels.cu", "gemm_tcgen05.cu", "prefill_kernels.cu", "batch_kernel.cu", "engine.cu", "attention_split.cu"]
+HEADERS = ["common.cuh", "engine_internal.h", "sampler.cuh", "gemm_tcgen05.h", "attention_split.h"]
 LM_LIB = CSRC / "liblm_b200.so"
 LM_SOURCES = ["lm_kernels.cu", "lm_mixers.cu", "lm_streams.cu", "lm_linear.cu", "lm_scan.cu", "lm_engine.cu", "gemm_tcgen05.cu",
               "attention_split.cu"]                                # the tensor-core GEMM is shared with Dia

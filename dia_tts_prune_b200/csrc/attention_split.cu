@@ -55,6 +55,7 @@ struct Geometry {
     int v0_layout, v_last_layout;            // widths in which the value groups lie in a slot (a latent's value group is its key group)
     int shared_kv;                           // the value is the head of the key row: value group i is key group i
     int slot_bytes, n_slots, q_bytes;
+    int o_bufs;                              // accumulators of the value product (2 where tensor memory has the columns)
     // the split keys and values in SplitAttention::work: SlotTiles per slot, then inverse scales [tile][part], then the tiles.  A
     // tile's parts: key groups (per kv head where the launch reads one head at a time), then value groups
     int parts, k_parts, cap_tiles;
@@ -105,11 +106,50 @@ __device__ __forceinline__ void commit_to(uint64_t* bar) {
 __device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_smem_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-__device__ __forceinline__ void tmem_load8(uint32_t addr, float (&v)[8]) {
+__device__ __forceinline__ void tmem_load32(uint32_t addr, float (&v)[32]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, "
+        "%20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+        : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7]), "=f"(v[8]), "=f"(v[9]),
+          "=f"(v[10]), "=f"(v[11]), "=f"(v[12]), "=f"(v[13]), "=f"(v[14]), "=f"(v[15]), "=f"(v[16]), "=f"(v[17]), "=f"(v[18]),
+          "=f"(v[19]), "=f"(v[20]), "=f"(v[21]), "=f"(v[22]), "=f"(v[23]), "=f"(v[24]), "=f"(v[25]), "=f"(v[26]), "=f"(v[27]),
+          "=f"(v[28]), "=f"(v[29]), "=f"(v[30]), "=f"(v[31])
+        : "r"(addr)
+        : "memory");
+}
+__device__ __forceinline__ void tmem_load8(uint32_t addr, float* v) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
                  : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
                  : "r"(addr)
                  : "memory");
+}
+template <int N>
+__device__ __forceinline__ void tmem_load_n(uint32_t addr, float (&v)[N]) {
+    if constexpr (N == 32) tmem_load32(addr, v);
+    else tmem_load8(addr, v);
+}
+// two fp32 operations in one instruction
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+    float2 d;
+    asm("{\n\t.reg .b64 a, b, c, d;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\tmov.b64 c, {%6, %7};\n\t"
+        "fma.rn.f32x2 d, a, b, c;\n\tmov.b64 {%0, %1}, d;\n\t}"
+        : "=f"(d.x), "=f"(d.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+    return d;
+}
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+    float2 d;
+    asm("{\n\t.reg .b64 a, b, d;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\tmul.rn.f32x2 d, a, b;\n\tmov.b64 {%0, %1}, d;\n\t}"
+        : "=f"(d.x), "=f"(d.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return d;
+}
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+    float2 d;
+    asm("{\n\t.reg .b64 a, b, d;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\tadd.rn.f32x2 d, a, b;\n\tmov.b64 {%0, %1}, d;\n\t}"
+        : "=f"(d.x), "=f"(d.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return d;
 }
 __device__ __forceinline__ void tmem_loaded() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tmem_store8(uint32_t addr, const uint32_t (&v)[8]) {
@@ -436,23 +476,26 @@ split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_co
         for (int c = 0; c < DVH; ++c) O[c] = 0.f;
         float m_run = -CUDART_INF_F, c_run = 0.f, l_run = 0.f, corr_prev = 1.f;
         bool ok = true;
-        auto add_values = [&](unsigned t) {                   // O <- corr O + value product of tile t
-            if (!wait_for(pv_done, t & 1u)) { ok = false; return; }
-            fence_after();
+        constexpr int OW = NVS == 1 ? 32 : 16;                // columns in flight
+        auto add_values = [&](unsigned t, float corr) {       // O <- corr O + value product of tile t (which is done)
             const float vi = v_inv[(t % kScaleRing) * 2 + (NVS == 1 ? 0 : hf)] * (1.0f / kWeightScale);
-            const bool same = __all_sync(0xffffffffu, corr_prev == 1.f);
+            const bool same = __all_sync(0xffffffffu, corr == 1.f);
+            const uint32_t from = t_mine + (geo.o_bufs == 2 ? (t & 1u) * 128u : 0u);
+            const float2 vi2 = make_float2(vi, vi), c2 = make_float2(corr, corr);
 #pragma unroll
-            for (int c = 0; c < DVH; c += 8) {
-                if (c < n_mine) {
-                    float v[8];
-                    tmem_load8(t_mine + c, v);
+            for (int c = 0; c < DVH; c += OW) {
+                if (c < n_mine) {                             // (columns beyond n_mine hold whatever they held; they are not stored)
+                    float v[OW];
+                    if constexpr (OW == 32) tmem_load32(from + c, v);
+                    else { tmem_load8(from + c, v); tmem_load8(from + c + 8, v + 8); }
                     tmem_loaded();
-                    if (same) {
 #pragma unroll
-                        for (int e = 0; e < 8; ++e) O[c + e] = fmaf(v[e], vi, O[c + e]);
-                    } else {
-#pragma unroll
-                        for (int e = 0; e < 8; ++e) O[c + e] = fmaf(v[e], vi, O[c + e] * corr_prev);
+                    for (int e = 0; e < OW; e += 2) {
+                        float2 o = make_float2(O[c + e], O[c + e + 1]);
+                        if (!same) o = mul2(o, c2);
+                        o = fma2(make_float2(v[e], v[e + 1]), vi2, o);
+                        O[c + e] = o.x;
+                        O[c + e + 1] = o.y;
                     }
                 }
             }
@@ -464,20 +507,19 @@ split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_co
             fence_after();
             float s[32];
             const float* ki = k_inv + (t % kScaleRing) * kMaxKStages * 4 + hf * 2;
+            constexpr int SW = NVS == 1 ? 32 : 8;             // scores in flight (a wide value leaves fewer registers)
 #pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                float v[8];
-                tmem_load8(t_s + lanes + hf * 32 + c * 8, v);
+            for (int c = 0; c < 32; c += SW) {
+                float v[SW];
+                tmem_load_n<SW>(t_s + lanes + hf * 32 + c, v);
                 tmem_loaded();
-                const float a = ki[c >> 1] * mult;
 #pragma unroll
-                for (int e = 0; e < 8; ++e) s[c * 8 + e] = v[e] * a;
+                for (int e = 0; e < SW; ++e) s[c + e] = v[e] * (ki[(c + e) >> 4] * mult);
                 for (int st = 1; st < geo.n_kst; ++st) {
-                    tmem_load8(t_s + lanes + st * 64 + hf * 32 + c * 8, v);
+                    tmem_load_n<SW>(t_s + lanes + st * 64 + hf * 32 + c, v);
                     tmem_loaded();
-                    const float b = ki[st * 4 + (c >> 1)] * mult;
 #pragma unroll
-                    for (int e = 0; e < 8; ++e) s[c * 8 + e] = fmaf(v[e], b, s[c * 8 + e]);
+                    for (int e = 0; e < SW; ++e) s[c + e] = fmaf(v[e], ki[st * 4 + ((c + e) >> 4)] * mult, s[c + e]);
                 }
             }
             fence_before();
@@ -515,34 +557,49 @@ split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_co
             const float m_new = fmaxf(m_run, mx);
             const float c_new = m_new == -CUDART_INF_F ? 0.f : m_new * kLog2e;
             const float corr = m_run == -CUDART_INF_F ? 0.f : ex2(c_run - c_new);
-            float sum0 = 0.f, sum1 = 0.f;
+            float2 sum = make_float2(0.f, 0.f);
+            const float2 l2 = make_float2(kLog2e, kLog2e), nc = make_float2(-c_new, -c_new);
 #pragma unroll
             for (int e = 0; e < 32; e += 2) {
-                s[e] = ex2(fmaf(s[e], kLog2e, -c_new));
-                s[e + 1] = ex2(fmaf(s[e + 1], kLog2e, -c_new));
-                sum0 += s[e];
-                sum1 += s[e + 1];
+                const float2 a = fma2(make_float2(s[e], s[e + 1]), l2, nc);
+                s[e] = ex2(a.x);
+                s[e + 1] = ex2(a.y);
+                sum = add2(sum, make_float2(s[e], s[e + 1]));
             }
-            l_run = fmaf(l_run, corr, sum0 + sum1);
+            l_run = fmaf(l_run, corr, sum.x + sum.y);
             m_run = m_new;
             c_run = c_new;
-            if (t > 0) add_values(t - 1);                     // (also: the weights' columns are free)
-            if (!ok) break;
+            // the value product of the tile before is done: the weights' columns are free, and its sum can be taken
+            if (t > 0) {
+                if (!wait_for(pv_done, (t - 1) & 1u)) { ok = false; break; }
+                fence_after();
+            }
+            const float2 ws = make_float2(kWeightScale, kWeightScale);
 #pragma unroll
             for (int c = 0; c < 2; ++c) {
                 uint32_t hi[8], lo[8];
 #pragma unroll
-                for (int e = 0; e < 8; ++e) split2(s[c * 16 + 2 * e] * kWeightScale, s[c * 16 + 2 * e + 1] * kWeightScale, hi[e], lo[e]);
+                for (int e = 0; e < 8; ++e) {
+                    const float2 q = mul2(make_float2(s[c * 16 + 2 * e], s[c * 16 + 2 * e + 1]), ws);
+                    split2(q.x, q.y, hi[e], lo[e]);
+                }
                 tmem_store8(t_p + lanes + hf * 16 + c * 8, hi);
                 tmem_store8(t_p + lanes + 32 + hf * 16 + c * 8, lo);
             }
+            // with two accumulators the next value product may start before the last one has been added
+            if (t > 0 && geo.o_bufs == 1) add_values(t - 1, corr_prev);
             asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
             fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(p_ready);
+            if (t > 0 && geo.o_bufs == 2) add_values(t - 1, corr_prev);
             corr_prev = corr;
         }
-        if (ok && t > 0) add_values(t - 1);
+        if (ok && t > 0) {
+            ok = wait_for(pv_done, (t - 1) & 1u);
+            fence_after();
+            add_values(t - 1, corr_prev);
+        }
         // ---- both threads' denominators, the sink's own term, normalise, store ----
         float* xl = row_x + (t & 1u) * 2 * kRows;
         xl[hf * kRows + row] = l_run;
@@ -733,7 +790,7 @@ split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_co
                     const uint32_t va = ring_addr + slot * geo.slot_bytes;
                     const uint64_t vh = block_desc(va, wp * 16u, 128u), vl = block_desc(va + kKeys * wp * 2u, wp * 16u, 128u);
                     const uint32_t step = 2u * wp;            // 16 keys, in descriptor units of 16 bytes
-                    const uint32_t d = t_o + 128u * vs;
+                    const uint32_t d = t_o + 128u * (geo.o_bufs == 2 ? t & 1u : (unsigned)vs);
                     if (elect_one_sync()) {
 #pragma unroll
                         for (uint32_t k = 0; k < 4; ++k) mma_ts(d, t_p + 32u + 8u * k, vh + k * step, idesc, k != 0);
@@ -828,6 +885,7 @@ bool geometry_of(const SplitAttention& a, Geometry& g, size_t& smem) {
         if (a.work_bytes > fixed) g.cap_tiles = (int)std::min<size_t>((a.work_bytes - fixed) / per, 65535);
         g.tile_off = (unsigned)((g.scale_off + 4u * g.parts * (unsigned)g.cap_tiles + 127u) & ~127u);
     }
+    g.o_bufs = g.n_vst == 1 && 64 * g.n_kst + 64 + 256 <= 512 ? 2 : 1;
     g.slot_bytes = kKeys * std::max(g.wk0, std::max(g.wv0, g.v0_layout)) * 4;
     g.q_bytes = ((g.n_kst - 1) * g.wk0 + g.wk_last) * kRows * 4;
     const int control = (2 * kMaxSlots + 5 + 4) * 8 + (kScaleRing * kMaxKStages * 4 + kScaleRing * 2 + 8 + 4 * kRows) * 4 + 2 * (kRows >> g.pk_shift) * 4;

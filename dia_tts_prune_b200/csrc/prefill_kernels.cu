@@ -1,7 +1,8 @@
 // prefill_kernels.cu - everything around the tcgen05 GEMMs of the T > 1 passes (encoder, cross-attention K/V
 // precompute, prompt prefill) that is not a dense contraction:
 //
-//   attention_rows_kernel   F.scaled_dot_product_attention call sites (dia/layers.py:329-337) for T > 1: causal GQA
+//   attention_rows_kernel   a few queries; more of them run on the tensor cores with split fp32 operands (attention_split.cu):
+//                           F.scaled_dot_product_attention call sites (dia/layers.py:329-337) for T > 1: causal GQA
 //                           self-attention of the prompt prefill, full / pad-partitioned encoder self-attention,
 //                           cross-attention over the valid text keys.  fp32 throughout (these K/V and outputs are
 //                           re-read by every later greedy step): flash-style, one CTA per (batch row, query head,
@@ -12,13 +13,14 @@
 //   silu_mul_kernel         MlpBlock gate: silu(gate) * up (dia/layers.py:95-101)
 //   embed_rows_kernel       nn.Embedding row gather (dia/layers.py:445-447)
 //
-// Bound: attention by the fp32 FMA pipe (no tensor cores: the operands may not be rounded), the rest by HBM.
+// Bound: attention_rows_kernel by the fp32 FMA pipe, the rest by HBM.
 #include <algorithm>
 
 #include <cuda_runtime.h>
 #include <math_constants.h>
 #include <stdint.h>
 
+#include "attention_split.h"
 #include "common.cuh"
 #include "engine_internal.h"
 
@@ -31,6 +33,7 @@ constexpr int kAK = 64;               // keys per tile
 constexpr int kQStride = 132;         // padded row stride (floats) of the Q and K tiles: conflict-free float4 reads
 constexpr int kPStride = 68;
 constexpr int kAttnThreads = 256;
+constexpr int kSplitRowsMin = 16;     // queries of a batch row from which the attention runs on the tensor cores
 constexpr int kAttnSmem = (kAQ * kQStride + kAK * kQStride + kAK * kHeadDim + kAQ * kPStride) * 4;
 
 }  // namespace
@@ -260,6 +263,17 @@ static int grid_for(long long n, int block) { return (int)std::min<long long>((n
 
 cudaError_t launch_attention_rows(const float* q, const float* k, const float* v, float* out, int B, int Tq, int Tk, int Hq,
                                   int Hkv, int Tk_stride, int mode, const int* n_valid_host, cudaStream_t st) {
+    SplitAttention s{};
+    if (B <= 16 && Tq > kSplitRowsMin) {                      // the tensor-core kernel with split fp32 operands
+        s.q = q; s.ldq = Hq * kHeadDim; s.qdim = kHeadDim;
+        s.kcache = k; s.vcache = v; s.page_size = Tk_stride;
+        s.heads = Hq; s.kv_heads = Hkv; s.kdim = s.vdim = s.vrow = kHeadDim;
+        s.scale = 0.08838834764831845f;                       // 1/sqrt(128)
+        s.M = B * Tq; s.rows_per_slot = Tq; s.mode = mode; s.n_keys = Tk;
+        for (int b = 0; b < B; ++b) s.n_valid[b] = n_valid_host ? n_valid_host[b] : Tk;
+        s.out = out; s.ldo = Hq * kHeadDim; s.out_scale = 1.f;
+        if (split_attention_ok(s)) return launch_split_attention(s, st);
+    }
     static bool attr[64] = {};
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
