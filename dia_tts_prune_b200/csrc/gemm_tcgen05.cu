@@ -335,6 +335,210 @@ dia_gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
     }
 }
 
+// ---------------------------------------------------------------------------------------------------------------------
+// Y = A W^T in the accuracy of fp32 FMA arithmetic, for callers that asked for it.  The accumulator of a tensor-core product loses
+// up to a unit in the last place at every step, towards zero (K = 2048: 2.1e-6 against 3.9e-7 of an FMA chain), so an accumulator
+// lives for one k-block only - the two small terms first, then the large one - and the epilogue warps add it to the tile's sums
+// in their registers while the next k-blocks are multiplied into the three other accumulators.  128 x 128 tiles: a thread holds
+// 128 sums.  Bound: 12 MMAs of 64 cycles per k-block against ~300 issue slots of draining it.
+constexpr int kFN = 128, kFASlots = 6, kFBSlots = 3, kFStride = kFN + 4;
+constexpr int kFStage = 4 * 32 * kFStride * 4;                // 32 rows of sums per epilogue warp
+constexpr int kFBars = 2 * kFASlots + 2 * kFBSlots + 8;
+constexpr int kFSmem = (kFASlots + kFBSlots) * kTileBytes + kFStage + 1024 + 256;
+static_assert(kFBars * 8 + 8 <= 256, "barrier region");
+
+__device__ __noinline__ float f32_act(int act, float z) {
+    if (act == 2) return fmaxf(z, 0.f) * fmaxf(z, 0.f);
+    return 0.5f * z * (1.0f + tanhf(0.7978845608028654f * fmaf(0.044715f * z * z, z, z)));
+}
+
+__global__ void __launch_bounds__(kGemmThreads, 1)
+dia_gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const __grid_constant__ F32Product p) {
+    const int M = p.M, N = p.N, K = p.K;
+    extern __shared__ unsigned char smem_raw[];
+    unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    unsigned char* a_ring = smem;
+    unsigned char* b_ring = smem + kFASlots * kTileBytes;
+    uint64_t* a_full = reinterpret_cast<uint64_t*>(b_ring + kFBSlots * kTileBytes);
+    uint64_t* a_empty = a_full + kFASlots;
+    uint64_t* b_full = a_empty + kFASlots;
+    uint64_t* b_empty = b_full + kFBSlots;
+    uint64_t* t_full = b_empty + kFBSlots;                  // [4] a k-block's products are complete / have been added
+    uint64_t* t_empty = t_full + 4;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(t_empty + 4);
+    float* stage = reinterpret_cast<float*>(reinterpret_cast<unsigned char*>(a_full) + 256);
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int n_kb = (K + BK - 1) / BK;
+    const int tiles_m = (M + BM - 1) / BM, tiles_n = (N + kFN - 1) / kFN, n_tiles = tiles_m * tiles_n * p.heads;
+    // tile t: row block t % tiles_m of column block (t / tiles_m) % tiles_n of head t / (tiles_m tiles_n)
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < kFASlots; ++i) { mbar_init(&a_full[i], 1); mbar_init(&a_empty[i], 1); }
+        for (int i = 0; i < kFBSlots; ++i) { mbar_init(&b_full[i], 1); mbar_init(&b_empty[i], 1); }
+        for (int i = 0; i < 4; ++i) { mbar_init(&t_full[i], 1); mbar_init(&t_empty[i], 4); }
+        fence_mbar_init();
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(4 * kFN));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::);
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem_base = *tmem_slot;
+
+    if (warp == 0) {
+        if (lane == 0) {
+            unsigned ia = 0, ib = 0;
+            for (int t = blockIdx.x; t < n_tiles; t += gridDim.x) {
+                const int hn = t / tiles_m, h = hn / tiles_n, n0 = (hn - h * tiles_n) * kFN, m0 = (t % tiles_m) * BM;
+                for (int kb = 0; kb < n_kb; ++kb) {
+                    const unsigned s = ib % kFBSlots;
+                    mbar_wait_bounded(&b_empty[s], ((ib / kFBSlots) & 1u) ^ 1u);
+                    mbar_arrive_expect_tx(&b_full[s], kTileBytes);
+                    tma_load_2d(smem_u32(b_ring + s * kTileBytes), &map_b, smem_u32(&b_full[s]), kb * BK, h * N + n0);
+                    ++ib;
+                    for (int tm = kTerms - 1; tm >= 0; --tm) {          // the smallest term first
+                        const unsigned sa = ia % kFASlots;
+                        mbar_wait_bounded(&a_empty[sa], ((ia / kFASlots) & 1u) ^ 1u);
+                        mbar_arrive_expect_tx(&a_full[sa], kTileBytes);
+                        tma_load_2d(smem_u32(a_ring + sa * kTileBytes), &map_a, smem_u32(&a_full[sa]), kb * BK, (tm * p.heads + h) * M + m0);
+                        ++ia;
+                    }
+                }
+            }
+        }
+    } else if (warp == 1) {
+        const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kFN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
+        unsigned ia = 0, ib = 0;
+        for (int t = blockIdx.x; t < n_tiles; t += gridDim.x) {
+            for (int kb = 0; kb < n_kb; ++kb) {
+                const unsigned acc = ib & 3u, sb = ib % kFBSlots;
+                mbar_wait_bounded(&t_empty[acc], ((ib >> 2) & 1u) ^ 1u);
+                mbar_wait_bounded(&b_full[sb], (ib / kFBSlots) & 1u);
+                const uint64_t bdesc = umma_desc(smem_u32(b_ring + sb * kTileBytes));
+                const uint32_t d = tmem_base + acc * kFN;
+                for (int tm = 0; tm < kTerms; ++tm) {
+                    const unsigned sa = ia % kFASlots;
+                    mbar_wait_bounded(&a_full[sa], (ia / kFASlots) & 1u);
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    const uint64_t adesc = umma_desc(smem_u32(a_ring + sa * kTileBytes));
+                    if (elect_one_sync()) {
+#pragma unroll
+                        for (int j = 0; j < BK / 16; ++j) umma_bf16(d, adesc + 2 * j, bdesc + 2 * j, idesc, (tm | j) != 0 ? 1u : 0u);
+                        umma_commit(&a_empty[sa]);
+                        if (tm == kTerms - 1) {
+                            umma_commit(&b_empty[sb]);
+                            umma_commit(&t_full[acc]);
+                        }
+                    }
+                    __syncwarp();
+                    ++ia;
+                }
+                ++ib;
+            }
+        }
+    } else {
+        const int q = warp & 3;
+        unsigned it = 0;
+        for (int t = blockIdx.x; t < n_tiles; t += gridDim.x) {
+            const int hn = t / tiles_m, h = hn / tiles_n, n0 = (hn - h * tiles_n) * kFN, m0 = (t % tiles_m) * BM;
+            float sum[kFN];
+#pragma unroll
+            for (int c = 0; c < kFN; ++c) sum[c] = 0.f;
+            for (int kb = 0; kb < n_kb; ++kb, ++it) {
+                const unsigned acc = it & 3u;
+                mbar_wait_bounded(&t_full[acc], (it >> 2) & 1u);
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+                for (int cb = 0; cb < kFN / 32; ++cb) {
+                    uint32_t v[32];
+                    const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + acc * kFN + cb * 32;
+                    asm volatile(
+                        "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
+                        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
+                        "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+                        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
+                          "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]),
+                          "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]),
+                          "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
+                        : "r"(taddr)
+                        : "memory");
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                    for (int i = 0; i < 32; ++i) sum[cb * 32 + i] += __uint_as_float(v[i]);
+                }
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&t_empty[acc]);
+            }
+            // The sums go out through shared memory, a row per step and four columns per lane: coalesced, and a short loop where the
+            // unrolled one (128 copies of the epilogue) was bound by instruction fetches.
+            float* tile = stage + (warp - 2) * 32 * kFStride;
+            const int rows = min(32, M - (m0 + q * 32)), n = n0 + 4 * lane;
+            __syncwarp();
+#pragma unroll
+            for (int c = 0; c < kFN; c += 4)
+                *reinterpret_cast<float4*>(tile + lane * kFStride + c) = make_float4(sum[c], sum[c + 1], sum[c + 2], sum[c + 3]);
+            __syncwarp();
+            if (n < N) {
+                const size_t m = (size_t)(m0 + q * 32), col = (size_t)h * p.y_hs + n;
+                const float* gate = p.gate ? p.gate + m * p.ldg + (p.head_gate ? (size_t)h : (size_t)h * N + n) : nullptr;
+#pragma unroll 1
+                for (int r = 0; r < rows; ++r) {
+                    float4 v = *reinterpret_cast<const float4*>(tile + r * kFStride + 4 * lane);
+                    v.x *= p.alpha; v.y *= p.alpha; v.z *= p.alpha; v.w *= p.alpha;
+                    if (p.act) { v.x = f32_act(p.act, v.x); v.y = f32_act(p.act, v.y); v.z = f32_act(p.act, v.z); v.w = f32_act(p.act, v.w); }
+                    if (gate) {
+                        const float* z = gate + (size_t)r * p.ldg;
+                        if (p.head_gate) {
+                            const float f = 1.0f / (1.0f + expf(-z[0]));
+                            v.x *= f; v.y *= f; v.z *= f; v.w *= f;
+                        } else {
+                            v.x *= 1.0f / (1.0f + expf(-z[0])); v.y *= 1.0f / (1.0f + expf(-z[1]));
+                            v.z *= 1.0f / (1.0f + expf(-z[2])); v.w *= 1.0f / (1.0f + expf(-z[3]));
+                        }
+                    }
+                    const size_t at = (m + r) * p.ldy + col;
+                    *reinterpret_cast<float4*>(p.y + at) = v;
+                    if (p.y_bf16) {
+                        const __nv_bfloat162 lo = __floats2bfloat162_rn(v.x, v.y), hi = __floats2bfloat162_rn(v.z, v.w);
+                        *reinterpret_cast<uint2*>(reinterpret_cast<__nv_bfloat16*>(p.y_bf16) + at) =
+                            make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+                    }
+                }
+            }
+        }
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (warp == 1) {
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(4 * kFN));
+    }
+}
+
+// three bf16 terms of every head's columns, [3][heads][M][K]; an infinity stays one in the first term
+__global__ void __launch_bounds__(256) split3_heads_kernel(const float* __restrict__ x, int ldx, int hs, __nv_bfloat16* __restrict__ xs, int H, int M, int K) {
+    const size_t n = (size_t)H * M * K;
+    const float* row = x + (size_t)blockIdx.x * ldx;
+    for (int i = threadIdx.x; i < H * (K >> 2); i += 256) {   // (K a multiple of 8)
+        const int h = i / (K >> 2), k = 4 * (i - h * (K >> 2));
+        const size_t o = ((size_t)h * M + blockIdx.x) * K + k;
+        __nv_bfloat16 t[3][4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const float v = row[(size_t)h * hs + k + e];
+            t[0][e] = __float2bfloat16_rn(v);
+            const float f0 = __bfloat162float(t[0][e]), r1 = fabsf(f0) <= 3.402823466e38f ? v - f0 : 0.f;
+            t[1][e] = __float2bfloat16_rn(r1);
+            t[2][e] = __float2bfloat16_rn(r1 - __bfloat162float(t[1][e]));
+        }
+#pragma unroll
+        for (int q = 0; q < 3; ++q) *reinterpret_cast<uint2*>(xs + q * n + o) = *reinterpret_cast<const uint2*>(t[q]);
+    }
+}
+
 // ---- host side ---------------------------------------------------------------------------------------------------
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
                                   const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
@@ -402,6 +606,27 @@ cudaError_t launch_gemm_tcgen05_bf16(const void* a_bf16, int terms, const void* 
         ma, mb, y, ep.residual, M, N, K, terms, ep.dyt_w, ep.dyt_b, ep.dyt_alpha,
         reinterpret_cast<__nv_bfloat16*>(ep.y_bf16), groups ? groups->row_group : nullptr,
         groups ? groups->group_rows : 0, groups ? groups->n_rows : nullptr);
+    return cudaGetLastError();
+}
+
+bool gemm_f32_ok(const F32Product& p) {
+    return p.heads > 0 && gemm_tcgen05_shape_ok(p.M, p.N, p.K) && p.ldy % 4 == 0 && p.y_hs % 4 == 0 && (reinterpret_cast<uintptr_t>(p.y) & 15) == 0 &&
+           (reinterpret_cast<uintptr_t>(p.y_bf16) & 7) == 0 && (reinterpret_cast<uintptr_t>(p.w) & 15) == 0;
+}
+
+cudaError_t launch_gemm_f32(const F32Product& p, void* work, cudaStream_t st) {
+    if (!gemm_f32_ok(p)) return cudaErrorNotSupported;
+    int dev = 0, sms = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(dia_gemm_f32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kFSmem);
+    if (e != cudaSuccess) return e;
+    CUtensorMap ma, mb;
+    if (!make_map(&ma, work, (long long)kTerms * p.heads * p.M, p.K, BM) || !make_map(&mb, p.w, (long long)p.heads * p.N, p.K, kFN))
+        return cudaErrorNotSupported;
+    split3_heads_kernel<<<p.M, 256, 0, st>>>(p.a, p.lda, p.a_hs, reinterpret_cast<__nv_bfloat16*>(work), p.heads, p.M, p.K);
+    const int n_tiles = p.heads * ((p.N + kFN - 1) / kFN) * ((p.M + BM - 1) / BM);
+    dia_gemm_f32_kernel<<<std::min(n_tiles, sms), kGemmThreads, kFSmem, st>>>(ma, mb, p);
     return cudaGetLastError();
 }
 

@@ -34,4 +34,21 @@ inline bool gemm_tcgen05_shape_ok(int M, int N, int K) { return M > 0 && N > 0 &
 cudaError_t launch_gemm_tcgen05_bf16(const void* a_bf16, int terms, const void* wt, long long wt_rows, float* y, int M, int N,
                                      int K, const GemmEpilogue& ep, const GemmGroups* groups, cudaStream_t st);
 
+// Per head h < heads: Y[m][h y_hs + n] = act(alpha sum_k A[m][h a_hs + k] W[h][n][k]) [* sigmoid of a gate column], as fp32 FMA
+// arithmetic gives it: A (fp32, row stride lda) is split into three bf16 terms (24 bits) in `work` (gemm_f32_work_bytes), every 64
+// products of a sum are accumulated in tensor memory and added to the sum in fp32 registers.  W: bf16 [heads * N][K].
+struct F32Product {
+    const float* a; int lda, a_hs;
+    const void* w;
+    float* y; int ldy, y_hs;
+    void* y_bf16;                            // a bf16 copy of y; null: none
+    int heads, M, N, K;
+    float alpha;
+    int act;                                 // 0: none, 2: max(z, 0)^2, 3: gelu, the tanh form
+    const float* gate; int ldg, head_gate;   // gate[m * ldg + h N + n], with head_gate gate[m * ldg + h]; null: none
+};
+bool gemm_f32_ok(const F32Product& p);
+inline size_t gemm_f32_work_bytes(size_t rows, size_t columns) { return 6 * rows * columns; }      // columns: heads * K
+cudaError_t launch_gemm_f32(const F32Product& p, void* work, cudaStream_t st);
+
 }  // namespace dia

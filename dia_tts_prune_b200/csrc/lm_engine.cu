@@ -157,6 +157,8 @@ struct lm_b200_engine {
     bool stream_form = false;
     float* split_ws;                             // partial results of the key splits of a few rows' attention
     unsigned* split_arrived;                     // ... and their arrival counters (zero between launches)
+    void* a_split;                               // the bf16 terms of an fp32 product's operand
+    size_t a_split_bytes;
     void* kv_split;                              // keys and values of a long step's attention, split for the tensor cores
     size_t kv_split_bytes;
     // steps of a few rows are captured once per (rows, sequences, wanted) into a CUDA graph over these fixed buffers
@@ -183,6 +185,28 @@ bool tensor_path(const lm_b200_engine* e, int M, int N, int K) {
 }
 
 const dia::GemmEpilogue kPlain{nullptr, nullptr, nullptr, 0.f, nullptr};
+
+// Y = act(A W^T) in fp32 arithmetic.  More than a few rows go to the tensor cores with the operand split into three terms where the
+// shape and the room allow it (4096 x 2048 x 2048: 1.2 ms on the FMA tiles); narrow products (the router) stay on the row kernel.
+cudaError_t linear_f32(lm_b200_engine* e, const float* A, int lda, const void* W, float* Y, int ldy, int M, int N, int K, cudaStream_t st,
+                       int act = lm::kActNone) {
+    if (M > lm::kRowsKernelMax && N > lm::kRowsKernelMaxOut && act != lm::kActXielu && e->a_split_bytes >= dia::gemm_f32_work_bytes(M, K)) {
+        const dia::F32Product p{A, lda, 0, W, Y, ldy, 0, nullptr, 1, M, N, K, 1.f, act, nullptr, 0, 0};
+        if (dia::gemm_f32_ok(p)) return dia::launch_gemm_f32(p, e->a_split, st);
+    }
+    return lm::launch_linear(A, lda, W, 0, Y, ldy, M, N, K, nullptr, st, act);
+}
+
+// per-head products (lm::launch_head_linear), likewise
+// (work: room for the operand's terms)
+cudaError_t head_linear(const float* A, int lda, const void* W, float* Y, int ldy, void* y_bf16, int M, int H, int N, int K,
+                        float alpha, const float* gate, int ldg, void* work, cudaStream_t st, int a_hs = 0, int y_hs = 0, bool head_gate = false) {
+    if (M > lm::kRowsKernelMax) {
+        const dia::F32Product p{A, lda, a_hs > 0 ? a_hs : K, W, Y, ldy, y_hs > 0 ? y_hs : N, y_bf16, H, M, N, K, alpha, 0, gate, ldg, head_gate ? 1 : 0};
+        if (dia::gemm_f32_ok(p)) return dia::launch_gemm_f32(p, work, st);
+    }
+    return lm::launch_head_linear(A, lda, W, Y, ldy, y_bf16, M, H, N, K, alpha, gate, ldg, st, a_hs, y_hs, head_gate);
+}
 
 struct StepView {
     const int *token, *want;
@@ -481,7 +505,7 @@ int mixer(lm_b200_engine* e, const lm_b200_layer& l, const float* h, const void*
         }
         LCK(dia::launch_gemm_tcgen05_bf16(hb, 1, l.w_qk, nq + nk, e->qk, M, nq + nk, D, kPlain, nullptr, st));
     } else {
-        LCK(lm::launch_linear(h, D, l.w_qk, 0, e->qk, nq + nk, M, nq + nk, D, nullptr, st));
+        LCK(linear_f32(e, h, D, l.w_qk, e->qk, nq + nk, M, nq + nk, D, st));
     }
     LCK(lm::launch_qk_norm_cache(e->qk, nq, nk, l.q_norm, l.k_norm, e->m.eps, l.k_pages, l.v_pages, pm, l.kv_heads, l.dim,
                                  v.rm, M, st));
@@ -500,7 +524,7 @@ int mixer(lm_b200_engine* e, const lm_b200_layer& l, const float* h, const void*
         LCK(lm::launch_linear_rows_residual(e->att, nq, l.w_o, fuse_x, M, D, nq, N(l.norm_mix_out), next, st));
         return LM_B200_OK;
     } else {
-        LCK(lm::launch_linear(e->att, nq, l.w_o, 0, y, D, M, D, nq, nullptr, st));
+        LCK(linear_f32(e, e->att, nq, l.w_o, y, D, M, D, nq, st));
     }
     if (fuse_x) LCK(lm::launch_residual_dyt(fuse_x, y, nullptr, nullptr, 0, N(l.norm_mix_out), M, D, st));
     return LM_B200_OK;
@@ -522,7 +546,7 @@ int feed_forward(lm_b200_engine* e, const lm_b200_layer& l, const float* h, cons
                                          nrm, next, st));
         return LM_B200_OK;
     }
-    LCK(lm::launch_linear(h, D, l.w_router, 0, e->z, E, M, E, D, nullptr, st));
+    LCK(linear_f32(e, h, D, l.w_router, e->z, E, M, E, D, st));
     LCK(lm::launch_router_topk(e->z, E, top, M, e->sel_e, e->sel_w, st));
     const int n_assign = M * top;
     // both expert products on the tensor cores, or neither: the groups are padded to the row tile of the kernel that runs
@@ -555,9 +579,9 @@ int feed_forward(lm_b200_engine* e, const lm_b200_layer& l, const float* h, cons
             LCK(lm::launch_silu_mul(e->sgu, nullptr, e->smidb, M, Sf, nullptr, st));
             LCK(dia::launch_gemm_tcgen05_bf16(e->smidb, 1, l.ws_down, D, e->y, M, D, Sf, kPlain, nullptr, st));
         } else {
-            LCK(lm::launch_linear(h, D, l.ws_gate_up, 0, e->sgu, 2 * Sf, M, 2 * Sf, D, nullptr, st));
+            LCK(linear_f32(e, h, D, l.ws_gate_up, e->sgu, 2 * Sf, M, 2 * Sf, D, st));
             LCK(lm::launch_silu_mul(e->sgu, e->smid, nullptr, M, Sf, nullptr, st));
-            LCK(lm::launch_linear(e->smid, Sf, l.ws_down, 0, e->y, D, M, D, Sf, nullptr, st));
+            LCK(linear_f32(e, e->smid, Sf, l.ws_down, e->y, D, M, D, Sf, st));
         }
     }
     LCK(lm::launch_residual_dyt(x, Sf > 0 ? e->y : nullptr, e->parts, e->slot_of, top, nrm, M, D, st));
@@ -574,14 +598,14 @@ int product(lm_b200_engine* e, const float* A, const void* Ab, int lda, const vo
         return LM_B200_OK;
     }
     if (!add) {
-        LCK(lm::launch_linear(A, lda, W, 0, out, N, M, N, K, nullptr, st));
+        LCK(linear_f32(e, A, lda, W, out, N, M, N, K, st));
         return LM_B200_OK;
     }
     if (M <= lm::kRowsKernelMax) {
         LCK(lm::launch_linear_rows_residual(A, lda, W, out, M, N, K, lm::NormW{nullptr, nullptr, 0.f}, lm::TapOut{}, st));
         return LM_B200_OK;
     }
-    LCK(lm::launch_linear(A, lda, W, 0, e->y, N, M, N, K, nullptr, st));
+    LCK(linear_f32(e, A, lda, W, e->y, N, M, N, K, st));
     LCK(lm::launch_add_rows(out, e->y, M, N, st));
     return LM_B200_OK;
 }
@@ -616,8 +640,8 @@ int mixer_kernels(lm_b200_engine* e, const lm_b200_layer& l, const InCols& c, fl
                       b0 = g0 + l.heads * l.vdim;
             // the second steps of the decay and gate projections: fp32 products (they enter the recurrence), straight into
             // the decay and gate columns of the recurrence inputs
-            LCK(lm::launch_linear(proj + c.a1, c.n, l.w_a2, 0, e->rec + d0, ldr, M, l.heads * l.dim, l.rank_a, nullptr, st));
-            LCK(lm::launch_linear(proj + c.g1, c.n, l.w_g2, 0, e->rec + g0, ldr, M, l.heads * l.vdim, l.rank_g, nullptr, st));
+            LCK(linear_f32(e, proj + c.a1, c.n, l.w_a2, e->rec + d0, ldr, M, l.heads * l.dim, l.rank_a, st));
+            LCK(linear_f32(e, proj + c.g1, c.n, l.w_g2, e->rec + g0, ldr, M, l.heads * l.vdim, l.rank_g, st));
             LCK(lm::launch_delta_prep(proj, c.n, c.beta, d, l.conv_tail, v.rm, e->rec, ldr, M, st));
             LCK(lm::launch_conv_tail(proj, c.n, C, l.conv_taps, l.conv_tail, v.sm, n_seq, st));
             const lm::ScanInputs si{0, k0, d0, v0, b0};
@@ -679,7 +703,7 @@ int product_ld(lm_b200_engine* e, const float* A, int lda, const void* Ab, const
         LCK(dia::launch_gemm_tcgen05_bf16(Ab, 1, W, N, out, M, N, K, kPlain, nullptr, st));
         return LM_B200_OK;
     }
-    LCK(lm::launch_linear(A, lda, W, 0, out, N, M, N, K, nullptr, st));
+    LCK(linear_f32(e, A, lda, W, out, N, M, N, K, st));
     return LM_B200_OK;
 }
 
@@ -708,7 +732,7 @@ int stream_mixer_kernels(lm_b200_engine* e, const lm_b200_layer& l, const MixPla
         if (rc) return rc;
         // scores q_h . (W_uk,h c_j) = (W_uk,h^T q_h) . c_j: the query goes into the latent space, with the score multiplier;
         // its turned part stands behind it, against the turned key part of the cached row
-        LCK(lm::launch_head_linear(e->qk, nq, l.w_uk_t, e->qlat, nl, nullptr, M, H, l.kv_rank, l.dim, l.scale, nullptr, 0, st, dq, RK));
+        LCK(head_linear(e->qk, nq, l.w_uk_t, e->qlat, nl, nullptr, M, H, l.kv_rank, l.dim, l.scale, nullptr, 0, e->olat, st, dq, RK));
         if (rd > 0)
             LCK(lm::launch_rot_rows(e->qk, nq, l.dim, dq, e->qlat, nl, l.kv_rank, RK, H, rd, rot, H, l.scale, l.scale, v.rm, M, st));
         if (lm::talk_attention_supported(latent_shape(l)))
@@ -718,7 +742,7 @@ int stream_mixer_kernels(lm_b200_engine* e, const lm_b200_layer& l, const MixPla
             LCK(lm::launch_latent_attention_rows(e->qlat, l.latent_pages, pm, H, l.kv_rank, l.sink, v.rm, e->olat, M, st, rd,
                                                  l.window > 0 ? l.window : 0));
         // sum_j p_j (W_uv,h c_j) = W_uv,h (sum_j p_j c_j), times the sigmoid of the gate columns
-        LCK(lm::launch_head_linear(e->olat, no, l.w_uv, at.out, at.ldo, at.out_b, M, H, l.vdim, l.kv_rank, at.scale, gate, ld, st,
+        LCK(head_linear(e->olat, no, l.w_uv, at.out, at.ldo, at.out_b, M, H, l.vdim, l.kv_rank, at.scale, gate, ld, e->qlat, st,
                                    0, 0, l.mixer_gate == LM_B200_GATE_SIGMOID_HEAD));
     } else if (l.mixer == LM_B200_MIXER_GATED_DELTA) {
         const lm::DeltaShape d{H, l.kv_heads, l.dim, l.vdim, l.conv_taps, l.unit_eps, l.conv_w, l.a_log, l.dt_bias};
@@ -808,7 +832,7 @@ int token_input(lm_b200_engine* e, const lm_b200_layer& l, const float* x, const
     const lm::TokenSide ts{l.side_table, l.side_ld, l.side_off, n, ids, e->m.vocab};
     if (M <= lm::kRowsKernelMax) {
         LCK(lm::launch_side_gate_rows(x, D, l.w_side_gate, ts, e->side_g, M, st));
-        LCK(lm::launch_linear(e->side_g, n, l.w_side_proj, 0, y, D, M, D, n, nullptr, st));
+        LCK(linear_f32(e, e->side_g, n, l.w_side_proj, y, D, M, D, n, st));
         return LM_B200_OK;
     }
     int rc = product_ld(e, x, D, xb, l.w_side_gate, e->side_z, M, n, D, st);
@@ -834,8 +858,8 @@ int plain_dense_unit(lm_b200_engine* e, const float* h, const void* hb, int M, i
         LCK(dia::launch_gemm_tcgen05_bf16(e->smidb, 1, w_down, D, out, M, D, F, kPlain, nullptr, st));
         return LM_B200_OK;
     }
-    LCK(lm::launch_linear(h, D, w_up, 0, e->smid, F, M, F, D, nullptr, st, act));
-    LCK(lm::launch_linear(e->smid, F, w_down, 0, out, D, M, D, F, nullptr, st));
+    LCK(linear_f32(e, h, D, w_up, e->smid, F, M, F, D, st, act));
+    LCK(linear_f32(e, e->smid, F, w_down, out, D, M, D, F, st));
     return LM_B200_OK;
 }
 
@@ -853,10 +877,10 @@ int gated_unit(lm_b200_engine* e, const lm_b200_layer& l, const float* h, const 
         const lm::GluAct act{glu_kind(l.act), limit, limit};
         LCK(lm::launch_gated_rows(h, D, nullptr, 0, nullptr, 0, F, D, nullptr, w_gu, e->smid, M, F, st, act));
     } else {
-        LCK(lm::launch_linear(h, D, w_gu, 0, e->sgu, 2 * F, M, 2 * F, D, nullptr, st));
+        LCK(linear_f32(e, h, D, w_gu, e->sgu, 2 * F, M, 2 * F, D, st));
         LCK(lm::launch_silu_mul(e->sgu, e->smid, nullptr, M, F, nullptr, st, glu_kind(l.act), limit));
     }
-    LCK(lm::launch_linear(e->smid, F, w_down, 0, out, D, M, D, F, nullptr, st));
+    LCK(linear_f32(e, e->smid, F, w_down, out, D, M, D, F, st));
     return LM_B200_OK;
 }
 
@@ -890,7 +914,7 @@ int stream_ff(lm_b200_engine* e, const lm_b200_layer& l, const float* h, const v
                                          grouped ? h : nullptr, sgate, zc));
         return LM_B200_OK;
     }
-    LCK(lm::launch_linear(h, D, l.w_router, 0, e->z, zc, M, zc, D, nullptr, st));
+    LCK(linear_f32(e, h, D, l.w_router, e->z, zc, M, zc, D, st));
     LCK(lm::launch_router_topk(e->z, zc, top, M, e->sel_e, e->sel_w, st, l.router_bias, !grouped, grouped ? &gr : nullptr));
     const bool tc = hb && tensor_path(e, M, 2 * F, D) && tensor_path(e, M, D, F);
     const int pad = tc ? dia::kGemmRowTile : lm::kTileRows;
@@ -981,7 +1005,7 @@ int lm_b200_engine_create(const lm_b200_model* model, const lm_b200_layer* layer
         s.n_slots = m.n_slots;
         kv_split = std::max(kv_split, dia::split_attention_work_bytes(s, (int)split_keys));
     };
-    size_t n_streams = 0, n_lat = 0, q_rank = 0, n_heads = 0, n_side = 0;
+    size_t n_streams = 0, n_lat = 0, q_rank = 0, n_heads = 0, n_side = 0, n_second = 0, olat_room = 0, qlat_room = 0;
     bool pre = false, any_parallel = false;
     e->stream_form = e->layers[0].form == LM_B200_FORM_STREAMS;
     for (const lm_b200_layer& l : e->layers) {
@@ -996,6 +1020,9 @@ int lm_b200_engine_create(const lm_b200_model* model, const lm_b200_layer* layer
                     qk = std::max(qk, (size_t)p.heads * (p.dim + p.rot_dim));
                     n_lat = std::max(n_lat, (size_t)p.heads * (p.kv_rank + p.rot_dim));
                     q_rank = std::max(q_rank, (size_t)p.q_rank);
+                    // the operands' terms of the per-head products lie in the other one's buffer
+                    olat_room = std::max(olat_room, dia::gemm_f32_work_bytes(R, (size_t)p.heads * p.dim));
+                    qlat_room = std::max(qlat_room, dia::gemm_f32_work_bytes(R, (size_t)p.heads * p.kv_rank));
                     if (lm::talk_attention_supported(latent_shape(p))) split_dim = std::max(split_dim, (size_t)p.heads * (p.kv_rank + 2));
                     split_room(p.heads, 1, p.kv_rank + p.rot_dim, p.kv_rank, true, nullptr);
                 } else if (p.mixer == LM_B200_MIXER_MLSTM) {
@@ -1022,6 +1049,7 @@ int lm_b200_engine_create(const lm_b200_model* model, const lm_b200_layer* layer
             n_in = std::max(n_in, (size_t)l.n_in);
             k_out = std::max(k_out, (size_t)l.k_out);
             n_rec = std::max(n_rec, (size_t)rec_cols(l));
+            if (l.mixer == LM_B200_MIXER_CHANNEL_DELTA) n_second = std::max(n_second, (size_t)std::max(l.rank_a, l.rank_g));
             pre = pre || l.w_pre;
             if (l.mixer == LM_B200_MIXER_TALK_ATTENTION) {
                 split_dim = std::max(split_dim, (size_t)l.heads * (l.vdim + 2));
@@ -1048,10 +1076,10 @@ int lm_b200_engine_create(const lm_b200_model* model, const lm_b200_layer* layer
                  o_y = take(R * D * 4), o_z = take(R * E * 4), o_sel_w = take(R * top * 4), o_sel_e = take(R * top * 4),
                  o_slot_of = take(R * top * 4), o_a_row = take(slots * 4), o_a_scale = take(slots * 4),
                  o_a_expert = take(slots * 4), o_n_slots = take(4), o_gu = take(slots * 2 * F * 4), o_mid = take(slots * F * 4),
-                 o_parts = take(slots * D * 4), o_sgu = take(R * 2 * Sf * 4), o_smid = take(R * Sf * 4), o_hw = take(R * D * 4);
+                 o_parts = take(slots * D * 4), o_sgu = take(R * 2 * Sf * 4), o_smid = take(R * Sf * 4), o_ff_end = off, o_hw = take(R * D * 4);
     const size_t o_x0 = take(pre ? R * D * 4 : 0), o_cat = take(pre ? R * 2 * D * 4 : 0), o_proj = take(R * n_in * 4),
                  o_rec = take(R * n_rec * 4), o_outcat = take(R * k_out * 4);
-    const size_t o_xs = take(R * n_streams * D * 4), o_qlat = take(R * n_lat * 4), o_olat = take(R * n_lat * 4),
+    const size_t o_xs = take(R * n_streams * D * 4), o_qlat = take(std::max(R * n_lat * 4, qlat_room)), o_olat = take(std::max(R * n_lat * 4, olat_room)),
                  o_floor = take(R * n_heads * 4), o_unit = take(2 * 4);
     const size_t o_ymix = take(any_parallel ? R * D * 4 : 0), o_h2 = take(any_parallel ? R * D * 4 : 0);
     const size_t o_split = take((size_t)lm::kAttnRowsKernelMax * lm::kAttnSplitsMax * split_dim * 4);
@@ -1066,7 +1094,13 @@ int lm_b200_engine_create(const lm_b200_model* model, const lm_b200_layer* layer
     const size_t o_catb = take(tcb && pre ? R * 2 * D * 2 : 0), o_outcatb = take(tcb ? R * k_out * 2 : 0);
     const size_t o_cqb = take(tcb ? R * q_rank * 2 : 0), o_h2b = take(tcb && any_parallel ? R * D * 2 : 0),
                  o_sidegb = take(tcb ? R * n_side * 2 : 0);
-    const size_t o_kvsplit = take(kv_split);
+    // (a feed-forward's buffers are not in use while a mixer runs)
+    const bool over_ff = o_ff_end - o_gu >= kv_split;
+    const size_t o_kvsplit = over_ff ? o_gu : take(kv_split);
+    // columns of the widest fp32 operand: with float32 precision every product's, otherwise the second steps' of two-step projections
+    size_t a_cols = n_second;
+    if (m.precision == LM_B200_PRECISION_FP32) a_cols = std::max({a_cols, 2 * D, att, Sf, k_out, q_rank, n_side});
+    const size_t a_split = dia::gemm_f32_work_bytes(R, a_cols), o_asplit = take(a_split);
     if (cudaMalloc(&e->arena, off) != cudaSuccess) {
         (void)cudaGetLastError();
         delete e;
@@ -1089,6 +1123,8 @@ int lm_b200_engine_create(const lm_b200_model* model, const lm_b200_layer* layer
     e->ymix = (float*)(b + o_ymix); e->h2 = (float*)(b + o_h2); e->h2b = b + o_h2b;
     e->side_z = (float*)(b + o_sidez); e->side_g = (float*)(b + o_sideg); e->side_gb = b + o_sidegb;
     e->split_ws = (float*)(b + o_split);
+    e->a_split = b + o_asplit;
+    e->a_split_bytes = a_split;
     e->kv_split = kv_split ? b + o_kvsplit : nullptr;
     e->kv_split_bytes = kv_split;
     e->split_arrived = (unsigned*)(b + o_arrived);
@@ -1139,7 +1175,7 @@ int head_rows(lm_b200_engine* e, const float* x, const StepView& v, int n_want, 
         if (tc)
             LCK(dia::launch_gemm_tcgen05_bf16(e->hwb, 1, e->m.head, e->m.vocab, logits_out, n_want, e->m.vocab, D, kPlain, nullptr, st));
         else
-            LCK(lm::launch_linear(e->hw, D, e->m.head, 0, logits_out, e->m.vocab, n_want, e->m.vocab, D, nullptr, st));
+            LCK(linear_f32(e, e->hw, D, e->m.head, logits_out, e->m.vocab, n_want, e->m.vocab, D, st));
     }
     return LM_B200_OK;
 }
