@@ -362,6 +362,7 @@ split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_co
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ float s_red[16];
     __shared__ uint32_t s_tmem;
+    __shared__ int s_rows[2];
     unsigned char* ring = smem;
     unsigned char* qs = ring + (size_t)geo.n_slots * geo.slot_bytes;
     uint64_t* full = reinterpret_cast<uint64_t*>(qs + geo.q_bytes);
@@ -383,8 +384,37 @@ split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_co
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int PK = 1 << geo.pk_shift;
     const int h0 = blockIdx.x * PK, rep = p.heads / p.kv_heads, g = h0 / rep;
-    const int r0 = (gridDim.y - 1 - blockIdx.y) * TT;         // later tokens see more keys: their tiles start first
-    const int n_tok = min(TT, p.M - r0);
+    // later tokens see more keys: their tiles start first.  With the step's sequences at hand a tile holds rows of one of them (a
+    // tile with the rows of 24 decoding sequences walked the keys of all 24 one after the other)
+    int r0 = (gridDim.y - 1 - blockIdx.y) * TT, n_tok = min(TT, p.M - r0);
+    if (p.n_seq > 0) {
+        if (tid == 0) s_rows[1] = 0;
+        __syncthreads();
+        if (warp == 0) {
+            const int want = gridDim.y - 1 - blockIdx.y;
+            int run = 0;
+            for (int s0 = 0; s0 < p.n_seq; s0 += 32) {
+                const int count = s0 + lane < p.n_seq ? p.seq_count[s0 + lane] : 0, n = (count + TT - 1) / TT;
+                int sum = n;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int v = __shfl_up_sync(0xffffffffu, sum, o);
+                    if (lane >= o) sum += v;
+                }
+                const int begin = run + sum - n;
+                if (want >= begin && want < begin + n) {
+                    s_rows[0] = p.seq_row0[s0 + lane] + (want - begin) * TT;
+                    s_rows[1] = min(TT, count - (want - begin) * TT);
+                }
+                run += __shfl_sync(0xffffffffu, sum, 31);
+                if (run > want) break;
+            }
+        }
+        __syncthreads();
+        r0 = s_rows[0];
+        n_tok = s_rows[1];
+        if (n_tok == 0) return;                               // (the grid is an upper bound)
+    }
 
     if (tid == 0) {
         for (int i = 0; i < kMaxSlots; ++i) { mbar_init(&full[i], 4); mbar_init(&empty[i], 1); }
@@ -934,7 +964,7 @@ cudaError_t launch_inst(const SplitAttention& a, const Geometry& g, size_t smem,
         if (e != cudaSuccess) return e;
         if (dev >= 0 && dev < 64) allowed[dev] = smem;
     }
-    const int tt = kRows >> g.pk_shift, tiles = (a.M + tt - 1) / tt;
+    const int tt = kRows >> g.pk_shift, tiles = a.n_seq > 0 ? a.M / tt + a.n_seq : (a.M + tt - 1) / tt;
     if (tiles > 65535) return cudaErrorNotSupported;
     if (a.work) split_keys_kernel<<<dim3(g.cap_tiles, g.parts), 256, 0, st>>>(a, g);
     split_attention_kernel<NVS><<<dim3(a.heads >> g.pk_shift, tiles), kSplitThreadsTC, smem, st>>>(a, g);

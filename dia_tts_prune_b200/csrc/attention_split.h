@@ -35,11 +35,12 @@ struct SplitAttention {
     float* out; int ldo; void* out_bf16;
     float out_scale;
     const float* gate; const float* head_gate; int ldg;
-    // Optional: room in which a launch in front splits the keys and values that the rows see once for all row tiles (null: every row
-    // tile splits them for itself).  seq_*: per sequence its slot, first row and row count; n_slots: slots there are.  Keys beyond
-    // the room's size are split by the row tiles.
-    void* work; size_t work_bytes; int n_slots;
+    // Optional (n_seq 0: not given): the step's sequences - slot, first row and row count of each
     const int* seq_slot; const int* seq_row0; const int* seq_count; int n_seq;
+    // Optional, with the sequences: room in which a launch in front splits the keys and values that the rows see once for all row
+    // tiles (null: every row tile splits them for itself).  n_slots: slots there are.  Keys beyond the room's size are split by the
+    // row tiles.
+    void* work; size_t work_bytes; int n_slots;
 };
 
 // whether the kernel takes the shape (head sizes, alignment); M does not matter

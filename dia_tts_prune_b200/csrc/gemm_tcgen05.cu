@@ -518,6 +518,181 @@ dia_gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     }
 }
 
+// ---------------------------------------------------------------------------------------------------------------------
+// Few rows: a cluster of S CTAs owns 128 weight rows, each CTA a range of k-blocks.
+//   warp 0    requests the CTA's weight tiles [128 x 64] (TMA, 128-byte swizzle) ahead of the rows - before the kernel's predecessor
+//             has ended, when launched early
+//   all warps split the rows' k range into three bf16 terms: column term * Mp + m of the [NB x 64] operand of a k-block
+//   warp 1    per k-block 4 MMAs (M = 128, N = NB) into an accumulator of its own
+//   warps 2-5 add the k-blocks' accumulators in fp32 registers (weight row = lane), then the three terms; the CTAs' partial sums
+//             meet in shared memory and every CTA of the cluster adds its share of the outputs, in the order of the k ranges
+// Bound: the weights' bytes.  The row kernel reads them once per row from L2 instead: 8 rows x 2048 x 6144 took 35 us.
+constexpr int kRThreads = 192, kRSlotsMost = 8, kRSmemMost = 226 * 1024;
+
+__device__ __forceinline__ uint32_t cluster_rank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ float load_remote(const float* local, uint32_t rank) {
+    uint32_t a;
+    float v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(local)), "r"(rank));
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
+    return v;
+}
+__device__ __forceinline__ void cluster_sync_all() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// NB: columns of the rows' operand (32 for up to 8 rows, 96 for up to 32)
+template <int NB>
+__global__ void __launch_bounds__(kRThreads, 1)
+dia_gemm_few_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ FewRowsProduct p, int kb_per, int n_slots) {
+    constexpr int Mp = NB / 3 / 8 * 8, kBufs = 512 / NB > 8 ? 8 : 512 / NB, kCols = kBufs * NB > 256 ? 512 : 256;
+    extern __shared__ unsigned char smem_raw[];
+    unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    __shared__ uint64_t w_full[kRSlotsMost], w_empty[kRSlotsMost], t_full[8], t_empty[8];
+    __shared__ uint32_t tmem_slot;
+    unsigned char* ring = smem;
+    unsigned char* rows = ring + n_slots * kTileBytes;                         // [kb_per][NB x 64] bf16
+    float* part = reinterpret_cast<float*>(rows + (size_t)kb_per * NB * 128);  // [Mp][128]
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int S = gridDim.y, n_kb = (p.K + BK - 1) / BK, rank = blockIdx.y, n0 = blockIdx.x * BM;
+    const int kb0 = rank * kb_per, kbs = max(0, min(kb_per, n_kb - kb0));
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if (tid == 0) {
+        for (int i = 0; i < kRSlotsMost; ++i) { mbar_init(&w_full[i], 1); mbar_init(&w_empty[i], 1); }
+        for (int i = 0; i < 8; ++i) { mbar_init(&t_full[i], 1); mbar_init(&t_empty[i], 4); }
+        fence_mbar_init();
+        for (int kb = 0; kb < min(kbs, n_slots); ++kb) {
+            mbar_arrive_expect_tx(&w_full[kb], kTileBytes);
+            tma_load_2d(smem_u32(ring + kb * kTileBytes), &map_w, smem_u32(&w_full[kb]), (kb0 + kb) * BK, n0);
+        }
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)), "r"(kCols));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::);
+    }
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    // ---- the rows' terms: 8 channels per item ----
+    for (int i = tid; i < Mp * kbs * 8; i += kRThreads) {
+        const int m = i / (kbs * 8), c = i - m * (kbs * 8), kb = c >> 3, ch = c & 7, k = (kb0 + kb) * BK + ch * 8;
+        float v[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) v[e] = 0.f;
+        if (m < p.M && k < p.K) {                             // (K a multiple of 8)
+            const float4* src = reinterpret_cast<const float4*>(p.a + (size_t)m * p.lda + k);
+            const float4 x = src[0], y = src[1];
+            v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w; v[4] = y.x; v[5] = y.y; v[6] = y.z; v[7] = y.w;
+        }
+        __nv_bfloat16 t[3][8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+            t[0][e] = __float2bfloat16_rn(v[e]);
+            const float f0 = __bfloat162float(t[0][e]), r1 = fabsf(f0) <= 3.402823466e38f ? v[e] - f0 : 0.f;
+            t[1][e] = __float2bfloat16_rn(r1);
+            t[2][e] = __float2bfloat16_rn(r1 - __bfloat162float(t[1][e]));
+        }
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+            const int r = q * Mp + m;
+            *reinterpret_cast<uint4*>(rows + (size_t)kb * NB * 128 + (r >> 3) * 1024 + (r & 7) * 128 + ((ch ^ (r & 7)) << 4)) =
+                *reinterpret_cast<const uint4*>(t[q]);
+        }
+    }
+    for (int i = tid; i < (NB - 3 * Mp) * kbs * 8; i += kRThreads) {           // columns that no row uses
+        const int r = 3 * Mp + i / (kbs * 8), c = i % (kbs * 8);
+        *reinterpret_cast<uint4*>(rows + (size_t)(c >> 3) * NB * 128 + (r >> 3) * 1024 + (r & 7) * 128 + ((c & 7) << 4)) = make_uint4(0u, 0u, 0u, 0u);
+    }
+    fence_proxy_async();
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = tmem_slot;
+    if (warp == 0) {
+        if (lane == 0)
+            for (int kb = n_slots; kb < kbs; ++kb) {
+                const int s = kb % n_slots;
+                mbar_wait_bounded(&w_empty[s], ((kb / n_slots) & 1u) ^ 1u);
+                mbar_arrive_expect_tx(&w_full[s], kTileBytes);
+                tma_load_2d(smem_u32(ring + s * kTileBytes), &map_w, smem_u32(&w_full[s]), (kb0 + kb) * BK, n0);
+            }
+    } else if (warp == 1) {
+        const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(NB >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
+        for (int kb = 0; kb < kbs; ++kb) {
+            const int s = kb % n_slots, acc = kb % kBufs;
+            mbar_wait_bounded(&t_empty[acc], ((kb / kBufs) & 1u) ^ 1u);
+            mbar_wait_bounded(&w_full[s], (kb / n_slots) & 1u);
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint64_t adesc = umma_desc(smem_u32(ring + s * kTileBytes)), bdesc = umma_desc(smem_u32(rows + (size_t)kb * NB * 128));
+            if (elect_one_sync()) {
+#pragma unroll
+                for (int j = 0; j < BK / 16; ++j) umma_bf16(tmem + acc * NB, adesc + 2 * j, bdesc + 2 * j, idesc, j != 0 ? 1u : 0u);
+                umma_commit(&w_empty[s]);
+                umma_commit(&t_full[acc]);
+            }
+            __syncwarp();
+        }
+    } else {
+        const int q = warp & 3;
+        float sum[NB];
+#pragma unroll
+        for (int c = 0; c < NB; ++c) sum[c] = 0.f;
+        for (int kb = 0; kb < kbs; ++kb) {
+            const int acc = kb % kBufs;
+            mbar_wait_bounded(&t_full[acc], (kb / kBufs) & 1u);
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+            for (int cb = 0; cb < NB / 16; ++cb) {
+                uint32_t v[16];
+                asm volatile(
+                    "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+                    : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]),
+                      "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+                    : "r"(tmem + ((uint32_t)(q * 32) << 16) + acc * NB + cb * 16)
+                    : "memory");
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                for (int i = 0; i < 16; ++i) sum[cb * 16 + i] += __uint_as_float(v[i]);
+            }
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&t_empty[acc]);
+        }
+#pragma unroll
+        for (int m = 0; m < Mp; ++m) part[m * BM + q * 32 + lane] = (sum[2 * Mp + m] + sum[Mp + m]) + sum[m];
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (warp == 1) {
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kCols));
+    }
+    if (S > 1) cluster_sync_all();
+    // ---- the outputs of the tile, dealt to the cluster's CTAs ----
+    for (int i = rank * kRThreads + tid; i < p.M * BM; i += S * kRThreads) {
+        const int m = i / BM, c = i - m * BM, n = n0 + c;
+        if (n >= p.N) continue;
+        float v;
+        if (S > 1) {
+            float u[8];
+#pragma unroll
+            for (int r = 0; r < 8; ++r) u[r] = r < S ? load_remote(part + i, r) : 0.f;
+            v = u[0];
+#pragma unroll
+            for (int r = 1; r < 8; ++r)
+                if (r < S) v += u[r];
+        } else {
+            v = part[i];
+        }
+        if (p.act) v = f32_act(p.act, v);
+        float* dst = p.y + (size_t)m * p.ldy + n;
+        *dst = p.add ? *dst + v : v;
+    }
+    if (S > 1) cluster_sync_all();                            // (the partial sums stay until every CTA has read them)
+}
+
 // three bf16 terms of every head's columns, [3][heads][M][K]; an infinity stays one in the first term
 __global__ void __launch_bounds__(256) split3_heads_kernel(const float* __restrict__ x, int ldx, int hs, __nv_bfloat16* __restrict__ xs, int H, int M, int K) {
     const size_t n = (size_t)H * M * K;
@@ -628,6 +803,60 @@ cudaError_t launch_gemm_f32(const F32Product& p, void* work, cudaStream_t st) {
     const int n_tiles = p.heads * ((p.N + kFN - 1) / kFN) * ((p.M + BM - 1) / BM);
     dia_gemm_f32_kernel<<<std::min(n_tiles, sms), kGemmThreads, kFSmem, st>>>(ma, mb, p);
     return cudaGetLastError();
+}
+
+// CTAs of a cluster: enough of them to fill the chip, at least two k-blocks each (a rule on N and K alone, so that a row's sums do
+// not depend on what shares its step)
+static int few_rows_split(int N, int K) {
+    const int tiles = (N + BM - 1) / BM, n_kb = (K + BK - 1) / BK;
+    int s = 1;
+    while (s < 8 && tiles * s < 120 && n_kb >= 4 * s) s *= 2;
+    return s;
+}
+static size_t few_rows_smem(int NB, int kb_per, int n_slots) {
+    return 1024 + (size_t)n_slots * kTileBytes + (size_t)kb_per * NB * 128 + (size_t)(NB / 3 / 8 * 8) * BM * 4;
+}
+
+bool gemm_few_rows_ok(const FewRowsProduct& p) {
+    if (p.M <= 0 || p.M > kGemmFewRowsMost || p.N <= 0 || p.K < BK || p.K % 8 || p.lda % 4 || (reinterpret_cast<uintptr_t>(p.a) & 15) ||
+        (reinterpret_cast<uintptr_t>(p.w) & 15))
+        return false;
+    const int n_kb = (p.K + BK - 1) / BK, s = few_rows_split(p.N, p.K), kb_per = (n_kb + s - 1) / s;
+    return few_rows_smem(p.M <= 8 ? 32 : 96, kb_per, std::min(kb_per, 2)) <= kRSmemMost;
+}
+
+template <int NB>
+static cudaError_t launch_few_rows(const FewRowsProduct& p, bool early, cudaStream_t st) {
+    const int n_kb = (p.K + BK - 1) / BK, s = few_rows_split(p.N, p.K), kb_per = (n_kb + s - 1) / s;
+    // two CTAs per SM where at least three slots fit: the next launch's weights are then requested while this one still runs
+    int n_slots = std::min(kRSlotsMost, kb_per);
+    while (n_slots > 3 && few_rows_smem(NB, kb_per, n_slots) > kRSmemMost / 2) --n_slots;
+    while (few_rows_smem(NB, kb_per, n_slots) > kRSmemMost) --n_slots;
+    const size_t smem = few_rows_smem(NB, kb_per, n_slots);
+    cudaError_t e = cudaFuncSetAttribute(dia_gemm_few_rows_kernel<NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    CUtensorMap mw;
+    if (!make_map(&mw, p.w, p.N, p.K, BM)) return cudaErrorNotSupported;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((p.N + BM - 1) / BM, s);
+    cfg.blockDim = dim3(kRThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 1;
+    attr[0].val.clusterDim.y = s;
+    attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = early ? 2 : 1;
+    return cudaLaunchKernelEx(&cfg, dia_gemm_few_rows_kernel<NB>, mw, p, kb_per, n_slots);
+}
+
+cudaError_t launch_gemm_few_rows(const FewRowsProduct& p, bool early, cudaStream_t st) {
+    if (!gemm_few_rows_ok(p)) return cudaErrorNotSupported;
+    return p.M <= 8 ? launch_few_rows<32>(p, early, st) : launch_few_rows<96>(p, early, st);
 }
 
 // fp32 activations: the three-term split (with the row's RMSNorm in front when norm_w is given), then the kernel

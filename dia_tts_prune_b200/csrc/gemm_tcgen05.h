@@ -51,4 +51,19 @@ bool gemm_f32_ok(const F32Product& p);
 inline size_t gemm_f32_work_bytes(size_t rows, size_t columns) { return 6 * rows * columns; }      // columns: heads * K
 cudaError_t launch_gemm_f32(const F32Product& p, void* work, cudaStream_t st);
 
+// The same for a few rows (decoding): Y[m][n] = [res +] act(sum_k A[m][k] W[n][k]).  The weights are the 128-row operand and stream
+// once for all rows; the rows' three terms are the columns of the other operand.  A sum's order depends on N and K only.
+// early: launched with programmatic stream serialization (the weights are requested before the predecessor has ended).
+constexpr int kGemmFewRowsMost = 32;
+struct FewRowsProduct {
+    const float* a; int lda;
+    const void* w;
+    float* y; int ldy;
+    int M, N, K;
+    int act;                                 // as in F32Product
+    int add;                                 // != 0: y += the product
+};
+bool gemm_few_rows_ok(const FewRowsProduct& p);
+cudaError_t launch_gemm_few_rows(const FewRowsProduct& p, bool early, cudaStream_t st);
+
 }  // namespace dia

@@ -172,6 +172,7 @@ struct lm_b200_engine {
 namespace {
 
 constexpr int kTensorRowsMin = 32;               // rows of a step from which its products run on the tensor cores
+constexpr int kFewRowsOutMost = 16384;           // outputs up to which a product of a few rows runs on the tensor cores
 constexpr int kHeadTensorRowsMin = 4;            // wanted rows from which the head does
 
 // assignment slots of `rows` rows when every expert group is padded to `pad` slots
@@ -186,10 +187,26 @@ bool tensor_path(const lm_b200_engine* e, int M, int N, int K) {
 
 const dia::GemmEpilogue kPlain{nullptr, nullptr, nullptr, 0.f, nullptr};
 
+// Whether a product of a few rows runs on the tensor-core kernel that streams the weights once for all rows.  Up to 8 rows the row
+// kernel, which reads them once per row, is the faster one while rows x weights are few: its weights are requested before its
+// predecessor ends, and it has no operand to prepare (a model of 4 layers at width 2048, 2 / 3 / 8 rows: 388 / 509 / 769 us on the row
+// kernel, 394 / 445 / 444 us here; at width 1024, 3 / 6 / 8 rows: 210 / 261 / 290 against 236 / 268 / 277 us).  Between 8 rows and a
+// prompt portion's bf16 products there are only the 64-row tiles beside it.  (The head stays on the row kernel: a wave and a half
+// of tiles.)
+bool few_rows(const lm_b200_engine* e, int M, int N, int K) {
+    if (M <= lm::kRowsKernelMax) return M > 2 && (long long)M * N * K >= 12LL << 20;
+    return e->m.precision == LM_B200_PRECISION_BF16 && M < kTensorRowsMin;
+}
+
 // Y = act(A W^T) in fp32 arithmetic.  More than a few rows go to the tensor cores with the operand split into three terms where the
 // shape and the room allow it (4096 x 2048 x 2048: 1.2 ms on the FMA tiles); narrow products (the router) stay on the row kernel.
 cudaError_t linear_f32(lm_b200_engine* e, const float* A, int lda, const void* W, float* Y, int ldy, int M, int N, int K, cudaStream_t st,
                        int act = lm::kActNone) {
+    const bool few = few_rows(e, M, N, K);
+    if (few && N > lm::kRowsKernelMaxOut && N <= kFewRowsOutMost && act != lm::kActXielu) {
+        const dia::FewRowsProduct p{A, lda, W, Y, ldy, M, N, K, act, 0};
+        if (dia::gemm_few_rows_ok(p)) return dia::launch_gemm_few_rows(p, M <= lm::kRowsKernelMax, st);
+    }
     if (M > lm::kRowsKernelMax && N > lm::kRowsKernelMaxOut && act != lm::kActXielu && e->a_split_bytes >= dia::gemm_f32_work_bytes(M, K)) {
         const dia::F32Product p{A, lda, 0, W, Y, ldy, 0, nullptr, 1, M, N, K, 1.f, act, nullptr, 0, 0};
         if (dia::gemm_f32_ok(p)) return dia::launch_gemm_f32(p, e->a_split, st);
@@ -602,6 +619,11 @@ int product(lm_b200_engine* e, const float* A, const void* Ab, int lda, const vo
         return LM_B200_OK;
     }
     if (M <= lm::kRowsKernelMax) {
+        const dia::FewRowsProduct p{A, lda, W, out, N, M, N, K, 0, 1};
+        if (few_rows(e, M, N, K) && N > lm::kRowsKernelMaxOut && N <= kFewRowsOutMost && dia::gemm_few_rows_ok(p)) {
+            LCK(dia::launch_gemm_few_rows(p, true, st));
+            return LM_B200_OK;
+        }
         LCK(lm::launch_linear_rows_residual(A, lda, W, out, M, N, K, lm::NormW{nullptr, nullptr, 0.f}, lm::TapOut{}, st));
         return LM_B200_OK;
     }
