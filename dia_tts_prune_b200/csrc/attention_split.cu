@@ -41,7 +41,7 @@ namespace {
 constexpr int kRows = 128, kKeys = 64, kGroupW = 128;        // query rows of a CTA, keys of a tile, channels of a stage
 constexpr int kSplitThreadsTC = 512;
 constexpr int kMaxSlots = 6, kScaleRing = 8, kMaxKStages = 4;
-constexpr int kSmemMost = 232448;
+constexpr int kSmemMost = 232448, kStaticMost = 128;       // dynamic and static; the few static words
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr float kWeightScale = 16384.f;                       // on the softmax weights (at most 1) before the split
 constexpr int kSplitOnceRows = 512;                           // rows of a kv head (M rep) from which the keys are split in advance
@@ -316,9 +316,10 @@ split_keys_kernel(const __grid_constant__ SplitAttention p, const __grid_constan
 // front of a token's first key are masked), so that a tile split in advance serves every row tile.
 struct Walk {
     const int* s_slot; const int* s_pos;
+    const uint32_t* breaks;                                   // bit i: token i does not continue token i - 1's segment
     int n, seg_a, seg_b, phase, j0, k_end, lo;
-    __device__ Walk(const int* slots, const int* pos, int n_tok)
-        : s_slot(slots), s_pos(pos), n(n_tok), seg_a(0), seg_b(0), phase(1), j0(0), k_end(0), lo(0) {}
+    __device__ Walk(const int* slots, const int* pos, const uint32_t* brk, int n_tok)
+        : s_slot(slots), s_pos(pos), breaks(brk), n(n_tok), seg_a(0), seg_b(0), phase(1), j0(0), k_end(0), lo(0) {}
     // true: tile [j0, min(j0 + 64, k_end)) of the segment's sequence
     __device__ bool next(const SplitAttention& p) {
         if (j0 < k_end) j0 += kKeys;                          // (the tile that was walked last)
@@ -335,9 +336,12 @@ struct Walk {
             if (seg_a >= n) return false;
             const int slot = s_slot[seg_a];
             const int nv = p.rows_per_slot > 0 ? p.n_valid[slot] : 0;
-            const bool split_at = p.rows_per_slot > 0 && p.mode == 1;
-            seg_b = seg_a + 1;
-            while (seg_b < n && s_slot[seg_b] == slot && s_pos[seg_b] == s_pos[seg_b - 1] + 1 && !(split_at && s_pos[seg_b] == nv)) ++seg_b;
+            seg_b = n;
+            for (int wd = (seg_a + 1) >> 5; wd < 4; ++wd) {
+                uint32_t m = breaks[wd];
+                if (wd == (seg_a + 1) >> 5) m &= 0xffffffffu << ((seg_a + 1) & 31);
+                if (m) { seg_b = min(n, wd * 32 + __ffs(m) - 1); break; }
+            }
             if (p.rows_per_slot > 0 && p.mode != 0) {
                 const bool tail = p.mode == 1 && s_pos[seg_a] >= nv;
                 phase = 1;
@@ -360,7 +364,8 @@ __global__ void __launch_bounds__(kSplitThreadsTC, 1)
 split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_constant__ Geometry geo) {
     constexpr int DVH = 64 * NVS;                             // output channels of a thread
     extern __shared__ __align__(128) unsigned char smem[];
-    __shared__ float s_red[16];
+    __shared__ float s_red[8];
+    __shared__ uint32_t s_breaks[4];
     __shared__ uint32_t s_tmem;
     __shared__ int s_rows[2];
     unsigned char* ring = smem;
@@ -372,7 +377,8 @@ split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_co
     uint64_t* p_ready = s_empty + 1;                          // weights of a tile are there / its value product is done
     uint64_t* pv_done = p_ready + 1;
     uint64_t* v_max = pv_done + 1;                            // the four fetching warps' largest values
-    uint64_t* pair = v_max + 1;                               // [4] the two warps that share rows
+    uint64_t* q_ready = v_max + 1;
+    uint64_t* pair = q_ready + 1;                               // [4] the two warps that share rows
     float* k_inv = reinterpret_cast<float*>(pair + 4);        // [kScaleRing][kMaxKStages][4] inverse scales of 16 keys
     float* v_inv = k_inv + kScaleRing * kMaxKStages * 4;      // [kScaleRing][2]
     float* vm_s = v_inv + kScaleRing * 2;                     // [2][4]
@@ -387,7 +393,7 @@ split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_co
     // later tokens see more keys: their tiles start first.  With the step's sequences at hand a tile holds rows of one of them (a
     // tile with the rows of 24 decoding sequences walked the keys of all 24 one after the other)
     int r0 = (gridDim.y - 1 - blockIdx.y) * TT, n_tok = min(TT, p.M - r0);
-    if (p.n_seq > 0) {
+    if (p.n_seq > 1) {
         if (tid == 0) s_rows[1] = 0;
         __syncthreads();
         if (warp == 0) {
@@ -423,6 +429,7 @@ split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_co
         mbar_init(p_ready, 8);
         mbar_init(pv_done, 1);
         mbar_init(v_max, 4);
+        mbar_init(q_ready, 8);
         for (int i = 0; i < 4; ++i) mbar_init(&pair[i], 2);
         fence_mbar_init();
     }
@@ -430,72 +437,23 @@ split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_co
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(&s_tmem)));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::);
     }
-    for (int i = tid; i < TT; i += kSplitThreadsTC) {
-        const int r = r0 + i;
-        const bool in = i < n_tok;
-        s_slot[i] = !in ? -1 : p.rows_per_slot > 0 ? r / p.rows_per_slot : p.row_slot[r];
-        s_pos[i] = !in ? -1 : p.rows_per_slot > 0 ? r % p.rows_per_slot : p.row_pos[r];
-    }
-
-    // ---- the query tile: largest magnitude, then both terms.  Row r of the tile is head h0 + r % PK of token r / PK ----
-    const int wk_sum = (geo.n_kst - 1) * geo.wk0 + geo.wk_last, chunks = wk_sum >> 3;
-    auto q_values = [&](int row, int ch, float (&v)[8]) {     // channels 8 ch .. of the padded row
-        const int i = row >> geo.pk_shift, h = h0 + (row & (PK - 1));
-        const int cpad = 8 * ch, st = cpad / geo.wk0, c = cpad - st * geo.wk0;
-        const int width = p.talk ? p.kdim : min(kGroupW, p.kdim - st * kGroupW);
-#pragma unroll
-        for (int e = 0; e < 8; ++e) v[e] = 0.f;
-        if (i >= n_tok || c >= width) return;
-        const float* src = p.q + (size_t)(r0 + i) * p.ldq;
-        const bool both = c + 4 < width;                      // (widths are multiples of 4)
-        if (!p.talk) {
-            src += (size_t)h * p.qdim + st * kGroupW + c;
-            const float4 a = *reinterpret_cast<const float4*>(src);
-            v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
-            if (both) {
-                const float4 b = *reinterpret_cast<const float4*>(src + 4);
-                v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
-            }
-            return;
-        }
-        for (int t = 0; t < rep; ++t) {                       // the mixed score is linear in the queries: mix those instead
-            const int gh = st * rep + t;
-            const float w = p.talk[h * p.heads + gh];
-            const float4 a = *reinterpret_cast<const float4*>(src + (size_t)gh * p.qdim + c);
-            v[0] = fmaf(w, a.x, v[0]); v[1] = fmaf(w, a.y, v[1]); v[2] = fmaf(w, a.z, v[2]); v[3] = fmaf(w, a.w, v[3]);
-            if (both) {
-                const float4 b = *reinterpret_cast<const float4*>(src + (size_t)gh * p.qdim + c + 4);
-                v[4] = fmaf(w, b.x, v[4]); v[5] = fmaf(w, b.y, v[5]); v[6] = fmaf(w, b.z, v[6]); v[7] = fmaf(w, b.w, v[7]);
+    if (tid < kRows) {
+        const int i = tid, r = r0 + i;
+        const bool in = i < n_tok, ranged = p.rows_per_slot > 0;
+        int slot = -1, pos = -1;
+        bool starts = true;
+        if (in) {
+            slot = ranged ? r / p.rows_per_slot : p.row_slot[r];
+            pos = ranged ? r % p.rows_per_slot : p.row_pos[r];
+            if (i > 0) {
+                starts = ranged ? pos == 0 : p.row_slot[r - 1] != slot || p.row_pos[r - 1] + 1 != pos;
+                if (ranged && p.mode == 1) starts = starts || pos == p.n_valid[slot];
             }
         }
-    };
-    float qm = 0.f;
-    for (int idx = tid; idx < kRows * chunks; idx += kSplitThreadsTC) {
-        const int rg = idx / (8 * chunks), rest = idx - rg * 8 * chunks, row = rg * 8 + (rest & 7), ch = rest >> 3;
-        float v[8];
-        q_values(row, ch, v);
-#pragma unroll
-        for (int e = 0; e < 8; ++e) qm = fmaxf(qm, finite_abs(v[e]));
+        if (i < TT) { s_slot[i] = slot; s_pos[i] = pos; }
+        const uint32_t m = __ballot_sync(0xffffffffu, starts);
+        if (lane == 0) s_breaks[warp] = m;
     }
-    qm = warp_max_of(qm);
-    if (lane == 0) s_red[warp] = qm;
-    __syncthreads();
-    for (int w = 0; w < 16; ++w) qm = fmaxf(qm, s_red[w]);
-    float q_inv;
-    const float q_scale = scale_of(qm, q_inv);
-    for (int idx = tid; idx < kRows * chunks; idx += kSplitThreadsTC) {
-        const int rg = idx / (8 * chunks), rest = idx - rg * 8 * chunks, row = rg * 8 + (rest & 7), ch = rest >> 3;
-        float v[8];
-        q_values(row, ch, v);
-        uint32_t hi[4], lo[4];
-#pragma unroll
-        for (int e = 0; e < 4; ++e) split2(v[2 * e] * q_scale, v[2 * e + 1] * q_scale, hi[e], lo[e]);
-        const int st = 8 * ch / geo.wk0, w = st == geo.n_kst - 1 ? geo.wk_last : geo.wk0, c8 = ch - st * (geo.wk0 >> 3);
-        unsigned char* dst = qs + (size_t)st * geo.wk0 * kRows * 4 + (size_t)((rg * (w >> 3) + c8) * 128 + (row & 7) * 16);
-        *reinterpret_cast<uint4*>(dst) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-        *reinterpret_cast<uint4*>(dst + (size_t)w * kRows * 2) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
-    }
-    fence_smem_async();
     fence_before();
     __syncthreads();
     fence_after();
@@ -505,6 +463,114 @@ split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_co
     if (warp < 8) {
         // ================= softmax: rows 32 (warp % 4) + lane, keys 32 (warp / 4) .. + 31 of a tile =================
         asm volatile("setmaxnreg.inc.sync.aligned.u32 184;");
+        // ---- the query tile: largest magnitude, then both terms.  Row r of the tile is head h0 + r % PK of token r / PK; a warp takes
+        // eight rows at a time, a lane eight channels of one.  (The first keys are on their way meanwhile: with the tile made by all
+        // warps in front of the roles, its loops unrolled, a launch of one key tile took 17 us, now 14: cold instruction fetches) ----
+        const int chunks = ((geo.n_kst - 1) * geo.wk0 + geo.wk_last) >> 3, wkb = geo.wk0 >> 3;
+        auto q_values = [&](int row, int ch, float (&v)[8]) { // channels 8 ch .. of the padded row
+            const int i = row >> geo.pk_shift, h = h0 + (row & (PK - 1)), st = geo.n_kst == 1 ? 0 : ch / wkb, c = 8 * (ch - st * wkb);
+            const int width = p.talk ? p.kdim : min(kGroupW, p.kdim - st * kGroupW);
+            const bool in = i < n_tok && ch < chunks, one = in && c < width, both = in && c + 4 < width;    // (widths are multiples of 4)
+            const float* src = p.q + (size_t)(r0 + i) * p.ldq + c;
+            const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (!p.talk) {
+                src += (size_t)h * p.qdim + st * kGroupW;
+                const float4 a = one ? *reinterpret_cast<const float4*>(src) : z, b = both ? *reinterpret_cast<const float4*>(src + 4) : z;
+                v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+                v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+                return;
+            }
+#pragma unroll
+            for (int e = 0; e < 8; ++e) v[e] = 0.f;
+            if (!one) return;
+            src += (size_t)st * rep * p.qdim;
+            const float* mix = p.talk + h * p.heads + st * rep;
+#pragma unroll 4
+            for (int t = 0; t < rep; ++t) {                   // the mixed score is linear in the queries: mix those instead
+                const float w = mix[t];
+                const float4 a = *reinterpret_cast<const float4*>(src + (size_t)t * p.qdim);
+                const float4 b = both ? *reinterpret_cast<const float4*>(src + (size_t)t * p.qdim + 4) : z;
+                v[0] = fmaf(w, a.x, v[0]); v[1] = fmaf(w, a.y, v[1]); v[2] = fmaf(w, a.z, v[2]); v[3] = fmaf(w, a.w, v[3]);
+                v[4] = fmaf(w, b.x, v[4]); v[5] = fmaf(w, b.y, v[5]); v[6] = fmaf(w, b.z, v[6]); v[7] = fmaf(w, b.w, v[7]);
+            }
+        };
+        float q_inv, q_scale;
+        bool q_finite;
+        auto q_scaled = [&](float m) {                        // the tile's scale from all warps' largest magnitudes
+            m = warp_max_of(m);
+            if (lane == 0) s_red[warp] = m;
+            asm volatile("bar.sync 1, 256;" ::: "memory");
+#pragma unroll
+            for (int w = 0; w < 8; ++w) m = fmaxf(m, s_red[w]);
+            q_finite = m <= 3.402823466e38f;
+            q_scale = scale_of(m, q_inv);
+        };
+        auto q_store = [&](int row, int ch, const float (&v)[8]) {
+            if (ch >= chunks) return;
+            uint32_t hi[4], lo[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) split2(v[2 * e] * q_scale, v[2 * e + 1] * q_scale, hi[e], lo[e]);
+            const int st = geo.n_kst == 1 ? 0 : ch / wkb, w = st == geo.n_kst - 1 ? geo.wk_last : geo.wk0, c8 = ch - st * wkb;
+            unsigned char* dst = qs + (size_t)st * geo.wk0 * kRows * 4 + (size_t)(((row >> 3) * (w >> 3) + c8) * 128 + (row & 7) * 16);
+            *reinterpret_cast<uint4*>(dst) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+            *reinterpret_cast<uint4*>(dst + (size_t)w * kRows * 2) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+        };
+        float qm = 0.f;
+        const int qrow = warp * 8 + (lane & 7), qch = lane >> 3;
+        bool made = false;
+        if (!p.talk && geo.n_kst == 1) {                      // all of it fits the registers
+            float4 v[8][2];
+#pragma unroll
+            for (int rg = 0; rg < 2; ++rg) {
+                const int row = qrow + 64 * rg, i = row >> geo.pk_shift;
+                const float* src = p.q + (size_t)(r0 + i) * p.ldq + (size_t)(h0 + (row & (PK - 1))) * p.qdim + 8 * qch;
+                const int left = i < n_tok ? p.kdim - 8 * qch : 0;
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        v[rg * 4 + k][e] = make_float4(0.f, 0.f, 0.f, 0.f);
+                        if (32 * k + 4 * e < left) v[rg * 4 + k][e] = *reinterpret_cast<const float4*>(src + 32 * k + 4 * e);
+                    }
+            }
+#pragma unroll
+            for (int i = 0; i < 8; ++i) qm = max_abs4(max_abs4(qm, v[i][0]), v[i][1]);
+            q_scaled(qm);
+            if (q_finite) {                                   // (the same for all warps)
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const float x[8] = {v[i][0].x, v[i][0].y, v[i][0].z, v[i][0].w, v[i][1].x, v[i][1].y, v[i][1].z, v[i][1].w};
+                    q_store(qrow + 64 * (i >> 2), qch + 4 * (i & 3), x);
+                }
+                made = true;
+            } else {
+                asm volatile("bar.sync 1, 256;" ::: "memory");    // (all have read the first maxima)
+                qm = 0.f;
+            }
+        }
+        if (!made) {
+            for (int pass = 0; pass < 2; ++pass) {
+                for (int rg = 0; rg < 2; ++rg)
+                    for (int ch = qch; ch < chunks; ch += 16) {
+                        float v[4][8];
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) q_values(qrow + 64 * rg, ch + 4 * i, v[i]);
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            if (pass == 0) {
+#pragma unroll
+                                for (int e = 0; e < 8; ++e) qm = fmaxf(qm, finite_abs(v[i][e]));
+                            } else {
+                                q_store(qrow + 64 * rg, ch + 4 * i, v[i]);
+                            }
+                        }
+                    }
+                if (pass == 0) q_scaled(qm);
+            }
+        }
+        fence_smem_async();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(q_ready);
         const int qt = warp & 3, hf = warp >> 2, row = qt * 32 + lane, tok = row >> geo.pk_shift, h = h0 + (row & (PK - 1));
         const uint32_t lanes = (uint32_t)(qt * 32) << 16;
         const int my_pos = s_pos[tok];
@@ -545,7 +611,7 @@ split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_co
             }
         };
         unsigned t = 0;
-        Walk w(s_slot, s_pos, n_tok);
+        Walk w(s_slot, s_pos, s_breaks, n_tok);
         for (; w.next(p); ++t) {
             if (!wait_for(s_full, t & 1u)) { ok = false; break; }
             fence_after();
@@ -665,31 +731,43 @@ split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_co
         ok = ok && wait_for(&pair[qt], t & 1u);
         float l = l_run + xl[(hf ^ 1) * kRows + row];
         if (p.sink) l += ex2(fmaf(p.sink[h], kLog2e, -c_run));
-        if (tok < n_tok) {
-            float f = l > 0.f ? p.out_scale / l : 0.f;
-            if (!ok) f = CUDART_NAN_F;
-            const int r = r0 + tok;
-            if (p.head_gate) f *= p.head_gate[(size_t)r * p.ldg + h];
-            const int c0 = NVS == 1 ? hf * half : hf * 128;
-            const size_t at = (size_t)r * p.ldo + (size_t)h * p.vdim + c0;
-            const float* gate = p.gate ? p.gate + (size_t)r * p.ldg + (size_t)h * p.vdim + c0 : nullptr;
+        // through shared memory (the ring and the queries are read; 32 rows of this warp's channels): whole lines reach the output, and
+        // one rolled loop serves every kind of output.  (Stored from the registers, row by row, 5500 cycles of a CTA, mostly fetching
+        // the unrolled code; 3500 now)
+        float f = tok < n_tok && l > 0.f ? p.out_scale / l : 0.f;
+        if (p.head_gate && tok < n_tok) f *= p.head_gate[(size_t)(r0 + tok) * p.ldg + h];
+        if (t == 0 && ok) asm volatile("bar.sync 1, 256;" ::: "memory");    // (no keys: all warps' queries are stored first)
+        ok = __all_sync(0xffffffffu, ok);
+        const int c0 = NVS == 1 ? hf * half : hf * 128, ldst = half + 4;
+        float* stage = reinterpret_cast<float*>(smem) + (size_t)warp * 32 * ldst;
 #pragma unroll
-            for (int c = 0; c < DVH; c += 4) {                // (vdim is a multiple of 4)
-                if (c < n_mine && c0 + c < p.vdim) {
-                    float4 o = make_float4(O[c] * f, O[c + 1] * f, O[c + 2] * f, O[c + 3] * f);
-                    if (gate) {
-                        const float4 z = *reinterpret_cast<const float4*>(gate + c);
-                        o.x *= 1.0f / (1.0f + expf(-z.x)); o.y *= 1.0f / (1.0f + expf(-z.y));
-                        o.z *= 1.0f / (1.0f + expf(-z.z)); o.w *= 1.0f / (1.0f + expf(-z.w));
-                    }
-                    if (p.out) *reinterpret_cast<float4*>(p.out + at + c) = o;
-                    if (p.out_bf16) {
-                        const __nv_bfloat162 a = __floats2bfloat162_rn(o.x, o.y), b = __floats2bfloat162_rn(o.z, o.w);
-                        *reinterpret_cast<uint2*>(reinterpret_cast<__nv_bfloat16*>(p.out_bf16) + at + c) =
-                            make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
-                    }
+        for (int c = 0; c < DVH; c += 4)
+            if (c < n_mine) *reinterpret_cast<float4*>(stage + lane * ldst + c) = make_float4(O[c] * f, O[c + 1] * f, O[c + 2] * f, O[c + 3] * f);
+        __syncwarp();
+        const int w4 = min(n_mine, p.vdim - c0) >> 2;         // (vdim is a multiple of 4)
+        int sr = 0, sc = lane;                                // row and group of 4 channels of this lane's turn
+        while (w4 > 0 && sc >= w4) { sc -= w4; ++sr; }
+#pragma unroll 2
+        for (int it = 0; it < w4; ++it) {
+            const int rw = qt * 32 + sr, tk = rw >> geo.pk_shift, c = 4 * sc;
+            if (tk < n_tok) {
+                const size_t head = (size_t)(h0 + (rw & (PK - 1))) * p.vdim + c0 + c, at = (size_t)(r0 + tk) * p.ldo + head;
+                float4 o = *reinterpret_cast<const float4*>(stage + sr * ldst + c);
+                if (!ok) o = make_float4(CUDART_NAN_F, CUDART_NAN_F, CUDART_NAN_F, CUDART_NAN_F);
+                if (p.gate) {
+                    const float4 z = *reinterpret_cast<const float4*>(p.gate + (size_t)(r0 + tk) * p.ldg + head);
+                    o.x *= 1.0f / (1.0f + expf(-z.x)); o.y *= 1.0f / (1.0f + expf(-z.y));
+                    o.z *= 1.0f / (1.0f + expf(-z.z)); o.w *= 1.0f / (1.0f + expf(-z.w));
+                }
+                if (p.out) *reinterpret_cast<float4*>(p.out + at) = o;
+                if (p.out_bf16) {
+                    const __nv_bfloat162 a = __floats2bfloat162_rn(o.x, o.y), b = __floats2bfloat162_rn(o.z, o.w);
+                    *reinterpret_cast<uint2*>(reinterpret_cast<__nv_bfloat16*>(p.out_bf16) + at) =
+                        make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
                 }
             }
+            sc += 32;
+            while (sc >= w4) { sc -= w4; ++sr; }
         }
     } else if (warp < 12) {
         // ================= keys and values: warp lw takes keys 16 lw .. + 15 of a tile, a lane one key of either eight =================
@@ -801,7 +879,7 @@ split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_co
         };
         int tile = -1, prev_tile = -1;
         unsigned t = 0;
-        Walk w(s_slot, s_pos, n_tok);
+        Walk w(s_slot, s_pos, s_breaks, n_tok);
         for (; ok && w.next(p); ++t) {
             const int slot = s_slot[w.seg_a];
             prev_tile = tile;
@@ -863,7 +941,8 @@ split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_co
                 }
             };
             unsigned t = 0;
-            Walk w(s_slot, s_pos, n_tok);
+            Walk w(s_slot, s_pos, s_breaks, n_tok);
+            ok = wait_warp(q_ready, 0);
             for (; ok && w.next(p); ++t) {
                 if (t > 0 && !wait_warp(s_empty, (t - 1) & 1u)) { ok = false; break; }
                 for (int st = 0; st < geo.n_kst; ++st) {
@@ -945,26 +1024,23 @@ bool geometry_of(const SplitAttention& a, Geometry& g, size_t& smem) {
     g.o_bufs = g.n_vst == 1 && 64 * g.n_kst + 64 + 256 <= 512 ? 2 : 1;
     g.slot_bytes = kKeys * std::max(g.wk0, std::max(g.wv0, g.v0_layout)) * 4;
     g.q_bytes = ((g.n_kst - 1) * g.wk0 + g.wk_last) * kRows * 4;
-    const int control = (2 * kMaxSlots + 5 + 4) * 8 + (kScaleRing * kMaxKStages * 4 + kScaleRing * 2 + 8 + 4 * kRows) * 4 + 2 * (kRows >> g.pk_shift) * 4;
-    g.n_slots = (kSmemMost - 128 - g.q_bytes - control) / g.slot_bytes;      // (128: the few static words)
+    const int control = (2 * kMaxSlots + 6 + 4) * 8 + (kScaleRing * kMaxKStages * 4 + kScaleRing * 2 + 8 + 4 * kRows) * 4 + 2 * (kRows >> g.pk_shift) * 4;
+    g.n_slots = (kSmemMost - kStaticMost - g.q_bytes - control) / g.slot_bytes;
     if (g.n_slots < 2) return false;
     g.n_slots = std::min(g.n_slots, kMaxSlots);
+    // the output is staged in the ring and the queries: 8 warps of 32 rows, 4 floats between the rows
+    const int staged = kRows * 2 * (g.n_vst == 1 ? g.wv0 / 2 + 4 : 128 + 4) * 4;
+    g.q_bytes = std::max(g.q_bytes, staged - g.n_slots * g.slot_bytes);
     smem = (size_t)g.n_slots * g.slot_bytes + g.q_bytes + control;
-    return true;
+    return smem <= (size_t)(kSmemMost - kStaticMost);
 }
 
 template <int NVS>
 cudaError_t launch_inst(const SplitAttention& a, const Geometry& g, size_t smem, cudaStream_t st) {
-    static size_t allowed[64] = {};
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
+    // (the same size for every launch: another thread's cannot lower what this one needs)
+    const cudaError_t e = cudaFuncSetAttribute(split_attention_kernel<NVS>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMost - kStaticMost);
     if (e != cudaSuccess) return e;
-    if (dev < 0 || dev >= 64 || allowed[dev] < smem) {
-        e = cudaFuncSetAttribute(split_attention_kernel<NVS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-        if (dev >= 0 && dev < 64) allowed[dev] = smem;
-    }
-    const int tt = kRows >> g.pk_shift, tiles = a.n_seq > 0 ? a.M / tt + a.n_seq : (a.M + tt - 1) / tt;
+    const int tt = kRows >> g.pk_shift, tiles = a.n_seq > 1 ? a.M / tt + a.n_seq : (a.M + tt - 1) / tt;
     if (tiles > 65535) return cudaErrorNotSupported;
     if (a.work) split_keys_kernel<<<dim3(g.cap_tiles, g.parts), 256, 0, st>>>(a, g);
     split_attention_kernel<NVS><<<dim3(a.heads >> g.pk_shift, tiles), kSplitThreadsTC, smem, st>>>(a, g);
