@@ -105,8 +105,11 @@ __global__ void split3_rows_kernel(const float* __restrict__ x, __nv_bfloat16* _
 
 // the same with torch.nn.RMSNorm of the row fused in front (dia/layers.py:541,560,579,714: the norm that precedes
 // every projection): xs = split3((x * rsqrt(mean(x^2) + eps)) * w).  One CTA per row.
+// SPLIT: the normed rows' three terms; otherwise the normed rows themselves
+template <bool SPLIT>
 __global__ void __launch_bounds__(256) split3_norm_rows_kernel(const float* __restrict__ x, const float* __restrict__ w, float eps,
-                                                               __nv_bfloat16* __restrict__ xs, int M, int K) {
+                                                               void* __restrict__ out, int M, int K) {
+    __nv_bfloat16* xs = reinterpret_cast<__nv_bfloat16*>(out);
     __shared__ float part[8];
     const int row = blockIdx.x;
     const float* xr = x + (size_t)row * K;
@@ -122,6 +125,10 @@ __global__ void __launch_bounds__(256) split3_norm_rows_kernel(const float* __re
     const size_t n = (size_t)M * K;
     for (int i = threadIdx.x; i < K; i += 256) {
         const float v = (xr[i] * inv) * w[i];
+        if (!SPLIT) {
+            reinterpret_cast<float*>(out)[(size_t)row * K + i] = v;
+            continue;
+        }
         const __nv_bfloat16 h = __float2bfloat16_rn(v);
         const float r1 = v - __bfloat162float(h);
         const __nv_bfloat16 l = __float2bfloat16_rn(r1);
@@ -335,12 +342,31 @@ dia_gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
     }
 }
 
+__device__ __forceinline__ float load_remote(const float* local, uint32_t rank) {
+    uint32_t a;
+    float v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(local)), "r"(rank));
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
+    return v;
+}
+__device__ __forceinline__ float4 load_remote4(const float* local, uint32_t rank) {
+    uint32_t a;
+    float4 v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(local)), "r"(rank));
+    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a) : "memory");
+    return v;
+}
+__device__ __forceinline__ void cluster_sync_all() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
 // ---------------------------------------------------------------------------------------------------------------------
 // Y = A W^T in the accuracy of fp32 FMA arithmetic, for callers that asked for it.  The accumulator of a tensor-core product loses
 // up to a unit in the last place at every step, towards zero (K = 2048: 2.1e-6 against 3.9e-7 of an FMA chain), so an accumulator
 // lives for one k-block only - the two small terms first, then the large one - and the epilogue warps add it to the tile's sums
 // in their registers while the next k-blocks are multiplied into the three other accumulators.  128 x 128 tiles: a thread holds
-// 128 sums.  Bound: 12 MMAs of 64 cycles per k-block against ~300 issue slots of draining it.
+// 128 sums.  Bound: 12 MMAs of 64 cycles per k-block against ~300 issue slots of draining it.  Where the tiles leave most of the chip
+// idle, a cluster of gridDim.y CTAs shares a tile: each takes a range of k-blocks, and the sums meet in shared memory.
 constexpr int kFN = 128, kFASlots = 6, kFBSlots = 3, kFStride = kFN + 4;
 constexpr int kFStage = 4 * 32 * kFStride * 4;                // 32 rows of sums per epilogue warp
 constexpr int kFBars = 2 * kFASlots + 2 * kFBSlots + 8;
@@ -369,8 +395,54 @@ dia_gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     float* stage = reinterpret_cast<float*>(reinterpret_cast<unsigned char*>(a_full) + 256);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int n_kb = (K + BK - 1) / BK;
+    const int S = gridDim.y, kb_all = (K + BK - 1) / BK, kb_per = (kb_all + S - 1) / S, kb0 = blockIdx.y * kb_per;
+    const int n_kb = max(0, min(kb_per, kb_all - kb0));
     const int tiles_m = (M + BM - 1) / BM, tiles_n = (N + kFN - 1) / kFN, n_tiles = tiles_m * tiles_n * p.heads;
+    // an epilogue warp's 32 rows of sums, from row r0 on every S-th, four columns per lane
+    float* const tile = stage + (warp - 2) * 32 * kFStride;
+    auto emit = [&](int t, int r0) {
+        const int q = warp & 3, hn = t / tiles_m, h = hn / tiles_n, n0 = (hn - h * tiles_n) * kFN, m0 = (t % tiles_m) * BM;
+        const int rows = min(32, M - (m0 + q * 32)), n = n0 + 4 * lane;
+                    if (n < N) {
+                        const size_t m = (size_t)(m0 + q * 32), col = (size_t)h * p.y_hs + n;
+                        const float* gate = p.gate ? p.gate + m * p.ldg + (p.head_gate ? (size_t)h : (size_t)h * N + n) : nullptr;
+        #pragma unroll 1
+                        for (int r = r0; r < rows; r += S) {
+                            float4 v = *reinterpret_cast<const float4*>(tile + r * kFStride + 4 * lane);
+                if (S > 1) {
+                    float4 u[8];
+#pragma unroll
+                    for (int c = 0; c < 8; ++c) if (c < S) u[c] = load_remote4(tile + r * kFStride + 4 * lane, c);
+                    v = u[0];
+#pragma unroll
+                    for (int c = 1; c < 8; ++c) if (c < S) { v.x += u[c].x; v.y += u[c].y; v.z += u[c].z; v.w += u[c].w; }
+                }
+                            v.x *= p.alpha; v.y *= p.alpha; v.z *= p.alpha; v.w *= p.alpha;
+                            if (p.act) { v.x = f32_act(p.act, v.x); v.y = f32_act(p.act, v.y); v.z = f32_act(p.act, v.z); v.w = f32_act(p.act, v.w); }
+                            if (gate) {
+                                const float* z = gate + (size_t)r * p.ldg;
+                                if (p.head_gate) {
+                                    const float f = 1.0f / (1.0f + expf(-z[0]));
+                                    v.x *= f; v.y *= f; v.z *= f; v.w *= f;
+                                } else {
+                                    v.x *= 1.0f / (1.0f + expf(-z[0])); v.y *= 1.0f / (1.0f + expf(-z[1]));
+                                    v.z *= 1.0f / (1.0f + expf(-z[2])); v.w *= 1.0f / (1.0f + expf(-z[3]));
+                                }
+                            }
+                            const size_t at = (m + r) * p.ldy + col;
+                            if (p.add) {
+                    const float4 o = *reinterpret_cast<const float4*>(p.add + at);
+                    v.x += o.x; v.y += o.y; v.z += o.z; v.w += o.w;
+                }
+                *reinterpret_cast<float4*>(p.y + at) = v;
+                            if (p.y_bf16) {
+                                const __nv_bfloat162 lo = __floats2bfloat162_rn(v.x, v.y), hi = __floats2bfloat162_rn(v.z, v.w);
+                                *reinterpret_cast<uint2*>(reinterpret_cast<__nv_bfloat16*>(p.y_bf16) + at) =
+                                    make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+                            }
+                        }
+                    }
+    };
     // tile t: row block t % tiles_m of column block (t / tiles_m) % tiles_n of head t / (tiles_m tiles_n)
     if (threadIdx.x == 0) {
         for (int i = 0; i < kFASlots; ++i) { mbar_init(&a_full[i], 1); mbar_init(&a_empty[i], 1); }
@@ -396,13 +468,13 @@ dia_gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                     const unsigned s = ib % kFBSlots;
                     mbar_wait_bounded(&b_empty[s], ((ib / kFBSlots) & 1u) ^ 1u);
                     mbar_arrive_expect_tx(&b_full[s], kTileBytes);
-                    tma_load_2d(smem_u32(b_ring + s * kTileBytes), &map_b, smem_u32(&b_full[s]), kb * BK, h * N + n0);
+                    tma_load_2d(smem_u32(b_ring + s * kTileBytes), &map_b, smem_u32(&b_full[s]), (kb0 + kb) * BK, h * N + n0);
                     ++ib;
                     for (int tm = kTerms - 1; tm >= 0; --tm) {          // the smallest term first
                         const unsigned sa = ia % kFASlots;
                         mbar_wait_bounded(&a_empty[sa], ((ia / kFASlots) & 1u) ^ 1u);
                         mbar_arrive_expect_tx(&a_full[sa], kTileBytes);
-                        tma_load_2d(smem_u32(a_ring + sa * kTileBytes), &map_a, smem_u32(&a_full[sa]), kb * BK, (tm * p.heads + h) * M + m0);
+                        tma_load_2d(smem_u32(a_ring + sa * kTileBytes), &map_a, smem_u32(&a_full[sa]), (kb0 + kb) * BK, (tm * p.heads + h) * M + m0);
                         ++ia;
                     }
                 }
@@ -442,7 +514,6 @@ dia_gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         const int q = warp & 3;
         unsigned it = 0;
         for (int t = blockIdx.x; t < n_tiles; t += gridDim.x) {
-            const int hn = t / tiles_m, h = hn / tiles_n, n0 = (hn - h * tiles_n) * kFN, m0 = (t % tiles_m) * BM;
             float sum[kFN];
 #pragma unroll
             for (int c = 0; c < kFN; ++c) sum[c] = 0.f;
@@ -474,40 +545,12 @@ dia_gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             }
             // The sums go out through shared memory, a row per step and four columns per lane: coalesced, and a short loop where the
             // unrolled one (128 copies of the epilogue) was bound by instruction fetches.
-            float* tile = stage + (warp - 2) * 32 * kFStride;
-            const int rows = min(32, M - (m0 + q * 32)), n = n0 + 4 * lane;
             __syncwarp();
 #pragma unroll
             for (int c = 0; c < kFN; c += 4)
                 *reinterpret_cast<float4*>(tile + lane * kFStride + c) = make_float4(sum[c], sum[c + 1], sum[c + 2], sum[c + 3]);
             __syncwarp();
-            if (n < N) {
-                const size_t m = (size_t)(m0 + q * 32), col = (size_t)h * p.y_hs + n;
-                const float* gate = p.gate ? p.gate + m * p.ldg + (p.head_gate ? (size_t)h : (size_t)h * N + n) : nullptr;
-#pragma unroll 1
-                for (int r = 0; r < rows; ++r) {
-                    float4 v = *reinterpret_cast<const float4*>(tile + r * kFStride + 4 * lane);
-                    v.x *= p.alpha; v.y *= p.alpha; v.z *= p.alpha; v.w *= p.alpha;
-                    if (p.act) { v.x = f32_act(p.act, v.x); v.y = f32_act(p.act, v.y); v.z = f32_act(p.act, v.z); v.w = f32_act(p.act, v.w); }
-                    if (gate) {
-                        const float* z = gate + (size_t)r * p.ldg;
-                        if (p.head_gate) {
-                            const float f = 1.0f / (1.0f + expf(-z[0]));
-                            v.x *= f; v.y *= f; v.z *= f; v.w *= f;
-                        } else {
-                            v.x *= 1.0f / (1.0f + expf(-z[0])); v.y *= 1.0f / (1.0f + expf(-z[1]));
-                            v.z *= 1.0f / (1.0f + expf(-z[2])); v.w *= 1.0f / (1.0f + expf(-z[3]));
-                        }
-                    }
-                    const size_t at = (m + r) * p.ldy + col;
-                    *reinterpret_cast<float4*>(p.y + at) = v;
-                    if (p.y_bf16) {
-                        const __nv_bfloat162 lo = __floats2bfloat162_rn(v.x, v.y), hi = __floats2bfloat162_rn(v.z, v.w);
-                        *reinterpret_cast<uint2*>(reinterpret_cast<__nv_bfloat16*>(p.y_bf16) + at) =
-                            make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
-                    }
-                }
-            }
+            if (S == 1) emit(t, 0);
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -515,6 +558,11 @@ dia_gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     if (warp == 1) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(4 * kFN));
+    }
+    if (S > 1) {
+        cluster_sync_all();
+        if (warp >= 2) emit(blockIdx.x, blockIdx.y);
+        cluster_sync_all();                                   // (the sums stay until every CTA has read them)
     }
 }
 
@@ -529,27 +577,11 @@ dia_gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
 // Bound: the weights' bytes.  The row kernel reads them once per row from L2 instead: 8 rows x 2048 x 6144 took 35 us.
 constexpr int kRThreads = 192, kRSlotsMost = 8, kRSmemMost = 226 * 1024;
 
-__device__ __forceinline__ uint32_t cluster_rank() {
-    uint32_t r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
-__device__ __forceinline__ float load_remote(const float* local, uint32_t rank) {
-    uint32_t a;
-    float v;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(local)), "r"(rank));
-    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
-    return v;
-}
-__device__ __forceinline__ void cluster_sync_all() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-
 // NB: columns of the rows' operand (32 for up to 8 rows, 96 for up to 32)
 template <int NB>
 __global__ void __launch_bounds__(kRThreads, 1)
 dia_gemm_few_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ FewRowsProduct p, int kb_per, int n_slots) {
-    constexpr int Mp = NB / 3 / 8 * 8, kBufs = 512 / NB > 8 ? 8 : 512 / NB, kCols = kBufs * NB > 256 ? 512 : 256;
+    constexpr int Mp = NB / 3 / 8 * 8, kBufs = NB == 32 ? 8 : 2, kCols = 256;      // (two CTAs per SM)
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     __shared__ uint64_t w_full[kRSlotsMost], w_empty[kRSlotsMost], t_full[8], t_empty[8];
@@ -558,7 +590,8 @@ dia_gemm_few_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid
     unsigned char* rows = ring + n_slots * kTileBytes;                         // [kb_per][NB x 64] bf16
     float* part = reinterpret_cast<float*>(rows + (size_t)kb_per * NB * 128);  // [Mp][128]
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int S = gridDim.y, n_kb = (p.K + BK - 1) / BK, rank = blockIdx.y, n0 = blockIdx.x * BM;
+    const int S = gridDim.y, n_kb = (p.K + BK - 1) / BK, rank = blockIdx.y, n0 = blockIdx.x * BM, m0 = blockIdx.z * kGemmFewRowsGroup;
+    const int M = min(p.M - m0, kGemmFewRowsGroup);
     const int kb0 = rank * kb_per, kbs = max(0, min(kb_per, n_kb - kb0));
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     if (tid == 0) {
@@ -581,8 +614,8 @@ dia_gemm_few_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid
         float v[8];
 #pragma unroll
         for (int e = 0; e < 8; ++e) v[e] = 0.f;
-        if (m < p.M && k < p.K) {                             // (K a multiple of 8)
-            const float4* src = reinterpret_cast<const float4*>(p.a + (size_t)m * p.lda + k);
+        if (m < M && k < p.K) {                               // (K a multiple of 8)
+            const float4* src = reinterpret_cast<const float4*>(p.a + (size_t)(m0 + m) * p.lda + k);
             const float4 x = src[0], y = src[1];
             v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w; v[4] = y.x; v[5] = y.y; v[6] = y.z; v[7] = y.w;
         }
@@ -643,19 +676,18 @@ dia_gemm_few_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid
             const int acc = kb % kBufs;
             mbar_wait_bounded(&t_full[acc], (kb / kBufs) & 1u);
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            uint32_t v[NB];
 #pragma unroll
-            for (int cb = 0; cb < NB / 16; ++cb) {
-                uint32_t v[16];
+            for (int c = 0; c < NB; c += 16)
                 asm volatile(
                     "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-                    : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]),
-                      "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-                    : "r"(tmem + ((uint32_t)(q * 32) << 16) + acc * NB + cb * 16)
+                    : "=r"(v[c]), "=r"(v[c + 1]), "=r"(v[c + 2]), "=r"(v[c + 3]), "=r"(v[c + 4]), "=r"(v[c + 5]), "=r"(v[c + 6]), "=r"(v[c + 7]),
+                      "=r"(v[c + 8]), "=r"(v[c + 9]), "=r"(v[c + 10]), "=r"(v[c + 11]), "=r"(v[c + 12]), "=r"(v[c + 13]), "=r"(v[c + 14]), "=r"(v[c + 15])
+                    : "r"(tmem + ((uint32_t)(q * 32) << 16) + acc * NB + c)
                     : "memory");
-                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-                for (int i = 0; i < 16; ++i) sum[cb * 16 + i] += __uint_as_float(v[i]);
-            }
+            for (int c = 0; c < NB; ++c) sum[c] += __uint_as_float(v[c]);
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
             if (lane == 0) mbar_arrive(&t_empty[acc]);
@@ -671,7 +703,7 @@ dia_gemm_few_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid
     }
     if (S > 1) cluster_sync_all();
     // ---- the outputs of the tile, dealt to the cluster's CTAs ----
-    for (int i = rank * kRThreads + tid; i < p.M * BM; i += S * kRThreads) {
+    for (int i = rank * kRThreads + tid; i < M * BM; i += S * kRThreads) {
         const int m = i / BM, c = i - m * BM, n = n0 + c;
         if (n >= p.N) continue;
         float v;
@@ -687,8 +719,8 @@ dia_gemm_few_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid
             v = part[i];
         }
         if (p.act) v = f32_act(p.act, v);
-        float* dst = p.y + (size_t)m * p.ldy + n;
-        *dst = p.add ? *dst + v : v;
+        const size_t at = (size_t)(m0 + m) * p.ldy + n;
+        p.y[at] = p.add ? p.add[at] + v : v;
     }
     if (S > 1) cluster_sync_all();                            // (the partial sums stay until every CTA has read them)
 }
@@ -789,56 +821,97 @@ bool gemm_f32_ok(const F32Product& p) {
            (reinterpret_cast<uintptr_t>(p.y_bf16) & 7) == 0 && (reinterpret_cast<uintptr_t>(p.w) & 15) == 0;
 }
 
-cudaError_t launch_gemm_f32(const F32Product& p, void* work, cudaStream_t st) {
-    if (!gemm_f32_ok(p)) return cudaErrorNotSupported;
+// Which kernel takes a product of M fp32 rows.  Up to 32 rows the few-rows kernel (N = 2048, K = 1024, 32 rows: 25 us on the 128 x 256
+// tiles, 11 here; N = K = 2048: 42 and 22).
+static bool dense_rows_few(int M) { return M <= kGemmFewRowsGroup; }
+// CTAs that share a 128 x 128 tile of the fp32-sum kernel: as many as the chip has room for, two k-blocks each at least
+static int f32_splits(int tiles, int n_kb, int most, int sms) {
+    int s = 1;
+    while (2 * s <= most && tiles * 2 * s <= sms && n_kb >= 4 * s) s *= 2;
+    return s;
+}
+// Beyond 32 rows the fp32-sum kernel where its rounds of tiles are the shorter ones: a k-block of a round of its 128 x 128 tiles takes
+// three quarters of one of 128 x 256 tiles (1.1 and 1.4 us; both are bound by the operands' way from L2), its tiles are twice as many, and
+// where they leave the chip idle its clusters split K (us, 128 x 256 tiles / here: 200 rows N = 2048, K = 1024 27 / 14, N = 1024, K = 4096
+// 77 / 31, N = 8192, K = 1024 29 / 26, N = 16384, K = 2048 51 / 73; 1024 rows N = 2048, K = 1024 30 / 27; 1722 rows 33 / 45)
+static bool dense_rows_f32(int M, int N, int K, int sms) {
+    const int tm = (M + BM - 1) / BM, n_kb = (K + BK - 1) / BK;
+    const long long narrow = (long long)tm * ((N + kFN - 1) / kFN), wide = (long long)tm * ((N + BN - 1) / BN);
+    const int s = narrow < sms ? f32_splits((int)narrow, n_kb, 8, sms) : 1;
+    return ((narrow * s + sms - 1) / sms) * ((n_kb + s - 1) / s) * 3 < ((wide + sms - 1) / sms) * n_kb * 4;
+}
+
+
+// splits: the most CTAs that may share a tile (1: a sum's order does not depend on the rows beside it)
+static cudaError_t run_gemm_f32(const F32Product& p, const void* terms, int splits, cudaStream_t st) {
     int dev = 0, sms = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(dia_gemm_f32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kFSmem);
     if (e != cudaSuccess) return e;
     CUtensorMap ma, mb;
-    if (!make_map(&ma, work, (long long)kTerms * p.heads * p.M, p.K, BM) || !make_map(&mb, p.w, (long long)p.heads * p.N, p.K, kFN))
+    if (!make_map(&ma, terms, (long long)kTerms * p.heads * p.M, p.K, BM) || !make_map(&mb, p.w, (long long)p.heads * p.N, p.K, kFN))
         return cudaErrorNotSupported;
-    split3_heads_kernel<<<p.M, 256, 0, st>>>(p.a, p.lda, p.a_hs, reinterpret_cast<__nv_bfloat16*>(work), p.heads, p.M, p.K);
-    const int n_tiles = p.heads * ((p.N + kFN - 1) / kFN) * ((p.M + BM - 1) / BM);
-    dia_gemm_f32_kernel<<<std::min(n_tiles, sms), kGemmThreads, kFSmem, st>>>(ma, mb, p);
-    return cudaGetLastError();
+    const int n_tiles = p.heads * ((p.N + kFN - 1) / kFN) * ((p.M + BM - 1) / BM), n_kb = (p.K + BK - 1) / BK;
+    const int s = f32_splits(n_tiles, n_kb, splits, sms);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(s > 1 ? n_tiles : std::min(n_tiles, sms), s);
+    cfg.blockDim = dim3(kGemmThreads);
+    cfg.dynamicSmemBytes = kFSmem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = 1;
+    attr.val.clusterDim.y = s;
+    attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, dia_gemm_f32_kernel, ma, mb, p);
 }
 
-// CTAs of a cluster: enough of them to fill the chip, at least two k-blocks each (a rule on N and K alone, so that a row's sums do
-// not depend on what shares its step)
-static int few_rows_split(int N, int K) {
-    const int tiles = (N + BM - 1) / BM, n_kb = (K + BK - 1) / BK;
-    int s = 1;
-    while (s < 8 && tiles * s < 120 && n_kb >= 4 * s) s *= 2;
-    return s;
+cudaError_t launch_gemm_f32(const F32Product& p, void* work, cudaStream_t st) {
+    if (!gemm_f32_ok(p)) return cudaErrorNotSupported;
+    split3_heads_kernel<<<p.M, 256, 0, st>>>(p.a, p.lda, p.a_hs, reinterpret_cast<__nv_bfloat16*>(work), p.heads, p.M, p.K);
+    return run_gemm_f32(p, work, 1, st);
 }
+
 static size_t few_rows_smem(int NB, int kb_per, int n_slots) {
     return 1024 + (size_t)n_slots * kTileBytes + (size_t)kb_per * NB * 128 + (size_t)(NB / 3 / 8 * 8) * BM * 4;
 }
+// CTAs of a cluster: enough of them to fill the chip, at least two k-blocks each (for one group of rows a rule on N and K alone, so
+// that a row's sums do not depend on what shares its step); several groups also split until two CTAs fit an SM
+static int few_rows_split(int NB, int N, int K, int groups) {
+    const int tiles = (N + BM - 1) / BM, n_kb = (K + BK - 1) / BK;
+    int s = 1;
+    while (s < 8 && n_kb >= 4 * s && (tiles * groups * s < 120 || (groups > 1 && few_rows_smem(NB, (n_kb + s - 1) / s, 2) > kRSmemMost / 2))) s *= 2;
+    return s;
+}
 
 bool gemm_few_rows_ok(const FewRowsProduct& p) {
-    if (p.M <= 0 || p.M > kGemmFewRowsMost || p.N <= 0 || p.K < BK || p.K % 8 || p.lda % 4 || (reinterpret_cast<uintptr_t>(p.a) & 15) ||
+    const int groups = (p.M + kGemmFewRowsGroup - 1) / kGemmFewRowsGroup, NB = p.M <= 8 ? 32 : 96;
+    if (p.M <= 0 || groups > 65535 || p.N <= 0 || p.K < BK || p.K % 8 || p.lda % 4 || (reinterpret_cast<uintptr_t>(p.a) & 15) ||
         (reinterpret_cast<uintptr_t>(p.w) & 15))
         return false;
-    const int n_kb = (p.K + BK - 1) / BK, s = few_rows_split(p.N, p.K), kb_per = (n_kb + s - 1) / s;
-    return few_rows_smem(p.M <= 8 ? 32 : 96, kb_per, std::min(kb_per, 2)) <= kRSmemMost;
+    const int n_kb = (p.K + BK - 1) / BK, s = few_rows_split(NB, p.N, p.K, groups), kb_per = (n_kb + s - 1) / s;
+    return few_rows_smem(NB, kb_per, std::min(kb_per, 2)) <= kRSmemMost;
 }
 
 template <int NB>
 static cudaError_t launch_few_rows(const FewRowsProduct& p, bool early, cudaStream_t st) {
-    const int n_kb = (p.K + BK - 1) / BK, s = few_rows_split(p.N, p.K), kb_per = (n_kb + s - 1) / s;
+    const int groups = (p.M + kGemmFewRowsGroup - 1) / kGemmFewRowsGroup;
+    const int n_kb = (p.K + BK - 1) / BK, s = few_rows_split(NB, p.N, p.K, groups), kb_per = (n_kb + s - 1) / s;
     // two CTAs per SM where at least three slots fit: the next launch's weights are then requested while this one still runs
     int n_slots = std::min(kRSlotsMost, kb_per);
-    while (n_slots > 3 && few_rows_smem(NB, kb_per, n_slots) > kRSmemMost / 2) --n_slots;
+    while (n_slots > (groups > 1 ? 2 : 3) && few_rows_smem(NB, kb_per, n_slots) > kRSmemMost / 2) --n_slots;
     while (few_rows_smem(NB, kb_per, n_slots) > kRSmemMost) --n_slots;
     const size_t smem = few_rows_smem(NB, kb_per, n_slots);
-    cudaError_t e = cudaFuncSetAttribute(dia_gemm_few_rows_kernel<NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    // (the same size for every launch: another thread's cannot lower what this one needs)
+    const cudaError_t e = cudaFuncSetAttribute(dia_gemm_few_rows_kernel<NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, kRSmemMost);
     if (e != cudaSuccess) return e;
     CUtensorMap mw;
     if (!make_map(&mw, p.w, p.N, p.K, BM)) return cudaErrorNotSupported;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((p.N + BM - 1) / BM, s);
+    cfg.gridDim = dim3((p.N + BM - 1) / BM, s, groups);
     cfg.blockDim = dim3(kRThreads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
@@ -864,11 +937,27 @@ cudaError_t launch_gemm_tcgen05(const float* x, const float* norm_w, float eps, 
                                 float* y, void* workspace, int M, int N, int K, cudaStream_t st) {
     if (M <= 0 || N % 4 || N <= 0 || K % BK || K < BK) return cudaErrorNotSupported;
     const long long n = (long long)M * K;
+    FewRowsProduct few{x, K, wt, y, N, M, N, K, 0, residual};
+    if (dense_rows_few(M)) {
+        if (norm_w) few.a = reinterpret_cast<const float*>(workspace);
+        // (the rows are read while outputs are written)
+        const bool apart = norm_w || x + n <= y || y + (long long)M * N <= x;
+        if (apart && gemm_few_rows_ok(few)) {
+            if (norm_w) split3_norm_rows_kernel<false><<<M, 256, 0, st>>>(x, norm_w, eps, workspace, M, K);
+            return launch_gemm_few_rows(few, false, st);
+        }
+    }
     if (norm_w)
-        split3_norm_rows_kernel<<<M, 256, 0, st>>>(x, norm_w, eps, reinterpret_cast<__nv_bfloat16*>(workspace), M, K);
+        split3_norm_rows_kernel<true><<<M, 256, 0, st>>>(x, norm_w, eps, workspace, M, K);
     else
         split3_rows_kernel<<<(int)std::min<long long>((n + 255) / 256, 148 * 16), 256, 0, st>>>(
             x, reinterpret_cast<__nv_bfloat16*>(workspace), n);
+    const F32Product wide{nullptr, 0, 0, wt, y, N, N, nullptr, 1, M, N, K, 1.f, 0, nullptr, 0, 0, residual};
+    int dev = 0, sms = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e != cudaSuccess) return e;
+    if (dense_rows_f32(M, N, K, sms) && gemm_f32_ok(wide)) return run_gemm_f32(wide, workspace, 8, st);
     const GemmEpilogue ep{residual, nullptr, nullptr, 0.f, nullptr};
     return launch_gemm_tcgen05_bf16(workspace, kTerms, wt, N, y, M, N, K, ep, nullptr, st);
 }

@@ -46,22 +46,24 @@ struct F32Product {
     float alpha;
     int act;                                 // 0: none, 2: max(z, 0)^2, 3: gelu, the tanh form
     const float* gate; int ldg, head_gate;   // gate[m * ldg + h N + n], with head_gate gate[m * ldg + h]; null: none
+    const float* add;                        // laid out as y, added last (may be y); null: none
 };
 bool gemm_f32_ok(const F32Product& p);
 inline size_t gemm_f32_work_bytes(size_t rows, size_t columns) { return 6 * rows * columns; }      // columns: heads * K
 cudaError_t launch_gemm_f32(const F32Product& p, void* work, cudaStream_t st);
 
-// The same for a few rows (decoding): Y[m][n] = [res +] act(sum_k A[m][k] W[n][k]).  The weights are the 128-row operand and stream
-// once for all rows; the rows' three terms are the columns of the other operand.  A sum's order depends on N and K only.
+// The same for a few rows (decoding, a text): Y[m][n] = [add +] act(sum_k A[m][k] W[n][k]).  The weights are the 128-row operand and
+// stream once for 32 rows; the rows' three terms are the columns of the other operand.  Up to 32 rows a sum's order depends on N and
+// K (and on whether there are more than 8 rows) only.
 // early: launched with programmatic stream serialization (the weights are requested before the predecessor has ended).
-constexpr int kGemmFewRowsMost = 32;
+constexpr int kGemmFewRowsGroup = 32;
 struct FewRowsProduct {
     const float* a; int lda;
     const void* w;
     float* y; int ldy;
     int M, N, K;
     int act;                                 // as in F32Product
-    int add;                                 // != 0: y += the product
+    const float* add;                        // [M][ldy] added to the product (y itself: it is accumulated), or null
 };
 bool gemm_few_rows_ok(const FewRowsProduct& p);
 cudaError_t launch_gemm_few_rows(const FewRowsProduct& p, bool early, cudaStream_t st);

@@ -204,7 +204,7 @@ cudaError_t linear_f32(lm_b200_engine* e, const float* A, int lda, const void* W
                        int act = lm::kActNone) {
     const bool few = few_rows(e, M, N, K);
     if (few && N > lm::kRowsKernelMaxOut && N <= kFewRowsOutMost && act != lm::kActXielu) {
-        const dia::FewRowsProduct p{A, lda, W, Y, ldy, M, N, K, act, 0};
+        const dia::FewRowsProduct p{A, lda, W, Y, ldy, M, N, K, act, nullptr};
         if (dia::gemm_few_rows_ok(p)) return dia::launch_gemm_few_rows(p, M <= lm::kRowsKernelMax, st);
     }
     if (M > lm::kRowsKernelMax && N > lm::kRowsKernelMaxOut && act != lm::kActXielu && e->a_split_bytes >= dia::gemm_f32_work_bytes(M, K)) {
@@ -619,7 +619,7 @@ int product(lm_b200_engine* e, const float* A, const void* Ab, int lda, const vo
         return LM_B200_OK;
     }
     if (M <= lm::kRowsKernelMax) {
-        const dia::FewRowsProduct p{A, lda, W, out, N, M, N, K, 0, 1};
+        const dia::FewRowsProduct p{A, lda, W, out, N, M, N, K, 0, out};
         if (few_rows(e, M, N, K) && N > lm::kRowsKernelMaxOut && N <= kFewRowsOutMost && dia::gemm_few_rows_ok(p)) {
             LCK(dia::launch_gemm_few_rows(p, true, st));
             return LM_B200_OK;

@@ -55,3 +55,53 @@ def test_per_head_products(heads, dim, kv_rank, vdim, rows):
     o = torch.einsum("hij,jhd->ihd", torch.softmax(s.masked_fill(torch.ones(n, n).triu(1).bool(), -torch.inf), -1), v)
     ref = (o * torch.sigmoid(x @ p["g"].T)[:, :, None]).reshape(n, heads * vdim) @ p["o"].T
     assert (got - ref).abs().max() <= 2e-5 * ref.abs().max()
+
+
+@pytest.mark.parametrize("dtype,rows,width,ff", [("float32", 3, 2056, 2060), ("float32", 8, 4104, 1544), ("bfloat16", 9, 136, 132),
+                                                 ("bfloat16", 31, 264, 1000)])
+def test_products_of_a_few_rows(dtype, rows, width, ff):
+    """The same unit where the few-rows kernel takes it (3 to 8 rows of large matrices; up to 31 rows of bf16 products), with clusters that
+    split K, a remainder of K and of N, and up to 8 and up to 32 rows per operand; the bound is the one above."""
+    from dia_tts_prune_b200 import synthetic as SY
+    from dia_tts_prune_b200.lm_config import ForilornConfig
+    from dia_tts_prune_b200.lm_model import CausalLM
+    cfg = SY.forilorn_config(width=width, kinds=["latent_attention"], heads=2, dim=16, vocab=64, lat_dim=16, rot_dim=8, lat_vdim=16, q_rank=72,
+                             kv_rank=24, ff=ff)
+    w = SY.forilorn_weights(cfg, 3)
+    model = CausalLM(ForilornConfig.model_validate(cfg), w, dtype=dtype, device="cuda:0", max_tokens=64, max_sequences=1, max_rows=64)
+    h = torch.randn((rows, width), generator=torch.Generator().manual_seed(4))
+    got = model.engine.op_ff(0, h.cuda()).double().cpu()
+    up, down = w["l0.mlp.up"].double(), w["l0.mlp.down"].double()
+    ref = torch.nn.functional.gelu(h.double() @ up.T, approximate="tanh") @ down.T
+    assert (got - ref).abs().max() <= 1e-5 * ref.abs().max()
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 4, 64), (32, 100, 128), (31, 2048, 4096), (33, 2048, 1024), (129, 260, 192), (200, 1024, 4096),
+                                   (128, 128, 8192), (300, 9252, 128)])
+def test_dense_rows_of_fp32_sums(M, N, K):
+    """The dense layers of the text and prompt passes on the two kernels that add every 64 products in fp32 registers: norm in front and
+    residual behind, one CTA per tile and clusters over K.  The bound is the one above, on the product's largest magnitude."""
+    from dia_tts_prune_b200 import engine as E
+    g = torch.Generator().manual_seed(M + N + K)
+    x, nw = torch.randn(M, K, generator=g), torch.rand(K, generator=g) + 0.5
+    w, res = (torch.randn(K, N, generator=g) * K ** -0.5).to(torch.bfloat16), torch.randn(M, N, generator=g)
+    wt = E.dense_prepare_weight(w.cuda())
+    xd = x.double()
+    xn = xd * torch.rsqrt((xd * xd).mean(-1, keepdim=True) + 1e-5) * nw.double()
+    for norm in (False, True):
+        ref = (xn if norm else xd) @ w.double()
+        r = res.clone().cuda()
+        y = E.dense_forward(x.cuda(), wt, norm_weight=nw.cuda() if norm else None, residual=r)
+        assert (y.cpu().double() - (ref + res.double())).abs().max() <= 1e-5 * ref.abs().max()
+
+
+@pytest.mark.parametrize("rows", [9, 515, 1100])
+def test_grouping_of_many_assignments(rows):
+    """The expert units of a step with more assignments than the grouping kernel has threads against those of the same rows in short
+    steps, where no grouping takes place; both within fp32 rounding of the products."""
+    import test_lm_gpu as T
+    model, _ = T.build(T.small_config(), 7, max_rows=1100)
+    h = torch.randn((rows, 96), generator=torch.Generator().manual_seed(8)).cuda()
+    whole = model.engine.op_ff(0, h)
+    parts = torch.cat([model.engine.op_ff(0, h[i:i + 8]) for i in range(0, rows, 8)])
+    assert (whole - parts).abs().max() <= 1e-5 * parts.abs().max()
