@@ -378,6 +378,8 @@ __device__ __noinline__ float f32_act(int act, float z) {
     return 0.5f * z * (1.0f + tanhf(0.7978845608028654f * fmaf(0.044715f * z * z, z, z)));
 }
 
+// TERMS: terms of A (3: fp32 rows, 1: bf16 rows)
+template <int TERMS>
 __global__ void __launch_bounds__(kGemmThreads, 1)
 dia_gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const __grid_constant__ F32Product p) {
     const int M = p.M, N = p.N, K = p.K;
@@ -430,11 +432,16 @@ dia_gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                                 }
                             }
                             const size_t at = (m + r) * p.ldy + col;
-                            if (p.add) {
+                            if (p.dyt_w) {
+                const float4 w4 = *reinterpret_cast<const float4*>(p.dyt_w + col), b4 = *reinterpret_cast<const float4*>(p.dyt_b + col);
+                v.x = fmaf(tanhf(p.dyt_alpha * v.x), w4.x, b4.x); v.y = fmaf(tanhf(p.dyt_alpha * v.y), w4.y, b4.y);
+                v.z = fmaf(tanhf(p.dyt_alpha * v.z), w4.z, b4.z); v.w = fmaf(tanhf(p.dyt_alpha * v.w), w4.w, b4.w);
+            }
+            if (p.add) {
                     const float4 o = *reinterpret_cast<const float4*>(p.add + at);
                     v.x += o.x; v.y += o.y; v.z += o.z; v.w += o.w;
                 }
-                *reinterpret_cast<float4*>(p.y + at) = v;
+                if (p.y) *reinterpret_cast<float4*>(p.y + at) = v;
                             if (p.y_bf16) {
                                 const __nv_bfloat162 lo = __floats2bfloat162_rn(v.x, v.y), hi = __floats2bfloat162_rn(v.z, v.w);
                                 *reinterpret_cast<uint2*>(reinterpret_cast<__nv_bfloat16*>(p.y_bf16) + at) =
@@ -470,7 +477,7 @@ dia_gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                     mbar_arrive_expect_tx(&b_full[s], kTileBytes);
                     tma_load_2d(smem_u32(b_ring + s * kTileBytes), &map_b, smem_u32(&b_full[s]), (kb0 + kb) * BK, h * N + n0);
                     ++ib;
-                    for (int tm = kTerms - 1; tm >= 0; --tm) {          // the smallest term first
+                    for (int tm = TERMS - 1; tm >= 0; --tm) {          // the smallest term first
                         const unsigned sa = ia % kFASlots;
                         mbar_wait_bounded(&a_empty[sa], ((ia / kFASlots) & 1u) ^ 1u);
                         mbar_arrive_expect_tx(&a_full[sa], kTileBytes);
@@ -490,7 +497,7 @@ dia_gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                 mbar_wait_bounded(&b_full[sb], (ib / kFBSlots) & 1u);
                 const uint64_t bdesc = umma_desc(smem_u32(b_ring + sb * kTileBytes));
                 const uint32_t d = tmem_base + acc * kFN;
-                for (int tm = 0; tm < kTerms; ++tm) {
+                for (int tm = 0; tm < TERMS; ++tm) {
                     const unsigned sa = ia % kFASlots;
                     mbar_wait_bounded(&a_full[sa], (ia / kFASlots) & 1u);
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -499,7 +506,7 @@ dia_gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
 #pragma unroll
                         for (int j = 0; j < BK / 16; ++j) umma_bf16(d, adesc + 2 * j, bdesc + 2 * j, idesc, (tm | j) != 0 ? 1u : 0u);
                         umma_commit(&a_empty[sa]);
-                        if (tm == kTerms - 1) {
+                        if (tm == TERMS - 1) {
                             umma_commit(&b_empty[sb]);
                             umma_commit(&t_full[acc]);
                         }
@@ -786,6 +793,9 @@ cudaError_t launch_transpose_to_bf16(const void* w, int src_bf16, void* wt, int 
 
 // A: bf16 [terms * M][K], the terms of the activation stacked (terms = 1: the activation itself); Wt: bf16 [wt_rows][K].
 // Returns cudaErrorNotSupported for shapes the tiling does not cover (the caller decides what to do).
+static bool dense_rows_f32(int terms, int M, int N, int K, int sms);
+static cudaError_t run_gemm_f32(const F32Product& p, const void* a_terms, int terms, int splits, cudaStream_t st);
+
 cudaError_t launch_gemm_tcgen05_bf16(const void* a_bf16, int terms, const void* wt, long long wt_rows, float* y, int M, int N,
                                      int K, const GemmEpilogue& ep, const GemmGroups* groups, cudaStream_t st) {
     if (!gemm_tcgen05_shape_ok(M, N, K) || terms < 1 || terms > kTerms || wt_rows < N) return cudaErrorNotSupported;
@@ -808,6 +818,11 @@ cudaError_t launch_gemm_tcgen05_bf16(const void* a_bf16, int terms, const void* 
         if (dev < 0 || dev >= 64) n_sm[0] = n; else n_sm[dev] = n;
     }
     const int sms = (dev < 0 || dev >= 64) ? n_sm[0] : n_sm[dev];
+    if (terms == 1 && !groups && wt_rows == N && dense_rows_f32(1, M, N, K, sms)) {
+        const F32Product narrow{nullptr, 0, 0, wt, ep.y_bf16 ? nullptr : y, N, N, ep.y_bf16, 1, M, N, K, 1.f, ep.y_bf16 ? 3 : 0, nullptr, 0, 0,
+                                ep.residual, ep.dyt_w, ep.dyt_b, ep.dyt_alpha};
+        if (gemm_f32_ok(narrow)) return run_gemm_f32(narrow, a_bf16, 1, 8, st);
+    }
     const int n_tiles = ((N + BN - 1) / BN) * ((M + BM - 1) / BM);
     dia_gemm_tcgen05_kernel<<<std::min(n_tiles, sms), kGemmThreads, kGemmSmem, st>>>(
         ma, mb, y, ep.residual, M, N, K, terms, ep.dyt_w, ep.dyt_b, ep.dyt_alpha,
@@ -830,27 +845,31 @@ static int f32_splits(int tiles, int n_kb, int most, int sms) {
     while (2 * s <= most && tiles * 2 * s <= sms && n_kb >= 4 * s) s *= 2;
     return s;
 }
-// Beyond 32 rows the fp32-sum kernel where its rounds of tiles are the shorter ones: a k-block of a round of its 128 x 128 tiles takes
-// three quarters of one of 128 x 256 tiles (1.1 and 1.4 us; both are bound by the operands' way from L2), its tiles are twice as many, and
-// where they leave the chip idle its clusters split K (us, 128 x 256 tiles / here: 200 rows N = 2048, K = 1024 27 / 14, N = 1024, K = 4096
-// 77 / 31, N = 8192, K = 1024 29 / 26, N = 16384, K = 2048 51 / 73; 1024 rows N = 2048, K = 1024 30 / 27; 1722 rows 33 / 45)
-static bool dense_rows_f32(int M, int N, int K, int sms) {
+// Beyond 32 rows (and for bf16 rows) the fp32-sum kernel where its rounds of tiles are the shorter ones: its 128 x 128 tiles are twice
+// as many, and where they leave the chip idle its clusters split K.  Three terms: a k-block of a round takes three quarters of one of
+// 128 x 256 tiles (1.1 and 1.4 us; both are bound by the operands' way from L2).  us, 128 x 256 tiles / here: 200 rows N = 2048,
+// K = 1024 27 / 14, N = 1024, K = 4096 77 / 31, N = 8192, K = 1024 29 / 26, N = 16384, K = 2048 51 / 73; 1024 rows N = 2048, K = 1024
+// 30 / 27; 1722 rows 33 / 45.  One term: about the same per k-block, a shorter start and end.  150 rows N = K = 2048 23 / 12, N = 2048,
+// K = 6144 53 / 20, N = 288, K = 96 11 / 9; 1024 rows N = 2048, K = 6144 55 / 59, N = 512, K = 2048 22 / 12
+static bool dense_rows_f32(int terms, int M, int N, int K, int sms) {
     const int tm = (M + BM - 1) / BM, n_kb = (K + BK - 1) / BK;
     const long long narrow = (long long)tm * ((N + kFN - 1) / kFN), wide = (long long)tm * ((N + BN - 1) / BN);
     const int s = narrow < sms ? f32_splits((int)narrow, n_kb, 8, sms) : 1;
-    return ((narrow * s + sms - 1) / sms) * ((n_kb + s - 1) / s) * 3 < ((wide + sms - 1) / sms) * n_kb * 4;
+    const long long here = (narrow * s + sms - 1) / sms, there = (wide + sms - 1) / sms;
+    const int kb = (n_kb + s - 1) / s;
+    return terms == 1 ? here * (21 * kb + 100) < there * (20 * n_kb + 130) : here * kb * 3 < there * n_kb * 4;
 }
 
-
 // splits: the most CTAs that may share a tile (1: a sum's order does not depend on the rows beside it)
-static cudaError_t run_gemm_f32(const F32Product& p, const void* terms, int splits, cudaStream_t st) {
+static cudaError_t run_gemm_f32(const F32Product& p, const void* a_terms, int terms, int splits, cudaStream_t st) {
     int dev = 0, sms = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(dia_gemm_f32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kFSmem);
+    const auto kernel = terms == 1 ? dia_gemm_f32_kernel<1> : dia_gemm_f32_kernel<kTerms>;
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kFSmem);
     if (e != cudaSuccess) return e;
     CUtensorMap ma, mb;
-    if (!make_map(&ma, terms, (long long)kTerms * p.heads * p.M, p.K, BM) || !make_map(&mb, p.w, (long long)p.heads * p.N, p.K, kFN))
+    if (!make_map(&ma, a_terms, (long long)terms * p.heads * p.M, p.K, BM) || !make_map(&mb, p.w, (long long)p.heads * p.N, p.K, kFN))
         return cudaErrorNotSupported;
     const int n_tiles = p.heads * ((p.N + kFN - 1) / kFN) * ((p.M + BM - 1) / BM), n_kb = (p.K + BK - 1) / BK;
     const int s = f32_splits(n_tiles, n_kb, splits, sms);
@@ -866,13 +885,13 @@ static cudaError_t run_gemm_f32(const F32Product& p, const void* terms, int spli
     attr.val.clusterDim.z = 1;
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, dia_gemm_f32_kernel, ma, mb, p);
+    return cudaLaunchKernelEx(&cfg, kernel, ma, mb, p);
 }
 
 cudaError_t launch_gemm_f32(const F32Product& p, void* work, cudaStream_t st) {
     if (!gemm_f32_ok(p)) return cudaErrorNotSupported;
     split3_heads_kernel<<<p.M, 256, 0, st>>>(p.a, p.lda, p.a_hs, reinterpret_cast<__nv_bfloat16*>(work), p.heads, p.M, p.K);
-    return run_gemm_f32(p, work, 1, st);
+    return run_gemm_f32(p, work, kTerms, 1, st);
 }
 
 static size_t few_rows_smem(int NB, int kb_per, int n_slots) {
@@ -957,7 +976,7 @@ cudaError_t launch_gemm_tcgen05(const float* x, const float* norm_w, float eps, 
     cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (e != cudaSuccess) return e;
-    if (dense_rows_f32(M, N, K, sms) && gemm_f32_ok(wide)) return run_gemm_f32(wide, workspace, 8, st);
+    if (dense_rows_f32(kTerms, M, N, K, sms) && gemm_f32_ok(wide)) return run_gemm_f32(wide, workspace, kTerms, 8, st);
     const GemmEpilogue ep{residual, nullptr, nullptr, 0.f, nullptr};
     return launch_gemm_tcgen05_bf16(workspace, kTerms, wt, N, y, M, N, K, ep, nullptr, st);
 }

@@ -47,6 +47,7 @@ struct F32Product {
     int act;                                 // 0: none, 2: max(z, 0)^2, 3: gelu, the tanh form
     const float* gate; int ldg, head_gate;   // gate[m * ldg + h N + n], with head_gate gate[m * ldg + h]; null: none
     const float* add;                        // laid out as y, added last (may be y); null: none
+    const float* dyt_w; const float* dyt_b; float dyt_alpha;      // as in GemmEpilogue, in front of add
 };
 bool gemm_f32_ok(const F32Product& p);
 inline size_t gemm_f32_work_bytes(size_t rows, size_t columns) { return 6 * rows * columns; }      // columns: heads * K

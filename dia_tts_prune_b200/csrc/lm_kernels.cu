@@ -5,8 +5,9 @@
 // portions, single decoded tokens and mixed batches are the same launch sequence.  Every kernel here computes a row's
 // result from that row (and the sequence state it points at) alone, in an order of operations that does not depend on
 // which other rows are in the batch - so the value at a position does not depend on how the prompt was cut or batched.
-// (The only thing the row count selects is which of the two linear kernels runs; they sum in different orders, so a
-// position computed in a step of a few rows and in a long one agrees to rounding, and to the bit within either kind.)
+// (The only thing the row count selects is which linear and attention kernels run; they sum in different orders, so a position
+// computed in steps of different kinds - a row or two, up to 8 rows, longer; with bf16 products also by the tiles of a long step -
+// agrees to rounding, and to the bit within a kind.)
 //
 // Precision: activations, the residual stream, norms, router, attention scores / weights and the K/V pages are fp32;
 // matrices are bf16 in memory and multiplied with fp32 accumulation.

@@ -105,3 +105,21 @@ def test_grouping_of_many_assignments(rows):
     whole = model.engine.op_ff(0, h)
     parts = torch.cat([model.engine.op_ff(0, h[i:i + 8]) for i in range(0, rows, 8)])
     assert (whole - parts).abs().max() <= 1e-5 * parts.abs().max()
+
+
+@pytest.mark.parametrize("M,N,K", [(32, 2048, 2048), (150, 288, 96), (200, 100, 72), (129, 132, 4104), (1024, 2048, 6144), (1, 8, 8)])
+def test_products_of_bf16_rows(M, N, K):
+    """A bf16 operand on both sides of the rule between 128 x 256 tiles and 128 x 128 tiles with split sums.  The wider tiles add K products
+    in tensor memory, each addition cut off at 2^-23 of the sum: K 2^-23 of its magnitude at most, against 2e-6 + K 2^-24 here (the errors
+    do not all add up)."""
+    import ctypes as C
+
+    from dia_tts_prune_b200 import _lm_lib
+    lib, g = _lm_lib.load(), torch.Generator().manual_seed(M + N + K)
+    x, w = torch.randn(M, K, generator=g).cuda(), (torch.randn(N, K, generator=g) * K ** -0.5).to(torch.bfloat16).cuda()
+    y, xb = torch.empty(M, N, device="cuda"), torch.empty(M, K, device="cuda", dtype=torch.bfloat16)
+    p = lambda t: C.c_void_p(t.data_ptr())                                                       # noqa: E731
+    _lm_lib.check(lib.lm_b200_op_linear_tc(p(x), p(w), p(y), p(xb), M, N, K, C.c_void_p(torch.cuda.current_stream().cuda_stream)), "op_linear_tc")
+    assert torch.equal(xb, x.to(torch.bfloat16))
+    ref = x.to(torch.bfloat16).double() @ w.double().T
+    assert (y - ref).abs().max() <= (2e-6 + K * 2.0 ** -24) * ref.abs().max()
