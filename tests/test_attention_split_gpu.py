@@ -112,3 +112,22 @@ def test_mixed_scores(H, G, d, dv, rows):
         ref.append(torch.stack(out, 1).reshape(n, H * dv))
     ref = torch.cat(ref)
     close(got, ref, ref.abs().max().item())
+
+
+@pytest.mark.parametrize("mode,B,Tq,Tk,Hq,Hkv,n_valid", [(0, 2, 256, 256, 4, 1, None), (1, 2, 300, 300, 2, 2, [37, 257]), (1, 1, 256, 256, 3, 3, [0]),
+                                                         (2, 2, 257, 130, 4, 2, [0, 129]), (2, 1, 511, 64, 2, 2, [64])])
+def test_row_modes(mode, B, Tq, Tk, Hq, Hkv, n_valid):
+    """Dia's causal, pad-partitioned and prefix attention where the split kernel takes them (256 queries and more), against 64 bits.  Both
+    factors keep 22 bits: 2^-21 of a score of at most about 6 here and of the value, a few times over."""
+    from dia_tts_prune_b200 import engine as E
+    g = torch.Generator().manual_seed(Tq + Tk)
+    q, k, v = (torch.randn(s, generator=g) for s in ((B, Tq, Hq, 128), (B, Hkv, Tk, 128), (B, Hkv, Tk, 128)))
+    got = E.attention_rows(q.cuda(), k.cuda(), v.cuda(), Tk, mode, n_valid).cpu().double()
+    i, j = torch.arange(Tq)[:, None], torch.arange(Tk)[None, :]
+    for b in range(B):
+        n = n_valid[b] if n_valid else Tk
+        see = j <= i if mode == 0 else (i < n) == (j < n) if mode == 1 else (j < n).expand(Tq, Tk)
+        s = (torch.einsum("ihd,hjd->hij", q[b].double(), k[b].double().repeat_interleave(Hq // Hkv, 0)) * 128 ** -0.5).masked_fill(~see, -torch.inf)
+        w = torch.nan_to_num(torch.softmax(s, -1), nan=0.0)
+        ref = torch.einsum("hij,hjd->ihd", w, v[b].double().repeat_interleave(Hq // Hkv, 0))
+        assert (got[b] - ref).abs().max() <= 2e-5 * max(1.0, ref.abs().max())
