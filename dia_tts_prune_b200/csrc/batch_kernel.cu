@@ -217,26 +217,6 @@ __device__ __forceinline__ void umma_bf16_b(uint32_t tmem_d, uint64_t adesc, uin
         ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
         : "memory");
 }
-// the same arrive delivered to the barrier at this offset in every CTA of `mask` (the CTA pair shares each activation stage)
-__device__ __forceinline__ void umma_commit_mc_b(uint64_t* bar, uint16_t mask) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(smem_u32(bar)), "h"(mask) : "memory");
-}
-__device__ __forceinline__ void bulk_g2s_mc(void* dst_smem, const void* src_gmem, uint32_t bytes, uint64_t* bar, uint16_t mask) {
-    asm volatile(
-        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.multicast::cluster [%0], [%1], %2, [%3], %4;" ::"r"(
-            smem_u32(dst_smem)),
-        "l"(src_gmem), "r"(bytes), "r"(smem_u32(bar)), "h"(mask)
-        : "memory");
-}
-__device__ __forceinline__ uint32_t cluster_ctarank() {
-    uint32_t r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
-__device__ __forceinline__ void cluster_sync_all() {
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
 __device__ __forceinline__ void umma_commit_b(uint64_t* bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
@@ -378,7 +358,6 @@ __device__ void act_loop_b(const BatchParams& p, unsigned char* scratch, BMisc* 
     unsigned bctr = 0;
     const bool prof = p.prof != nullptr && blockIdx.x == 0;
     long long t_ready = 0, t_bempty = 0, tq = 0;
-    const uint32_t rank = p.mc ? cluster_ctarank() : 0u;
 #pragma unroll 1
     for (int n = 0; n < p.n_steps; ++n) {
 #pragma unroll 1
@@ -430,22 +409,13 @@ __device__ void act_loop_b(const BatchParams& p, unsigned char* scratch, BMisc* 
                 // and its pair too - has finished the stage that produced it, i.e. all MMAs of its previous GEMM have retired and
                 // every activation stage is free (a wait changes no barrier state; an mbarrier test costs ~120 cycles, and the four
                 // issuers start with copies 0..3)
-                // (not when a CTA pair shares its stages: the pair's multicast arrive may still be in flight)
-                if (su >= kActStages || p.mc) {
+                if (su >= kActStages) {
                     if (prof) tq = clock64();
                     mbar_spin(&misc->bempty[bs], ((bi / kActStages) & 1u) ^ 1u, p.err, kErrEmptyBarrierTimeout, (seq << 8) | 0xc0 | bs);
                     if (prof) t_bempty += clock64() - tq;
                 }
                 mbar_arrive_expect_tx(&misc->bfull[bs], kActStageBytes);
-                if (p.mc) {
-                    // this CTA fetches its half of the stage (the chunk of its cluster rank) for both CTAs of the pair; the
-                    // peer's half arrives the same way.  bempty[bs] has collected the commits of BOTH CTAs' MMA warps.
-                    const uint32_t half = rank * (kActStageBytes / 2);
-                    bulk_g2s_mc(scratch + bs * kActStageBytes + half, src + (size_t)st * kActStageBytes + half, kActStageBytes / 2,
-                                &misc->bfull[bs], (uint16_t)3);
-                } else {
-                    bulk_g2s(scratch + bs * kActStageBytes, src + (size_t)st * kActStageBytes, kActStageBytes, &misc->bfull[bs]);
-                }
+                bulk_g2s(scratch + bs * kActStageBytes, src + (size_t)st * kActStageBytes, kActStageBytes, &misc->bfull[bs]);
             }
             bctr += (unsigned)n_st;
         }
@@ -541,10 +511,7 @@ __device__ __forceinline__ void issue_gemm_b(BCtx& c, int gt, int K, int gc) {
                     umma_bf16_b(d0 + (uint32_t)(j & (kAccPerIssuer - 1)) * (2 * kRows), adesc + 2 * j, bdesc + 2 * j, idesc,
                                 (cc != 0 || j >= kAccPerIssuer) ? 1u : 0u);
                 if (in_slot == cps - 1) umma_commit_b(&misc->empty[slot]);
-                if (jc == kStageChunks - 1) {
-                    if (p.mc) umma_commit_mc_b(&misc->bempty[bs], (uint16_t)3);
-                    else umma_commit_b(&misc->bempty[bs]);
-                }
+                if (jc == kStageChunks - 1) umma_commit_b(&misc->bempty[bs]);
             }
             __syncwarp();
         }
@@ -1207,9 +1174,8 @@ extern "C" __global__ void __launch_bounds__(kBThreads, 1) dia_batch_step_kernel
     if (tid == 0) {
         // every ring slot and activation stage has ONE consumer (the issuer whose quarter of the contraction it belongs to)
         for (int i = 0; i < kBNumSlots; ++i) { mbar_init(&misc->full[i], 1); mbar_init(&misc->empty[i], 1); }
-        // a stage is filled by one bulk copy (or two multicast halves: one arrive.expect_tx for both) and released by
-        // its issuer's commit - of both CTAs when a pair shares its activation stages
-        for (int i = 0; i < kActStages; ++i) { mbar_init(&misc->bfull[i], 1); mbar_init(&misc->bempty[i], p.mc ? 2 : 1); }
+        // a stage is filled by one bulk copy and released by its issuer's commit
+        for (int i = 0; i < kActStages; ++i) { mbar_init(&misc->bfull[i], 1); mbar_init(&misc->bempty[i], 1); }
         mbar_init(&misc->acc_full, kBIssuers);
         misc->stages_done = 0;
         misc->ready_seq = 0;
@@ -1228,7 +1194,6 @@ extern "C" __global__ void __launch_bounds__(kBThreads, 1) dia_batch_step_kernel
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    if (p.mc) cluster_sync_all();          // the peer's barriers exist before anything is multicast to them
 
     const int S = 8 * p.L + 3, n_stage = p.with_sample ? S : S - 1;
     asm volatile(".reg .pred dia_pw_bfull;" ::);       // mma_loop_b: result of the early test of the next activation stage's barrier
@@ -1285,7 +1250,6 @@ extern "C" __global__ void __launch_bounds__(kBThreads, 1) dia_batch_step_kernel
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
-    if (p.mc) cluster_sync_all();          // no CTA leaves while its peer may still multicast into its shared memory
     if (warp == kMmaWarp) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(misc->tmem_base), "r"(kTmemCols));
@@ -1307,13 +1271,11 @@ cudaError_t launch_batch_kernel(const BatchParams& p, cudaStream_t st) {
     cfg.blockDim = dim3(kBThreads);
     cfg.dynamicSmemBytes = kBSmem;
     cfg.stream = st;
-    cudaLaunchAttribute at[2];
-    at[0].id = cudaLaunchAttributeCooperative;
-    at[0].val.cooperative = 1;
-    at[1].id = cudaLaunchAttributeClusterDimension;
-    at[1].val.clusterDim.x = 2; at[1].val.clusterDim.y = 1; at[1].val.clusterDim.z = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = p.mc ? 2 : 1;           // CTA pairs (the two SMs of a TPC) when the pair shares its activation stages
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeCooperative;
+    at.val.cooperative = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, dia_batch_step_kernel, p);
 }
 

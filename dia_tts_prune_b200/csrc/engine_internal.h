@@ -191,7 +191,6 @@ struct BatchParams {
     int Kdim[G_COUNT];
     float eps;
     int G, U, R;                       // CTAs, utterances, batch rows (2 U: row 2u = unconditional, 2u + 1 = conditional)
-    int mc;                            // 1: launched as clusters of 2 CTAs that share every activation stage (multicast halves)
     int sa_nsplit, ca_nsplit;
     const unsigned char* wstream;
     const CtaTable* cta_tab;

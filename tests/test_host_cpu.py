@@ -392,3 +392,13 @@ def test_row_compaction_plan_is_exact():
     SY.init_synthetic_(dia2.model.named_parameters(), 3)
     sd2 = dict(dia2.model.decoder.named_parameters())
     assert PU.plan_row_compaction({n: sd2[n].detach() for n in decoder_tensor_names(cfg)}, L) == {}
+
+
+def test_no_load_is_multicast_to_a_cluster():
+    """Replicas of these kernels run on several GPUs, where a load that is multicast to a cluster is not safe: no source issues one."""
+    csrc = os.path.join(REPO, "dia_tts_prune_b200", "csrc")
+    sources = [f for f in os.listdir(csrc) if f.endswith((".cu", ".cuh", ".h"))]
+    assert sources
+    for f in sources:
+        with open(os.path.join(csrc, f)) as src:
+            assert not re.search(r"cp\.async\.bulk[^\"]*\.multicast", src.read()), f
