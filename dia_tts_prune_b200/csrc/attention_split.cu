@@ -16,9 +16,11 @@
 // over K = 2048).  So no accumulator lives longer than one tile and one channel group, and sums over tiles are fp32 additions
 // in registers: measured against 64 bits the output is as close as the fp32 FMA kernels' (2.6e-7 both at 300 rows, d = 128).
 //
-// Scaling: a query tile, a group of 16 keys and a tile of values are each brought to a largest magnitude of [2^14, 2^15) before
-// the split (the largest finite one; powers of two, undone exactly), so the fp16 range costs nothing: an element down to 2^-17 of
-// its group's largest keeps its 22 bits.  Softmax weights carry 2^14.
+// Scaling: every query row, key row and value row is brought to a largest magnitude of [2^14, 2^15) by a power of two of its own
+// before the split.  A query's and a key's are undone on the score; a value's joins the weight, and the weights of a row and a tile
+// of keys, times their values' magnitudes, are brought to the same range before they are split.  So an element down to 2^-17 of its
+// row's largest keeps its 22 bits, what a row of the output sums loses at most 2^-39 of the largest weight x value that it sees, and
+// nothing of a token that it does not see, or of another row, enters its result: the bits do not depend on what shares the launch.
 //
 // Bound: per 64 keys and 128 rows 3 x 128 x 64 x (dk + dv) multiply-adds on the tensor pipe (1536 cycles at 128 + 128) against
 // about as many issue slots for splitting and softmax.
@@ -40,10 +42,9 @@ namespace {
 
 constexpr int kRows = 128, kKeys = 64, kGroupW = 128;        // query rows of a CTA, keys of a tile, channels of a stage
 constexpr int kSplitThreadsTC = 512;
-constexpr int kMaxSlots = 6, kScaleRing = 8, kMaxKStages = 4;
-constexpr int kSmemMost = 232448, kStaticMost = 128;       // dynamic and static; the few static words
+constexpr int kMaxSlots = 6, kMaxDepth = 5, kMaxKStages = 4;
+constexpr int kSmemMost = 232448;                             // all of it dynamic
 constexpr float kLog2e = 1.4426950408889634f;
-constexpr float kWeightScale = 16384.f;                       // on the softmax weights (at most 1) before the split
 constexpr int kSplitOnceRows = 512;                           // rows of a kv head (M rep) from which the keys are split in advance
 constexpr unsigned kSpinMost = 4000000u;
 
@@ -56,9 +57,12 @@ struct Geometry {
     int shared_kv;                           // the value is the head of the key row: value group i is key group i
     int slot_bytes, n_slots, q_bytes;
     int o_bufs;                              // accumulators of the value product (2 where tensor memory has the columns)
-    // the split keys and values in SplitAttention::work: SlotTiles per slot, then inverse scales [tile][part], then the tiles.  A
-    // tile's parts: key groups (per kv head where the launch reads one head at a time), then value groups
-    int parts, k_parts, cap_tiles;
+    int k_sets;                              // scales of a key: one, with mixed scores one per kv head
+    int depth;                               // tiles whose scales are in shared memory
+    // the split keys and values in SplitAttention::work: SlotTiles per slot, then inverse scales [tile][set][key], then the tiles.  A
+    // tile's parts: key groups (per kv head where the launch reads one head at a time), then value groups; its sets of scales: the keys
+    // of each kv head, then the values of each (shared_kv: the keys' only)
+    int parts, k_parts, sets, cap_tiles;
     unsigned tile_bytes, scale_off, tile_off;
 };
 // where the tiles of a slot's sequence lie: tile j / 64 of its keys is tile base + j / 64 of the room for first <= j / 64 < end; its
@@ -165,6 +169,16 @@ __device__ __forceinline__ float2 tanh_near_zero(float2 x) {
     q = fma2(q, u, make_float2(-3.33333332312e-1f, -3.33333332312e-1f));
     return fma2(mul2(x, u), q, x);
 }
+// v[i] *= f[i] (16-byte aligned; the same addresses for all lanes)
+template <int N>
+__device__ __forceinline__ void scale_by(float* v, const float* f) {
+#pragma unroll
+    for (int e = 0; e < N; e += 4) {
+        const float4 k = *reinterpret_cast<const float4*>(f + e);
+        const float2 a = mul2(make_float2(v[e], v[e + 1]), make_float2(k.x, k.y)), b = mul2(make_float2(v[e + 2], v[e + 3]), make_float2(k.z, k.w));
+        v[e] = a.x; v[e + 1] = a.y; v[e + 2] = b.x; v[e + 3] = b.y;
+    }
+}
 __device__ __forceinline__ void tmem_loaded() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tmem_store8(uint32_t addr, const uint32_t (&v)[8]) {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(addr), "r"(v[0]), "r"(v[1]),
@@ -186,14 +200,14 @@ __device__ __forceinline__ float scale_of(float m, float& inverse) {
     inverse = __uint_as_float((uint32_t)(e + 113) << 23);
     return __uint_as_float((uint32_t)(min(141 - e, 254)) << 23);
 }
-__device__ __forceinline__ float max_abs4(float m, const float4& v) {
-    return fmaxf(fmaxf(fmaxf(m, fabsf(v.x)), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w)));
-}
 __device__ __forceinline__ float finite_abs(float x) { const float a = fabsf(x); return a <= 3.402823466e38f ? a : 0.f; }
-__device__ __forceinline__ float warp_max_of(float v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
-    return v;
+__device__ __forceinline__ float max_finite4(float m, const float4& v) {
+    return fmaxf(fmaxf(fmaxf(m, finite_abs(v.x)), finite_abs(v.y)), fmaxf(finite_abs(v.z), finite_abs(v.w)));
+}
+// lanes 8 apart hold the channels of one row
+__device__ __forceinline__ float row_max(float v) {
+    v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, 8));
+    return fmaxf(v, __shfl_xor_sync(0xffffffffu, v, 16));
 }
 __device__ __forceinline__ int first_key_of(int i, int window, int chunk) {
     const int w = window > 0 ? max(0, i - window + 1) : 0;
@@ -213,7 +227,6 @@ __device__ __forceinline__ size_t part_offset(const Geometry& geo, int part) {
 __global__ void __launch_bounds__(256)
 split_keys_kernel(const __grid_constant__ SplitAttention p, const __grid_constant__ Geometry geo) {
     __shared__ int s_first, s_seq, s_run;
-    __shared__ float s_m[8];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, tile = blockIdx.x, part = blockIdx.y;
     const bool writes_plan = tile == 0 && part == 0;
     SlotTiles* plan = reinterpret_cast<SlotTiles*>(p.work);
@@ -272,7 +285,7 @@ split_keys_kernel(const __grid_constant__ SplitAttention p, const __grid_constan
     const float* src = is_v ? p.vcache : p.kcache;
     if (in) {
         const int page = p.table[(size_t)slot * p.max_pages + j / p.page_size];
-        src += (((size_t)page * p.kv_heads + g) * p.page_size + j % p.page_size) * width + c0;
+        src += (((size_t)page * p.kv_heads + g) * p.page_size + j % p.page_size) * width;
     }
     float4 v[8];
     float m = 0.f;
@@ -280,20 +293,22 @@ split_keys_kernel(const __grid_constant__ SplitAttention p, const __grid_constan
     for (int i = 0; i < 4; ++i) {
         const int c = 8 * (cq + 4 * i);
         const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
-        v[2 * i] = in && c < w ? *reinterpret_cast<const float4*>(src + c) : z;
-        v[2 * i + 1] = in && c + 4 < w ? *reinterpret_cast<const float4*>(src + c + 4) : z;
+        v[2 * i] = in && c < w ? *reinterpret_cast<const float4*>(src + c0 + c) : z;
+        v[2 * i + 1] = in && c + 4 < w ? *reinterpret_cast<const float4*>(src + c0 + c + 4) : z;
     }
+    // the scale is that of the whole row (a latent's value is a part of its key row)
+    const int row_w = is_v ? p.vdim : p.kdim;
 #pragma unroll
-    for (int i = 0; i < 8; ++i) m = fmaxf(fmaxf(fmaxf(m, finite_abs(v[i].x)), finite_abs(v[i].y)), fmaxf(finite_abs(v[i].z), finite_abs(v[i].w)));
-    m = warp_max_of(m);
-    if (lane == 0) s_m[warp] = m;
-    __syncthreads();
-#pragma unroll
-    for (int i = 0; i < 8; ++i) m = fmaxf(m, s_m[i]);
+    for (int i = 0; i < 8; ++i) m = max_finite4(m, v[i]);
+    if (w < row_w && in)
+        for (int c = 4 * cq; c < row_w; c += 16) m = max_finite4(m, *reinterpret_cast<const float4*>(src + c));
+    m = row_max(m);
     float inverse;
     const float sc = scale_of(m, inverse);
     unsigned char* work = reinterpret_cast<unsigned char*>(p.work);
-    if (tid == 0) *reinterpret_cast<float*>(work + geo.scale_off + 4 * ((size_t)tile * geo.parts + part)) = inverse;
+    const int set = is_v ? p.kv_heads + gg : talk ? st : gg;
+    if (cq == 0 && (talk || st == 0))
+        reinterpret_cast<float*>(work + geo.scale_off)[((size_t)tile * geo.sets + set) * kKeys + warp * 8 + kin] = inverse;
     unsigned char* base = work + geo.tile_off + (size_t)tile * geo.tile_bytes + part_offset(geo, part);
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
@@ -363,11 +378,10 @@ template <int NVS>
 __global__ void __launch_bounds__(kSplitThreadsTC, 1)
 split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_constant__ Geometry geo) {
     constexpr int DVH = 64 * NVS;                             // output channels of a thread
+    // the block is launched with 128 registers a thread: 256 of kRowRegs, 128 of kFetchRegs and 128 of 32
+    constexpr int kRowRegs = NVS == 1 ? 176 : 184, kFetchRegs = NVS == 1 ? 128 : 112;
+    static_assert(256 * kRowRegs + 128 * kFetchRegs + 128 * 32 <= 128 * kSplitThreadsTC, "registers of the block");
     extern __shared__ __align__(128) unsigned char smem[];
-    __shared__ float s_red[8];
-    __shared__ uint32_t s_breaks[4];
-    __shared__ uint32_t s_tmem;
-    __shared__ int s_rows[2];
     unsigned char* ring = smem;
     unsigned char* qs = ring + (size_t)geo.n_slots * geo.slot_bytes;
     uint64_t* full = reinterpret_cast<uint64_t*>(qs + geo.q_bytes);
@@ -376,14 +390,16 @@ split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_co
     uint64_t* s_empty = s_full + 1;
     uint64_t* p_ready = s_empty + 1;                          // weights of a tile are there / its value product is done
     uint64_t* pv_done = p_ready + 1;
-    uint64_t* v_max = pv_done + 1;                            // the four fetching warps' largest values
-    uint64_t* q_ready = v_max + 1;
-    uint64_t* pair = q_ready + 1;                               // [4] the two warps that share rows
-    float* k_inv = reinterpret_cast<float*>(pair + 4);        // [kScaleRing][kMaxKStages][4] inverse scales of 16 keys
-    float* v_inv = k_inv + kScaleRing * kMaxKStages * 4;      // [kScaleRing][2]
-    float* vm_s = v_inv + kScaleRing * 2;                     // [2][4]
-    float* row_x = vm_s + 8;                                  // [2][2][128] what the two threads of a row tell each other
-    int* s_slot = reinterpret_cast<int*>(row_x + 4 * kRows);  // [tokens]
+    uint64_t* q_ready = pv_done + 1;
+    uint64_t* pair = q_ready + 1;                             // [4] the two warps that share rows
+    uint64_t* v_ready = pair + 4;                             // [depth] the scales of a tile's values are there
+    float* k_inv = reinterpret_cast<float*>(v_ready + kMaxDepth);      // [depth][k_sets][64] inverse scales of the keys
+    float* v_inv = geo.shared_kv ? k_inv : k_inv + geo.depth * geo.k_sets * kKeys;      // [depth][64] of the values
+    float* row_x = v_inv + geo.depth * kKeys;                 // [2][2][128] what the two threads of a row tell each other
+    uint32_t* s_breaks = reinterpret_cast<uint32_t*>(row_x + 4 * kRows);      // [4]
+    uint32_t* s_tmem = s_breaks + 4;
+    int* s_rows = reinterpret_cast<int*>(s_tmem + 1);         // [2]
+    int* s_slot = s_rows + 3;                                 // [tokens]
     const int TT = kRows >> geo.pk_shift;
     int* s_pos = s_slot + TT;
 
@@ -428,13 +444,13 @@ split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_co
         mbar_init(s_empty, 8);
         mbar_init(p_ready, 8);
         mbar_init(pv_done, 1);
-        mbar_init(v_max, 4);
         mbar_init(q_ready, 8);
         for (int i = 0; i < 4; ++i) mbar_init(&pair[i], 2);
+        for (int i = 0; i < kMaxDepth; ++i) mbar_init(&v_ready[i], 4);
         fence_mbar_init();
     }
     if (warp == 12) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(&s_tmem)));
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(s_tmem)));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::);
     }
     if (tid < kRows) {
@@ -457,12 +473,12 @@ split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_co
     fence_before();
     __syncthreads();
     fence_after();
-    const uint32_t tmem = s_tmem;
+    const uint32_t tmem = *s_tmem;
     const uint32_t t_s = tmem, t_p = tmem + 64u * geo.n_kst, t_o = t_p + 64u;    // scores | weights (hi, lo) | value product
 
     if (warp < 8) {
         // ================= softmax: rows 32 (warp % 4) + lane, keys 32 (warp / 4) .. + 31 of a tile =================
-        asm volatile("setmaxnreg.inc.sync.aligned.u32 184;");
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kRowRegs));
         // ---- the query tile: largest magnitude, then both terms.  Row r of the tile is head h0 + r % PK of token r / PK; a warp takes
         // eight rows at a time, a lane eight channels of one.  (The first keys are on their way meanwhile: with the tile made by all
         // warps in front of the roles, its loops unrolled, a launch of one key tile took 17 us, now 14: cold instruction fetches) ----
@@ -494,30 +510,24 @@ split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_co
                 v[4] = fmaf(w, b.x, v[4]); v[5] = fmaf(w, b.y, v[5]); v[6] = fmaf(w, b.z, v[6]); v[7] = fmaf(w, b.w, v[7]);
             }
         };
-        float q_inv, q_scale;
-        bool q_finite;
-        auto q_scaled = [&](float m) {                        // the tile's scale from all warps' largest magnitudes
-            m = warp_max_of(m);
-            if (lane == 0) s_red[warp] = m;
-            asm volatile("bar.sync 1, 256;" ::: "memory");
-#pragma unroll
-            for (int w = 0; w < 8; ++w) m = fmaxf(m, s_red[w]);
-            q_finite = m <= 3.402823466e38f;
-            q_scale = scale_of(m, q_inv);
+        float* const q_inv = row_x + 2 * kRows;               // [128] (read by a row's two threads before they exchange anything there)
+        auto q_scale = [&](float m, int row) {                // a row's scale from the four lanes that hold it
+            float inverse;
+            const float scale = scale_of(row_max(m), inverse);
+            if (lane < 8) q_inv[row] = inverse;
+            return scale;
         };
-        auto q_store = [&](int row, int ch, const float (&v)[8]) {
+        auto q_store = [&](int row, int ch, float scale, const float (&v)[8]) {
             if (ch >= chunks) return;
             uint32_t hi[4], lo[4];
 #pragma unroll
-            for (int e = 0; e < 4; ++e) split2(v[2 * e] * q_scale, v[2 * e + 1] * q_scale, hi[e], lo[e]);
+            for (int e = 0; e < 4; ++e) split2(v[2 * e] * scale, v[2 * e + 1] * scale, hi[e], lo[e]);
             const int st = geo.n_kst == 1 ? 0 : ch / wkb, w = st == geo.n_kst - 1 ? geo.wk_last : geo.wk0, c8 = ch - st * wkb;
             unsigned char* dst = qs + (size_t)st * geo.wk0 * kRows * 4 + (size_t)(((row >> 3) * (w >> 3) + c8) * 128 + (row & 7) * 16);
             *reinterpret_cast<uint4*>(dst) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
             *reinterpret_cast<uint4*>(dst + (size_t)w * kRows * 2) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
         };
-        float qm = 0.f;
         const int qrow = warp * 8 + (lane & 7), qch = lane >> 3;
-        bool made = false;
         if (!p.talk && geo.n_kst == 1) {                      // all of it fits the registers
             float4 v[8][2];
 #pragma unroll
@@ -534,23 +544,22 @@ split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_co
                     }
             }
 #pragma unroll
-            for (int i = 0; i < 8; ++i) qm = max_abs4(max_abs4(qm, v[i][0]), v[i][1]);
-            q_scaled(qm);
-            if (q_finite) {                                   // (the same for all warps)
+            for (int rg = 0; rg < 2; ++rg) {
+                float m = 0.f;
 #pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    const float x[8] = {v[i][0].x, v[i][0].y, v[i][0].z, v[i][0].w, v[i][1].x, v[i][1].y, v[i][1].z, v[i][1].w};
-                    q_store(qrow + 64 * (i >> 2), qch + 4 * (i & 3), x);
+                for (int i = 0; i < 4; ++i) m = max_finite4(max_finite4(m, v[rg * 4 + i][0]), v[rg * 4 + i][1]);
+                const float scale = q_scale(m, qrow + 64 * rg);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const float4 a = v[rg * 4 + i][0], b = v[rg * 4 + i][1];
+                    const float x[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+                    q_store(qrow + 64 * rg, qch + 4 * i, scale, x);
                 }
-                made = true;
-            } else {
-                asm volatile("bar.sync 1, 256;" ::: "memory");    // (all have read the first maxima)
-                qm = 0.f;
             }
-        }
-        if (!made) {
-            for (int pass = 0; pass < 2; ++pass) {
-                for (int rg = 0; rg < 2; ++rg)
+        } else {
+            for (int rg = 0; rg < 2; ++rg) {
+                float m = 0.f, scale = 0.f;
+                for (int pass = 0; pass < 2; ++pass) {
                     for (int ch = qch; ch < chunks; ch += 16) {
                         float v[4][8];
 #pragma unroll
@@ -559,24 +568,26 @@ split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_co
                         for (int i = 0; i < 4; ++i) {
                             if (pass == 0) {
 #pragma unroll
-                                for (int e = 0; e < 8; ++e) qm = fmaxf(qm, finite_abs(v[i][e]));
+                                for (int e = 0; e < 8; ++e) m = fmaxf(m, finite_abs(v[i][e]));
                             } else {
-                                q_store(qrow + 64 * rg, ch + 4 * i, v[i]);
+                                q_store(qrow + 64 * rg, ch + 4 * i, scale, v[i]);
                             }
                         }
                     }
-                if (pass == 0) q_scaled(qm);
+                    if (pass == 0) scale = q_scale(m, qrow + 64 * rg);
+                }
             }
         }
         fence_smem_async();
         __syncwarp();
         if (lane == 0) mbar_arrive(q_ready);
+        asm volatile("bar.sync 1, 256;" ::: "memory");          // (the rows' scales)
         const int qt = warp & 3, hf = warp >> 2, row = qt * 32 + lane, tok = row >> geo.pk_shift, h = h0 + (row & (PK - 1));
         const uint32_t lanes = (uint32_t)(qt * 32) << 16;
         const int my_pos = s_pos[tok];
         const int my_lo = first_key_of(max(my_pos, 0), p.window, p.chunk), kept = p.window > 0 ? p.keep_first : 0;
         const bool ranged = p.rows_per_slot > 0 && p.mode != 0;
-        const float mult = q_inv * p.scale * (p.temp ? p.temp[h] : 1.f), cap = p.cap, inv_cap = cap > 0.f ? 1.0f / cap : 0.f;
+        const float mult = q_inv[row] * p.scale * (p.temp ? p.temp[h] : 1.f), cap = p.cap, inv_cap = cap > 0.f ? 1.0f / cap : 0.f;
         const float slope = p.slopes ? p.slopes[h] : 0.f;
         const int half = NVS == 1 ? geo.wv0 >> 1 : 128;       // channels of this thread (NVS == 2: a whole group)
         const uint32_t t_mine = t_o + (NVS == 1 ? hf * half : hf * 128) + lanes;
@@ -584,11 +595,10 @@ split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_co
         float O[DVH];
 #pragma unroll
         for (int c = 0; c < DVH; ++c) O[c] = 0.f;
-        float m_run = -CUDART_INF_F, c_run = 0.f, l_run = 0.f, corr_prev = 1.f;
+        float m_run = -CUDART_INF_F, c_run = 0.f, l_run = 0.f, corr_prev = 1.f, wi_prev = 0.f;
         bool ok = true;
         constexpr int OW = NVS == 1 ? 32 : 16;                // columns in flight
-        auto add_values = [&](unsigned t, float corr) {       // O <- corr O + value product of tile t (which is done)
-            const float vi = v_inv[(t % kScaleRing) * 2 + (NVS == 1 ? 0 : hf)] * (1.0f / kWeightScale);
+        auto add_values = [&](unsigned t, float corr, float vi) {      // O <- corr O + vi * value product of tile t (which is done)
             const bool same = __all_sync(0xffffffffu, corr == 1.f);
             const uint32_t from = t_mine + (geo.o_bufs == 2 ? (t & 1u) * 128u : 0u);
             const float2 vi2 = make_float2(vi, vi), c2 = make_float2(corr, corr);
@@ -616,7 +626,7 @@ split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_co
             if (!wait_for(s_full, t & 1u)) { ok = false; break; }
             fence_after();
             float s[32];
-            const float* ki = k_inv + (t % kScaleRing) * kMaxKStages * 4 + hf * 2;
+            const float* ki = k_inv + (t % geo.depth) * geo.k_sets * kKeys + hf * 32;
             constexpr int SW = NVS == 1 ? 32 : 8;             // scores in flight (a wide value leaves fewer registers)
 #pragma unroll
             for (int c = 0; c < 32; c += SW) {
@@ -624,13 +634,23 @@ split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_co
                 tmem_load_n<SW>(t_s + lanes + hf * 32 + c, v);
                 tmem_loaded();
 #pragma unroll
-                for (int e = 0; e < SW; ++e) s[c + e] = v[e] * (ki[(c + e) >> 4] * mult);
+                for (int e = 0; e < SW; ++e) s[c + e] = v[e];
+                if (geo.k_sets > 1) scale_by<SW>(s + c, ki + c);
                 for (int st = 1; st < geo.n_kst; ++st) {
                     tmem_load_n<SW>(t_s + lanes + st * 64 + hf * 32 + c, v);
                     tmem_loaded();
+                    if (geo.k_sets > 1) scale_by<SW>(v, ki + st * kKeys + c);
 #pragma unroll
-                    for (int e = 0; e < SW; ++e) s[c + e] = fmaf(v[e], ki[st * 4 + ((c + e) >> 4)] * mult, s[c + e]);
+                    for (int e = 0; e < SW; ++e) s[c + e] += v[e];
                 }
+                if (geo.k_sets == 1) scale_by<SW>(s + c, ki + c);
+            }
+            const float2 mult2 = make_float2(mult, mult);
+#pragma unroll
+            for (int e = 0; e < 32; e += 2) {
+                const float2 x = mul2(make_float2(s[e], s[e + 1]), mult2);
+                s[e] = x.x;
+                s[e + 1] = x.y;
             }
             fence_before();
             __syncwarp();
@@ -671,12 +691,12 @@ split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_co
             float mx = s[0];
 #pragma unroll
             for (int e = 1; e < 32; ++e) mx = fmaxf(mx, s[e]);
-            float* xm = row_x + (t & 1u) * 2 * kRows;
-            xm[hf * kRows + row] = mx;
+            // (two exchanges a tile in two places: whoever writes one has seen the other thread leave the one before)
+            row_x[hf * kRows + row] = mx;
             __syncwarp();
             if (lane == 0) mbar_arrive(&pair[qt]);
-            if (!wait_for(&pair[qt], t & 1u)) { ok = false; break; }
-            mx = fmaxf(mx, xm[(hf ^ 1) * kRows + row]);
+            if (!wait_for(&pair[qt], 0)) { ok = false; break; }
+            mx = fmaxf(mx, row_x[(hf ^ 1) * kRows + row]);
             const float m_new = fmaxf(m_run, mx);
             const float c_new = m_new == -CUDART_INF_F ? 0.f : m_new * kLog2e;
             const float corr = m_run == -CUDART_INF_F ? 0.f : ex2(c_run - c_new);
@@ -692,12 +712,24 @@ split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_co
             l_run = fmaf(l_run, corr, sum.x + sum.y);
             m_run = m_new;
             c_run = c_new;
-            // the value product of the tile before is done: the weights' columns are free, and its sum can be taken
+            // weight x its value's magnitude, and the largest of them that this row has in the tile
+            if (!geo.shared_kv && !wait_for(&v_ready[t % geo.depth], (t / geo.depth) & 1u)) { ok = false; break; }
+            scale_by<32>(s, v_inv + (t % geo.depth) * kKeys + hf * 32);
+            float wm = s[0];
+#pragma unroll
+            for (int e = 1; e < 32; ++e) wm = fmaxf(wm, s[e]);
+            row_x[(2 + hf) * kRows + row] = wm;
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&pair[qt]);
+            // (meanwhile) the value product of the tile before is done: the weights' columns are free, and its sum can be taken
             if (t > 0) {
                 if (!wait_for(pv_done, (t - 1) & 1u)) { ok = false; break; }
                 fence_after();
             }
-            const float2 ws = make_float2(kWeightScale, kWeightScale);
+            if (!wait_for(&pair[qt], 1)) { ok = false; break; }
+            float wi;
+            const float wscale = scale_of(fmaxf(wm, row_x[(2 + (hf ^ 1)) * kRows + row]), wi);
+            const float2 ws = make_float2(wscale, wscale);
 #pragma unroll
             for (int c = 0; c < 2; ++c) {
                 uint32_t hi[8], lo[8];
@@ -710,26 +742,26 @@ split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_co
                 tmem_store8(t_p + lanes + 32 + hf * 16 + c * 8, lo);
             }
             // with two accumulators the next value product may start before the last one has been added
-            if (t > 0 && geo.o_bufs == 1) add_values(t - 1, corr_prev);
+            if (t > 0 && geo.o_bufs == 1) add_values(t - 1, corr_prev, wi_prev);
             asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
             fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(p_ready);
-            if (t > 0 && geo.o_bufs == 2) add_values(t - 1, corr_prev);
+            if (t > 0 && geo.o_bufs == 2) add_values(t - 1, corr_prev, wi_prev);
             corr_prev = corr;
+            wi_prev = wi;
         }
         if (ok && t > 0) {
             ok = wait_for(pv_done, (t - 1) & 1u);
             fence_after();
-            add_values(t - 1, corr_prev);
+            add_values(t - 1, corr_prev, wi_prev);
         }
         // ---- both threads' denominators, the sink's own term, normalise, store ----
-        float* xl = row_x + (t & 1u) * 2 * kRows;
-        xl[hf * kRows + row] = l_run;
+        row_x[hf * kRows + row] = l_run;
         __syncwarp();
         if (lane == 0) mbar_arrive(&pair[qt]);
-        ok = ok && wait_for(&pair[qt], t & 1u);
-        float l = l_run + xl[(hf ^ 1) * kRows + row];
+        ok = ok && wait_for(&pair[qt], 0);
+        float l = l_run + row_x[(hf ^ 1) * kRows + row];
         if (p.sink) l += ex2(fmaf(p.sink[h], kLog2e, -c_run));
         // through shared memory (the ring and the queries are read; 32 rows of this warp's channels): whole lines reach the output, and
         // one rolled loop serves every kind of output.  (Stored from the registers, row by row, 5500 cycles of a CTA, mostly fetching
@@ -771,10 +803,9 @@ split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_co
         }
     } else if (warp < 12) {
         // ================= keys and values: warp lw takes keys 16 lw .. + 15 of a tile, a lane one key of either eight =================
-        asm volatile("setmaxnreg.dec.sync.aligned.u32 112;");
+        if constexpr (kFetchRegs < 128) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kFetchRegs));
         const int lw = warp - 8, kin = lane & 7, cq = lane >> 3;
         unsigned at = 0;                                      // ring position
-        unsigned v_turn = 0;
         bool ok = true;
         size_t cur[2] = {~(size_t)0, ~(size_t)0}, prev[2];    // row of the two keys in the pages of kv head 0 (~0: none)
         const SlotTiles* const plan = reinterpret_cast<const SlotTiles*>(p.work);
@@ -784,35 +815,48 @@ split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_co
             const int j = j0 / kKeys;
             return j >= s.first && j < s.end ? s.base + j : j == 0 ? s.zero : -1;
         };
-        auto copied = [&](int tile, int part, unsigned bytes, float* inv, int n_inv) {    // a part that is split already
+        // a part that is split already; with scales, the tile's come along: warp 1 brings its keys' and warp 2 its values' (whose tile is t)
+        auto copied = [&](int tile, int part, unsigned bytes, bool scales, unsigned t) {
             const unsigned slot = at % geo.n_slots;
-            if (lane == 0) {
-                const unsigned char* work = reinterpret_cast<const unsigned char*>(p.work);
-                float scale = 0.f;
-                if (lw == 1) scale = *reinterpret_cast<const float*>(work + geo.scale_off + 4 * ((size_t)tile * geo.parts + part));
-                ok = wait_for(&empty[slot], ((at / geo.n_slots) & 1u) ^ 1u);
-                if (ok && lw == 0) {
-                    mbar_arrive_expect_tx(&full[slot], bytes);
-                    const size_t off = (size_t)tile * geo.tile_bytes + part_offset(geo, part);
-                    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                                     smem_u32(ring + (size_t)slot * geo.slot_bytes)),
-                                 "l"(work + geo.tile_off + off), "r"(bytes), "r"(smem_u32(&full[slot]))
-                                 : "memory");
-                } else if (ok) {
-                    if (lw == 1)
-                        for (int i = 0; i < n_inv; ++i) inv[i] = scale;
-                    mbar_arrive(&full[slot]);
-                }
-            }
+            if (lane == 0) ok = wait_for(&empty[slot], ((at / geo.n_slots) & 1u) ^ 1u);
             ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
+            if (!ok) return;
+            const unsigned char* work = reinterpret_cast<const unsigned char*>(p.work);
+            if (lw == 0 && lane == 0) {
+                mbar_arrive_expect_tx(&full[slot], bytes);
+                const size_t off = (size_t)tile * geo.tile_bytes + part_offset(geo, part);
+                asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                                 smem_u32(ring + (size_t)slot * geo.slot_bytes)),
+                             "l"(work + geo.tile_off + off), "r"(bytes), "r"(smem_u32(&full[slot]))
+                             : "memory");
+            }
+            if (scales) {
+                const float* src = reinterpret_cast<const float*>(work + geo.scale_off) + (size_t)tile * geo.sets * kKeys + 2 * lane;
+                const unsigned at_t = t % geo.depth;
+                if (lw == 1)
+                    for (int i = 0; i < geo.k_sets; ++i)
+                        *reinterpret_cast<float2*>(k_inv + (at_t * geo.k_sets + i) * kKeys + 2 * lane) =
+                            *reinterpret_cast<const float2*>(src + (geo.k_sets > 1 ? i : g) * kKeys);
+                if (lw == 2 && !geo.shared_kv)
+                    *reinterpret_cast<float2*>(v_inv + at_t * kKeys + 2 * lane) = *reinterpret_cast<const float2*>(src + (p.kv_heads + g) * kKeys);
+                __syncwarp();
+                if (lane == 0 && !geo.shared_kv) mbar_arrive(&v_ready[at_t]);
+            }
+            if (lw != 0 && lane == 0) mbar_arrive(&full[slot]);
             ++at;
         };
-        auto stage = [&](const float* cache, int width, int c0, int w, int wp, int gg, const size_t (&rows)[2], float* inv, bool value) {
+        auto row_of = [&](const float* cache, int width, int gg, size_t row) {
+            return cache + (row != ~(size_t)0 ? (row + (size_t)gg * p.page_size) * width : 0);
+        };
+        // channels [c0, c0 + w) of rows of `width` floats, of which [0, row_w) set the scale.  m_row: the rows' largest magnitudes - taken
+        // (first) or as taken by the first group; inv: where the scales go (null: they are there); ready: told when they are
+        auto stage = [&](const float* cache, int width, int row_w, int c0, int w, int wp, int gg, const size_t (&rows)[2], float (&m_row)[2],
+                         bool first, float* inv, uint64_t* ready) {
             float4 v[16];
 #pragma unroll
             for (int kg = 0; kg < 2; ++kg) {
                 const bool in = rows[kg] != ~(size_t)0;
-                const float* src = cache + (in ? (rows[kg] + (size_t)gg * p.page_size) * width + c0 : 0);
+                const float* src = row_of(cache, width, gg, rows[kg]) + c0;
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
                     const int c = 8 * (cq + 4 * i);
@@ -821,28 +865,35 @@ split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_co
                     v[kg * 8 + 2 * i + 1] = in && c + 4 < w ? *reinterpret_cast<const float4*>(src + c + 4) : z;
                 }
             }
+            if (first) {
+#pragma unroll
+                for (int kg = 0; kg < 2; ++kg) {
+                    float m = 0.f;
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) m = max_finite4(m, v[kg * 8 + i]);
+                    if (w < row_w && rows[kg] != ~(size_t)0)
+                        for (int c = w + 4 * cq; c < row_w; c += 16)
+                            m = max_finite4(m, *reinterpret_cast<const float4*>(row_of(cache, width, gg, rows[kg]) + c));
+                    m_row[kg] = row_max(m);
+                }
+            }
+            float sc[2], inverse[2];
+#pragma unroll
+            for (int kg = 0; kg < 2; ++kg) sc[kg] = scale_of(m_row[kg], inverse[kg]);
+            auto put_scales = [&] {
+                if (inv && lane < 8) {
+#pragma unroll
+                    for (int kg = 0; kg < 2; ++kg) inv[lw * 16 + kg * 8 + lane] = inverse[kg];
+                }
+            };
+            if (ready) {                                      // (their place is free by then: see geometry_of)
+                put_scales();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(ready);
+            }
             const unsigned slot = at % geo.n_slots;
             if (!wait_for(&empty[slot], ((at / geo.n_slots) & 1u) ^ 1u)) { ok = false; return; }
-            float m = 0.f;
-#pragma unroll
-            for (int i = 0; i < 16; ++i) m = max_abs4(m, v[i]);
-            m = warp_max_of(m);
-            if (!(m <= 3.402823466e38f)) {                    // an infinity among them: it stays one, the others set the scale
-                m = 0.f;
-#pragma unroll
-                for (int i = 0; i < 16; ++i) m = fmaxf(fmaxf(fmaxf(m, finite_abs(v[i].x)), finite_abs(v[i].y)), fmaxf(finite_abs(v[i].z), finite_abs(v[i].w)));
-                m = warp_max_of(m);
-            }
-            if (value) {                                      // values are summed over the tile's keys: one scale for all of them
-                float* vm = vm_s + (v_turn & 1u) * 4;
-                if (lane == 0) { vm[lw] = m; mbar_arrive(v_max); }
-                if (!wait_for(v_max, v_turn & 1u)) { ok = false; return; }
-                ++v_turn;
-                m = fmaxf(fmaxf(vm[0], vm[1]), fmaxf(vm[2], vm[3]));
-            }
-            float inverse;
-            const float sc = scale_of(m, inverse);
-            if (lane == 0 && (!value || lw == 0)) *inv = inverse;
+            if (!ready) put_scales();
             unsigned char* base = ring + (size_t)slot * geo.slot_bytes;
             const int blocks = wp >> 3;
 #pragma unroll
@@ -853,10 +904,10 @@ split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_co
                     if (c8 < blocks) {
                         const float4 a = v[kg * 8 + 2 * i], b = v[kg * 8 + 2 * i + 1];
                         uint32_t hi[4], lo[4];
-                        split2(a.x * sc, a.y * sc, hi[0], lo[0]);
-                        split2(a.z * sc, a.w * sc, hi[1], lo[1]);
-                        split2(b.x * sc, b.y * sc, hi[2], lo[2]);
-                        split2(b.z * sc, b.w * sc, hi[3], lo[3]);
+                        split2(a.x * sc[kg], a.y * sc[kg], hi[0], lo[0]);
+                        split2(a.z * sc[kg], a.w * sc[kg], hi[1], lo[1]);
+                        split2(b.x * sc[kg], b.y * sc[kg], hi[2], lo[2]);
+                        split2(b.z * sc[kg], b.w * sc[kg], hi[3], lo[3]);
                         unsigned char* dst = base + ((lw * 2 + kg) * blocks + c8) * 128 + kin * 16;
                         *reinterpret_cast<uint4*>(dst) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
                         *reinterpret_cast<uint4*>(dst + kKeys * wp * 2) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
@@ -867,17 +918,21 @@ split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_co
             if (lane == 0) mbar_arrive(&full[slot]);
             ++at;
         };
-        auto values = [&](unsigned t, const size_t (&rows)[2], int tile) {
+        // the value groups of tile t; a shared row's scale is its key's, m_key
+        auto values = [&](unsigned t, const size_t (&rows)[2], int tile, const float (&m_key)[2]) {
+            float m_row[2] = {m_key[0], m_key[1]};
             for (int vs = 0; vs < NVS && ok; ++vs) {
                 const int wl = vs == geo.n_vst - 1 ? geo.v_last_layout : geo.v0_layout;
-                float* inv = v_inv + (t % kScaleRing) * 2 + vs;
+                const bool owns = vs == 0 && !geo.shared_kv;
                 if (tile >= 0)
-                    copied(tile, geo.shared_kv ? vs : geo.k_parts + g * geo.n_vst + vs, kKeys * wl * 4, inv, 1);
+                    copied(tile, geo.shared_kv ? vs : geo.k_parts + g * geo.n_vst + vs, kKeys * wl * 4, false, t);
                 else
-                    stage(p.vcache, p.vrow, vs * kGroupW, min(kGroupW, (geo.shared_kv ? p.kdim : p.vdim) - vs * kGroupW), wl, g, rows, inv, true);
+                    stage(p.vcache, p.vrow, p.vdim, vs * kGroupW, min(kGroupW, (geo.shared_kv ? p.kdim : p.vdim) - vs * kGroupW), wl, g, rows, m_row, owns,
+                          owns ? v_inv + (t % geo.depth) * kKeys : nullptr, owns ? &v_ready[t % geo.depth] : nullptr);
             }
         };
         int tile = -1, prev_tile = -1;
+        float m_key[2] = {0.f, 0.f}, m_prev[2];
         unsigned t = 0;
         Walk w(s_slot, s_pos, s_breaks, n_tok);
         for (; ok && w.next(p); ++t) {
@@ -894,18 +949,20 @@ split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_co
                     cur[kg] = (size_t)page * p.kv_heads * p.page_size + (p.table ? j % p.page_size : j);
                 }
             }
+            m_prev[0] = m_key[0];
+            m_prev[1] = m_key[1];
             for (int st = 0; st < geo.n_kst && ok; ++st) {
                 const int wp = st == geo.n_kst - 1 ? geo.wk_last : geo.wk0;
-                float* inv = k_inv + ((t % kScaleRing) * kMaxKStages + st) * 4;
+                const bool first = st == 0 || geo.k_sets > 1;
                 if (tile >= 0)
-                    copied(tile, p.talk ? st : g * geo.n_kst + st, kKeys * wp * 4, inv, 4);
+                    copied(tile, p.talk ? st : g * geo.n_kst + st, kKeys * wp * 4, st == 0, t);
                 else
-                    stage(p.kcache, p.kdim, p.talk ? 0 : st * kGroupW, p.talk ? p.kdim : min(kGroupW, p.kdim - st * kGroupW), wp, p.talk ? st : g, cur,
-                          inv + lw, false);
+                    stage(p.kcache, p.kdim, p.kdim, p.talk ? 0 : st * kGroupW, p.talk ? p.kdim : min(kGroupW, p.kdim - st * kGroupW), wp, p.talk ? st : g,
+                          cur, m_key, first, first ? k_inv + ((t % geo.depth) * geo.k_sets + (geo.k_sets > 1 ? st : 0)) * kKeys : nullptr, nullptr);
             }
-            if (t > 0 && ok) values(t - 1, prev, prev_tile);
+            if (t > 0 && ok) values(t - 1, prev, prev_tile, m_prev);
         }
-        if (t > 0 && ok) values(t - 1, cur, tile);
+        if (t > 0 && ok) values(t - 1, cur, tile, m_key);
     } else {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 32;");
         if (warp == 12) {
@@ -1013,32 +1070,43 @@ bool geometry_of(const SplitAttention& a, Geometry& g, size_t& smem) {
     const int k_heads = a.talk ? 1 : a.kv_heads;              // (a mixed score's key groups are all kv heads)
     g.k_parts = k_heads * g.n_kst;
     g.parts = g.k_parts + (g.shared_kv ? 0 : a.kv_heads * g.n_vst);
+    g.k_sets = a.talk ? a.kv_heads : 1;
+    g.sets = a.kv_heads * (g.shared_kv ? 1 : 2);
     g.tile_bytes = kKeys * 4u * (k_heads * ((g.n_kst - 1) * g.wk0 + g.wk_last) + (g.shared_kv ? 0 : a.kv_heads * ((g.n_vst - 1) * g.wv0 + g.wv_last)));
     g.cap_tiles = 0;
     if (a.work && a.table && a.rows_per_slot <= 0 && a.n_seq > 0 && aligned(a.work)) {
         g.scale_off = (unsigned)a.n_slots * sizeof(SlotTiles);
-        const size_t per = g.tile_bytes + 4u * g.parts, fixed = g.scale_off + 128;
+        const size_t per = g.tile_bytes + 4u * kKeys * g.sets, fixed = g.scale_off + 128;
         if (a.work_bytes > fixed) g.cap_tiles = (int)std::min<size_t>((a.work_bytes - fixed) / per, 65535);
-        g.tile_off = (unsigned)((g.scale_off + 4u * g.parts * (unsigned)g.cap_tiles + 127u) & ~127u);
+        g.tile_off = (unsigned)((g.scale_off + 4u * kKeys * g.sets * (unsigned)g.cap_tiles + 127u) & ~127u);
     }
     g.o_bufs = g.n_vst == 1 && 64 * g.n_kst + 64 + 256 <= 512 ? 2 : 1;
     g.slot_bytes = kKeys * std::max(g.wk0, std::max(g.wv0, g.v0_layout)) * 4;
     g.q_bytes = ((g.n_kst - 1) * g.wk0 + g.wk_last) * kRows * 4;
-    const int control = (2 * kMaxSlots + 6 + 4) * 8 + (kScaleRing * kMaxKStages * 4 + kScaleRing * 2 + 8 + 4 * kRows) * 4 + 2 * (kRows >> g.pk_shift) * 4;
-    g.n_slots = (kSmemMost - kStaticMost - g.q_bytes - control) / g.slot_bytes;
+    // A tile's scales are written when its first key group has its slot: the stage n_slots places before is done.  They lie depth tiles
+    // apart so that this stage is no earlier than the first value group of the tile whose scales were there (a value group is multiplied
+    // after the rows have used all scales of its tile).  In order, a tile is n_kst key groups and, behind those of the next, n_vst value groups.
+    const int per_tile = g.n_kst + g.n_vst;
+    auto depth_of = [&](int slots) { return 1 + (slots + g.n_kst + per_tile - 1) / per_tile; };
+    auto control_of = [&](int slots) {
+        return (2 * kMaxSlots + 5 + 4 + kMaxDepth + 1) / 2 * 16 + (depth_of(slots) * kKeys * (g.k_sets + (g.shared_kv ? 0 : 1)) + 4 * kRows + 8) * 4 + 2 * (kRows >> g.pk_shift) * 4;
+    };
+    for (g.n_slots = kMaxSlots; g.n_slots >= 2; --g.n_slots)
+        if (g.n_slots * g.slot_bytes + g.q_bytes + control_of(g.n_slots) <= kSmemMost) break;
     if (g.n_slots < 2) return false;
-    g.n_slots = std::min(g.n_slots, kMaxSlots);
+    g.depth = depth_of(g.n_slots);
+    const int control = control_of(g.n_slots);
     // the output is staged in the ring and the queries: 8 warps of 32 rows, 4 floats between the rows
     const int staged = kRows * 2 * (g.n_vst == 1 ? g.wv0 / 2 + 4 : 128 + 4) * 4;
     g.q_bytes = std::max(g.q_bytes, staged - g.n_slots * g.slot_bytes);
     smem = (size_t)g.n_slots * g.slot_bytes + g.q_bytes + control;
-    return smem <= (size_t)(kSmemMost - kStaticMost);
+    return smem <= (size_t)kSmemMost;
 }
 
 template <int NVS>
 cudaError_t launch_inst(const SplitAttention& a, const Geometry& g, size_t smem, cudaStream_t st) {
     // (the same size for every launch: another thread's cannot lower what this one needs)
-    const cudaError_t e = cudaFuncSetAttribute(split_attention_kernel<NVS>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMost - kStaticMost);
+    const cudaError_t e = cudaFuncSetAttribute(split_attention_kernel<NVS>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMost);
     if (e != cudaSuccess) return e;
     const int tt = kRows >> g.pk_shift, tiles = a.n_seq > 1 ? a.M / tt + a.n_seq : (a.M + tt - 1) / tt;
     if (tiles > 65535) return cudaErrorNotSupported;
@@ -1059,7 +1127,7 @@ size_t split_attention_work_bytes(const SplitAttention& a, int keys) {
     Geometry g;
     size_t smem;
     if (!geometry_of(a, g, smem)) return 0;
-    return (size_t)a.n_slots * sizeof(SlotTiles) + 256 + (size_t)((keys + kKeys - 1) / kKeys) * (g.tile_bytes + 4u * g.parts);
+    return (size_t)a.n_slots * sizeof(SlotTiles) + 256 + (size_t)((keys + kKeys - 1) / kKeys) * (g.tile_bytes + 4u * kKeys * g.sets);
 }
 
 cudaError_t launch_split_attention(const SplitAttention& a, cudaStream_t st) {

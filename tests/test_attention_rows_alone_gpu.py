@@ -1,0 +1,135 @@
+"""The tensor-core attention (csrc/attention_split.cu) gives a row what the row and the tokens that it sees make of it: magnitudes far apart
+inside a tile, and the same bits however a prompt is cut and whatever shares the step."""
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def reference(q, k, v, see):
+    """softmax(q k / sqrt(d)) v in 64 bits; q [T, H, d], k / v [G, T, d], see [T, T]"""
+    H, G = q.shape[1], k.shape[0]
+    k, v = k.double().repeat_interleave(H // G, 0), v.double().repeat_interleave(H // G, 0)
+    s = (torch.einsum("ihd,hjd->hij", q.double(), k) * q.shape[-1] ** -0.5).masked_fill(~see, -torch.inf)
+    return torch.einsum("hij,hjd->ihd", torch.softmax(s, -1), v)
+
+
+def spiked(what, factor, at=200, T=300):
+    """One utterance whose token ``at`` is larger by ``factor``; a value's token has a weight of about e^-60 where it is seen."""
+    g = torch.Generator().manual_seed(7)
+    q, k, v = torch.randn(1, T, 4, 128, generator=g), torch.randn(1, 2, T, 128, generator=g), torch.randn(1, 2, T, 128, generator=g)
+    if what == "faint":
+        q[..., 0], k[:, :, at, :] = 8.0, 0.0
+        k[:, :, at, 0] = -85.0
+    plain = [t.clone() for t in (q, k, v)]
+    if what == "query":
+        q[:, at] *= factor
+    elif what == "key":
+        k[:, :, at] *= factor
+    else:
+        v[:, :, at] *= factor
+    return (q, k, v), plain
+
+
+@pytest.mark.parametrize("what,factor", [(w, f) for w in ("query", "value", "faint") for f in (1e6, 1e9, 1e12)] + [("key", 1e6)])
+def test_a_token_far_larger_than_its_neighbours(what, factor):
+    """Rows in front of the large token do not see it: the same bits as without it.  Every row's error is measured against the row's own
+    largest output: 22-bit factors and fp32 sums, 2^-21 of a score of at most about 8 and of the largest weight x value that it sees, a
+    few times over."""
+    from dia_tts_prune_b200 import engine as E
+    (q, k, v), plain = spiked(what, factor)
+    T, see = q.shape[1], torch.ones(q.shape[1], q.shape[1]).tril().bool()
+    got = E.attention_rows(q.cuda(), k.cuda(), v.cuda(), T, 0, None).cpu()
+    base = E.attention_rows(*[t.cuda() for t in plain], T, 0, None).cpu()
+    assert torch.equal(got[:, :200], base[:, :200])
+    ref = reference(q[0], k[0], v[0], see)
+    top = ref.abs().amax(-1, keepdim=True)
+    # (a score of a large query or key has an error of its own size: where it decides between two keys there is nothing to hold the row to)
+    rows = torch.ones(T, dtype=torch.bool)
+    if what == "query":
+        rows[200] = False
+    err = ((got[0].double() - ref).abs() / top)[rows]
+    assert err.max() <= 2e-5, err.max()
+
+
+@pytest.mark.parametrize("mode", [0, 2])
+def test_one_utterance_does_not_set_the_scale_of_another(mode):
+    from dia_tts_prune_b200 import engine as E
+    g = torch.Generator().manual_seed(8)
+    q, k, v = torch.randn(2, 257, 4, 128, generator=g), torch.randn(2, 2, 257, 128, generator=g), torch.randn(2, 2, 257, 128, generator=g)
+    one = E.attention_rows(q.cuda(), k.cuda(), v.cuda(), 257, mode, [130, 257]).cpu()
+    q[1], k[1], v[1] = q[1] * 1e9, k[1] * 1e-9, v[1] * 1e9
+    two = E.attention_rows(q.cuda(), k.cuda(), v.cuda(), 257, mode, [130, 257]).cpu()
+    assert torch.equal(one[0], two[0])
+
+
+def cuts(n, parts):
+    assert sum(parts) == n
+    at = [sum(parts[:i]) for i in range(len(parts))]
+    return [(a, a + p) for a, p in zip(at, parts)]
+
+
+def grouped(heads, kv_heads, dim, window, keep, cap, page):
+    from dia_tts_prune_b200 import synthetic as SY
+    from dia_tts_prune_b200.lm_config import PubopelConfig
+    from dia_tts_prune_b200.lm_model import CausalLM
+    cfg = SY.pubopel_config(width=32, layers=1, heads=heads, kv_heads=kv_heads, dim=dim, experts=1, top=1, expert_ff=8, shared_ff=None, vocab=64,
+                            window=window or None, keep_first=keep, softcap=cap or None)
+    model = CausalLM(PubopelConfig.model_validate(cfg), SY.pubopel_weights(cfg, 3), dtype="bfloat16", device="cuda:0", max_tokens=4096,
+                     max_sequences=6, page_size=page, max_rows=1024)
+    return model, (heads + kv_heads) * dim, lambda x, parts: model.engine.op_attention(0, x.clone(), parts)
+
+
+def mixed(heads, kv_heads, dim, vdim):
+    from dia_tts_prune_b200 import synthetic as SY
+    from dia_tts_prune_b200.lm_config import KupelixConfig
+    from dia_tts_prune_b200.lm_model import CausalLM
+    cfg = SY.kupelix_config(width=32, kinds=["attention"], heads=heads, kv_heads=kv_heads, dim=dim, vdim=vdim, ff=8, vocab=64)
+    w = SY.kupelix_weights(cfg, 3)
+    cfg["layers"][0]["mlp"] = None
+    model = CausalLM(KupelixConfig.model_validate(cfg), w, dtype="bfloat16", device="cuda:0", max_tokens=4096, max_sequences=6, max_rows=1024)
+    return model, model.layers[0].layer.n_in, lambda x, parts: model.engine.op_mixer_kernels(0, x.clone(), parts)
+
+
+def latent(heads, dim, kv_rank, rot_dim, vdim, window):
+    from dia_tts_prune_b200 import synthetic as SY
+    from dia_tts_prune_b200.lm_config import FipadraConfig
+    from dia_tts_prune_b200.lm_model import CausalLM
+    cfg = SY.fipadra_config(width=64, kinds=["latent_attention"], heads=heads, dim=dim, rot_dim=rot_dim, vdim=vdim, q_rank=72, kv_rank=kv_rank,
+                            window=window, vocab=64)
+    cfg["layers"][0]["mlp"] = None
+    w = SY.fipadra_weights(cfg, 3)
+    model = CausalLM(FipadraConfig.model_validate(cfg), w, dtype="float32", device="cuda:0", max_tokens=4096, max_sequences=6, max_rows=1024)
+    return model, 64, lambda x, parts: model.engine.op_mixer(0, x.clone(), parts)
+
+
+@pytest.mark.parametrize("make,args", [(grouped, (4, 2, 64, 0, 0, 0.0, 64)), (grouped, (8, 1, 128, 100, 3, 0.0, 16)), (grouped, (2, 1, 200, 0, 0, 0.0, 7)),
+                                       (mixed, (8, 2, 64, 128)), (latent, (4, 32, 192, 16, 64, 0)), (latent, (2, 16, 40, 8, 16, 90))])
+def test_a_row_has_the_same_bits_in_any_step(make, args):
+    """A prompt of 300 rows in one step, in portions of more than 8 rows, and beside other sequences whose tokens are larger: with few rows the
+    row tiles split the keys themselves, with many a launch in front does it."""
+    model, n_in, op = make(*args)
+    g = torch.Generator().manual_seed(9)
+    x, other = torch.randn(300, n_in, generator=g).cuda(), (1000 * torch.randn(400, n_in, generator=g)).cuda()
+
+    def run(parts, beside):
+        seq = model.state.open("a")
+        model.state.reserve(seq, 300)
+        out = []
+        for i, (a, b) in enumerate(cuts(300, parts)):
+            rows, h = [(seq, b - a, a)], x[a:b]
+            if beside:
+                o = model.state.open(f"o{i}")
+                model.state.reserve(o, beside)
+                rows, h = [(o, beside, 0), *rows], torch.cat([other[:beside], h])
+            y = op(h, rows)
+            out.append((y[0] if isinstance(y, (tuple, list)) else y)[-(b - a):].clone())
+            if beside:
+                model.state.close(f"o{i}")
+        model.state.close("a")
+        return torch.cat(out)
+
+    whole = run([300], 0)
+    for parts, beside in (([100, 9, 191], 0), ([300], 33), ([9, 9, 60, 222], 400)):
+        assert torch.equal(whole, run(parts, beside)), (parts, beside)
