@@ -105,7 +105,7 @@ def load(build_if_missing: bool = True) -> C.CDLL:
     if _lib is not None:
         return _lib
     path = _build.LIB
-    override = os.environ.get("DIA_B200_LIB")            # A/B timing of two builds on one box (tools/ab.sh)
+    override = os.environ.get("DIA_B200_LIB")            # A/B timing of two builds on one box
     if override:
         path, build_if_missing = Path(override), False
     if build_if_missing and _build.is_stale():

@@ -1,5 +1,5 @@
 #!/usr/bin/env python
-"""Turn the outputs of tools/ncu_bench.sh (gpurun_out/launches_<tag>.csv, gpurun_out/step_<tag>_full.ncu-rep and, when
+"""Turn the outputs of tools/ncu_bench.sh ($OUT/launches_<tag>.csv, $OUT/step_<tag>_full.ncu-rep and, when
 present, batch_<tag>_full.ncu-rep / gemm_<tag>_full.ncu-rep) into the committed summaries under profiles/: the launch list
 (shares), the metrics of the full captures and
 step_kernel_traffic.json (read by bench.py for roofline.traffic).
@@ -14,7 +14,7 @@ import os
 import subprocess
 
 REPO = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
-OUT = os.path.join(REPO, "gpurun_out")
+OUT = os.environ.get("OUT", os.path.join(REPO, "ncu_out"))
 PROF = os.path.join(REPO, "profiles")
 
 METRICS = ["gpu__time_duration.sum", "dram__bytes_read.sum", "dram__bytes_write.sum", "dram__bytes_read.sum.per_second",
