@@ -587,15 +587,17 @@ split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_co
         const int my_pos = s_pos[tok];
         const int my_lo = first_key_of(max(my_pos, 0), p.window, p.chunk), kept = p.window > 0 ? p.keep_first : 0;
         const bool ranged = p.rows_per_slot > 0 && p.mode != 0;
-        const float mult = q_inv[row] * p.scale * (p.temp ? p.temp[h] : 1.f), cap = p.cap, inv_cap = cap > 0.f ? 1.0f / cap : 0.f;
-        const float slope = p.slopes ? p.slopes[h] : 0.f;
+        // scores and maxima are in units of log 2 (a capped score from its cap on): the largest score's weight is exactly 1 at any magnitude
+        const float cap = p.cap, inv_cap = cap > 0.f ? 1.0f / cap : 0.f;
+        const float mult = q_inv[row] * p.scale * (p.temp ? p.temp[h] : 1.f) * (cap > 0.f ? 1.f : kLog2e);
+        const float slope = p.slopes ? p.slopes[h] * kLog2e : 0.f;
         const int half = NVS == 1 ? geo.wv0 >> 1 : 128;       // channels of this thread (NVS == 2: a whole group)
         const uint32_t t_mine = t_o + (NVS == 1 ? hf * half : hf * 128) + lanes;
         const int n_mine = NVS == 1 ? half : (hf ? geo.wv_last : geo.wv0);
         float O[DVH];
 #pragma unroll
         for (int c = 0; c < DVH; ++c) O[c] = 0.f;
-        float m_run = -CUDART_INF_F, c_run = 0.f, l_run = 0.f, corr_prev = 1.f, wi_prev = 0.f;
+        float m_run = -CUDART_INF_F, l_run = 0.f, corr_prev = 1.f, wi_prev = 0.f;
         bool ok = true;
         constexpr int OW = NVS == 1 ? 32 : 16;                // columns in flight
         auto add_values = [&](unsigned t, float corr, float vi) {      // O <- corr O + vi * value product of tile t (which is done)
@@ -662,7 +664,7 @@ split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_co
 #pragma unroll
                 for (int e = 0; e < 32; ++e) big = fmaxf(big, fabsf(s[e]));
                 if (__all_sync(0xffffffffu, big * inv_cap <= kTanhRange)) {
-                    const float2 ic = make_float2(inv_cap, inv_cap), cc = make_float2(cap, cap);
+                    const float2 ic = make_float2(inv_cap, inv_cap), cc = make_float2(cap * kLog2e, cap * kLog2e);
 #pragma unroll
                     for (int e = 0; e < 32; e += 2) {
                         const float2 r = mul2(tanh_near_zero(mul2(make_float2(s[e], s[e + 1]), ic)), cc);
@@ -671,7 +673,7 @@ split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_co
                     }
                 } else {
 #pragma unroll
-                    for (int e = 0; e < 32; ++e) s[e] = cap * tanhf(s[e] * inv_cap);
+                    for (int e = 0; e < 32; ++e) s[e] = cap * kLog2e * tanhf(s[e] * inv_cap);
                 }
             }
             if (p.slopes) {
@@ -698,20 +700,18 @@ split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_co
             if (!wait_for(&pair[qt], 0)) { ok = false; break; }
             mx = fmaxf(mx, row_x[(hf ^ 1) * kRows + row]);
             const float m_new = fmaxf(m_run, mx);
-            const float c_new = m_new == -CUDART_INF_F ? 0.f : m_new * kLog2e;
-            const float corr = m_run == -CUDART_INF_F ? 0.f : ex2(c_run - c_new);
+            const float base = m_new == -CUDART_INF_F ? 0.f : m_new, corr = m_run == -CUDART_INF_F ? 0.f : ex2(m_run - base);
             float2 sum = make_float2(0.f, 0.f);
-            const float2 l2 = make_float2(kLog2e, kLog2e), nc = make_float2(-c_new, -c_new);
+            const float2 nb = make_float2(-base, -base);
 #pragma unroll
             for (int e = 0; e < 32; e += 2) {
-                const float2 a = fma2(make_float2(s[e], s[e + 1]), l2, nc);
+                const float2 a = add2(make_float2(s[e], s[e + 1]), nb);
                 s[e] = ex2(a.x);
                 s[e + 1] = ex2(a.y);
                 sum = add2(sum, make_float2(s[e], s[e + 1]));
             }
             l_run = fmaf(l_run, corr, sum.x + sum.y);
             m_run = m_new;
-            c_run = c_new;
             // weight x its value's magnitude, and the largest of them that this row has in the tile
             if (!geo.shared_kv && !wait_for(&v_ready[t % geo.depth], (t / geo.depth) & 1u)) { ok = false; break; }
             scale_by<32>(s, v_inv + (t % geo.depth) * kKeys + hf * 32);
@@ -762,7 +762,7 @@ split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_co
         if (lane == 0) mbar_arrive(&pair[qt]);
         ok = ok && wait_for(&pair[qt], 0);
         float l = l_run + row_x[(hf ^ 1) * kRows + row];
-        if (p.sink) l += ex2(fmaf(p.sink[h], kLog2e, -c_run));
+        if (p.sink) l += ex2(fmaf(p.sink[h], kLog2e, m_run == -CUDART_INF_F ? 0.f : -m_run));
         // through shared memory (the ring and the queries are read; 32 rows of this warp's channels): whole lines reach the output, and
         // one rolled loop serves every kind of output.  (Stored from the registers, row by row, 5500 cycles of a CTA, mostly fetching
         // the unrolled code; 3500 now)

@@ -32,7 +32,7 @@ def spiked(what, factor, at=200, T=300):
     return (q, k, v), plain
 
 
-@pytest.mark.parametrize("what,factor", [(w, f) for w in ("query", "value", "faint") for f in (1e6, 1e9, 1e12)] + [("key", 1e6)])
+@pytest.mark.parametrize("what,factor", [(w, f) for w in ("query", "key", "value", "faint") for f in (1e6, 1e9, 1e12)])
 def test_a_token_far_larger_than_its_neighbours(what, factor):
     """Rows in front of the large token do not see it: the same bits as without it.  Every row's error is measured against the row's own
     largest output: 22-bit factors and fp32 sums, 2^-21 of a score of at most about 8 and of the largest weight x value that it sees, a
