@@ -663,8 +663,9 @@ split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_co
                 float big = 0.f;
 #pragma unroll
                 for (int e = 0; e < 32; ++e) big = fmaxf(big, fabsf(s[e]));
+                // each score takes the form that its own magnitude asks for; whether all of them are near zero decides the speed only
+                const float2 ic = make_float2(inv_cap, inv_cap), cc = make_float2(cap * kLog2e, cap * kLog2e);
                 if (__all_sync(0xffffffffu, big * inv_cap <= kTanhRange)) {
-                    const float2 ic = make_float2(inv_cap, inv_cap), cc = make_float2(cap * kLog2e, cap * kLog2e);
 #pragma unroll
                     for (int e = 0; e < 32; e += 2) {
                         const float2 r = mul2(tanh_near_zero(mul2(make_float2(s[e], s[e + 1]), ic)), cc);
@@ -673,7 +674,15 @@ split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_co
                     }
                 } else {
 #pragma unroll
-                    for (int e = 0; e < 32; ++e) s[e] = cap * kLog2e * tanhf(s[e] * inv_cap);
+                    for (int e = 0; e < 32; e += 2) {
+                        const float2 x = mul2(make_float2(s[e], s[e + 1]), ic);
+                        float2 r = tanh_near_zero(x);
+                        if (!(fabsf(x.x) <= kTanhRange)) r.x = tanhf(x.x);
+                        if (!(fabsf(x.y) <= kTanhRange)) r.y = tanhf(x.y);
+                        r = mul2(r, cc);
+                        s[e] = r.x;
+                        s[e + 1] = r.y;
+                    }
                 }
             }
             if (p.slopes) {

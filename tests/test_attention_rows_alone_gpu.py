@@ -105,6 +105,7 @@ def latent(heads, dim, kv_rank, rot_dim, vdim, window):
 
 
 @pytest.mark.parametrize("make,args", [(grouped, (4, 2, 64, 0, 0, 0.0, 64)), (grouped, (8, 1, 128, 100, 3, 0.0, 16)), (grouped, (2, 1, 200, 0, 0, 0.0, 7)),
+                                       (grouped, (4, 2, 64, 0, 0, 4.0, 64)), (grouped, (2, 1, 200, 100, 3, 2.0, 16)),    # scores on both sides of the polynomial's range
                                        (mixed, (8, 2, 64, 128)), (latent, (4, 32, 192, 16, 64, 0)), (latent, (2, 16, 40, 8, 16, 90))])
 def test_a_row_has_the_same_bits_in_any_step(make, args):
     """A prompt of 300 rows in one step, in portions of more than 8 rows, and beside other sequences whose tokens are larger: with few rows the
