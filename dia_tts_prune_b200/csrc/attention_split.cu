@@ -200,14 +200,32 @@ __device__ __forceinline__ float scale_of(float m, float& inverse) {
     inverse = __uint_as_float((uint32_t)(e + 113) << 23);
     return __uint_as_float((uint32_t)(min(141 - e, 254)) << 23);
 }
-__device__ __forceinline__ float finite_abs(float x) { const float a = fabsf(x); return a <= 3.402823466e38f ? a : 0.f; }
-__device__ __forceinline__ float max_finite4(float m, const float4& v) {
-    return fmaxf(fmaxf(fmaxf(m, finite_abs(v.x)), finite_abs(v.y)), fmaxf(finite_abs(v.z), finite_abs(v.w)));
+constexpr float kFloatMost = 3.402823466e38f;
+__device__ __forceinline__ float max_nan(float a, float b) {  // (fmaxf drops a NaN)
+    float m;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(m) : "f"(a), "f"(b));
+    return m;
+}
+__device__ __forceinline__ float warp_max_nan(float v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v = max_nan(v, __shfl_xor_sync(0xffffffffu, v, o));
+    return v;
+}
+__device__ __forceinline__ float max_abs4(float m, const float4& v) {
+    return max_nan(max_nan(max_nan(max_nan(m, fabsf(v.x)), fabsf(v.y)), fabsf(v.z)), fabsf(v.w));
 }
 // lanes 8 apart hold the channels of one row
 __device__ __forceinline__ float row_max(float v) {
-    v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, 8));
-    return fmaxf(v, __shfl_xor_sync(0xffffffffu, v, 16));
+    v = max_nan(v, __shfl_xor_sync(0xffffffffu, v, 8));
+    return max_nan(v, __shfl_xor_sync(0xffffffffu, v, 16));
+}
+// A row with an infinity or a NaN cannot be split: its terms are zeros (true), and its inverse scale is NaN, which makes the scores, or the
+// weights, of those that see it NaN and nobody else's; they are computed once more by plain_row.
+__device__ __forceinline__ bool scale_row(float m, float& scale, float& inverse) {
+    scale = scale_of(m, inverse);
+    const bool bad = !(m <= kFloatMost);
+    if (bad) inverse = CUDART_NAN_F;
+    return bad;
 }
 __device__ __forceinline__ int first_key_of(int i, int window, int chunk) {
     const int w = window > 0 ? max(0, i - window + 1) : 0;
@@ -299,12 +317,14 @@ split_keys_kernel(const __grid_constant__ SplitAttention p, const __grid_constan
     // the scale is that of the whole row (a latent's value is a part of its key row)
     const int row_w = is_v ? p.vdim : p.kdim;
 #pragma unroll
-    for (int i = 0; i < 8; ++i) m = max_finite4(m, v[i]);
+    for (int i = 0; i < 8; ++i) m = max_abs4(m, v[i]);
     if (w < row_w && in)
-        for (int c = 4 * cq; c < row_w; c += 16) m = max_finite4(m, *reinterpret_cast<const float4*>(src + c));
-    m = row_max(m);
-    float inverse;
-    const float sc = scale_of(m, inverse);
+        for (int c = 4 * cq; c < row_w; c += 16) m = max_abs4(m, *reinterpret_cast<const float4*>(src + c));
+    float sc, inverse;
+    if (scale_row(row_max(m), sc, inverse)) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
     unsigned char* work = reinterpret_cast<unsigned char*>(p.work);
     const int set = is_v ? p.kv_heads + gg : talk ? st : gg;
     if (cq == 0 && (talk || st == 0))
@@ -372,6 +392,75 @@ struct Walk {
         }
     }
 };
+
+// Row r (position pos of a slot's sequence), head h, in plain fp32, for a row whose sum is NaN: one that sees an infinity or a NaN, or has one
+// in its query.  As the row kernels have it: a key that is not seen does not enter, an infinity or a NaN counts in the channels where it is.
+// One warp; channels c0 .. c0 + n - 1 (at most 128) to dst, in front of the gate.
+__device__ __noinline__ void plain_row(const SplitAttention& p, int r, int slot, int pos, int h, int c0, int n, float* dst) {
+    const int lane = threadIdx.x & 31, rep = p.heads / p.kv_heads;
+    const bool ranged = p.rows_per_slot > 0;
+    const int nv = ranged ? p.n_valid[slot] : 0;
+    int lo = 0, end = pos + 1, kept = 0;
+    if (ranged && p.mode != 0) {
+        const bool tail = p.mode == 1 && pos >= nv;
+        lo = tail ? nv : 0;
+        end = tail ? p.n_keys : min(nv, p.n_keys);
+    } else {
+        lo = first_key_of(pos, p.window, p.chunk);
+        kept = p.window > 0 ? min(p.keep_first, lo) : 0;
+        if (ranged) end = min(end, p.n_keys);
+    }
+    auto row_at = [&](int j, int g) {
+        const int page = p.table ? p.table[(size_t)slot * p.max_pages + j / p.page_size] : slot;
+        return ((size_t)page * p.kv_heads + g) * p.page_size + (p.table ? j % p.page_size : j);
+    };
+    auto dot = [&](int head, int j) {
+        const float* q = p.q + (size_t)r * p.ldq + (size_t)head * p.qdim;
+        const float* k = p.kcache + row_at(j, head / rep) * p.kdim;
+        float s = 0.f;
+        for (int c = 0; c < p.kdim; ++c) s = fmaf(q[c], k[c], s);
+        return s;
+    };
+    float m = p.sink ? p.sink[h] : -CUDART_INF_F, l = 0.f, o[4] = {0.f, 0.f, 0.f, 0.f};
+    for (int part = 0; part < 2; ++part) {
+        const int a = part == 0 ? 0 : lo, b = part == 0 ? kept : end;
+        for (int j0 = a; j0 < b; j0 += 32) {
+            const int j = j0 + lane;
+            float s = -CUDART_INF_F;
+            if (j < b) {
+                if (p.talk) {
+                    s = 0.f;
+                    for (int t = 0; t < p.heads; ++t) s = fmaf(p.talk[(size_t)h * p.heads + t], dot(t, j), s);
+                    s *= p.scale;
+                } else {
+                    s = dot(h, j) * (p.scale * (p.temp ? p.temp[h] : 1.f));
+                }
+                if (p.cap > 0.f) s = p.cap * tanhf(s / p.cap);
+                if (p.slopes) s -= p.slopes[h] * (float)(pos - j);
+            }
+            const float m_new = max_nan(m, warp_max_nan(s));
+            const bool none = m_new == -CUDART_INF_F;
+            const float e = j < b && !none ? expf(s - m_new) : 0.f, corr = none ? 1.f : expf(m - m_new);
+            l = l * corr + warp_sum(e);
+            m = m_new;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) o[i] *= corr;
+            for (int i = 0; i < min(32, b - j0); ++i) {
+                const float w = __shfl_sync(0xffffffffu, e, i);
+                const float* v = p.vcache + row_at(j0 + i, h / rep) * p.vrow + c0;
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+                    if (lane + 32 * u < n) o[u] = fmaf(w, v[lane + 32 * u], o[u]);
+            }
+        }
+    }
+    if (p.sink) l += expf(p.sink[h] - m);
+    float f = l > 0.f ? p.out_scale / l : 0.f;
+    if (p.head_gate) f *= p.head_gate[(size_t)r * p.ldg + h];
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+        if (lane + 32 * u < n) dst[lane + 32 * u] = o[u] * f;
+}
 
 // NVS: channel groups of a value (1: up to 128 channels, a thread of a row keeps half of them; 2: up to 256, a group each)
 template <int NVS>
@@ -511,17 +600,17 @@ split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_co
             }
         };
         float* const q_inv = row_x + 2 * kRows;               // [128] (read by a row's two threads before they exchange anything there)
-        auto q_scale = [&](float m, int row) {                // a row's scale from the four lanes that hold it
-            float inverse;
-            const float scale = scale_of(row_max(m), inverse);
+        auto q_scale = [&](float m, int row, bool& bad) {     // a row's scale from the four lanes that hold it
+            float scale, inverse;
+            bad = scale_row(row_max(m), scale, inverse);
             if (lane < 8) q_inv[row] = inverse;
             return scale;
         };
-        auto q_store = [&](int row, int ch, float scale, const float (&v)[8]) {
+        auto q_store = [&](int row, int ch, float scale, bool bad, const float (&v)[8]) {
             if (ch >= chunks) return;
             uint32_t hi[4], lo[4];
 #pragma unroll
-            for (int e = 0; e < 4; ++e) split2(v[2 * e] * scale, v[2 * e + 1] * scale, hi[e], lo[e]);
+            for (int e = 0; e < 4; ++e) split2(bad ? 0.f : v[2 * e] * scale, bad ? 0.f : v[2 * e + 1] * scale, hi[e], lo[e]);
             const int st = geo.n_kst == 1 ? 0 : ch / wkb, w = st == geo.n_kst - 1 ? geo.wk_last : geo.wk0, c8 = ch - st * wkb;
             unsigned char* dst = qs + (size_t)st * geo.wk0 * kRows * 4 + (size_t)(((row >> 3) * (w >> 3) + c8) * 128 + (row & 7) * 16);
             *reinterpret_cast<uint4*>(dst) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
@@ -547,18 +636,20 @@ split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_co
             for (int rg = 0; rg < 2; ++rg) {
                 float m = 0.f;
 #pragma unroll
-                for (int i = 0; i < 4; ++i) m = max_finite4(max_finite4(m, v[rg * 4 + i][0]), v[rg * 4 + i][1]);
-                const float scale = q_scale(m, qrow + 64 * rg);
+                for (int i = 0; i < 4; ++i) m = max_abs4(max_abs4(m, v[rg * 4 + i][0]), v[rg * 4 + i][1]);
+                bool bad;
+                const float scale = q_scale(m, qrow + 64 * rg, bad);
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
                     const float4 a = v[rg * 4 + i][0], b = v[rg * 4 + i][1];
                     const float x[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-                    q_store(qrow + 64 * rg, qch + 4 * i, scale, x);
+                    q_store(qrow + 64 * rg, qch + 4 * i, scale, bad, x);
                 }
             }
         } else {
             for (int rg = 0; rg < 2; ++rg) {
                 float m = 0.f, scale = 0.f;
+                bool bad = false;
                 for (int pass = 0; pass < 2; ++pass) {
                     for (int ch = qch; ch < chunks; ch += 16) {
                         float v[4][8];
@@ -568,13 +659,13 @@ split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_co
                         for (int i = 0; i < 4; ++i) {
                             if (pass == 0) {
 #pragma unroll
-                                for (int e = 0; e < 8; ++e) m = fmaxf(m, finite_abs(v[i][e]));
+                                for (int e = 0; e < 8; ++e) m = max_nan(m, fabsf(v[i][e]));
                             } else {
-                                q_store(qrow + 64 * rg, ch + 4 * i, scale, v[i]);
+                                q_store(qrow + 64 * rg, ch + 4 * i, scale, bad, v[i]);
                             }
                         }
                     }
-                    if (pass == 0) scale = q_scale(m, qrow + 64 * rg);
+                    if (pass == 0) scale = q_scale(m, qrow + 64 * rg, bad);
                 }
             }
         }
@@ -690,25 +781,27 @@ split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_co
 #pragma unroll
                 for (int e = 0; e < 32; ++e) s[e] -= slope * (base - (float)e);
             }
-            const bool live = tok >= w.seg_a && tok < w.seg_b;
-            const int last = live ? min(w.k_end - 1, ranged ? 0x7fffffff : my_pos) : -1, first = ranged ? w.lo : my_lo;
-            if (!__all_sync(0xffffffffu, k0 + 31 <= last && (k0 >= first || k0 + 31 < kept))) {
+            auto hide = [&](float x) {                        // x in the place of every key that the row does not see
+                const bool live = tok >= w.seg_a && tok < w.seg_b;
+                const int last = live ? min(w.k_end - 1, ranged ? 0x7fffffff : my_pos) : -1, first = ranged ? w.lo : my_lo;
+                if (__all_sync(0xffffffffu, k0 + 31 <= last && (k0 >= first || k0 + 31 < kept))) return;
 #pragma unroll
                 for (int e = 0; e < 32; ++e) {
                     const int j = k0 + e;
-                    if (!(j <= last && (j >= first || j < kept))) s[e] = -CUDART_INF_F;
+                    if (!(j <= last && (j >= first || j < kept))) s[e] = x;
                 }
-            }
+            };
+            hide(-CUDART_INF_F);
             float mx = s[0];
 #pragma unroll
-            for (int e = 1; e < 32; ++e) mx = fmaxf(mx, s[e]);
+            for (int e = 1; e < 32; ++e) mx = max_nan(mx, s[e]);
             // (two exchanges a tile in two places: whoever writes one has seen the other thread leave the one before)
             row_x[hf * kRows + row] = mx;
             __syncwarp();
             if (lane == 0) mbar_arrive(&pair[qt]);
             if (!wait_for(&pair[qt], 0)) { ok = false; break; }
-            mx = fmaxf(mx, row_x[(hf ^ 1) * kRows + row]);
-            const float m_new = fmaxf(m_run, mx);
+            mx = max_nan(mx, row_x[(hf ^ 1) * kRows + row]);
+            const float m_new = max_nan(m_run, mx);
             const float base = m_new == -CUDART_INF_F ? 0.f : m_new, corr = m_run == -CUDART_INF_F ? 0.f : ex2(m_run - base);
             float2 sum = make_float2(0.f, 0.f);
             const float2 nb = make_float2(-base, -base);
@@ -724,9 +817,18 @@ split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_co
             // weight x its value's magnitude, and the largest of them that this row has in the tile
             if (!geo.shared_kv && !wait_for(&v_ready[t % geo.depth], (t / geo.depth) & 1u)) { ok = false; break; }
             scale_by<32>(s, v_inv + (t % geo.depth) * kKeys + hf * 32);
-            float wm = s[0];
+            auto largest = [&] {
+                float v = s[0];
 #pragma unroll
-            for (int e = 1; e < 32; ++e) wm = fmaxf(wm, s[e]);
+                for (int e = 1; e < 32; ++e) v = max_nan(v, s[e]);
+                return v;
+            };
+            float wm = largest();
+            if (__any_sync(0xffffffffu, wm != wm)) {          // a value that cannot be split, 0 x NaN where it is not seen
+                hide(0.f);
+                wm = largest();
+                if (wm != wm) l_run = CUDART_NAN_F;
+            }
             row_x[(2 + hf) * kRows + row] = wm;
             __syncwarp();
             if (lane == 0) mbar_arrive(&pair[qt]);
@@ -786,6 +888,11 @@ split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_co
             if (c < n_mine) *reinterpret_cast<float4*>(stage + lane * ldst + c) = make_float4(O[c] * f, O[c + 1] * f, O[c + 2] * f, O[c + 3] * f);
         __syncwarp();
         const int w4 = min(n_mine, p.vdim - c0) >> 2;         // (vdim is a multiple of 4)
+        for (unsigned again = __ballot_sync(0xffffffffu, ok && tok < n_tok && l != l); again; again &= again - 1) {
+            const int r = __ffs(again) - 1, rw = qt * 32 + r, tk = rw >> geo.pk_shift;
+            plain_row(p, r0 + tk, s_slot[tk], s_pos[tk], h0 + (rw & (PK - 1)), c0, 4 * w4, stage + r * ldst);
+        }
+        __syncwarp();
         int sr = 0, sc = lane;                                // row and group of 4 channels of this lane's turn
         while (w4 > 0 && sc >= w4) { sc -= w4; ++sr; }
 #pragma unroll 2
@@ -879,16 +986,20 @@ split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_co
                 for (int kg = 0; kg < 2; ++kg) {
                     float m = 0.f;
 #pragma unroll
-                    for (int i = 0; i < 8; ++i) m = max_finite4(m, v[kg * 8 + i]);
+                    for (int i = 0; i < 8; ++i) m = max_abs4(m, v[kg * 8 + i]);
                     if (w < row_w && rows[kg] != ~(size_t)0)
                         for (int c = w + 4 * cq; c < row_w; c += 16)
-                            m = max_finite4(m, *reinterpret_cast<const float4*>(row_of(cache, width, gg, rows[kg]) + c));
+                            m = max_abs4(m, *reinterpret_cast<const float4*>(row_of(cache, width, gg, rows[kg]) + c));
                     m_row[kg] = row_max(m);
                 }
             }
             float sc[2], inverse[2];
 #pragma unroll
-            for (int kg = 0; kg < 2; ++kg) sc[kg] = scale_of(m_row[kg], inverse[kg]);
+            for (int kg = 0; kg < 2; ++kg)
+                if (scale_row(m_row[kg], sc[kg], inverse[kg])) {
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) v[kg * 8 + i] = make_float4(0.f, 0.f, 0.f, 0.f);
+                }
             auto put_scales = [&] {
                 if (inv && lane < 8) {
 #pragma unroll

@@ -134,3 +134,60 @@ def test_a_row_has_the_same_bits_in_any_step(make, args):
     whole = run([300], 0)
     for parts, beside in (([100, 9, 191], 0), ([300], 33), ([9, 9, 60, 222], 400)):
         assert torch.equal(whole, run(parts, beside)), (parts, beside)
+
+
+def by_rows(q, k, v, see):
+    """The same in 64 bits, row by row over the keys that the row sees: an infinity or a NaN elsewhere does not enter"""
+    T, H, d = q.shape
+    out = torch.zeros(T, H, v.shape[-1], dtype=torch.float64)
+    for i in range(T):
+        j = see[i].nonzero()[:, 0]
+        for h in range(H):
+            g = h * k.shape[0] // H
+            s = (q[i, h].double() * k[g, j].double()).sum(-1) * d ** -0.5
+            out[i, h] = (torch.softmax(s, -1)[:, None] * v[g, j].double()).sum(0)
+    return out
+
+
+@pytest.mark.parametrize("what,x", [("value", torch.inf), ("value", -torch.inf), ("value", torch.nan), ("key", torch.inf), ("key", torch.nan),
+                                    ("query", torch.inf), ("query", torch.nan)])
+def test_a_number_that_is_not_finite(what, x):
+    """One infinity or NaN: rows that do not see it keep their bits, rows that do get what fp32 arithmetic makes of it, channel by channel."""
+    from dia_tts_prune_b200 import engine as E
+    g, at, T = torch.Generator().manual_seed(11), 200, 257
+    q, k, v = torch.randn(2, T, 4, 128, generator=g), torch.randn(2, 2, T, 128, generator=g), torch.randn(2, 2, T, 128, generator=g)
+    base = E.attention_rows(q.cuda(), k.cuda(), v.cuda(), T, 0, None).cpu()
+    if what == "query":
+        q[0, at, 1, 5] = x
+        touched = torch.zeros(2, T, 4, dtype=torch.bool)
+        touched[0, at, 1] = True
+    else:
+        (k if what == "key" else v)[0, 1, at, 5] = x
+        touched = torch.zeros(2, T, 4, dtype=torch.bool)
+        touched[0, at:, 2:] = True
+    got = E.attention_rows(q.cuda(), k.cuda(), v.cuda(), T, 0, None).cpu()
+    assert torch.equal(got[~touched], base[~touched])
+    ref = by_rows(q[0], k[0], v[0], torch.ones(T, T).tril().bool())[touched[0]]
+    torch.testing.assert_close(got[touched].double(), ref, rtol=2e-5, atol=2e-5, equal_nan=True)
+
+
+@pytest.mark.parametrize("rows", [150, 300])
+@pytest.mark.parametrize("make,args,window", [(grouped, (4, 2, 64, 33, 3, 20.0, 16), 33), (mixed, (8, 2, 64, 160), 0), (latent, (4, 32, 192, 16, 64, 40), 40)])
+def test_a_token_of_a_step_that_is_not_finite(make, args, window, rows):
+    """A token of NaN in a step: rows in front of it and rows whose window has left it behind keep their bits.  Keys split by the row tiles and
+    in advance."""
+    model, n_in, op = make(*args)
+    x = torch.randn(rows, n_in, generator=torch.Generator().manual_seed(12)).cuda()
+
+    def run(h):
+        seq = model.state.open("a")
+        model.state.reserve(seq, rows)
+        y = op(h, [(seq, rows, 0)])
+        model.state.close("a")
+        return (y[0] if isinstance(y, (tuple, list)) else y).clone()
+
+    base, h, at = run(x), x.clone(), 70
+    h[at] = torch.nan
+    got, after = run(h), at + window if window else rows
+    assert torch.equal(got[:at], base[:at]) and torch.equal(got[after:], base[after:])
+    assert torch.isfinite(base).all() and got[at:after].isnan().any(-1).all()
