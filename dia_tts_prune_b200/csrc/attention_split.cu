@@ -494,15 +494,16 @@ split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_co
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int PK = 1 << geo.pk_shift;
-    const int h0 = blockIdx.x * PK, rep = p.heads / p.kv_heads, g = h0 / rep;
+    const int h_tiles = p.heads >> geo.pk_shift, row_tile = (int)(gridDim.x / h_tiles) - 1 - (int)(blockIdx.x / h_tiles);
+    const int h0 = (int)(blockIdx.x % h_tiles) * PK, rep = p.heads / p.kv_heads, g = h0 / rep;
     // later tokens see more keys: their tiles start first.  With the step's sequences at hand a tile holds rows of one of them (a
     // tile with the rows of 24 decoding sequences walked the keys of all 24 one after the other)
-    int r0 = (gridDim.y - 1 - blockIdx.y) * TT, n_tok = min(TT, p.M - r0);
+    int r0 = row_tile * TT, n_tok = min(TT, p.M - r0);
     if (p.n_seq > 1) {
         if (tid == 0) s_rows[1] = 0;
         __syncthreads();
         if (warp == 0) {
-            const int want = gridDim.y - 1 - blockIdx.y;
+            const int want = row_tile;
             int run = 0;
             for (int s0 = 0; s0 < p.n_seq; s0 += 32) {
                 const int count = s0 + lane < p.n_seq ? p.seq_count[s0 + lane] : 0, n = (count + TT - 1) / TT;
@@ -1229,9 +1230,8 @@ cudaError_t launch_inst(const SplitAttention& a, const Geometry& g, size_t smem,
     const cudaError_t e = cudaFuncSetAttribute(split_attention_kernel<NVS>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMost);
     if (e != cudaSuccess) return e;
     const int tt = kRows >> g.pk_shift, tiles = a.n_seq > 1 ? a.M / tt + a.n_seq : (a.M + tt - 1) / tt;
-    if (tiles > 65535) return cudaErrorNotSupported;
     if (a.work) split_keys_kernel<<<dim3(g.cap_tiles, g.parts), 256, 0, st>>>(a, g);
-    split_attention_kernel<NVS><<<dim3(a.heads >> g.pk_shift, tiles), kSplitThreadsTC, smem, st>>>(a, g);
+    split_attention_kernel<NVS><<<(a.heads >> g.pk_shift) * tiles, kSplitThreadsTC, smem, st>>>(a, g);
     return cudaGetLastError();
 }
 

@@ -191,3 +191,21 @@ def test_a_token_of_a_step_that_is_not_finite(make, args, window, rows):
     got, after = run(h), at + window if window else rows
     assert torch.equal(got[:at], base[:at]) and torch.equal(got[after:], base[after:])
     assert torch.isfinite(base).all() and got[at:after].isnan().any(-1).all()
+
+
+def test_more_row_tiles_than_a_grid_is_high():
+    """128 heads that share their keys leave one token to a row tile: a step of more than 65535 rows"""
+    model_rows, heads, dim, window = 65600, 128, 4, 5
+    from dia_tts_prune_b200 import synthetic as SY
+    from dia_tts_prune_b200.lm_config import PubopelConfig
+    from dia_tts_prune_b200.lm_model import CausalLM
+    cfg = SY.pubopel_config(width=32, layers=1, heads=heads, kv_heads=1, dim=dim, experts=1, top=1, expert_ff=8, shared_ff=None, vocab=64, window=window,
+                            keep_first=0, softcap=None)
+    model = CausalLM(PubopelConfig.model_validate(cfg), SY.pubopel_weights(cfg, 3), dtype="bfloat16", device="cuda:0", max_tokens=model_rows + 64,
+                     max_sequences=1, page_size=64, max_rows=model_rows)
+    x = torch.randn(model_rows, (heads + 1) * dim, generator=torch.Generator().manual_seed(13)).cuda()
+    seq = model.state.open("a")
+    model.state.reserve(seq, model_rows)
+    got = model.engine.op_attention(0, x.clone(), [(seq, model_rows, 0)])
+    again = model.engine.op_attention(0, x[65500:].clone(), [(seq, 100, 65500)])
+    assert torch.equal(got[65500:], again) and torch.isfinite(got).all() and got.abs().amax(-1).min() > 0
