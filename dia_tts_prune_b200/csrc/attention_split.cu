@@ -46,6 +46,7 @@ constexpr int kMaxSlots = 6, kMaxDepth = 5, kMaxKStages = 4;
 constexpr int kSmemMost = 232448;                             // all of it dynamic
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr int kSplitOnceRows = 512;                           // rows of a kv head (M rep) from which the keys are split in advance
+constexpr int kSplitGrid = 148 * 16;                           // CTAs of the launch that splits them
 constexpr unsigned kSpinMost = 4000000u;
 
 struct Geometry {
@@ -241,107 +242,111 @@ __device__ __forceinline__ size_t part_offset(const Geometry& geo, int part) {
 
 // Splits the keys and values that the step's rows see, once for all row tiles: without it each of the M rep / 128 row tiles of a
 // key/value head converts every tile it walks, and that conversion (two thirds of the instructions) bounds the kernel below.
-// One CTA per (tile of the room, part); tiles are dealt to the sequences in order.  Warp w takes keys 8 w .. of the tile.
+// A CTA per (tile of the room, part), and two rounds of them at most: a room for many sequences has far more tiles than a short step
+// fills.  Tiles are dealt to the sequences in order.  Warp w takes keys 8 w .. of the tile.
 __global__ void __launch_bounds__(256)
 split_keys_kernel(const __grid_constant__ SplitAttention p, const __grid_constant__ Geometry geo) {
     __shared__ int s_first, s_seq, s_run;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, tile = blockIdx.x, part = blockIdx.y;
-    const bool writes_plan = tile == 0 && part == 0;
-    SlotTiles* plan = reinterpret_cast<SlotTiles*>(p.work);
-    // ---- which sequence's tile is this? ----
-    if (tid == 0) { s_seq = -1; s_run = 0; }
-    __syncthreads();
-    for (int s0 = 0; s0 < p.n_seq; s0 += 32) {                // warp 0: 32 sequences at a time, running sum of their tiles
-        if (warp == 0) {
-            const int s = s0 + lane;
-            int first = 0, n = 0, slot = 0, extra = 0, end = 0;
-            if (s < p.n_seq) {
-                slot = p.seq_slot[s];
-                const int r = p.seq_row0[s], pos = p.row_pos[r];
-                first = first_key_of(pos, p.window, p.chunk) / kKeys;
-                end = (pos + p.seq_count[s] + kKeys - 1) / kKeys;
-                extra = p.window > 0 && p.keep_first > 0 && first > 0 ? 1 : 0;    // tile 0 holds the kept keys (of at most 64)
-                n = end - first + extra;
-            }
-            int sum = n;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, part = blockIdx.y;
+    for (int tile = blockIdx.x; tile < geo.cap_tiles; tile += gridDim.x) {
+        const bool writes_plan = tile == 0 && part == 0;
+        SlotTiles* plan = reinterpret_cast<SlotTiles*>(p.work);
+        // ---- which sequence's tile is this? ----
+        __syncthreads();                                          // (the last tile's answer has been read)
+        if (tid == 0) { s_seq = -1; s_run = 0; }
+        __syncthreads();
+        for (int s0 = 0; s0 < p.n_seq; s0 += 32) {                // warp 0: 32 sequences at a time, running sum of their tiles
+            if (warp == 0) {
+                const int s = s0 + lane;
+                int first = 0, n = 0, slot = 0, extra = 0, end = 0;
+                if (s < p.n_seq) {
+                    slot = p.seq_slot[s];
+                    const int r = p.seq_row0[s], pos = p.row_pos[r];
+                    first = first_key_of(pos, p.window, p.chunk) / kKeys;
+                    end = (pos + p.seq_count[s] + kKeys - 1) / kKeys;
+                    extra = p.window > 0 && p.keep_first > 0 && first > 0 ? 1 : 0;    // tile 0 holds the kept keys (of at most 64)
+                    n = end - first + extra;
+                }
+                int sum = n;
 #pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int v = __shfl_up_sync(0xffffffffu, sum, o);
-                if (lane >= o) sum += v;
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int v = __shfl_up_sync(0xffffffffu, sum, o);
+                    if (lane >= o) sum += v;
+                }
+                const int begin = s_run + sum - n;
+                if (writes_plan && s < p.n_seq) {
+                    SlotTiles t;
+                    t.zero = extra && begin < geo.cap_tiles ? begin : -1;
+                    t.base = begin + extra - first;
+                    t.first = first;
+                    t.end = min(end, geo.cap_tiles - t.base);
+                    plan[slot] = t;
+                }
+                if (s < p.n_seq && tile >= begin && tile < begin + n) {
+                    s_seq = s;
+                    s_first = extra && tile == begin ? 0 : first + tile - begin - extra;
+                }
+                __syncwarp();
+                if (lane == 31) s_run += sum;
+                __syncwarp();
             }
-            const int begin = s_run + sum - n;
-            if (writes_plan && s < p.n_seq) {
-                SlotTiles t;
-                t.zero = extra && begin < geo.cap_tiles ? begin : -1;
-                t.base = begin + extra - first;
-                t.first = first;
-                t.end = min(end, geo.cap_tiles - t.base);
-                plan[slot] = t;
-            }
-            if (s < p.n_seq && tile >= begin && tile < begin + n) {
-                s_seq = s;
-                s_first = extra && tile == begin ? 0 : first + tile - begin - extra;
-            }
-            __syncwarp();
-            if (lane == 31) s_run += sum;
-            __syncwarp();
+            __syncthreads();
+            if (s_seq >= 0 && !writes_plan) break;                // (the same for all threads: read behind the barrier)
+            __syncthreads();
         }
-        __syncthreads();
-        if (s_seq >= 0 && !writes_plan) break;                // (the same for all threads: read behind the barrier)
-        __syncthreads();
-    }
-    if (s_seq < 0) return;
-    const int seq = s_seq, slot = p.seq_slot[seq], pos0 = p.row_pos[p.seq_row0[seq]], k_end = pos0 + p.seq_count[seq], j0 = s_first * kKeys;
-    // ---- which rows and channels? ----
-    const bool is_v = part >= geo.k_parts;
-    const int q = is_v ? part - geo.k_parts : part, per = is_v ? geo.n_vst : geo.n_kst, gg = q / per, st = q % per;
-    const bool talk = p.talk != nullptr && !is_v;             // (a key group is a whole kv head there)
-    const int g = talk ? st : gg, c0 = talk ? 0 : st * kGroupW;
-    const int w = talk ? p.kdim : min(kGroupW, (is_v ? p.vdim : p.kdim) - c0), wp = is_v ? (st == per - 1 ? geo.wv_last : geo.wv0) : (st == per - 1 ? geo.wk_last : geo.wk0);
-    const int width = is_v ? p.vrow : p.kdim, kin = lane & 7, cq = lane >> 3, j = j0 + warp * 8 + kin, blocks = wp >> 3;
-    const bool in = j < k_end;
-    const float* src = is_v ? p.vcache : p.kcache;
-    if (in) {
-        const int page = p.table[(size_t)slot * p.max_pages + j / p.page_size];
-        src += (((size_t)page * p.kv_heads + g) * p.page_size + j % p.page_size) * width;
-    }
-    float4 v[8];
-    float m = 0.f;
+        if (s_seq < 0) return;                                // (nor does any later tile belong to one)
+        const int seq = s_seq, slot = p.seq_slot[seq], pos0 = p.row_pos[p.seq_row0[seq]], k_end = pos0 + p.seq_count[seq], j0 = s_first * kKeys;
+        // ---- which rows and channels? ----
+        const bool is_v = part >= geo.k_parts;
+        const int q = is_v ? part - geo.k_parts : part, per = is_v ? geo.n_vst : geo.n_kst, gg = q / per, st = q % per;
+        const bool talk = p.talk != nullptr && !is_v;             // (a key group is a whole kv head there)
+        const int g = talk ? st : gg, c0 = talk ? 0 : st * kGroupW;
+        const int w = talk ? p.kdim : min(kGroupW, (is_v ? p.vdim : p.kdim) - c0), wp = is_v ? (st == per - 1 ? geo.wv_last : geo.wv0) : (st == per - 1 ? geo.wk_last : geo.wk0);
+        const int width = is_v ? p.vrow : p.kdim, kin = lane & 7, cq = lane >> 3, j = j0 + warp * 8 + kin, blocks = wp >> 3;
+        const bool in = j < k_end;
+        const float* src = is_v ? p.vcache : p.kcache;
+        if (in) {
+            const int page = p.table[(size_t)slot * p.max_pages + j / p.page_size];
+            src += (((size_t)page * p.kv_heads + g) * p.page_size + j % p.page_size) * width;
+        }
+        float4 v[8];
+        float m = 0.f;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int c = 8 * (cq + 4 * i);
-        const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
-        v[2 * i] = in && c < w ? *reinterpret_cast<const float4*>(src + c0 + c) : z;
-        v[2 * i + 1] = in && c + 4 < w ? *reinterpret_cast<const float4*>(src + c0 + c + 4) : z;
-    }
-    // the scale is that of the whole row (a latent's value is a part of its key row)
-    const int row_w = is_v ? p.vdim : p.kdim;
+        for (int i = 0; i < 4; ++i) {
+            const int c = 8 * (cq + 4 * i);
+            const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
+            v[2 * i] = in && c < w ? *reinterpret_cast<const float4*>(src + c0 + c) : z;
+            v[2 * i + 1] = in && c + 4 < w ? *reinterpret_cast<const float4*>(src + c0 + c + 4) : z;
+        }
+        // the scale is that of the whole row (a latent's value is a part of its key row)
+        const int row_w = is_v ? p.vdim : p.kdim;
 #pragma unroll
-    for (int i = 0; i < 8; ++i) m = max_abs4(m, v[i]);
-    if (w < row_w && in)
-        for (int c = 4 * cq; c < row_w; c += 16) m = max_abs4(m, *reinterpret_cast<const float4*>(src + c));
-    float sc, inverse;
-    if (scale_row(row_max(m), sc, inverse)) {
+        for (int i = 0; i < 8; ++i) m = max_abs4(m, v[i]);
+        if (w < row_w && in)
+            for (int c = 4 * cq; c < row_w; c += 16) m = max_abs4(m, *reinterpret_cast<const float4*>(src + c));
+        float sc, inverse;
+        if (scale_row(row_max(m), sc, inverse)) {
 #pragma unroll
-        for (int i = 0; i < 8; ++i) v[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-    unsigned char* work = reinterpret_cast<unsigned char*>(p.work);
-    const int set = is_v ? p.kv_heads + gg : talk ? st : gg;
-    if (cq == 0 && (talk || st == 0))
-        reinterpret_cast<float*>(work + geo.scale_off)[((size_t)tile * geo.sets + set) * kKeys + warp * 8 + kin] = inverse;
-    unsigned char* base = work + geo.tile_off + (size_t)tile * geo.tile_bytes + part_offset(geo, part);
+            for (int i = 0; i < 8; ++i) v[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        unsigned char* work = reinterpret_cast<unsigned char*>(p.work);
+        const int set = is_v ? p.kv_heads + gg : talk ? st : gg;
+        if (cq == 0 && (talk || st == 0))
+            reinterpret_cast<float*>(work + geo.scale_off)[((size_t)tile * geo.sets + set) * kKeys + warp * 8 + kin] = inverse;
+        unsigned char* base = work + geo.tile_off + (size_t)tile * geo.tile_bytes + part_offset(geo, part);
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int c8 = cq + 4 * i;
-        if (c8 >= blocks) continue;
-        uint32_t hi[4], lo[4];
-        split2(v[2 * i].x * sc, v[2 * i].y * sc, hi[0], lo[0]);
-        split2(v[2 * i].z * sc, v[2 * i].w * sc, hi[1], lo[1]);
-        split2(v[2 * i + 1].x * sc, v[2 * i + 1].y * sc, hi[2], lo[2]);
-        split2(v[2 * i + 1].z * sc, v[2 * i + 1].w * sc, hi[3], lo[3]);
-        unsigned char* dst = base + (warp * blocks + c8) * 128 + kin * 16;
-        *reinterpret_cast<uint4*>(dst) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-        *reinterpret_cast<uint4*>(dst + kKeys * wp * 2) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+        for (int i = 0; i < 4; ++i) {
+            const int c8 = cq + 4 * i;
+            if (c8 >= blocks) continue;
+            uint32_t hi[4], lo[4];
+            split2(v[2 * i].x * sc, v[2 * i].y * sc, hi[0], lo[0]);
+            split2(v[2 * i].z * sc, v[2 * i].w * sc, hi[1], lo[1]);
+            split2(v[2 * i + 1].x * sc, v[2 * i + 1].y * sc, hi[2], lo[2]);
+            split2(v[2 * i + 1].z * sc, v[2 * i + 1].w * sc, hi[3], lo[3]);
+            unsigned char* dst = base + (warp * blocks + c8) * 128 + kin * 16;
+            *reinterpret_cast<uint4*>(dst) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+            *reinterpret_cast<uint4*>(dst + kKeys * wp * 2) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+        }
     }
 }
 
@@ -1230,7 +1235,7 @@ cudaError_t launch_inst(const SplitAttention& a, const Geometry& g, size_t smem,
     const cudaError_t e = cudaFuncSetAttribute(split_attention_kernel<NVS>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMost);
     if (e != cudaSuccess) return e;
     const int tt = kRows >> g.pk_shift, tiles = a.n_seq > 1 ? a.M / tt + a.n_seq : (a.M + tt - 1) / tt;
-    if (a.work) split_keys_kernel<<<dim3(g.cap_tiles, g.parts), 256, 0, st>>>(a, g);
+    if (a.work) split_keys_kernel<<<dim3(std::min(g.cap_tiles, std::max(1, kSplitGrid / g.parts)), g.parts), 256, 0, st>>>(a, g);
     split_attention_kernel<NVS><<<(a.heads >> g.pk_shift) * tiles, kSplitThreadsTC, smem, st>>>(a, g);
     return cudaGetLastError();
 }

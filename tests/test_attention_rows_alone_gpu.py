@@ -112,7 +112,8 @@ def test_a_row_has_the_same_bits_in_any_step(make, args):
     row tiles split the keys themselves, with many a launch in front does it."""
     model, n_in, op = make(*args)
     g = torch.Generator().manual_seed(9)
-    x, other = torch.randn(300, n_in, generator=g).cuda(), (1000 * torch.randn(400, n_in, generator=g)).cuda()
+    x = (torch.randn(300, n_in, generator=g) * 10.0 ** torch.randint(-2, 3, (300, 1), generator=g)).cuda()
+    other = (1000 * torch.randn(400, n_in, generator=g)).cuda()
 
     def run(parts, beside):
         seq = model.state.open("a")
@@ -209,3 +210,14 @@ def test_more_row_tiles_than_a_grid_is_high():
     got = model.engine.op_attention(0, x.clone(), [(seq, model_rows, 0)])
     again = model.engine.op_attention(0, x[65500:].clone(), [(seq, 100, 65500)])
     assert torch.equal(got[65500:], again) and torch.isfinite(got).all() and got.abs().amax(-1).min() > 0
+
+
+def test_keys_split_in_several_rounds():
+    """More tiles of keys than the launch that splits them has CTAs for a part: against the keys that the row tiles split for themselves"""
+    model, n_in, op = grouped(32, 32, 16, 0, 0, 0.0, 64)
+    x = torch.randn(3000, n_in, generator=torch.Generator().manual_seed(14)).cuda()
+    seq = model.state.open("a")
+    model.state.reserve(seq, 3000)
+    parts = [op(x[a:b], [(seq, b - a, a)]).clone() for a, b in ((0, 1024), (1024, 2048), (2048, 3000))]
+    for a in (1900, 2048, 2980):
+        assert torch.equal(op(x[a:a + 20], [(seq, 20, a)]), torch.cat(parts)[a:a + 20])
