@@ -472,8 +472,10 @@ template <int NVS>
 __global__ void __launch_bounds__(kSplitThreadsTC, 1)
 split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_constant__ Geometry geo) {
     constexpr int DVH = 64 * NVS;                             // output channels of a thread
-    // the block is launched with 128 registers a thread: 256 of kRowRegs, 128 of kFetchRegs and 128 of 32
-    constexpr int kRowRegs = NVS == 1 ? 176 : 184, kFetchRegs = NVS == 1 ? 128 : 112;
+    // The block is launched with 128 registers a thread: 256 of kRowRegs, 128 of kFetchRegs and 128 of 32.  (latent_4096's attention, wide
+    // values: 184 and 112 452 us, 192 and 96 443, 200 and 80 421: what the fetching warps spill is used for keys that are not split in
+    // advance only.)
+    constexpr int kRowRegs = NVS == 1 ? 176 : 200, kFetchRegs = NVS == 1 ? 128 : 80;
     static_assert(256 * kRowRegs + 128 * kFetchRegs + 128 * 32 <= 128 * kSplitThreadsTC, "registers of the block");
     extern __shared__ __align__(128) unsigned char smem[];
     unsigned char* ring = smem;

@@ -221,3 +221,27 @@ def test_keys_split_in_several_rounds():
     parts = [op(x[a:b], [(seq, b - a, a)]).clone() for a, b in ((0, 1024), (1024, 2048), (2048, 3000))]
     for a in (1900, 2048, 2980):
         assert torch.equal(op(x[a:a + 20], [(seq, 20, a)]), torch.cat(parts)[a:a + 20])
+
+
+def kernels_of(call):
+    from torch.profiler import ProfilerActivity, profile
+    call()
+    torch.cuda.synchronize()
+    with profile(activities=[ProfilerActivity.CUDA]) as p:
+        call()
+        torch.cuda.synchronize()
+    return [e.name for e in p.events() if e.device_type == torch.autograd.DeviceType.CUDA and "emcpy" not in e.name and "emset" not in e.name]
+
+
+@pytest.mark.parametrize("heads", [4, 8, 16])
+def test_the_widest_latent_rows(heads):
+    """Latent rows of 256 + 64 channels leave the row tile's queries and two slots of keys 3 KB of shared memory for all else, whatever the number
+    of heads; against the row kernels of short steps"""
+    model, n_in, op = latent(heads, 32, 256, 64, 64, 0)
+    x = torch.randn(200, n_in, generator=torch.Generator().manual_seed(15)).cuda()
+    seq = model.state.open("a")
+    model.state.reserve(seq, 200)
+    assert any("split_attention_kernel" in n for n in kernels_of(lambda: op(x, [(seq, 200, 0)])))
+    whole = op(x, [(seq, 200, 0)]).clone()
+    short = torch.cat([op(x[a:a + 8], [(seq, 8, a)]) for a in range(0, 200, 8)])
+    assert (whole - short).abs().max() <= 2e-5 * short.abs().max()
