@@ -582,7 +582,11 @@ dia_gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
 //   warps 2-5 add the k-blocks' accumulators in fp32 registers (weight row = lane), then the three terms; the CTAs' partial sums
 //             meet in shared memory and every CTA of the cluster adds its share of the outputs, in the order of the k ranges
 // Bound: the weights' bytes.  The row kernel reads them once per row from L2 instead: 8 rows x 2048 x 6144 took 35 us.
-constexpr int kRThreads = 192, kRSlotsMost = 8, kRSmemMost = 226 * 1024;
+// An SM holds two of its CTAs at most, whatever the shape: a launch may start before its predecessors have ended, and its CTAs keep
+// their half of tensor memory while they wait for them.  With three on an SM a predecessor's CTA could find all of it taken by CTAs
+// that wait for that CTA.
+constexpr int kRThreads = 192, kRSlotsMost = 8, kRSmemMost = 226 * 1024, kRSmemLeast = 78 * 1024;
+static_assert(3 * kRSmemLeast > 228 * 1024, "two CTAs on an SM");
 
 // NB: columns of the rows' operand (32 for up to 8 rows, 96 for up to 32)
 template <int NB>
@@ -923,7 +927,7 @@ static cudaError_t launch_few_rows(const FewRowsProduct& p, bool early, cudaStre
     int n_slots = std::min(kRSlotsMost, kb_per);
     while (n_slots > (groups > 1 ? 2 : 3) && few_rows_smem(NB, kb_per, n_slots) > kRSmemMost / 2) --n_slots;
     while (few_rows_smem(NB, kb_per, n_slots) > kRSmemMost) --n_slots;
-    const size_t smem = few_rows_smem(NB, kb_per, n_slots);
+    const size_t smem = std::max<size_t>(few_rows_smem(NB, kb_per, n_slots), kRSmemLeast);
     // (the same size for every launch: another thread's cannot lower what this one needs)
     const cudaError_t e = cudaFuncSetAttribute(dia_gemm_few_rows_kernel<NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, kRSmemMost);
     if (e != cudaSuccess) return e;

@@ -1,0 +1,30 @@
+"""The products of a few rows (few_rows of csrc/gemm_tcgen05.cu) in chains of launches that start before their predecessors have ended."""
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("requests", [4, 8])
+def test_chains_of_early_launches(requests):
+    """Products small enough that an SM could hold four CTAs, each with half of its tensor memory: a step is repeated through its graph, and
+    has the same bits each time"""
+    from dia_tts_prune_b200 import synthetic as SY
+    from dia_tts_prune_b200.lm_config import ForilornConfig
+    from dia_tts_prune_b200.lm_model import CausalLM
+    cfg = SY.forilorn_config(width=2048, kinds=["latent_attention"] * 6, heads=8, dim=64, vocab=64, lat_dim=64, rot_dim=16, lat_vdim=64, q_rank=512,
+                             kv_rank=64, ff=2048)
+    model = CausalLM(ForilornConfig.model_validate(cfg), SY.forilorn_weights(cfg, 3), dtype="bfloat16", device="cuda:0", max_tokens=64 * requests,
+                     max_sequences=requests, max_rows=64)
+    for i in range(requests):
+        model.run_step([{"id": str(i), "tokens": [1 + i, 2, 3], "want": []}])
+    entries = [{"id": str(i), "tokens": [5 + i], "want": [0]} for i in range(requests)]
+    first = None
+    for _ in range(300):
+        out = model.run_step(entries).clone()
+        for e in entries:
+            model.state.sequences[e["id"]].length -= 1
+        first = out if first is None else first
+        assert torch.equal(out, first)
+    assert torch.isfinite(first).all()
