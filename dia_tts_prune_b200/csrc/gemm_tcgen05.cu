@@ -405,50 +405,49 @@ dia_gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     auto emit = [&](int t, int r0) {
         const int q = warp & 3, hn = t / tiles_m, h = hn / tiles_n, n0 = (hn - h * tiles_n) * kFN, m0 = (t % tiles_m) * BM;
         const int rows = min(32, M - (m0 + q * 32)), n = n0 + 4 * lane;
-                    if (n < N) {
-                        const size_t m = (size_t)(m0 + q * 32), col = (size_t)h * p.y_hs + n;
-                        const float* gate = p.gate ? p.gate + m * p.ldg + (p.head_gate ? (size_t)h : (size_t)h * N + n) : nullptr;
-        #pragma unroll 1
-                        for (int r = r0; r < rows; r += S) {
-                            float4 v = *reinterpret_cast<const float4*>(tile + r * kFStride + 4 * lane);
-                if (S > 1) {
-                    float4 u[8];
+        if (n >= N) return;
+        const size_t m = (size_t)(m0 + q * 32), col = (size_t)h * p.y_hs + n;
+        const float* gate = p.gate ? p.gate + m * p.ldg + (p.head_gate ? (size_t)h : (size_t)h * N + n) : nullptr;
+#pragma unroll 1
+        for (int r = r0; r < rows; r += S) {
+            float4 v = *reinterpret_cast<const float4*>(tile + r * kFStride + 4 * lane);
+            if (S > 1) {
+                float4 u[8];
 #pragma unroll
-                    for (int c = 0; c < 8; ++c) if (c < S) u[c] = load_remote4(tile + r * kFStride + 4 * lane, c);
-                    v = u[0];
+                for (int c = 0; c < 8; ++c) if (c < S) u[c] = load_remote4(tile + r * kFStride + 4 * lane, c);
+                v = u[0];
 #pragma unroll
-                    for (int c = 1; c < 8; ++c) if (c < S) { v.x += u[c].x; v.y += u[c].y; v.z += u[c].z; v.w += u[c].w; }
+                for (int c = 1; c < 8; ++c) if (c < S) { v.x += u[c].x; v.y += u[c].y; v.z += u[c].z; v.w += u[c].w; }
+            }
+            v.x *= p.alpha; v.y *= p.alpha; v.z *= p.alpha; v.w *= p.alpha;
+            if (p.act) { v.x = f32_act(p.act, v.x); v.y = f32_act(p.act, v.y); v.z = f32_act(p.act, v.z); v.w = f32_act(p.act, v.w); }
+            if (gate) {
+                const float* z = gate + (size_t)r * p.ldg;
+                if (p.head_gate) {
+                    const float f = 1.0f / (1.0f + expf(-z[0]));
+                    v.x *= f; v.y *= f; v.z *= f; v.w *= f;
+                } else {
+                    v.x *= 1.0f / (1.0f + expf(-z[0])); v.y *= 1.0f / (1.0f + expf(-z[1]));
+                    v.z *= 1.0f / (1.0f + expf(-z[2])); v.w *= 1.0f / (1.0f + expf(-z[3]));
                 }
-                            v.x *= p.alpha; v.y *= p.alpha; v.z *= p.alpha; v.w *= p.alpha;
-                            if (p.act) { v.x = f32_act(p.act, v.x); v.y = f32_act(p.act, v.y); v.z = f32_act(p.act, v.z); v.w = f32_act(p.act, v.w); }
-                            if (gate) {
-                                const float* z = gate + (size_t)r * p.ldg;
-                                if (p.head_gate) {
-                                    const float f = 1.0f / (1.0f + expf(-z[0]));
-                                    v.x *= f; v.y *= f; v.z *= f; v.w *= f;
-                                } else {
-                                    v.x *= 1.0f / (1.0f + expf(-z[0])); v.y *= 1.0f / (1.0f + expf(-z[1]));
-                                    v.z *= 1.0f / (1.0f + expf(-z[2])); v.w *= 1.0f / (1.0f + expf(-z[3]));
-                                }
-                            }
-                            const size_t at = (m + r) * p.ldy + col;
-                            if (p.dyt_w) {
+            }
+            const size_t at = (m + r) * p.ldy + col;
+            if (p.dyt_w) {
                 const float4 w4 = *reinterpret_cast<const float4*>(p.dyt_w + col), b4 = *reinterpret_cast<const float4*>(p.dyt_b + col);
                 v.x = fmaf(tanhf(p.dyt_alpha * v.x), w4.x, b4.x); v.y = fmaf(tanhf(p.dyt_alpha * v.y), w4.y, b4.y);
                 v.z = fmaf(tanhf(p.dyt_alpha * v.z), w4.z, b4.z); v.w = fmaf(tanhf(p.dyt_alpha * v.w), w4.w, b4.w);
             }
             if (p.add) {
-                    const float4 o = *reinterpret_cast<const float4*>(p.add + at);
-                    v.x += o.x; v.y += o.y; v.z += o.z; v.w += o.w;
-                }
-                if (p.y) *reinterpret_cast<float4*>(p.y + at) = v;
-                            if (p.y_bf16) {
-                                const __nv_bfloat162 lo = __floats2bfloat162_rn(v.x, v.y), hi = __floats2bfloat162_rn(v.z, v.w);
-                                *reinterpret_cast<uint2*>(reinterpret_cast<__nv_bfloat16*>(p.y_bf16) + at) =
-                                    make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
-                            }
-                        }
-                    }
+                const float4 o = *reinterpret_cast<const float4*>(p.add + at);
+                v.x += o.x; v.y += o.y; v.z += o.z; v.w += o.w;
+            }
+            if (p.y) *reinterpret_cast<float4*>(p.y + at) = v;
+            if (p.y_bf16) {
+                const __nv_bfloat162 lo = __floats2bfloat162_rn(v.x, v.y), hi = __floats2bfloat162_rn(v.z, v.w);
+                *reinterpret_cast<uint2*>(reinterpret_cast<__nv_bfloat16*>(p.y_bf16) + at) =
+                    make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+            }
+        }
     };
     // tile t: row block t % tiles_m of column block (t / tiles_m) % tiles_n of head t / (tiles_m tiles_n)
     if (threadIdx.x == 0) {
@@ -601,8 +600,7 @@ dia_gemm_few_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid
     unsigned char* rows = ring + n_slots * kTileBytes;                         // [kb_per][NB x 64] bf16
     float* part = reinterpret_cast<float*>(rows + (size_t)kb_per * NB * 128);  // [Mp][128]
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int S = gridDim.y, n_kb = (p.K + BK - 1) / BK, rank = blockIdx.y, n0 = blockIdx.x * BM, m0 = blockIdx.z * kGemmFewRowsGroup;
-    const int M = min(p.M - m0, kGemmFewRowsGroup);
+    const int S = gridDim.y, n_kb = (p.K + BK - 1) / BK, rank = blockIdx.y, n0 = blockIdx.x * BM, M = p.M;
     const int kb0 = rank * kb_per, kbs = max(0, min(kb_per, n_kb - kb0));
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     if (tid == 0) {
@@ -626,7 +624,7 @@ dia_gemm_few_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid
 #pragma unroll
         for (int e = 0; e < 8; ++e) v[e] = 0.f;
         if (m < M && k < p.K) {                               // (K a multiple of 8)
-            const float4* src = reinterpret_cast<const float4*>(p.a + (size_t)(m0 + m) * p.lda + k);
+            const float4* src = reinterpret_cast<const float4*>(p.a + (size_t)m * p.lda + k);
             const float4 x = src[0], y = src[1];
             v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w; v[4] = y.x; v[5] = y.y; v[6] = y.z; v[7] = y.w;
         }
@@ -730,7 +728,7 @@ dia_gemm_few_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid
             v = part[i];
         }
         if (p.act) v = f32_act(p.act, v);
-        const size_t at = (size_t)(m0 + m) * p.ldy + n;
+        const size_t at = (size_t)m * p.ldy + n;
         p.y[at] = p.add ? p.add[at] + v : v;
     }
     if (S > 1) cluster_sync_all();                            // (the partial sums stay until every CTA has read them)
@@ -795,11 +793,11 @@ cudaError_t launch_transpose_to_bf16(const void* w, int src_bf16, void* wt, int 
     return cudaGetLastError();
 }
 
-// A: bf16 [terms * M][K], the terms of the activation stacked (terms = 1: the activation itself); Wt: bf16 [wt_rows][K].
-// Returns cudaErrorNotSupported for shapes the tiling does not cover (the caller decides what to do).
 static bool dense_rows_f32(int terms, int M, int N, int K, int sms);
 static cudaError_t run_gemm_f32(const F32Product& p, const void* a_terms, int terms, int splits, cudaStream_t st);
 
+// A: bf16 [terms * M][K], the terms of the activation stacked (terms = 1: the activation itself); Wt: bf16 [wt_rows][K].
+// Returns cudaErrorNotSupported for shapes the tiling does not cover (the caller decides what to do).
 cudaError_t launch_gemm_tcgen05_bf16(const void* a_bf16, int terms, const void* wt, long long wt_rows, float* y, int M, int N,
                                      int K, const GemmEpilogue& ep, const GemmGroups* groups, cudaStream_t st) {
     if (!gemm_tcgen05_shape_ok(M, N, K) || terms < 1 || terms > kTerms || wt_rows < N) return cudaErrorNotSupported;
@@ -842,7 +840,7 @@ bool gemm_f32_ok(const F32Product& p) {
 
 // Which kernel takes a product of M fp32 rows.  Up to 32 rows the few-rows kernel (N = 2048, K = 1024, 32 rows: 25 us on the 128 x 256
 // tiles, 11 here; N = K = 2048: 42 and 22).
-static bool dense_rows_few(int M) { return M <= kGemmFewRowsGroup; }
+static bool dense_rows_few(int M) { return M <= kGemmFewRowsMost; }
 // CTAs that share a 128 x 128 tile of the fp32-sum kernel: as many as the chip has room for, two k-blocks each at least
 static int f32_splits(int tiles, int n_kb, int most, int sms) {
     int s = 1;
@@ -901,31 +899,29 @@ cudaError_t launch_gemm_f32(const F32Product& p, void* work, cudaStream_t st) {
 static size_t few_rows_smem(int NB, int kb_per, int n_slots) {
     return 1024 + (size_t)n_slots * kTileBytes + (size_t)kb_per * NB * 128 + (size_t)(NB / 3 / 8 * 8) * BM * 4;
 }
-// CTAs of a cluster: enough of them to fill the chip, at least two k-blocks each (for one group of rows a rule on N and K alone, so
-// that a row's sums do not depend on what shares its step); several groups also split until two CTAs fit an SM
-static int few_rows_split(int NB, int N, int K, int groups) {
+// CTAs of a cluster: enough of them to fill the chip, at least two k-blocks each (a rule on N and K alone, so that a row's sums do not
+// depend on what shares its step)
+static int few_rows_split(int N, int K) {
     const int tiles = (N + BM - 1) / BM, n_kb = (K + BK - 1) / BK;
     int s = 1;
-    while (s < 8 && n_kb >= 4 * s && (tiles * groups * s < 120 || (groups > 1 && few_rows_smem(NB, (n_kb + s - 1) / s, 2) > kRSmemMost / 2))) s *= 2;
+    while (s < 8 && n_kb >= 4 * s && tiles * s < 120) s *= 2;
     return s;
 }
 
 bool gemm_few_rows_ok(const FewRowsProduct& p) {
-    const int groups = (p.M + kGemmFewRowsGroup - 1) / kGemmFewRowsGroup, NB = p.M <= 8 ? 32 : 96;
-    if (p.M <= 0 || groups > 65535 || p.N <= 0 || p.K < BK || p.K % 8 || p.lda % 4 || (reinterpret_cast<uintptr_t>(p.a) & 15) ||
+    if (p.M <= 0 || p.M > kGemmFewRowsMost || p.N <= 0 || p.K < BK || p.K % 8 || p.lda % 4 || (reinterpret_cast<uintptr_t>(p.a) & 15) ||
         (reinterpret_cast<uintptr_t>(p.w) & 15))
         return false;
-    const int n_kb = (p.K + BK - 1) / BK, s = few_rows_split(NB, p.N, p.K, groups), kb_per = (n_kb + s - 1) / s;
-    return few_rows_smem(NB, kb_per, std::min(kb_per, 2)) <= kRSmemMost;
+    const int n_kb = (p.K + BK - 1) / BK, s = few_rows_split(p.N, p.K), kb_per = (n_kb + s - 1) / s;
+    return few_rows_smem(p.M <= 8 ? 32 : 96, kb_per, std::min(kb_per, 2)) <= kRSmemMost;
 }
 
 template <int NB>
 static cudaError_t launch_few_rows(const FewRowsProduct& p, bool early, cudaStream_t st) {
-    const int groups = (p.M + kGemmFewRowsGroup - 1) / kGemmFewRowsGroup;
-    const int n_kb = (p.K + BK - 1) / BK, s = few_rows_split(NB, p.N, p.K, groups), kb_per = (n_kb + s - 1) / s;
+    const int n_kb = (p.K + BK - 1) / BK, s = few_rows_split(p.N, p.K), kb_per = (n_kb + s - 1) / s;
     // two CTAs per SM where at least three slots fit: the next launch's weights are then requested while this one still runs
     int n_slots = std::min(kRSlotsMost, kb_per);
-    while (n_slots > (groups > 1 ? 2 : 3) && few_rows_smem(NB, kb_per, n_slots) > kRSmemMost / 2) --n_slots;
+    while (n_slots > 3 && few_rows_smem(NB, kb_per, n_slots) > kRSmemMost / 2) --n_slots;
     while (few_rows_smem(NB, kb_per, n_slots) > kRSmemMost) --n_slots;
     const size_t smem = std::max<size_t>(few_rows_smem(NB, kb_per, n_slots), kRSmemLeast);
     // (the same size for every launch: another thread's cannot lower what this one needs)
@@ -934,7 +930,7 @@ static cudaError_t launch_few_rows(const FewRowsProduct& p, bool early, cudaStre
     CUtensorMap mw;
     if (!make_map(&mw, p.w, p.N, p.K, BM)) return cudaErrorNotSupported;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((p.N + BM - 1) / BM, s, groups);
+    cfg.gridDim = dim3((p.N + BM - 1) / BM, s);
     cfg.blockDim = dim3(kRThreads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;

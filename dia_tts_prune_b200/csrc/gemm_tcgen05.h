@@ -53,11 +53,11 @@ bool gemm_f32_ok(const F32Product& p);
 inline size_t gemm_f32_work_bytes(size_t rows, size_t columns) { return 6 * rows * columns; }      // columns: heads * K
 cudaError_t launch_gemm_f32(const F32Product& p, void* work, cudaStream_t st);
 
-// The same for a few rows (decoding, a text): Y[m][n] = [add +] act(sum_k A[m][k] W[n][k]).  The weights are the 128-row operand and
-// stream once for 32 rows; the rows' three terms are the columns of the other operand.  Up to 32 rows a sum's order depends on N and
-// K (and on whether there are more than 8 rows) only.
+// The same for at most 32 rows (decoding, a short text): Y[m][n] = [add +] act(sum_k A[m][k] W[n][k]).  The weights are the 128-row
+// operand and stream once for all rows; the rows' three terms are the columns of the other operand.  A sum's order depends on N and K
+// (and on whether there are more than 8 rows) only.
 // early: launched with programmatic stream serialization (the weights are requested before the predecessor has ended).
-constexpr int kGemmFewRowsGroup = 32;
+constexpr int kGemmFewRowsMost = 32;
 struct FewRowsProduct {
     const float* a; int lda;
     const void* w;
