@@ -89,17 +89,21 @@ __device__ __forceinline__ float gelu_to_bf16_range(float z) {
     return __fdividef(z, 1.0f + __expf(fminf(-u2, 80.f)));
 }
 
-// x = hi + lo + lo2 per element, three stacked bf16 matrices [3][M][K]
+// v = t0 + t1 + t2 in bf16.  An infinity stays one, alone; a number within half a bf16 unit of the largest ones, which would round up to
+// an infinity, is rounded towards zero instead.
+__device__ __forceinline__ void split3(float v, __nv_bfloat16& t0, __nv_bfloat16& t1, __nv_bfloat16& t2) {
+    constexpr float most = 3.402823466e38f;
+    t0 = __float2bfloat16_rn(v);
+    if (fabsf(__bfloat162float(t0)) > most && fabsf(v) <= most) t0 = __float2bfloat16_rz(v);
+    const float f0 = __bfloat162float(t0), r1 = fabsf(f0) <= most ? v - f0 : 0.f;
+    t1 = __float2bfloat16_rn(r1);
+    t2 = __float2bfloat16_rn(r1 - __bfloat162float(t1));
+}
+
+// three terms per element, three stacked bf16 matrices [3][M][K]
 __global__ void split3_rows_kernel(const float* __restrict__ x, __nv_bfloat16* __restrict__ xs, long long n) {
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        const float v = x[i];
-        const __nv_bfloat16 h = __float2bfloat16_rn(v);
-        const float r1 = v - __bfloat162float(h);
-        const __nv_bfloat16 l = __float2bfloat16_rn(r1);
-        const float r2 = r1 - __bfloat162float(l);
-        xs[i] = h;
-        xs[n + i] = l;
-        xs[2 * n + i] = __float2bfloat16_rn(r2);
+        split3(x[i], xs[i], xs[n + i], xs[2 * n + i]);
     }
 }
 
@@ -129,14 +133,8 @@ __global__ void __launch_bounds__(256) split3_norm_rows_kernel(const float* __re
             reinterpret_cast<float*>(out)[(size_t)row * K + i] = v;
             continue;
         }
-        const __nv_bfloat16 h = __float2bfloat16_rn(v);
-        const float r1 = v - __bfloat162float(h);
-        const __nv_bfloat16 l = __float2bfloat16_rn(r1);
-        const float r2 = r1 - __bfloat162float(l);
         const size_t o = (size_t)row * K + i;
-        xs[o] = h;
-        xs[n + o] = l;
-        xs[2 * n + o] = __float2bfloat16_rn(r2);
+        split3(v, xs[o], xs[n + o], xs[2 * n + o]);
     }
 }
 
@@ -631,10 +629,7 @@ dia_gemm_few_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid
         __nv_bfloat16 t[3][8];
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
-            t[0][e] = __float2bfloat16_rn(v[e]);
-            const float f0 = __bfloat162float(t[0][e]), r1 = fabsf(f0) <= 3.402823466e38f ? v[e] - f0 : 0.f;
-            t[1][e] = __float2bfloat16_rn(r1);
-            t[2][e] = __float2bfloat16_rn(r1 - __bfloat162float(t[1][e]));
+            split3(v[e], t[0][e], t[1][e], t[2][e]);
         }
 #pragma unroll
         for (int q = 0; q < 3; ++q) {
@@ -734,7 +729,7 @@ dia_gemm_few_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid
     if (S > 1) cluster_sync_all();                            // (the partial sums stay until every CTA has read them)
 }
 
-// three bf16 terms of every head's columns, [3][heads][M][K]; an infinity stays one in the first term
+// three bf16 terms of every head's columns, [3][heads][M][K]
 __global__ void __launch_bounds__(256) split3_heads_kernel(const float* __restrict__ x, int ldx, int hs, __nv_bfloat16* __restrict__ xs, int H, int M, int K) {
     const size_t n = (size_t)H * M * K;
     const float* row = x + (size_t)blockIdx.x * ldx;
@@ -744,11 +739,7 @@ __global__ void __launch_bounds__(256) split3_heads_kernel(const float* __restri
         __nv_bfloat16 t[3][4];
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-            const float v = row[(size_t)h * hs + k + e];
-            t[0][e] = __float2bfloat16_rn(v);
-            const float f0 = __bfloat162float(t[0][e]), r1 = fabsf(f0) <= 3.402823466e38f ? v - f0 : 0.f;
-            t[1][e] = __float2bfloat16_rn(r1);
-            t[2][e] = __float2bfloat16_rn(r1 - __bfloat162float(t[1][e]));
+            split3(row[(size_t)h * hs + k + e], t[0][e], t[1][e], t[2][e]);
         }
 #pragma unroll
         for (int q = 0; q < 3; ++q) *reinterpret_cast<uint2*>(xs + q * n + o) = *reinterpret_cast<const uint2*>(t[q]);

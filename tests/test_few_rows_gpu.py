@@ -28,3 +28,18 @@ def test_chains_of_early_launches(requests):
         first = out if first is None else first
         assert torch.equal(out, first)
     assert torch.isfinite(first).all()
+
+
+@pytest.mark.parametrize("M", [4, 200, 2000])
+def test_the_largest_numbers(M):
+    """Numbers that a bf16 would round up to an infinity, in dense layers of few, some and many rows; an infinity stays one.  The bound on the
+    others is that of fp32 sums of 64 products: 2^-21 of the result, a few times over."""
+    from dia_tts_prune_b200 import engine as E
+    g = torch.Generator().manual_seed(M)
+    x, w = torch.randn(M, 128, generator=g), (torch.rand(128, 64, generator=g) * 1e-3 + 1e-4).to(torch.bfloat16)
+    x[0, 3], x[1, 7], x[3, 9] = 3.4e38, -3.4028234e38, torch.inf
+    y = E.dense_forward(x.cuda(), E.dense_prepare_weight(w.cuda())).cpu().double()
+    ref = x.double() @ w.double()
+    assert (y[3] == torch.inf).all()
+    rows = torch.arange(M) != 3
+    assert ((y - ref)[rows].abs() / ref[rows].abs().amax(-1, keepdim=True)).max() <= 1e-5
