@@ -35,6 +35,7 @@
 
 #include "attention_split.h"
 #include "common.cuh"
+#include "gemm_tcgen05.h"
 
 namespace dia {
 
@@ -1237,7 +1238,10 @@ cudaError_t launch_inst(const SplitAttention& a, const Geometry& g, size_t smem,
     const cudaError_t e = cudaFuncSetAttribute(split_attention_kernel<NVS>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMost);
     if (e != cudaSuccess) return e;
     const int tt = kRows >> g.pk_shift, tiles = a.n_seq > 1 ? a.M / tt + a.n_seq : (a.M + tt - 1) / tt;
-    if (a.work) split_keys_kernel<<<dim3(std::min(g.cap_tiles, std::max(1, kSplitGrid / g.parts)), g.parts), 256, 0, st>>>(a, g);
+    if (a.work) {
+        split_keys_kernel<<<dim3(std::min(g.cap_tiles, std::max(1, kSplitGrid / g.parts)), g.parts), 256, 0, st>>>(a, g);
+        ++extra_launches();
+    }
     split_attention_kernel<NVS><<<(a.heads >> g.pk_shift) * tiles, kSplitThreadsTC, smem, st>>>(a, g);
     return cudaGetLastError();
 }

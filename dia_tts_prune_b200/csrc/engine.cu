@@ -8,6 +8,7 @@
 #include <cstring>
 #include <new>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "common.cuh"
@@ -996,7 +997,7 @@ int dia_b200_dense_forward_fused(const float* x, const float* norm_weight, float
     cudaError_t e = launch_gemm_tcgen05(x, norm_weight, eps, wt_bf16, residual, y, workspace, M, N, K, S(stream));
     if (e == cudaErrorNotSupported) { (void)cudaGetLastError(); return DIA_B200_EUNSUPPORTED; }
     CK(e);
-    g_launches += M > kGemmFewRowsMost || norm_weight ? 2 : 1;
+    g_launches += 1 + std::exchange(extra_launches(), 0);
     return DIA_B200_OK;
 }
 

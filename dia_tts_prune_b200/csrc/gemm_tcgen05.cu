@@ -884,6 +884,7 @@ static cudaError_t run_gemm_f32(const F32Product& p, const void* a_terms, int te
 cudaError_t launch_gemm_f32(const F32Product& p, void* work, cudaStream_t st) {
     if (!gemm_f32_ok(p)) return cudaErrorNotSupported;
     split3_heads_kernel<<<p.M, 256, 0, st>>>(p.a, p.lda, p.a_hs, reinterpret_cast<__nv_bfloat16*>(work), p.heads, p.M, p.K);
+    ++extra_launches();
     return run_gemm_f32(p, work, kTerms, 1, st);
 }
 
@@ -953,7 +954,10 @@ cudaError_t launch_gemm_tcgen05(const float* x, const float* norm_w, float eps, 
         // (the rows are read while outputs are written)
         const bool apart = norm_w || x + n <= y || y + (long long)M * N <= x;
         if (apart && gemm_few_rows_ok(few)) {
-            if (norm_w) split3_norm_rows_kernel<false><<<M, 256, 0, st>>>(x, norm_w, eps, workspace, M, K);
+            if (norm_w) {
+                split3_norm_rows_kernel<false><<<M, 256, 0, st>>>(x, norm_w, eps, workspace, M, K);
+                ++extra_launches();
+            }
             return launch_gemm_few_rows(few, false, st);
         }
     }
@@ -962,6 +966,7 @@ cudaError_t launch_gemm_tcgen05(const float* x, const float* norm_w, float eps, 
     else
         split3_rows_kernel<<<(int)std::min<long long>((n + 255) / 256, 148 * 16), 256, 0, st>>>(
             x, reinterpret_cast<__nv_bfloat16*>(workspace), n);
+    ++extra_launches();
     const F32Product wide{nullptr, 0, 0, wt, y, N, N, nullptr, 1, M, N, K, 1.f, 0, nullptr, 0, 0, residual};
     int dev = 0, sms = 0;
     cudaError_t e = cudaGetDevice(&dev);

@@ -29,6 +29,12 @@ struct GemmGroups {
 };
 
 // K a multiple of 8 (16-byte rows for the TMA), N a multiple of 4 (float4 stores)
+// Kernels that launchers on this thread launched beyond one per call, for the caller that counts launches (it takes them)
+inline long long& extra_launches() {
+    static thread_local long long n = 0;
+    return n;
+}
+
 inline bool gemm_tcgen05_shape_ok(int M, int N, int K) { return M > 0 && N > 0 && K >= 8 && K % 8 == 0 && N % 4 == 0; }
 
 cudaError_t launch_gemm_tcgen05_bf16(const void* a_bf16, int terms, const void* wt, long long wt_rows, float* y, int M, int N,

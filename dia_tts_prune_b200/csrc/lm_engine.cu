@@ -86,6 +86,7 @@
 #include <map>
 #include <new>
 #include <tuple>
+#include <utility>
 #include <vector>
 
 #include <cuda_runtime.h>
@@ -120,7 +121,7 @@ inline int cuda_fail(cudaError_t e) {
     do {                                                \
         cudaError_t e__ = (call);                       \
         if (e__ != cudaSuccess) return cuda_fail(e__);  \
-        g_launches++;                                   \
+        g_launches += 1 + std::exchange(dia::extra_launches(), 0); \
     } while (0)
 
 inline cudaStream_t S(void* s) { return reinterpret_cast<cudaStream_t>(s); }

@@ -43,3 +43,30 @@ def test_the_largest_numbers(M):
     assert (y[3] == torch.inf).all()
     rows = torch.arange(M) != 3
     assert ((y - ref)[rows].abs() / ref[rows].abs().amax(-1, keepdim=True)).max() <= 1e-5
+
+
+def test_launches_are_counted_kernel_by_kernel():
+    """The launch counters against the kernels that a profiler sees: products that prepare their operand, attention that splits its keys first"""
+    import test_attention_rows_alone_gpu as A
+
+    from dia_tts_prune_b200 import engine as E
+    from dia_tts_prune_b200.lm_engine import launch_count
+    model, n_in, op = A.grouped(8, 1, 64, 0, 0, 0.0, 64)
+    x = torch.randn(200, n_in, generator=torch.Generator().manual_seed(1)).cuda()
+    seq = model.state.open("a")
+    model.state.reserve(seq, 200)
+    lat, lat_in, lat_op = A.latent(4, 32, 64, 16, 64, 0)
+    h = torch.randn(40, lat_in, generator=torch.Generator().manual_seed(2)).cuda()
+    lseq = lat.state.open("a")
+    lat.state.reserve(lseq, 40)
+    w = E.dense_prepare_weight(torch.randn(128, 256).to(torch.bfloat16).cuda())
+    nw = torch.rand(128).cuda()
+    own = lambda names: sum("dia::" in n or "lm::" in n or "dia_" in n for n in names)                    # noqa: E731
+    for count, call in [(launch_count, lambda: op(x[:200], [(seq, 200, 0)])), (launch_count, lambda: op(x[:12], [(seq, 12, 0)])),
+                        (launch_count, lambda: lat_op(h, [(lseq, 40, 0)])),
+                        *[(E.launch_count, lambda M=M, n=n: E.dense_forward(torch.randn(M, 128).cuda(), w, norm_weight=n))
+                          for M in (4, 40, 4000) for n in (None, nw)]]:
+        seen = own(A.kernels_of(call))
+        before = count()
+        call()
+        assert count() - before == seen, seen
