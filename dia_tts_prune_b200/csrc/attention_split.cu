@@ -24,8 +24,10 @@
 //
 // Bound: per 64 keys and 128 rows 3 x 128 x 64 x (dk + dv) multiply-adds on the tensor pipe (1536 cycles at 128 + 128) against
 // about as many issue slots for splitting and softmax.
-// Every wait is bounded: a wait that runs out makes the CTA write NaN and end.
+// Every wait is bounded: a wait that runs out makes the CTA write NaN, note it in a word that the host reads, and end; the next launch
+// on the device returns an error.
 #include <algorithm>
+#include <mutex>
 
 #include <cuda_fp16.h>
 #include <cuda_bf16.h>
@@ -65,6 +67,7 @@ struct Geometry {
     // tile's parts: key groups (per kv head where the launch reads one head at a time), then value groups; its sets of scales: the keys
     // of each kv head, then the values of each (shared_kv: the keys' only)
     int parts, k_parts, sets, cap_tiles;
+    int* ran_out;                            // the device's word (null: none)
     unsigned tile_bytes, scale_off, tile_off;
 };
 // where the tiles of a slot's sequence lie: tile j / 64 of its keys is tile base + j / 64 of the room for first <= j / 64 < end; its
@@ -890,6 +893,10 @@ split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_co
         if (p.head_gate && tok < n_tok) f *= p.head_gate[(size_t)(r0 + tok) * p.ldg + h];
         if (t == 0 && ok) asm volatile("bar.sync 1, 256;" ::: "memory");    // (no keys: all warps' queries are stored first)
         ok = __all_sync(0xffffffffu, ok);
+        if (!ok && lane == 0 && geo.ran_out) {
+            *reinterpret_cast<volatile int*>(geo.ran_out) = 1;
+            __threadfence_system();
+        }
         const int c0 = NVS == 1 ? hf * half : hf * 128, ldst = half + 4;
         float* stage = reinterpret_cast<float*>(smem) + (size_t)warp * 32 * ldst;
 #pragma unroll
@@ -1248,6 +1255,26 @@ cudaError_t launch_inst(const SplitAttention& a, const Geometry& g, size_t smem,
 
 }  // namespace
 
+// A word of `device` in mapped host memory, which a kernel sets when one of its waits has run out (null: there is none yet, and a stream
+// that is being captured is no place to make one)
+int* split_attention_ran_out(int device, cudaStream_t st) {
+    static std::mutex lock;
+    static int* words[64] = {};
+    if (device < 0 || device >= 64) return nullptr;
+    const std::lock_guard<std::mutex> hold(lock);
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (!words[device] && cudaStreamIsCapturing(st, &capture) == cudaSuccess && capture == cudaStreamCaptureStatusNone) {
+        int* w = nullptr;
+        if (cudaHostAlloc(reinterpret_cast<void**>(&w), sizeof(int), cudaHostAllocMapped) == cudaSuccess) {
+            *w = 0;
+            words[device] = w;
+        } else {
+            (void)cudaGetLastError();
+        }
+    }
+    return words[device];
+}
+
 bool split_attention_ok(const SplitAttention& a) {
     Geometry g;
     size_t smem;
@@ -1265,6 +1292,14 @@ cudaError_t launch_split_attention(const SplitAttention& a, cudaStream_t st) {
     Geometry g;
     size_t smem;
     if (a.M <= 0 || !geometry_of(a, g, smem)) return cudaErrorNotSupported;
+    int device = 0;
+    const cudaError_t e = cudaGetDevice(&device);
+    if (e != cudaSuccess) return e;
+    g.ran_out = split_attention_ran_out(device, st);          // (mapped and unified: one address on both sides)
+    if (g.ran_out && *reinterpret_cast<volatile int*>(g.ran_out)) {
+        *g.ran_out = 0;
+        return cudaErrorLaunchTimeout;
+    }
     SplitAttention with = a;
     if (g.cap_tiles <= 0 || (long long)a.M * (a.heads / a.kv_heads) < kSplitOnceRows) with.work = nullptr;
     return g.n_vst == 1 ? launch_inst<1>(with, g, smem, st) : launch_inst<2>(with, g, smem, st);

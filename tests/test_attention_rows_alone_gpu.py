@@ -245,3 +245,21 @@ def test_the_widest_latent_rows(heads):
     whole = op(x, [(seq, 200, 0)]).clone()
     short = torch.cat([op(x[a:a + 8], [(seq, 8, a)]) for a in range(0, 200, 8)])
     assert (whole - short).abs().max() <= 2e-5 * short.abs().max()
+
+
+def test_a_wait_that_ran_out_reaches_the_caller():
+    """The word that a kernel sets when a wait of its ran out, set by hand: the next launch returns an error, the one after it runs"""
+    import ctypes as C
+
+    from dia_tts_prune_b200 import _lib
+    from dia_tts_prune_b200 import engine as E
+    q, k, v = torch.randn(1, 256, 2, 128).cuda(), torch.randn(1, 1, 256, 128).cuda(), torch.randn(1, 1, 256, 128).cuda()
+    good = E.attention_rows(q, k, v, 256, 0, None)
+    word_of = getattr(_lib.load(), "_ZN3dia23split_attention_ran_outEiP11CUstream_st")
+    word_of.restype, word_of.argtypes = C.POINTER(C.c_int), [C.c_int, C.c_void_p]
+    word = word_of(torch.cuda.current_device(), None)
+    assert word and word[0] == 0
+    word[0] = 1
+    with pytest.raises(Exception):
+        E.attention_rows(q, k, v, 256, 0, None)
+    assert word[0] == 0 and torch.equal(E.attention_rows(q, k, v, 256, 0, None), good)
