@@ -14,13 +14,17 @@
 //                   product of the tile before is added to the row's fp32 registers
 // The accumulator of a tensor-core product loses up to one unit in the last place at every step, towards zero (measured: 2e-6
 // over K = 2048).  So no accumulator lives longer than one tile and one channel group, and sums over tiles are fp32 additions
-// in registers: measured against 64 bits the output is as close as the fp32 FMA kernels' (2.6e-7 both at 300 rows, d = 128).
+// in registers: measured against 64 bits the output is closer than the fp32 FMA kernels' (relative 2-norm, 300 rows, two heads of 128,
+// capped: 2.4e-7 against 2.9e-7; 1500 rows, 4 heads of 128: 2.7e-7 against 4.1e-7).
 //
 // Scaling: every query row, key row and value row is brought to a largest magnitude of [2^14, 2^15) by a power of two of its own
 // before the split.  A query's and a key's are undone on the score; a value's joins the weight, and the weights of a row and a tile
 // of keys, times their values' magnitudes, are brought to the same range before they are split.  So an element down to 2^-17 of its
-// row's largest keeps its 22 bits, what a row of the output sums loses at most 2^-39 of the largest weight x value that it sees, and
-// nothing of a token that it does not see, or of another row, enters its result: the bits do not depend on what shares the launch.
+// row's largest keeps its 22 bits (a smaller one is off by at most 2^-39 of the largest: a channel that is 2^17 times below the others of
+// its tokens has fewer), and nothing of a token that a row does not see, or of another row, enters its result: the bits do not depend on
+// what shares the launch.  Cost, against one scale per tile of rows, keys and values: 4096 rows, 16 heads of 128 over 4, window 1024
+// 237 -> 264 us; mixed scores, three prompts of 2048 rows, 8 heads of 128 over 2, 127 -> 146, of which the factors per key and per
+// value 5 us each; 16 keys that share a factor (scales in steps of 2^8) take as long.
 //
 // Bound: per 64 keys and 128 rows 3 x 128 x 64 x (dk + dv) multiply-adds on the tensor pipe (1536 cycles at 128 + 128) against
 // about as many issue slots for splitting and softmax.
@@ -476,9 +480,9 @@ template <int NVS>
 __global__ void __launch_bounds__(kSplitThreadsTC, 1)
 split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_constant__ Geometry geo) {
     constexpr int DVH = 64 * NVS;                             // output channels of a thread
-    // The block is launched with 128 registers a thread: 256 of kRowRegs, 128 of kFetchRegs and 128 of 32.  (latent_4096's attention, wide
-    // values: 184 and 112 452 us, 192 and 96 443, 200 and 80 421: what the fetching warps spill is used for keys that are not split in
-    // advance only.)
+    // The block is launched with 128 registers a thread: 256 of kRowRegs, 128 of kFetchRegs and 128 of 32.  (Wide values, 4096 rows, 16
+    // heads over latent rows of 256 + 32, window 1024: 184 and 112 452 us, 192 and 96 443, 200 and 80 421.  What the fetching warps
+    // spill is used for keys that are not split in advance only.)
     constexpr int kRowRegs = NVS == 1 ? 176 : 200, kFetchRegs = NVS == 1 ? 128 : 80;
     static_assert(256 * kRowRegs + 128 * kFetchRegs + 128 * 32 <= 128 * kSplitThreadsTC, "registers of the block");
     extern __shared__ __align__(128) unsigned char smem[];

@@ -1,8 +1,9 @@
 // attention_split.h - softmax attention for many query rows on the tensor cores (attention_split.cu).
 //
 // Queries, keys, values and softmax weights are fp32; every product takes them as two fp16 terms of a scaled value (22
-// significand bits) and is accumulated in fp32.  Serves grouped-query attention over paged keys and values, attention over one
-// cached latent per position (the value is the head of the key row), and attention whose scores are mixed across heads.
+// significand bits) and is accumulated in fp32.  A row's result depends on the row and the keys that it sees alone.  Serves
+// grouped-query attention over paged keys and values, attention over one cached latent per position (the value is the head of the
+// key row), and attention whose scores are mixed across heads.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -43,7 +44,10 @@ struct SplitAttention {
     void* work; size_t work_bytes; int n_slots;
 };
 
-// whether the kernel takes the shape (head sizes, alignment); M does not matter
+// Whether the kernel takes the shape; M does not matter.  Channel counts and strides that are multiples of 4 on 16-byte aligned pointers, values
+// of at most 256 channels, keys of at most 4 groups of 128 (mixed scores: as many key heads of at most 128) for which tensor memory has the
+// columns, and shared memory for the queries of 128 (token, head) rows beside two slots of 64 keys: latent rows of 256 + 64 channels fit
+// from 4 heads on, mixed scores with 4 key heads of 128 channels do not.
 bool split_attention_ok(const SplitAttention& a);
 // bytes of `work` for `keys` keys of this shape (0: the shape is not taken)
 size_t split_attention_work_bytes(const SplitAttention& a, int keys);

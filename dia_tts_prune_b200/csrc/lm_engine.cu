@@ -71,13 +71,16 @@
 // the softmax over all router outputs with a choice correction, groups, identity experts (they add weight x input inside
 // the next streams_step or down_combine_rows) and a sigmoid gate number on the shared unit (a column of the router logits).
 //
-// Products.  With float32 precision every product runs on the fp32 FMA kernels.  With bfloat16 precision a step of at
+// Products.  With float32 precision every product has fp32 accuracy: a row or two, and 3 to 8 rows of small matrices, run on the
+// fp32 FMA row kernels, 3 to 8 rows of large matrices and longer steps on the tensor cores with the operand in three bf16 terms and
+// fp32 sums (linear_f32).  With bfloat16 precision a step of at
 // least kTensorRowsMin rows (a prompt portion) runs its products on the tensor cores (the tcgen05 kernel of
 // gemm_tcgen05.cu, bf16 operands, fp32 accumulation in tensor memory): the norm / attention / gate kernels write the
 // bf16 operand beside their fp32 result, the expert groups are packed (gathered, scaled by the router score, padded to
 // the 128-row tile) into one bf16 operand, and the output projection's epilogue applies the DynamicTanh and adds the
-// residual stream.  Shorter steps (decoding) stream the weights once per row on the row kernels.  The router, norms,
-// scores, softmax, pages and the residual stream are fp32 in both.
+// residual stream.  Shorter steps run their products as with float32 precision: 3 rows and more of large matrices read the
+// weights once for all rows, otherwise the row kernels read them once per row.  The attention of more than 8 rows splits its fp32
+// operands into fp16 pairs, 22 bits (attention_split.cu).  The router, norms, softmax, pages and the residual stream are fp32 in both.
 #include <algorithm>
 #include <atomic>
 #include <cmath>
@@ -173,7 +176,7 @@ struct lm_b200_engine {
 namespace {
 
 constexpr int kTensorRowsMin = 32;               // rows of a step from which its products run on the tensor cores
-constexpr int kFewRowsOutMost = 16384;           // outputs up to which a product of a few rows runs on the tensor cores
+constexpr int kFewRowsOutMost = 16384;           // outputs up to which a product of a few rows runs there: one round of its 128-output tiles
 constexpr int kHeadTensorRowsMin = 4;            // wanted rows from which the head does
 
 // assignment slots of `rows` rows when every expert group is padded to `pad` slots
@@ -192,8 +195,8 @@ const dia::GemmEpilogue kPlain{nullptr, nullptr, nullptr, 0.f, nullptr};
 // kernel, which reads them once per row, is the faster one while rows x weights are few: its weights are requested before its
 // predecessor ends, and it has no operand to prepare (a model of 4 layers at width 2048, 2 / 3 / 8 rows: 388 / 509 / 769 us on the row
 // kernel, 394 / 445 / 444 us here; at width 1024, 3 / 6 / 8 rows: 210 / 261 / 290 against 236 / 268 / 277 us).  Between 8 rows and a
-// prompt portion's bf16 products there are only the 64-row tiles beside it.  (The head stays on the row kernel: a wave and a half
-// of tiles.)
+// prompt portion's bf16 products there are only the 64-row tiles beside it.  (A head of more than kFewRowsOutMost words stays on the
+// row kernel: a round and more of tiles.)
 bool few_rows(const lm_b200_engine* e, int M, int N, int K) {
     if (M <= lm::kRowsKernelMax) return M > 2 && (long long)M * N * K >= 12LL << 20;
     return e->m.precision == LM_B200_PRECISION_BF16 && M < kTensorRowsMin;
@@ -243,8 +246,8 @@ StepView view(const int32_t* step, int M, int n_seq) {
     return v;
 }
 
-// The attention of more than a few rows runs on the tensor cores with split fp32 operands, whatever the precision of the products: its
-// error against 64 bits is that of the fp32 FMA kernels (attention_split.cu).
+// The attention of more than a few rows runs on the tensor cores with split fp32 operands where the kernel takes the shape, whatever the
+// precision of the products: its error against 64 bits is not above that of the fp32 FMA kernels (attention_split.cu).
 struct SplitUse { lm::SplitRoom room; bool use; operator const lm::SplitRoom*() const { return use ? &room : nullptr; } };
 SplitUse split_operands(const lm_b200_engine* e, const StepView& v, int M) {
     return SplitUse{lm::SplitRoom{e->kv_split, e->kv_split_bytes, e->m.n_slots, v.sm, v.n_seq}, M > lm::kAttnRowsKernelMax};

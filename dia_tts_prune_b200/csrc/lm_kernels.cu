@@ -5,9 +5,10 @@
 // portions, single decoded tokens and mixed batches are the same launch sequence.  Every kernel here computes a row's
 // result from that row (and the sequence state it points at) alone, in an order of operations that does not depend on
 // which other rows are in the batch - so the value at a position does not depend on how the prompt was cut or batched.
-// (The only thing the row count selects is which linear and attention kernels run; they sum in different orders, so a position
-// computed in steps of different kinds - a row or two, up to 8 rows, longer; with bf16 products also by the tiles of a long step -
-// agrees to rounding, and to the bit within a kind.)
+// (The row count selects which linear and attention kernels run; they sum in different orders, so a position computed in steps of
+// different sizes agrees to rounding.  To the bit it agrees between steps of one or two rows, and, where the products are fp32, between
+// steps of more than 8 rows: attention and products of those do not depend on what shares the step.  With 3 to 8 rows rows x weights
+// pick the product's kernel, and bf16 products of a long step split their sums by its tiles.)
 //
 // Precision: activations, the residual stream, norms, router, attention scores / weights and the K/V pages are fp32;
 // matrices are bf16 in memory and multiplied with fp32 accumulation.

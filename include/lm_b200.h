@@ -74,8 +74,10 @@ enum lm_b200_router_kind { LM_B200_ROUTER_SIGMOID_INPUT = 0, LM_B200_ROUTER_SOFT
 enum lm_b200_gate_kind { LM_B200_GATE_SIGMOID = 0, LM_B200_GATE_NONE = 1, LM_B200_GATE_SILU = 2, LM_B200_GATE_SIGMOID_HEAD = 3 };
 /* which channels of a head form a rotary pair: (2i, 2i + 1), or (i, i + rot_dims / 2) */
 enum lm_b200_rot_layout { LM_B200_ROT_INTERLEAVED = 0, LM_B200_ROT_HALF = 1 };
-/* FP32: every product is fp32 FMA arithmetic on the stored weights.  BF16: the products of a long step (a prompt portion)
- * run on the tensor cores with bf16 operands and fp32 accumulation; everything else stays fp32. */
+/* FP32: every product has fp32 accuracy on the stored weights (fp32 FMA chains, or on the tensor cores with the activation in three
+ * bf16 terms, 24 bits, and fp32 sums of 64 products).  BF16: the products of a long step (a prompt portion) run on the tensor cores
+ * with bf16 operands and fp32 accumulation.  In both, the attention of a step of more than 8 rows multiplies queries, keys, softmax
+ * weights and values as pairs of fp16 terms (22 bits, scaled per row) with fp32 sums; everything else stays fp32. */
 enum lm_b200_precision { LM_B200_PRECISION_FP32 = 0, LM_B200_PRECISION_BF16 = 1 };
 
 /* DYT: y = tanh(alpha x) w + b.  LAYER: y = (x - mean) / sqrt(var + eps) * w + b with the model's eps.
