@@ -90,14 +90,20 @@ __device__ __forceinline__ float gelu_to_bf16_range(float z) {
 }
 
 // v = t0 + t1 + t2 in bf16.  An infinity stays one, alone; a number within half a bf16 unit of the largest ones, which would round up to
-// an infinity, is rounded towards zero instead.
+// an infinity, is rounded towards zero instead.  (Both show in the remainder: one test on the way of all others.  The terms may go to
+// memory and are not read back.)
 __device__ __forceinline__ void split3(float v, __nv_bfloat16& t0, __nv_bfloat16& t1, __nv_bfloat16& t2) {
-    constexpr float most = 3.402823466e38f;
-    t0 = __float2bfloat16_rn(v);
-    if (fabsf(__bfloat162float(t0)) > most && fabsf(v) <= most) t0 = __float2bfloat16_rz(v);
-    const float f0 = __bfloat162float(t0), r1 = fabsf(f0) <= most ? v - f0 : 0.f;
-    t1 = __float2bfloat16_rn(r1);
-    t2 = __float2bfloat16_rn(r1 - __bfloat162float(t1));
+    __nv_bfloat16 a = __float2bfloat16_rn(v);
+    float r1 = v - __bfloat162float(a);
+    if (!(fabsf(r1) <= 3.402823466e38f)) {
+        const bool finite = fabsf(v) <= 3.402823466e38f;
+        if (finite) a = __float2bfloat16_rz(v);
+        r1 = finite ? v - __bfloat162float(a) : 0.f;
+    }
+    const __nv_bfloat16 b = __float2bfloat16_rn(r1);
+    t0 = a;
+    t1 = b;
+    t2 = __float2bfloat16_rn(r1 - __bfloat162float(b));
 }
 
 // three terms per element, three stacked bf16 matrices [3][M][K]
