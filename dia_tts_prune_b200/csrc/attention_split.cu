@@ -688,7 +688,7 @@ split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_co
         fence_smem_async();
         __syncwarp();
         if (lane == 0) mbar_arrive(q_ready);
-        asm volatile("bar.sync 1, 256;" ::: "memory");          // (the rows' scales)
+        asm volatile("bar.sync 1, 256;" ::: "memory");          // (all queries are stored, and the rows' scales are there)
         const int qt = warp & 3, hf = warp >> 2, row = qt * 32 + lane, tok = row >> geo.pk_shift, h = h0 + (row & (PK - 1));
         const uint32_t lanes = (uint32_t)(qt * 32) << 16;
         const int my_pos = s_pos[tok];
@@ -895,7 +895,6 @@ split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_co
         // the unrolled code; 3500 now)
         float f = tok < n_tok && l > 0.f ? p.out_scale / l : 0.f;
         if (p.head_gate && tok < n_tok) f *= p.head_gate[(size_t)(r0 + tok) * p.ldg + h];
-        if (t == 0 && ok) asm volatile("bar.sync 1, 256;" ::: "memory");    // (no keys: all warps' queries are stored first)
         ok = __all_sync(0xffffffffu, ok);
         if (!ok && lane == 0 && geo.ran_out) {
             *reinterpret_cast<volatile int*>(geo.ran_out) = 1;
