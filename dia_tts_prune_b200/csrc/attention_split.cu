@@ -26,8 +26,9 @@
 // 237 -> 264 us; mixed scores, three prompts of 2048 rows, 8 heads of 128 over 2, 127 -> 146, of which the factors per key and per
 // value 5 us each; 16 keys that share a factor (scales in steps of 2^8) take as long.
 //
-// Bound: per 64 keys and 128 rows 3 x 128 x 64 x (dk + dv) multiply-adds on the tensor pipe (1536 cycles at 128 + 128) against
-// about as many issue slots for splitting and softmax.
+// Bound: the latencies of a row warp's dependent steps.  Per 64 keys and 128 rows 3 x 128 x 64 x (dk + dv) multiply-adds on the tensor
+// pipe (1536 cycles at 128 + 128) stand against about 7000 cycles of a tile, in which two row warps per scheduler issue on a third of
+// them (tensor pipe busy 18 %, shared memory 6 %: profiles/split_kernels_ncu.txt).
 // Every wait is bounded: a wait that runs out makes the CTA write NaN, note it in a word that the host reads, and end; the next launch
 // on the device returns an error.
 #include <algorithm>
