@@ -53,7 +53,7 @@ constexpr int kSplitThreadsTC = 512;
 constexpr int kMaxSlots = 6, kMaxDepth = 5, kMaxKStages = 4;
 constexpr int kSmemMost = 232448;                             // all of it dynamic
 constexpr float kLog2e = 1.4426950408889634f;
-constexpr int kSplitOnceRows = 512;                           // rows of a kv head (M rep) from which the keys are split in advance
+constexpr int kSplitOnceRows = 512;                           // rows of a kv head (M rep) from which keys with values of up to 128 channels are split in advance
 constexpr int kSplitGrid = 148 * 16;                           // CTAs of the launch that splits them
 constexpr unsigned kSpinMost = 4000000u;
 
@@ -1305,7 +1305,10 @@ cudaError_t launch_split_attention(const SplitAttention& a, cudaStream_t st) {
         return cudaErrorLaunchTimeout;
     }
     SplitAttention with = a;
-    if (g.cap_tiles <= 0 || (long long)a.M * (a.heads / a.kv_heads) < kSplitOnceRows) with.work = nullptr;
+    // Wide values are split in advance in every step: the fetching warps have few registers for them (9 and 24 decoding sequences over 1000
+    // cached keys, latent rows of 256 + 32, 4 layers: 1714 and 1833 us split by the row tiles, 1139 and 1250 in advance; over 100 keys 867
+    // and 863)
+    if (g.cap_tiles <= 0 || (g.n_vst == 1 && (long long)a.M * (a.heads / a.kv_heads) < kSplitOnceRows)) with.work = nullptr;
     return g.n_vst == 1 ? launch_inst<1>(with, g, smem, st) : launch_inst<2>(with, g, smem, st);
 }
 

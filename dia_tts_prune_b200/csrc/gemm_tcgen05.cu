@@ -106,6 +106,37 @@ __device__ __forceinline__ void split3(float v, __nv_bfloat16& t0, __nv_bfloat16
     t2 = __float2bfloat16_rn(r1 - __bfloat162float(b));
 }
 
+struct Terms { __nv_bfloat16 t0, t1, t2; };
+__device__ __noinline__ Terms split3_one(float v) {
+    Terms x;
+    split3(v, x.t0, x.t1, x.t2);
+    return x;
+}
+// The same for N neighbours: one test for all of them (of each, it cost a product of 16 rows 10 %: every CTA splits the rows).  A NaN needs
+// no care.
+template <int N>
+__device__ __forceinline__ void split3(const float (&v)[N], __nv_bfloat16 (&t)[3][N]) {
+    float most = 0.f;
+#pragma unroll
+    for (int e = 0; e < N; ++e) most = fmaxf(most, fabsf(v[e]));
+#pragma unroll
+    for (int e = 0; e < N; ++e) {
+        t[0][e] = __float2bfloat16_rn(v[e]);
+        const float r1 = v[e] - __bfloat162float(t[0][e]);
+        t[1][e] = __float2bfloat16_rn(r1);
+        t[2][e] = __float2bfloat16_rn(r1 - __bfloat162float(t[1][e]));
+    }
+    if (most > 3.3895e38f) {
+#pragma unroll
+        for (int e = 0; e < N; ++e) {
+            const Terms x = split3_one(v[e]);
+            t[0][e] = x.t0;
+            t[1][e] = x.t1;
+            t[2][e] = x.t2;
+        }
+    }
+}
+
 // three terms per element, three stacked bf16 matrices [3][M][K]
 __global__ void split3_rows_kernel(const float* __restrict__ x, __nv_bfloat16* __restrict__ xs, long long n) {
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
@@ -633,10 +664,7 @@ dia_gemm_few_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid
             v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w; v[4] = y.x; v[5] = y.y; v[6] = y.z; v[7] = y.w;
         }
         __nv_bfloat16 t[3][8];
-#pragma unroll
-        for (int e = 0; e < 8; ++e) {
-            split3(v[e], t[0][e], t[1][e], t[2][e]);
-        }
+        split3(v, t);
 #pragma unroll
         for (int q = 0; q < 3; ++q) {
             const int r = q * Mp + m;
@@ -742,11 +770,11 @@ __global__ void __launch_bounds__(256) split3_heads_kernel(const float* __restri
     for (int i = threadIdx.x; i < H * (K >> 2); i += 256) {   // (K a multiple of 8)
         const int h = i / (K >> 2), k = 4 * (i - h * (K >> 2));
         const size_t o = ((size_t)h * M + blockIdx.x) * K + k;
+        float v[4];
         __nv_bfloat16 t[3][4];
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            split3(row[(size_t)h * hs + k + e], t[0][e], t[1][e], t[2][e]);
-        }
+        for (int e = 0; e < 4; ++e) v[e] = row[(size_t)h * hs + k + e];
+        split3(v, t);
 #pragma unroll
         for (int q = 0; q < 3; ++q) *reinterpret_cast<uint2*>(xs + q * n + o) = *reinterpret_cast<const uint2*>(t[q]);
     }
