@@ -89,9 +89,9 @@ __device__ __forceinline__ float gelu_to_bf16_range(float z) {
     return __fdividef(z, 1.0f + __expf(fminf(-u2, 80.f)));
 }
 
-// v = t0 + t1 + t2 in bf16.  An infinity stays one, alone; a number within half a bf16 unit of the largest ones, which would round up to
-// an infinity, is rounded towards zero instead.  (Both show in the remainder: one test on the way of all others.  The terms may go to
-// memory and are not read back.)
+// v = t0 + t1 + t2 in bf16.  An infinity stays one, alone; the largest numbers, which would round up to an infinity, are rounded towards
+// zero in their first term.  (Both show in the remainder: one test on the way of all others.  The terms may go to memory and are not
+// read back.)
 __device__ __forceinline__ void split3(float v, __nv_bfloat16& t0, __nv_bfloat16& t1, __nv_bfloat16& t2) {
     __nv_bfloat16 a = __float2bfloat16_rn(v);
     float r1 = v - __bfloat162float(a);
@@ -105,36 +105,15 @@ __device__ __forceinline__ void split3(float v, __nv_bfloat16& t0, __nv_bfloat16
     t1 = b;
     t2 = __float2bfloat16_rn(r1 - __bfloat162float(b));
 }
-
-struct Terms { __nv_bfloat16 t0, t1, t2; };
-__device__ __noinline__ Terms split3_one(float v) {
-    Terms x;
-    split3(v, x.t0, x.t1, x.t2);
-    return x;
-}
-// The same for N neighbours: one test for all of them (of each, it cost a product of 16 rows 10 %: every CTA splits the rows).  A NaN needs
-// no care.
-template <int N>
-__device__ __forceinline__ void split3(const float (&v)[N], __nv_bfloat16 (&t)[3][N]) {
-    float most = 0.f;
-#pragma unroll
-    for (int e = 0; e < N; ++e) most = fmaxf(most, fabsf(v[e]));
-#pragma unroll
-    for (int e = 0; e < N; ++e) {
-        t[0][e] = __float2bfloat16_rn(v[e]);
-        const float r1 = v[e] - __bfloat162float(t[0][e]);
-        t[1][e] = __float2bfloat16_rn(r1);
-        t[2][e] = __float2bfloat16_rn(r1 - __bfloat162float(t[1][e]));
-    }
-    if (most > 3.3895e38f) {
-#pragma unroll
-        for (int e = 0; e < N; ++e) {
-            const Terms x = split3_one(v[e]);
-            t[0][e] = x.t0;
-            t[1][e] = x.t1;
-            t[2][e] = x.t2;
-        }
-    }
+// The same with every first term rounded towards zero (8 bits, the nearest 8 of the other 16, the at most 8 that are left): no test, for the
+// kernels whose accumulators live for 64 products (the test cost a product of 16 rows, whose every CTA splits the rows, 21.0 -> 22.5
+// us; sums of all K products in tensor memory, which cuts off, are closer with terms of either sign: 861 rows through Dia's decoder
+// 2.8e-5 against 3.0e-5)
+__device__ __forceinline__ void split3_down(float v, __nv_bfloat16& t0, __nv_bfloat16& t1, __nv_bfloat16& t2) {
+    t0 = __float2bfloat16_rz(v);
+    const float f0 = __bfloat162float(t0), r1 = fabsf(f0) <= 3.402823466e38f ? v - f0 : 0.f;
+    t1 = __float2bfloat16_rn(r1);
+    t2 = __float2bfloat16_rn(r1 - __bfloat162float(t1));
 }
 
 // three terms per element, three stacked bf16 matrices [3][M][K]
@@ -664,7 +643,8 @@ dia_gemm_few_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid
             v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w; v[4] = y.x; v[5] = y.y; v[6] = y.z; v[7] = y.w;
         }
         __nv_bfloat16 t[3][8];
-        split3(v, t);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) split3_down(v[e], t[0][e], t[1][e], t[2][e]);
 #pragma unroll
         for (int q = 0; q < 3; ++q) {
             const int r = q * Mp + m;
@@ -770,11 +750,9 @@ __global__ void __launch_bounds__(256) split3_heads_kernel(const float* __restri
     for (int i = threadIdx.x; i < H * (K >> 2); i += 256) {   // (K a multiple of 8)
         const int h = i / (K >> 2), k = 4 * (i - h * (K >> 2));
         const size_t o = ((size_t)h * M + blockIdx.x) * K + k;
-        float v[4];
         __nv_bfloat16 t[3][4];
 #pragma unroll
-        for (int e = 0; e < 4; ++e) v[e] = row[(size_t)h * hs + k + e];
-        split3(v, t);
+        for (int e = 0; e < 4; ++e) split3_down(row[(size_t)h * hs + k + e], t[0][e], t[1][e], t[2][e]);
 #pragma unroll
         for (int q = 0; q < 3; ++q) *reinterpret_cast<uint2*>(xs + q * n + o) = *reinterpret_cast<const uint2*>(t[q]);
     }
