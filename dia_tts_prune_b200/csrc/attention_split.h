@@ -51,6 +51,7 @@ struct SplitAttention {
 bool split_attention_ok(const SplitAttention& a);
 // bytes of `work` for `keys` keys of this shape (0: the shape is not taken)
 size_t split_attention_work_bytes(const SplitAttention& a, int keys);
+int* split_attention_ran_out(int device, cudaStream_t st);      // the word that a kernel sets when one of its waits has run out
 cudaError_t launch_split_attention(const SplitAttention& a, cudaStream_t st);
 
 }  // namespace dia

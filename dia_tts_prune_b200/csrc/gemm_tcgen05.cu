@@ -19,6 +19,7 @@
 //             fp32 stores) while the MMAs of tile i + 1 fill the other accumulator
 // W is kept as a K-major bf16 copy [N][K] made once per weight (transpose_to_bf16_kernel), so that A and B use the
 // same canonical UMMA layout.  Every wait is bounded (a stuck pipeline traps instead of hanging the GPU).
+// More than 128 rows run on pairs of SMs (dia_gemm_pair_kernel); this kernel keeps the shorter ones and small expert groups.
 //
 // The same kernel serves callers whose activations are bf16 already (terms = 1: one MMA per k-step, the operand is read
 // as it is), row tiles that belong to different weight matrices (expert groups: the group of a tile's first row picks
@@ -26,6 +27,7 @@
 // k-block (the TMA fills the tail of both operands with zeros), a DynamicTanh in front of the residual add, and a gelu whose
 // result leaves as the bf16 operand of the product that follows.
 #include <algorithm>
+#include <atomic>
 
 #include <cuda.h>
 #include <cuda_bf16.h>
@@ -33,6 +35,7 @@
 #include "common.cuh"
 #include "engine_internal.h"
 #include "gemm_tcgen05.h"
+#include "attention_split.h"
 
 namespace dia {
 
@@ -356,6 +359,239 @@ dia_gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
     }
 }
 
+// ---------------------------------------------------------------------------------------------------------------------
+// The same product on pairs of SMs: a cluster of two CTAs owns a 256 x BN tile, and one tcgen05.mma of the pair (cta_group::2) multiplies the
+// 256 rows of both by the BN columns of both.  Each CTA holds its own 128 rows and half of the columns, so the operands of a k-block that an
+// SM takes from L2 shrink from (terms x 16 + 32) to (terms x 16 + 16) KB - which is what bounds the kernel above.
+//   warp 0    one lane per CTA: TMA loads of the CTA's halves into a ring of stages; every byte of both CTAs counts on the leader's barrier
+//   warp 1    leader only: one elected lane issues the pair's MMAs, commits to the barriers of both CTAs
+//   warps 2-5 epilogue of the CTA's 128 rows while the next tile is multiplied into the other accumulator; 32 x 32 blocks turn through
+//             shared memory so that whole lines are stored (row by row, 4096 x 2048 x 2048 was bound by those stores)
+// us, one SM per tile / pairs: one term 4096 x 8192 x 2048 135 / 94 (1.46 PFLOP/s), 4096 x 2048 x 6144 106 / 80, 1722 x 16384 x 2048 126 / 90;
+// three terms 256 / 209 (1.66 PFLOP/s), 4096 x 6144 x 2048 227 / 187.  Bound: the MMAs (four of one term take 512 cycles to run and 540 to
+// issue; the products of a long pass are at the power limit).  A wait that runs out ends every role; the kernel sets the device's word, which the next launch reports.
+constexpr int kPairSlots = 13, kPairStagesMost = 8, kPairStageBytes = 4 * 4096;          // ring, and the epilogue's 32 x 32 blocks
+constexpr int kPairSmem = kPairSlots * kTileBytes + kPairStageBytes + 1024 + 256;
+constexpr unsigned kPairPolls = 4000000u;
+static_assert((2 * kPairStagesMost + 4) * 8 + 8 <= 256, "barrier region");
+
+struct PairProduct {
+    float* y; const float* residual;
+    int M, N, K, BN, stages;
+    const float* dyt_w; const float* dyt_b; float dyt_alpha;
+    __nv_bfloat16* y_bf16;
+    const int* row_group; int group_rows; const int* n_rows;
+    int* ran_out;
+};
+
+__device__ __forceinline__ uint32_t at_rank(const void* local, uint32_t rank) {
+    uint32_t a;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(local)), "r"(rank));
+    return a;
+}
+__device__ __forceinline__ bool pair_wait(uint64_t* bar, uint32_t parity) {       // one answer for a converged warp
+    for (unsigned i = 0; i < kPairPolls; ++i)
+        if (__any_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+    return false;
+}
+__device__ __forceinline__ bool lane_wait(uint64_t* bar, uint32_t parity) {
+    for (unsigned i = 0; i < kPairPolls; ++i)
+        if (mbar_try_wait(bar, parity)) return true;
+    return false;
+}
+// a load of this CTA that counts on a barrier of the pair's leader
+__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1) {
+    asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
+                 ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(c0), "r"(c1)
+                 : "memory");
+}
+__device__ __forceinline__ void umma_bf16_pair(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+__device__ __forceinline__ void umma_commit_pair(uint64_t* bar) {                // the barrier at this place in both CTAs
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
+                 ::"r"(smem_u32(bar)), "h"((uint16_t)3) : "memory");
+}
+__device__ __forceinline__ void cluster_sync_all() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+template <int TERMS>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
+dia_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const __grid_constant__ PairProduct p) {
+    extern __shared__ unsigned char smem_raw[];
+    unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    unsigned char* turn = smem + kPairSlots * kTileBytes;
+    uint64_t* full = reinterpret_cast<uint64_t*>(turn + kPairStageBytes);        // (the leader's alone)
+    uint64_t* empty = full + kPairStagesMost;
+    uint64_t* t_full = empty + kPairStagesMost;
+    uint64_t* t_empty = t_full + 2;                                              // (the leader's alone)
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(t_empty + 2);
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t rank = blockIdx.x & 1;
+    const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
+    const int BN = p.BN, half = BN >> 1, M = p.M, N = p.N;
+    const int n_kb = (p.K + BK - 1) / BK, n_stages = p.stages;
+    const int m_lim = p.n_rows ? min(M, *p.n_rows) : M;
+    const int tiles_m = (M + 2 * BM - 1) / (2 * BM), n_tiles = tiles_m * ((N + BN - 1) / BN);
+    const int stage_bytes = TERMS * kTileBytes + half * 128;
+
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < kPairStagesMost; ++i) { mbar_init(&full[i], 1); mbar_init(&empty[i], 1); }
+        for (int i = 0; i < 2; ++i) { mbar_init(&t_full[i], 1); mbar_init(&t_empty[i], 8); }
+        fence_mbar_init();
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(512));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::);
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    cluster_sync_all();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem_base = *tmem_slot;
+    bool ok = true;
+
+    if (warp == 0) {
+        if (lane == 0) {
+            unsigned i = 0;
+            for (int t = pair; t < n_tiles && ok; t += pairs) {
+                const int n0 = (t / tiles_m) * BN, m0 = (t % tiles_m) * 2 * BM;
+                if (m0 >= m_lim) continue;
+                const int a_row = m0 + (int)rank * BM, b_row = n0 + (int)rank * half + (p.row_group ? p.row_group[m0] * p.group_rows : 0);
+                for (int kb = 0; kb < n_kb; ++kb, ++i) {
+                    const unsigned s = i % n_stages;
+                    if (!lane_wait(&empty[s], ((i / n_stages) & 1u) ^ 1u)) { ok = false; break; }
+                    if (rank == 0) mbar_arrive_expect_tx(&full[s], 2u * stage_bytes);
+                    const uint32_t bar = at_rank(&full[s], 0), dst = smem_u32(smem + s * stage_bytes);
+                    tma_load_2d_pair(dst + TERMS * kTileBytes, &map_b, bar, kb * BK, b_row);
+#pragma unroll
+                    for (int tm = 0; tm < TERMS; ++tm) tma_load_2d_pair(dst + tm * kTileBytes, &map_a, bar, kb * BK, tm * M + a_row);
+                }
+            }
+            // (the leader's last commits arrive here: not after this CTA has gone)
+            for (unsigned j = i > (unsigned)n_stages ? i - n_stages : 0; j < i && ok; ++j) ok = lane_wait(&empty[j % n_stages], (j / n_stages) & 1u);
+        }
+    } else if (warp == 1) {
+        if (rank == 0) {
+            const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(2 * BM >> 4) << 24);
+            unsigned i = 0, it = 0;
+            for (int t = pair; t < n_tiles && ok; t += pairs) {
+                if ((t % tiles_m) * 2 * BM >= m_lim) continue;
+                const unsigned acc = it & 1u;
+                if (!pair_wait(&t_empty[acc], ((it >> 1) & 1u) ^ 1u)) { ok = false; break; }
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint32_t d = tmem_base + acc * 256;
+                for (int kb = 0; kb < n_kb; ++kb, ++i) {
+                    const unsigned s = i % n_stages;
+                    if (!pair_wait(&full[s], (i / n_stages) & 1u)) { ok = false; break; }
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    const uint32_t at = smem_u32(smem + s * stage_bytes);
+                    const uint64_t adesc = umma_desc(at), bdesc = umma_desc(at + TERMS * kTileBytes);
+                    if (elect_one_sync()) {
+#pragma unroll
+                        for (int tm = 0; tm < TERMS; ++tm)
+#pragma unroll
+                            for (int j = 0; j < BK / 16; ++j)
+                                umma_bf16_pair(d, adesc + (tm * kTileBytes >> 4) + 2 * j, bdesc + 2 * j, idesc, (tm | j) != 0 ? 1u : (kb != 0 ? 1u : 0u));
+                        umma_commit_pair(&empty[s]);
+                        if (kb == n_kb - 1) umma_commit_pair(&t_full[acc]);
+                    }
+                    __syncwarp();
+                }
+                ++it;
+            }
+        }
+    } else {
+        const int q = warp & 3;
+        float* const blk = reinterpret_cast<float*>(turn + (warp - 2) * 4096);
+        const int rr = lane >> 3, ch = lane & 7;              // a lane's row of four and its 16-byte piece of a 32-column block
+        unsigned it = 0;
+        for (int t = pair; t < n_tiles; t += pairs) {
+            const int n0 = (t / tiles_m) * BN, m0 = (t % tiles_m) * 2 * BM;
+            if (m0 >= m_lim) continue;
+            const unsigned acc = it & 1u;
+            if (!pair_wait(&t_full[acc], (it >> 1) & 1u)) { ok = false; break; }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const int row0 = m0 + (int)rank * BM + q * 32, rows = min(32, M - row0);
+#pragma unroll 1
+            for (int cb = 0; cb < BN / 32; ++cb) {
+                const int c0 = n0 + cb * 32;
+                if (c0 >= N || rows <= 0) break;              // (uniform)
+                uint32_t v[32];
+                asm volatile(
+                    "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
+                    "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
+                    "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+                    : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
+                      "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]),
+                      "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]),
+                      "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
+                    : "r"(tmem_base + ((uint32_t)(q * 32) << 16) + acc * 256 + cb * 32)
+                    : "memory");
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                // lane = row: its 16-byte piece c goes to place c ^ (row % 8) of its 128 bytes, and is read a row per eight lanes
+#pragma unroll
+                for (int c = 0; c < 8; ++c)
+                    *reinterpret_cast<uint4*>(blk + lane * 32 + ((c ^ (lane & 7)) << 2)) = make_uint4(v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]);
+                __syncwarp();
+                const int n = c0 + 4 * ch;
+                if (n < N) {                                  // (N is a multiple of 4)
+                    float4 w4 = make_float4(0.f, 0.f, 0.f, 0.f), b4 = w4;
+                    if (p.dyt_w) {
+                        w4 = *reinterpret_cast<const float4*>(p.dyt_w + n);
+                        b4 = *reinterpret_cast<const float4*>(p.dyt_b + n);
+                    }
+#pragma unroll
+                    for (int g = 0; g < 8; ++g) {
+                        const int r = 4 * g + rr;
+                        if (r >= rows) break;
+                        float4 a = *reinterpret_cast<const float4*>(blk + r * 32 + ((ch ^ (r & 7)) << 2));
+                        const size_t at = (size_t)(row0 + r) * N + n;
+                        if (p.y_bf16) {                       // the activation of an up product, as the next product's operand
+                            const __nv_bfloat162 lo = __floats2bfloat162_rn(gelu_to_bf16_range(a.x), gelu_to_bf16_range(a.y));
+                            const __nv_bfloat162 hi = __floats2bfloat162_rn(gelu_to_bf16_range(a.z), gelu_to_bf16_range(a.w));
+                            *reinterpret_cast<uint2*>(p.y_bf16 + at) = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+                            continue;
+                        }
+                        if (p.dyt_w) {                        // DynamicTanh of the product: tanh(alpha a) w + b per column
+                            a.x = fmaf(tanhf(p.dyt_alpha * a.x), w4.x, b4.x); a.y = fmaf(tanhf(p.dyt_alpha * a.y), w4.y, b4.y);
+                            a.z = fmaf(tanhf(p.dyt_alpha * a.z), w4.z, b4.z); a.w = fmaf(tanhf(p.dyt_alpha * a.w), w4.w, b4.w);
+                        }
+                        if (p.residual) {
+                            const float4 r4 = *reinterpret_cast<const float4*>(p.residual + at);
+                            a.x += r4.x; a.y += r4.y; a.z += r4.z; a.w += r4.w;
+                        }
+                        *reinterpret_cast<float4*>(p.y + at) = a;
+                    }
+                }
+                __syncwarp();
+            }
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0)
+                asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(at_rank(&t_empty[acc], 0)) : "memory");
+            ++it;
+        }
+    }
+    if (!ok && lane == 0 && p.ran_out) {
+        *reinterpret_cast<volatile int*>(p.ran_out) = 1;
+        __threadfence_system();
+    }
+    __syncwarp();
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    cluster_sync_all();                                       // neither CTA's memory goes while the other still reads it or arrives there
+    if (warp == 1) {
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512));
+    }
+}
+
 __device__ __forceinline__ float load_remote(const float* local, uint32_t rank) {
     uint32_t a;
     float v;
@@ -369,9 +605,6 @@ __device__ __forceinline__ float4 load_remote4(const float* local, uint32_t rank
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(local)), "r"(rank));
     asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a) : "memory");
     return v;
-}
-__device__ __forceinline__ void cluster_sync_all() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
 // ---------------------------------------------------------------------------------------------------------------------
@@ -796,9 +1029,44 @@ cudaError_t launch_transpose_to_bf16(const void* w, int src_bf16, void* wt, int 
     return cudaGetLastError();
 }
 
-static bool dense_rows_f32(int terms, int M, int N, int K, int sms);
+static bool dense_rows_f32(int terms, int M, int N, int K, int sms, int pairs);
 static cudaError_t run_gemm_f32(const F32Product& p, const void* a_terms, int terms, int splits, cudaStream_t st);
 
+// clusters of two CTAs of the pair kernel that run at the same time
+static cudaError_t pairs_of(int dev, int* out) {
+    static std::atomic<int> known[64];
+    if (dev >= 0 && dev < 64 && (*out = known[dev].load(std::memory_order_relaxed)) > 0) return cudaSuccess;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(2);
+    cfg.blockDim = dim3(kGemmThreads);
+    cfg.dynamicSmemBytes = kPairSmem;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = 2;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    cudaError_t e = cudaFuncSetAttribute(dia_gemm_pair_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmem);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(out, dia_gemm_pair_kernel<1>, &cfg);
+    if (e != cudaSuccess) return e;
+    if (*out < 1) return cudaErrorNotSupported;
+    if (dev >= 0 && dev < 64) known[dev].store(*out, std::memory_order_relaxed);
+    return cudaSuccess;
+}
+
+// Columns of a pair's tile: the width whose rounds of tiles end first.  A round's time grows with its columns where the MMAs bound it (three
+// terms, us per k-block alone on the chip: 0.44 at 128, 0.63 at 192, 0.83 at 256) and hardly where issuing four of them does (one term:
+// 0.30 and 0.28).  1722 rows x 16384 columns, K = 2048, three terms: 7 rounds of 256 223 us, 7 of 224 209; 3072 columns: 2 of 256 69, 2 of 160 49
+static int pair_columns(int terms, int M, int N, int pairs, long long* rounds) {
+    const int tiles_m = (M + 2 * BM - 1) / (2 * BM), fixed = terms == 1 ? 700 : 30;
+    int best = 0;
+    long long least = 0;
+    for (int bn = 256; bn >= 128; bn -= 32) {
+        const long long r = ((long long)tiles_m * ((N + bn - 1) / bn) + pairs - 1) / pairs, cost = r * (fixed + bn);
+        if (!best || cost < least) best = bn, least = cost, *rounds = r;
+    }
+    return best;
+}
 // A: bf16 [terms * M][K], the terms of the activation stacked (terms = 1: the activation itself); Wt: bf16 [wt_rows][K].
 // Returns cudaErrorNotSupported for shapes the tiling does not cover (the caller decides what to do).
 cudaError_t launch_gemm_tcgen05_bf16(const void* a_bf16, int terms, const void* wt, long long wt_rows, float* y, int M, int N,
@@ -823,10 +1091,31 @@ cudaError_t launch_gemm_tcgen05_bf16(const void* a_bf16, int terms, const void* 
         if (dev < 0 || dev >= 64) n_sm[0] = n; else n_sm[dev] = n;
     }
     const int sms = (dev < 0 || dev >= 64) ? n_sm[0] : n_sm[dev];
-    if (terms == 1 && !groups && wt_rows == N && dense_rows_f32(1, M, N, K, sms)) {
+    int pairs = 0;
+    e0 = pairs_of(dev, &pairs);
+    if (e0 != cudaSuccess) return e0;
+    if (terms == 1 && !groups && wt_rows == N && dense_rows_f32(1, M, N, K, sms, pairs)) {
         const F32Product narrow{nullptr, 0, 0, wt, ep.y_bf16 ? nullptr : y, N, N, ep.y_bf16, 1, M, N, K, 1.f, ep.y_bf16 ? 3 : 0, nullptr, 0, 0,
                                 ep.residual, ep.dyt_w, ep.dyt_b, ep.dyt_alpha};
         if (gemm_f32_ok(narrow)) return run_gemm_f32(narrow, a_bf16, 1, 8, st);
+    }
+    if (M > BM && (terms == 1 || terms == kTerms) && (!groups || groups->tile_rows % (2 * BM) == 0)) {
+        const auto kernel = terms == 1 ? dia_gemm_pair_kernel<1> : dia_gemm_pair_kernel<kTerms>;
+        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmem);
+        if (e != cudaSuccess) return e;
+        long long rounds = 0;
+        const int bn = pair_columns(terms, M, N, pairs, &rounds);
+        const PairProduct q{y, ep.residual, M, N, K, bn, std::min(kPairStagesMost, kPairSlots * kTileBytes / (terms * kTileBytes + bn / 2 * 128)),
+                            ep.dyt_w, ep.dyt_b, ep.dyt_alpha, reinterpret_cast<__nv_bfloat16*>(ep.y_bf16), groups ? groups->row_group : nullptr,
+                            groups ? groups->group_rows : 0, groups ? groups->n_rows : nullptr, split_attention_ran_out(dev, st)};
+        if (q.ran_out && *reinterpret_cast<volatile int*>(q.ran_out)) {
+            *q.ran_out = 0;
+            return cudaErrorLaunchTimeout;
+        }
+        if (!make_map(&mb, wt, wt_rows, K, bn / 2)) return cudaErrorNotSupported;
+        const int n_tiles = ((N + bn - 1) / bn) * ((M + 2 * BM - 1) / (2 * BM));
+        kernel<<<2 * std::min(n_tiles, pairs), kGemmThreads, kPairSmem, st>>>(ma, mb, q);
+        return cudaGetLastError();
     }
     const int n_tiles = ((N + BN - 1) / BN) * ((M + BM - 1) / BM);
     dia_gemm_tcgen05_kernel<<<std::min(n_tiles, sms), kGemmThreads, kGemmSmem, st>>>(
@@ -851,18 +1140,22 @@ static int f32_splits(int tiles, int n_kb, int most, int sms) {
     return s;
 }
 // Beyond 32 rows (and for bf16 rows) the fp32-sum kernel where its rounds of tiles are the shorter ones: its 128 x 128 tiles are twice
-// as many, and where they leave the chip idle its clusters split K.  Three terms: a k-block of a round takes three quarters of one of
-// 128 x 256 tiles (1.1 and 1.4 us; both are bound by the operands' way from L2).  us, 128 x 256 tiles / here: 200 rows N = 2048,
-// K = 1024 27 / 14, N = 1024, K = 4096 77 / 31, N = 8192, K = 1024 29 / 26, N = 16384, K = 2048 51 / 73; 1024 rows N = 2048, K = 1024
-// 30 / 27; 1722 rows 33 / 45.  One term: about the same per k-block, a shorter start and end.  150 rows N = K = 2048 23 / 12, N = 2048,
-// K = 6144 53 / 20, N = 288, K = 96 11 / 9; 1024 rows N = 2048, K = 6144 55 / 59, N = 512, K = 2048 22 / 12
-static bool dense_rows_f32(int terms, int M, int N, int K, int sms) {
+// as many as 128 x 256 ones, and where they leave the chip idle its clusters split K.  Three terms: a k-block of a round takes three quarters
+// of one of 128 x 256 tiles on one SM (1.1 and 1.4 us).  (Pairs of SMs take 0.4 to 0.8 us, but their sums of all K products in tensor memory
+// are ten times further off: what had fp32 sums keeps them.)  One term, us, pair / here: 512 rows N = K = 2048 18 / 16, 1024 rows 18 / 22; 1722
+// rows N = 768 18 / 22, 800 rows 17 / 16: a k-block takes 0.34 us there and 0.46 here, and starting and ending 1 us longer.  Up to 128 rows half
+// of a pair's tile would be empty: against one SM's 128 x 256 tiles 21 to 20 units a k-block (100 rows N = 32768, K = 2048 21 us, pairs 33)
+static bool dense_rows_f32(int terms, int M, int N, int K, int sms, int pairs) {
     const int tm = (M + BM - 1) / BM, n_kb = (K + BK - 1) / BK;
     const long long narrow = (long long)tm * ((N + kFN - 1) / kFN), wide = (long long)tm * ((N + BN - 1) / BN);
     const int s = narrow < sms ? f32_splits((int)narrow, n_kb, 8, sms) : 1;
     const long long here = (narrow * s + sms - 1) / sms, there = (wide + sms - 1) / sms;
     const int kb = (n_kb + s - 1) / s;
-    return terms == 1 ? here * (21 * kb + 100) < there * (20 * n_kb + 130) : here * kb * 3 < there * n_kb * 4;
+    if (terms != 1) return here * kb * 3 < there * n_kb * 4;
+    if (M <= BM) return here * (21 * kb + 100) < there * (20 * n_kb + 130);
+    long long rounds = 0;
+    (void)pair_columns(terms, M, N, pairs, &rounds);
+    return here * kb * 460 < rounds * n_kb * 340 + 1000;
 }
 
 // splits: the most CTAs that may share a tile (1: a sum's order does not depend on the rows beside it)
@@ -983,8 +1276,10 @@ cudaError_t launch_gemm_tcgen05(const float* x, const float* norm_w, float eps, 
     int dev = 0, sms = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    int pairs = 0;
+    if (e == cudaSuccess) e = pairs_of(dev, &pairs);
     if (e != cudaSuccess) return e;
-    if (dense_rows_f32(kTerms, M, N, K, sms) && gemm_f32_ok(wide)) return run_gemm_f32(wide, workspace, kTerms, 8, st);
+    if (dense_rows_f32(kTerms, M, N, K, sms, pairs) && gemm_f32_ok(wide)) return run_gemm_f32(wide, workspace, kTerms, 8, st);
     const GemmEpilogue ep{residual, nullptr, nullptr, 0.f, nullptr};
     return launch_gemm_tcgen05_bf16(workspace, kTerms, wt, N, y, M, N, K, ep, nullptr, st);
 }

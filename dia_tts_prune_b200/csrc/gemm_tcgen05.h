@@ -13,6 +13,7 @@
 namespace dia {
 
 constexpr int kGemmRowTile = 128;            // rows of A per output tile: the padding unit of a row group
+constexpr int kGemmPairRows = 256;           // the same of a pair of SMs
 
 struct GemmEpilogue {
     const float* residual;                   // [M][N] added to the result (may alias Y), or null
@@ -26,6 +27,7 @@ struct GemmGroups {
     const int* row_group;                    // device [M]: group of every row of A (read at the first row of a tile)
     int group_rows;                          // rows of Wt per group
     const int* n_rows;                       // device: rows of A in use (row tiles at or beyond it are skipped); null: M
+    int tile_rows;                           // every group starts on a multiple of it: kGemmRowTile or kGemmPairRows
 };
 
 // K a multiple of 8 (16-byte rows for the TMA), N a multiple of 4 (float4 stores)

@@ -185,6 +185,10 @@ int slots_bound(int rows, int top, int experts, int pad) {
     return n + std::min(experts, n) * (pad - 1);
 }
 
+// Rows to which an expert's group is padded for the tensor-core products: those of a pair of SMs, unless the groups would mostly be padding
+// (width 2048, 8 experts of 2048, pairs / single SMs: 4096 rows, two experts each 321 / 375 us, 300 rows 111 / 111)
+int group_rows(int assignments, int experts) { return assignments >= 64LL * experts ? dia::kGemmPairRows : dia::kGemmRowTile; }
+
 bool tensor_path(const lm_b200_engine* e, int M, int N, int K) {
     return e->m.precision == LM_B200_PRECISION_BF16 && M >= kTensorRowsMin && dia::gemm_tcgen05_shape_ok(M, N, K);
 }
@@ -572,13 +576,13 @@ int feed_forward(lm_b200_engine* e, const lm_b200_layer& l, const float* h, cons
     const int n_assign = M * top;
     // both expert products on the tensor cores, or neither: the groups are padded to the row tile of the kernel that runs
     const bool tc = tensor_path(e, M, 2 * F, D) && tensor_path(e, M, D, F);
-    const int pad = tc ? dia::kGemmRowTile : lm::kTileRows;
+    const int pad = tc ? group_rows(M * top, E) : lm::kTileRows;
     const int bound = slots_bound(M, top, E, pad);
     const lm::GroupMap gm{e->a_row, e->a_scale, e->a_expert, e->n_slots};
     LCK(lm::launch_moe_group(e->sel_e, e->sel_w, n_assign, top, E, pad, gm, e->slot_of, bound, st));
     if (tc) {
         LCK(lm::launch_pack_rows_bf16(h, e->packb, bound, D, &gm, st));
-        const dia::GemmGroups gu_groups{e->a_expert, 2 * F, e->n_slots}, down_groups{e->a_expert, D, e->n_slots};
+        const dia::GemmGroups gu_groups{e->a_expert, 2 * F, e->n_slots, pad}, down_groups{e->a_expert, D, e->n_slots, pad};
         LCK(dia::launch_gemm_tcgen05_bf16(e->packb, 1, l.w_gate_up, (long long)E * 2 * F, e->gu, bound, 2 * F, D, kPlain,
                                           &gu_groups, st));
         LCK(lm::launch_silu_mul(e->gu, nullptr, e->midb, bound, F, &gm, st));
@@ -943,14 +947,14 @@ int stream_ff(lm_b200_engine* e, const lm_b200_layer& l, const float* h, const v
     LCK(linear_f32(e, h, D, l.w_router, e->z, zc, M, zc, D, st));
     LCK(lm::launch_router_topk(e->z, zc, top, M, e->sel_e, e->sel_w, st, l.router_bias, !grouped, grouped ? &gr : nullptr));
     const bool tc = hb && tensor_path(e, M, 2 * F, D) && tensor_path(e, M, D, F);
-    const int pad = tc ? dia::kGemmRowTile : lm::kTileRows;
+    const int pad = tc ? group_rows(M * top, E) : lm::kTileRows;
     const int bound = slots_bound(M, top, E, pad);
     const lm::GroupMap gm{e->a_row, e->a_scale, e->a_expert, e->n_slots};
     const lm::GroupMap gather{e->a_row, nullptr, e->a_expert, e->n_slots};
     LCK(lm::launch_moe_group(e->sel_e, e->sel_w, M * top, top, E, pad, gm, e->slot_of, bound, st));
     if (tc) {
         LCK(lm::launch_pack_rows_bf16(h, e->packb, bound, D, &gather, st));
-        const dia::GemmGroups gu_groups{e->a_expert, 2 * F, e->n_slots}, down_groups{e->a_expert, D, e->n_slots};
+        const dia::GemmGroups gu_groups{e->a_expert, 2 * F, e->n_slots, pad}, down_groups{e->a_expert, D, e->n_slots, pad};
         LCK(dia::launch_gemm_tcgen05_bf16(e->packb, 1, l.w_gate_up, (long long)E * 2 * F, e->gu, bound, 2 * F, D, kPlain,
                                           &gu_groups, st));
         LCK(lm::launch_silu_mul(e->gu, nullptr, e->midb, bound, F, &gm, st, act, l.act_limit));
@@ -1067,7 +1071,7 @@ int lm_b200_engine_create(const lm_b200_model* model, const lm_b200_layer* layer
                 top = std::max(top, (size_t)l.top);
                 F = std::max(F, (size_t)l.expert_ff);
                 Sf = std::max(Sf, (size_t)l.shared_ff);
-                slots = std::max(slots, (size_t)slots_bound(m.max_rows, l.top, l.experts, dia::kGemmRowTile));
+                slots = std::max(slots, (size_t)slots_bound(m.max_rows, l.top, l.experts, group_rows(m.max_rows * l.top, l.experts)));
             }
             continue;
         }
@@ -1092,7 +1096,7 @@ int lm_b200_engine_create(const lm_b200_model* model, const lm_b200_layer* layer
             top = std::max(top, (size_t)l.top);
             F = std::max(F, (size_t)l.expert_ff);
             Sf = std::max(Sf, (size_t)l.shared_ff);
-            slots = std::max(slots, (size_t)slots_bound(m.max_rows, l.top, l.experts, dia::kGemmRowTile));
+            slots = std::max(slots, (size_t)slots_bound(m.max_rows, l.top, l.experts, group_rows(m.max_rows * l.top, l.experts)));
         }
     }
     e->max_slots = (int)slots;
