@@ -79,6 +79,9 @@ _SIGNATURES = {
     "dia_b200_batch_generate_steps": (_i, [_vp, _i, _vp]),
     "dia_b200_batch_generate_status": (_i, [_vp, C.POINTER(GenStatus), _vp]),
     "dia_b200_dense_forward_fused": (_i, [_fp, _fp, C.c_float, _vp, _fp, _fp, _vp, _i, _i, _i, _vp]),
+    "dia_b200_dense_half_rows": (_i, [_i, _i, _i]),
+    "dia_b200_dense_prepare_half": (_i, [_vp, _i, _vp, _fp, _i32p, _i, _i, _vp]),
+    "dia_b200_dense_forward_half": (_i, [_fp, _fp, C.c_float, _i, _vp, _fp, _fp, _fp, _vp, _i, _i, _i, _vp]),
     "dia_b200_attention_rows": (_i, [_fp, _fp, _fp, _fp, _i, _i, _i, _i, _i, _i, _i, C.POINTER(C.c_int32), _vp]),
     "dia_b200_rope_rows": (_i, [_fp, _fp, _fp, _fp, _i32p, _i, _i, _i, _i, _i, _i, _i, _i, _vp]),
     "dia_b200_rmsnorm_rows": (_i, [_fp, _fp, C.c_float, _fp, _i, _i, _vp]),

@@ -1001,6 +1001,31 @@ int dia_b200_dense_forward_fused(const float* x, const float* norm_weight, float
     return DIA_B200_OK;
 }
 
+int dia_b200_dense_half_rows(int M, int N, int K) { return gemm_half_ok(M, N, K) ? 1 : 0; }
+
+int dia_b200_dense_prepare_half(const void* w, int src_dtype, void* wt_half, float* magnitudes, int32_t* inexact, int K, int N, void* stream) {
+    if (!w || !wt_half || !magnitudes || !inexact || K <= 0 || N <= 0 || (src_dtype != 0 && src_dtype != 1)) return DIA_B200_EINVAL;
+    CK(launch_prepare_half(w, src_dtype, wt_half, magnitudes, inexact, K, N, S(stream)));
+    g_launches += 1 + std::exchange(extra_launches(), 0);
+    return DIA_B200_OK;
+}
+
+int dia_b200_dense_forward_half(const float* x, const float* norm_weight, float eps, int gated, const void* wt_half, const float* magnitudes,
+                                const float* residual, float* y, void* workspace, int M, int N, int K, void* stream) {
+    if (M < 0 || N <= 0 || K <= 0) return DIA_B200_EINVAL;
+    if (M == 0) return DIA_B200_OK;
+    if (!x || !wt_half || !magnitudes || !y || !workspace) return DIA_B200_EINVAL;
+    if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(norm_weight) | reinterpret_cast<uintptr_t>(wt_half) |
+         reinterpret_cast<uintptr_t>(magnitudes) | reinterpret_cast<uintptr_t>(workspace) | reinterpret_cast<uintptr_t>(y) |
+         reinterpret_cast<uintptr_t>(residual)) & 15)
+        return DIA_B200_EINVAL;
+    const cudaError_t e = launch_gemm_half(x, norm_weight, eps, gated != 0, wt_half, magnitudes, residual, y, workspace, M, N, K, S(stream));
+    if (e == cudaErrorNotSupported) { (void)cudaGetLastError(); return DIA_B200_EUNSUPPORTED; }
+    CK(e);
+    g_launches += 1 + std::exchange(extra_launches(), 0);
+    return DIA_B200_OK;
+}
+
 int dia_b200_dense_forward(const float* x, const void* wt_bf16, float* y, void* workspace, int M, int N, int K, void* stream) {
     return dia_b200_dense_forward_fused(x, nullptr, 0.f, wt_bf16, nullptr, y, workspace, M, N, K, stream);
 }

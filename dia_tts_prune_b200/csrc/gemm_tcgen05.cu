@@ -31,6 +31,7 @@
 
 #include <cuda.h>
 #include <cuda_bf16.h>
+#include <cuda_fp16.h>
 
 #include "common.cuh"
 #include "engine_internal.h"
@@ -174,6 +175,136 @@ __global__ void transpose_to_bf16_kernel(const void* __restrict__ w, int src_bf1
         const int n = n0 + r, k = k0 + threadIdx.x;
         if (k < K && n < N) wt[(size_t)n * K + k] = __float2bfloat16_rn(tile[threadIdx.x][r]);
     }
+}
+
+// Largest magnitude of every column of W [K][N] into mag (zeros before), as the bits of a float
+__global__ void __launch_bounds__(256) column_magnitudes_kernel(const void* __restrict__ w, int src_bf16, uint32_t* __restrict__ mag, int K, int N) {
+    const int n = blockIdx.x * 256 + threadIdx.x, k1 = min(K, ((int)blockIdx.y + 1) * 64);
+    if (n >= N) return;
+    uint32_t m = 0;
+#pragma unroll 8
+    for (int k = blockIdx.y * 64; k < k1; ++k) {
+        const size_t at = (size_t)k * N + n;
+        const uint32_t b = src_bf16 ? (uint32_t)reinterpret_cast<const uint16_t*>(w)[at] << 16
+                                    : __float_as_uint(__bfloat162float(__float2bfloat16_rn(reinterpret_cast<const float*>(w)[at])));
+        m = max(m, b & 0x7fffffffu);
+    }
+    atomicMax(mag + n, m);
+}
+
+// W [K][N] (values of bf16) -> Wt [N][K] fp16, every column times a power of two that brings its largest magnitude to [2^14, 2^15).  fp16
+// then holds the 8 bits of every value down to 2^-31 of that; *inexact is set where it does not, and for columns of infinities, NaNs or
+// magnitudes whose power of two is out of range.
+__global__ void transpose_to_half_kernel(const void* __restrict__ w, int src_bf16, const float* __restrict__ mag, __half* __restrict__ wt, int* __restrict__ inexact,
+                                         int K, int N) {
+    __shared__ float tile[32][33];
+    const int n0 = blockIdx.x * 32, k0 = blockIdx.y * 32;
+    for (int r = threadIdx.y; r < 32; r += blockDim.y) {
+        const int k = k0 + r, n = n0 + threadIdx.x;
+        float v = 0.f;
+        if (k < K && n < N)
+            v = src_bf16 ? __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(w)[(size_t)k * N + n])
+                         : __bfloat162float(__float2bfloat16_rn(reinterpret_cast<const float*>(w)[(size_t)k * N + n]));
+        tile[r][threadIdx.x] = v;
+    }
+    __syncthreads();
+    for (int r = threadIdx.y; r < 32; r += blockDim.y) {
+        const int n = n0 + r, k = k0 + threadIdx.x;
+        if (k >= K || n >= N) continue;
+        const int e = (int)(__float_as_uint(mag[n]) >> 23) - 127;
+        const bool fits = e >= -112 && e < 128;               // (a column of zeros: e = -127, and zeros)
+        const float v = tile[threadIdx.x][r], scaled = fits ? v * __uint_as_float((uint32_t)(141 - e) << 23) : 0.f;
+        const __half h = __float2half_rn(scaled);
+        if (fits ? __half2float(h) != scaled : mag[n] != 0.f) *inexact = 1;
+        wt[(size_t)n * K + k] = h;
+    }
+}
+
+// Rows as two fp16 terms, hi = fp16(v), lo = fp16(v - hi), each row times a power of two that brings its largest magnitude to [2^14, 2^15): a
+// value keeps 22 bits and more (a quarter of all fp32 numbers change by their last bit, the others not) down to 2^-17 of its row's largest, and
+// is off by at most 2^-39 of that below.  out: [2][M][K], then the rows' inverse scales [M].  A row with an infinity or a NaN gives nothing but
+// infinities and NaNs in its products: the other values are left out.  norm_w: RMSNorm of the row in front (dia/layers.py:541,560,579,714).
+// GATED: the row is silu(x[0 .. K)) x[K .. 2K) (dia/layers.py:95-101).  One CTA per row, which stays in registers up to 8192 channels.
+template <bool GATED>
+__global__ void __launch_bounds__(256) split2_rows_kernel(const float* __restrict__ x, const float* __restrict__ norm_w, float eps, __half* __restrict__ out,
+                                                          float* __restrict__ row_inv, int M, int K) {
+    constexpr int kHeld = 8;
+    __shared__ float part[8], most[8];
+    const int tid = threadIdx.x, row = blockIdx.x, n4 = K >> 2;
+    const float4* xr = reinterpret_cast<const float4*>(x + (size_t)row * K * (GATED ? 2 : 1));
+    auto raw = [&](int i) {
+        float4 v = xr[i];
+        if (GATED) {
+            const float4 u = xr[n4 + i];
+            v.x = v.x / (1.0f + expf(-v.x)) * u.x; v.y = v.y / (1.0f + expf(-v.y)) * u.y;
+            v.z = v.z / (1.0f + expf(-v.z)) * u.z; v.w = v.w / (1.0f + expf(-v.w)) * u.w;
+        }
+        return v;
+    };
+    float4 held[kHeld];
+#pragma unroll
+    for (int j = 0; j < kHeld; ++j)
+        if (j * 256 + tid < n4) held[j] = raw(j * 256 + tid);
+    float inv = 1.f;
+    if (norm_w) {
+        float ss = 0.f;
+        auto add = [&](const float4& v) { ss = fmaf(v.x, v.x, ss); ss = fmaf(v.y, v.y, ss); ss = fmaf(v.z, v.z, ss); ss = fmaf(v.w, v.w, ss); };
+#pragma unroll
+        for (int j = 0; j < kHeld; ++j)
+            if (j * 256 + tid < n4) add(held[j]);
+        for (int i = kHeld * 256 + tid; i < n4; i += 256) add(raw(i));
+        ss = warp_sum(ss);
+        if ((tid & 31) == 0) part[tid >> 5] = ss;
+        __syncthreads();
+        float tot = 0.f;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) tot += part[i];
+        inv = 1.0f / sqrtf(tot / (float)K + eps);
+    }
+    auto value = [&](const float4& v, int i) {
+        if (!norm_w) return v;
+        const float4 w = reinterpret_cast<const float4*>(norm_w)[i];
+        return make_float4((v.x * inv) * w.x, (v.y * inv) * w.y, (v.z * inv) * w.z, (v.w * inv) * w.w);
+    };
+    uint32_t m = 0;                                           // magnitudes as bits: an infinity or a NaN is the largest
+    auto see = [&](const float4& v) {
+        m = max(max(max(m, __float_as_uint(v.x) & 0x7fffffffu), __float_as_uint(v.y) & 0x7fffffffu),
+                max(__float_as_uint(v.z) & 0x7fffffffu, __float_as_uint(v.w) & 0x7fffffffu));
+    };
+#pragma unroll
+    for (int j = 0; j < kHeld; ++j)
+        if (j * 256 + tid < n4) {
+            held[j] = value(held[j], j * 256 + tid);
+            see(held[j]);
+        }
+    for (int i = kHeld * 256 + tid; i < n4; i += 256) see(value(raw(i), i));
+    m = __reduce_max_sync(0xffffffffu, m);
+    if ((tid & 31) == 0) most[tid >> 5] = __uint_as_float(m);
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 8; ++i) m = max(m, __float_as_uint(most[i]));
+    const bool bad = m >= 0x7f800000u;
+    const int e = max((int)(m >> 23), 1) - 127, s = 14 - e, s1 = min(s, 100);       // the scale 2^s as 2^s1 2^(s - s1): s may be 140
+    const float f1 = bad ? 1.f : __uint_as_float((uint32_t)(s1 + 127) << 23), f2 = bad ? 1.f : __uint_as_float((uint32_t)(s - s1 + 127) << 23);
+    if (tid == 0) row_inv[row] = bad ? 1.f : ldexpf(1.f, -s);
+    const size_t plane = (size_t)M * K;
+    __half* hi_row = out + (size_t)row * K;
+    auto put = [&](const float4& v, int i) {
+        float a[4] = {v.x, v.y, v.z, v.w};
+        __half hi[4], lo[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const float t = bad ? ((__float_as_uint(a[k]) & 0x7f800000u) == 0x7f800000u ? a[k] : 0.f) : a[k] * f1 * f2;
+            hi[k] = __float2half_rn(t);
+            lo[k] = __float2half_rn(bad ? 0.f : t - __half2float(hi[k]));
+        }
+        *reinterpret_cast<uint2*>(hi_row + 4 * i) = *reinterpret_cast<const uint2*>(hi);
+        *reinterpret_cast<uint2*>(hi_row + plane + 4 * i) = *reinterpret_cast<const uint2*>(lo);
+    };
+#pragma unroll
+    for (int j = 0; j < kHeld; ++j)
+        if (j * 256 + tid < n4) put(held[j], j * 256 + tid);
+    for (int i = kHeld * 256 + tid; i < n4; i += 256) put(value(raw(i), i), i);
 }
 
 __global__ void __launch_bounds__(kGemmThreads, 1)
@@ -370,8 +501,21 @@ dia_gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
 // us, one SM per tile / pairs: one term 4096 x 8192 x 2048 135 / 94 (1.46 PFLOP/s), 4096 x 2048 x 6144 106 / 80, 1722 x 16384 x 2048 126 / 90;
 // three terms 256 / 209 (1.66 PFLOP/s), 4096 x 6144 x 2048 227 / 187.  Bound: the MMAs (four of one term take 512 cycles to run and 540 to
 // issue; the products of a long pass are at the power limit).  A wait that runs out ends every role; the kernel sets the device's word, which the next launch reports.
-constexpr int kPairSlots = 13, kPairStagesMost = 8, kPairStageBytes = 4 * 4096;          // ring, and the epilogue's 32 x 32 blocks
-constexpr int kPairSmem = kPairSlots * kTileBytes + kPairStageBytes + 1024 + 256;
+//
+// SUMS: fp32 rows as two fp16 terms (split2_rows_kernel) and weights as fp16 (transpose_to_half_kernel), every row and every column with a power
+// of two of its own; an accumulator lives for kPairChunk k-blocks and eight epilogue warps add it to the tile's sums in their registers (two
+// threads per row, up to 128 columns each) while the next ones are multiplied into the other.  Against three terms and sums of all products
+// in tensor memory: 1722 rows, K = 2048, 16384 columns 209 -> 162 us, 2048 columns 37 -> 28, K = 8192 118 -> 85; relative error 7.0e-6 -> 5.8e-7
+// (861 rows through Dia's decoder 2.8e-5 -> 4.1e-6).  Chunks of 1, 2 and 4 k-blocks: 282, 215 and 162 us, 1.5e-7, 2.9e-7 and 5.8e-7 (the
+// accumulators of a chunk are read while the MMAs update the others, and the two slow each other down).
+template <bool SUMS>
+struct Pair {
+    static constexpr int kFirst = SUMS ? 4 : 2, kWarps = SUMS ? 8 : 4, kThreads = 32 * (kFirst + kWarps);  // (registers go by groups of 4 warps)
+    static constexpr int kSumRegs = 208, kFewRegs = 88, kRegs = (kSumRegs * 8 + kFewRegs * 4) / 12;        // 168 a thread at launch
+    static constexpr int kSlots = SUMS ? 12 : 13;                                                          // ring, and 32 x 32 blocks to turn
+    static constexpr int kSmem = kSlots * kTileBytes + kWarps * 4096 + 1024 + 256;
+};
+constexpr int kPairStagesMost = 8, kPairChunk = 4;
 constexpr unsigned kPairPolls = 4000000u;
 static_assert((2 * kPairStagesMost + 4) * 8 + 8 <= 256, "barrier region");
 
@@ -382,6 +526,7 @@ struct PairProduct {
     __nv_bfloat16* y_bf16;
     const int* row_group; int group_rows; const int* n_rows;
     int* ran_out;
+    const float* row_inv; const float* col_mag;              // SUMS: inverse scales of the rows, largest magnitudes of the columns
 };
 
 __device__ __forceinline__ uint32_t at_rank(const void* local, uint32_t rank) {
@@ -421,13 +566,18 @@ __device__ __forceinline__ void cluster_sync_all() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
-template <int TERMS>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
+// the inverse of a column's scale 2^(14 - e), where its largest magnitude lies in [2^e, 2^(e + 1)) (0 for a column of zeros)
+__device__ __forceinline__ float column_inverse(float magnitude) {
+    return __uint_as_float((uint32_t)max((int)(__float_as_uint(magnitude) >> 23) - 14, 0) << 23);
+}
+
+template <int TERMS, bool SUMS>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Pair<SUMS>::kThreads, 1)
 dia_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const __grid_constant__ PairProduct p) {
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-    unsigned char* turn = smem + kPairSlots * kTileBytes;
-    uint64_t* full = reinterpret_cast<uint64_t*>(turn + kPairStageBytes);        // (the leader's alone)
+    unsigned char* turn = smem + Pair<SUMS>::kSlots * kTileBytes;
+    uint64_t* full = reinterpret_cast<uint64_t*>(turn + Pair<SUMS>::kWarps * 4096);      // (the leader's alone)
     uint64_t* empty = full + kPairStagesMost;
     uint64_t* t_full = empty + kPairStagesMost;
     uint64_t* t_empty = t_full + 2;                                              // (the leader's alone)
@@ -444,7 +594,7 @@ dia_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
 
     if (threadIdx.x == 0) {
         for (int i = 0; i < kPairStagesMost; ++i) { mbar_init(&full[i], 1); mbar_init(&empty[i], 1); }
-        for (int i = 0; i < 2; ++i) { mbar_init(&t_full[i], 1); mbar_init(&t_empty[i], 8); }
+        for (int i = 0; i < 2; ++i) { mbar_init(&t_full[i], 1); mbar_init(&t_empty[i], 2 * Pair<SUMS>::kWarps); }
         fence_mbar_init();
     }
     if (warp == 1) {
@@ -456,60 +606,146 @@ dia_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem_base = *tmem_slot;
     bool ok = true;
-
-    if (warp == 0) {
-        if (lane == 0) {
-            unsigned i = 0;
-            for (int t = pair; t < n_tiles && ok; t += pairs) {
-                const int n0 = (t / tiles_m) * BN, m0 = (t % tiles_m) * 2 * BM;
-                if (m0 >= m_lim) continue;
-                const int a_row = m0 + (int)rank * BM, b_row = n0 + (int)rank * half + (p.row_group ? p.row_group[m0] * p.group_rows : 0);
-                for (int kb = 0; kb < n_kb; ++kb, ++i) {
-                    const unsigned s = i % n_stages;
-                    if (!lane_wait(&empty[s], ((i / n_stages) & 1u) ^ 1u)) { ok = false; break; }
-                    if (rank == 0) mbar_arrive_expect_tx(&full[s], 2u * stage_bytes);
-                    const uint32_t bar = at_rank(&full[s], 0), dst = smem_u32(smem + s * stage_bytes);
-                    tma_load_2d_pair(dst + TERMS * kTileBytes, &map_b, bar, kb * BK, b_row);
+    if (warp < Pair<SUMS>::kFirst) {
+        if constexpr (SUMS) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(Pair<SUMS>::kFewRegs));
+        if (warp == 0) {
+            if (lane == 0) {
+                unsigned i = 0;
+                for (int t = pair; t < n_tiles && ok; t += pairs) {
+                    const int n0 = (t / tiles_m) * BN, m0 = (t % tiles_m) * 2 * BM;
+                    if (m0 >= m_lim) continue;
+                    const int a_row = m0 + (int)rank * BM, b_row = n0 + (int)rank * half + (p.row_group ? p.row_group[m0] * p.group_rows : 0);
+                    for (int kb = 0; kb < n_kb; ++kb, ++i) {
+                        const unsigned s = i % n_stages;
+                        if (!lane_wait(&empty[s], ((i / n_stages) & 1u) ^ 1u)) { ok = false; break; }
+                        if (rank == 0) mbar_arrive_expect_tx(&full[s], 2u * stage_bytes);
+                        const uint32_t bar = at_rank(&full[s], 0), dst = smem_u32(smem + s * stage_bytes);
+                        tma_load_2d_pair(dst + TERMS * kTileBytes, &map_b, bar, kb * BK, b_row);
 #pragma unroll
-                    for (int tm = 0; tm < TERMS; ++tm) tma_load_2d_pair(dst + tm * kTileBytes, &map_a, bar, kb * BK, tm * M + a_row);
+                        for (int tm = 0; tm < TERMS; ++tm) tma_load_2d_pair(dst + tm * kTileBytes, &map_a, bar, kb * BK, tm * M + a_row);
+                    }
+                }
+                // (the leader's last commits arrive here: not after this CTA has gone)
+                for (unsigned j = i > (unsigned)n_stages ? i - n_stages : 0; j < i && ok; ++j) ok = lane_wait(&empty[j % n_stages], (j / n_stages) & 1u);
+            }
+        } else if (warp == 1) {
+            if (rank == 0) {
+                const uint32_t types = SUMS ? 0u : (1u << 7) | (1u << 10);           // fp16 or bf16
+                const uint32_t idesc = (1u << 4) | types | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(2 * BM >> 4) << 24);
+                unsigned i = 0, it = 0;                           // k-blocks and uses of an accumulator so far
+                for (int t = pair; t < n_tiles && ok; t += pairs) {
+                    if ((t % tiles_m) * 2 * BM >= m_lim) continue;
+                    for (int kb = 0; kb < n_kb; ++kb, ++i) {
+                        const bool first = SUMS ? kb % kPairChunk == 0 : kb == 0, last = kb == n_kb - 1 || (SUMS && kb % kPairChunk == kPairChunk - 1);
+                        if (first) {
+                            if (!pair_wait(&t_empty[it & 1u], ((it >> 1) & 1u) ^ 1u)) { ok = false; break; }
+                            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                        }
+                        const uint32_t d = tmem_base + (it & 1u) * 256;
+                        const unsigned s = i % n_stages;
+                        if (!pair_wait(&full[s], (i / n_stages) & 1u)) { ok = false; break; }
+                        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                        const uint32_t at = smem_u32(smem + s * stage_bytes);
+                        const uint64_t adesc = umma_desc(at), bdesc = umma_desc(at + TERMS * kTileBytes);
+                        if (elect_one_sync()) {
+#pragma unroll
+                            for (int u = 0; u < TERMS; ++u) {
+                                const int tm = SUMS ? TERMS - 1 - u : u;             // the smallest term first
+#pragma unroll
+                                for (int j = 0; j < BK / 16; ++j)
+                                    umma_bf16_pair(d, adesc + (tm * kTileBytes >> 4) + 2 * j, bdesc + 2 * j, idesc, (u | j) != 0 ? 1u : (first ? 0u : 1u));
+                            }
+                            umma_commit_pair(&empty[s]);
+                            if (last) umma_commit_pair(&t_full[it & 1u]);
+                        }
+                        __syncwarp();
+                        if (last) ++it;
+                    }
                 }
             }
-            // (the leader's last commits arrive here: not after this CTA has gone)
-            for (unsigned j = i > (unsigned)n_stages ? i - n_stages : 0; j < i && ok; ++j) ok = lane_wait(&empty[j % n_stages], (j / n_stages) & 1u);
         }
-    } else if (warp == 1) {
-        if (rank == 0) {
-            const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(2 * BM >> 4) << 24);
-            unsigned i = 0, it = 0;
-            for (int t = pair; t < n_tiles && ok; t += pairs) {
-                if ((t % tiles_m) * 2 * BM >= m_lim) continue;
-                const unsigned acc = it & 1u;
-                if (!pair_wait(&t_empty[acc], ((it >> 1) & 1u) ^ 1u)) { ok = false; break; }
+    } else if constexpr (SUMS) {
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(Pair<SUMS>::kSumRegs));      // (there are as many: see pairs_of)
+        const int q = warp & 3, h0 = ((warp - Pair<SUMS>::kFirst) >> 2) * half;
+        float* const blk = reinterpret_cast<float*>(turn + (warp - Pair<SUMS>::kFirst) * 4096);
+        const int rr = lane >> 3, ch = lane & 7;
+        unsigned i = 0;
+        for (int t = pair; t < n_tiles && ok; t += pairs) {
+            const int n0 = (t / tiles_m) * BN, m0 = (t % tiles_m) * 2 * BM;
+            float sum[128];
+#pragma unroll
+            for (int c = 0; c < 128; ++c) sum[c] = 0.f;
+            for (int kb = 0; kb < n_kb; kb += kPairChunk, ++i) {
+                const unsigned acc = i & 1u;
+                if (!pair_wait(&t_full[acc], (i >> 1) & 1u)) { ok = false; break; }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t d = tmem_base + acc * 256;
-                for (int kb = 0; kb < n_kb; ++kb, ++i) {
-                    const unsigned s = i % n_stages;
-                    if (!pair_wait(&full[s], (i / n_stages) & 1u)) { ok = false; break; }
-                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    const uint32_t at = smem_u32(smem + s * stage_bytes);
-                    const uint64_t adesc = umma_desc(at), bdesc = umma_desc(at + TERMS * kTileBytes);
-                    if (elect_one_sync()) {
 #pragma unroll
-                        for (int tm = 0; tm < TERMS; ++tm)
+                for (int cb = 0; cb < 4; ++cb) {
+                    if (cb * 32 >= half) break;               // (columns of the last block beyond the half are read and not stored)
+                    uint32_t v[32];
+                    asm volatile(
+                        "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
+                        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
+                        "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+                        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
+                          "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]),
+                          "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]),
+                          "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
+                        : "r"(tmem_base + ((uint32_t)(q * 32) << 16) + acc * 256 + h0 + cb * 32)
+                        : "memory");
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-                            for (int j = 0; j < BK / 16; ++j)
-                                umma_bf16_pair(d, adesc + (tm * kTileBytes >> 4) + 2 * j, bdesc + 2 * j, idesc, (tm | j) != 0 ? 1u : (kb != 0 ? 1u : 0u));
-                        umma_commit_pair(&empty[s]);
-                        if (kb == n_kb - 1) umma_commit_pair(&t_full[acc]);
-                    }
-                    __syncwarp();
+                    for (int e = 0; e < 32; ++e) sum[cb * 32 + e] += __uint_as_float(v[e]);
                 }
-                ++it;
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                __syncwarp();
+                if (lane == 0)
+                    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(at_rank(&t_empty[acc], 0)) : "memory");
+            }
+            const int row0 = m0 + (int)rank * BM + q * 32, rows = min(32, M - row0);
+            float ri[8];                                      // (loads ahead of their uses: the output of a tile took 3.2 us with one row after the other)
+#pragma unroll
+            for (int g = 0; g < 8; ++g) ri[g] = 4 * g + rr < rows ? p.row_inv[row0 + 4 * g + rr] : 0.f;
+#pragma unroll
+            for (int cb = 0; cb < 4; ++cb) {
+                const int n = n0 + h0 + cb * 32 + 4 * ch;     // (BN and N are multiples of 4)
+                if (cb * 32 >= half || rows <= 0) break;
+                const bool in = n < N && cb * 32 + 4 * ch < half;
+                float4 mag = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (in) mag = *reinterpret_cast<const float4*>(p.col_mag + n);
+#pragma unroll
+                for (int c = 0; c < 8; ++c)
+                    *reinterpret_cast<float4*>(blk + lane * 32 + ((c ^ (lane & 7)) << 2)) =
+                        make_float4(sum[cb * 32 + 4 * c], sum[cb * 32 + 4 * c + 1], sum[cb * 32 + 4 * c + 2], sum[cb * 32 + 4 * c + 3]);
+                __syncwarp();
+                const float f[4] = {column_inverse(mag.x), column_inverse(mag.y), column_inverse(mag.z), column_inverse(mag.w)};
+                const size_t at0 = (size_t)(row0 + rr) * N + n;
+#pragma unroll
+                for (int g0 = 0; g0 < 8; g0 += 4) {
+                    float4 add[4];
+#pragma unroll
+                    for (int g = 0; g < 4; ++g) {
+                        add[g] = make_float4(0.f, 0.f, 0.f, 0.f);
+                        if (p.residual && in && 4 * (g0 + g) + rr < rows) add[g] = *reinterpret_cast<const float4*>(p.residual + at0 + (size_t)(4 * (g0 + g)) * N);
+                    }
+#pragma unroll
+                    for (int g = 0; g < 4; ++g) {
+                        const int r = 4 * (g0 + g) + rr;
+                        const float4 a = *reinterpret_cast<const float4*>(blk + r * 32 + ((ch ^ (r & 7)) << 2));
+                        const float o[4] = {a.x, a.y, a.z, a.w}, z[4] = {add[g].x, add[g].y, add[g].z, add[g].w};
+                        float y[4];
+#pragma unroll
+                        for (int e = 0; e < 4; ++e)           // (no step out of range that the result is not)
+                            y[e] = o[e] * fminf(ri[g0 + g], f[e]) * fmaxf(ri[g0 + g], f[e]) + z[e];
+                        if (in && r < rows) *reinterpret_cast<float4*>(p.y + at0 + (size_t)(4 * (g0 + g)) * N) = make_float4(y[0], y[1], y[2], y[3]);
+                    }
+                }
+                __syncwarp();
             }
         }
     } else {
         const int q = warp & 3;
-        float* const blk = reinterpret_cast<float*>(turn + (warp - 2) * 4096);
+        float* const blk = reinterpret_cast<float*>(turn + (warp - Pair<SUMS>::kFirst) * 4096);
         const int rr = lane >> 3, ch = lane & 7;              // a lane's row of four and its 16-byte piece of a 32-column block
         unsigned it = 0;
         for (int t = pair; t < n_tiles; t += pairs) {
@@ -1033,22 +1269,27 @@ static bool dense_rows_f32(int terms, int M, int N, int K, int sms, int pairs);
 static cudaError_t run_gemm_f32(const F32Product& p, const void* a_terms, int terms, int splits, cudaStream_t st);
 
 // clusters of two CTAs of the pair kernel that run at the same time
+template <int TERMS, bool SUMS>
 static cudaError_t pairs_of(int dev, int* out) {
     static std::atomic<int> known[64];
     if (dev >= 0 && dev < 64 && (*out = known[dev].load(std::memory_order_relaxed)) > 0) return cudaSuccess;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(2);
-    cfg.blockDim = dim3(kGemmThreads);
-    cfg.dynamicSmemBytes = kPairSmem;
+    cfg.blockDim = dim3(Pair<SUMS>::kThreads);
+    cfg.dynamicSmemBytes = Pair<SUMS>::kSmem;
     cudaLaunchAttribute attr;
     attr.id = cudaLaunchAttributeClusterDimension;
     attr.val.clusterDim.x = 2;
     attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
-    cudaError_t e = cudaFuncSetAttribute(dia_gemm_pair_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmem);
-    if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(out, dia_gemm_pair_kernel<1>, &cfg);
+    const auto kernel = dia_gemm_pair_kernel<TERMS, SUMS>;
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Pair<SUMS>::kSmem);
+    cudaFuncAttributes built;
+    if (e == cudaSuccess) e = cudaFuncGetAttributes(&built, kernel);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(out, kernel, &cfg);
     if (e != cudaSuccess) return e;
+    if (SUMS && built.numRegs < Pair<SUMS>::kRegs) return cudaErrorNotSupported;      // (its roles would wait for registers that are not there)
     if (*out < 1) return cudaErrorNotSupported;
     if (dev >= 0 && dev < 64) known[dev].store(*out, std::memory_order_relaxed);
     return cudaSuccess;
@@ -1056,9 +1297,9 @@ static cudaError_t pairs_of(int dev, int* out) {
 
 // Columns of a pair's tile: the width whose rounds of tiles end first.  A round's time grows with its columns where the MMAs bound it (three
 // terms, us per k-block alone on the chip: 0.44 at 128, 0.63 at 192, 0.83 at 256) and hardly where issuing four of them does (one term:
-// 0.30 and 0.28).  1722 rows x 16384 columns, K = 2048, three terms: 7 rounds of 256 223 us, 7 of 224 209; 3072 columns: 2 of 256 69, 2 of 160 49
+// 0.30 and 0.28; two terms with fp32 sums, seven rounds of 32 k-blocks, 16.2 at 128 and 24.5 at 256 a round).  1722 rows x 16384 columns, K = 2048, three terms: 7 rounds of 256 223 us, 7 of 224 209; 3072 columns: 2 of 256 69, 2 of 160 49
 static int pair_columns(int terms, int M, int N, int pairs, long long* rounds) {
-    const int tiles_m = (M + 2 * BM - 1) / (2 * BM), fixed = terms == 1 ? 700 : 30;
+    const int tiles_m = (M + 2 * BM - 1) / (2 * BM), fixed = terms == 1 ? 700 : terms == 2 ? 100 : 30;
     int best = 0;
     long long least = 0;
     for (int bn = 256; bn >= 128; bn -= 32) {
@@ -1067,6 +1308,28 @@ static int pair_columns(int terms, int M, int N, int pairs, long long* rounds) {
     }
     return best;
 }
+template <int TERMS, bool SUMS>
+static cudaError_t run_pair(const CUtensorMap& ma, const void* wt, long long wt_rows, PairProduct& q, int dev, cudaStream_t st) {
+    int pairs = 0;
+    cudaError_t e = pairs_of<TERMS, SUMS>(dev, &pairs);
+    const auto kernel = dia_gemm_pair_kernel<TERMS, SUMS>;
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Pair<SUMS>::kSmem);
+    if (e != cudaSuccess) return e;
+    q.ran_out = split_attention_ran_out(dev, st);
+    if (q.ran_out && *reinterpret_cast<volatile int*>(q.ran_out)) {
+        *q.ran_out = 0;
+        return cudaErrorLaunchTimeout;
+    }
+    long long rounds = 0;
+    q.BN = pair_columns(TERMS, q.M, q.N, pairs, &rounds);
+    q.stages = std::min(kPairStagesMost, Pair<SUMS>::kSlots * kTileBytes / (TERMS * kTileBytes + q.BN / 2 * 128));
+    CUtensorMap mb;
+    if (!make_map(&mb, wt, wt_rows, q.K, q.BN / 2)) return cudaErrorNotSupported;
+    const int n_tiles = ((q.N + q.BN - 1) / q.BN) * ((q.M + 2 * BM - 1) / (2 * BM));
+    kernel<<<2 * std::min(n_tiles, pairs), Pair<SUMS>::kThreads, Pair<SUMS>::kSmem, st>>>(ma, mb, q);
+    return cudaGetLastError();
+}
+
 // A: bf16 [terms * M][K], the terms of the activation stacked (terms = 1: the activation itself); Wt: bf16 [wt_rows][K].
 // Returns cudaErrorNotSupported for shapes the tiling does not cover (the caller decides what to do).
 cudaError_t launch_gemm_tcgen05_bf16(const void* a_bf16, int terms, const void* wt, long long wt_rows, float* y, int M, int N,
@@ -1092,7 +1355,7 @@ cudaError_t launch_gemm_tcgen05_bf16(const void* a_bf16, int terms, const void* 
     }
     const int sms = (dev < 0 || dev >= 64) ? n_sm[0] : n_sm[dev];
     int pairs = 0;
-    e0 = pairs_of(dev, &pairs);
+    e0 = pairs_of<1, false>(dev, &pairs);
     if (e0 != cudaSuccess) return e0;
     if (terms == 1 && !groups && wt_rows == N && dense_rows_f32(1, M, N, K, sms, pairs)) {
         const F32Product narrow{nullptr, 0, 0, wt, ep.y_bf16 ? nullptr : y, N, N, ep.y_bf16, 1, M, N, K, 1.f, ep.y_bf16 ? 3 : 0, nullptr, 0, 0,
@@ -1100,22 +1363,11 @@ cudaError_t launch_gemm_tcgen05_bf16(const void* a_bf16, int terms, const void* 
         if (gemm_f32_ok(narrow)) return run_gemm_f32(narrow, a_bf16, 1, 8, st);
     }
     if (M > BM && (terms == 1 || terms == kTerms) && (!groups || groups->tile_rows % (2 * BM) == 0)) {
-        const auto kernel = terms == 1 ? dia_gemm_pair_kernel<1> : dia_gemm_pair_kernel<kTerms>;
-        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmem);
-        if (e != cudaSuccess) return e;
-        long long rounds = 0;
-        const int bn = pair_columns(terms, M, N, pairs, &rounds);
-        const PairProduct q{y, ep.residual, M, N, K, bn, std::min(kPairStagesMost, kPairSlots * kTileBytes / (terms * kTileBytes + bn / 2 * 128)),
-                            ep.dyt_w, ep.dyt_b, ep.dyt_alpha, reinterpret_cast<__nv_bfloat16*>(ep.y_bf16), groups ? groups->row_group : nullptr,
-                            groups ? groups->group_rows : 0, groups ? groups->n_rows : nullptr, split_attention_ran_out(dev, st)};
-        if (q.ran_out && *reinterpret_cast<volatile int*>(q.ran_out)) {
-            *q.ran_out = 0;
-            return cudaErrorLaunchTimeout;
-        }
-        if (!make_map(&mb, wt, wt_rows, K, bn / 2)) return cudaErrorNotSupported;
-        const int n_tiles = ((N + bn - 1) / bn) * ((M + 2 * BM - 1) / (2 * BM));
-        kernel<<<2 * std::min(n_tiles, pairs), kGemmThreads, kPairSmem, st>>>(ma, mb, q);
-        return cudaGetLastError();
+        PairProduct q{};
+        q.y = y; q.residual = ep.residual; q.M = M; q.N = N; q.K = K;
+        q.dyt_w = ep.dyt_w; q.dyt_b = ep.dyt_b; q.dyt_alpha = ep.dyt_alpha; q.y_bf16 = reinterpret_cast<__nv_bfloat16*>(ep.y_bf16);
+        if (groups) { q.row_group = groups->row_group; q.group_rows = groups->group_rows; q.n_rows = groups->n_rows; }
+        return terms == 1 ? run_pair<1, false>(ma, wt, wt_rows, q, dev, st) : run_pair<kTerms, false>(ma, wt, wt_rows, q, dev, st);
     }
     const int n_tiles = ((N + BN - 1) / BN) * ((M + BM - 1) / BM);
     dia_gemm_tcgen05_kernel<<<std::min(n_tiles, sms), kGemmThreads, kGemmSmem, st>>>(
@@ -1141,10 +1393,10 @@ static int f32_splits(int tiles, int n_kb, int most, int sms) {
 }
 // Beyond 32 rows (and for bf16 rows) the fp32-sum kernel where its rounds of tiles are the shorter ones: its 128 x 128 tiles are twice
 // as many as 128 x 256 ones, and where they leave the chip idle its clusters split K.  Three terms: a k-block of a round takes three quarters
-// of one of 128 x 256 tiles on one SM (1.1 and 1.4 us).  (Pairs of SMs take 0.4 to 0.8 us, but their sums of all K products in tensor memory
-// are ten times further off: what had fp32 sums keeps them.)  One term, us, pair / here: 512 rows N = K = 2048 18 / 16, 1024 rows 18 / 22; 1722
-// rows N = 768 18 / 22, 800 rows 17 / 16: a k-block takes 0.34 us there and 0.46 here, and starting and ending 1 us longer.  Up to 128 rows half
-// of a pair's tile would be empty: against one SM's 128 x 256 tiles 21 to 20 units a k-block (100 rows N = 32768, K = 2048 21 us, pairs 33)
+// of one of 128 x 256 tiles on one SM (1.1 and 1.4 us).  (Pairs of SMs take 0.4 to 0.8 us, but their sums are two to ten times further off:
+// what had sums of 64 products keeps them.)  One term, us, pair / here: 512 rows N = K = 2048 18 / 16, 1024 rows 18 / 22; 1722 rows N = 768 18 /
+// 22, 800 rows 17 / 16: a k-block takes 0.34 us there and 0.46 here, and starting and ending 1 us longer.  Up to 128 rows half of a
+// pair's tile would be empty: against one SM's 128 x 256 tiles 21 to 20 units a k-block (100 rows N = 32768, K = 2048 21 us, pairs 33)
 static bool dense_rows_f32(int terms, int M, int N, int K, int sms, int pairs) {
     const int tm = (M + BM - 1) / BM, n_kb = (K + BK - 1) / BK;
     const long long narrow = (long long)tm * ((N + kFN - 1) / kFN), wide = (long long)tm * ((N + BN - 1) / BN);
@@ -1248,6 +1500,45 @@ cudaError_t launch_gemm_few_rows(const FewRowsProduct& p, bool early, cudaStream
     return p.M <= 8 ? launch_few_rows<32>(p, early, st) : launch_few_rows<96>(p, early, st);
 }
 
+// Whether M fp32 rows go as two fp16 terms to the pair kernel with fp32 sums: beyond 128 rows, what the 128 x 128 tiles of three terms do not take.
+bool gemm_half_ok(int M, int N, int K) {
+    int dev = 0, sms = 0;
+    if (M <= BM || N <= 0 || N % 4 || K < BK || K % BK) return false;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return false;
+    return !dense_rows_f32(kTerms, M, N, K, sms, 0);
+}
+
+cudaError_t launch_prepare_half(const void* w, int src_bf16, void* wt, float* mag, int* inexact, int K, int N, cudaStream_t st) {
+    const cudaError_t e = cudaMemsetAsync(mag, 0, (size_t)N * 4, st);
+    if (e != cudaSuccess) return e;
+    column_magnitudes_kernel<<<dim3((N + 255) / 256, (K + 63) / 64), 256, 0, st>>>(w, src_bf16, reinterpret_cast<uint32_t*>(mag), K, N);
+    transpose_to_half_kernel<<<dim3((N + 31) / 32, (K + 31) / 32), dim3(32, 8), 0, st>>>(w, src_bf16, mag, reinterpret_cast<__half*>(wt), inexact, K, N);
+    ++extra_launches();
+    return cudaGetLastError();
+}
+
+// y = [residual +] x W for fp32 rows: two fp16 terms and fp32 sums of 64-product pieces, on pairs of SMs.
+cudaError_t launch_gemm_half(const float* x, const float* norm_w, float eps, bool gated, const void* wt, const float* mag, const float* residual, float* y,
+                             void* workspace, int M, int N, int K, cudaStream_t st) {
+    if (M <= 0 || N <= 0 || N % 4 || K < BK || K % BK || (gated && norm_w)) return cudaErrorNotSupported;
+    __half* const terms = reinterpret_cast<__half*>(workspace);
+    float* const row_inv = reinterpret_cast<float*>(terms + 2 * (size_t)M * K);
+    if (gated)
+        split2_rows_kernel<true><<<M, 256, 0, st>>>(x, nullptr, 0.f, terms, row_inv, M, K);
+    else
+        split2_rows_kernel<false><<<M, 256, 0, st>>>(x, norm_w, eps, terms, row_inv, M, K);
+    ++extra_launches();
+    CUtensorMap ma;
+    int dev = 0;
+    const cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    if (!make_map(&ma, terms, 2LL * M, K, BM)) return cudaErrorNotSupported;
+    PairProduct q{};
+    q.y = y; q.residual = residual; q.M = M; q.N = N; q.K = K;
+    q.row_inv = row_inv; q.col_mag = mag;
+    return run_pair<2, true>(ma, wt, N, q, dev, st);
+}
+
 // fp32 activations: the three-term split (with the row's RMSNorm in front when norm_w is given), then the kernel
 cudaError_t launch_gemm_tcgen05(const float* x, const float* norm_w, float eps, const void* wt, const float* residual,
                                 float* y, void* workspace, int M, int N, int K, cudaStream_t st) {
@@ -1276,10 +1567,8 @@ cudaError_t launch_gemm_tcgen05(const float* x, const float* norm_w, float eps, 
     int dev = 0, sms = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    int pairs = 0;
-    if (e == cudaSuccess) e = pairs_of(dev, &pairs);
     if (e != cudaSuccess) return e;
-    if (dense_rows_f32(kTerms, M, N, K, sms, pairs) && gemm_f32_ok(wide)) return run_gemm_f32(wide, workspace, kTerms, 8, st);
+    if (dense_rows_f32(kTerms, M, N, K, sms, 0) && gemm_f32_ok(wide)) return run_gemm_f32(wide, workspace, kTerms, 8, st);
     const GemmEpilogue ep{residual, nullptr, nullptr, 0.f, nullptr};
     return launch_gemm_tcgen05_bf16(workspace, kTerms, wt, N, y, M, N, K, ep, nullptr, st);
 }

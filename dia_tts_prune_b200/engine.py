@@ -7,6 +7,7 @@ arithmetic happens in ``csrc/`` kernels; there is no eager / CPU fallback here.
 from __future__ import annotations
 
 import ctypes as C
+import functools
 
 import torch
 
@@ -442,6 +443,45 @@ def dense_forward(x_MxK: torch.Tensor, wt_NxK: torch.Tensor, norm_weight: torch.
     _lib.check(lib.dia_b200_dense_forward_fused(_ptr(x), _ptr(nw) if nw is not None else None, float(eps), _ptr(wt_NxK),
                                                 _ptr(residual) if residual is not None else None, _ptr(y), _ptr(ws),
                                                 M, N, K, _stream(x.device)), "dense_forward")
+    return y
+
+
+@functools.lru_cache(maxsize=4096)
+def _half_rows(device: int, M: int, N: int, K: int) -> bool:
+    with torch.cuda.device(device):
+        return bool(_lib.load().dia_b200_dense_half_rows(M, N, K))
+
+
+def dense_half_rows(M: int, N: int, K: int, device: torch.device) -> bool:
+    """Whether a product of ``M`` float32 rows belongs to :func:`dense_forward_half`."""
+    return M > 128 and _half_rows(device.index if device.index is not None else torch.cuda.current_device(), M, N, K)
+
+
+def dense_prepare_half(w_KxN: torch.Tensor, inexact: torch.Tensor) -> tuple[torch.Tensor, torch.Tensor]:
+    """K-major fp16 copy ``[N, K]`` of a DenseGeneral kernel, a power of two per column, and the columns' largest magnitudes ``[N]``.
+    ``inexact`` (int32, one element on the device) is set where fp16 cannot hold the bf16 values."""
+    lib = _lib.load()
+    w = w_KxN.contiguous()
+    K, N = w.shape
+    wt = torch.empty((N, K), dtype=torch.float16, device=w.device)
+    mag = torch.empty((N,), dtype=torch.float32, device=w.device)
+    _lib.check(lib.dia_b200_dense_prepare_half(_ptr(w), 1 if w.dtype == torch.bfloat16 else 0, _ptr(wt), _ptr(mag), _ptr(inexact), K, N,
+                                               _stream(w.device)), "dense_prepare_half")
+    return wt, mag
+
+
+def dense_forward_half(x: torch.Tensor, half: tuple[torch.Tensor, torch.Tensor], norm_weight: torch.Tensor | None = None, eps: float = 1e-5,
+                       residual: torch.Tensor | None = None, gated: bool = False) -> torch.Tensor:
+    """:func:`dense_forward` for many rows, ``half`` from :func:`dense_prepare_half`; ``gated``: ``x`` is ``[M, 2, K]`` (gate, up)."""
+    lib = _lib.load()
+    wt, mag = half
+    N, K = wt.shape
+    M = x.shape[0]
+    y = residual if residual is not None else torch.empty((M, N), dtype=torch.float32, device=x.device)
+    ws = torch.empty((int(lib.dia_b200_dense_workspace_bytes(M, K)),), dtype=torch.uint8, device=x.device)
+    _lib.check(lib.dia_b200_dense_forward_half(_ptr(x), _ptr(norm_weight) if norm_weight is not None else None, float(eps), int(gated), _ptr(wt),
+                                               _ptr(mag), _ptr(residual) if residual is not None else None, _ptr(y), _ptr(ws), M, N, K,
+                                               _stream(x.device)), "dense_forward_half")
     return y
 
 

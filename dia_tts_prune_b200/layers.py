@@ -76,17 +76,21 @@ class DenseGeneral(nn.Module):
     # land on the very address the old one had
     def __setattr__(self, name, value):
         if name in ("weight", "weight_orig", "weight_mask"):
-            self.__dict__.pop("_b200_wt", None)
+            self._drop_copies()
         super().__setattr__(name, value)
 
     def __delattr__(self, name):
         if name in ("weight", "weight_orig", "weight_mask"):
-            self.__dict__.pop("_b200_wt", None)
+            self._drop_copies()
         super().__delattr__(name)
 
     def _apply(self, fn, *a, **kw):
-        self.__dict__.pop("_b200_wt", None)
+        self._drop_copies()
         return super()._apply(fn, *a, **kw)
+
+    def _drop_copies(self) -> None:
+        self.__dict__.pop("_b200_wt", None)
+        self.__dict__.pop("_b200_half", None)
 
     def forward(self, inputs: Tensor) -> Tensor:
         """``tensordot(x, W)`` over ``axis`` (dia/layers.py:55-66).  On a CUDA device every call runs on the tcgen05
@@ -117,9 +121,25 @@ class DenseGeneral(nn.Module):
             self._b200_wt = cached
         return cached[1]
 
+    def kernel_weight_half(self) -> tuple[Tensor, Tensor] | None:
+        """The fp16 copy that products of many rows read (made once per weight version), or None: fp16 cannot hold these weights, or the
+        stream is being captured and there is no copy yet."""
+        key = self._weight_key()
+        cached = self.__dict__.get("_b200_half")
+        if cached is None or cached[0] != key:
+            if torch.cuda.is_current_stream_capturing():
+                return None
+            prepare_half_kernels([self])
+            cached = self._b200_half
+        return cached[1]
+
+    def _weight_key(self):
+        w = self.weight
+        return (w.data_ptr(), w._version, w.dtype, w.device)
+
     def _forward_tcgen05(self, inputs: Tensor, x_axes: tuple[int, ...], norm_weight: Tensor | None = None,
                          eps: float = 1e-5, residual: Tensor | None = None) -> Tensor:
-        """``x @ W`` on the tcgen05 tensor cores with the activations split into three bf16 terms (float32-operand
+        """``x @ W`` on the tcgen05 tensor cores with the activations split into three bf16 terms or, for many rows, two fp16 terms (float32-operand
         accuracy).  ``norm_weight``: RMSNorm of the input rows fused into the split pass; ``residual``: added in the
         epilogue (the result aliases it)."""
         from . import engine as _engine
@@ -134,9 +154,48 @@ class DenseGeneral(nn.Module):
         if not _engine.dense_supported(M, N, K):
             raise NotImplementedError(f"dense layer [{M} x {K}] . [{K} x {N}] does not fit the tcgen05 tiling "
                                       f"(K must be a multiple of 64, N of 4)")
+        if _engine.dense_half_rows(M, N, K, inputs.device):
+            x, r = inputs.reshape(M, K), None if residual is None else residual.reshape(M, N)
+            half = self.kernel_weight_half() if _plain(x, norm_weight, r) else None
+            if half is not None:
+                return _engine.dense_forward_half(x, half, norm_weight, eps, r).reshape(*lead, *self.out_features)
         y = _engine.dense_forward(inputs.reshape(M, K), self.kernel_weight_kmajor(), norm_weight=norm_weight, eps=eps,
                                   residual=None if residual is None else residual.reshape(M, N))
         return y.reshape(*lead, *self.out_features)
+
+
+def _plain(*tensors: Tensor | None) -> bool:
+    """float32, contiguous and 16-byte aligned."""
+    return all(t is None or (t.dtype == torch.float32 and t.is_contiguous() and t.data_ptr() % 16 == 0) for t in tensors)
+
+
+@torch.no_grad()
+def prepare_half_kernels(modules: list["DenseGeneral"]) -> None:
+    """The fp16 copies of these kernels, with one look at whether they are exact for all of them."""
+    from . import engine as _engine
+    def missing(m):
+        cached = m.__dict__.get("_b200_half")
+        return cached is None or cached[0] != m._weight_key()
+
+    todo = [m for m in modules if missing(m)]
+    for m in todo:
+        canonicalize_dense_kernel_(m)
+    if not todo:
+        return
+    flags = torch.zeros((len(todo),), dtype=torch.int32, device=todo[0].weight.device)
+    halves = [_engine.dense_prepare_half(m.weight.detach().reshape(math.prod(m.in_shapes), math.prod(m.out_features)), flags[i:i + 1])
+              for i, m in enumerate(todo)]
+    for m, half, inexact in zip(todo, halves, flags.tolist()):
+        m._b200_half = (m._weight_key(), None if inexact else half)
+
+
+def _prepare_for_rows(module: nn.Module, probe: "DenseGeneral", M: int) -> None:
+    """The fp16 copies of those dense kernels inside ``module`` whose products of ``M`` rows read them, unless ``probe`` has its own."""
+    from . import engine as _engine
+    cached = probe.__dict__.get("_b200_half")
+    if M > 128 and (cached is None or cached[0] != probe._weight_key()) and not torch.cuda.is_current_stream_capturing():
+        prepare_half_kernels([m for m in module.modules() if isinstance(m, DenseGeneral) and m.weight.is_cuda and
+                              _engine.dense_half_rows(M, math.prod(m.out_features), math.prod(m.in_shapes), m.weight.device)])
 
 
 _ROUNDING_WARNED = False
@@ -191,6 +250,11 @@ class MlpBlock(nn.Module):
         from . import engine as _k
         lead = x.shape[:-1]
         gu = self.wi_fused._forward_tcgen05(x, (x.ndim - 1,), norm_weight=None if norm is None else norm.weight, eps=eps)
+        if residual is not None and _k.dense_half_rows(gu.numel() // (2 * gu.shape[-1]), residual.shape[-1], gu.shape[-1], gu.device):
+            half = self.wo.kernel_weight_half() if _plain(gu, residual) else None
+            if half is not None:                            # the gate inside the split pass of the second GEMM
+                return _k.dense_forward_half(gu.reshape(-1, 2, gu.shape[-1]), half, residual=residual.reshape(-1, residual.shape[-1]),
+                                             gated=True).reshape(residual.shape)
         h = _k.silu_mul(gu.reshape(-1, 2, gu.shape[-1]))
         return self.wo._forward_tcgen05(h.reshape(*lead, -1), (x.ndim - 1,), residual=residual)
 
@@ -644,6 +708,7 @@ class Decoder(nn.Module):
         if tgt_ids_BxTxC.is_cuda and not torch.is_grad_enabled():
             # own kernels end to end: embedding gather-sum, 18 x (fused-norm GEMMs, RoPE + cache scatter, fp32 attention,
             # gate, residual epilogues), final norm fused into the logits GEMM
+            _prepare_for_rows(self, self.layers[0].mlp.wi_fused, B * T)
             x = self.engine().embed_sum(tgt_ids_BxTxC.reshape(B * T, C)).reshape(B, T, -1)
             state.extras.pop("prefill_pos", None)
             for i, layer in enumerate(self.layers):

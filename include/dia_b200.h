@@ -238,6 +238,16 @@ int dia_b200_dense_forward(const float *x, const void *wt_bf16, float *y, void *
 int dia_b200_dense_forward_fused(const float *x, const float *norm_weight, float eps, const void *wt_bf16,
                                  const float *residual, float *y, void *workspace, int M, int N, int K, void *stream);
 
+/* The same for many rows (dia_b200_dense_half_rows says which): x as two fp16 terms with a power of two per row, W as the K-major fp16 copy
+ * wt_half[N][K] with a power of two per column, products summed in fp32.  magnitudes: float32 [N], the columns' largest magnitudes.
+ * prepare_half sets *inexact (device int32, zeroed by the caller) where fp16 cannot hold the bf16 weights, beyond 2^31 between a column's
+ * largest and smallest value: such weights stay with dense_forward_fused.  gated: x is [M][2][K], and the rows are silu(x[m][0]) x[m][1]
+ * (norm_weight NULL).  x, norm_weight and all buffers 16-byte aligned; K % 64 == 0 and N % 4 == 0. */
+int dia_b200_dense_half_rows(int M, int N, int K);
+int dia_b200_dense_prepare_half(const void *w, int src_dtype, void *wt_half, float *magnitudes, int32_t *inexact, int K, int N, void *stream);
+int dia_b200_dense_forward_half(const float *x, const float *norm_weight, float eps, int gated, const void *wt_half, const float *magnitudes,
+                                const float *residual, float *y, void *workspace, int M, int N, int K, void *stream);
+
 /* ---- the rest of the T > 1 passes (once per utterance): no library kernel on the path ---------------------------
  * F.scaled_dot_product_attention call sites (dia/layers.py:329-337) for more than one query row, fp32.
  *   q, out float32 [B][Tq][Hq][128] (q already rotated); k, v float32 [B][Hkv][Tk_stride][128] (KVCache layout,

@@ -56,3 +56,69 @@ def test_expert_groups(rows, top):
     ref = O.routed_experts(h.double(), p, cfg["layers"][0]["mlp"])
     got = model.engine.op_ff(0, h.cuda()).double().cpu()
     assert (got - ref).norm() <= 2.0 ** -7 * ref.norm()
+
+
+@pytest.mark.parametrize("M,N,K,gated,norm,residual", [(129, 16388, 64, False, False, True), (257, 9252, 320, False, True, False),
+                                                       (300, 2052, 8256, False, True, True), (511, 260, 576, True, False, True),
+                                                       (1722, 2048, 256, False, False, False), (300, 132, 8256, True, False, False)])
+def test_two_fp16_terms(M, N, K, gated, norm, residual):
+    """Edges of the row tiles, of every tile width, of chunks of four k-blocks and of the rows that fit a CTA's registers (8192 channels).  Terms and
+    weights are exact to 2^-22 of a value, an accumulator takes 32 additions that cut off, and there are K / 256 fp32 additions."""
+    from dia_tts_prune_b200 import engine
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    x = torch.randn((M, 2 * K if gated else K), generator=g, device="cuda") * torch.exp2(torch.randint(-50, 50, (M, 1), generator=g, device="cuda").float())
+    if gated:
+        x = x.clamp(-1e9, 1e9)
+    w = (torch.randn((K, N), generator=g, device="cuda") * torch.exp2(torch.randint(-20, 20, (1, N), generator=g, device="cuda").float())).bfloat16()
+    nw = torch.rand((K,), generator=g, device="cuda") + 0.5 if norm else None
+    inexact = torch.zeros((1,), dtype=torch.int32, device="cuda")
+    half = engine.dense_prepare_half(w, inexact)
+    assert inexact.item() == 0
+    xd = x.double()
+    if gated:
+        xd = torch.nn.functional.silu(xd[:, :K]) * xd[:, K:]
+    if norm:
+        xd = xd * torch.rsqrt((xd * xd).mean(-1, keepdim=True) + 1e-5) * nw.double()
+    ref, size = xd @ w.double(), xd.abs() @ w.double().abs()
+    r = torch.randn((M, N), generator=g, device="cuda") * ref.abs().max(1, keepdim=True).values.float() if residual else None
+    if residual:
+        ref, size = ref + r.double(), size + r.double().abs()
+    got = engine.dense_forward_half(x.reshape(M, 2, K) if gated else x, half, nw, 1e-5, r.clone() if residual else None, gated)
+    assert ((got - ref).abs() <= 2.0 ** -23 * (8 + 34 + K / 256) * size).all()
+
+
+def test_two_fp16_terms_at_the_ends_of_fp32():
+    """Rows of the smallest and the largest numbers, zeros, infinities and NaNs beside ordinary ones, against three bf16 terms."""
+    from dia_tts_prune_b200 import engine
+    g = torch.Generator(device="cuda").manual_seed(1)
+    x, w = torch.randn((130, 128), generator=g, device="cuda"), torch.randn((128, 128), generator=g, device="cuda").bfloat16()
+    x[0], x[1] = x[0] * 1e-38, x[1].clamp(-3, 3) * 1e36
+    x[2] = 0.0
+    x[3, 5], x[4, 6] = float("inf"), float("nan")
+    inexact = torch.zeros((1,), dtype=torch.int32, device="cuda")
+    got, ref = engine.dense_forward_half(x, engine.dense_prepare_half(w, inexact)), x.double() @ w.double()
+    assert (got[0] - ref[0]).abs().max() <= 1e-5 * ref[0].abs().max() and (got[1] - ref[1]).abs().max() <= 1e-5 * ref[1].abs().max()
+    assert (got[2] == 0).all() and not torch.isfinite(got[3:5]).any() and torch.isnan(got[4]).all()
+    assert (torch.isinf(got[3]) & (got[3].double() == ref[3])).sum() == torch.isinf(ref[3]).sum()
+    assert (got[5:] - ref[5:]).abs().max() <= 1e-5 * ref[5:].abs().max()
+
+
+def test_weights_that_fp16_cannot_hold():
+    """2^33 between the values of one column, or an infinity: told by the flag, and such a layer keeps its three bf16 terms."""
+    from dia_tts_prune_b200 import engine
+    from dia_tts_prune_b200.layers import DenseGeneral
+    for small, big, fits in ((2.0 ** -31, 1.0, True), (2.0 ** -33 * 1.0078125, 1.0, False), (1.0, float("inf"), False)):
+        w = torch.full((64, 4), small, device="cuda").bfloat16()
+        w[3, 2] = big
+        inexact = torch.zeros((1,), dtype=torch.int32, device="cuda")
+        engine.dense_prepare_half(w, inexact)
+        assert (inexact.item() == 0) == fits
+    d = DenseGeneral((64,), (16384,), weight_dtype=torch.bfloat16, device="cuda")
+    with torch.no_grad():
+        d.weight.normal_()
+        x = torch.randn((600, 64), device="cuda")
+        assert engine.dense_half_rows(600, 16384, 64, x.device) and d.kernel_weight_half() is not None
+        d.weight[7, 9] = 2.0 ** -40
+        assert d.kernel_weight_half() is None
+        ref = x.double() @ d.weight.double()
+        assert (d(x) - ref).norm() <= 1e-6 * ref.norm()
