@@ -3,13 +3,13 @@
 //
 // A CTA owns 128 (token, head) rows: up to 128 / PK consecutive tokens times PK query heads that read the same key/value head, so
 // that a tile of keys serves all of them.  It walks its keys 64 at a time:
-//   warps 8 .. 11   fetch key and value rows from the pages, scale them by a power of two, split x = hi + lo into fp16 and put both
+//   4 warps         fetch key and value rows from the pages, scale them by a power of two, split x = hi + lo into fp16 and put both
 //                   into a ring of shared-memory slots ([key / 8][channel / 8] blocks of 8 x 16 bytes: the layout is the K-major
 //                   operand of the scores and the MN-major operand of the value product)
-//   warp 12         issues tcgen05.mma: scores S = Q K^T (M = 128, N = 64; lo hi, hi lo, then hi hi, so that the small terms are
+//   1 warp          issues tcgen05.mma: scores S = Q K^T (M = 128, N = 64; lo hi, hi lo, then hi hi, so that the small terms are
 //                   added first) per group of at most 128 channels, and the value product of the tile before (weights as the
 //                   operand in tensor memory)
-//   warps 0 .. 7    two threads per row, 32 keys each: scores from tensor memory (the channel groups are summed here, in fp32),
+//   8 or 16 warps   two or four threads per row, 32 or 16 keys each: scores from tensor memory (the channel groups are summed here, in fp32),
 //                   cap, bias, mask, online softmax in base 2, weights split and written to tensor memory; then the value
 //                   product of the tile before is added to the row's fp32 registers
 // The accumulator of a tensor-core product loses up to one unit in the last place at every step, towards zero (measured: 2e-6
@@ -26,9 +26,9 @@
 // 237 -> 264 us; mixed scores, three prompts of 2048 rows, 8 heads of 128 over 2, 127 -> 146, of which the factors per key and per
 // value 5 us each; 16 keys that share a factor (scales in steps of 2^8) take as long.
 //
-// Bound: the latencies of a row warp's dependent steps.  Per 64 keys and 128 rows 3 x 128 x 64 x (dk + dv) multiply-adds on the tensor
-// pipe (1536 cycles at 128 + 128) stand against about 7000 cycles of a tile, in which two row warps per scheduler issue on a third of
-// them (tensor pipe busy 18 %, shared memory 6 %: profiles/split_kernels_ncu.txt).
+// Bound: the instructions of the row warps and their latencies.  Per 64 keys and 128 rows 3 x 128 x 64 x (dk + dv) multiply-adds on the tensor
+// pipe (1536 cycles at 128 + 128) stand against about 6400 cycles of a tile, on 2900 of which a scheduler issues (four row warps on each;
+// with two row warps 7000 and 2400).  Instruction fetches and fixed latencies are the largest waits.
 // Every wait is bounded: a wait that runs out makes the CTA write NaN, note it in a word that the host reads, and end; the next launch
 // on the device returns an error.
 #include <algorithm>
@@ -49,7 +49,8 @@ namespace dia {
 namespace {
 
 constexpr int kRows = 128, kKeys = 64, kGroupW = 128;        // query rows of a CTA, keys of a tile, channels of a stage
-constexpr int kSplitThreadsTC = 512;
+template <int RT>
+constexpr int kSplitThreads = 32 * (4 * RT + 8);
 constexpr int kMaxSlots = 6, kMaxDepth = 5, kMaxKStages = 4;
 constexpr int kSmemMost = 232448;                             // all of it dynamic
 constexpr float kLog2e = 1.4426950408889634f;
@@ -137,9 +138,18 @@ __device__ __forceinline__ void tmem_load8(uint32_t addr, float* v) {
                  : "r"(addr)
                  : "memory");
 }
+__device__ __forceinline__ void tmem_load16(uint32_t addr, float* v) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+        : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7]), "=f"(v[8]), "=f"(v[9]),
+          "=f"(v[10]), "=f"(v[11]), "=f"(v[12]), "=f"(v[13]), "=f"(v[14]), "=f"(v[15])
+        : "r"(addr)
+        : "memory");
+}
 template <int N>
 __device__ __forceinline__ void tmem_load_n(uint32_t addr, float (&v)[N]) {
     if constexpr (N == 32) tmem_load32(addr, v);
+    else if constexpr (N == 16) tmem_load16(addr, v);
     else tmem_load8(addr, v);
 }
 // two fp32 operations in one instruction
@@ -476,16 +486,19 @@ __device__ __noinline__ void plain_row(const SplitAttention& p, int r, int slot,
         if (lane + 32 * u < n) dst[lane + 32 * u] = o[u] * f;
 }
 
-// NVS: channel groups of a value (1: up to 128 channels, a thread of a row keeps half of them; 2: up to 256, a group each)
-template <int NVS>
-__global__ void __launch_bounds__(kSplitThreadsTC, 1)
+// NVS: channel groups of a value (1: up to 128 channels, 2: up to 256).  RT: threads of a row; each takes 64 / RT keys of a tile and an equal
+// share of the output channels
+template <int NVS, int RT>
+__global__ void __launch_bounds__(kSplitThreads<RT>, 1)
 split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_constant__ Geometry geo) {
-    constexpr int DVH = 64 * NVS;                             // output channels of a thread
-    // The block is launched with 128 registers a thread: 256 of kRowRegs, 128 of kFetchRegs and 128 of 32.  (Wide values, 4096 rows, 16
-    // heads over latent rows of 256 + 32, window 1024: 184 and 112 452 us, 192 and 96 443, 200 and 80 421.  What the fetching warps
-    // spill is used for keys that are not split in advance only.)
-    constexpr int kRowRegs = NVS == 1 ? 176 : 200, kFetchRegs = NVS == 1 ? 128 : 80;
-    static_assert(256 * kRowRegs + 128 * kFetchRegs + 128 * 32 <= 128 * kSplitThreadsTC, "registers of the block");
+    constexpr int DVH = 128 * NVS / RT;                       // output channels of a thread
+    constexpr int KP = kKeys / RT, RW = 4 * RT;               // keys of a thread, row warps
+    // The block is launched with 128 registers a thread (RT = 4: 80).  (Wide values with two threads per row, 4096 rows, 16 heads over latent
+    // rows of 256 + 32, window 1024: 184 and 112 452 us, 192 and 96 443, 200 and 80 421.  What the fetching warps spill is used for
+    // keys that are not split in advance only.)
+    constexpr int kLaunchRegs = RT == 4 ? 80 : 128;
+    constexpr int kRowRegs = RT == 4 ? (NVS == 1 ? 96 : 104) : (NVS == 1 ? 176 : 200), kFetchRegs = RT == 4 ? (NVS == 1 ? 64 : 32) : (NVS == 1 ? 128 : 80);
+    static_assert(32 * RW * kRowRegs + 128 * kFetchRegs + 128 * 32 <= kLaunchRegs * kSplitThreads<RT>, "registers of the block");
     extern __shared__ __align__(128) unsigned char smem[];
     unsigned char* ring = smem;
     unsigned char* qs = ring + (size_t)geo.n_slots * geo.slot_bytes;
@@ -496,12 +509,12 @@ split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_co
     uint64_t* p_ready = s_empty + 1;                          // weights of a tile are there / its value product is done
     uint64_t* pv_done = p_ready + 1;
     uint64_t* q_ready = pv_done + 1;
-    uint64_t* pair = q_ready + 1;                             // [4] the two warps that share rows
+    uint64_t* pair = q_ready + 1;                             // [4] the warps that share rows
     uint64_t* v_ready = pair + 4;                             // [depth] the scales of a tile's values are there
     float* k_inv = reinterpret_cast<float*>(v_ready + kMaxDepth);      // [depth][k_sets][64] inverse scales of the keys
     float* v_inv = geo.shared_kv ? k_inv : k_inv + geo.depth * geo.k_sets * kKeys;      // [depth][64] of the values
-    float* row_x = v_inv + geo.depth * kKeys;                 // [2][2][128] what the two threads of a row tell each other
-    uint32_t* s_breaks = reinterpret_cast<uint32_t*>(row_x + 4 * kRows);      // [4]
+    float* row_x = v_inv + geo.depth * kKeys;                 // [2][RT][128] what the threads of a row tell each other
+    uint32_t* s_breaks = reinterpret_cast<uint32_t*>(row_x + 2 * RT * kRows);      // [4]
     uint32_t* s_tmem = s_breaks + 4;
     int* s_rows = reinterpret_cast<int*>(s_tmem + 1);         // [2]
     int* s_slot = s_rows + 3;                                 // [tokens]
@@ -547,15 +560,15 @@ split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_co
     if (tid == 0) {
         for (int i = 0; i < kMaxSlots; ++i) { mbar_init(&full[i], 4); mbar_init(&empty[i], 1); }
         mbar_init(s_full, 1);
-        mbar_init(s_empty, 8);
-        mbar_init(p_ready, 8);
+        mbar_init(s_empty, RW);
+        mbar_init(p_ready, RW);
         mbar_init(pv_done, 1);
-        mbar_init(q_ready, 8);
-        for (int i = 0; i < 4; ++i) mbar_init(&pair[i], 2);
+        mbar_init(q_ready, RW);
+        for (int i = 0; i < 4; ++i) mbar_init(&pair[i], RT);
         for (int i = 0; i < kMaxDepth; ++i) mbar_init(&v_ready[i], 4);
         fence_mbar_init();
     }
-    if (warp == 12) {
+    if (warp == RW + 4) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(s_tmem)));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::);
     }
@@ -582,8 +595,8 @@ split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_co
     const uint32_t tmem = *s_tmem;
     const uint32_t t_s = tmem, t_p = tmem + 64u * geo.n_kst, t_o = t_p + 64u;    // scores | weights (hi, lo) | value product
 
-    if (warp < 8) {
-        // ================= softmax: rows 32 (warp % 4) + lane, keys 32 (warp / 4) .. + 31 of a tile =================
+    if (warp < RW) {
+        // ================= softmax: rows 32 (warp % 4) + lane, keys KP (warp / 4) .. of a tile =================
         asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kRowRegs));
         // ---- the query tile: largest magnitude, then both terms.  Row r of the tile is head h0 + r % PK of token r / PK; a warp takes
         // eight rows at a time, a lane eight channels of one.  (The first keys are on their way meanwhile: with the tile made by all
@@ -616,7 +629,7 @@ split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_co
                 v[4] = fmaf(w, b.x, v[4]); v[5] = fmaf(w, b.y, v[5]); v[6] = fmaf(w, b.z, v[6]); v[7] = fmaf(w, b.w, v[7]);
             }
         };
-        float* const q_inv = row_x + 2 * kRows;               // [128] (read by a row's two threads before they exchange anything there)
+        float* const q_inv = row_x + RT * kRows;              // [128] (read by a row's threads before they exchange anything there)
         auto q_scale = [&](float m, int row, bool& bad) {     // a row's scale from the four lanes that hold it
             float scale, inverse;
             bad = scale_row(row_max(m), scale, inverse);
@@ -633,12 +646,13 @@ split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_co
             *reinterpret_cast<uint4*>(dst) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
             *reinterpret_cast<uint4*>(dst + (size_t)w * kRows * 2) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
         };
+        constexpr int RG = 4 / RT;                            // groups of 8 RW rows
         const int qrow = warp * 8 + (lane & 7), qch = lane >> 3;
         if (!p.talk && geo.n_kst == 1) {                      // all of it fits the registers
-            float4 v[8][2];
+            float4 v[4 * RG][2];
 #pragma unroll
-            for (int rg = 0; rg < 2; ++rg) {
-                const int row = qrow + 64 * rg, i = row >> geo.pk_shift;
+            for (int rg = 0; rg < RG; ++rg) {
+                const int row = qrow + 8 * RW * rg, i = row >> geo.pk_shift;
                 const float* src = p.q + (size_t)(r0 + i) * p.ldq + (size_t)(h0 + (row & (PK - 1))) * p.qdim + 8 * qch;
                 const int left = i < n_tok ? p.kdim - 8 * qch : 0;
 #pragma unroll
@@ -650,46 +664,46 @@ split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_co
                     }
             }
 #pragma unroll
-            for (int rg = 0; rg < 2; ++rg) {
+            for (int rg = 0; rg < RG; ++rg) {
                 float m = 0.f;
 #pragma unroll
                 for (int i = 0; i < 4; ++i) m = max_abs4(max_abs4(m, v[rg * 4 + i][0]), v[rg * 4 + i][1]);
                 bool bad;
-                const float scale = q_scale(m, qrow + 64 * rg, bad);
+                const float scale = q_scale(m, qrow + 8 * RW * rg, bad);
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
                     const float4 a = v[rg * 4 + i][0], b = v[rg * 4 + i][1];
                     const float x[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-                    q_store(qrow + 64 * rg, qch + 4 * i, scale, bad, x);
+                    q_store(qrow + 8 * RW * rg, qch + 4 * i, scale, bad, x);
                 }
             }
         } else {
-            for (int rg = 0; rg < 2; ++rg) {
+            for (int rg = 0; rg < RG; ++rg) {
                 float m = 0.f, scale = 0.f;
                 bool bad = false;
                 for (int pass = 0; pass < 2; ++pass) {
                     for (int ch = qch; ch < chunks; ch += 16) {
                         float v[4][8];
 #pragma unroll
-                        for (int i = 0; i < 4; ++i) q_values(qrow + 64 * rg, ch + 4 * i, v[i]);
+                        for (int i = 0; i < 4; ++i) q_values(qrow + 8 * RW * rg, ch + 4 * i, v[i]);
 #pragma unroll
                         for (int i = 0; i < 4; ++i) {
                             if (pass == 0) {
 #pragma unroll
                                 for (int e = 0; e < 8; ++e) m = max_nan(m, fabsf(v[i][e]));
                             } else {
-                                q_store(qrow + 64 * rg, ch + 4 * i, scale, bad, v[i]);
+                                q_store(qrow + 8 * RW * rg, ch + 4 * i, scale, bad, v[i]);
                             }
                         }
                     }
-                    if (pass == 0) scale = q_scale(m, qrow + 64 * rg, bad);
+                    if (pass == 0) scale = q_scale(m, qrow + 8 * RW * rg, bad);
                 }
             }
         }
         fence_smem_async();
         __syncwarp();
         if (lane == 0) mbar_arrive(q_ready);
-        asm volatile("bar.sync 1, 256;" ::: "memory");          // (all queries are stored, and the rows' scales are there)
+        asm volatile("bar.sync 1, %0;" ::"n"(32 * RW) : "memory");          // (all queries are stored, and the rows' scales are there)
         const int qt = warp & 3, hf = warp >> 2, row = qt * 32 + lane, tok = row >> geo.pk_shift, h = h0 + (row & (PK - 1));
         const uint32_t lanes = (uint32_t)(qt * 32) << 16;
         const int my_pos = s_pos[tok];
@@ -697,17 +711,19 @@ split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_co
         const bool ranged = p.rows_per_slot > 0 && p.mode != 0;
         // scores and maxima are in units of log 2 (a capped score from its cap on): the largest score's weight is exactly 1 at any magnitude
         const float cap = p.cap, inv_cap = cap > 0.f ? 1.0f / cap : 0.f;
-        const float mult = q_inv[row] * p.scale * (p.temp ? p.temp[h] : 1.f) * (cap > 0.f ? 1.f : kLog2e);
+        const float mult = q_inv[row] * p.scale * (p.temp ? p.temp[h] : 1.f) * (cap > 0.f ? inv_cap : kLog2e);      // (a capped score: over its cap)
         const float slope = p.slopes ? p.slopes[h] * kLog2e : 0.f;
-        const int half = NVS == 1 ? geo.wv0 >> 1 : 128;       // channels of this thread (NVS == 2: a whole group)
-        const uint32_t t_mine = t_o + (NVS == 1 ? hf * half : hf * 128) + lanes;
-        const int n_mine = NVS == 1 ? half : (hf ? geo.wv_last : geo.wv0);
+        // channels of this thread: c0 .. + n_mine, at t_mine in tensor memory
+        const int share = NVS == 1 ? (geo.wv0 + 8 * RT - 1) / (8 * RT) * 8 : DVH, part = NVS == 1 ? hf : hf % (RT / 2), group = NVS == 1 ? 0 : hf / (RT / 2);
+        const int n_mine = max(0, min(share, (group ? geo.wv_last : geo.wv0) - part * share)), c0 = group * 128 + part * share;
+        const uint32_t t_mine = t_o + c0 + lanes;
         float O[DVH];
 #pragma unroll
         for (int c = 0; c < DVH; ++c) O[c] = 0.f;
-        float m_run = -CUDART_INF_F, l_run = 0.f, corr_prev = 1.f, wi_prev = 0.f;
+        constexpr int LP = KP / 16;                           // denominators: a sum per 16 keys of a tile, the same with any threads per row
+        float m_run = -CUDART_INF_F, l_run[LP] = {}, corr_prev = 1.f, wi_prev = 0.f;
         bool ok = true;
-        constexpr int OW = NVS == 1 ? 32 : 16;                // columns in flight
+        constexpr int OW = NVS == 1 && RT == 2 ? 32 : 16;     // columns in flight
         auto add_values = [&](unsigned t, float corr, float vi) {      // O <- corr O + vi * value product of tile t (which is done)
             const bool same = __all_sync(0xffffffffu, corr == 1.f);
             const uint32_t from = t_mine + (geo.o_bufs == 2 ? (t & 1u) * 128u : 0u);
@@ -730,24 +746,24 @@ split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_co
                 }
             }
         };
-        unsigned t = 0;
+        unsigned t = 0, at_t = 0, round = 0;                  // t % depth, t / depth % 2
         Walk w(s_slot, s_pos, s_breaks, n_tok);
         for (; w.next(p); ++t) {
             if (!wait_for(s_full, t & 1u)) { ok = false; break; }
             fence_after();
-            float s[32];
-            const float* ki = k_inv + (t % geo.depth) * geo.k_sets * kKeys + hf * 32;
-            constexpr int SW = NVS == 1 ? 32 : 8;             // scores in flight (a wide value leaves fewer registers)
+            float s[KP];
+            const float* ki = k_inv + at_t * geo.k_sets * kKeys + hf * KP;
+            constexpr int SW = NVS == 1 ? KP : 8;             // scores in flight (a wide value leaves fewer registers)
 #pragma unroll
-            for (int c = 0; c < 32; c += SW) {
+            for (int c = 0; c < KP; c += SW) {
                 float v[SW];
-                tmem_load_n<SW>(t_s + lanes + hf * 32 + c, v);
+                tmem_load_n<SW>(t_s + lanes + hf * KP + c, v);
                 tmem_loaded();
 #pragma unroll
                 for (int e = 0; e < SW; ++e) s[c + e] = v[e];
                 if (geo.k_sets > 1) scale_by<SW>(s + c, ki + c);
                 for (int st = 1; st < geo.n_kst; ++st) {
-                    tmem_load_n<SW>(t_s + lanes + st * 64 + hf * 32 + c, v);
+                    tmem_load_n<SW>(t_s + lanes + st * 64 + hf * KP + c, v);
                     tmem_loaded();
                     if (geo.k_sets > 1) scale_by<SW>(v, ki + st * kKeys + c);
 #pragma unroll
@@ -757,7 +773,7 @@ split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_co
             }
             const float2 mult2 = make_float2(mult, mult);
 #pragma unroll
-            for (int e = 0; e < 32; e += 2) {
+            for (int e = 0; e < KP; e += 2) {
                 const float2 x = mul2(make_float2(s[e], s[e + 1]), mult2);
                 s[e] = x.x;
                 s[e + 1] = x.y;
@@ -766,27 +782,29 @@ split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_co
             __syncwarp();
             if (lane == 0) mbar_arrive(s_empty);
             // ---- cap, distance bias, visibility ----
-            const int k0 = w.j0 + hf * 32;
+            const int k0 = w.j0 + hf * KP;
             if (cap > 0.f) {
                 float big = 0.f;
 #pragma unroll
-                for (int e = 0; e < 32; ++e) big = fmaxf(big, fabsf(s[e]));
+                for (int e = 0; e < KP; ++e) big = fmaxf(big, fabsf(s[e]));
                 // each score takes the form that its own magnitude asks for; whether all of them are near zero decides the speed only
-                const float2 ic = make_float2(inv_cap, inv_cap), cc = make_float2(cap * kLog2e, cap * kLog2e);
-                if (__all_sync(0xffffffffu, big * inv_cap <= kTanhRange)) {
+                const float2 cc = make_float2(cap * kLog2e, cap * kLog2e);
+                const bool near = __all_sync(0xffffffffu, big <= kTanhRange);
+                if (NVS == 1 && near) {                       // (wide values: one copy of the code, whose registers are few)
 #pragma unroll
-                    for (int e = 0; e < 32; e += 2) {
-                        const float2 r = mul2(tanh_near_zero(mul2(make_float2(s[e], s[e + 1]), ic)), cc);
+                    for (int e = 0; e < KP; e += 2) {
+                        const float2 r = mul2(tanh_near_zero(make_float2(s[e], s[e + 1])), cc);
                         s[e] = r.x;
                         s[e + 1] = r.y;
                     }
                 } else {
 #pragma unroll
-                    for (int e = 0; e < 32; e += 2) {
-                        const float2 x = mul2(make_float2(s[e], s[e + 1]), ic);
-                        float2 r = tanh_near_zero(x);
-                        if (!(fabsf(x.x) <= kTanhRange)) r.x = tanhf(x.x);
-                        if (!(fabsf(x.y) <= kTanhRange)) r.y = tanhf(x.y);
+                    for (int e = 0; e < KP; e += 2) {
+                        float2 r = tanh_near_zero(make_float2(s[e], s[e + 1]));
+                        if (NVS == 1 || !near) {
+                            if (!(fabsf(s[e]) <= kTanhRange)) r.x = tanhf(s[e]);
+                            if (!(fabsf(s[e + 1]) <= kTanhRange)) r.y = tanhf(s[e + 1]);
+                        }
                         r = mul2(r, cc);
                         s[e] = r.x;
                         s[e + 1] = r.y;
@@ -795,15 +813,20 @@ split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_co
             }
             if (p.slopes) {
                 const float base = (float)(my_pos - k0);
+                const float2 ns = make_float2(-slope, -slope);
 #pragma unroll
-                for (int e = 0; e < 32; ++e) s[e] -= slope * (base - (float)e);
+                for (int e = 0; e < KP; e += 2) {
+                    const float2 r = fma2(ns, make_float2(base - (float)e, base - (float)(e + 1)), make_float2(s[e], s[e + 1]));
+                    s[e] = r.x;
+                    s[e + 1] = r.y;
+                }
             }
             auto hide = [&](float x) {                        // x in the place of every key that the row does not see
                 const bool live = tok >= w.seg_a && tok < w.seg_b;
                 const int last = live ? min(w.k_end - 1, ranged ? 0x7fffffff : my_pos) : -1, first = ranged ? w.lo : my_lo;
-                if (__all_sync(0xffffffffu, k0 + 31 <= last && (k0 >= first || k0 + 31 < kept))) return;
+                if (__all_sync(0xffffffffu, k0 + KP - 1 <= last && (k0 >= first || k0 + KP - 1 < kept))) return;
 #pragma unroll
-                for (int e = 0; e < 32; ++e) {
+                for (int e = 0; e < KP; ++e) {
                     const int j = k0 + e;
                     if (!(j <= last && (j >= first || j < kept))) s[e] = x;
                 }
@@ -811,42 +834,46 @@ split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_co
             hide(-CUDART_INF_F);
             float mx = s[0];
 #pragma unroll
-            for (int e = 1; e < 32; ++e) mx = max_nan(mx, s[e]);
-            // (two exchanges a tile in two places: whoever writes one has seen the other thread leave the one before)
+            for (int e = 1; e < KP; ++e) mx = max_nan(mx, s[e]);
+            // (two exchanges a tile in two places: whoever writes one has seen the other threads leave the one before)
             row_x[hf * kRows + row] = mx;
             __syncwarp();
             if (lane == 0) mbar_arrive(&pair[qt]);
             if (!wait_for(&pair[qt], 0)) { ok = false; break; }
-            mx = max_nan(mx, row_x[(hf ^ 1) * kRows + row]);
+#pragma unroll
+            for (int i = 1; i < RT; ++i) mx = max_nan(mx, row_x[(hf ^ i) * kRows + row]);
             const float m_new = max_nan(m_run, mx);
             const float base = m_new == -CUDART_INF_F ? 0.f : m_new, corr = m_run == -CUDART_INF_F ? 0.f : ex2(m_run - base);
-            float2 sum = make_float2(0.f, 0.f);
             const float2 nb = make_float2(-base, -base);
 #pragma unroll
-            for (int e = 0; e < 32; e += 2) {
-                const float2 a = add2(make_float2(s[e], s[e + 1]), nb);
-                s[e] = ex2(a.x);
-                s[e + 1] = ex2(a.y);
-                sum = add2(sum, make_float2(s[e], s[e + 1]));
+            for (int c = 0; c < LP; ++c) {
+                float2 sum = make_float2(0.f, 0.f);
+#pragma unroll
+                for (int e = 16 * c; e < 16 * c + 16; e += 2) {
+                    const float2 a = add2(make_float2(s[e], s[e + 1]), nb);
+                    s[e] = ex2(a.x);
+                    s[e + 1] = ex2(a.y);
+                    sum = add2(sum, make_float2(s[e], s[e + 1]));
+                }
+                l_run[c] = fmaf(l_run[c], corr, sum.x + sum.y);
             }
-            l_run = fmaf(l_run, corr, sum.x + sum.y);
             m_run = m_new;
             // weight x its value's magnitude, and the largest of them that this row has in the tile
-            if (!geo.shared_kv && !wait_for(&v_ready[t % geo.depth], (t / geo.depth) & 1u)) { ok = false; break; }
-            scale_by<32>(s, v_inv + (t % geo.depth) * kKeys + hf * 32);
+            if (!geo.shared_kv && !wait_for(&v_ready[at_t], round)) { ok = false; break; }
+            scale_by<KP>(s, v_inv + at_t * kKeys + hf * KP);
             auto largest = [&] {
                 float v = s[0];
 #pragma unroll
-                for (int e = 1; e < 32; ++e) v = max_nan(v, s[e]);
+                for (int e = 1; e < KP; ++e) v = max_nan(v, s[e]);
                 return v;
             };
             float wm = largest();
             if (__any_sync(0xffffffffu, wm != wm)) {          // a value that cannot be split, 0 x NaN where it is not seen
                 hide(0.f);
                 wm = largest();
-                if (wm != wm) l_run = CUDART_NAN_F;
+                if (wm != wm) l_run[0] = CUDART_NAN_F;
             }
-            row_x[(2 + hf) * kRows + row] = wm;
+            row_x[(RT + hf) * kRows + row] = wm;
             __syncwarp();
             if (lane == 0) mbar_arrive(&pair[qt]);
             // (meanwhile) the value product of the tile before is done: the weights' columns are free, and its sum can be taken
@@ -856,18 +883,20 @@ split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_co
             }
             if (!wait_for(&pair[qt], 1)) { ok = false; break; }
             float wi;
-            const float wscale = scale_of(fmaxf(wm, row_x[(2 + (hf ^ 1)) * kRows + row]), wi);
+#pragma unroll
+            for (int i = 1; i < RT; ++i) wm = fmaxf(wm, row_x[(RT + (hf ^ i)) * kRows + row]);
+            const float wscale = scale_of(wm, wi);
             const float2 ws = make_float2(wscale, wscale);
 #pragma unroll
-            for (int c = 0; c < 2; ++c) {
+            for (int c = 0; c < KP / 16; ++c) {
                 uint32_t hi[8], lo[8];
 #pragma unroll
                 for (int e = 0; e < 8; ++e) {
                     const float2 q = mul2(make_float2(s[c * 16 + 2 * e], s[c * 16 + 2 * e + 1]), ws);
                     split2(q.x, q.y, hi[e], lo[e]);
                 }
-                tmem_store8(t_p + lanes + hf * 16 + c * 8, hi);
-                tmem_store8(t_p + lanes + 32 + hf * 16 + c * 8, lo);
+                tmem_store8(t_p + lanes + hf * (KP / 2) + c * 8, hi);
+                tmem_store8(t_p + lanes + 32 + hf * (KP / 2) + c * 8, lo);
             }
             // with two accumulators the next value product may start before the last one has been added
             if (t > 0 && geo.o_bufs == 1) add_values(t - 1, corr_prev, wi_prev);
@@ -878,18 +907,23 @@ split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_co
             if (t > 0 && geo.o_bufs == 2) add_values(t - 1, corr_prev, wi_prev);
             corr_prev = corr;
             wi_prev = wi;
+            if (++at_t == (unsigned)geo.depth) at_t = 0, round ^= 1u;
         }
         if (ok && t > 0) {
             ok = wait_for(pv_done, (t - 1) & 1u);
             fence_after();
             add_values(t - 1, corr_prev, wi_prev);
         }
-        // ---- both threads' denominators, the sink's own term, normalise, store ----
-        row_x[hf * kRows + row] = l_run;
+        // ---- the threads' denominators, the sink's own term, normalise, store ----
+        // (with two threads they fill the place of the second exchange too: every thread has left it before the last value product)
+#pragma unroll
+        for (int c = 0; c < LP; ++c) row_x[(hf * LP + c) * kRows + row] = l_run[c];
         __syncwarp();
         if (lane == 0) mbar_arrive(&pair[qt]);
         ok = ok && wait_for(&pair[qt], 0);
-        float l = l_run + row_x[(hf ^ 1) * kRows + row];
+        float l = 0.f;
+#pragma unroll
+        for (int i = 0; i < RT * LP; ++i) l += row_x[i * kRows + row];
         if (p.sink) l += ex2(fmaf(p.sink[h], kLog2e, m_run == -CUDART_INF_F ? 0.f : -m_run));
         // through shared memory (the ring and the queries are read; 32 rows of this warp's channels): whole lines reach the output, and
         // one rolled loop serves every kind of output.  (Stored from the registers, row by row, 5500 cycles of a CTA, mostly fetching
@@ -901,14 +935,14 @@ split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_co
             *reinterpret_cast<volatile int*>(geo.ran_out) = 1;
             __threadfence_system();
         }
-        const int c0 = NVS == 1 ? hf * half : hf * 128, ldst = half + 4;
+        const int ldst = share + 4;
         float* stage = reinterpret_cast<float*>(smem) + (size_t)warp * 32 * ldst;
 #pragma unroll
         for (int c = 0; c < DVH; c += 4)
             if (c < n_mine) *reinterpret_cast<float4*>(stage + lane * ldst + c) = make_float4(O[c] * f, O[c + 1] * f, O[c + 2] * f, O[c + 3] * f);
         __syncwarp();
-        const int w4 = min(n_mine, p.vdim - c0) >> 2;         // (vdim is a multiple of 4)
-        for (unsigned again = __ballot_sync(0xffffffffu, ok && tok < n_tok && l != l); again; again &= again - 1) {
+        const int w4 = max(0, min(n_mine, p.vdim - c0)) >> 2; // (vdim is a multiple of 4)
+        for (unsigned again = __ballot_sync(0xffffffffu, ok && tok < n_tok && l != l && w4 > 0); again; again &= again - 1) {
             const int r = __ffs(again) - 1, rw = qt * 32 + r, tk = rw >> geo.pk_shift;
             plain_row(p, r0 + tk, s_slot[tk], s_pos[tk], h0 + (rw & (PK - 1)), c0, 4 * w4, stage + r * ldst);
         }
@@ -937,10 +971,10 @@ split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_co
             sc += 32;
             while (sc >= w4) { sc -= w4; ++sr; }
         }
-    } else if (warp < 12) {
+    } else if (warp < RW + 4) {
         // ================= keys and values: warp lw takes keys 16 lw .. + 15 of a tile, a lane one key of either eight =================
-        if constexpr (kFetchRegs < 128) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kFetchRegs));
-        const int lw = warp - 8, kin = lane & 7, cq = lane >> 3;
+        if constexpr (kFetchRegs < kLaunchRegs) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kFetchRegs));
+        const int lw = warp - RW, kin = lane & 7, cq = lane >> 3;
         unsigned at = 0;                                      // ring position
         bool ok = true;
         size_t cur[2] = {~(size_t)0, ~(size_t)0}, prev[2];    // row of the two keys in the pages of kv head 0 (~0: none)
@@ -988,71 +1022,77 @@ split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_co
         // (first) or as taken by the first group; inv: where the scales go (null: they are there); ready: told when they are
         auto stage = [&](const float* cache, int width, int row_w, int c0, int w, int wp, int gg, const size_t (&rows)[2], float (&m_row)[2],
                          bool first, float* inv, uint64_t* ready) {
-            float4 v[16];
-#pragma unroll
-            for (int kg = 0; kg < 2; ++kg) {
-                const bool in = rows[kg] != ~(size_t)0;
-                const float* src = row_of(cache, width, gg, rows[kg]) + c0;
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const int c = 8 * (cq + 4 * i);
-                    const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
-                    v[kg * 8 + 2 * i] = in && c < w ? *reinterpret_cast<const float4*>(src + c) : z;
-                    v[kg * 8 + 2 * i + 1] = in && c + 4 < w ? *reinterpret_cast<const float4*>(src + c + 4) : z;
-                }
-            }
-            if (first) {
-#pragma unroll
-                for (int kg = 0; kg < 2; ++kg) {
-                    float m = 0.f;
-#pragma unroll
-                    for (int i = 0; i < 8; ++i) m = max_abs4(m, v[kg * 8 + i]);
-                    if (w < row_w && rows[kg] != ~(size_t)0)
-                        for (int c = w + 4 * cq; c < row_w; c += 16)
-                            m = max_abs4(m, *reinterpret_cast<const float4*>(row_of(cache, width, gg, rows[kg]) + c));
-                    m_row[kg] = row_max(m);
-                }
-            }
-            float sc[2], inverse[2];
-#pragma unroll
-            for (int kg = 0; kg < 2; ++kg)
-                if (scale_row(m_row[kg], sc[kg], inverse[kg])) {
-#pragma unroll
-                    for (int i = 0; i < 8; ++i) v[kg * 8 + i] = make_float4(0.f, 0.f, 0.f, 0.f);
-                }
-            auto put_scales = [&] {
-                if (inv && lane < 8) {
-#pragma unroll
-                    for (int kg = 0; kg < 2; ++kg) inv[lw * 16 + kg * 8 + lane] = inverse[kg];
-                }
-            };
-            if (ready) {                                      // (their place is free by then: see geometry_of)
-                put_scales();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(ready);
-            }
+            constexpr int KG = RT == 4 ? 1 : 2;               // groups of eight keys at a time (16 float4 of two do not fit 64 registers)
             const unsigned slot = at % geo.n_slots;
-            if (!wait_for(&empty[slot], ((at / geo.n_slots) & 1u) ^ 1u)) { ok = false; return; }
-            if (!ready) put_scales();
-            unsigned char* base = ring + (size_t)slot * geo.slot_bytes;
-            const int blocks = wp >> 3;
+#pragma unroll 1
+            for (int half = 0; half < 2; half += KG) {
+                float4 v[8 * KG];
 #pragma unroll
-            for (int kg = 0; kg < 2; ++kg)
+                for (int u = 0; u < KG; ++u) {
+                    const size_t at_row = half + u ? rows[1] : rows[0];
+                    const bool in = at_row != ~(size_t)0;
+                    const float* src = row_of(cache, width, gg, at_row) + c0;
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const int c8 = cq + 4 * i;
-                    if (c8 < blocks) {
-                        const float4 a = v[kg * 8 + 2 * i], b = v[kg * 8 + 2 * i + 1];
-                        uint32_t hi[4], lo[4];
-                        split2(a.x * sc[kg], a.y * sc[kg], hi[0], lo[0]);
-                        split2(a.z * sc[kg], a.w * sc[kg], hi[1], lo[1]);
-                        split2(b.x * sc[kg], b.y * sc[kg], hi[2], lo[2]);
-                        split2(b.z * sc[kg], b.w * sc[kg], hi[3], lo[3]);
-                        unsigned char* dst = base + ((lw * 2 + kg) * blocks + c8) * 128 + kin * 16;
-                        *reinterpret_cast<uint4*>(dst) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-                        *reinterpret_cast<uint4*>(dst + kKeys * wp * 2) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+                    for (int i = 0; i < 4; ++i) {
+                        const int c = 8 * (cq + 4 * i);
+                        const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
+                        v[u * 8 + 2 * i] = in && c < w ? *reinterpret_cast<const float4*>(src + c) : z;
+                        v[u * 8 + 2 * i + 1] = in && c + 4 < w ? *reinterpret_cast<const float4*>(src + c + 4) : z;
                     }
                 }
+                float sc[KG], inverse[KG];
+#pragma unroll
+                for (int u = 0; u < KG; ++u) {
+                    float m = half + u ? m_row[1] : m_row[0];
+                    if (first) {
+                        const size_t at_row = half + u ? rows[1] : rows[0];
+                        m = 0.f;
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) m = max_abs4(m, v[u * 8 + i]);
+                        if (w < row_w && at_row != ~(size_t)0)
+                            for (int c = w + 4 * cq; c < row_w; c += 16) m = max_abs4(m, *reinterpret_cast<const float4*>(row_of(cache, width, gg, at_row) + c));
+                        m = row_max(m);
+                        if (half + u) m_row[1] = m;
+                        else m_row[0] = m;
+                    }
+                    if (scale_row(m, sc[u], inverse[u])) {
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) v[u * 8 + i] = make_float4(0.f, 0.f, 0.f, 0.f);
+                    }
+                }
+                auto put_scales = [&] {
+                    if (inv && lane < 8) {
+#pragma unroll
+                        for (int u = 0; u < KG; ++u) inv[lw * 16 + (half + u) * 8 + lane] = inverse[u];
+                    }
+                };
+                if (ready) {                                  // (their place is free by then: see geometry_of)
+                    put_scales();
+                    __syncwarp();
+                    if (half + KG == 2 && lane == 0) mbar_arrive(ready);
+                }
+                if (half == 0 && !wait_for(&empty[slot], ((at / geo.n_slots) & 1u) ^ 1u)) { ok = false; return; }
+                if (!ready) put_scales();
+                unsigned char* base = ring + (size_t)slot * geo.slot_bytes;
+                const int blocks = wp >> 3;
+#pragma unroll
+                for (int u = 0; u < KG; ++u)
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const int c8 = cq + 4 * i;
+                        if (c8 < blocks) {
+                            const float4 a = v[u * 8 + 2 * i], b = v[u * 8 + 2 * i + 1];
+                            uint32_t hi[4], lo[4];
+                            split2(a.x * sc[u], a.y * sc[u], hi[0], lo[0]);
+                            split2(a.z * sc[u], a.w * sc[u], hi[1], lo[1]);
+                            split2(b.x * sc[u], b.y * sc[u], hi[2], lo[2]);
+                            split2(b.z * sc[u], b.w * sc[u], hi[3], lo[3]);
+                            unsigned char* dst = base + ((lw * 2 + half + u) * blocks + c8) * 128 + kin * 16;
+                            *reinterpret_cast<uint4*>(dst) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+                            *reinterpret_cast<uint4*>(dst + kKeys * wp * 2) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+                        }
+                    }
+            }
             fence_smem_async();
             __syncwarp();
             if (lane == 0) mbar_arrive(&full[slot]);
@@ -1105,7 +1145,7 @@ split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_co
         if (t > 0 && ok) values(t - 1, cur, tile, m_key);
     } else {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 32;");
-        if (warp == 12) {
+        if (warp == RW + 4) {
             // ================= the MMA issuer: the whole warp walks, one elected lane issues =================
             const uint32_t idesc_s = (1u << 4) | ((uint32_t)(kKeys >> 3) << 17) | ((uint32_t)(kRows >> 4) << 24);
             const uint32_t q_addr = smem_u32(qs), ring_addr = smem_u32(ring);
@@ -1169,13 +1209,14 @@ split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_co
     }
     fence_before();
     __syncthreads();
-    if (warp == 12) {
+    if (warp == RW + 4) {
         fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem));
     }
 }
 
-bool geometry_of(const SplitAttention& a, Geometry& g, size_t& smem) {
+// with rt threads per row
+bool geometry_of(const SplitAttention& a, Geometry& g, size_t& smem, int rt) {
     if (a.heads <= 0 || a.kv_heads <= 0 || a.heads % a.kv_heads || a.kdim <= 0 || a.vdim <= 0) return false;
     auto mul4 = [](int v) { return v % 4 == 0; };
     auto aligned = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
@@ -1229,31 +1270,31 @@ bool geometry_of(const SplitAttention& a, Geometry& g, size_t& smem) {
     const int per_tile = g.n_kst + g.n_vst;
     auto depth_of = [&](int slots) { return 1 + (slots + g.n_kst + per_tile - 1) / per_tile; };
     auto control_of = [&](int slots) {
-        return (2 * kMaxSlots + 5 + 4 + kMaxDepth + 1) / 2 * 16 + (depth_of(slots) * kKeys * (g.k_sets + (g.shared_kv ? 0 : 1)) + 4 * kRows + 8) * 4 + 2 * (kRows >> g.pk_shift) * 4;
+        return (2 * kMaxSlots + 5 + 4 + kMaxDepth + 1) / 2 * 16 + (depth_of(slots) * kKeys * (g.k_sets + (g.shared_kv ? 0 : 1)) + 2 * rt * kRows + 8) * 4 + 2 * (kRows >> g.pk_shift) * 4;
     };
     for (g.n_slots = kMaxSlots; g.n_slots >= 2; --g.n_slots)
         if (g.n_slots * g.slot_bytes + g.q_bytes + control_of(g.n_slots) <= kSmemMost) break;
     if (g.n_slots < 2) return false;
     g.depth = depth_of(g.n_slots);
     const int control = control_of(g.n_slots);
-    // the output is staged in the ring and the queries: 8 warps of 32 rows, 4 floats between the rows
-    const int staged = kRows * 2 * (g.n_vst == 1 ? g.wv0 / 2 + 4 : 128 + 4) * 4;
+    // the output is staged in the ring and the queries: 4 rt warps of 32 rows, 4 floats between the rows
+    const int staged = kRows * rt * ((g.n_vst == 1 ? (g.wv0 + 8 * rt - 1) / (8 * rt) * 8 : 256 / rt) + 4) * 4;
     g.q_bytes = std::max(g.q_bytes, staged - g.n_slots * g.slot_bytes);
     smem = (size_t)g.n_slots * g.slot_bytes + g.q_bytes + control;
     return smem <= (size_t)kSmemMost;
 }
 
-template <int NVS>
+template <int NVS, int RT>
 cudaError_t launch_inst(const SplitAttention& a, const Geometry& g, size_t smem, cudaStream_t st) {
     // (the same size for every launch: another thread's cannot lower what this one needs)
-    const cudaError_t e = cudaFuncSetAttribute(split_attention_kernel<NVS>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMost);
+    const cudaError_t e = cudaFuncSetAttribute(split_attention_kernel<NVS, RT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMost);
     if (e != cudaSuccess) return e;
     const int tt = kRows >> g.pk_shift, tiles = a.n_seq > 1 ? a.M / tt + a.n_seq : (a.M + tt - 1) / tt;
     if (a.work) {
         split_keys_kernel<<<dim3(std::min(g.cap_tiles, std::max(1, kSplitGrid / g.parts)), g.parts), 256, 0, st>>>(a, g);
         ++extra_launches();
     }
-    split_attention_kernel<NVS><<<(a.heads >> g.pk_shift) * tiles, kSplitThreadsTC, smem, st>>>(a, g);
+    split_attention_kernel<NVS, RT><<<(a.heads >> g.pk_shift) * tiles, kSplitThreads<RT>, smem, st>>>(a, g);
     return cudaGetLastError();
 }
 
@@ -1282,20 +1323,20 @@ int* split_attention_ran_out(int device, cudaStream_t st) {
 bool split_attention_ok(const SplitAttention& a) {
     Geometry g;
     size_t smem;
-    return geometry_of(a, g, smem);
+    return geometry_of(a, g, smem, 2);
 }
 
 size_t split_attention_work_bytes(const SplitAttention& a, int keys) {
     Geometry g;
     size_t smem;
-    if (!geometry_of(a, g, smem)) return 0;
+    if (!geometry_of(a, g, smem, 2)) return 0;
     return (size_t)a.n_slots * sizeof(SlotTiles) + 256 + (size_t)((keys + kKeys - 1) / kKeys) * (g.tile_bytes + 4u * kKeys * g.sets);
 }
 
 cudaError_t launch_split_attention(const SplitAttention& a, cudaStream_t st) {
     Geometry g;
     size_t smem;
-    if (a.M <= 0 || !geometry_of(a, g, smem)) return cudaErrorNotSupported;
+    if (a.M <= 0 || !geometry_of(a, g, smem, 2)) return cudaErrorNotSupported;
     int device = 0;
     const cudaError_t e = cudaGetDevice(&device);
     if (e != cudaSuccess) return e;
@@ -1309,7 +1350,17 @@ cudaError_t launch_split_attention(const SplitAttention& a, cudaStream_t st) {
     // cached keys, latent rows of 256 + 32, 4 layers: 1714 and 1833 us split by the row tiles, 1139 and 1250 in advance; over 100 keys 867
     // and 863)
     if (g.cap_tiles <= 0 || (g.n_vst == 1 && (long long)a.M * (a.heads / a.kv_heads) < kSplitOnceRows)) with.work = nullptr;
-    return g.n_vst == 1 ? launch_inst<1>(with, g, smem, st) : launch_inst<2>(with, g, smem, st);
+    if (g.n_vst == 2) return launch_inst<2, 2>(with, g, smem, st);
+    // Four threads per row where the keys are split in advance (us, two / four: windowed 4096 rows, 16 heads of 128 over 4 266 / 245, mixed
+    // scores, three prompts of 2048 rows 147 / 117, 4096 rows in chunks of 2048 303 / 263, float32 model 80 / 63).  Their fetching warps have half
+    // the registers (861 rows of Dia, whose keys every row tile splits for itself, 81 / 107); wide values do not fit theirs (451 / 459).
+    Geometry g4;
+    size_t smem4;
+    if (with.work && geometry_of(a, g4, smem4, 4)) {
+        g4.ran_out = g.ran_out;
+        return launch_inst<1, 4>(with, g4, smem4, st);
+    }
+    return launch_inst<1, 2>(with, g, smem, st);
 }
 
 }  // namespace dia
