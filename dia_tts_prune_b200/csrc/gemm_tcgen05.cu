@@ -850,8 +850,9 @@ __device__ __forceinline__ float4 load_remote4(const float* local, uint32_t rank
 // in their registers while the next k-blocks are multiplied into the three other accumulators.  128 x 128 tiles: a thread holds
 // 128 sums.  Bound: 12 MMAs of 64 cycles per k-block against ~300 issue slots of draining it.  Where the tiles leave most of the chip
 // idle, a cluster of gridDim.y CTAs shares a tile: each takes a range of k-blocks, and the sums meet in shared memory.
-constexpr int kFN = 128, kFASlots = 6, kFBSlots = 3, kFStride = kFN + 4;
-constexpr int kFStage = 4 * 32 * kFStride * 4;                // 32 rows of sums per epilogue warp
+constexpr int kFN = 128, kFASlots = 6, kFBSlots = 3;
+constexpr int kFWarps = 8, kFThreads = 64 + 32 * kFWarps, kFCols = kFN / 2, kFStride = kFCols + 4;      // epilogue warps, columns of one
+constexpr int kFStage = kFWarps * 32 * kFStride * 4;          // 32 rows of sums per epilogue warp
 constexpr int kFBars = 2 * kFASlots + 2 * kFBSlots + 8;
 constexpr int kFSmem = (kFASlots + kFBSlots) * kTileBytes + kFStage + 1024 + 256;
 static_assert(kFBars * 8 + 8 <= 256, "barrier region");
@@ -863,7 +864,7 @@ __device__ __noinline__ float f32_act(int act, float z) {
 
 // TERMS: terms of A (3: fp32 rows, 1: bf16 rows)
 template <int TERMS>
-__global__ void __launch_bounds__(kGemmThreads, 1)
+__global__ void __launch_bounds__(kFThreads, 1)
 dia_gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const __grid_constant__ F32Product p) {
     const int M = p.M, N = p.N, K = p.K;
     extern __shared__ unsigned char smem_raw[];
@@ -883,21 +884,21 @@ dia_gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     const int S = gridDim.y, kb_all = (K + BK - 1) / BK, kb_per = (kb_all + S - 1) / S, kb0 = blockIdx.y * kb_per;
     const int n_kb = max(0, min(kb_per, kb_all - kb0));
     const int tiles_m = (M + BM - 1) / BM, tiles_n = (N + kFN - 1) / kFN, n_tiles = tiles_m * tiles_n * p.heads;
-    // an epilogue warp's 32 rows of sums, from row r0 on every S-th, four columns per lane
+    // an epilogue warp's 32 rows of sums, from rows 2 r0 and 2 r0 + 1 on every S-th pair, four columns per lane
     float* const tile = stage + (warp - 2) * 32 * kFStride;
     auto emit = [&](int t, int r0) {
         const int q = warp & 3, hn = t / tiles_m, h = hn / tiles_n, n0 = (hn - h * tiles_n) * kFN, m0 = (t % tiles_m) * BM;
-        const int rows = min(32, M - (m0 + q * 32)), n = n0 + 4 * lane;
+        const int rows = min(32, M - (m0 + q * 32)), c4 = 4 * (lane & 15), n = n0 + ((warp - 2) >> 2) * kFCols + c4;
         if (n >= N) return;
         const size_t m = (size_t)(m0 + q * 32), col = (size_t)h * p.y_hs + n;
         const float* gate = p.gate ? p.gate + m * p.ldg + (p.head_gate ? (size_t)h : (size_t)h * N + n) : nullptr;
 #pragma unroll 1
-        for (int r = r0; r < rows; r += S) {
-            float4 v = *reinterpret_cast<const float4*>(tile + r * kFStride + 4 * lane);
+        for (int r = 2 * r0 + (lane >> 4); r < rows; r += 2 * S) {
+            float4 v = *reinterpret_cast<const float4*>(tile + r * kFStride + c4);
             if (S > 1) {
                 float4 u[8];
 #pragma unroll
-                for (int c = 0; c < 8; ++c) if (c < S) u[c] = load_remote4(tile + r * kFStride + 4 * lane, c);
+                for (int c = 0; c < 8; ++c) if (c < S) u[c] = load_remote4(tile + r * kFStride + c4, c);
                 v = u[0];
 #pragma unroll
                 for (int c = 1; c < 8; ++c) if (c < S) { v.x += u[c].x; v.y += u[c].y; v.z += u[c].z; v.w += u[c].w; }
@@ -936,7 +937,7 @@ dia_gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     if (threadIdx.x == 0) {
         for (int i = 0; i < kFASlots; ++i) { mbar_init(&a_full[i], 1); mbar_init(&a_empty[i], 1); }
         for (int i = 0; i < kFBSlots; ++i) { mbar_init(&b_full[i], 1); mbar_init(&b_empty[i], 1); }
-        for (int i = 0; i < 4; ++i) { mbar_init(&t_full[i], 1); mbar_init(&t_empty[i], 4); }
+        for (int i = 0; i < 4; ++i) { mbar_init(&t_full[i], 1); mbar_init(&t_empty[i], kFWarps); }
         fence_mbar_init();
     }
     if (warp == 1) {
@@ -1003,17 +1004,17 @@ dia_gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         const int q = warp & 3;
         unsigned it = 0;
         for (int t = blockIdx.x; t < n_tiles; t += gridDim.x) {
-            float sum[kFN];
+            float sum[kFCols];
 #pragma unroll
-            for (int c = 0; c < kFN; ++c) sum[c] = 0.f;
+            for (int c = 0; c < kFCols; ++c) sum[c] = 0.f;
             for (int kb = 0; kb < n_kb; ++kb, ++it) {
                 const unsigned acc = it & 3u;
                 mbar_wait_bounded(&t_full[acc], (it >> 2) & 1u);
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
-                for (int cb = 0; cb < kFN / 32; ++cb) {
+                for (int cb = 0; cb < kFCols / 32; ++cb) {
                     uint32_t v[32];
-                    const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + acc * kFN + cb * 32;
+                    const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + acc * kFN + ((warp - 2) >> 2) * kFCols + cb * 32;
                     asm volatile(
                         "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
                         "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
@@ -1036,7 +1037,7 @@ dia_gemm_f32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             // unrolled one (128 copies of the epilogue) was bound by instruction fetches.
             __syncwarp();
 #pragma unroll
-            for (int c = 0; c < kFN; c += 4)
+            for (int c = 0; c < kFCols; c += 4)
                 *reinterpret_cast<float4*>(tile + lane * kFStride + c) = make_float4(sum[c], sum[c + 1], sum[c + 2], sum[c + 3]);
             __syncwarp();
             if (S == 1) emit(t, 0);
@@ -1425,7 +1426,7 @@ static cudaError_t run_gemm_f32(const F32Product& p, const void* a_terms, int te
     const int s = f32_splits(n_tiles, n_kb, splits, sms);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(s > 1 ? n_tiles : std::min(n_tiles, sms), s);
-    cfg.blockDim = dim3(kGemmThreads);
+    cfg.blockDim = dim3(kFThreads);
     cfg.dynamicSmemBytes = kFSmem;
     cfg.stream = st;
     cudaLaunchAttribute attr;
