@@ -40,6 +40,18 @@ class GenStatus(C.Structure):
                                          "steps_run", "device_error", "reserved")]
 
 
+class DenseRef(C.Structure):
+    _fields_ = [(n, C.c_void_p) for n in ("wt_bf16", "wt_half", "magnitudes")]
+
+
+class RowsLayer(C.Structure):
+    _fields_ = [(n, C.c_int32) for n in ("B", "T", "D", "F", "heads", "kv_heads", "slots", "mode", "cross_heads", "cross_slots", "n_pos")] + \
+               [("eps", C.c_float), ("n_valid", C.c_int32 * 16), ("cross_valid", C.c_int32 * 16)] + \
+               [(n, C.c_void_p) for n in ("x_in", "x", "sin_table", "cos_table", "positions", "norm_self", "norm_cross", "norm_mlp")] + \
+               [(n, DenseRef) for n in ("q", "k", "v", "o", "cross_q", "cross_o", "wi", "wo")] + \
+               [(n, C.c_void_p) for n in ("k_cache", "v_cache", "cross_k", "cross_v", "work")]
+
+
 _vp, _i, _i32p, _fp = C.c_void_p, C.c_int, C.c_void_p, C.c_void_p
 _SIGNATURES = {
     "dia_b200_abi_version": (C.c_int, []),
@@ -82,6 +94,8 @@ _SIGNATURES = {
     "dia_b200_dense_half_rows": (_i, [_i, _i, _i]),
     "dia_b200_dense_prepare_half": (_i, [_vp, _i, _vp, _fp, _i32p, _i, _i, _vp]),
     "dia_b200_dense_forward_half": (_i, [_fp, _fp, C.c_float, _i, _vp, _fp, _fp, _fp, _vp, _i, _i, _i, _vp]),
+    "dia_b200_rows_layer_work_bytes": (C.c_size_t, [C.POINTER(RowsLayer)]),
+    "dia_b200_rows_layer_forward": (_i, [C.POINTER(RowsLayer), _vp]),
     "dia_b200_attention_rows": (_i, [_fp, _fp, _fp, _fp, _i, _i, _i, _i, _i, _i, _i, C.POINTER(C.c_int32), _vp]),
     "dia_b200_rope_rows": (_i, [_fp, _fp, _fp, _fp, _i32p, _i, _i, _i, _i, _i, _i, _i, _i, _vp]),
     "dia_b200_rmsnorm_rows": (_i, [_fp, _fp, C.c_float, _fp, _i, _i, _vp]),

@@ -994,7 +994,7 @@ int dia_b200_dense_forward_fused(const float* x, const float* norm_weight, float
     if ((reinterpret_cast<uintptr_t>(wt_bf16) | reinterpret_cast<uintptr_t>(workspace) | reinterpret_cast<uintptr_t>(y) |
          reinterpret_cast<uintptr_t>(residual)) & 15)
         return DIA_B200_EINVAL;
-    cudaError_t e = launch_gemm_tcgen05(x, norm_weight, eps, wt_bf16, residual, y, workspace, M, N, K, S(stream));
+    cudaError_t e = launch_gemm_tcgen05(x, norm_weight, eps, false, wt_bf16, residual, y, workspace, M, N, K, S(stream));
     if (e == cudaErrorNotSupported) { (void)cudaGetLastError(); return DIA_B200_EUNSUPPORTED; }
     CK(e);
     g_launches += 1 + std::exchange(extra_launches(), 0);
@@ -1044,6 +1044,103 @@ int dia_b200_attention_rows(const float* q, const float* k, const float* v, floa
     CK(launch_attention_rows(q, k, v, out, B, Tq, Tk, Hq, Hkv, Tk_stride, mode, n_valid_host, S(stream)));
     g_launches++;
     return DIA_B200_OK;
+}
+
+namespace {
+
+// What a layer of many rows keeps in its workspace: [q | k | v] rows, turned queries and attention output share the room of the gated unit's rows.
+struct RowsRoom { size_t qkv, q, att, gu, split, bytes; };
+RowsRoom rows_room(const dia_b200_rows_layer& a) {
+    const size_t M = (size_t)a.B * a.T, most = std::max({(size_t)a.D, (size_t)a.heads * 128, (size_t)a.cross_heads * 128, (size_t)a.F});
+    const size_t heads = std::max(a.heads, a.cross_heads);
+    RowsRoom r;
+    r.qkv = 0;
+    r.q = r.qkv + M * (size_t)std::max(a.heads + 2 * a.kv_heads, a.cross_heads) * 512;
+    r.att = r.q + M * heads * 512;
+    r.gu = 0;
+    r.split = std::max(r.att + M * heads * 512, M * 8 * (size_t)a.F);
+    r.bytes = r.split + gemm_workspace_bytes((int)M, (int)most);
+    return r;
+}
+
+int rows_dense(const dia_b200_dense_ref& w, const float* x, const float* norm, float eps, bool gated, const float* residual, float* y, void* work,
+               int M, int N, int K, cudaStream_t st) {
+    const cudaError_t e = w.wt_half ? launch_gemm_half(x, norm, eps, gated, w.wt_half, w.magnitudes, residual, y, work, M, N, K, st)
+                                    : launch_gemm_tcgen05(x, norm, eps, gated, w.wt_bf16, residual, y, work, M, N, K, st);
+    if (e == cudaErrorNotSupported) { (void)cudaGetLastError(); return DIA_B200_EUNSUPPORTED; }
+    CK(e);
+    g_launches += 1 + std::exchange(extra_launches(), 0);
+    return DIA_B200_OK;
+}
+
+int rows_attention(const float* q, const float* k, const float* v, float* out, int B, int Tq, int Tk, int Hq, int Hkv, int slots, int mode,
+                   const int32_t* n_valid, cudaStream_t st) {
+    CK(launch_attention_rows(q, k, v, out, B, Tq, Tk, Hq, Hkv, slots, mode, n_valid, st));
+    g_launches += 1 + std::exchange(extra_launches(), 0);
+    return DIA_B200_OK;
+}
+
+}  // namespace
+
+size_t dia_b200_rows_layer_work_bytes(const dia_b200_rows_layer* a) {
+    return a && a->B > 0 && a->T > 0 && a->D > 0 && a->heads > 0 && a->kv_heads > 0 && a->cross_heads >= 0 && a->F > 0 ? rows_room(*a).bytes : 0;
+}
+
+int dia_b200_rows_layer_forward(const dia_b200_rows_layer* args, void* stream) {
+    if (!args) return DIA_B200_EINVAL;
+    const dia_b200_rows_layer& a = *args;
+    if (a.B < 0 || a.B > 16 || a.T < 0 || a.D <= 0 || a.heads <= 0 || a.kv_heads <= 0 || a.heads % a.kv_heads || a.F <= 0 || a.mode < 0 || a.mode > 2 ||
+        a.T > a.slots || a.cross_heads < 0 || a.n_pos <= 0)
+        return DIA_B200_EINVAL;
+    if (a.B == 0 || a.T == 0) return DIA_B200_OK;
+    if (!a.x_in || !a.x || !a.sin_table || !a.cos_table || !a.positions || !a.k_cache || !a.v_cache || !a.work || !a.norm_self || !a.norm_mlp)
+        return DIA_B200_EINVAL;
+    const bool cross = a.cross_heads > 0;
+    if (cross && (!a.norm_cross || !a.cross_k || !a.cross_v || a.cross_slots <= 0)) return DIA_B200_EINVAL;
+    const dia_b200_dense_ref* const used[] = {&a.q, &a.k, &a.v, &a.o, &a.wi, &a.wo, &a.cross_q, &a.cross_o};
+    uintptr_t bits = 0;
+    for (int i = 0; i < (cross ? 8 : 6); ++i) {
+        if (used[i]->wt_half ? !used[i]->magnitudes : !used[i]->wt_bf16) return DIA_B200_EINVAL;
+        bits |= reinterpret_cast<uintptr_t>(used[i]->wt_half) | reinterpret_cast<uintptr_t>(used[i]->wt_bf16) | reinterpret_cast<uintptr_t>(used[i]->magnitudes);
+    }
+    for (const void* p : {(const void*)a.x_in, (const void*)a.x, (const void*)a.sin_table, (const void*)a.cos_table, (const void*)a.k_cache,
+                          (const void*)a.v_cache, (const void*)a.work, (const void*)a.cross_k, (const void*)a.cross_v})
+        bits |= reinterpret_cast<uintptr_t>(p);
+    if (bits & 15) return DIA_B200_EINVAL;
+    for (int b = 0; b < a.B; ++b)
+        if (a.n_valid[b] < 0 || a.n_valid[b] > a.T || (cross && (a.cross_valid[b] < 0 || a.cross_valid[b] > a.cross_slots))) return DIA_B200_EINVAL;
+    cudaStream_t st = S(stream);
+    const RowsRoom room = rows_room(a);
+    unsigned char* const work = static_cast<unsigned char*>(a.work);
+    float *qkv = reinterpret_cast<float*>(work + room.qkv), *q = reinterpret_cast<float*>(work + room.q), *att = reinterpret_cast<float*>(work + room.att),
+          *gu = reinterpret_cast<float*>(work + room.gu);
+    void* const split = work + room.split;
+    const int M = a.B * a.T, nq = a.heads * 128, nk = a.kv_heads * 128, D = a.D;
+    int rc;
+    // projections whose K-major copies lie one behind the other are one product
+    auto follows = [&](const dia_b200_dense_ref& u, const dia_b200_dense_ref& w, int n) {
+        return !u.wt_half && !w.wt_half && static_cast<const unsigned char*>(u.wt_bf16) + (size_t)n * D * 2 == w.wt_bf16;
+    };
+    const bool kv = follows(a.k, a.v, nk), all = kv && follows(a.q, a.k, nq);
+    float *k = all ? qkv + nq : qkv + (size_t)M * nq, *v = all || kv ? k + nk : k + (size_t)M * nk;
+    const int ldq = all ? nq + 2 * nk : nq, ldkv = all ? ldq : kv ? 2 * nk : nk;
+    if ((rc = rows_dense(a.q, a.x_in, a.norm_self, a.eps, false, nullptr, qkv, split, M, ldq, D, st))) return rc;
+    if (!all && (rc = rows_dense(a.k, a.x_in, a.norm_self, a.eps, false, nullptr, k, split, M, ldkv, D, st))) return rc;
+    if (!kv && (rc = rows_dense(a.v, a.x_in, a.norm_self, a.eps, false, nullptr, v, split, M, nk, D, st))) return rc;
+    CK(launch_head_rows(qkv, ldq, k, v, ldkv, q, a.k_cache, a.v_cache, a.sin_table, a.cos_table, a.positions, a.B, a.T, a.heads, a.kv_heads, a.slots, a.n_pos, st));
+    g_launches++;
+    if ((rc = rows_attention(q, a.k_cache, a.v_cache, att, a.B, a.T, a.T, a.heads, a.kv_heads, a.slots, a.mode, a.n_valid, st))) return rc;
+    if ((rc = rows_dense(a.o, att, nullptr, 0.f, false, a.x_in, a.x, split, M, D, nq, st))) return rc;
+    if (cross) {
+        const int nc = a.cross_heads * 128;
+        if ((rc = rows_dense(a.cross_q, a.x, a.norm_cross, a.eps, false, nullptr, qkv, split, M, nc, D, st))) return rc;
+        CK(launch_head_rows(qkv, nc, nullptr, nullptr, 0, q, nullptr, nullptr, a.sin_table, a.cos_table, a.positions, a.B, a.T, a.cross_heads, 0, 0, a.n_pos, st));
+        g_launches++;
+        if ((rc = rows_attention(q, a.cross_k, a.cross_v, att, a.B, a.T, a.cross_slots, a.cross_heads, a.cross_heads, a.cross_slots, 2, a.cross_valid, st))) return rc;
+        if ((rc = rows_dense(a.cross_o, att, nullptr, 0.f, false, a.x, a.x, split, M, D, nc, st))) return rc;
+    }
+    if ((rc = rows_dense(a.wi, a.x, a.norm_mlp, a.eps, false, nullptr, gu, split, M, 2 * a.F, D, st))) return rc;
+    return rows_dense(a.wo, gu, nullptr, 0.f, true, a.x, a.x, split, M, D, a.F, st);
 }
 
 int dia_b200_rope_rows(const float* src, float* dst, const float* sin_tab, const float* cos_tab, const int32_t* pos, int B,

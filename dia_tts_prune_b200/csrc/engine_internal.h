@@ -288,7 +288,7 @@ bool gemm_half_ok(int M, int N, int K);
 cudaError_t launch_prepare_half(const void* w, int src_bf16, void* wt, float* mag, int* inexact, int K, int N, cudaStream_t st);
 cudaError_t launch_gemm_half(const float* x, const float* norm_w, float eps, bool gated, const void* wt, const float* mag, const float* residual, float* y,
                              void* workspace, int M, int N, int K, cudaStream_t st);
-cudaError_t launch_gemm_tcgen05(const float* x, const float* norm_w, float eps, const void* wt, const float* residual,
+cudaError_t launch_gemm_tcgen05(const float* x, const float* norm_w, float eps, bool gated, const void* wt, const float* residual,
                                 float* y, void* workspace, int M, int N, int K, cudaStream_t st);
 
 // the rest of the T > 1 passes (prefill_kernels.cu)
@@ -296,6 +296,9 @@ cudaError_t launch_attention_rows(const float* q, const float* k, const float* v
                                   int Hkv, int Tk_stride, int mode, const int* n_valid_host, cudaStream_t st);
 cudaError_t launch_rope_rows(const float* src, float* dst, const float* sin_tab, const float* cos_tab, const int* pos, int B,
                              int T, int H, int rotate, int to_cache, int dst_T, int dst_t0, int n_pos, cudaStream_t st);
+cudaError_t launch_head_rows(const float* q, int ldq, const float* k, const float* v, int ldkv, float* q_out, float* k_cache, float* v_cache,
+                             const float* sin_tab, const float* cos_tab, const int* pos, int B, int T, int Hq, int Hkv, int slots, int n_pos,
+                             cudaStream_t st);
 cudaError_t launch_rmsnorm_rows(const float* x, const float* w, float eps, float* y, int M, int D, cudaStream_t st);
 cudaError_t launch_silu_mul(const float* gu, float* h, int M, int F, cudaStream_t st);
 cudaError_t launch_embed_rows(const float* table, const int* ids, float* out, int n_rows, int vocab, int D, cudaStream_t st);

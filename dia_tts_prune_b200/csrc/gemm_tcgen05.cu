@@ -120,44 +120,6 @@ __device__ __forceinline__ void split3_down(float v, __nv_bfloat16& t0, __nv_bfl
     t2 = __float2bfloat16_rn(r1 - __bfloat162float(t1));
 }
 
-// three terms per element, three stacked bf16 matrices [3][M][K]
-__global__ void split3_rows_kernel(const float* __restrict__ x, __nv_bfloat16* __restrict__ xs, long long n) {
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        split3(x[i], xs[i], xs[n + i], xs[2 * n + i]);
-    }
-}
-
-// the same with torch.nn.RMSNorm of the row fused in front (dia/layers.py:541,560,579,714: the norm that precedes
-// every projection): xs = split3((x * rsqrt(mean(x^2) + eps)) * w).  One CTA per row.
-// SPLIT: the normed rows' three terms; otherwise the normed rows themselves
-template <bool SPLIT>
-__global__ void __launch_bounds__(256) split3_norm_rows_kernel(const float* __restrict__ x, const float* __restrict__ w, float eps,
-                                                               void* __restrict__ out, int M, int K) {
-    __nv_bfloat16* xs = reinterpret_cast<__nv_bfloat16*>(out);
-    __shared__ float part[8];
-    const int row = blockIdx.x;
-    const float* xr = x + (size_t)row * K;
-    float ss = 0.f;
-    for (int i = threadIdx.x; i < K; i += 256) { const float v = xr[i]; ss = fmaf(v, v, ss); }
-    ss = warp_sum(ss);
-    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = ss;
-    __syncthreads();
-    float tot = 0.f;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) tot += part[i];
-    const float inv = 1.0f / sqrtf(tot / (float)K + eps);
-    const size_t n = (size_t)M * K;
-    for (int i = threadIdx.x; i < K; i += 256) {
-        const float v = (xr[i] * inv) * w[i];
-        if (!SPLIT) {
-            reinterpret_cast<float*>(out)[(size_t)row * K + i] = v;
-            continue;
-        }
-        const size_t o = (size_t)row * K + i;
-        split3(v, xs[o], xs[n + o], xs[2 * n + o]);
-    }
-}
-
 // W [K][N] (fp32 or bf16, N contiguous) -> Wt [N][K] bf16 (K contiguous)
 __global__ void transpose_to_bf16_kernel(const void* __restrict__ w, int src_bf16, __nv_bfloat16* __restrict__ wt, int K, int N) {
     __shared__ float tile[32][33];
@@ -220,22 +182,27 @@ __global__ void transpose_to_half_kernel(const void* __restrict__ w, int src_bf1
     }
 }
 
-// Rows as two fp16 terms, hi = fp16(v), lo = fp16(v - hi), each row times a power of two that brings its largest magnitude to [2^14, 2^15): a
-// value keeps 22 bits and more (a quarter of all fp32 numbers change by their last bit, the others not) down to 2^-17 of its row's largest, and
-// is off by at most 2^-39 of that below.  out: [2][M][K], then the rows' inverse scales [M].  A row with an infinity or a NaN gives nothing but
-// infinities and NaNs in its products: the other values are left out.  norm_w: RMSNorm of the row in front (dia/layers.py:541,560,579,714).
-// GATED: the row is silu(x[0 .. K)) x[K .. 2K) (dia/layers.py:95-101).  One CTA per row, which stays in registers up to 8192 channels.
-template <bool GATED>
-__global__ void __launch_bounds__(256) split2_rows_kernel(const float* __restrict__ x, const float* __restrict__ norm_w, float eps, __half* __restrict__ out,
-                                                          float* __restrict__ row_inv, int M, int K) {
+// Rows of a product's operand.  TERMS 3: three bf16 terms, stacked as [3][M][K]; 0: the rows themselves, in fp32; 2: two fp16 terms, hi =
+// fp16(v), lo = fp16(v - hi), each row times a power of two that brings its largest magnitude to [2^14, 2^15): a value keeps 22 bits and more (a
+// quarter of all fp32 numbers change by their last bit, the others not) down to 2^-17 of its row's largest, and is off by at most 2^-39 of
+// that below.  [2][M][K], and the rows' inverse scales [M] in row_inv.  A row with an infinity or a NaN gives nothing but infinities and
+// NaNs in its products: the other values are left out.  norm_w: RMSNorm of the row in front (dia/layers.py:541,560,579,714).
+// GATED: the row is silu(x[0 .. K)) x[K .. 2K) (dia/layers.py:95-101).  One CTA per row, which stays in registers up to 8192 channels
+// (1722 rows of 8192 gated channels: 51 us for the gate and 22 for the split, 42 together).
+template <int TERMS, bool GATED>
+__global__ void __launch_bounds__(256) split_rows_kernel(const float* __restrict__ x, const float* __restrict__ norm_w, float eps, void* __restrict__ out,
+                                                         float* __restrict__ row_inv, int M, int K, int aligned) {
     constexpr int kHeld = 8;
     __shared__ float part[8], most[8];
     const int tid = threadIdx.x, row = blockIdx.x, n4 = K >> 2;
-    const float4* xr = reinterpret_cast<const float4*>(x + (size_t)row * K * (GATED ? 2 : 1));
+    const float* xr = x + (size_t)row * K * (GATED ? 2 : 1);
+    auto four = [&](const float* p, int i) {
+        return aligned ? reinterpret_cast<const float4*>(p)[i] : make_float4(p[4 * i], p[4 * i + 1], p[4 * i + 2], p[4 * i + 3]);
+    };
     auto raw = [&](int i) {
-        float4 v = xr[i];
+        float4 v = four(xr, i);
         if (GATED) {
-            const float4 u = xr[n4 + i];
+            const float4 u = four(xr, n4 + i);
             v.x = v.x / (1.0f + expf(-v.x)) * u.x; v.y = v.y / (1.0f + expf(-v.y)) * u.y;
             v.z = v.z / (1.0f + expf(-v.z)) * u.z; v.w = v.w / (1.0f + expf(-v.w)) * u.w;
         }
@@ -263,9 +230,29 @@ __global__ void __launch_bounds__(256) split2_rows_kernel(const float* __restric
     }
     auto value = [&](const float4& v, int i) {
         if (!norm_w) return v;
-        const float4 w = reinterpret_cast<const float4*>(norm_w)[i];
+        const float4 w = four(norm_w, i);
         return make_float4((v.x * inv) * w.x, (v.y * inv) * w.y, (v.z * inv) * w.z, (v.w * inv) * w.w);
     };
+    const size_t plane = (size_t)M * K, at = (size_t)row * K;
+    if (TERMS != 2) {
+        auto put = [&](const float4& v, int i) {
+            if (TERMS == 0) {
+                reinterpret_cast<float4*>(reinterpret_cast<float*>(out) + at)[i] = v;
+                return;
+            }
+            __nv_bfloat16 t[3][4];
+            split3(v.x, t[0][0], t[1][0], t[2][0]); split3(v.y, t[0][1], t[1][1], t[2][1]);
+            split3(v.z, t[0][2], t[1][2], t[2][2]); split3(v.w, t[0][3], t[1][3], t[2][3]);
+#pragma unroll
+            for (int q = 0; q < 3; ++q)
+                *reinterpret_cast<uint2*>(reinterpret_cast<__nv_bfloat16*>(out) + q * plane + at + 4 * i) = *reinterpret_cast<const uint2*>(t[q]);
+        };
+#pragma unroll
+        for (int j = 0; j < kHeld; ++j)
+            if (j * 256 + tid < n4) put(value(held[j], j * 256 + tid), j * 256 + tid);
+        for (int i = kHeld * 256 + tid; i < n4; i += 256) put(value(raw(i), i), i);
+        return;
+    }
     uint32_t m = 0;                                           // magnitudes as bits: an infinity or a NaN is the largest
     auto see = [&](const float4& v) {
         m = max(max(max(m, __float_as_uint(v.x) & 0x7fffffffu), __float_as_uint(v.y) & 0x7fffffffu),
@@ -287,10 +274,9 @@ __global__ void __launch_bounds__(256) split2_rows_kernel(const float* __restric
     const int e = max((int)(m >> 23), 1) - 127, s = 14 - e, s1 = min(s, 100);       // the scale 2^s as 2^s1 2^(s - s1): s may be 140
     const float f1 = bad ? 1.f : __uint_as_float((uint32_t)(s1 + 127) << 23), f2 = bad ? 1.f : __uint_as_float((uint32_t)(s - s1 + 127) << 23);
     if (tid == 0) row_inv[row] = bad ? 1.f : ldexpf(1.f, -s);
-    const size_t plane = (size_t)M * K;
-    __half* hi_row = out + (size_t)row * K;
+    __half* const hi_row = reinterpret_cast<__half*>(out) + at;
     auto put = [&](const float4& v, int i) {
-        float a[4] = {v.x, v.y, v.z, v.w};
+        const float a[4] = {v.x, v.y, v.z, v.w};
         __half hi[4], lo[4];
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
@@ -502,7 +488,7 @@ dia_gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
 // three terms 256 / 209 (1.66 PFLOP/s), 4096 x 6144 x 2048 227 / 187.  Bound: the MMAs (four of one term take 512 cycles to run and 540 to
 // issue; the products of a long pass are at the power limit).  A wait that runs out ends every role; the kernel sets the device's word, which the next launch reports.
 //
-// SUMS: fp32 rows as two fp16 terms (split2_rows_kernel) and weights as fp16 (transpose_to_half_kernel), every row and every column with a power
+// SUMS: fp32 rows as two fp16 terms (split_rows_kernel) and weights as fp16 (transpose_to_half_kernel), every row and every column with a power
 // of two of its own; an accumulator lives for kPairChunk k-blocks and eight epilogue warps add it to the tile's sums in their registers (two
 // threads per row, up to 128 columns each) while the next ones are multiplied into the other.  Against three terms and sums of all products
 // in tensor memory: 1722 rows, K = 2048, 16384 columns 209 -> 162 us, 2048 columns 37 -> 28, K = 8192 118 -> 85; relative error 7.0e-6 -> 5.8e-7
@@ -1258,6 +1244,26 @@ static bool make_map(CUtensorMap* map, const void* base, long long rows, int K, 
                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// SMs of the current device
+static cudaError_t current_sms(int* dev, int* sms) {
+    static std::atomic<int> known[64];
+    const cudaError_t e = cudaGetDevice(dev);
+    if (e != cudaSuccess) return e;
+    if (*dev < 64 && (*sms = known[*dev].load(std::memory_order_relaxed)) > 0) return cudaSuccess;
+    const cudaError_t a = cudaDeviceGetAttribute(sms, cudaDevAttrMultiProcessorCount, *dev);
+    if (a == cudaSuccess && *dev < 64) known[*dev].store(*sms, std::memory_order_relaxed);
+    return a;
+}
+// Dynamic shared memory of a kernel, the same size for every launch: asked for once per device
+template <auto KERNEL>
+static cudaError_t ask_smem(int dev, int bytes) {
+    static std::atomic<bool> asked[64];
+    if (dev < 64 && asked[dev].load(std::memory_order_relaxed)) return cudaSuccess;
+    const cudaError_t e = cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e == cudaSuccess && dev < 64) asked[dev].store(true, std::memory_order_relaxed);
+    return e;
+}
+
 size_t gemm_workspace_bytes(int M, int K) { return (size_t)kTerms * M * K * 2; }
 
 cudaError_t launch_transpose_to_bf16(const void* w, int src_bf16, void* wt, int K, int N, cudaStream_t st) {
@@ -1314,7 +1320,7 @@ static cudaError_t run_pair(const CUtensorMap& ma, const void* wt, long long wt_
     int pairs = 0;
     cudaError_t e = pairs_of<TERMS, SUMS>(dev, &pairs);
     const auto kernel = dia_gemm_pair_kernel<TERMS, SUMS>;
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Pair<SUMS>::kSmem);
+    if (e == cudaSuccess) e = ask_smem<dia_gemm_pair_kernel<TERMS, SUMS>>(dev, Pair<SUMS>::kSmem);
     if (e != cudaSuccess) return e;
     q.ran_out = split_attention_ran_out(dev, st);
     if (q.ran_out && *reinterpret_cast<volatile int*>(q.ran_out)) {
@@ -1336,25 +1342,11 @@ static cudaError_t run_pair(const CUtensorMap& ma, const void* wt, long long wt_
 cudaError_t launch_gemm_tcgen05_bf16(const void* a_bf16, int terms, const void* wt, long long wt_rows, float* y, int M, int N,
                                      int K, const GemmEpilogue& ep, const GemmGroups* groups, cudaStream_t st) {
     if (!gemm_tcgen05_shape_ok(M, N, K) || terms < 1 || terms > kTerms || wt_rows < N) return cudaErrorNotSupported;
-    static bool attr[64] = {};                         // function attributes are per device
-    int dev = 0;
-    cudaError_t e0 = cudaGetDevice(&dev);
+    int dev = 0, sms = 0;
+    cudaError_t e0 = current_sms(&dev, &sms);
+    if (e0 == cudaSuccess) e0 = ask_smem<dia_gemm_tcgen05_kernel>(dev, kGemmSmem);
     if (e0 != cudaSuccess) return e0;
-    if (dev < 0 || dev >= 64 || !attr[dev]) {
-        cudaError_t e = cudaFuncSetAttribute(dia_gemm_tcgen05_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kGemmSmem);
-        if (e != cudaSuccess) return e;
-        if (dev >= 0 && dev < 64) attr[dev] = true;
-    }
     CUtensorMap ma, mb;
-    if (!make_map(&ma, a_bf16, (long long)terms * M, K, BM) || !make_map(&mb, wt, wt_rows, K, BN)) return cudaErrorNotSupported;
-    static int n_sm[64] = {};
-    if (dev < 0 || dev >= 64 || n_sm[dev] == 0) {
-        int n = 0;
-        cudaError_t e = cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-        if (e != cudaSuccess) return e;
-        if (dev < 0 || dev >= 64) n_sm[0] = n; else n_sm[dev] = n;
-    }
-    const int sms = (dev < 0 || dev >= 64) ? n_sm[0] : n_sm[dev];
     int pairs = 0;
     e0 = pairs_of<1, false>(dev, &pairs);
     if (e0 != cudaSuccess) return e0;
@@ -1363,6 +1355,7 @@ cudaError_t launch_gemm_tcgen05_bf16(const void* a_bf16, int terms, const void* 
                                 ep.residual, ep.dyt_w, ep.dyt_b, ep.dyt_alpha};
         if (gemm_f32_ok(narrow)) return run_gemm_f32(narrow, a_bf16, 1, 8, st);
     }
+    if (!make_map(&ma, a_bf16, (long long)terms * M, K, BM)) return cudaErrorNotSupported;
     if (M > BM && (terms == 1 || terms == kTerms) && (!groups || groups->tile_rows % (2 * BM) == 0)) {
         PairProduct q{};
         q.y = y; q.residual = ep.residual; q.M = M; q.N = N; q.K = K;
@@ -1370,6 +1363,7 @@ cudaError_t launch_gemm_tcgen05_bf16(const void* a_bf16, int terms, const void* 
         if (groups) { q.row_group = groups->row_group; q.group_rows = groups->group_rows; q.n_rows = groups->n_rows; }
         return terms == 1 ? run_pair<1, false>(ma, wt, wt_rows, q, dev, st) : run_pair<kTerms, false>(ma, wt, wt_rows, q, dev, st);
     }
+    if (!make_map(&mb, wt, wt_rows, K, BN)) return cudaErrorNotSupported;
     const int n_tiles = ((N + BN - 1) / BN) * ((M + BM - 1) / BM);
     dia_gemm_tcgen05_kernel<<<std::min(n_tiles, sms), kGemmThreads, kGemmSmem, st>>>(
         ma, mb, y, ep.residual, M, N, K, terms, ep.dyt_w, ep.dyt_b, ep.dyt_alpha,
@@ -1414,10 +1408,9 @@ static bool dense_rows_f32(int terms, int M, int N, int K, int sms, int pairs) {
 // splits: the most CTAs that may share a tile (1: a sum's order does not depend on the rows beside it)
 static cudaError_t run_gemm_f32(const F32Product& p, const void* a_terms, int terms, int splits, cudaStream_t st) {
     int dev = 0, sms = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    cudaError_t e = current_sms(&dev, &sms);
     const auto kernel = terms == 1 ? dia_gemm_f32_kernel<1> : dia_gemm_f32_kernel<kTerms>;
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kFSmem);
+    if (e == cudaSuccess) e = terms == 1 ? ask_smem<dia_gemm_f32_kernel<1>>(dev, kFSmem) : ask_smem<dia_gemm_f32_kernel<kTerms>>(dev, kFSmem);
     if (e != cudaSuccess) return e;
     CUtensorMap ma, mb;
     if (!make_map(&ma, a_terms, (long long)terms * p.heads * p.M, p.K, BM) || !make_map(&mb, p.w, (long long)p.heads * p.N, p.K, kFN))
@@ -1474,8 +1467,9 @@ static cudaError_t launch_few_rows(const FewRowsProduct& p, bool early, cudaStre
     while (n_slots > 3 && few_rows_smem(NB, kb_per, n_slots) > kRSmemMost / 2) --n_slots;
     while (few_rows_smem(NB, kb_per, n_slots) > kRSmemMost) --n_slots;
     const size_t smem = std::max<size_t>(few_rows_smem(NB, kb_per, n_slots), kRSmemLeast);
-    // (the same size for every launch: another thread's cannot lower what this one needs)
-    const cudaError_t e = cudaFuncSetAttribute(dia_gemm_few_rows_kernel<NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, kRSmemMost);
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = ask_smem<dia_gemm_few_rows_kernel<NB>>(dev, kRSmemMost);
     if (e != cudaSuccess) return e;
     CUtensorMap mw;
     if (!make_map(&mw, p.w, p.N, p.K, BM)) return cudaErrorNotSupported;
@@ -1505,7 +1499,7 @@ cudaError_t launch_gemm_few_rows(const FewRowsProduct& p, bool early, cudaStream
 bool gemm_half_ok(int M, int N, int K) {
     int dev = 0, sms = 0;
     if (M <= BM || N <= 0 || N % 4 || K < BK || K % BK) return false;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return false;
+    if (current_sms(&dev, &sms) != cudaSuccess) return false;
     return !dense_rows_f32(kTerms, M, N, K, sms, 0);
 }
 
@@ -1518,16 +1512,20 @@ cudaError_t launch_prepare_half(const void* w, int src_bf16, void* wt, float* ma
     return cudaGetLastError();
 }
 
+template <int TERMS>
+static void split_rows(const float* x, const float* norm_w, float eps, bool gated, void* out, float* row_inv, int M, int K, cudaStream_t st) {
+    const int aligned = ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(norm_w)) & 15) == 0;
+    if (gated) split_rows_kernel<TERMS, true><<<M, 256, 0, st>>>(x, nullptr, 0.f, out, row_inv, M, K, aligned);
+    else split_rows_kernel<TERMS, false><<<M, 256, 0, st>>>(x, norm_w, eps, out, row_inv, M, K, aligned);
+}
+
 // y = [residual +] x W for fp32 rows: two fp16 terms and fp32 sums of 64-product pieces, on pairs of SMs.
 cudaError_t launch_gemm_half(const float* x, const float* norm_w, float eps, bool gated, const void* wt, const float* mag, const float* residual, float* y,
                              void* workspace, int M, int N, int K, cudaStream_t st) {
     if (M <= 0 || N <= 0 || N % 4 || K < BK || K % BK || (gated && norm_w)) return cudaErrorNotSupported;
     __half* const terms = reinterpret_cast<__half*>(workspace);
     float* const row_inv = reinterpret_cast<float*>(terms + 2 * (size_t)M * K);
-    if (gated)
-        split2_rows_kernel<true><<<M, 256, 0, st>>>(x, nullptr, 0.f, terms, row_inv, M, K);
-    else
-        split2_rows_kernel<false><<<M, 256, 0, st>>>(x, norm_w, eps, terms, row_inv, M, K);
+    split_rows<2>(x, norm_w, eps, gated, terms, row_inv, M, K, st);
     ++extra_launches();
     CUtensorMap ma;
     int dev = 0;
@@ -1540,34 +1538,31 @@ cudaError_t launch_gemm_half(const float* x, const float* norm_w, float eps, boo
     return run_pair<2, true>(ma, wt, N, q, dev, st);
 }
 
-// fp32 activations: the three-term split (with the row's RMSNorm in front when norm_w is given), then the kernel
-cudaError_t launch_gemm_tcgen05(const float* x, const float* norm_w, float eps, const void* wt, const float* residual,
+// fp32 activations: the three-term split (with the row's RMSNorm in front when norm_w is given, or with the gate of [M][2][K] rows), then
+// the kernel
+cudaError_t launch_gemm_tcgen05(const float* x, const float* norm_w, float eps, bool gated, const void* wt, const float* residual,
                                 float* y, void* workspace, int M, int N, int K, cudaStream_t st) {
-    if (M <= 0 || N % 4 || N <= 0 || K % BK || K < BK) return cudaErrorNotSupported;
+    if (M <= 0 || N % 4 || N <= 0 || K % BK || K < BK || (gated && norm_w)) return cudaErrorNotSupported;
     const long long n = (long long)M * K;
     FewRowsProduct few{x, K, wt, y, N, M, N, K, 0, residual};
     if (dense_rows_few(M)) {
-        if (norm_w) few.a = reinterpret_cast<const float*>(workspace);
+        const bool made = norm_w || gated;                    // (the rows lie in the workspace)
+        if (made) few.a = reinterpret_cast<const float*>(workspace);
         // (the rows are read while outputs are written)
-        const bool apart = norm_w || x + n <= y || y + (long long)M * N <= x;
+        const bool apart = made || x + n <= y || y + (long long)M * N <= x;
         if (apart && gemm_few_rows_ok(few)) {
-            if (norm_w) {
-                split3_norm_rows_kernel<false><<<M, 256, 0, st>>>(x, norm_w, eps, workspace, M, K);
+            if (made) {
+                split_rows<0>(x, norm_w, eps, gated, workspace, nullptr, M, K, st);
                 ++extra_launches();
             }
             return launch_gemm_few_rows(few, false, st);
         }
     }
-    if (norm_w)
-        split3_norm_rows_kernel<true><<<M, 256, 0, st>>>(x, norm_w, eps, workspace, M, K);
-    else
-        split3_rows_kernel<<<(int)std::min<long long>((n + 255) / 256, 148 * 16), 256, 0, st>>>(
-            x, reinterpret_cast<__nv_bfloat16*>(workspace), n);
+    split_rows<kTerms>(x, norm_w, eps, gated, workspace, nullptr, M, K, st);
     ++extra_launches();
     const F32Product wide{nullptr, 0, 0, wt, y, N, N, nullptr, 1, M, N, K, 1.f, 0, nullptr, 0, 0, residual};
     int dev = 0, sms = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const cudaError_t e = current_sms(&dev, &sms);
     if (e != cudaSuccess) return e;
     if (dense_rows_f32(kTerms, M, N, K, sms, 0) && gemm_f32_ok(wide)) return run_gemm_f32(wide, workspace, kTerms, 8, st);
     const GemmEpilogue ep{residual, nullptr, nullptr, 0.f, nullptr};

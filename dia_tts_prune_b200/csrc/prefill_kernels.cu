@@ -6,7 +6,8 @@
 //                           self-attention of the prompt prefill, full / pad-partitioned encoder self-attention,
 //                           cross-attention over the valid text keys.  fp32 throughout (these K/V and outputs are
 //                           re-read by every later greedy step): flash-style, one CTA per (batch row, query head,
-//                           64 queries), K/V tiles of 64 keys staged in padded shared memory, online softmax.
+//                           64 or 32 queries), K/V tiles of 64 keys staged in padded shared memory, online softmax.
+//   head_rows_kernel        the turned heads of a layer's projections, keys and values into the cache, in one launch
 //   rope_rows_kernel        RotaryEmbedding (dia/layers.py:108-173) on projected heads, fused with the layout change
 //                           into the [B, H, T, 128] cache (KVCache.prefill / from_kv, dia/state.py:88-109)
 //   rmsnorm_rows_kernel     torch.nn.RMSNorm over rows (dia/layers.py:462, encoder final norm)
@@ -28,7 +29,6 @@ namespace dia {
 
 namespace {
 
-constexpr int kAQ = 64;               // queries per CTA
 constexpr int kAK = 64;               // keys per tile
 constexpr int kQStride = 132;         // padded row stride (floats) of the Q and K tiles: conflict-free float4 reads
 constexpr int kPStride = 68;
@@ -37,7 +37,9 @@ constexpr int kAttnThreads = 256;
 // itself.  us, 16 heads of 128, this kernel / the tensor cores: one text of 64 17 / 24, 200 45 / 43, 256 47 / 44, 861 290 / 99; two texts of
 // 200 45 / 55, 256 48 / 44; two prompts with 4 key heads 400 111 / 56; cross attention over 200 bytes 200 45 / 55, 400 88 / 58.
 constexpr int kSplitRowsMin = 256;
-constexpr int kAttnSmem = (kAQ * kQStride + kAK * kQStride + kAK * kHeadDim + kAQ * kPStride) * 4;
+// AQ: queries per CTA, 64, or 32 where those leave SMs without a CTA (16 heads, one text of 200: 64 CTAs 42 us, 112 31)
+template <int AQ>
+constexpr int kAttnSmem = (AQ * kQStride + kAK * kQStride + kAK * kHeadDim + AQ * kPStride) * 4;
 
 }  // namespace
 
@@ -45,18 +47,20 @@ constexpr int kAttnSmem = (kAQ * kQStride + kAK * kQStride + kAK * kHeadDim + kA
 // mode 1: partition - query t < n attends keys [0, n), t >= n keys [n, Tk)   (encoder mask, dia/state.py:24-31)
 // mode 2: prefix - every query attends keys [0, n); n == 0 gives exact zeros (cross-attention)
 // n = n_valid[b].  q / out: [B][Tq][Hq][128]; k / v: [B][Hkv][Tk_stride][128]; query head h reads kv head h / (Hq / Hkv).
+template <int AQ>
 __global__ void __launch_bounds__(kAttnThreads, 1)
 attention_rows_kernel(const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ v,
                       float* __restrict__ out, int Tq, int Tk, int Hq, int Hkv, int Tk_stride, int mode,
                       DelayArg n_valid) {
+    constexpr int R = AQ / 16;                                // query rows of a thread
     extern __shared__ __align__(16) float smem_f[];
     float* Qs = smem_f;
-    float* Ks = Qs + kAQ * kQStride;
+    float* Ks = Qs + AQ * kQStride;
     float* Vs = Ks + kAK * kQStride;
     float* Ps = Vs + kAK * kHeadDim;
 
     const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-    const int q0 = blockIdx.x * kAQ, h = blockIdx.y, b = blockIdx.z;
+    const int q0 = blockIdx.x * AQ, h = blockIdx.y, b = blockIdx.z;
     const int kvh = h / (Hq / Hkv);
     const int n = n_valid.d[b];
     const float scale = 0.08838834764831845f;                 // 1/sqrt(128)
@@ -64,7 +68,7 @@ attention_rows_kernel(const float* __restrict__ q, const float* __restrict__ k, 
     const float* vb = v + ((size_t)(b * Hkv + kvh) * Tk_stride) * kHeadDim;
 
     // ---- the query tile (pre-scaled) ----
-    for (int i = tid; i < kAQ * 32; i += kAttnThreads) {
+    for (int i = tid; i < AQ * 32; i += kAttnThreads) {
         const int r = i >> 5, c4 = i & 31, t = q0 + r;
         float4 val = make_float4(0.f, 0.f, 0.f, 0.f);
         if (t < Tq) {
@@ -74,9 +78,9 @@ attention_rows_kernel(const float* __restrict__ q, const float* __restrict__ k, 
         *reinterpret_cast<float4*>(Qs + r * kQStride + c4 * 4) = val;
     }
 
-    float m_run[4], l_run[4], o[4][8];
+    float m_run[R], l_run[R], o[R][8];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
+    for (int i = 0; i < R; ++i) {
         m_run[i] = -CUDART_INF_F; l_run[i] = 0.f;
 #pragma unroll
         for (int j = 0; j < 8; ++j) o[i][j] = 0.f;
@@ -84,10 +88,10 @@ attention_rows_kernel(const float* __restrict__ q, const float* __restrict__ k, 
 
     // key range this query tile can see
     int k_begin = 0, k_end = Tk;
-    if (mode == 0) k_end = min(Tk, q0 + kAQ);
+    if (mode == 0) k_end = min(Tk, q0 + AQ);
     else if (mode == 2) k_end = min(Tk, n);
     else if (mode == 1) {
-        if (q0 + kAQ <= n) k_end = min(Tk, n);               // all queries of the tile are valid text
+        if (q0 + AQ <= n) k_end = min(Tk, n);               // all queries of the tile are valid text
         else if (q0 >= n) k_begin = (n / kAK) * kAK;         // all queries are padding
     }
 
@@ -105,20 +109,20 @@ attention_rows_kernel(const float* __restrict__ q, const float* __restrict__ k, 
         }
         __syncthreads();
         // ---- S = Q K^T: rows ty*4 + i, columns tx + 16 j ----
-        float s[4][4];
+        float s[R][4];
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
+        for (int i = 0; i < R; ++i)
 #pragma unroll
             for (int j = 0; j < 4; ++j) s[i][j] = 0.f;
 #pragma unroll 4
         for (int d4 = 0; d4 < 32; ++d4) {
-            float4 qa[4], ka[4];
+            float4 qa[R], ka[4];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) qa[i] = *reinterpret_cast<const float4*>(Qs + (ty * 4 + i) * kQStride + d4 * 4);
+            for (int i = 0; i < R; ++i) qa[i] = *reinterpret_cast<const float4*>(Qs + (ty * R + i) * kQStride + d4 * 4);
 #pragma unroll
             for (int j = 0; j < 4; ++j) ka[j] = *reinterpret_cast<const float4*>(Ks + (tx + 16 * j) * kQStride + d4 * 4);
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
+            for (int i = 0; i < R; ++i)
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
                     s[i][j] = fmaf(qa[i].x, ka[j].x, s[i][j]);
@@ -129,8 +133,8 @@ attention_rows_kernel(const float* __restrict__ q, const float* __restrict__ k, 
         }
         // ---- mask, online softmax (row statistics across the 16 threads that share a row) ----
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int t = q0 + ty * 4 + i;
+        for (int i = 0; i < R; ++i) {
+            const int t = q0 + ty * R + i;
             float mx = -CUDART_INF_F;
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
@@ -160,21 +164,21 @@ attention_rows_kernel(const float* __restrict__ q, const float* __restrict__ k, 
 #pragma unroll
             for (int j = 0; j < 8; ++j) o[i][j] *= corr;
 #pragma unroll
-            for (int j = 0; j < 4; ++j) Ps[(ty * 4 + i) * kPStride + tx + 16 * j] = s[i][j];
+            for (int j = 0; j < 4; ++j) Ps[(ty * R + i) * kPStride + tx + 16 * j] = s[i][j];
         }
         __syncthreads();
         // ---- O += P V: rows ty*4 + i, output dims tx*4 .. +3 and 64 + tx*4 .. +3 ----
 #pragma unroll 2
         for (int c4 = 0; c4 < kAK / 4; ++c4) {
-            float4 pa[4];
+            float4 pa[R];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) pa[i] = *reinterpret_cast<const float4*>(Ps + (ty * 4 + i) * kPStride + c4 * 4);
+            for (int i = 0; i < R; ++i) pa[i] = *reinterpret_cast<const float4*>(Ps + (ty * R + i) * kPStride + c4 * 4);
 #pragma unroll
             for (int cc = 0; cc < 4; ++cc) {
                 const float4 v0 = *reinterpret_cast<const float4*>(Vs + (c4 * 4 + cc) * kHeadDim + tx * 4);
                 const float4 v1 = *reinterpret_cast<const float4*>(Vs + (c4 * 4 + cc) * kHeadDim + 64 + tx * 4);
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
+                for (int i = 0; i < R; ++i) {
                     const float pv = cc == 0 ? pa[i].x : cc == 1 ? pa[i].y : cc == 2 ? pa[i].z : pa[i].w;
                     o[i][0] = fmaf(pv, v0.x, o[i][0]); o[i][1] = fmaf(pv, v0.y, o[i][1]);
                     o[i][2] = fmaf(pv, v0.z, o[i][2]); o[i][3] = fmaf(pv, v0.w, o[i][3]);
@@ -186,8 +190,8 @@ attention_rows_kernel(const float* __restrict__ q, const float* __restrict__ k, 
     }
     // ---- normalise and store; a query without any allowed key gives exact zeros ----
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int t = q0 + ty * 4 + i;
+    for (int i = 0; i < R; ++i) {
+        const int t = q0 + ty * R + i;
         if (t >= Tq) continue;
         const float inv = l_run[i] > 0.f ? 1.0f / l_run[i] : 0.f;
         float* dst = out + (((size_t)b * Tq + t) * Hq + h) * kHeadDim;
@@ -220,6 +224,38 @@ __global__ void rope_rows_kernel(const float* __restrict__ src, float* __restric
                             : dst + (row * H + hh) * kHeadDim;
         o[d] = o0;
         o[d + 64] = o1;
+    }
+}
+
+// The heads of a layer's projections in one launch: q [row][ldq] turned into q_out [row][Hq * 128], k [row][ldkv] turned and v [row][ldkv] into
+// slots [0, T) of the caches [B][Hkv][slots][128] (Hkv 0: q alone).  One CTA per row; a thread turns four channels and their partners, with
+// the arithmetic of rope_rows_kernel.  Bound: HBM.
+__global__ void __launch_bounds__(256)
+head_rows_kernel(const float* __restrict__ q, int ldq, const float* __restrict__ k, const float* __restrict__ v, int ldkv, float* __restrict__ q_out,
+                 float* __restrict__ k_cache, float* __restrict__ v_cache, const float* __restrict__ sin_tab, const float* __restrict__ cos_tab,
+                 const int* __restrict__ pos, int T, int Hq, int Hkv, int slots, int n_pos) {
+    const int row = blockIdx.x, b = row / T, t = row - b * T, p = min(max(pos[row], 0), n_pos - 1);
+    const int turned = (Hq + Hkv) * 16;
+    for (int i = threadIdx.x; i < turned + Hkv * 32; i += 256) {
+        if (i >= turned) {
+            const int h = (i - turned) >> 5, d = 4 * ((i - turned) & 31);
+            *reinterpret_cast<float4*>(v_cache + (((size_t)b * Hkv + h) * slots + t) * kHeadDim + d) =
+                *reinterpret_cast<const float4*>(v + (size_t)row * ldkv + h * kHeadDim + d);
+            continue;
+        }
+        const int h = i >> 4, d = 4 * (i & 15);
+        const bool is_q = h < Hq;
+        const float* src = is_q ? q + (size_t)row * ldq + h * kHeadDim + d : k + (size_t)row * ldkv + (h - Hq) * kHeadDim + d;
+        float* dst = is_q ? q_out + ((size_t)row * Hq + h) * kHeadDim + d : k_cache + (((size_t)b * Hkv + h - Hq) * slots + t) * kHeadDim + d;
+        const float4 x = *reinterpret_cast<const float4*>(src), y = *reinterpret_cast<const float4*>(src + 64);
+        const float4 sn = *reinterpret_cast<const float4*>(sin_tab + (size_t)p * 64 + d), cs = *reinterpret_cast<const float4*>(cos_tab + (size_t)p * 64 + d);
+        float4 lo, hi;                                        // separate roundings, like the reference's
+        lo.x = __fsub_rn(__fmul_rn(x.x, cs.x), __fmul_rn(y.x, sn.x)); hi.x = __fadd_rn(__fmul_rn(x.x, sn.x), __fmul_rn(y.x, cs.x));
+        lo.y = __fsub_rn(__fmul_rn(x.y, cs.y), __fmul_rn(y.y, sn.y)); hi.y = __fadd_rn(__fmul_rn(x.y, sn.y), __fmul_rn(y.y, cs.y));
+        lo.z = __fsub_rn(__fmul_rn(x.z, cs.z), __fmul_rn(y.z, sn.z)); hi.z = __fadd_rn(__fmul_rn(x.z, sn.z), __fmul_rn(y.z, cs.z));
+        lo.w = __fsub_rn(__fmul_rn(x.w, cs.w), __fmul_rn(y.w, sn.w)); hi.w = __fadd_rn(__fmul_rn(x.w, sn.w), __fmul_rn(y.w, cs.w));
+        *reinterpret_cast<float4*>(dst) = lo;
+        *reinterpret_cast<float4*>(dst + 64) = hi;
     }
 }
 
@@ -277,19 +313,14 @@ cudaError_t launch_attention_rows(const float* q, const float* k, const float* v
         s.out = out; s.ldo = Hq * kHeadDim; s.out_scale = 1.f;
         if (split_attention_ok(s)) return launch_split_attention(s, st);
     }
-    static bool attr[64] = {};
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e != cudaSuccess) return e;
-    if (dev < 0 || dev >= 64 || !attr[dev]) {
-        e = cudaFuncSetAttribute(attention_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kAttnSmem);
-        if (e != cudaSuccess) return e;
-        if (dev >= 0 && dev < 64) attr[dev] = true;
-    }
     DelayArg nv{};
     for (int b = 0; b < B; ++b) nv.d[b] = n_valid_host ? n_valid_host[b] : Tk;
-    dim3 grid((Tq + kAQ - 1) / kAQ, Hq, B);
-    attention_rows_kernel<<<grid, kAttnThreads, kAttnSmem, st>>>(q, k, v, out, Tq, Tk, Hq, Hkv, Tk_stride, mode, nv);
+    const bool small = (long long)((Tq + 63) / 64) * Hq * B < 148;
+    const int AQ = small ? 32 : 64, bytes = small ? kAttnSmem<32> : kAttnSmem<64>;
+    const auto kernel = small ? attention_rows_kernel<32> : attention_rows_kernel<64>;
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e != cudaSuccess) return e;
+    kernel<<<dim3((Tq + AQ - 1) / AQ, Hq, B), kAttnThreads, bytes, st>>>(q, k, v, out, Tq, Tk, Hq, Hkv, Tk_stride, mode, nv);
     return cudaGetLastError();
 }
 
@@ -298,6 +329,13 @@ cudaError_t launch_rope_rows(const float* src, float* dst, const float* sin_tab,
     const long long total = (long long)B * T * H * 64;
     rope_rows_kernel<<<grid_for(total, 256), 256, 0, st>>>(src, dst, sin_tab, cos_tab, pos, B, T, H, rotate, to_cache, dst_T,
                                                            dst_t0, n_pos);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_head_rows(const float* q, int ldq, const float* k, const float* v, int ldkv, float* q_out, float* k_cache, float* v_cache,
+                             const float* sin_tab, const float* cos_tab, const int* pos, int B, int T, int Hq, int Hkv, int slots, int n_pos,
+                             cudaStream_t st) {
+    head_rows_kernel<<<B * T, 256, 0, st>>>(q, ldq, k, v, ldkv, q_out, k_cache, v_cache, sin_tab, cos_tab, pos, T, Hq, Hkv, slots, n_pos);
     return cudaGetLastError();
 }
 

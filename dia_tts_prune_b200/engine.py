@@ -403,14 +403,14 @@ def launch_count() -> int:
 
 
 # ---- tcgen05 GEMM for dense layers with more than one row (encoder, cross-KV precompute, prefill) ---------------------
-def dense_prepare_weight(w_KxN: torch.Tensor) -> torch.Tensor:
-    """K-major bf16 copy ``[N, K]`` of a DenseGeneral kernel viewed as ``[K, N]`` (float32 or bfloat16, CUDA)."""
+def dense_prepare_weight(w_KxN: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
+    """K-major bf16 copy ``[N, K]`` of a DenseGeneral kernel viewed as ``[K, N]`` (float32 or bfloat16, CUDA), in ``out`` when given."""
     lib = _lib.load()
     if not w_KxN.is_cuda or w_KxN.dim() != 2 or w_KxN.dtype not in (torch.float32, torch.bfloat16):
         raise ValueError("expected a 2-D float32 / bfloat16 CUDA tensor")
     w = w_KxN.contiguous()
     K, N = w.shape
-    wt = torch.empty((N, K), dtype=torch.bfloat16, device=w.device)
+    wt = torch.empty((N, K), dtype=torch.bfloat16, device=w.device) if out is None else out
     _lib.check(lib.dia_b200_dense_prepare_weight(_ptr(w), 1 if w.dtype == torch.bfloat16 else 0, _ptr(wt), K, N,
                                                  _stream(w.device)), "dense_prepare_weight")
     return wt
@@ -516,6 +516,17 @@ def rope_rows(src_BTxHd: torch.Tensor, pos: torch.Tensor | None, B: int, T: int,
                                       0 if cache is None else 1, 0 if cache is None else cache.shape[2], int(cache_t0),
                                       sin.shape[0], _stream(src_BTxHd.device)), "rope_rows")
     return dst
+
+
+def rows_layer_work_bytes(args: "_lib.RowsLayer") -> int:
+    return int(_lib.load().dia_b200_rows_layer_work_bytes(C.byref(args)))
+
+
+def rows_layer_forward(args: "_lib.RowsLayer", work_bytes: int, device: torch.device) -> None:
+    """One encoder or decoder layer over many rows (``dia_b200_rows_layer_forward``); the workspace is taken here."""
+    work = torch.empty((work_bytes,), dtype=torch.uint8, device=device)
+    args.work = work.data_ptr()
+    _lib.check(_lib.load().dia_b200_rows_layer_forward(C.byref(args), _stream(device)), "rows_layer_forward")
 
 
 def attention_rows(q_BTHd: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, Tk: int, mode: int,

@@ -239,24 +239,12 @@ class MlpBlock(nn.Module):
         self.wo = DenseGeneral((intermediate_dim,), (embed_dim,), axis=(-1,), weight_dtype=compute_dtype)
 
     def forward(self, x: Tensor) -> Tensor:
-        if x.is_cuda and not torch.is_grad_enabled():
-            return self._forward_b200(x, None, 0.0, None)
         gu = self.wi_fused(x)                               # [..., 2, F]: gate columns first, then up
+        if x.is_cuda and not torch.is_grad_enabled():
+            from . import engine as _k
+            h = _k.silu_mul(gu.reshape(-1, 2, gu.shape[-1]))
+            return self.wo(h.reshape(*x.shape[:-1], -1))
         return self.wo(F.silu(gu[..., 0, :].float()).to(x.dtype) * gu[..., 1, :])
-
-    def _forward_b200(self, x: Tensor, norm: RMSNorm | None, eps: float, residual: Tensor | None) -> Tensor:
-        """``residual + wo(silu(gate) * up)`` with ``[gate | up] = wi_fused(norm(x))`` on our kernels: RMSNorm in the
-        split pass of the first GEMM, the gate as one elementwise kernel, the residual add in the second epilogue."""
-        from . import engine as _k
-        lead = x.shape[:-1]
-        gu = self.wi_fused._forward_tcgen05(x, (x.ndim - 1,), norm_weight=None if norm is None else norm.weight, eps=eps)
-        if residual is not None and _k.dense_half_rows(gu.numel() // (2 * gu.shape[-1]), residual.shape[-1], gu.shape[-1], gu.device):
-            half = self.wo.kernel_weight_half() if _plain(gu, residual) else None
-            if half is not None:                            # the gate inside the split pass of the second GEMM
-                return _k.dense_forward_half(gu.reshape(-1, 2, gu.shape[-1]), half, residual=residual.reshape(-1, residual.shape[-1]),
-                                             gated=True).reshape(residual.shape)
-        h = _k.silu_mul(gu.reshape(-1, 2, gu.shape[-1]))
-        return self.wo._forward_tcgen05(h.reshape(*lead, -1), (x.ndim - 1,), residual=residual)
 
 
 class RotaryEmbedding(nn.Module):
@@ -330,38 +318,105 @@ class Attention(nn.Module):
             out = torch.where(attn_mask.any(dim=-1, keepdim=True), out, torch.zeros((), dtype=out.dtype, device=out.device))
         return self.o_proj(out.transpose(1, 2).contiguous()).to(Xq.dtype)
 
-    def _forward_b200(self, x: Tensor, norm: RMSNorm, eps: float, positions_i32: Tensor, tables, mode: int,
-                      n_valid: list[int] | None, cache: KVCache | None = None, prefill: bool = False) -> Tensor:
-        """``x + o_proj(attention(...))`` for T > 1 rows on our kernels (no library call): RMSNorm fused into the split
-        pass of the q / k / v GEMMs, RoPE fused with the scatter into the cache layout, fp32 flash-style attention,
-        residual add in the o_proj epilogue.  ``mode``: 0 causal self, 1 pad-partitioned self, 2 cross over the valid
-        prefix of ``cache`` (precomputed K/V).  Self-attention with ``cache`` + ``prefill`` writes slots [0, T)."""
-        from . import engine as _k
-        B, T, _ = x.shape
-        H, Hkv = self.num_query_heads, self.num_kv_heads
-        ax = (2,)
-        q = self.q_proj._forward_tcgen05(x, ax, norm_weight=norm.weight, eps=eps)            # [B, T, H, 128]
-        _k.rope_rows(q.reshape(B * T, H * 128), positions_i32, B, T, H, tables)
-        if self.is_cross_attn:
-            if cache is None:
-                raise NotImplementedError("cross-attention needs the precomputed K/V cache")
-            kc, vc, Tk = cache.k, cache.v, cache.k.shape[2]
-        else:
-            k = self.k_proj._forward_tcgen05(x, ax, norm_weight=norm.weight, eps=eps)        # [B, T, Hkv, 128]
-            v = self.v_proj._forward_tcgen05(x, ax, norm_weight=norm.weight, eps=eps)
-            if cache is not None:
-                if not prefill:
-                    raise NotImplementedError("T > 1 rows append through prefill only")
-                kc, vc = cache.k, cache.v
-                cache.current_idx = T - 1                                                  # KVCache.prefill (Appendix C Q2)
-            else:
-                kc = torch.empty((B, Hkv, T, 128), dtype=torch.float32, device=x.device)
-                vc = torch.empty_like(kc)
-            _k.rope_rows(k.reshape(B * T, Hkv * 128), positions_i32, B, T, Hkv, tables, cache=kc)
-            _k.rope_rows(v.reshape(B * T, Hkv * 128), None, B, T, Hkv, tables, rotate=False, cache=vc)
-            Tk = T
-        o = _k.attention_rows(q, kc, vc, Tk, mode, n_valid)
-        return self.o_proj._forward_tcgen05(o, (2, 3), residual=x)
+
+def _stack_kmajor(modules: list["DenseGeneral"]) -> None:
+    """The K-major copies of these kernels, one behind the other: products of the same rows are then one product."""
+    from . import engine as _engine
+    have = [m.__dict__.get("_b200_wt") for m in modules]
+    if all(h is not None and h[0] == m._weight_key() for h, m in zip(have, modules)):
+        at = [h[1].data_ptr() for h in have]
+        if all(b - a == 2 * h[1].numel() for a, b, h in zip(at, at[1:], have)) or torch.cuda.is_current_stream_capturing():
+            return
+    for m in modules:
+        canonicalize_dense_kernel_(m)
+    K, sizes = math.prod(modules[0].in_shapes), [math.prod(m.out_features) for m in modules]
+    rows = torch.empty((sum(sizes), K), dtype=torch.bfloat16, device=modules[0].weight.device)
+    for m, out in zip(modules, rows.split(sizes)):
+        m._b200_wt = (m._weight_key(), _engine.dense_prepare_weight(m.weight.detach().reshape(K, out.shape[0]), out))
+
+
+# Layer -> (key, arguments, copies, norms) of its last native call.  Not an attribute: a copied or unpickled layer starts without one.
+_ROWS: "weakref.WeakKeyDictionary[nn.Module, tuple]" = weakref.WeakKeyDictionary()
+
+
+def _rows_weights(M: int, D: int, attn: Attention, norm: RMSNorm, mlp: MlpBlock, norm_mlp: RMSNorm, eps: float, cross: Attention | None,
+                  norm_cross: RMSNorm | None, device):
+    """What a native layer call of ``M`` rows reads of the layer: the arguments, the copies of its weights that they point at, and its norms."""
+    from . import engine as _k
+    from ._lib import DenseRef, RowsLayer
+    keep, copies = [], []
+    a = RowsLayer(D=D, F=mlp.wo.in_shapes[0], heads=attn.num_query_heads, kv_heads=attn.num_kv_heads, eps=eps)
+
+    def vector(n: RMSNorm) -> int:
+        w = n.weight.detach().to(torch.float32).contiguous()
+        if w.numel() != D:
+            raise ValueError("norm weight length must equal K")
+        keep.extend((n.weight.detach(), w))
+        return w.data_ptr()
+
+    a.norm_self, a.norm_mlp = vector(norm), vector(norm_mlp)
+    if cross is not None:
+        a.cross_heads, a.norm_cross = cross.num_query_heads, vector(norm_cross)
+
+    def half(m: DenseGeneral):                                    # the product's rows go as two fp16 terms
+        K, N = math.prod(m.in_shapes), math.prod(m.out_features)
+        if not _k.dense_supported(M, N, K):
+            raise NotImplementedError(f"dense layer [{M} x {K}] . [{K} x {N}] does not fit the tcgen05 tiling (K must be a multiple of 64, N of 4)")
+        return m.kernel_weight_half() if _k.dense_half_rows(M, N, K, device) else None
+
+    def ref(m: DenseGeneral) -> DenseRef:
+        h = half(m)
+        if h is None:
+            m.kernel_weight_kmajor()
+        name = "_b200_wt" if h is None else "_b200_half"
+        copies.append((m, name, m.__dict__[name]))
+        return DenseRef(wt_bf16=copies[-1][2][1].data_ptr()) if h is None else DenseRef(wt_half=h[0].data_ptr(), magnitudes=h[1].data_ptr())
+
+    kv = [attn.k_proj, attn.v_proj]
+    if all(half(m) is None for m in kv):
+        _stack_kmajor(kv if half(attn.q_proj) is not None else [attn.q_proj, *kv])
+    a.q, a.k, a.v, a.o = ref(attn.q_proj), ref(attn.k_proj), ref(attn.v_proj), ref(attn.o_proj)
+    if cross is not None:
+        a.cross_q, a.cross_o = ref(cross.q_proj), ref(cross.o_proj)
+    a.wi, a.wo = ref(mlp.wi_fused), ref(mlp.wo)
+    return a, copies, keep
+
+
+def _rows_layer(owner: nn.Module, x: Tensor, attn: Attention, norm: RMSNorm, mlp: MlpBlock, norm_mlp: RMSNorm, eps: float, positions_i32: Tensor, tables,
+                mode: int, n_valid: list[int] | None, k: Tensor, v: Tensor, cross: tuple | None = None, out: Tensor | None = None) -> Tensor:
+    """One layer over ``x [B, T, D]`` (float32, contiguous) on our kernels, in one native call: RMSNorm in the split pass of the projections, RoPE with
+    the scatter into the caches ``k``, ``v [B, heads, slots, 128]``, attention, residual adds in the epilogues, the gate in the split pass of
+    the last product.  ``mode``: 0 causal, 1 pad-partitioned at ``n_valid``.  ``cross``: (attention, norm, cache, valid keys) of a cross-attention
+    behind the self-attention.  The result is in ``out`` (``x`` itself, say) or a new tensor."""
+    from . import engine as _k
+    B, T, D = x.shape
+    y = torch.empty_like(x) if out is None else out
+    if B * T == 0:
+        return y
+    if x.data_ptr() % 16:                                         # (a view of other memory)
+        x = x.clone()
+    ca, cn, cc, valid = cross if cross is not None else (None, None, None, None)
+    for t in (k, v) if cc is None else (k, v, cc.k, cc.v):
+        assert t.shape[0] == B and t.is_contiguous() and t.dtype == torch.float32 and t.shape[3] == 128
+    # the layer's arguments are made once per number of rows and set of weight copies (which a kernel drops when it changes)
+    norms = (norm.weight, norm_mlp.weight) if ca is None else (norm.weight, norm_mlp.weight, cn.weight)
+    key = (B * T, D, eps, *((w.data_ptr(), w._version, w.dtype) for w in norms))
+    made = _ROWS.get(owner)
+    if made is None or made[0] != key or any(m.__dict__.get(name) is not c or c[0] != m._weight_key() for m, name, c in made[2]):
+        made = (key, *_rows_weights(B * T, D, attn, norm, mlp, norm_mlp, eps, ca, cn, x.device))
+        if not torch.cuda.is_current_stream_capturing():          # (a capture may have to do without the fp16 copies)
+            _ROWS[owner] = made
+    a = type(made[1]).from_buffer_copy(made[1])
+    a.B, a.T, a.slots, a.mode, a.n_pos = B, T, k.shape[2], mode, tables[0].shape[0]
+    a.x_in, a.x, a.positions = x.data_ptr(), y.data_ptr(), positions_i32.data_ptr()
+    a.sin_table, a.cos_table, a.k_cache, a.v_cache = tables[0].data_ptr(), tables[1].data_ptr(), k.data_ptr(), v.data_ptr()
+    if n_valid is not None:
+        a.n_valid[:B] = [int(n) for n in n_valid]
+    if cc is not None:
+        a.cross_slots, a.cross_k, a.cross_v = cc.k.shape[2], cc.k.data_ptr(), cc.v.data_ptr()
+        a.cross_valid[:B] = [int(n) for n in valid]
+    _k.rows_layer_forward(a, _k.rows_layer_work_bytes(a), x.device)
+    return y
 
 
 class EncoderLayer(nn.Module):
@@ -380,13 +435,13 @@ class EncoderLayer(nn.Module):
             from . import engine as _k
             eps = self.config.model.normalization_layer_epsilon
             B, T, _ = x.shape
-            x = x.to(torch.float32).contiguous().clone()                                  # updated in place below
+            x = x.to(torch.float32).contiguous()
             pos = state.extras.get("pos_i32")
             if pos is None or pos.numel() != B * T:
                 pos = state.extras["pos_i32"] = _k.positions_i32(T, B, x.device)
-            x = self.self_attention._forward_b200(x, self.pre_sa_norm, eps, pos, _k.rope_tables_device(self.config, x.device),
-                                                  1, _encoder_valid_lens(state))
-            return self.mlp._forward_b200(x, self.post_sa_norm, eps, x)
+            kv = torch.empty((2, B, self.self_attention.num_kv_heads, T, 128), dtype=torch.float32, device=x.device)
+            return _rows_layer(self, x, self.self_attention, self.pre_sa_norm, self.mlp, self.post_sa_norm, eps, pos,
+                               _k.rope_tables_device(self.config, x.device), 1, _encoder_valid_lens(state), kv[0], kv[1])
         h = self.pre_sa_norm(x.float())
         x = x + self.self_attention(h, h, state.positions, state.positions, attn_mask=state.attn_mask)
         return x + self.mlp(self.post_sa_norm(x.float()))
@@ -479,11 +534,18 @@ class DecoderLayer(nn.Module):
             if state.text_len is None:
                 raise NotImplementedError("prefill needs DecoderInferenceState.text_len (valid text bytes)")
             x = x.to(torch.float32).contiguous()
-            x = self.self_attention._forward_b200(x, self.pre_sa_norm, eps, pos, tables, 0, None,
-                                                  cache=self_attn_cache, prefill=True)
-            x = self.cross_attention._forward_b200(x, self.pre_ca_norm, eps, pos, tables, 2,
-                                                   [0] * (B - 1) + [state.text_len], cache=cross_attn_cache)
-            return self.mlp._forward_b200(x, self.pre_mlp_norm, eps, x)
+            if self_attn_cache is not None:
+                if not prefill:
+                    raise NotImplementedError("T > 1 rows append through prefill only")
+                k, v = self_attn_cache.k, self_attn_cache.v
+                self_attn_cache.current_idx = T - 1                                        # KVCache.prefill (Appendix C Q2)
+            else:
+                k, v = torch.empty((2, B, self.self_attention.num_kv_heads, T, 128), dtype=torch.float32, device=x.device)
+            if cross_attn_cache is None:
+                raise NotImplementedError("cross-attention needs the precomputed K/V cache")
+            return _rows_layer(self, x, self.self_attention, self.pre_sa_norm, self.mlp, self.pre_mlp_norm, eps, pos, tables, 0, None, k, v,
+                               (self.cross_attention, self.pre_ca_norm, cross_attn_cache, [0] * (B - 1) + [state.text_len]),
+                               out=x if x.data_ptr() % 16 == 0 else None)
         # CPU (state-dict tooling and the CPU test suite): the reference's own formulation
         h = self.pre_sa_norm(x.float())
         x = x + self.self_attention(h, h, state.dec_positions, state.dec_positions, attn_mask=None,

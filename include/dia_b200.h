@@ -248,6 +248,37 @@ int dia_b200_dense_prepare_half(const void *w, int src_dtype, void *wt_half, flo
 int dia_b200_dense_forward_half(const float *x, const float *norm_weight, float eps, int gated, const void *wt_half, const float *magnitudes,
                                 const float *residual, float *y, void *workspace, int M, int N, int K, void *stream);
 
+/* One encoder or decoder layer over B x T rows in one call (EncoderLayer / DecoderLayer.forward, dia/layers.py:384-416, 530-584): the launches of
+ * the entry points around it, in their order.  x_in [B*T][D] is the residual stream, x what it becomes (the same or apart).  The
+ * self-attention's keys and values go to slots [0, T) of k_cache / v_cache [B][kv_heads][slots][128], with mode and n_valid as
+ * dia_b200_attention_rows has them; cross_heads > 0: cross-attention (mode 2, cross_valid) over cross_k / cross_v
+ * [B][cross_heads][cross_slots][128] follows.  Heads have 128 channels.
+ * A weight is its fp16 copy with its magnitudes (dia_b200_dense_prepare_half) or, with wt_half NULL, its bf16 copy; the bf16 copies of q, k and v (or
+ * of k and v) may lie one behind the other and are then one product.  All pointers 16-byte aligned, norms excepted. */
+typedef struct dia_b200_dense_ref {
+    const void *wt_bf16;
+    const void *wt_half;
+    const float *magnitudes;
+} dia_b200_dense_ref;
+typedef struct dia_b200_rows_layer {
+    int32_t B, T, D, F;
+    int32_t heads, kv_heads, slots, mode;
+    int32_t cross_heads, cross_slots, n_pos;
+    float eps;
+    int32_t n_valid[16], cross_valid[16];
+    const float *x_in;
+    float *x;
+    const float *sin_table, *cos_table;      /* [n_pos][64] */
+    const int32_t *positions;                /* [B*T] */
+    const float *norm_self, *norm_cross, *norm_mlp;
+    dia_b200_dense_ref q, k, v, o, cross_q, cross_o, wi, wo;
+    float *k_cache, *v_cache;
+    const float *cross_k, *cross_v;
+    void *work;                              /* dia_b200_rows_layer_work_bytes(a) bytes of device memory */
+} dia_b200_rows_layer;
+size_t dia_b200_rows_layer_work_bytes(const dia_b200_rows_layer *a);
+int dia_b200_rows_layer_forward(const dia_b200_rows_layer *a, void *stream);
+
 /* ---- the rest of the T > 1 passes (once per utterance): no library kernel on the path ---------------------------
  * F.scaled_dot_product_attention call sites (dia/layers.py:329-337) for more than one query row, fp32.
  *   q, out float32 [B][Tq][Hq][128] (q already rotated); k, v float32 [B][Hkv][Tk_stride][128] (KVCache layout,
