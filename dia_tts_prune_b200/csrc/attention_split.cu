@@ -711,7 +711,7 @@ split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_co
         const bool ranged = p.rows_per_slot > 0 && p.mode != 0;
         // scores and maxima are in units of log 2 (a capped score from its cap on): the largest score's weight is exactly 1 at any magnitude
         const float cap = p.cap, inv_cap = cap > 0.f ? 1.0f / cap : 0.f;
-        const float mult = q_inv[row] * p.scale * (p.temp ? p.temp[h] : 1.f) * (cap > 0.f ? inv_cap : kLog2e);      // (a capped score: over its cap)
+        const float mult = q_inv[row] * p.scale * (p.temp ? p.temp[h] : 1.f) * (cap > 0.f ? 1.f : kLog2e);
         const float slope = p.slopes ? p.slopes[h] * kLog2e : 0.f;
         // channels of this thread: c0 .. + n_mine, at t_mine in tensor memory
         const int share = NVS == 1 ? (geo.wv0 + 8 * RT - 1) / (8 * RT) * 8 : DVH, part = NVS == 1 ? hf : hf % (RT / 2), group = NVS == 1 ? 0 : hf / (RT / 2);
@@ -784,6 +784,13 @@ split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_co
             // ---- cap, distance bias, visibility ----
             const int k0 = w.j0 + hf * KP;
             if (cap > 0.f) {
+                const float2 ic = make_float2(inv_cap, inv_cap);
+#pragma unroll
+                for (int e = 0; e < KP; e += 2) {
+                    const float2 x = mul2(make_float2(s[e], s[e + 1]), ic);
+                    s[e] = x.x;
+                    s[e + 1] = x.y;
+                }
                 float big = 0.f;
 #pragma unroll
                 for (int e = 0; e < KP; ++e) big = fmaxf(big, fabsf(s[e]));
