@@ -1380,10 +1380,12 @@ bool gemm_f32_ok(const F32Product& p) {
 // Which kernel takes a product of M fp32 rows.  Up to 32 rows the few-rows kernel (N = 2048, K = 1024, 32 rows: 25 us on the 128 x 256
 // tiles, 11 here; N = K = 2048: 42 and 22).
 static bool dense_rows_few(int M) { return M <= kGemmFewRowsMost; }
-// CTAs that share a 128 x 128 tile of the fp32-sum kernel: as many as the chip has room for, two k-blocks each at least
+// CTAs that share a 128 x 128 tile of the fp32-sum kernel: as many as the chip has room for, two k-blocks each at least.  Clusters of eight
+// up to twelve tiles: more of them do not all find eight free SMs close to one another (three terms, us, with four / eight: 12 tiles K = 2048
+// 13.3 / 10.5, 16 tiles K = 1024 9.9 / 14.8, K = 4096 20.4 / 25.2)
 static int f32_splits(int tiles, int n_kb, int most, int sms) {
     int s = 1;
-    while (2 * s <= most && tiles * 2 * s <= sms && n_kb >= 4 * s) s *= 2;
+    while (2 * s <= most && tiles * 2 * s <= (s == 4 ? 96 : sms) && n_kb >= 4 * s) s *= 2;
     return s;
 }
 // Beyond 32 rows (and for bf16 rows) the fp32-sum kernel where its rounds of tiles are the shorter ones: its 128 x 128 tiles are twice
