@@ -76,6 +76,23 @@ cudaError_t launch_sink_attention(const float* qk, int q_stride, const float* kc
                                   const AttnShape& a, const RowMeta& rm, float* out, void* out_bf16, float* split_ws,
                                   unsigned* arrived, int M, cudaStream_t st, int ldo = 0, float out_scale = 1.f,
                                   const float* gate = nullptr, int ldg = 0, const SplitRoom* split = nullptr);
+// Attention of up to kAttnRowsKernelMax rows over the pages (lm_attention.cu): row r, head h reads q + r ldq + h kdim.  shared_kv: the value is
+// the head of the key row.  part: kAttnRowsKernelMax * heads * kAttnSplitsMax * (vdim + 2) floats; arrived: kAttnRowsKernelMax * heads zeroed counters.
+struct FewAttention {
+    const float* q; int ldq;
+    const float* kcache; const float* vcache; bool shared_kv;
+    const int* table; int max_pages, page_size;
+    int heads, kv_heads, kdim, vdim;
+    float scale, cap;                                                           // cap <= 0: none
+    const float* temp; const float* slopes; const float* sink;                  // [heads]; each may be null
+    int window, keep_first, chunk;
+    const int* row_slot; const int* row_pos;
+    float* part; unsigned* arrived;
+    float* out; int ldo; void* out_bf16; float out_scale;
+    const float* gate; const float* head_gate; int ldg;                         // sigmoid(gate[r ldg + h vdim + c]), head_gate[r ldg + h]; may be null
+};
+bool few_rows_attention_ok(const FewAttention& p);
+cudaError_t launch_few_rows_attention(const FewAttention& p, int M, cudaStream_t st);
 cudaError_t launch_router_topk(const float* z, int E, int top, int M, int* sel_e, float* sel_w, cudaStream_t st,
                                const float* bias = nullptr, bool softmax_top = false, const GroupedRoute* gr = nullptr);
 cudaError_t launch_moe_group(const int* sel_e, const float* sel_w, int n_assign, int top, int E, int pad, const GroupMap& gm,

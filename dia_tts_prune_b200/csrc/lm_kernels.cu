@@ -1363,6 +1363,10 @@ cudaError_t launch_sink_attention(const float* qk, int q_stride, const float* kc
             default: return launch_attention_tiles<4>(qk, q_stride, kcache, vcache, pm, a, rm, out, ob, ldo, out_scale, M, st, gate, ldg);
         }
     }
+    const FewAttention few{qk, q_stride, kcache, vcache, false, pm.table, pm.max_pages, pm.page_size, a.heads, a.kv_heads, a.dim, a.dim, a.scale, a.softcap,
+                           a.temp, a.slopes, a.sink, a.window, a.keep_first, a.chunk, rm.slot, rm.pos, split_ws, arrived, out, ldo, out_bf16, out_scale,
+                           gate, nullptr, ldg};
+    if (few_rows_attention_ok(few)) return launch_few_rows_attention(few, M, st);
     const int group = a.heads / a.kv_heads;
     if (group >= 4) return launch_attention_splits<4>(qk, q_stride, kcache, vcache, pm, a, rm, out, ob, ldo, out_scale, M, split_ws, arrived, st, gate, ldg);
     if (group >= 2) return launch_attention_splits<2>(qk, q_stride, kcache, vcache, pm, a, rm, out, ob, ldo, out_scale, M, split_ws, arrived, st, gate, ldg);

@@ -819,6 +819,13 @@ cudaError_t launch_talk_attention(const float* proj, int ld, int q_off, int gate
         s.seq_slot = split->sm.slot; s.seq_row0 = split->sm.row0; s.seq_count = split->sm.count; s.n_seq = split->n_seq;
         if (dia::split_attention_ok(s)) return dia::launch_split_attention(s, st);
     }
+    if (M <= kAttnRowsKernelMax && !a.talk) {
+        const bool latent = kcache == vcache && a.kv_heads == 1 && a.vdim <= a.dim;
+        const FewAttention few{proj + q_off, ld, kcache, vcache, latent, pm.table, pm.max_pages, pm.page_size, a.heads, a.kv_heads, a.dim, a.vdim, 1.f, 0.f,
+                               nullptr, nullptr, a.sink, a.window, 0, 0, rm.slot, rm.pos, split_ws, arrived, out, ldo, out_bf16, 1.f,
+                               nullptr, gate_off >= 0 ? proj + gate_off : nullptr, ld};
+        if ((latent || kcache != vcache) && few_rows_attention_ok(few)) return launch_few_rows_attention(few, M, st);
+    }
     const int vu = (a.vdim + 31) / 32;
 #define TALK_CASE(VU, NP, NW) \
     return launch_talk_inst<VU, NP, NW>(proj, ld, q_off, gate_off, kcache, vcache, pm, a, rm, out, ldo, ob, split_ws, arrived, M, TQ, S, st)
