@@ -4,7 +4,7 @@
 //
 // f is the identity, a DynamicTanh per output column, or an activation whose result is kept as the bf16 operand of the next
 // product (Yb[M][N] instead of Y).  With row groups, the rows of A are sorted by group, every
-// group starts on a multiple of kGemmRowTile rows, and group g multiplies rows [g * group_rows, g * group_rows + N)
+// group starts on a multiple of GemmGroups::tile_rows rows, and group g multiplies rows [g * group_rows, g * group_rows + N)
 // of Wt.
 #pragma once
 

@@ -25,7 +25,7 @@
 //   down_combine_rows_kernel   down products of a row's experts and the shared expert, their sum, norm, residual add
 //   router_rows_kernel         router logits, top experts, scores and the assignment maps of a handful of rows
 //   qk_norm_cache_kernel       whole-projection RMS norm of q and k, raw k and normed k scattered into the paged cache
-//   sink_attention_split_kernel   softmax attention over the pages for a handful of rows, split over
+//   sink_attention_split_kernel   softmax attention over the pages for a handful of rows (those that lm_attention.cu does not take), split over
 //                              the keys: per-head temperature, tanh cap, linear distance bias, a window that keeps the
 //                              first tokens, and a value-less sink term in the denominator
 //   sink_attention_tile_kernel the same for prompt portions: 64 queries share the key / value tiles (flash-style)

@@ -11,9 +11,9 @@ What runs where
     entirely in the hand-written sm_100a kernels of ``csrc/`` through the C ABI (``engine.py``).
     There is no eager fallback for them: without a CUDA device they raise.
   * ``Encoder``, ``Decoder.precompute_cross_attn_cache`` and the prompt prefill (``Decoder.forward``)
-    are once-per-utterance work.  Every dense layer of these T > 1 passes runs on
-    the tcgen05 / TMEM GEMM of ``csrc/gemm_tcgen05.cu`` (``DenseGeneral._forward_tcgen05``); their attention is
-    library SDPA in fp32.  The results feed the decode kernels through the KV caches.
+    are once-per-utterance work.  A layer of these T > 1 passes is one native call (``_rows_layer``): its dense layers run on
+    the tcgen05 / TMEM GEMMs of ``csrc/gemm_tcgen05.cu``, its attention on the kernels of ``csrc/prefill_kernels.cu`` and
+    ``csrc/attention_split.cu``.  The results feed the decode kernels through the KV caches.
   * Pruned checkpoints: ``Decoder.engine()`` drops exactly-dead MLP neurons from the weight stream and streams a
     2:4 model compressed on ``mma.sp`` (``pruning_utils``).
 
