@@ -354,6 +354,12 @@ def _rows_weights(M: int, D: int, attn: Attention, norm: RMSNorm, mlp: MlpBlock,
         keep.extend((n.weight.detach(), w))
         return w.data_ptr()
 
+    # the native call takes its sizes from D, F and the heads: every kernel it reads has to have just those
+    for m, K, N in ((attn.q_proj, D, a.heads * 128), (attn.k_proj, D, a.kv_heads * 128), (attn.v_proj, D, a.kv_heads * 128), (attn.o_proj, a.heads * 128, D),
+                    (mlp.wi_fused, D, 2 * a.F), (mlp.wo, a.F, D),
+                    *(((cross.q_proj, D, cross.num_query_heads * 128), (cross.o_proj, cross.num_query_heads * 128, D)) if cross is not None else ())):
+        if (math.prod(m.in_shapes), math.prod(m.out_features)) != (K, N):
+            raise NotImplementedError(f"a layer of width {D} on sm_100a has heads of 128 channels: dense kernel {tuple(m.kernel_shape)} where [{K} x {N}] is read")
     a.norm_self, a.norm_mlp = vector(norm), vector(norm_mlp)
     if cross is not None:
         a.cross_heads, a.norm_cross = cross.num_query_heads, vector(norm_cross)

@@ -1,0 +1,88 @@
+"""What the layers of many rows hand to their native call (dia_b200_rows_layer_forward), with the kernels stubbed: what does not fit is refused here,
+because the call takes pointers and sizes as they are."""
+
+import ctypes as C
+
+import pytest
+import torch
+
+from dia_tts_prune_b200 import engine
+from dia_tts_prune_b200.config import DataConfig, DecoderConfig, DiaConfig, EncoderConfig, ModelConfig
+from dia_tts_prune_b200.layers import DecoderLayer, EncoderLayer
+
+
+@pytest.fixture
+def calls(monkeypatch):
+    """The arguments of every native call.  Products of more than 128 rows and 1024 columns read fp16 copies, the others bf16 ones."""
+    made = []
+
+    def kmajor(w, out=None):
+        t = w.detach().t().contiguous().bfloat16()
+        return t if out is None else out.copy_(t)
+
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: False)
+    monkeypatch.setattr(engine, "dense_prepare_weight", kmajor)
+    monkeypatch.setattr(engine, "dense_prepare_half", lambda w, inexact: (w.detach().t().contiguous().half(), w.detach().abs().amax(0).float()))
+    monkeypatch.setattr(engine, "dense_half_rows", lambda M, N, K, device: M > 128 and N > 1024)
+    monkeypatch.setattr(engine, "rows_layer_work_bytes", lambda a: 0)
+    monkeypatch.setattr(engine, "rows_layer_forward", lambda a, n, device: made.append(type(a).from_buffer_copy(a)))
+    return made
+
+
+def config(head_dim=128, cross_head_dim=128, width=256):
+    return DiaConfig(model=ModelConfig(encoder=EncoderConfig(n_layer=1, n_embd=width, n_hidden=512, n_head=4, head_dim=head_dim),
+                                       decoder=DecoderConfig(n_layer=1, n_embd=width, n_hidden=576, gqa_query_heads=4, kv_heads=2, gqa_head_dim=head_dim,
+                                                             cross_query_heads=4, cross_head_dim=cross_head_dim), src_vocab_size=256, tgt_vocab_size=1028),
+                     data=DataConfig(text_length=512, audio_length=2048, channels=9))
+
+
+def filled(layer):
+    with torch.no_grad():
+        for p in layer.parameters():
+            p.copy_(torch.randn(p.shape).bfloat16())
+    return layer
+
+
+def run(layer, T, B=1, k=None, v=None, cross=None, cross_heads=4):
+    """The layer's native call for ``[B, T]`` rows; ``cross``: the (keys, values) of a decoder layer's cross-attention."""
+    from dia_tts_prune_b200.layers import _rows_layer
+    from dia_tts_prune_b200.state import KVCache
+    D = layer.mlp.wi_fused.in_shapes[0]
+    sa = layer.self_attention
+    shape = (B, sa.num_kv_heads, T, 128)
+    tables = (torch.zeros(2049, 64), torch.zeros(2049, 64))
+    pos = torch.arange(T, dtype=torch.int32).repeat(B)
+    ca = None
+    if isinstance(layer, DecoderLayer):
+        ck, cv = cross if cross is not None else (torch.zeros(B, cross_heads, 8, 128), torch.zeros(B, cross_heads, 8, 128))
+        ca = (layer.cross_attention, layer.pre_ca_norm, KVCache.from_kv(ck, cv), [8] * B)
+    norm, norm_mlp = (layer.pre_sa_norm, layer.pre_mlp_norm) if ca else (layer.pre_sa_norm, layer.post_sa_norm)
+    with torch.no_grad():
+        return _rows_layer(layer, torch.randn(B, T, D), sa, norm, layer.mlp, norm_mlp, 1e-5, pos, tables, 0 if ca else 1, None if ca else [T] * B,
+                           torch.zeros(shape) if k is None else k, torch.zeros(shape) if v is None else v, ca)
+
+
+@pytest.mark.parametrize("T", [5, 200])
+@pytest.mark.parametrize("head_dim,cross_head_dim", [(64, 128), (256, 128), (128, 64), (128, 256)])
+def test_heads_of_other_widths_are_refused(calls, head_dim, cross_head_dim, T):
+    """The call reads 128 rows of a copy per head"""
+    cfg = config(head_dim, cross_head_dim)
+    with pytest.raises(NotImplementedError):
+        run(filled(DecoderLayer(cfg, torch.bfloat16)), T)
+    if cross_head_dim == 128:
+        with pytest.raises(NotImplementedError):
+            run(filled(EncoderLayer(cfg, torch.bfloat16)), T)
+    assert not calls
+
+
+def test_kernels_of_another_size_are_refused(calls):
+    layer, wider = filled(EncoderLayer(config(), torch.bfloat16)), filled(EncoderLayer(config(width=320), torch.bfloat16))
+    run(layer, 5)
+    assert len(calls) == 1 and calls[0].heads == 4 and calls[0].D == 256 and calls[0].F == 512
+    for part, name in (("self_attention", "q_proj"), ("self_attention", "o_proj"), ("mlp", "wi_fused"), ("mlp", "wo")):
+        kept = getattr(getattr(layer, part), name)
+        setattr(getattr(layer, part), name, getattr(getattr(wider, part), name))
+        with pytest.raises(NotImplementedError):
+            run(layer, 6)
+        setattr(getattr(layer, part), name, kept)
+    assert len(calls) == 1
