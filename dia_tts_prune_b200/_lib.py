@@ -45,7 +45,7 @@ class DenseRef(C.Structure):
 
 
 class RowsLayer(C.Structure):
-    _fields_ = [(n, C.c_int32) for n in ("B", "T", "D", "F", "heads", "kv_heads", "slots", "mode", "cross_heads", "cross_slots", "n_pos")] + \
+    _fields_ = [(n, C.c_int32) for n in ("B", "T", "D", "F", "heads", "kv_heads", "slots", "mode", "cross_heads", "cross_kv_heads", "cross_slots", "n_pos")] + \
                [("eps", C.c_float), ("n_valid", C.c_int32 * 16), ("cross_valid", C.c_int32 * 16)] + \
                [(n, C.c_void_p) for n in ("x_in", "x", "sin_table", "cos_table", "positions", "norm_self", "norm_cross", "norm_mlp")] + \
                [(n, DenseRef) for n in ("q", "k", "v", "o", "cross_q", "cross_o", "wi", "wo")] + \

@@ -1096,7 +1096,7 @@ int dia_b200_rows_layer_forward(const dia_b200_rows_layer* args, void* stream) {
     if (!a.x_in || !a.x || !a.sin_table || !a.cos_table || !a.positions || !a.k_cache || !a.v_cache || !a.work || !a.norm_self || !a.norm_mlp)
         return DIA_B200_EINVAL;
     const bool cross = a.cross_heads > 0;
-    if (cross && (!a.norm_cross || !a.cross_k || !a.cross_v || a.cross_slots <= 0)) return DIA_B200_EINVAL;
+    if (cross && (!a.norm_cross || !a.cross_k || !a.cross_v || a.cross_slots <= 0 || a.cross_kv_heads <= 0 || a.cross_heads % a.cross_kv_heads)) return DIA_B200_EINVAL;
     const dia_b200_dense_ref* const used[] = {&a.q, &a.k, &a.v, &a.o, &a.wi, &a.wo, &a.cross_q, &a.cross_o};
     uintptr_t bits = 0;
     for (int i = 0; i < (cross ? 8 : 6); ++i) {
@@ -1136,7 +1136,7 @@ int dia_b200_rows_layer_forward(const dia_b200_rows_layer* args, void* stream) {
         if ((rc = rows_dense(a.cross_q, a.x, a.norm_cross, a.eps, false, nullptr, qkv, split, M, nc, D, st))) return rc;
         CK(launch_head_rows(qkv, nc, nullptr, nullptr, 0, q, nullptr, nullptr, a.sin_table, a.cos_table, a.positions, a.B, a.T, a.cross_heads, 0, 0, a.n_pos, st));
         g_launches++;
-        if ((rc = rows_attention(q, a.cross_k, a.cross_v, att, a.B, a.T, a.cross_slots, a.cross_heads, a.cross_heads, a.cross_slots, 2, a.cross_valid, st))) return rc;
+        if ((rc = rows_attention(q, a.cross_k, a.cross_v, att, a.B, a.T, a.cross_slots, a.cross_heads, a.cross_kv_heads, a.cross_slots, 2, a.cross_valid, st))) return rc;
         if ((rc = rows_dense(a.cross_o, att, nullptr, 0.f, false, a.x, a.x, split, M, D, nc, st))) return rc;
     }
     if ((rc = rows_dense(a.wi, a.x, a.norm_mlp, a.eps, false, nullptr, gu, split, M, 2 * a.F, D, st))) return rc;

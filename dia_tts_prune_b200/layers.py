@@ -388,6 +388,15 @@ def _rows_weights(M: int, D: int, attn: Attention, norm: RMSNorm, mlp: MlpBlock,
     return a, copies, keep
 
 
+def _check_caches(name: str, k: Tensor, v: Tensor, B: int, device: torch.device) -> None:
+    """Keys and values as the kernels read them: ``[B, heads, slots, 128]``, float32, contiguous, on the rows' device."""
+    for t in (k, v):
+        if t.dim() != 4 or t.shape[0] != B or t.shape[3] != 128 or t.dtype != torch.float32 or not t.is_contiguous() or t.device != device:
+            raise ValueError(f"{name} cache {tuple(t.shape)} {t.dtype} on {t.device}: contiguous float32 [{B}, heads, slots, 128] on {device} is read")
+    if k.shape != v.shape:
+        raise ValueError(f"{name} cache: keys {tuple(k.shape)}, values {tuple(v.shape)}")
+
+
 def _rows_layer(owner: nn.Module, x: Tensor, attn: Attention, norm: RMSNorm, mlp: MlpBlock, norm_mlp: RMSNorm, eps: float, positions_i32: Tensor, tables,
                 mode: int, n_valid: list[int] | None, k: Tensor, v: Tensor, cross: tuple | None = None, out: Tensor | None = None) -> Tensor:
     """One layer over ``x [B, T, D]`` (float32, contiguous) on our kernels, in one native call: RMSNorm in the split pass of the projections, RoPE with
@@ -402,8 +411,15 @@ def _rows_layer(owner: nn.Module, x: Tensor, attn: Attention, norm: RMSNorm, mlp
     if x.data_ptr() % 16:                                         # (a view of other memory)
         x = x.clone()
     ca, cn, cc, valid = cross if cross is not None else (None, None, None, None)
-    for t in (k, v) if cc is None else (k, v, cc.k, cc.v):
-        assert t.shape[0] == B and t.is_contiguous() and t.dtype == torch.float32 and t.shape[3] == 128
+    _check_caches("self-attention", k, v, B, x.device)
+    if k.shape[1] != attn.num_kv_heads or k.shape[2] < T:
+        raise ValueError(f"self-attention cache {tuple(k.shape)} for {attn.num_kv_heads} key heads and {T} rows")
+    if cc is not None:
+        _check_caches("cross-attention", cc.k, cc.v, B, x.device)
+        if not cc.k.shape[1] or ca.num_query_heads % cc.k.shape[1]:
+            raise ValueError(f"cross-attention cache {tuple(cc.k.shape)} for {ca.num_query_heads} query heads")
+    if positions_i32.numel() < B * T or positions_i32.dtype != torch.int32 or positions_i32.device != x.device:
+        raise ValueError(f"{B * T} int32 positions are read")
     # the layer's arguments are made once per number of rows and set of weight copies (which a kernel drops when it changes)
     norms = (norm.weight, norm_mlp.weight) if ca is None else (norm.weight, norm_mlp.weight, cn.weight)
     key = (B * T, D, eps, *((w.data_ptr(), w._version, w.dtype) for w in norms))
@@ -419,7 +435,7 @@ def _rows_layer(owner: nn.Module, x: Tensor, attn: Attention, norm: RMSNorm, mlp
     if n_valid is not None:
         a.n_valid[:B] = [int(n) for n in n_valid]
     if cc is not None:
-        a.cross_slots, a.cross_k, a.cross_v = cc.k.shape[2], cc.k.data_ptr(), cc.v.data_ptr()
+        a.cross_kv_heads, a.cross_slots, a.cross_k, a.cross_v = cc.k.shape[1], cc.k.shape[2], cc.k.data_ptr(), cc.v.data_ptr()
         a.cross_valid[:B] = [int(n) for n in valid]
     _k.rows_layer_forward(a, _k.rows_layer_work_bytes(a), x.device)
     return y

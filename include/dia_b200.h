@@ -252,7 +252,7 @@ int dia_b200_dense_forward_half(const float *x, const float *norm_weight, float 
  * the entry points around it, in their order.  x_in [B*T][D] is the residual stream, x what it becomes (the same or apart).  The
  * self-attention's keys and values go to slots [0, T) of k_cache / v_cache [B][kv_heads][slots][128], with mode and n_valid as
  * dia_b200_attention_rows has them; cross_heads > 0: cross-attention (mode 2, cross_valid) over cross_k / cross_v
- * [B][cross_heads][cross_slots][128] follows.  Heads have 128 channels.
+ * [B][cross_kv_heads][cross_slots][128] follows (query heads a multiple of cross_kv_heads).  Heads have 128 channels.
  * A weight is its fp16 copy with its magnitudes (dia_b200_dense_prepare_half) or, with wt_half NULL, its bf16 copy; the bf16 copies of q, k and v (or
  * of k and v) may lie one behind the other and are then one product.  All pointers 16-byte aligned, norms excepted. */
 typedef struct dia_b200_dense_ref {
@@ -263,7 +263,7 @@ typedef struct dia_b200_dense_ref {
 typedef struct dia_b200_rows_layer {
     int32_t B, T, D, F;
     int32_t heads, kv_heads, slots, mode;
-    int32_t cross_heads, cross_slots, n_pos;
+    int32_t cross_heads, cross_kv_heads, cross_slots, n_pos;
     float eps;
     int32_t n_valid[16], cross_valid[16];
     const float *x_in;

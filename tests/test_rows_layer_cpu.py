@@ -86,3 +86,25 @@ def test_kernels_of_another_size_are_refused(calls):
             run(layer, 6)
         setattr(getattr(layer, part), name, kept)
     assert len(calls) == 1
+
+
+def test_heads_of_the_caches(calls):
+    """The self-attention's cache has the layer's key heads; the cross-attention reads as many as its cache has, where they divide its query heads"""
+    layer = filled(DecoderLayer(config(), torch.bfloat16))
+    for heads in (1, 2, 4):
+        run(layer, 5, cross_heads=heads)
+        assert calls[-1].cross_heads == 4 and calls[-1].cross_kv_heads == heads
+    n = len(calls)
+    good = torch.zeros(1, 2, 7, 128)
+    for bad in (torch.zeros(1, 1, 7, 128), torch.zeros(1, 4, 7, 128), torch.zeros(1, 2, 4, 128), torch.zeros(2, 2, 7, 128), torch.zeros(1, 2, 7, 64),
+                good.double(), torch.zeros(1, 2, 128, 7).transpose(2, 3)):
+        with pytest.raises(ValueError):
+            run(layer, 5, k=bad, v=bad)
+    with pytest.raises(ValueError):
+        run(layer, 5, k=good, v=torch.zeros(1, 2, 9, 128))
+    for ck, cv in ((3, 3), (4, 2), (8, 8)):
+        with pytest.raises(ValueError):
+            run(layer, 5, cross=(torch.zeros(1, ck, 8, 128), torch.zeros(1, cv, 8, 128)))
+    assert len(calls) == n
+    run(layer, 5, k=good, v=good.clone())
+    assert calls[-1].slots == 7
