@@ -461,6 +461,8 @@ def dense_prepare_half(w_KxN: torch.Tensor, inexact: torch.Tensor) -> tuple[torc
     """K-major fp16 copy ``[N, K]`` of a DenseGeneral kernel, a power of two per column, and the columns' largest magnitudes ``[N]``.
     ``inexact`` (int32, one element on the device) is set where fp16 cannot hold the bf16 values."""
     lib = _lib.load()
+    if not w_KxN.is_cuda or w_KxN.dim() != 2 or w_KxN.dtype not in (torch.float32, torch.bfloat16):
+        raise ValueError("expected a 2-D float32 / bfloat16 CUDA tensor")
     w = w_KxN.contiguous()
     K, N = w.shape
     wt = torch.empty((N, K), dtype=torch.float16, device=w.device)
@@ -477,6 +479,15 @@ def dense_forward_half(x: torch.Tensor, half: tuple[torch.Tensor, torch.Tensor],
     wt, mag = half
     N, K = wt.shape
     M = x.shape[0]
+    # (the kernels read what they are told to: float32 rows, norms of K numbers)
+    if x.dtype != torch.float32 or not x.is_contiguous() or x.numel() != M * K * (2 if gated else 1):
+        raise ValueError(f"x must be contiguous float32 {'[M, 2, K]' if gated else '[M, K]'} with K = {K}")
+    if norm_weight is not None and (gated or norm_weight.numel() != K):
+        raise ValueError("norm weight length must equal K")
+    if norm_weight is not None and (norm_weight.dtype != torch.float32 or not norm_weight.is_contiguous()):
+        raise ValueError("norm weight must be contiguous float32")
+    if residual is not None and (residual.dtype != torch.float32 or not residual.is_contiguous() or tuple(residual.shape) != (M, N)):
+        raise ValueError("residual must be a contiguous float32 [M, N] tensor")
     y = residual if residual is not None else torch.empty((M, N), dtype=torch.float32, device=x.device)
     ws = torch.empty((int(lib.dia_b200_dense_workspace_bytes(M, K)),), dtype=torch.uint8, device=x.device)
     _lib.check(lib.dia_b200_dense_forward_half(_ptr(x), _ptr(norm_weight) if norm_weight is not None else None, float(eps), int(gated), _ptr(wt),
