@@ -42,6 +42,7 @@ except Exception:  # pragma: no cover - hub not installed
         def __init_subclass__(cls, **kw):
             super().__init_subclass__()
 
+from ._lib import RowsLayer
 from .config import DiaConfig
 from .state import DecoderInferenceState, EncoderInferenceState, KVCache
 
@@ -108,25 +109,19 @@ class DenseGeneral(nn.Module):
     # ---- sm_100a path (encoder, cross-attention K/V precompute, prompt prefill) ----------------------------------
     def kernel_weight_kmajor(self) -> Tensor:
         """The K-major bf16 copy ``[N, K]`` of the kernel the tcgen05 GEMM reads (made once per weight version)."""
-        from . import engine as _engine
-        w = self.weight
-        K, N = math.prod(self.in_shapes), math.prod(self.out_features)
-        key = (w.data_ptr(), w._version, w.dtype, w.device)
-        cached = getattr(self, "_b200_wt", None)
-        if cached is None or cached[0] != key:
+        cached = self.__dict__.get("_b200_wt")
+        if cached is None or cached[0] != self._weight_key():
+            from . import engine as _engine
             canonicalize_dense_kernel_(self)
-            w = self.weight
-            key = (w.data_ptr(), w._version, w.dtype, w.device)
-            cached = (key, _engine.dense_prepare_weight(w.detach().reshape(K, N)))
-            self._b200_wt = cached
+            wt = _engine.dense_prepare_weight(self.weight.detach().reshape(math.prod(self.in_shapes), math.prod(self.out_features)))
+            cached = self._b200_wt = (self._weight_key(), wt)
         return cached[1]
 
     def kernel_weight_half(self) -> tuple[Tensor, Tensor] | None:
         """The fp16 copy that products of many rows read (made once per weight version), or None: fp16 cannot hold these weights, or the
         stream is being captured and there is no copy yet."""
-        key = self._weight_key()
         cached = self.__dict__.get("_b200_half")
-        if cached is None or cached[0] != key:
+        if cached is None or cached[0] != self._weight_key():
             if torch.cuda.is_current_stream_capturing():
                 return None
             prepare_half_kernels([self])
@@ -327,6 +322,8 @@ def _stack_kmajor(modules: list["DenseGeneral"]) -> None:
         at = [h[1].data_ptr() for h in have]
         if all(b - a == 2 * h[1].numel() for a, b, h in zip(at, at[1:], have)) or torch.cuda.is_current_stream_capturing():
             return
+    if len({math.prod(m.in_shapes) for m in modules}) > 1:        # (not products of the same rows)
+        return
     for m in modules:
         canonicalize_dense_kernel_(m)
     K, sizes = math.prod(modules[0].in_shapes), [math.prod(m.out_features) for m in modules]
@@ -335,57 +332,50 @@ def _stack_kmajor(modules: list["DenseGeneral"]) -> None:
         m._b200_wt = (m._weight_key(), _engine.dense_prepare_weight(m.weight.detach().reshape(K, out.shape[0]), out))
 
 
-# Layer -> (key, arguments, copies, norms) of its last native call.  Not an attribute: a copied or unpickled layer starts without one.
-_ROWS: "weakref.WeakKeyDictionary[nn.Module, tuple]" = weakref.WeakKeyDictionary()
-
-
-def _rows_weights(M: int, D: int, attn: Attention, norm: RMSNorm, mlp: MlpBlock, norm_mlp: RMSNorm, eps: float, cross: Attention | None,
-                  norm_cross: RMSNorm | None, device):
-    """What a native layer call of ``M`` rows reads of the layer: the arguments, the copies of its weights that they point at, and its norms."""
+def _rows_weights(a, M: int, attn: Attention, norm: RMSNorm, mlp: MlpBlock, norm_mlp: RMSNorm, cross: Attention | None, norm_cross: RMSNorm | None,
+                  device) -> list:
+    """Points the arguments of a native layer call of ``M`` rows at the layer's weights.  Returns what has to live until the call has been made.
+    Nothing is kept from one call for the next but the copies that the kernels hold themselves: arguments kept per layer held copies that their
+    kernels had dropped, and were made anew for every other number of rows (host time of a layer's
+    arguments, us: 35 for any number of rows; kept ones 17 for the last number and 62 for another)."""
     from . import engine as _k
-    from ._lib import DenseRef, RowsLayer
-    keep, copies = [], []
-    a = RowsLayer(D=D, F=mlp.wo.in_shapes[0], heads=attn.num_query_heads, kv_heads=attn.num_kv_heads, eps=eps)
-
-    def vector(n: RMSNorm) -> int:
-        w = n.weight.detach().to(torch.float32).contiguous()
+    D, keep = a.D, []
+    F, H, Hk = mlp.wo.in_shapes[0], attn.num_query_heads, attn.num_kv_heads
+    a.F, a.heads, a.kv_heads = F, H, Hk
+    parts = [("q", attn.q_proj, D, H * 128), ("k", attn.k_proj, D, Hk * 128), ("v", attn.v_proj, D, Hk * 128), ("o", attn.o_proj, H * 128, D),
+             ("wi", mlp.wi_fused, D, 2 * F), ("wo", mlp.wo, F, D)]
+    norms = [("norm_self", norm), ("norm_mlp", norm_mlp)]
+    if cross is not None:
+        Hc = a.cross_heads = cross.num_query_heads
+        parts += [("cross_q", cross.q_proj, D, Hc * 128), ("cross_o", cross.o_proj, Hc * 128, D)]
+        norms.append(("norm_cross", norm_cross))
+    for name, n in norms:
+        w = n.weight
         if w.numel() != D:
             raise ValueError("norm weight length must equal K")
-        keep.extend((n.weight.detach(), w))
-        return w.data_ptr()
-
-    # the native call takes its sizes from D, F and the heads: every kernel it reads has to have just those
-    for m, K, N in ((attn.q_proj, D, a.heads * 128), (attn.k_proj, D, a.kv_heads * 128), (attn.v_proj, D, a.kv_heads * 128), (attn.o_proj, a.heads * 128, D),
-                    (mlp.wi_fused, D, 2 * a.F), (mlp.wo, a.F, D),
-                    *(((cross.q_proj, D, cross.num_query_heads * 128), (cross.o_proj, cross.num_query_heads * 128, D)) if cross is not None else ())):
-        if (math.prod(m.in_shapes), math.prod(m.out_features)) != (K, N):
-            raise NotImplementedError(f"a layer of width {D} on sm_100a has heads of 128 channels: dense kernel {tuple(m.kernel_shape)} where [{K} x {N}] is read")
-    a.norm_self, a.norm_mlp = vector(norm), vector(norm_mlp)
-    if cross is not None:
-        a.cross_heads, a.norm_cross = cross.num_query_heads, vector(norm_cross)
-
-    def half(m: DenseGeneral):                                    # the product's rows go as two fp16 terms
-        K, N = math.prod(m.in_shapes), math.prod(m.out_features)
+        if w.dtype != torch.float32 or not w.is_contiguous():
+            w = w.detach().to(torch.float32).contiguous()
+        keep.append(w)
+        setattr(a, name, w.data_ptr())
+    halves = []
+    for _, m, K, N in parts:
         if not _k.dense_supported(M, N, K):
             raise NotImplementedError(f"dense layer [{M} x {K}] . [{K} x {N}] does not fit the tcgen05 tiling (K must be a multiple of 64, N of 4)")
-        return m.kernel_weight_half() if _k.dense_half_rows(M, N, K, device) else None
-
-    def ref(m: DenseGeneral) -> DenseRef:
-        h = half(m)
+        halves.append(m.kernel_weight_half() if _k.dense_half_rows(M, N, K, device) else None)      # (the product's rows go as two fp16 terms)
+    if halves[1] is None and halves[2] is None:
+        _stack_kmajor([m for _, m, _, _ in parts[0 if halves[0] is None else 1:3]])
+    for (name, m, K, N), h in zip(parts, halves):
+        wt = m.kernel_weight_kmajor() if h is None else h[0]
+        if wt.shape != (N, K):                                    # the native call takes its sizes from D, F and the heads
+            raise NotImplementedError(f"a layer of width {D} on sm_100a has heads of 128 channels: dense kernel {tuple(m.kernel_shape)} where [{K} x {N}] is read")
+        keep.append(wt)
+        r = getattr(a, name)
         if h is None:
-            m.kernel_weight_kmajor()
-        name = "_b200_wt" if h is None else "_b200_half"
-        copies.append((m, name, m.__dict__[name]))
-        return DenseRef(wt_bf16=copies[-1][2][1].data_ptr()) if h is None else DenseRef(wt_half=h[0].data_ptr(), magnitudes=h[1].data_ptr())
-
-    kv = [attn.k_proj, attn.v_proj]
-    if all(half(m) is None for m in kv):
-        _stack_kmajor(kv if half(attn.q_proj) is not None else [attn.q_proj, *kv])
-    a.q, a.k, a.v, a.o = ref(attn.q_proj), ref(attn.k_proj), ref(attn.v_proj), ref(attn.o_proj)
-    if cross is not None:
-        a.cross_q, a.cross_o = ref(cross.q_proj), ref(cross.o_proj)
-    a.wi, a.wo = ref(mlp.wi_fused), ref(mlp.wo)
-    return a, copies, keep
+            r.wt_bf16 = wt.data_ptr()
+        else:
+            r.wt_half, r.magnitudes = wt.data_ptr(), h[1].data_ptr()
+            keep.append(h)
+    return keep
 
 
 def _check_caches(name: str, k: Tensor, v: Tensor, B: int, device: torch.device) -> None:
@@ -397,7 +387,7 @@ def _check_caches(name: str, k: Tensor, v: Tensor, B: int, device: torch.device)
         raise ValueError(f"{name} cache: keys {tuple(k.shape)}, values {tuple(v.shape)}")
 
 
-def _rows_layer(owner: nn.Module, x: Tensor, attn: Attention, norm: RMSNorm, mlp: MlpBlock, norm_mlp: RMSNorm, eps: float, positions_i32: Tensor, tables,
+def _rows_layer(x: Tensor, attn: Attention, norm: RMSNorm, mlp: MlpBlock, norm_mlp: RMSNorm, eps: float, positions_i32: Tensor, tables,
                 mode: int, n_valid: list[int] | None, k: Tensor, v: Tensor, cross: tuple | None = None, out: Tensor | None = None) -> Tensor:
     """One layer over ``x [B, T, D]`` (float32, contiguous) on our kernels, in one native call: RMSNorm in the split pass of the projections, RoPE with
     the scatter into the caches ``k``, ``v [B, heads, slots, 128]``, attention, residual adds in the epilogues, the gate in the split pass of
@@ -420,15 +410,8 @@ def _rows_layer(owner: nn.Module, x: Tensor, attn: Attention, norm: RMSNorm, mlp
             raise ValueError(f"cross-attention cache {tuple(cc.k.shape)} for {ca.num_query_heads} query heads")
     if positions_i32.numel() < B * T or positions_i32.dtype != torch.int32 or positions_i32.device != x.device:
         raise ValueError(f"{B * T} int32 positions are read")
-    # the layer's arguments are made once per number of rows and set of weight copies (which a kernel drops when it changes)
-    norms = (norm.weight, norm_mlp.weight) if ca is None else (norm.weight, norm_mlp.weight, cn.weight)
-    key = (B * T, D, eps, *((w.data_ptr(), w._version, w.dtype) for w in norms))
-    made = _ROWS.get(owner)
-    if made is None or made[0] != key or any(m.__dict__.get(name) is not c or c[0] != m._weight_key() for m, name, c in made[2]):
-        made = (key, *_rows_weights(B * T, D, attn, norm, mlp, norm_mlp, eps, ca, cn, x.device))
-        if not torch.cuda.is_current_stream_capturing():          # (a capture may have to do without the fp16 copies)
-            _ROWS[owner] = made
-    a = type(made[1]).from_buffer_copy(made[1])
+    a = RowsLayer(D=D, eps=eps)
+    keep = _rows_weights(a, B * T, attn, norm, mlp, norm_mlp, ca, cn, x.device)
     a.B, a.T, a.slots, a.mode, a.n_pos = B, T, k.shape[2], mode, tables[0].shape[0]
     a.x_in, a.x, a.positions = x.data_ptr(), y.data_ptr(), positions_i32.data_ptr()
     a.sin_table, a.cos_table, a.k_cache, a.v_cache = tables[0].data_ptr(), tables[1].data_ptr(), k.data_ptr(), v.data_ptr()
@@ -438,6 +421,7 @@ def _rows_layer(owner: nn.Module, x: Tensor, attn: Attention, norm: RMSNorm, mlp
         a.cross_kv_heads, a.cross_slots, a.cross_k, a.cross_v = cc.k.shape[1], cc.k.shape[2], cc.k.data_ptr(), cc.v.data_ptr()
         a.cross_valid[:B] = [int(n) for n in valid]
     _k.rows_layer_forward(a, _k.rows_layer_work_bytes(a), x.device)
+    del keep
     return y
 
 
@@ -462,7 +446,7 @@ class EncoderLayer(nn.Module):
             if pos is None or pos.numel() != B * T:
                 pos = state.extras["pos_i32"] = _k.positions_i32(T, B, x.device)
             kv = torch.empty((2, B, self.self_attention.num_kv_heads, T, 128), dtype=torch.float32, device=x.device)
-            return _rows_layer(self, x, self.self_attention, self.pre_sa_norm, self.mlp, self.post_sa_norm, eps, pos,
+            return _rows_layer(x, self.self_attention, self.pre_sa_norm, self.mlp, self.post_sa_norm, eps, pos,
                                _k.rope_tables_device(self.config, x.device), 1, _encoder_valid_lens(state), kv[0], kv[1])
         h = self.pre_sa_norm(x.float())
         x = x + self.self_attention(h, h, state.positions, state.positions, attn_mask=state.attn_mask)
@@ -565,7 +549,7 @@ class DecoderLayer(nn.Module):
                 k, v = torch.empty((2, B, self.self_attention.num_kv_heads, T, 128), dtype=torch.float32, device=x.device)
             if cross_attn_cache is None:
                 raise NotImplementedError("cross-attention needs the precomputed K/V cache")
-            return _rows_layer(self, x, self.self_attention, self.pre_sa_norm, self.mlp, self.pre_mlp_norm, eps, pos, tables, 0, None, k, v,
+            return _rows_layer(x, self.self_attention, self.pre_sa_norm, self.mlp, self.pre_mlp_norm, eps, pos, tables, 0, None, k, v,
                                (self.cross_attention, self.pre_ca_norm, cross_attn_cache, [0] * (B - 1) + [state.text_len]),
                                out=x if x.data_ptr() % 16 == 0 else None)
         # CPU (state-dict tooling and the CPU test suite): the reference's own formulation

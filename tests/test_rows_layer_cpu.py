@@ -47,7 +47,7 @@ def run(layer, T, B=1, k=None, v=None, cross=None, cross_heads=4):
     """The layer's native call for ``[B, T]`` rows; ``cross``: the (keys, values) of a decoder layer's cross-attention."""
     from dia_tts_prune_b200.layers import _rows_layer
     from dia_tts_prune_b200.state import KVCache
-    D = layer.mlp.wi_fused.in_shapes[0]
+    D = layer.pre_sa_norm.weight.numel()
     sa = layer.self_attention
     shape = (B, sa.num_kv_heads, T, 128)
     tables = (torch.zeros(2049, 64), torch.zeros(2049, 64))
@@ -58,7 +58,7 @@ def run(layer, T, B=1, k=None, v=None, cross=None, cross_heads=4):
         ca = (layer.cross_attention, layer.pre_ca_norm, KVCache.from_kv(ck, cv), [8] * B)
     norm, norm_mlp = (layer.pre_sa_norm, layer.pre_mlp_norm) if ca else (layer.pre_sa_norm, layer.post_sa_norm)
     with torch.no_grad():
-        return _rows_layer(layer, torch.randn(B, T, D), sa, norm, layer.mlp, norm_mlp, 1e-5, pos, tables, 0 if ca else 1, None if ca else [T] * B,
+        return _rows_layer(torch.randn(B, T, D), sa, norm, layer.mlp, norm_mlp, 1e-5, pos, tables, 0 if ca else 1, None if ca else [T] * B,
                            torch.zeros(shape) if k is None else k, torch.zeros(shape) if v is None else v, ca)
 
 
@@ -108,3 +108,48 @@ def test_heads_of_the_caches(calls):
     assert len(calls) == n
     run(layer, 5, k=good, v=good.clone())
     assert calls[-1].slots == 7
+
+
+def copies(layer):
+    import weakref
+    return [weakref.ref(t) for m in layer.modules() for name in ("_b200_wt", "_b200_half") if name in m.__dict__
+            for t in (m.__dict__[name][1] if name == "_b200_half" else m.__dict__[name][1:])]
+
+
+@pytest.mark.parametrize("T", [5, 200])
+def test_dropped_copies_are_freed(calls, T):
+    """Copies of weights that were moved or replaced go with them: the layer holds none by another way"""
+    layer = filled(EncoderLayer(config(width=1280), torch.bfloat16))
+    run(layer, T)
+    old = copies(layer)
+    assert len(old) >= 6
+    layer.to(torch.float32)
+    assert not any(r() is not None for r in old)
+    run(layer, T)
+    old = copies(layer)
+    layer.mlp.wo.weight = torch.nn.Parameter(layer.mlp.wo.weight.detach().clone())
+    assert sum(r() is None for r in old) == (1 if T == 5 else 2)
+
+
+def test_a_replaced_part_is_read(calls):
+    """Another kernel, attention or MLP in the layer's place of one: its copies are read, not those of the one before"""
+    layer, other = filled(EncoderLayer(config(), torch.bfloat16)), filled(EncoderLayer(config(), torch.bfloat16))
+    run(layer, 5)
+    layer.mlp.wo = other.mlp.wo
+    run(layer, 5)
+    assert calls[-1].wo.wt_bf16 == other.mlp.wo.kernel_weight_kmajor().data_ptr() != calls[0].wo.wt_bf16
+    layer.self_attention = other.self_attention
+    run(layer, 5)
+    assert calls[-1].o.wt_bf16 == other.self_attention.o_proj.kernel_weight_kmajor().data_ptr() != calls[0].o.wt_bf16
+
+
+def test_numbers_of_rows_share_their_arguments(calls, monkeypatch):
+    """Texts of different lengths read the same copies: none is made anew"""
+    layer = filled(EncoderLayer(config(), torch.bfloat16))
+    run(layer, 40)
+    monkeypatch.setattr(engine, "dense_prepare_weight", None)
+    for T in (41, 7, 99, 40):
+        run(layer, T)
+        for name in ("q", "k", "v", "o", "wi", "wo"):
+            assert getattr(calls[-1], name).wt_bf16 == getattr(calls[0], name).wt_bf16
+        assert calls[-1].T == T and calls[-1].norm_self == calls[0].norm_self

@@ -81,7 +81,7 @@ def test_encoder_layer(T, valid):
     with torch.inference_mode():
         kept = x.clone()
         got, again = layer(x, text_state(T, valid)), layer(x, text_state(T, valid))
-    assert torch.equal(x, kept) and torch.equal(got, again)       # the input stays, and the arguments of the first call serve the second
+    assert torch.equal(x, kept) and torch.equal(got, again)       # the input stays
     assert (got[0] - want).norm() <= 4e-6 * want.norm()           # a few roundings of fp32 per sum and layer part
 
 
