@@ -315,15 +315,11 @@ class Attention(nn.Module):
 
 
 def _stack_kmajor(modules: list["DenseGeneral"]) -> None:
-    """The K-major copies of these kernels, one behind the other: products of the same rows are then one product."""
-    from . import engine as _engine
-    have = [m.__dict__.get("_b200_wt") for m in modules]
-    if all(h is not None and h[0] == m._weight_key() for h, m in zip(have, modules)):
-        at = [h[1].data_ptr() for h in have]
-        if all(b - a == 2 * h[1].numel() for a, b, h in zip(at, at[1:], have)) or torch.cuda.is_current_stream_capturing():
-            return
-    if len({math.prod(m.in_shapes) for m in modules}) > 1:        # (not products of the same rows)
+    """K-major copies of these kernels, one behind the other (products of the same rows may then be one product), where none of them has one yet:
+    a copy that is there may be read by another stream or a captured graph, and stays while its weights do."""
+    if any((c := m.__dict__.get("_b200_wt")) is not None and c[0] == m._weight_key() for m in modules) or len({math.prod(m.in_shapes) for m in modules}) > 1:
         return
+    from . import engine as _engine
     for m in modules:
         canonicalize_dense_kernel_(m)
     K, sizes = math.prod(modules[0].in_shapes), [math.prod(m.out_features) for m in modules]
@@ -362,8 +358,8 @@ def _rows_weights(a, M: int, attn: Attention, norm: RMSNorm, mlp: MlpBlock, norm
         if not _k.dense_supported(M, N, K):
             raise NotImplementedError(f"dense layer [{M} x {K}] . [{K} x {N}] does not fit the tcgen05 tiling (K must be a multiple of 64, N of 4)")
         halves.append(m.kernel_weight_half() if _k.dense_half_rows(M, N, K, device) else None)      # (the product's rows go as two fp16 terms)
-    if halves[1] is None and halves[2] is None:
-        _stack_kmajor([m for _, m, _, _ in parts[0 if halves[0] is None else 1:3]])
+    if None in halves[:3]:
+        _stack_kmajor([m for _, m, _, _ in parts[:3]])            # (all three, whichever of them these rows read)
     for (name, m, K, N), h in zip(parts, halves):
         wt = m.kernel_weight_kmajor() if h is None else h[0]
         if wt.shape != (N, K):                                    # the native call takes its sizes from D, F and the heads

@@ -153,3 +153,25 @@ def test_numbers_of_rows_share_their_arguments(calls, monkeypatch):
         for name in ("q", "k", "v", "o", "wi", "wo"):
             assert getattr(calls[-1], name).wt_bf16 == getattr(calls[0], name).wt_bf16
         assert calls[-1].T == T and calls[-1].norm_self == calls[0].norm_self
+
+
+def test_copies_that_are_there_stay(calls):
+    """Calls of many rows and of few read different kinds of copies; neither replaces one that another stream or a captured graph may be reading"""
+    layer = filled(DecoderLayer(DiaConfig(model=ModelConfig(
+        encoder=EncoderConfig(n_layer=1, n_embd=256, n_hidden=512, n_head=4, head_dim=128),
+        decoder=DecoderConfig(n_layer=1, n_embd=256, n_hidden=576, gqa_query_heads=12, kv_heads=2, gqa_head_dim=128, cross_query_heads=4, cross_head_dim=128),
+        src_vocab_size=256, tgt_vocab_size=1028), data=DataConfig(text_length=512, audio_length=2048, channels=9)), torch.bfloat16))
+    sa = layer.self_attention
+    run(layer, 200)                                               # (1536 columns of q: an fp16 copy; k and v bf16 ones)
+    assert calls[-1].q.wt_half and not calls[-1].q.wt_bf16 and calls[-1].k.wt_bf16
+    kept = [m.kernel_weight_kmajor() for m in (sa.q_proj, sa.k_proj, sa.v_proj)] + [sa.q_proj.kernel_weight_half()[0]]
+    for T in (5, 200, 7, 300):
+        run(layer, T)
+        assert all(a is b for a, b in zip(kept, [m.kernel_weight_kmajor() for m in (sa.q_proj, sa.k_proj, sa.v_proj)] + [sa.q_proj.kernel_weight_half()[0]]))
+    q, k, v = (calls[-2].q.wt_bf16, calls[-2].k.wt_bf16, calls[-2].v.wt_bf16)
+    assert k - q == 2 * 1536 * 256 and v - k == 2 * 256 * 256     # one behind the other
+    layer = filled(EncoderLayer(config(), torch.bfloat16))
+    sa = layer.self_attention
+    kept = [sa.k_proj.kernel_weight_kmajor()]                     # (the product was called by itself before)
+    run(layer, 5)
+    assert sa.k_proj.kernel_weight_kmajor() is kept[0] and calls[-1].k.wt_bf16 == kept[0].data_ptr()
