@@ -1064,9 +1064,9 @@ RowsRoom rows_room(const dia_b200_rows_layer& a) {
 }
 
 int rows_dense(const dia_b200_dense_ref& w, const float* x, const float* norm, float eps, bool gated, const float* residual, float* y, void* work,
-               int M, int N, int K, cudaStream_t st) {
+               int M, int N, int K, cudaStream_t st, bool sums = false) {
     const cudaError_t e = w.wt_half ? launch_gemm_half(x, norm, eps, gated, w.wt_half, w.magnitudes, residual, y, work, M, N, K, st)
-                                    : launch_gemm_tcgen05(x, norm, eps, gated, w.wt_bf16, residual, y, work, M, N, K, st);
+                                    : launch_gemm_tcgen05(x, norm, eps, gated, w.wt_bf16, residual, y, work, M, N, K, st, sums);
     if (e == cudaErrorNotSupported) { (void)cudaGetLastError(); return DIA_B200_EUNSUPPORTED; }
     CK(e);
     g_launches += 1 + std::exchange(extra_launches(), 0);
@@ -1117,15 +1117,22 @@ int dia_b200_rows_layer_forward(const dia_b200_rows_layer* args, void* stream) {
     void* const split = work + room.split;
     const int M = a.B * a.T, nq = a.heads * 128, nk = a.kv_heads * 128, D = a.D;
     int rc;
-    // projections whose K-major copies lie one behind the other are one product
+    // Projections whose K-major copies lie one behind the other may be one product, summed as they would be by themselves: a stacked product has
+    // so many columns that it would leave the kernel of fp32 sums earlier (768 encoder rows, D = 1024, 3 x 2048 columns: relative error of the values
+    // 1.5e-7, and 7e-6 on the kernel that its columns ask for).  The split that ends first, at seven k-blocks for a launch and its split of the rows.
     auto follows = [&](const dia_b200_dense_ref& u, const dia_b200_dense_ref& w, int n) {
         return !u.wt_half && !w.wt_half && static_cast<const unsigned char*>(u.wt_bf16) + (size_t)n * D * 2 == w.wt_bf16;
     };
-    const bool kv = follows(a.k, a.v, nk), all = kv && follows(a.q, a.k, nq);
+    constexpr int kStart = 7;
+    const bool kv_next = follows(a.k, a.v, nk), all_next = kv_next && follows(a.q, a.k, nq);
+    const int bq = a.q.wt_half ? 0 : gemm_sums_blocks(M, nq, D, false), bk = a.k.wt_half ? 0 : gemm_sums_blocks(M, nk, D, false);      // (0: other sums)
+    const int b_kv = gemm_sums_blocks(M, 2 * nk, D, true), apart = bk ? std::min(b_kv + kStart, 2 * (bk + kStart)) : 0;
+    const bool all = all_next && (bq != 0) == (bk != 0) && (!bq || gemm_sums_blocks(M, nq + 2 * nk, D, true) + kStart <= bq + kStart + apart);
+    const bool kv = all || (kv_next && (!bk || b_kv + kStart <= 2 * (bk + kStart)));
     float *k = all ? qkv + nq : qkv + (size_t)M * nq, *v = all || kv ? k + nk : k + (size_t)M * nk;
     const int ldq = all ? nq + 2 * nk : nq, ldkv = all ? ldq : kv ? 2 * nk : nk;
-    if ((rc = rows_dense(a.q, a.x_in, a.norm_self, a.eps, false, nullptr, qkv, split, M, ldq, D, st))) return rc;
-    if (!all && (rc = rows_dense(a.k, a.x_in, a.norm_self, a.eps, false, nullptr, k, split, M, ldkv, D, st))) return rc;
+    if ((rc = rows_dense(a.q, a.x_in, a.norm_self, a.eps, false, nullptr, qkv, split, M, ldq, D, st, bq != 0))) return rc;
+    if (!all && (rc = rows_dense(a.k, a.x_in, a.norm_self, a.eps, false, nullptr, k, split, M, ldkv, D, st, bk != 0))) return rc;
     if (!kv && (rc = rows_dense(a.v, a.x_in, a.norm_self, a.eps, false, nullptr, v, split, M, nk, D, st))) return rc;
     CK(launch_head_rows(qkv, ldq, k, v, ldkv, q, a.k_cache, a.v_cache, a.sin_table, a.cos_table, a.positions, a.B, a.T, a.heads, a.kv_heads, a.slots, a.n_pos, st));
     g_launches++;

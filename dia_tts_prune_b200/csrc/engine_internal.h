@@ -285,11 +285,12 @@ size_t gemm_workspace_bytes(int M, int K);
 cudaError_t launch_transpose_to_bf16(const void* w, int src_bf16, void* wt, int K, int N, cudaStream_t st);
 // y = (residual ? residual : 0) + (norm_w ? rmsnorm(x; norm_w, eps) : x) . W        (y may alias residual)
 bool gemm_half_ok(int M, int N, int K);
+int gemm_sums_blocks(int M, int N, int K, bool always);
 cudaError_t launch_prepare_half(const void* w, int src_bf16, void* wt, float* mag, int* inexact, int K, int N, cudaStream_t st);
 cudaError_t launch_gemm_half(const float* x, const float* norm_w, float eps, bool gated, const void* wt, const float* mag, const float* residual, float* y,
                              void* workspace, int M, int N, int K, cudaStream_t st);
 cudaError_t launch_gemm_tcgen05(const float* x, const float* norm_w, float eps, bool gated, const void* wt, const float* residual,
-                                float* y, void* workspace, int M, int N, int K, cudaStream_t st);
+                                float* y, void* workspace, int M, int N, int K, cudaStream_t st, bool sums = false);
 
 // the rest of the T > 1 passes (prefill_kernels.cu)
 cudaError_t launch_attention_rows(const float* q, const float* k, const float* v, float* out, int B, int Tq, int Tk, int Hq,

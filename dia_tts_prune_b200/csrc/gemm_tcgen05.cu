@@ -1505,6 +1505,15 @@ bool gemm_half_ok(int M, int N, int K) {
     return !dense_rows_f32(kTerms, M, N, K, sms, 0);
 }
 
+// k-blocks that the fp32-sum kernel takes for M fp32 rows, one after the other, or 0 where launch_gemm_tcgen05 does not sum them in fp32 by itself
+int gemm_sums_blocks(int M, int N, int K, bool always) {
+    int dev = 0, sms = 0;
+    if (dense_rows_few(M)) return 1;
+    if (current_sms(&dev, &sms) != cudaSuccess || (!always && !dense_rows_f32(kTerms, M, N, K, sms, 0))) return 0;
+    const int tiles = (M + BM - 1) / BM * ((N + kFN - 1) / kFN), n_kb = (K + BK - 1) / BK, s = tiles < sms ? f32_splits(tiles, n_kb, 8, sms) : 1;
+    return (tiles * s + sms - 1) / sms * ((n_kb + s - 1) / s);
+}
+
 cudaError_t launch_prepare_half(const void* w, int src_bf16, void* wt, float* mag, int* inexact, int K, int N, cudaStream_t st) {
     const cudaError_t e = cudaMemsetAsync(mag, 0, (size_t)N * 4, st);
     if (e != cudaSuccess) return e;
@@ -1541,9 +1550,9 @@ cudaError_t launch_gemm_half(const float* x, const float* norm_w, float eps, boo
 }
 
 // fp32 activations: the three-term split (with the row's RMSNorm in front when norm_w is given, or with the gate of [M][2][K] rows), then
-// the kernel
+// the kernel; sums: the one of fp32 sums, whatever is the faster one
 cudaError_t launch_gemm_tcgen05(const float* x, const float* norm_w, float eps, bool gated, const void* wt, const float* residual,
-                                float* y, void* workspace, int M, int N, int K, cudaStream_t st) {
+                                float* y, void* workspace, int M, int N, int K, cudaStream_t st, bool sums) {
     if (M <= 0 || N % 4 || N <= 0 || K % BK || K < BK || (gated && norm_w)) return cudaErrorNotSupported;
     const long long n = (long long)M * K;
     FewRowsProduct few{x, K, wt, y, N, M, N, K, 0, residual};
@@ -1566,7 +1575,7 @@ cudaError_t launch_gemm_tcgen05(const float* x, const float* norm_w, float eps, 
     int dev = 0, sms = 0;
     const cudaError_t e = current_sms(&dev, &sms);
     if (e != cudaSuccess) return e;
-    if (dense_rows_f32(kTerms, M, N, K, sms, 0) && gemm_f32_ok(wide)) return run_gemm_f32(wide, workspace, kTerms, 8, st);
+    if ((sums || dense_rows_f32(kTerms, M, N, K, sms, 0)) && gemm_f32_ok(wide)) return run_gemm_f32(wide, workspace, kTerms, 8, st);
     const GemmEpilogue ep{residual, nullptr, nullptr, 0.f, nullptr};
     return launch_gemm_tcgen05_bf16(workspace, kTerms, wt, N, y, M, N, K, ep, nullptr, st);
 }

@@ -60,7 +60,7 @@ def encode(layer, x, valid):
     T = x.shape[1]
     pos, sa, y = torch.arange(T, device="cuda"), layer.self_attention, x[0].double()
     h = rms(y, layer.pre_sa_norm)
-    q, k, v = (dense(h, m).reshape(T, 3, 128) for m in (sa.q_proj, sa.k_proj, sa.v_proj))
+    q, k, v = (dense(h, m).reshape(T, -1, 128) for m in (sa.q_proj, sa.k_proj, sa.v_proj))
     y = y + dense(attend(turn(q, pos), turn(k, pos), v, (pos[:, None] < valid) == (pos[None, :] < valid)), sa.o_proj)
     return y + mlp(rms(y, layer.post_sa_norm), layer.mlp)
 
@@ -83,6 +83,33 @@ def test_encoder_layer(T, valid):
         got, again = layer(x, text_state(T, valid)), layer(x, text_state(T, valid))
     assert torch.equal(x, kept) and torch.equal(got, again)       # the input stays
     assert (got[0] - want).norm() <= 4e-6 * want.norm()           # a few roundings of fp32 per sum and layer part
+
+
+@pytest.mark.parametrize("width,heads,kv_heads,B,T", [(1024, 16, 16, 1, 300), (1024, 16, 16, 1, 400), (1024, 16, 16, 1, 700), (1024, 16, 16, 1, 1024),
+                                                      (2048, 16, 4, 2, 300), (2048, 16, 4, 2, 500), (2048, 16, 4, 2, 861), (2048, 16, 4, 2, 1300)])
+def test_projections_keep_their_sums(width, heads, kv_heads, B, T):
+    """Widths and heads of Dia's encoder and decoder.  By themselves the values (which every later frame of a prompt reads) are sums of 64 products that are
+    added in fp32; one product of q, k and v has so many columns that it would be summed on the tensor cores, from 385 encoder rows and 769 prompt rows on, and one of
+    k and v from 2305 prompt rows on.  K / 64 fp32 additions and terms that are exact to 2^-24: 1e-6; all K products in one accumulator that cuts off: 5e-6 and more."""
+    from dia_tts_prune_b200 import engine
+    from dia_tts_prune_b200.config import DataConfig, DecoderConfig, DiaConfig, EncoderConfig, ModelConfig
+    from dia_tts_prune_b200.layers import EncoderLayer, _rows_layer
+    cfg = DiaConfig(model=ModelConfig(encoder=EncoderConfig(n_layer=1, n_embd=width, n_hidden=128, n_head=heads, head_dim=128), decoder=DecoderConfig(
+        n_layer=1, n_embd=256, n_hidden=256, gqa_query_heads=2, kv_heads=1, gqa_head_dim=128, cross_query_heads=2, cross_head_dim=128),
+        src_vocab_size=256, tgt_vocab_size=1028), data=DataConfig(text_length=1024, audio_length=2048, channels=9))
+    layer = EncoderLayer(cfg, torch.bfloat16)
+    if kv_heads != heads:
+        from dia_tts_prune_b200.layers import Attention
+        layer.self_attention = Attention(cfg, width, width, heads, kv_heads, 128, torch.bfloat16, out_embed_dim=width)
+    layer, sa = layer.cuda(), layer.self_attention
+    g = weights(layer, T)
+    x = torch.randn((B, T, width), generator=g, device="cuda")
+    k, v = torch.zeros((2, B, kv_heads, T, 128), device="cuda")
+    with torch.inference_mode():
+        _rows_layer(x, sa, layer.pre_sa_norm, layer.mlp, layer.post_sa_norm, 1e-5, engine.positions_i32(T, B, x.device), engine.rope_tables_device(cfg, x.device),
+                    0, None, k, v)
+    want = dense(rms(x.double(), layer.pre_sa_norm), sa.v_proj).reshape(B, T, kv_heads, 128).transpose(1, 2)
+    assert (v - want).norm() <= 1e-6 * want.norm()
 
 
 def test_arguments_follow_the_weights():
