@@ -9,6 +9,7 @@ from __future__ import annotations
 import ctypes as C
 import os
 import re
+import struct
 from pathlib import Path
 
 from . import build as _build
@@ -48,8 +49,13 @@ class RowsLayer(C.Structure):
     _fields_ = [(n, C.c_int32) for n in ("B", "T", "D", "F", "heads", "kv_heads", "slots", "mode", "cross_heads", "cross_kv_heads", "cross_slots", "n_pos")] + \
                [("eps", C.c_float), ("n_valid", C.c_int32 * 16), ("cross_valid", C.c_int32 * 16)] + \
                [(n, C.c_void_p) for n in ("x_in", "x", "sin_table", "cos_table", "positions", "norm_self", "norm_cross", "norm_mlp")] + \
-               [(n, DenseRef) for n in ("q", "k", "v", "o", "cross_q", "cross_o", "wi", "wo")] + \
+               [(n, DenseRef) for n in ("q", "k", "v", "o", "wi", "wo", "cross_q", "cross_o")] + \
                [(n, C.c_void_p) for n in ("k_cache", "v_cache", "cross_k", "cross_v", "work")]
+
+
+def set_kernels(a: RowsLayer, pointers: list[int]) -> None:
+    """The first kernels of ``a`` (q, k, v, o, wi, wo, then those of the cross-attention), three pointers each."""
+    struct.pack_into(f"{len(pointers)}P", a, RowsLayer.q.offset, *pointers)
 
 
 _vp, _i, _i32p, _fp = C.c_void_p, C.c_int, C.c_void_p, C.c_void_p

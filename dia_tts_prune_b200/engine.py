@@ -457,6 +457,15 @@ def dense_half_rows(M: int, N: int, K: int, device: torch.device) -> bool:
     return M > 128 and _half_rows(device.index if device.index is not None else torch.cuda.current_device(), M, N, K)
 
 
+@functools.lru_cache(maxsize=4096)
+def dense_half_choice(M: int, sizes: tuple[tuple[int, int], ...], device: torch.device) -> tuple[bool, ...]:
+    """:func:`dense_half_rows` of the products of a layer, ``(N, K)`` each; raises for one that no kernel takes."""
+    for N, K in sizes:
+        if not dense_supported(M, N, K):
+            raise NotImplementedError(f"dense layer [{M} x {K}] . [{K} x {N}] does not fit the tcgen05 tiling (K must be a multiple of 64, N of 4)")
+    return tuple(dense_half_rows(M, N, K, device) for N, K in sizes)
+
+
 def dense_prepare_half(w_KxN: torch.Tensor, inexact: torch.Tensor) -> tuple[torch.Tensor, torch.Tensor]:
     """K-major fp16 copy ``[N, K]`` of a DenseGeneral kernel, a power of two per column, and the columns' largest magnitudes ``[N]``.
     ``inexact`` (int32, one element on the device) is set where fp16 cannot hold the bf16 values."""

@@ -42,6 +42,7 @@ except Exception:  # pragma: no cover - hub not installed
         def __init_subclass__(cls, **kw):
             super().__init_subclass__()
 
+from . import _lib
 from ._lib import RowsLayer
 from .config import DiaConfig
 from .state import DecoderInferenceState, EncoderInferenceState, KVCache
@@ -333,17 +334,19 @@ def _rows_weights(a, M: int, attn: Attention, norm: RMSNorm, mlp: MlpBlock, norm
     """Points the arguments of a native layer call of ``M`` rows at the layer's weights.  Returns what has to live until the call has been made.
     Nothing is kept from one call for the next but the copies that the kernels hold themselves: arguments kept per layer held copies that their
     kernels had dropped, and were made anew for every other number of rows (host time of a layer's
-    arguments, us: 35 for any number of rows; kept ones 17 for the last number and 62 for another)."""
+    arguments, us: 27 for any number of rows; kept ones 16 for the last number and 60 for another)."""
     from . import engine as _k
     D, keep = a.D, []
-    F, H, Hk = mlp.wo.in_shapes[0], attn.num_query_heads, attn.num_kv_heads
-    a.F, a.heads, a.kv_heads = F, H, Hk
-    parts = [("q", attn.q_proj, D, H * 128), ("k", attn.k_proj, D, Hk * 128), ("v", attn.v_proj, D, Hk * 128), ("o", attn.o_proj, H * 128, D),
-             ("wi", mlp.wi_fused, D, 2 * F), ("wo", mlp.wo, F, D)]
+    wo = mlp.wo
+    F, Nq, Nk = wo.in_shapes[0], attn.num_query_heads * 128, attn.num_kv_heads * 128
+    a.F, a.heads, a.kv_heads = F, attn.num_query_heads, attn.num_kv_heads
+    modules = [attn.q_proj, attn.k_proj, attn.v_proj, attn.o_proj, mlp.wi_fused, wo]
+    sizes = ((Nq, D), (Nk, D), (Nk, D), (D, Nq), (2 * F, D), (D, F))
     norms = [("norm_self", norm), ("norm_mlp", norm_mlp)]
     if cross is not None:
-        Hc = a.cross_heads = cross.num_query_heads
-        parts += [("cross_q", cross.q_proj, D, Hc * 128), ("cross_o", cross.o_proj, Hc * 128, D)]
+        Nc, a.cross_heads = cross.num_query_heads * 128, cross.num_query_heads
+        modules += (cross.q_proj, cross.o_proj)
+        sizes += ((Nc, D), (D, Nc))
         norms.append(("norm_cross", norm_cross))
     for name, n in norms:
         w = n.weight
@@ -353,24 +356,21 @@ def _rows_weights(a, M: int, attn: Attention, norm: RMSNorm, mlp: MlpBlock, norm
             w = w.detach().to(torch.float32).contiguous()
         keep.append(w)
         setattr(a, name, w.data_ptr())
-    halves = []
-    for _, m, K, N in parts:
-        if not _k.dense_supported(M, N, K):
-            raise NotImplementedError(f"dense layer [{M} x {K}] . [{K} x {N}] does not fit the tcgen05 tiling (K must be a multiple of 64, N of 4)")
-        halves.append(m.kernel_weight_half() if _k.dense_half_rows(M, N, K, device) else None)      # (the product's rows go as two fp16 terms)
+    halves = [m.kernel_weight_half() if two else None for m, two in zip(modules, _k.dense_half_choice(M, sizes, device))]      # (rows as two fp16 terms)
     if None in halves[:3]:
-        _stack_kmajor([m for _, m, _, _ in parts[:3]])            # (all three, whichever of them these rows read)
-    for (name, m, K, N), h in zip(parts, halves):
+        _stack_kmajor(modules[:3])                                # (all three, whichever of them these rows read)
+    pointers = []
+    for m, size, h in zip(modules, sizes, halves):
         wt = m.kernel_weight_kmajor() if h is None else h[0]
-        if wt.shape != (N, K):                                    # the native call takes its sizes from D, F and the heads
-            raise NotImplementedError(f"a layer of width {D} on sm_100a has heads of 128 channels: dense kernel {tuple(m.kernel_shape)} where [{K} x {N}] is read")
+        if wt.shape != size:                                      # the native call takes its sizes from D, F and the heads
+            raise NotImplementedError(f"a layer of width {D} on sm_100a has heads of 128 channels: dense kernel {tuple(m.kernel_shape)} where {size[::-1]} is read")
         keep.append(wt)
-        r = getattr(a, name)
         if h is None:
-            r.wt_bf16 = wt.data_ptr()
+            pointers += (wt.data_ptr(), 0, 0)
         else:
-            r.wt_half, r.magnitudes = wt.data_ptr(), h[1].data_ptr()
             keep.append(h)
+            pointers += (0, wt.data_ptr(), h[1].data_ptr())
+    _lib.set_kernels(a, pointers)
     return keep
 
 

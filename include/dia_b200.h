@@ -271,7 +271,7 @@ typedef struct dia_b200_rows_layer {
     const float *sin_table, *cos_table;      /* [n_pos][64] */
     const int32_t *positions;                /* [B*T] */
     const float *norm_self, *norm_cross, *norm_mlp;
-    dia_b200_dense_ref q, k, v, o, cross_q, cross_o, wi, wo;
+    dia_b200_dense_ref q, k, v, o, wi, wo, cross_q, cross_o;
     float *k_cache, *v_cache;
     const float *cross_k, *cross_v;
     void *work;                              /* dia_b200_rows_layer_work_bytes(a) bytes of device memory */

@@ -23,7 +23,7 @@ def calls(monkeypatch):
     monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: False)
     monkeypatch.setattr(engine, "dense_prepare_weight", kmajor)
     monkeypatch.setattr(engine, "dense_prepare_half", lambda w, inexact: (w.detach().t().contiguous().half(), w.detach().abs().amax(0).float()))
-    monkeypatch.setattr(engine, "dense_half_rows", lambda M, N, K, device: M > 128 and N > 1024)
+    monkeypatch.setattr(engine, "dense_half_choice", lambda M, sizes, device: [M > 128 and N > 1024 for N, K in sizes])
     monkeypatch.setattr(engine, "rows_layer_work_bytes", lambda a: 0)
     monkeypatch.setattr(engine, "rows_layer_forward", lambda a, n, device: made.append(type(a).from_buffer_copy(a)))
     return made
