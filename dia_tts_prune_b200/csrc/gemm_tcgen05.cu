@@ -1272,7 +1272,7 @@ cudaError_t launch_transpose_to_bf16(const void* w, int src_bf16, void* wt, int 
     return cudaGetLastError();
 }
 
-static bool dense_rows_f32(int terms, int M, int N, int K, int sms, int pairs);
+static bool dense_rows_f32(int terms, int M, int N, int K, int sms);
 static cudaError_t run_gemm_f32(const F32Product& p, const void* a_terms, int terms, int splits, cudaStream_t st);
 
 // clusters of two CTAs of the pair kernel that run at the same time
@@ -1305,13 +1305,13 @@ static cudaError_t pairs_of(int dev, int* out) {
 // Columns of a pair's tile: the width whose rounds of tiles end first.  A round's time grows with its columns where the MMAs bound it (three
 // terms, us per k-block alone on the chip: 0.44 at 128, 0.63 at 192, 0.83 at 256) and hardly where issuing four of them does (one term:
 // 0.30 and 0.28; two terms with fp32 sums, seven rounds of 32 k-blocks, 16.2 at 128 and 24.5 at 256 a round).  1722 rows x 16384 columns, K = 2048, three terms: 7 rounds of 256 223 us, 7 of 224 209; 3072 columns: 2 of 256 69, 2 of 160 49
-static int pair_columns(int terms, int M, int N, int pairs, long long* rounds) {
+static int pair_columns(int terms, int M, int N, int pairs) {
     const int tiles_m = (M + 2 * BM - 1) / (2 * BM), fixed = terms == 1 ? 700 : terms == 2 ? 100 : 30;
     int best = 0;
     long long least = 0;
     for (int bn = 256; bn >= 128; bn -= 32) {
         const long long r = ((long long)tiles_m * ((N + bn - 1) / bn) + pairs - 1) / pairs, cost = r * (fixed + bn);
-        if (!best || cost < least) best = bn, least = cost, *rounds = r;
+        if (!best || cost < least) best = bn, least = cost;
     }
     return best;
 }
@@ -1327,8 +1327,7 @@ static cudaError_t run_pair(const CUtensorMap& ma, const void* wt, long long wt_
         *q.ran_out = 0;
         return cudaErrorLaunchTimeout;
     }
-    long long rounds = 0;
-    q.BN = pair_columns(TERMS, q.M, q.N, pairs, &rounds);
+    q.BN = pair_columns(TERMS, q.M, q.N, pairs);
     q.stages = std::min(kPairStagesMost, Pair<SUMS>::kSlots * kTileBytes / (TERMS * kTileBytes + q.BN / 2 * 128));
     CUtensorMap mb;
     if (!make_map(&mb, wt, wt_rows, q.K, q.BN / 2)) return cudaErrorNotSupported;
@@ -1347,10 +1346,7 @@ cudaError_t launch_gemm_tcgen05_bf16(const void* a_bf16, int terms, const void* 
     if (e0 == cudaSuccess) e0 = ask_smem<dia_gemm_tcgen05_kernel>(dev, kGemmSmem);
     if (e0 != cudaSuccess) return e0;
     CUtensorMap ma, mb;
-    int pairs = 0;
-    e0 = pairs_of<1, false>(dev, &pairs);
-    if (e0 != cudaSuccess) return e0;
-    if (terms == 1 && !groups && wt_rows == N && dense_rows_f32(1, M, N, K, sms, pairs)) {
+    if (terms == 1 && !groups && wt_rows == N && dense_rows_f32(1, M, N, K, sms)) {
         const F32Product narrow{nullptr, 0, 0, wt, ep.y_bf16 ? nullptr : y, N, N, ep.y_bf16, 1, M, N, K, 1.f, ep.y_bf16 ? 3 : 0, nullptr, 0, 0,
                                 ep.residual, ep.dyt_w, ep.dyt_b, ep.dyt_alpha};
         if (gemm_f32_ok(narrow)) return run_gemm_f32(narrow, a_bf16, 1, 8, st);
@@ -1388,23 +1384,19 @@ static int f32_splits(int tiles, int n_kb, int most, int sms) {
     while (2 * s <= most && tiles * 2 * s <= (s == 4 ? 96 : sms) && n_kb >= 4 * s) s *= 2;
     return s;
 }
-// Beyond 32 rows (and for bf16 rows) the fp32-sum kernel where its rounds of tiles are the shorter ones: its 128 x 128 tiles are twice
-// as many as 128 x 256 ones, and where they leave the chip idle its clusters split K.  Three terms: a k-block of a round takes three quarters
-// of one of 128 x 256 tiles on one SM (1.1 and 1.4 us).  (Pairs of SMs take 0.4 to 0.8 us, but their sums are two to ten times further off:
-// what had sums of 64 products keeps them.)  One term, us, pair / here: 512 rows N = K = 2048 18 / 16, 1024 rows 18 / 22; 1722 rows N = 768 18 /
-// 22, 800 rows 17 / 16: a k-block takes 0.34 us there and 0.46 here, and starting and ending 1 us longer.  Up to 128 rows half of a
-// pair's tile would be empty: against one SM's 128 x 256 tiles 21 to 20 units a k-block (100 rows N = 32768, K = 2048 21 us, pairs 33)
-static bool dense_rows_f32(int terms, int M, int N, int K, int sms, int pairs) {
+// Beyond 32 rows (and for bf16 rows) the fp32-sum kernel where its rounds of tiles are shorter than those of 128 x 256 tiles on one SM: its
+// 128 x 128 tiles are twice as many, and where they leave the chip idle its clusters split K.  Three terms: a k-block of a round takes three quarters
+// of one of 128 x 256 tiles (1.1 and 1.4 us).  One term: 21 to 20 units a k-block (100 rows N = 32768, K = 2048 21 us, pairs 33).  Pairs of SMs do not
+// count here: they take 0.4 to 0.8 us a k-block (three terms) and 0.34 to 0.46 here (one), but their sums of all K products cut off and are two to ten
+// times further off, so what has sums of 64 products keeps them (bf16 rows, all
+// positive, 1024 x 2048 x 1024: 12.9 us and 1.7e-6 on pairs, 15.4 us and 8.9e-8 here; 2048 x 1024 x 1536 16.5 and 3.4e-6, 20.5 and 1.0e-7).
+static bool dense_rows_f32(int terms, int M, int N, int K, int sms) {
     const int tm = (M + BM - 1) / BM, n_kb = (K + BK - 1) / BK;
     const long long narrow = (long long)tm * ((N + kFN - 1) / kFN), wide = (long long)tm * ((N + BN - 1) / BN);
     const int s = narrow < sms ? f32_splits((int)narrow, n_kb, 8, sms) : 1;
     const long long here = (narrow * s + sms - 1) / sms, there = (wide + sms - 1) / sms;
     const int kb = (n_kb + s - 1) / s;
-    if (terms != 1) return here * kb * 3 < there * n_kb * 4;
-    if (M <= BM) return here * (21 * kb + 100) < there * (20 * n_kb + 130);
-    long long rounds = 0;
-    (void)pair_columns(terms, M, N, pairs, &rounds);
-    return here * kb * 460 < rounds * n_kb * 340 + 1000;
+    return terms == 1 ? here * (21 * kb + 100) < there * (20 * n_kb + 130) : here * kb * 3 < there * n_kb * 4;
 }
 
 // splits: the most CTAs that may share a tile (1: a sum's order does not depend on the rows beside it)
@@ -1502,14 +1494,14 @@ bool gemm_half_ok(int M, int N, int K) {
     int dev = 0, sms = 0;
     if (M <= BM || N <= 0 || N % 4 || K < BK || K % BK) return false;
     if (current_sms(&dev, &sms) != cudaSuccess) return false;
-    return !dense_rows_f32(kTerms, M, N, K, sms, 0);
+    return !dense_rows_f32(kTerms, M, N, K, sms);
 }
 
 // k-blocks that the fp32-sum kernel takes for M fp32 rows, one after the other, or 0 where launch_gemm_tcgen05 does not sum them in fp32 by itself
 int gemm_sums_blocks(int M, int N, int K, bool always) {
     int dev = 0, sms = 0;
     if (dense_rows_few(M)) return 1;
-    if (current_sms(&dev, &sms) != cudaSuccess || (!always && !dense_rows_f32(kTerms, M, N, K, sms, 0))) return 0;
+    if (current_sms(&dev, &sms) != cudaSuccess || (!always && !dense_rows_f32(kTerms, M, N, K, sms))) return 0;
     const int tiles = (M + BM - 1) / BM * ((N + kFN - 1) / kFN), n_kb = (K + BK - 1) / BK, s = tiles < sms ? f32_splits(tiles, n_kb, 8, sms) : 1;
     return (tiles * s + sms - 1) / sms * ((n_kb + s - 1) / s);
 }
@@ -1575,7 +1567,7 @@ cudaError_t launch_gemm_tcgen05(const float* x, const float* norm_w, float eps, 
     int dev = 0, sms = 0;
     const cudaError_t e = current_sms(&dev, &sms);
     if (e != cudaSuccess) return e;
-    if ((sums || dense_rows_f32(kTerms, M, N, K, sms, 0)) && gemm_f32_ok(wide)) return run_gemm_f32(wide, workspace, kTerms, 8, st);
+    if ((sums || dense_rows_f32(kTerms, M, N, K, sms)) && gemm_f32_ok(wide)) return run_gemm_f32(wide, workspace, kTerms, 8, st);
     const GemmEpilogue ep{residual, nullptr, nullptr, 0.f, nullptr};
     return launch_gemm_tcgen05_bf16(workspace, kTerms, wt, N, y, M, N, K, ep, nullptr, st);
 }

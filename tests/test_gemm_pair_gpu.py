@@ -122,3 +122,14 @@ def test_weights_that_fp16_cannot_hold():
         assert d.kernel_weight_half() is None
         ref = x.double() @ d.weight.double()
         assert (d(x) - ref).norm() <= 1e-6 * ref.norm()
+
+
+@pytest.mark.parametrize("M,N,K", [(1024, 2048, 1024), (513, 2048, 1024), (1153, 1024, 1536), (2305, 512, 1024), (768, 3072, 1024), (128, 2048, 1024)])
+def test_products_that_keep_fp32_sums(M, N, K):
+    """bf16 rows whose 128 x 128 tiles fit one round: pieces of 64 products added in fp32, also where one sum of all products on a pair of SMs is
+    the faster one.  All products positive, so that what is cut off adds up: about half a unit of 2^-23 per 16 products of a sum, 2.4e-7 for pieces of 64
+    and 3.8e-6 for 1024."""
+    g = torch.Generator(device="cuda").manual_seed(M)
+    x, w = torch.rand((M, K), generator=g, device="cuda"), (torch.rand((N, K), generator=g, device="cuda") * K ** -0.5).bfloat16()
+    ref = x.bfloat16().double() @ w.double().T
+    assert (product(x, w) - ref).norm() <= 1e-6 * ref.norm()
