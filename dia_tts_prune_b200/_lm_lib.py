@@ -76,6 +76,7 @@ _SIGNATURES = {
     "lm_b200_engine_create": (_ci, [C.POINTER(Model), C.POINTER(Layer), _ci, C.POINTER(_vp)]),
     "lm_b200_engine_destroy": (_ci, [_vp]),
     "lm_b200_engine_workspace_bytes": (C.c_size_t, [_vp]),
+    "lm_b200_check": (_ci, [_vp, _vp]),
     "lm_b200_forward": (_ci, [_vp, _vp, _ci, _ci, _ci, _vp, _vp, _vp]),
     "lm_b200_op_norm_tapmix": (_ci, [_vp, _ci, _ci, _vp, _vp, _ci, _ci, _vp, _vp]),
     "lm_b200_op_mixer": (_ci, [_vp, _ci, _vp, _vp, _ci, _ci, _vp, _vp]),

@@ -1315,9 +1315,10 @@ int* split_attention_ran_out(int device, cudaStream_t st) {
     if (device < 0 || device >= 64) return nullptr;
     const std::lock_guard<std::mutex> hold(lock);
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-    if (!words[device] && cudaStreamIsCapturing(st, &capture) == cudaSuccess && capture == cudaStreamCaptureStatusNone) {
+    if (!words[device]) {
         int* w = nullptr;
-        if (cudaHostAlloc(reinterpret_cast<void**>(&w), sizeof(int), cudaHostAllocMapped) == cudaSuccess) {
+        if (cudaStreamIsCapturing(st, &capture) == cudaSuccess && capture == cudaStreamCaptureStatusNone &&
+            cudaHostAlloc(reinterpret_cast<void**>(&w), sizeof(int), cudaHostAllocMapped) == cudaSuccess) {
             *w = 0;
             words[device] = w;
         } else {
@@ -1325,6 +1326,13 @@ int* split_attention_ran_out(int device, cudaStream_t st) {
         }
     }
     return words[device];
+}
+
+bool take_ran_out(int device, cudaStream_t st) {
+    int* const word = split_attention_ran_out(device, st);
+    if (!word || !*reinterpret_cast<volatile int*>(word)) return false;
+    *reinterpret_cast<volatile int*>(word) = 0;
+    return true;
 }
 
 bool split_attention_ok(const SplitAttention& a) {
@@ -1348,10 +1356,7 @@ cudaError_t launch_split_attention(const SplitAttention& a, cudaStream_t st) {
     const cudaError_t e = cudaGetDevice(&device);
     if (e != cudaSuccess) return e;
     g.ran_out = split_attention_ran_out(device, st);          // (mapped and unified: one address on both sides)
-    if (g.ran_out && *reinterpret_cast<volatile int*>(g.ran_out)) {
-        *g.ran_out = 0;
-        return cudaErrorLaunchTimeout;
-    }
+    if (take_ran_out(device, st)) return cudaErrorLaunchTimeout;
     SplitAttention with = a;
     // Wide values are split in advance in every step: the fetching warps have few registers for them (9 and 24 decoding sequences over 1000
     // cached keys, latent rows of 256 + 32, 4 layers: 1714 and 1833 us split by the row tiles, 1139 and 1250 in advance; over 100 keys 867

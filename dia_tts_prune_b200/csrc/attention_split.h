@@ -51,7 +51,10 @@ struct SplitAttention {
 bool split_attention_ok(const SplitAttention& a);
 // bytes of `work` for `keys` keys of this shape (0: the shape is not taken)
 size_t split_attention_work_bytes(const SplitAttention& a, int keys);
-int* split_attention_ran_out(int device, cudaStream_t st);      // the word that a kernel sets when one of its waits has run out
+// The word of `device` that a kernel sets when one of its waits has run out (its outputs are NaN then).  Made by the first call outside of a capture: engines
+// and weight copies are made with one, so that products that are captured have it.
+int* split_attention_ran_out(int device, cudaStream_t st);
+bool take_ran_out(int device, cudaStream_t st);                 // whether a wait has run out since the last look; the word is zero afterwards
 cudaError_t launch_split_attention(const SplitAttention& a, cudaStream_t st);
 
 }  // namespace dia

@@ -14,6 +14,7 @@
 #include "common.cuh"
 #include "engine_internal.h"
 #include "gemm_tcgen05.h"
+#include "attention_split.h"
 
 using namespace dia;
 
@@ -47,6 +48,8 @@ struct DeviceGuard {
     }
     ~DeviceGuard() { if (prev >= 0) cudaSetDevice(prev); }
 };
+// behind a synchronisation: a wait of a kernel that ran out (its outputs are NaN) is an error here
+#define CK_WAITS(dev, st) CK(take_ran_out(dev, st) ? cudaErrorLaunchTimeout : cudaSuccess)
 #define ON_DEVICE(dev) DeviceGuard _guard(dev); CK(_guard.err)
 
 }  // namespace
@@ -249,6 +252,7 @@ static int create_engine(const dia_b200_shape* shape, int device, int n_ctas, in
     int coop = 0;
     CK(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device));
     if (!coop) { g_last_cuda_error = "cooperative launch unsupported"; return DIA_B200_EUNSUPPORTED; }
+    (void)split_attention_ran_out(device, nullptr);
 
     dia_b200_engine* e = new (std::nothrow) dia_b200_engine();
     if (!e) return DIA_B200_ENOMEM;
@@ -663,6 +667,7 @@ int dia_b200_generate_begin(dia_b200_engine* e, int32_t* grid, const dia_b200_ge
     if (rc) return rc;
     ON_DEVICE(e->device);
     CK(cudaStreamSynchronize(S(stream)));     // h_gs staging reuse
+    CK_WAITS(e->device, S(stream));
     int dmax = 0;
     for (int c = 0; c < e->shape.channels; ++c) dmax = std::max(dmax, (int)e->shape.delay_pattern[c]);
     std::memset(e->h_gs, 0, sizeof(GenState));
@@ -718,6 +723,7 @@ int dia_b200_generate_status(dia_b200_engine* e, dia_b200_gen_status* out, void*
     ON_DEVICE(e->device);
     CK(cudaMemcpyAsync(e->h_gs, e->d_gs, sizeof(GenState), cudaMemcpyDeviceToHost, S(stream)));
     CK(cudaStreamSynchronize(S(stream)));
+    CK_WAITS(e->device, S(stream));
     out->dec_step = e->h_gs->dec_step;
     out->finished = e->h_gs->finished;
     out->eos_detected = e->h_gs->eos_detected;
@@ -844,6 +850,7 @@ int dia_b200_batch_generate_begin(dia_b200_engine* e, int n_utterances, int32_t*
     if (rc) return rc;
     ON_DEVICE(e->device);
     CK(cudaStreamSynchronize(S(stream)));
+    CK_WAITS(e->device, S(stream));
     int dmax = 0;
     for (int c = 0; c < e->shape.channels; ++c) dmax = std::max(dmax, (int)e->shape.delay_pattern[c]);
     std::memset(e->h_gs, 0, sizeof(GenState) * kMaxUtt);
@@ -914,6 +921,7 @@ int dia_b200_batch_generate_status(dia_b200_engine* e, dia_b200_gen_status* out,
     ON_DEVICE(e->device);
     CK(cudaMemcpyAsync(e->h_gs, e->d_gs, sizeof(GenState) * kMaxUtt, cudaMemcpyDeviceToHost, S(stream)));
     CK(cudaStreamSynchronize(S(stream)));
+    CK_WAITS(e->device, S(stream));
     for (int u = 0; u < e->n_active; ++u) {
         const GenState& g = e->h_gs[u];
         out[u].dec_step = g.dec_step; out[u].finished = g.finished; out[u].eos_detected = g.eos_detected;

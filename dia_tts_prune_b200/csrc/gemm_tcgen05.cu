@@ -18,8 +18,8 @@
 //   warps 2-5 epilogue of tile i (tcgen05.ld, 32 lanes x 32 columns per instruction -> registers -> residual add ->
 //             fp32 stores) while the MMAs of tile i + 1 fill the other accumulator
 // W is kept as a K-major bf16 copy [N][K] made once per weight (transpose_to_bf16_kernel), so that A and B use the
-// same canonical UMMA layout.  Every wait is bounded (a stuck pipeline traps instead of hanging the GPU).
-// More than 128 rows run on pairs of SMs (dia_gemm_pair_kernel); this kernel keeps the shorter ones and small expert groups.
+// same canonical UMMA layout.  Every wait of the kernels of one SM is bounded: a stuck pipeline traps instead of hanging the GPU.
+// More than 128 rows run on pairs of SMs (dia_gemm_pair_kernel, whose waits end without a trap); this kernel keeps the shorter ones and small expert groups.
 //
 // The same kernel serves callers whose activations are bf16 already (terms = 1: one MMA per k-step, the operand is read
 // as it is), row tiles that belong to different weight matrices (expert groups: the group of a tile's first row picks
@@ -486,7 +486,8 @@ dia_gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
 //             shared memory so that whole lines are stored (row by row, 4096 x 2048 x 2048 was bound by those stores)
 // us, one SM per tile / pairs: one term 4096 x 8192 x 2048 135 / 94 (1.46 PFLOP/s), 4096 x 2048 x 6144 106 / 80, 1722 x 16384 x 2048 126 / 90;
 // three terms 256 / 209 (1.66 PFLOP/s), 4096 x 6144 x 2048 227 / 187.  Bound: the MMAs (four of one term take 512 cycles to run and 540 to
-// issue; the products of a long pass are at the power limit).  A wait that runs out ends every role; the kernel sets the device's word, which the next launch reports.
+// issue; the products of a long pass are at the power limit).  A wait that runs out ends every role: the tiles that have no result become NaN, and
+// the kernel sets the device's word, which the next launch and the calls that wait for the device report.
 //
 // SUMS: fp32 rows as two fp16 terms (split_rows_kernel) and weights as fp16 (transpose_to_half_kernel), every row and every column with a power
 // of two of its own; an accumulator lives for kPairChunk k-blocks and eight epilogue warps add it to the tile's sums in their registers (two
@@ -502,7 +503,7 @@ struct Pair {
     static constexpr int kSmem = kSlots * kTileBytes + kWarps * 4096 + 1024 + 256;
 };
 constexpr int kPairStagesMost = 8, kPairChunk = 4;
-constexpr unsigned kPairPolls = 4000000u;
+constexpr unsigned kPairPolls = 4000000u;                     // a few seconds
 static_assert((2 * kPairStagesMost + 4) * 8 + 8 <= 256, "barrier region");
 
 struct PairProduct {
@@ -513,20 +514,28 @@ struct PairProduct {
     const int* row_group; int group_rows; const int* n_rows;
     int* ran_out;
     const float* row_inv; const float* col_mag;              // SUMS: inverse scales of the rows, largest magnitudes of the columns
+    unsigned polls;                                           // looks at a barrier until a wait has run out
 };
+
+// How often a wait of the pair kernel looks at its barrier, in products that this thread launches.  With 0 each wait runs out before anything has
+// been issued, which is how a test sees what then becomes of the outputs.
+unsigned& gemm_pair_polls() {
+    static thread_local unsigned polls = kPairPolls;
+    return polls;
+}
 
 __device__ __forceinline__ uint32_t at_rank(const void* local, uint32_t rank) {
     uint32_t a;
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(local)), "r"(rank));
     return a;
 }
-__device__ __forceinline__ bool pair_wait(uint64_t* bar, uint32_t parity) {       // one answer for a converged warp
-    for (unsigned i = 0; i < kPairPolls; ++i)
+__device__ __forceinline__ bool pair_wait(uint64_t* bar, uint32_t parity, unsigned polls) {       // one answer for a converged warp
+    for (unsigned i = 0; i < polls; ++i)
         if (__any_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
     return false;
 }
-__device__ __forceinline__ bool lane_wait(uint64_t* bar, uint32_t parity) {
-    for (unsigned i = 0; i < kPairPolls; ++i)
+__device__ __forceinline__ bool lane_wait(uint64_t* bar, uint32_t parity, unsigned polls) {
+    for (unsigned i = 0; i < polls; ++i)
         if (mbar_try_wait(bar, parity)) return true;
     return false;
 }
@@ -550,6 +559,17 @@ __device__ __forceinline__ void umma_commit_pair(uint64_t* bar) {               
 }
 __device__ __forceinline__ void cluster_sync_all() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// NaN for rows [row0, row0 + rows) and columns [c0, c1) of a product that has no result (a multiple of 4 columns)
+__device__ __noinline__ void pair_no_result(const PairProduct& p, int row0, int rows, int c0, int c1, int lane) {
+    const uint32_t nan = 0x7fffffffu, two = 0x7fff7fffu;      // (as fp32 and as two bf16)
+    for (int r = 0; r < rows; ++r)
+        for (int n = c0 + 4 * lane; n < c1; n += 128) {
+            const size_t at = (size_t)(row0 + r) * p.N + n;
+            if (p.y_bf16) *reinterpret_cast<uint2*>(p.y_bf16 + at) = make_uint2(two, two);
+            else *reinterpret_cast<uint4*>(p.y + at) = make_uint4(nan, nan, nan, nan);
+        }
 }
 
 // the inverse of a column's scale 2^(14 - e), where its largest magnitude lies in [2^e, 2^(e + 1)) (0 for a column of zeros)
@@ -603,7 +623,7 @@ dia_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
                     const int a_row = m0 + (int)rank * BM, b_row = n0 + (int)rank * half + (p.row_group ? p.row_group[m0] * p.group_rows : 0);
                     for (int kb = 0; kb < n_kb; ++kb, ++i) {
                         const unsigned s = i % n_stages;
-                        if (!lane_wait(&empty[s], ((i / n_stages) & 1u) ^ 1u)) { ok = false; break; }
+                        if (!lane_wait(&empty[s], ((i / n_stages) & 1u) ^ 1u, p.polls)) { ok = false; break; }
                         if (rank == 0) mbar_arrive_expect_tx(&full[s], 2u * stage_bytes);
                         const uint32_t bar = at_rank(&full[s], 0), dst = smem_u32(smem + s * stage_bytes);
                         tma_load_2d_pair(dst + TERMS * kTileBytes, &map_b, bar, kb * BK, b_row);
@@ -612,7 +632,9 @@ dia_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
                     }
                 }
                 // (the leader's last commits arrive here: not after this CTA has gone)
-                for (unsigned j = i > (unsigned)n_stages ? i - n_stages : 0; j < i && ok; ++j) ok = lane_wait(&empty[j % n_stages], (j / n_stages) & 1u);
+                for (unsigned j = i > (unsigned)n_stages ? i - n_stages : 0; j < i && ok; ++j) ok = lane_wait(&empty[j % n_stages], (j / n_stages) & 1u, p.polls);
+                // (nor do copies arrive that were issued before a wait ran out)
+                for (unsigned j = i > (unsigned)n_stages ? i - n_stages : 0; j < i && !ok && rank == 0; ++j) (void)lane_wait(&full[j % n_stages], (j / n_stages) & 1u, p.polls);
             }
         } else if (warp == 1) {
             if (rank == 0) {
@@ -624,12 +646,12 @@ dia_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
                     for (int kb = 0; kb < n_kb; ++kb, ++i) {
                         const bool first = SUMS ? kb % kPairChunk == 0 : kb == 0, last = kb == n_kb - 1 || (SUMS && kb % kPairChunk == kPairChunk - 1);
                         if (first) {
-                            if (!pair_wait(&t_empty[it & 1u], ((it >> 1) & 1u) ^ 1u)) { ok = false; break; }
+                            if (!pair_wait(&t_empty[it & 1u], ((it >> 1) & 1u) ^ 1u, p.polls)) { ok = false; break; }
                             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                         }
                         const uint32_t d = tmem_base + (it & 1u) * 256;
                         const unsigned s = i % n_stages;
-                        if (!pair_wait(&full[s], (i / n_stages) & 1u)) { ok = false; break; }
+                        if (!pair_wait(&full[s], (i / n_stages) & 1u, p.polls)) { ok = false; break; }
                         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                         const uint32_t at = smem_u32(smem + s * stage_bytes);
                         const uint64_t adesc = umma_desc(at), bdesc = umma_desc(at + TERMS * kTileBytes);
@@ -656,14 +678,14 @@ dia_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
         float* const blk = reinterpret_cast<float*>(turn + (warp - Pair<SUMS>::kFirst) * 4096);
         const int rr = lane >> 3, ch = lane & 7;
         unsigned i = 0;
-        for (int t = pair; t < n_tiles && ok; t += pairs) {
+        for (int t = pair; t < n_tiles; t += pairs) {
             const int n0 = (t / tiles_m) * BN, m0 = (t % tiles_m) * 2 * BM;
             float sum[128];
 #pragma unroll
             for (int c = 0; c < 128; ++c) sum[c] = 0.f;
-            for (int kb = 0; kb < n_kb; kb += kPairChunk, ++i) {
+            for (int kb = 0; kb < n_kb && ok; kb += kPairChunk, ++i) {
                 const unsigned acc = i & 1u;
-                if (!pair_wait(&t_full[acc], (i >> 1) & 1u)) { ok = false; break; }
+                if (!pair_wait(&t_full[acc], (i >> 1) & 1u, p.polls)) { ok = false; break; }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
                 for (int cb = 0; cb < 4; ++cb) {
@@ -689,6 +711,10 @@ dia_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
                     asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(at_rank(&t_empty[acc], 0)) : "memory");
             }
             const int row0 = m0 + (int)rank * BM + q * 32, rows = min(32, M - row0);
+            if (!ok) {                                        // the sums of this tile lack products, and no later one has any
+                pair_no_result(p, row0, rows, n0 + h0, min(n0 + h0 + half, N), lane);
+                continue;
+            }
             float ri[8];                                      // (loads ahead of their uses: the output of a tile took 3.2 us with one row after the other)
 #pragma unroll
             for (int g = 0; g < 8; ++g) ri[g] = 4 * g + rr < rows ? p.row_inv[row0 + 4 * g + rr] : 0.f;
@@ -737,10 +763,14 @@ dia_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
         for (int t = pair; t < n_tiles; t += pairs) {
             const int n0 = (t / tiles_m) * BN, m0 = (t % tiles_m) * 2 * BM;
             if (m0 >= m_lim) continue;
-            const unsigned acc = it & 1u;
-            if (!pair_wait(&t_full[acc], (it >> 1) & 1u)) { ok = false; break; }
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const int row0 = m0 + (int)rank * BM + q * 32, rows = min(32, M - row0);
+            const unsigned acc = it & 1u;
+            ok = ok && pair_wait(&t_full[acc], (it >> 1) & 1u, p.polls);
+            if (!ok) {
+                pair_no_result(p, row0, rows, n0, min(n0 + BN, N), lane);
+                continue;
+            }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll 1
             for (int cb = 0; cb < BN / 32; ++cb) {
                 const int c0 = n0 + cb * 32;
@@ -1266,7 +1296,17 @@ static cudaError_t ask_smem(int dev, int bytes) {
 
 size_t gemm_workspace_bytes(int M, int K) { return (size_t)kTerms * M * K * 2; }
 
+// (the word of waits that ran out: there before a product of these weights can be captured)
+static cudaError_t make_ran_out(cudaStream_t st) {
+    int dev = 0;
+    const cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) (void)split_attention_ran_out(dev, st);
+    return e;
+}
+
 cudaError_t launch_transpose_to_bf16(const void* w, int src_bf16, void* wt, int K, int N, cudaStream_t st) {
+    const cudaError_t e = make_ran_out(st);
+    if (e != cudaSuccess) return e;
     dim3 grid((N + 31) / 32, (K + 31) / 32), block(32, 8);
     transpose_to_bf16_kernel<<<grid, block, 0, st>>>(w, src_bf16, reinterpret_cast<__nv_bfloat16*>(wt), K, N);
     return cudaGetLastError();
@@ -1322,11 +1362,9 @@ static cudaError_t run_pair(const CUtensorMap& ma, const void* wt, long long wt_
     const auto kernel = dia_gemm_pair_kernel<TERMS, SUMS>;
     if (e == cudaSuccess) e = ask_smem<dia_gemm_pair_kernel<TERMS, SUMS>>(dev, Pair<SUMS>::kSmem);
     if (e != cudaSuccess) return e;
+    q.polls = gemm_pair_polls();
     q.ran_out = split_attention_ran_out(dev, st);
-    if (q.ran_out && *reinterpret_cast<volatile int*>(q.ran_out)) {
-        *q.ran_out = 0;
-        return cudaErrorLaunchTimeout;
-    }
+    if (take_ran_out(dev, st)) return cudaErrorLaunchTimeout;
     q.BN = pair_columns(TERMS, q.M, q.N, pairs);
     q.stages = std::min(kPairStagesMost, Pair<SUMS>::kSlots * kTileBytes / (TERMS * kTileBytes + q.BN / 2 * 128));
     CUtensorMap mb;
@@ -1507,7 +1545,8 @@ int gemm_sums_blocks(int M, int N, int K, bool always) {
 }
 
 cudaError_t launch_prepare_half(const void* w, int src_bf16, void* wt, float* mag, int* inexact, int K, int N, cudaStream_t st) {
-    const cudaError_t e = cudaMemsetAsync(mag, 0, (size_t)N * 4, st);
+    cudaError_t e = make_ran_out(st);
+    if (e == cudaSuccess) e = cudaMemsetAsync(mag, 0, (size_t)N * 4, st);
     if (e != cudaSuccess) return e;
     column_magnitudes_kernel<<<dim3((N + 255) / 256, (K + 63) / 64), 256, 0, st>>>(w, src_bf16, reinterpret_cast<uint32_t*>(mag), K, N);
     transpose_to_half_kernel<<<dim3((N + 31) / 32, (K + 31) / 32), dim3(32, 8), 0, st>>>(w, src_bf16, mag, reinterpret_cast<__half*>(wt), inexact, K, N);
@@ -1522,7 +1561,7 @@ static void split_rows(const float* x, const float* norm_w, float eps, bool gate
     else split_rows_kernel<TERMS, false><<<M, 256, 0, st>>>(x, norm_w, eps, out, row_inv, M, K, aligned);
 }
 
-// y = [residual +] x W for fp32 rows: two fp16 terms and fp32 sums of 64-product pieces, on pairs of SMs.
+// y = [residual +] x W for fp32 rows: two fp16 terms and fp32 sums of pieces of 256 products, on pairs of SMs.
 cudaError_t launch_gemm_half(const float* x, const float* norm_w, float eps, bool gated, const void* wt, const float* mag, const float* residual, float* y,
                              void* workspace, int M, int N, int K, cudaStream_t st) {
     if (M <= 0 || N <= 0 || N % 4 || K < BK || K % BK || (gated && norm_w)) return cudaErrorNotSupported;

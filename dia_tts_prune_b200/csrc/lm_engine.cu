@@ -1019,6 +1019,7 @@ int lm_b200_engine_create(const lm_b200_model* model, const lm_b200_layer* layer
         if (l.form == LM_B200_FORM_STREAMS && l.mixer == LM_B200_MIXER_PAIR)
             for (int q = 0; q < 2; ++q) l.part[q] = &e->parts_of_pairs[next_part++];
     e->device = device;
+    (void)dia::split_attention_ran_out(device, nullptr);      // (before a step is captured)
     const size_t R = (size_t)m.max_rows, D = (size_t)m.width;
     size_t qk = 0, att = 0, E = 1, top = 1, F = 1, Sf = 1, slots = 1;
     size_t n_in = 0, k_out = 0, n_rec = 0, split_dim = 0, kv_split = 0;
@@ -1406,6 +1407,13 @@ int run_step_graph(lm_b200_engine* e, const int32_t* step, int M, int n_seq, int
 
 extern "C" {
 
+int lm_b200_check(lm_b200_engine* e, void* stream) {
+    if (!e) return LM_B200_EINVAL;
+    Guard g(e->device);
+    if (!g.ok) return LM_B200_ECUDA;
+    return dia::take_ran_out(e->device, S(stream)) ? cuda_fail(cudaErrorLaunchTimeout) : LM_B200_OK;
+}
+
 int lm_b200_forward(lm_b200_engine* e, const int32_t* step, int M, int n_seq, int n_want, float* logits_out, float* layers_out,
                     void* stream) {
     if (!e || !step || M <= 0 || M > e->m.max_rows || n_seq <= 0 || n_seq > M || n_want < 0 || n_want > M ||
@@ -1413,6 +1421,7 @@ int lm_b200_forward(lm_b200_engine* e, const int32_t* step, int M, int n_seq, in
         return LM_B200_EINVAL;
     Guard g(e->device);
     if (!g.ok) return LM_B200_ECUDA;
+    if (dia::take_ran_out(e->device, S(stream))) return cuda_fail(cudaErrorLaunchTimeout);
     if (e->m.step_graphs && M <= lm::kRowsKernelMax && !layers_out)
         return run_step_graph(e, step, M, n_seq, n_want, logits_out, S(stream));
     return run_step(e, step, M, n_seq, n_want, logits_out, layers_out, S(stream));

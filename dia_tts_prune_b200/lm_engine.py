@@ -111,6 +111,10 @@ class LMEngine:
             t = t.pin_memory()
         return t.to(self.device, non_blocking=True), n_rows, S, len(want)
 
+    def check(self) -> None:
+        """Behind a synchronisation: raises if a wait of a kernel ran out since the last look (what it wrote is NaN)."""
+        _lm_lib.check(self.lib.lm_b200_check(self._h, _stream(self.device)), "check")
+
     def _forward(self, parts, logits_out: torch.Tensor | None, layers_out: torch.Tensor | None = None) -> None:
         buf, M, S, W = self._pack(parts)
         self.state.sync_table()

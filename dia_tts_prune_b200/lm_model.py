@@ -310,6 +310,8 @@ class Scheduler:
                     sampled.append(req)
         logits = self.model.engine.step(entries)
         tokens = self.model.sample(logits, sampled).tolist() if sampled else []
+        if sampled:
+            self.model.engine.check()
         finished = []
         for req, tok in zip(sampled, tokens):
             req.output.append(int(tok))

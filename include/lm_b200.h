@@ -249,6 +249,9 @@ int lm_b200_engine_create(const lm_b200_model *model, const lm_b200_layer *layer
 int lm_b200_engine_destroy(lm_b200_engine *e);
 size_t lm_b200_engine_workspace_bytes(const lm_b200_engine *e);
 
+/* Behind a synchronisation: LM_B200_ECUDA if a wait of a kernel ran out on the engine's device since the last look (its outputs are NaN). */
+int lm_b200_check(lm_b200_engine *e, void *stream);
+
 /* One step: embeds the rows, runs every layer (appending to the pages and tails of the rows' sequences), and writes the
  * logits of the wanted rows, float32 [n_want][vocab].  layers_out (optional): the residual stream after every layer,
  * float32 [n_layer][M][width]. */

@@ -7,14 +7,15 @@ import torch
 pytestmark = pytest.mark.gpu
 
 
-def product(x, w):
+def product(x, w, y=None):
     from dia_tts_prune_b200 import _lm_lib
     lib = _lm_lib.load()
     (M, K), N = x.shape, w.shape[0]
-    y = torch.full((M, N), float("nan"), device="cuda")
+    y = torch.full((M, N), float("nan"), device="cuda") if y is None else y
     xb = torch.empty((M, K), dtype=torch.bfloat16, device="cuda")
     rc = lib.lm_b200_op_linear_tc(x.data_ptr(), w.data_ptr(), y.data_ptr(), xb.data_ptr(), M, N, K, torch.cuda.current_stream().cuda_stream)
-    assert rc == 0
+    if rc:
+        raise RuntimeError(rc)
     return y
 
 
@@ -133,3 +134,58 @@ def test_products_that_keep_fp32_sums(M, N, K):
     x, w = torch.rand((M, K), generator=g, device="cuda"), (torch.rand((N, K), generator=g, device="cuda") * K ** -0.5).bfloat16()
     ref = x.bfloat16().double() @ w.double().T
     assert (product(x, w) - ref).norm() <= 1e-6 * ref.norm()
+
+
+def ran_out(lib):
+    """(the word that a kernel sets when a wait of its ran out, how often the waits of this thread's products look at their barriers)"""
+    import ctypes as C
+    word_of, polls_of = getattr(lib, "_ZN3dia23split_attention_ran_outEiP11CUstream_st"), getattr(lib, "_ZN3dia15gemm_pair_pollsEv")
+    word_of.restype, word_of.argtypes = C.POINTER(C.c_int), [C.c_int, C.c_void_p]
+    polls_of.restype, polls_of.argtypes = C.POINTER(C.c_uint), []
+    return word_of(torch.cuda.current_device(), None), polls_of()
+
+
+@pytest.mark.parametrize("M,N,K,half", [(600, 16384, 192, False), (129, 18948, 264, False), (600, 16384, 192, True), (1722, 3076, 576, True)])
+def test_a_wait_that_ran_out(M, N, K, half):
+    """Waits that run out before anything is issued (no look at a barrier): the whole result is NaN, the next launch returns an error, the one after it
+    has the result"""
+    from dia_tts_prune_b200 import _lib, _lm_lib, engine
+    x, w = torch.randn((M, K), device="cuda"), (torch.randn((N, K), device="cuda") * K ** -0.5).bfloat16()
+    if half:
+        copy = engine.dense_prepare_half(w.t().contiguous(), torch.zeros((1,), dtype=torch.int32, device="cuda"))
+        call = lambda r: engine.dense_forward_half(x, copy, residual=r)
+    else:
+        call = lambda r: product(x, w, r)
+    word, polls = ran_out((_lib if half else _lm_lib).load())
+    good, kept = call(torch.zeros((M, N), device="cuda")), polls[0]
+    assert word[0] == 0 and kept > 1000000
+    polls[0] = 0
+    try:
+        bad = call(torch.zeros((M, N), device="cuda"))
+        torch.cuda.synchronize()
+    finally:
+        polls[0] = kept
+    assert torch.isnan(bad).all() and word[0] == 1
+    with pytest.raises(RuntimeError):
+        call(torch.zeros((M, N), device="cuda"))
+    assert word[0] == 0 and torch.equal(call(torch.zeros((M, N), device="cuda")), good)
+
+
+def test_a_wait_that_ran_out_reaches_a_step():
+    """The word set by hand between a step's launches and the look behind its synchronisation"""
+    from dia_tts_prune_b200 import _lm_lib, synthetic as SY
+    from dia_tts_prune_b200.lm_config import PubopelConfig
+    from dia_tts_prune_b200.lm_model import CausalLM
+    cfg = SY.pubopel_config(width=128, layers=1, heads=1, kv_heads=1, dim=16, experts=3, top=1, expert_ff=64, shared_ff=None, vocab=64)
+    model = CausalLM(PubopelConfig.model_validate(cfg), SY.pubopel_weights(cfg, 3), dtype="bfloat16", device="cuda:0", max_tokens=64, max_sequences=1, max_rows=32)
+    word, _ = ran_out(_lm_lib.load())
+    assert model.generate([[1, 2, 3]], max_new_tokens=3)
+    model.engine.check()
+    word[0] = 1
+    with pytest.raises(RuntimeError):
+        model.engine.check()
+    assert word[0] == 0
+    model.engine.check()
+    word[0] = 1
+    with pytest.raises(RuntimeError):
+        model.generate([[1, 2, 3]], max_new_tokens=3)
