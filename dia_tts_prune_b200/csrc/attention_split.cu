@@ -1293,8 +1293,9 @@ bool geometry_of(const SplitAttention& a, Geometry& g, size_t& smem, int rt) {
 
 template <int NVS, int RT>
 cudaError_t launch_inst(const SplitAttention& a, const Geometry& g, size_t smem, cudaStream_t st) {
-    // (the same size for every launch: another thread's cannot lower what this one needs)
-    const cudaError_t e = cudaFuncSetAttribute(split_attention_kernel<NVS, RT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMost);
+    int device = 0;
+    cudaError_t e = cudaGetDevice(&device);
+    if (e == cudaSuccess) e = ask_smem<split_attention_kernel<NVS, RT>>(device, kSmemMost);
     if (e != cudaSuccess) return e;
     const int tt = kRows >> g.pk_shift, tiles = a.n_seq > 1 ? a.M / tt + a.n_seq : (a.M + tt - 1) / tt;
     if (a.work) {

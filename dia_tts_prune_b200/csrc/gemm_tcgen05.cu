@@ -1274,26 +1274,6 @@ static bool make_map(CUtensorMap* map, const void* base, long long rows, int K, 
                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// SMs of the current device
-static cudaError_t current_sms(int* dev, int* sms) {
-    static std::atomic<int> known[64];
-    const cudaError_t e = cudaGetDevice(dev);
-    if (e != cudaSuccess) return e;
-    if (*dev < 64 && (*sms = known[*dev].load(std::memory_order_relaxed)) > 0) return cudaSuccess;
-    const cudaError_t a = cudaDeviceGetAttribute(sms, cudaDevAttrMultiProcessorCount, *dev);
-    if (a == cudaSuccess && *dev < 64) known[*dev].store(*sms, std::memory_order_relaxed);
-    return a;
-}
-// Dynamic shared memory of a kernel, the same size for every launch: asked for once per device
-template <auto KERNEL>
-static cudaError_t ask_smem(int dev, int bytes) {
-    static std::atomic<bool> asked[64];
-    if (dev < 64 && asked[dev].load(std::memory_order_relaxed)) return cudaSuccess;
-    const cudaError_t e = cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    if (e == cudaSuccess && dev < 64) asked[dev].store(true, std::memory_order_relaxed);
-    return e;
-}
-
 size_t gemm_workspace_bytes(int M, int K) { return (size_t)kTerms * M * K * 2; }
 
 // (the word of waits that ran out: there before a product of these weights can be captured)

@@ -8,9 +8,32 @@
 // of Wt.
 #pragma once
 
+#include <atomic>
+
 #include <cuda_runtime.h>
 
 namespace dia {
+
+// What is asked for once per device (static: two libraries in one process hold kernels of the same names, and an inline function's statics would be
+// theirs together).  SMs of the current device:
+static inline cudaError_t current_sms(int* dev, int* sms) {
+    static std::atomic<int> known[64];
+    const cudaError_t e = cudaGetDevice(dev);
+    if (e != cudaSuccess) return e;
+    if (*dev < 64 && (*sms = known[*dev].load(std::memory_order_relaxed)) > 0) return cudaSuccess;
+    const cudaError_t a = cudaDeviceGetAttribute(sms, cudaDevAttrMultiProcessorCount, *dev);
+    if (a == cudaSuccess && *dev < 64) known[*dev].store(*sms, std::memory_order_relaxed);
+    return a;
+}
+// Dynamic shared memory of a kernel, the same size for every launch:
+template <auto KERNEL>
+static cudaError_t ask_smem(int dev, int bytes) {
+    static std::atomic<bool> asked[64];
+    if (dev < 64 && asked[dev].load(std::memory_order_relaxed)) return cudaSuccess;
+    const cudaError_t e = cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e == cudaSuccess && dev < 64) asked[dev].store(true, std::memory_order_relaxed);
+    return e;
+}
 
 constexpr int kGemmRowTile = 128;            // rows of A per output tile: the padding unit of a row group
 constexpr int kGemmPairRows = 256;           // the same of a pair of SMs

@@ -15,13 +15,13 @@
 // kernel before to the end, a warp per key with a dependent softmax per key and one merging CTA / here, over 1000 cached keys: 16 heads of 128
 // over 4, one row 16 / 13, eight 53 / 33; 16 heads over latent rows of 256 + 32, one row 34 / 20, eight 34 / 29.
 #include <algorithm>
-#include <atomic>
 
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <math_constants.h>
 #include <stdint.h>
 
+#include "gemm_tcgen05.h"
 #include "lm_device.cuh"
 #include "lm_internal.h"
 
@@ -278,10 +278,10 @@ few_rows_attention_kernel(const __grid_constant__ FewAttention p, int cluster) {
 
 // CTAs of a row and head group that share its keys: a power of two, for up to four CTAs per SM, and 16 keys each at least where the window
 // or the chunk bounds them
-static int few_shares(int others, long long max_keys) {
+static int few_shares(int others, long long max_keys, int sms) {
     static_assert(kAttnSplitsMax <= 4 * kFewCluster, "clusters that the last merge reads");
     int S = 1;
-    while (S * 2 <= kAttnSplitsMax && others * S * 2 <= 4 * 148 && (long long)S * 16 < max_keys) S *= 2;
+    while (S * 2 <= kAttnSplitsMax && others * S * 2 <= 4 * sms && (long long)S * 16 < max_keys) S *= 2;
     return S;
 }
 static int few_heads(const FewAttention& p) {
@@ -302,19 +302,14 @@ bool few_rows_attention_ok(const FewAttention& p) {
 template <int HT>
 static cudaError_t launch_few(const FewAttention& p, int M, cudaStream_t st) {
     const size_t smem = (size_t)few_smem_floats(HT, p.kdim, p.vdim, p.shared_kv) * 4;
-    static std::atomic<bool> asked[64];
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
+    int dev = 0, sms = 0;
+    cudaError_t e = dia::current_sms(&dev, &sms);
+    if (e == cudaSuccess) e = dia::ask_smem<few_rows_attention_kernel<HT>>(dev, 220 * 1024);
     if (e != cudaSuccess) return e;
-    if (dev >= 64 || !asked[dev].load(std::memory_order_relaxed)) {
-        e = cudaFuncSetAttribute(few_rows_attention_kernel<HT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
-        if (e != cudaSuccess) return e;
-        if (dev < 64) asked[dev].store(true, std::memory_order_relaxed);
-    }
     const int rep = p.heads / p.kv_heads, groups = p.kv_heads * ((rep + HT - 1) / HT);
     long long max_keys = p.window > 0 ? (long long)p.window + p.keep_first : (long long)p.max_pages * p.page_size;
     if (p.chunk > 0) max_keys = std::min<long long>(max_keys, (long long)p.chunk + (p.window > 0 ? p.keep_first : 0));
-    const int S = few_shares(M * groups, max_keys), cluster = std::min(S, kFewCluster);
+    const int S = few_shares(M * groups, max_keys, sms), cluster = std::min(S, kFewCluster);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(S, groups, M);
     cfg.blockDim = dim3(kFewThreads);

@@ -24,6 +24,7 @@
 #include "attention_split.h"
 #include "common.cuh"
 #include "engine_internal.h"
+#include "gemm_tcgen05.h"
 
 namespace dia {
 
@@ -108,7 +109,7 @@ attention_rows_kernel(const float* __restrict__ q, const float* __restrict__ k, 
             *reinterpret_cast<float4*>(Vs + r * kHeadDim + c4 * 4) = vv;
         }
         __syncthreads();
-        // ---- S = Q K^T: rows ty*4 + i, columns tx + 16 j ----
+        // ---- S = Q K^T: rows ty*R + i, columns tx + 16 j ----
         float s[R][4];
 #pragma unroll
         for (int i = 0; i < R; ++i)
@@ -167,7 +168,7 @@ attention_rows_kernel(const float* __restrict__ q, const float* __restrict__ k, 
             for (int j = 0; j < 4; ++j) Ps[(ty * R + i) * kPStride + tx + 16 * j] = s[i][j];
         }
         __syncthreads();
-        // ---- O += P V: rows ty*4 + i, output dims tx*4 .. +3 and 64 + tx*4 .. +3 ----
+        // ---- O += P V: rows ty*R + i, output dims tx*4 .. +3 and 64 + tx*4 .. +3 ----
 #pragma unroll 2
         for (int c4 = 0; c4 < kAK / 4; ++c4) {
             float4 pa[R];
@@ -315,10 +316,13 @@ cudaError_t launch_attention_rows(const float* q, const float* k, const float* v
     }
     DelayArg nv{};
     for (int b = 0; b < B; ++b) nv.d[b] = n_valid_host ? n_valid_host[b] : Tk;
-    const bool small = (long long)((Tq + 63) / 64) * Hq * B < 148;
+    int dev = 0, sms = 0;
+    cudaError_t e = current_sms(&dev, &sms);
+    if (e != cudaSuccess) return e;
+    const bool small = (long long)((Tq + 63) / 64) * Hq * B < sms;
     const int AQ = small ? 32 : 64, bytes = small ? kAttnSmem<32> : kAttnSmem<64>;
     const auto kernel = small ? attention_rows_kernel<32> : attention_rows_kernel<64>;
-    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    e = small ? ask_smem<attention_rows_kernel<32>>(dev, bytes) : ask_smem<attention_rows_kernel<64>>(dev, bytes);
     if (e != cudaSuccess) return e;
     kernel<<<dim3((Tq + AQ - 1) / AQ, Hq, B), kAttnThreads, bytes, st>>>(q, k, v, out, Tq, Tk, Hq, Hkv, Tk_stride, mode, nv);
     return cudaGetLastError();
