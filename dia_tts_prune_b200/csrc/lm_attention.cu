@@ -29,6 +29,10 @@ namespace lm {
 namespace {
 
 constexpr int kFewKeys = 32, kFewThreads = 256, kFewWarps = 8, kFewCluster = 8;
+// Keys of a CTA at least, unless one cluster has room for all: a second cluster costs a merge through global memory (four layers of width 2048, steps of
+// one and of eight rows, us: over 100 keys 275 and 356 with all 32 CTAs, 257 and 319 with one cluster; over 600 keys with 16, 32 and 64 keys a CTA 277, 276
+// and 291, 372, 368 and 382)
+constexpr int kFewLeast = 32;
 
 __device__ __forceinline__ uint32_t shared_at(const void* local, uint32_t rank) {
     uint32_t a;
@@ -61,7 +65,7 @@ few_rows_attention_kernel(const __grid_constant__ FewAttention p, int cluster) {
     __shared__ int s_last;
     pdl_release();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int S = gridDim.x, sp = blockIdx.x, rank = sp % cluster, r = blockIdx.z;
+    const int sp = blockIdx.x, rank = sp % cluster, cl = sp / cluster, r = blockIdx.z;
     const int rep = p.heads / p.kv_heads, chunks = (rep + HT - 1) / HT, g = blockIdx.y / chunks, h0 = g * rep + (blockIdx.y % chunks) * HT;
     const int nh = min(HT, (g + 1) * rep - h0), kdim = p.kdim, vdim = p.vdim, KS = kdim + 4, K4 = kdim >> 2;
     float* Q = sm;                                            // [HT][kdim]
@@ -75,7 +79,10 @@ few_rows_attention_kernel(const __grid_constant__ FewAttention p, int cluster) {
     float *m_s = stat + HT, *l_s = m_s + HT, *all_m = l_s + HT, *w_s = all_m + HT;      // w_s: [HT][8] weights of the cluster's shares
     pdl_wait();
     const int i = p.row_pos[r], lo = first_key(i, p.window, p.chunk), n_keep = p.window > 0 ? min(p.keep_first, lo) : 0;
-    const int n_keys = n_keep + (i - lo + 1), per = ((n_keys + S - 1) / S + 3) & ~3, k0 = min(n_keys, sp * per), k1 = min(n_keys, k0 + per);
+    // as many clusters as the keys that are there fill (the grid has room for those that there may be)
+    const int n_keys = n_keep + (i - lo + 1), shares = min((int)gridDim.x / cluster, (n_keys + cluster * kFewLeast - 1) / (cluster * kFewLeast));
+    if (cl >= shares) return;                                 // (all its CTAs)
+    const int S = shares * cluster, per = ((n_keys + S - 1) / S + 3) & ~3, k0 = min(n_keys, sp * per), k1 = min(n_keys, k0 + per);
     const int* pages = p.table + (size_t)p.row_slot[r] * p.max_pages;
     auto gather = [&](int t0, int buf) {                      // keys t0 .. of the share: warp w rows 4 w .. + 3
         size_t at[4];
@@ -204,7 +211,6 @@ few_rows_attention_kernel(const __grid_constant__ FewAttention p, int cluster) {
         if (lane == 0) { all_m[hh] = m; stat[hh] = l; }
     }
     __syncthreads();
-    const int shares = S / cluster, cl = sp / cluster;        // clusters of this row and head group
     const size_t stride = (size_t)vdim + 2;
     auto finish = [&](int hh, int c, float o) {
         const int h = h0 + hh;
