@@ -1029,7 +1029,9 @@ split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_co
         // (first) or as taken by the first group; inv: where the scales go (null: they are there); ready: told when they are
         auto stage = [&](const float* cache, int width, int row_w, int c0, int w, int wp, int gg, const size_t (&rows)[2], float (&m_row)[2],
                          bool first, float* inv, uint64_t* ready) {
-            constexpr int KG = RT == 4 ? 1 : 2;               // groups of eight keys at a time (16 float4 of two do not fit 64 registers)
+            // groups of eight keys at a time: 16 float4 of two do not fit 64 or 80 registers (us, wide values, two / one: nine sequences over
+            // 1134 keys that the room for split keys does not hold 320 / 241, 4096 rows over latent rows of 256 + 32 440 / 405)
+            constexpr int KG = RT == 4 || NVS == 2 ? 1 : 2;
             const unsigned slot = at % geo.n_slots;
 #pragma unroll 1
             for (int half = 0; half < 2; half += KG) {
