@@ -797,7 +797,7 @@ bool talk_attention_supported(const TalkShape& a) {
            a.heads <= talk_max_pairs(a.vdim) && talk_smem(a, 1) <= 200 * 1024;
 }
 
-// split_ws: kAttnRowsKernelMax * heads * kAttnSplitsMax * (vdim + 2) floats; arrived: kAttnRowsKernelMax zeroed counters.
+// split_ws: kAttnRowsKernelMax * heads * kAttnSplitsMax * (vdim + 2) floats; arrived: kAttnRowsKernelMax * heads zeroed counters.
 // Prompt portions run 16 warps per CTA (up to 8 pairs per warp: half the accumulators of an 8-warp CTA, twice the warps
 // to hide the latencies of a tile's dependent phases); a handful of rows run 8 warps per (row, share of the keys).
 cudaError_t launch_talk_attention(const float* proj, int ld, int q_off, int gate_off, const float* kcache, const float* vcache,
