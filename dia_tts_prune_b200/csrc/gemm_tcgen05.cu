@@ -493,7 +493,9 @@ dia_gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
 // of two of its own; an accumulator lives for kPairChunk k-blocks and eight epilogue warps add it to the tile's sums in their registers (two
 // threads per row, up to 128 columns each) while the next ones are multiplied into the other.  Against three terms and sums of all products
 // in tensor memory: 1722 rows, K = 2048, 16384 columns 209 -> 162 us, 2048 columns 37 -> 28, K = 8192 118 -> 85; relative error 7.0e-6 -> 5.8e-7
-// (861 rows through Dia's decoder 2.8e-5 -> 4.1e-6).  Chunks of 1, 2 and 4 k-blocks: 282, 215 and 162 us, 1.5e-7, 2.9e-7 and 5.8e-7 (the
+// (861 frames through two of Dia's decoder layers 1.25e-5 -> 3.9e-6).  A row's numbers keep 22 bits where three terms kept 24, which the sums make up
+// for: over Dia's widths and 130 to 3000 rows (normal, gated, positive numbers) 5.8e-7 to 9.0e-7 against 3.5e-6 to 4.0e-5, and 1.2e-6 against 3.5e-6
+// in columns that see only the other numbers of rows with one 2^20 times as large.  Chunks of 1, 2 and 4 k-blocks: 282, 215 and 162 us, 1.5e-7, 2.9e-7 and 5.8e-7 (the
 // accumulators of a chunk are read while the MMAs update the others, and the two slow each other down).
 template <bool SUMS>
 struct Pair {

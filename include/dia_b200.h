@@ -239,7 +239,8 @@ int dia_b200_dense_forward_fused(const float *x, const float *norm_weight, float
                                  const float *residual, float *y, void *workspace, int M, int N, int K, void *stream);
 
 /* The same for many rows (dia_b200_dense_half_rows says which): x as two fp16 terms with a power of two per row, W as the K-major fp16 copy
- * wt_half[N][K] with a power of two per column, products summed in fp32.  magnitudes: float32 [N], the columns' largest magnitudes.
+ * wt_half[N][K] with a power of two per column, pieces of 256 products summed in fp32.  A
+ * row's numbers keep 22 bits, those below 2^-17 of its largest are off by up to 2^-39 of that.  magnitudes: float32 [N], the columns' largest magnitudes.
  * prepare_half sets *inexact (device int32, zeroed by the caller) where fp16 cannot hold the bf16 weights, beyond 2^31 between a column's
  * largest and smallest value: such weights stay with dense_forward_fused.  gated: x is [M][2][K], and the rows are silu(x[m][0]) x[m][1]
  * (norm_weight NULL).  x, norm_weight and all buffers 16-byte aligned; K % 64 == 0 and N % 4 == 0. */

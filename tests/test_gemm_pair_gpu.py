@@ -88,6 +88,29 @@ def test_two_fp16_terms(M, N, K, gated, norm, residual):
     assert ((got - ref).abs() <= 2.0 ** -23 * (8 + 34 + K / 256) * size).all()
 
 
+@pytest.mark.parametrize("M,N,K", [(600, 16384, 2048), (1722, 2048, 2048), (1722, 2048, 8192), (1000, 8192, 1024)])
+@pytest.mark.parametrize("rows", ["normal", "gated", "positive", "outlier"])
+def test_two_fp16_terms_beside_three_bf16_terms(M, N, K, rows):
+    """The widths of Dia's layers: 22 bits of a row's numbers and sums of 256 products are nowhere further off than 24 bits and one sum of all products
+    on the tensor cores (an addition that cuts off per 16 products and term), which these rows would take.  Outlier: a channel 2^16 times the others,
+    and columns with a zero weight there, which see the others alone."""
+    from dia_tts_prune_b200 import engine
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    x, w = torch.randn((M, K), generator=g, device="cuda"), (torch.randn((K, N), generator=g, device="cuda") * K ** -0.5).bfloat16()
+    if rows == "gated":
+        x = torch.nn.functional.silu(2 * x) * torch.randn((M, K), generator=g, device="cuda") * 3
+    elif rows == "positive":
+        x, w = x.abs(), w.abs()
+    elif rows == "outlier":
+        x[:, 5], w[5] = 2.0 ** 16, 0.0
+    assert engine.dense_half_rows(M, N, K, x.device)
+    two = engine.dense_forward_half(x, engine.dense_prepare_half(w, torch.zeros((1,), dtype=torch.int32, device="cuda")))
+    three, ref = engine.dense_forward(x, engine.dense_prepare_weight(w)), x.double() @ w.double()
+    off, was = (two - ref).norm() / ref.norm(), (three - ref).norm() / ref.norm()
+    # 16 additions per accumulator that cut off half a unit of 2^-23 each, as a bias where all numbers are positive; K / 256 rounded ones
+    assert off <= was and off <= 2.0 ** -23 * 10
+
+
 def test_two_fp16_terms_at_the_ends_of_fp32():
     """Rows of the smallest and the largest numbers, zeros, infinities and NaNs beside ordinary ones, against three bf16 terms."""
     from dia_tts_prune_b200 import engine
