@@ -27,7 +27,7 @@ import contextlib
 import math
 import os
 import weakref
-from typing import Optional
+from typing import Callable, Optional
 
 import torch
 import torch.nn as nn
@@ -383,12 +383,13 @@ def _check_caches(name: str, k: Tensor, v: Tensor, B: int, device: torch.device)
         raise ValueError(f"{name} cache: keys {tuple(k.shape)}, values {tuple(v.shape)}")
 
 
-def _rows_layer(x: Tensor, attn: Attention, norm: RMSNorm, mlp: MlpBlock, norm_mlp: RMSNorm, eps: float, positions_i32: Tensor, tables,
+def _rows_layer(x: Tensor, attn: Attention, norm: RMSNorm, mlp: MlpBlock, norm_mlp: RMSNorm, eps: float, positions: Callable[[], Tensor], tables,
                 mode: int, n_valid: list[int] | None, k: Tensor, v: Tensor, cross: tuple | None = None, out: Tensor | None = None) -> Tensor:
     """One layer over ``x [B, T, D]`` (float32, contiguous) on our kernels, in one native call: RMSNorm in the split pass of the projections, RoPE with
     the scatter into the caches ``k``, ``v [B, heads, slots, 128]``, attention, residual adds in the epilogues, the gate in the split pass of
     the last product.  ``mode``: 0 causal, 1 pad-partitioned at ``n_valid``.  ``cross``: (attention, norm, cache, valid keys) of a cross-attention
-    behind the self-attention.  The result is in ``out`` (``x`` itself, say) or a new tensor."""
+    behind the self-attention.  The result is in ``out`` (``x`` itself, say) or a new tensor.  ``positions`` gives int32 ``[B * T]`` and is asked last: where
+    they have to be made, their copy waits for the device, which then has the layer's launches to do at once."""
     from . import engine as _k
     B, T, D = x.shape
     y = torch.empty_like(x) if out is None else out
@@ -404,18 +405,20 @@ def _rows_layer(x: Tensor, attn: Attention, norm: RMSNorm, mlp: MlpBlock, norm_m
         _check_caches("cross-attention", cc.k, cc.v, B, x.device)
         if not cc.k.shape[1] or ca.num_query_heads % cc.k.shape[1]:
             raise ValueError(f"cross-attention cache {tuple(cc.k.shape)} for {ca.num_query_heads} query heads")
-    if positions_i32.numel() < B * T or positions_i32.dtype != torch.int32 or positions_i32.device != x.device:
-        raise ValueError(f"{B * T} int32 positions are read")
     a = RowsLayer(D=D, eps=eps)
     keep = _rows_weights(a, B * T, attn, norm, mlp, norm_mlp, ca, cn, x.device)
     a.B, a.T, a.slots, a.mode, a.n_pos = B, T, k.shape[2], mode, tables[0].shape[0]
-    a.x_in, a.x, a.positions = x.data_ptr(), y.data_ptr(), positions_i32.data_ptr()
+    a.x_in, a.x = x.data_ptr(), y.data_ptr()
     a.sin_table, a.cos_table, a.k_cache, a.v_cache = tables[0].data_ptr(), tables[1].data_ptr(), k.data_ptr(), v.data_ptr()
     if n_valid is not None:
         a.n_valid[:B] = [int(n) for n in n_valid]
     if cc is not None:
         a.cross_kv_heads, a.cross_slots, a.cross_k, a.cross_v = cc.k.shape[1], cc.k.shape[2], cc.k.data_ptr(), cc.v.data_ptr()
         a.cross_valid[:B] = [int(n) for n in valid]
+    pos = positions()
+    if pos.numel() < B * T or pos.dtype != torch.int32 or pos.device != x.device:
+        raise ValueError(f"{B * T} int32 positions are read")
+    a.positions = pos.data_ptr()
     _k.rows_layer_forward(a, _k.rows_layer_work_bytes(a), x.device)
     del keep
     return y
@@ -438,11 +441,15 @@ class EncoderLayer(nn.Module):
             eps = self.config.model.normalization_layer_epsilon
             B, T, _ = x.shape
             x = x.to(torch.float32).contiguous()
-            pos = state.extras.get("pos_i32")
-            if pos is None or pos.numel() != B * T:
-                pos = state.extras["pos_i32"] = _k.positions_i32(T, B, x.device)
+
+            def positions():
+                pos = state.extras.get("pos_i32")
+                if pos is None or pos.numel() != B * T:
+                    pos = state.extras["pos_i32"] = _k.positions_i32(T, B, x.device)
+                return pos
+
             kv = torch.empty((2, B, self.self_attention.num_kv_heads, T, 128), dtype=torch.float32, device=x.device)
-            return _rows_layer(x, self.self_attention, self.pre_sa_norm, self.mlp, self.post_sa_norm, eps, pos,
+            return _rows_layer(x, self.self_attention, self.pre_sa_norm, self.mlp, self.post_sa_norm, eps, positions,
                                _k.rope_tables_device(self.config, x.device), 1, _encoder_valid_lens(state), kv[0], kv[1])
         h = self.pre_sa_norm(x.float())
         x = x + self.self_attention(h, h, state.positions, state.positions, attn_mask=state.attn_mask)
@@ -529,10 +536,13 @@ class DecoderLayer(nn.Module):
             eps = self.config.model.normalization_layer_epsilon
             B, T, _ = x.shape
             tables = _k.rope_tables_device(self.config, x.device)
-            pos = state.extras.get("prefill_pos")
-            if pos is None or pos.numel() != B * T:
-                pos = _k.positions_i32(state.step_to - state.step_from, B, x.device, start=state.step_from)
-                state.extras["prefill_pos"] = pos
+
+            def positions():
+                pos = state.extras.get("prefill_pos")
+                if pos is None or pos.numel() != B * T:
+                    pos = state.extras["prefill_pos"] = _k.positions_i32(state.step_to - state.step_from, B, x.device, start=state.step_from)
+                return pos
+
             if state.text_len is None:
                 raise NotImplementedError("prefill needs DecoderInferenceState.text_len (valid text bytes)")
             x = x.to(torch.float32).contiguous()
@@ -545,7 +555,7 @@ class DecoderLayer(nn.Module):
                 k, v = torch.empty((2, B, self.self_attention.num_kv_heads, T, 128), dtype=torch.float32, device=x.device)
             if cross_attn_cache is None:
                 raise NotImplementedError("cross-attention needs the precomputed K/V cache")
-            return _rows_layer(x, self.self_attention, self.pre_sa_norm, self.mlp, self.pre_mlp_norm, eps, pos, tables, 0, None, k, v,
+            return _rows_layer(x, self.self_attention, self.pre_sa_norm, self.mlp, self.pre_mlp_norm, eps, positions, tables, 0, None, k, v,
                                (self.cross_attention, self.pre_ca_norm, cross_attn_cache, [0] * (B - 1) + [state.text_len]),
                                out=x if x.data_ptr() % 16 == 0 else None)
         # CPU (state-dict tooling and the CPU test suite): the reference's own formulation

@@ -58,7 +58,7 @@ def run(layer, T, B=1, k=None, v=None, cross=None, cross_heads=4):
         ca = (layer.cross_attention, layer.pre_ca_norm, KVCache.from_kv(ck, cv), [8] * B)
     norm, norm_mlp = (layer.pre_sa_norm, layer.pre_mlp_norm) if ca else (layer.pre_sa_norm, layer.post_sa_norm)
     with torch.no_grad():
-        return _rows_layer(torch.randn(B, T, D), sa, norm, layer.mlp, norm_mlp, 1e-5, pos, tables, 0 if ca else 1, None if ca else [T] * B,
+        return _rows_layer(torch.randn(B, T, D), sa, norm, layer.mlp, norm_mlp, 1e-5, lambda: pos, tables, 0 if ca else 1, None if ca else [T] * B,
                            torch.zeros(shape) if k is None else k, torch.zeros(shape) if v is None else v, ca)
 
 

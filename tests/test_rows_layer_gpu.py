@@ -106,7 +106,7 @@ def test_projections_keep_their_sums(width, heads, kv_heads, B, T):
     x = torch.randn((B, T, width), generator=g, device="cuda")
     k, v = torch.zeros((2, B, kv_heads, T, 128), device="cuda")
     with torch.inference_mode():
-        _rows_layer(x, sa, layer.pre_sa_norm, layer.mlp, layer.post_sa_norm, 1e-5, engine.positions_i32(T, B, x.device), engine.rope_tables_device(cfg, x.device),
+        _rows_layer(x, sa, layer.pre_sa_norm, layer.mlp, layer.post_sa_norm, 1e-5, lambda: engine.positions_i32(T, B, x.device), engine.rope_tables_device(cfg, x.device),
                     0, None, k, v)
     want = dense(rms(x.double(), layer.pre_sa_norm), sa.v_proj).reshape(B, T, kv_heads, 128).transpose(1, 2)
     assert (v - want).norm() <= 1e-6 * want.norm()
