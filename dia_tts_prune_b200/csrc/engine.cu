@@ -1127,11 +1127,12 @@ int dia_b200_rows_layer_forward(const dia_b200_rows_layer* args, void* stream) {
     int rc;
     // Projections whose K-major copies lie one behind the other may be one product, summed as they would be by themselves: a stacked product has
     // so many columns that it would leave the kernel of fp32 sums earlier (768 encoder rows, D = 1024, 3 x 2048 columns: relative error of the values
-    // 1.5e-7, and 7e-6 on the kernel that its columns ask for).  The split that ends first, at seven k-blocks for a launch and its split of the rows.
+    // 1.5e-7, and 7e-6 on the kernel that its columns ask for).  The split that ends first, at ten k-blocks for a launch and its split of the rows
+    // (texts of 450 bytes, 12 layers: with seven, q apart from k and v, 2512 us, with ten 2430; with seventeen the same).
     auto follows = [&](const dia_b200_dense_ref& u, const dia_b200_dense_ref& w, int n) {
         return !u.wt_half && !w.wt_half && static_cast<const unsigned char*>(u.wt_bf16) + (size_t)n * D * 2 == w.wt_bf16;
     };
-    constexpr int kStart = 7;
+    constexpr int kStart = 10;
     const bool kv_next = follows(a.k, a.v, nk), all_next = kv_next && follows(a.q, a.k, nq);
     const int bq = a.q.wt_half ? 0 : gemm_sums_blocks(M, nq, D, false), bk = a.k.wt_half ? 0 : gemm_sums_blocks(M, nk, D, false);      // (0: other sums)
     const int b_kv = gemm_sums_blocks(M, 2 * nk, D, true), apart = bk ? std::min(b_kv + kStart, 2 * (bk + kStart)) : 0;
