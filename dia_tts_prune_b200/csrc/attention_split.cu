@@ -27,8 +27,8 @@
 // value 5 us each; 16 keys that share a factor (scales in steps of 2^8) take as long.
 //
 // Bound: the instructions of the row warps and their latencies.  Per 64 keys and 128 rows 3 x 128 x 64 x (dk + dv) multiply-adds on the tensor
-// pipe (1536 cycles at 128 + 128) stand against about 6400 cycles of a tile, on 2900 of which a scheduler issues (four row warps on each;
-// with two row warps 7000 and 2400).  Instruction fetches and fixed latencies are the largest waits.
+// pipe (1536 cycles at 128 + 128) stand against about 8000 cycles of a tile with its share of the CTA's start and end, on 47 % of which a scheduler
+// issues (four row warps on each; with two row warps 8800 and 34 %; profiles/split_kernels_ncu.txt).
 // Every wait is bounded: a wait that runs out makes the CTA write NaN, note it in a word that the host reads, and end; the next launch
 // on the device returns an error.
 #include <algorithm>

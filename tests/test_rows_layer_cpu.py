@@ -135,12 +135,14 @@ def test_a_replaced_part_is_read(calls):
     """Another kernel, attention or MLP in the layer's place of one: its copies are read, not those of the one before"""
     layer, other = filled(EncoderLayer(config(), torch.bfloat16)), filled(EncoderLayer(config(), torch.bfloat16))
     run(layer, 5)
+    kept = layer.mlp.wo, layer.self_attention                     # (their copies' addresses are not given to others)
     layer.mlp.wo = other.mlp.wo
     run(layer, 5)
     assert calls[-1].wo.wt_bf16 == other.mlp.wo.kernel_weight_kmajor().data_ptr() != calls[0].wo.wt_bf16
     layer.self_attention = other.self_attention
     run(layer, 5)
     assert calls[-1].o.wt_bf16 == other.self_attention.o_proj.kernel_weight_kmajor().data_ptr() != calls[0].o.wt_bf16
+    assert calls[0].wo.wt_bf16 == kept[0].kernel_weight_kmajor().data_ptr()
 
 
 def test_numbers_of_rows_share_their_arguments(calls, monkeypatch):
