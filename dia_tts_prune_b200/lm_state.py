@@ -80,8 +80,7 @@ class PagedState:
         self.rec_states, self.rec_aux = [r.rec_state for r in self.records], [r.rec_aux for r in self.records]
         self.latent_pages = [r.latent_pages for r in self.records]
         self.token_pages = torch.zeros((self.n_pages, self.page_size), dtype=torch.int32, device=self.device) if keep_tokens else None
-        self._table_host = torch.zeros((self.n_slots, self.max_pages), dtype=torch.int32).pin_memory() \
-            if self.device.type == "cuda" else torch.zeros((self.n_slots, self.max_pages), dtype=torch.int32)
+        self._table_host = torch.zeros((self.n_slots, self.max_pages), dtype=torch.int32)
         self.page_table = torch.zeros((self.n_slots, self.max_pages), dtype=torch.int32, device=self.device)
         self._dirty = False
         self._free_pages = list(range(self.n_pages - 1, -1, -1))        # pop() takes page 0 first
@@ -158,8 +157,12 @@ class PagedState:
         seq.pages = []
 
     def sync_table(self) -> torch.Tensor:
-        """The device page table, refreshed if pages were taken since the last call (stream-ordered copy)."""
+        """The device page table, refreshed if pages were taken since the last call (stream-ordered copy).  The copy may run long after the call: it reads
+        a table of its own, which later steps do not write (the pinned block is taken again once it has been read)."""
         if self._dirty:
-            self.page_table.copy_(self._table_host, non_blocking=True)
+            table = self._table_host
+            if self.device.type == "cuda":
+                table = torch.empty(table.shape, dtype=table.dtype, pin_memory=True).copy_(table)
+            self.page_table.copy_(table, non_blocking=True)
             self._dirty = False
         return self.page_table

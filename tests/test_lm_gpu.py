@@ -301,6 +301,33 @@ def test_freed_pages_and_slots_are_used_again():
 
 
 # ---- a key that stands out: far away, at page borders, at the window's and the kept prefix's edges ----------------------
+def test_steps_queued_behind_one_another():
+    """Steps whose requests take other pages each time, queued while the device has not begun the first: each reads its own pages.  (The copies of the page
+    table run long after the calls.)"""
+    cfg = small_config()
+    model, _ = build(cfg, 21, max_sequences=2, page_size=4)
+    prompts = [[tokens(cfg, n, 100 + 10 * i + k) for k, n in enumerate((23, 9))] for i in range(4)]
+
+    def step(i):
+        entries = [{"id": f"{i}.{k}", "tokens": t, "want": [len(t) - 1]} for k, t in enumerate(prompts[i])]
+        return model.run_step(entries, [e["id"] for e in entries])
+
+    def passes(wait):
+        out = []
+        if not wait:
+            torch.cuda._sleep(400_000_000)                        # (about 0.2 s, which the device is busy for)
+        for i in (0, 1, 2, 3, 0, 2):
+            if wait:
+                torch.cuda.synchronize()
+            out.append(step(i).clone())
+        torch.cuda.synchronize()
+        return out
+
+    want = passes(True)
+    got = passes(False)
+    assert all(torch.equal(a, b) for a, b in zip(got, want))
+
+
 def standout_model(size, keep, page_size):
     """One layer whose query and key projections coincide, so that a position whose input equals the query's input gets a
     score far above all others; a small distance slope keeps far keys visible."""
