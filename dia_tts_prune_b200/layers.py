@@ -411,7 +411,9 @@ def _rows_layer(x: Tensor, attn: Attention, norm: RMSNorm, mlp: MlpBlock, norm_m
     a.x_in, a.x = x.data_ptr(), y.data_ptr()
     a.sin_table, a.cos_table, a.k_cache, a.v_cache = tables[0].data_ptr(), tables[1].data_ptr(), k.data_ptr(), v.data_ptr()
     if n_valid is not None:
-        a.n_valid[:B] = [int(n) for n in n_valid]
+        if len(n_valid) > min(B, 16):
+            raise ValueError(f"{len(n_valid)} numbers of valid keys for a batch of {B} (16 at most)")
+        a.n_valid[:len(n_valid)] = [int(n) for n in n_valid]      # (rows without one have none)
     if cc is not None:
         a.cross_kv_heads, a.cross_slots, a.cross_k, a.cross_v = cc.k.shape[1], cc.k.shape[2], cc.k.data_ptr(), cc.v.data_ptr()
         a.cross_valid[:B] = [int(n) for n in valid]

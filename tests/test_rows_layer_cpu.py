@@ -43,7 +43,7 @@ def filled(layer):
     return layer
 
 
-def run(layer, T, B=1, k=None, v=None, cross=None, cross_heads=4):
+def run(layer, T, B=1, k=None, v=None, cross=None, cross_heads=4, valid=None):
     """The layer's native call for ``[B, T]`` rows; ``cross``: the (keys, values) of a decoder layer's cross-attention."""
     from dia_tts_prune_b200.layers import _rows_layer
     from dia_tts_prune_b200.state import KVCache
@@ -58,7 +58,7 @@ def run(layer, T, B=1, k=None, v=None, cross=None, cross_heads=4):
         ca = (layer.cross_attention, layer.pre_ca_norm, KVCache.from_kv(ck, cv), [8] * B)
     norm, norm_mlp = (layer.pre_sa_norm, layer.pre_mlp_norm) if ca else (layer.pre_sa_norm, layer.post_sa_norm)
     with torch.no_grad():
-        return _rows_layer(torch.randn(B, T, D), sa, norm, layer.mlp, norm_mlp, 1e-5, lambda: pos, tables, 0 if ca else 1, None if ca else [T] * B,
+        return _rows_layer(torch.randn(B, T, D), sa, norm, layer.mlp, norm_mlp, 1e-5, lambda: pos, tables, 0 if ca else 1, None if ca else [T] * B if valid is None else valid,
                            torch.zeros(shape) if k is None else k, torch.zeros(shape) if v is None else v, ca)
 
 
@@ -177,3 +177,15 @@ def test_copies_that_are_there_stay(calls):
     kept = [sa.k_proj.kernel_weight_kmajor()]                     # (the product was called by itself before)
     run(layer, 5)
     assert sa.k_proj.kernel_weight_kmajor() is kept[0] and calls[-1].k.wt_bf16 == kept[0].data_ptr()
+
+
+def test_numbers_of_valid_keys(calls):
+    """One per batch row, none for the rows that have no number"""
+    layer = filled(EncoderLayer(config(), torch.bfloat16))
+    run(layer, 5, B=3, valid=[4])
+    assert list(calls[-1].n_valid)[:3] == [4, 0, 0] and calls[-1].B == 3
+    with pytest.raises(ValueError):
+        run(layer, 5, B=1, valid=[4, 4])
+    with pytest.raises(ValueError):
+        run(layer, 5, B=17)
+    assert len(calls) == 1
