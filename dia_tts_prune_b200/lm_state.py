@@ -157,11 +157,12 @@ class PagedState:
         seq.pages = []
 
     def sync_table(self) -> torch.Tensor:
-        """The device page table, refreshed if pages were taken since the last call (stream-ordered copy).  The copy may run long after the call: it reads
-        a table of its own, which later steps do not write (the pinned block is taken again once it has been read)."""
+        """The device page table, refreshed if pages were taken since the last call (stream-ordered copy).  The copy may run long after the call, when the
+        host's table holds a later step's pages: a small one is staged by the call, a larger one gets a pinned block of its own (which is not taken
+        again before it has been read)."""
         if self._dirty:
             table = self._table_host
-            if self.device.type == "cuda":
+            if self.device.type == "cuda" and table.numel() > 4096:
                 table = torch.empty(table.shape, dtype=table.dtype, pin_memory=True).copy_(table)
             self.page_table.copy_(table, non_blocking=True)
             self._dirty = False

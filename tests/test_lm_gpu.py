@@ -301,11 +301,12 @@ def test_freed_pages_and_slots_are_used_again():
 
 
 # ---- a key that stands out: far away, at page borders, at the window's and the kept prefix's edges ----------------------
-def test_steps_queued_behind_one_another():
-    """Steps whose requests take other pages each time, queued while the device has not begun the first: each reads its own pages.  (The copies of the page
+@pytest.mark.parametrize("longest", [512, 16384])
+def test_steps_queued_behind_one_another(longest):
+    """Page tables of 256 and 8192 numbers.  Steps whose requests take other pages each time, queued while the device has not begun the first: each reads its own pages.  (The copies of the page
     table run long after the calls.)"""
     cfg = small_config()
-    model, _ = build(cfg, 21, max_sequences=2, page_size=4)
+    model, _ = build(cfg, 21, max_sequences=2, page_size=4, max_sequence_tokens=longest)
     prompts = [[tokens(cfg, n, 100 + 10 * i + k) for k, n in enumerate((23, 9))] for i in range(4)]
 
     def step(i):
