@@ -110,13 +110,13 @@ class DenseGeneral(nn.Module):
     # ---- sm_100a path (encoder, cross-attention K/V precompute, prompt prefill) ----------------------------------
     def kernel_weight_kmajor(self) -> Tensor:
         """The K-major bf16 copy ``[N, K]`` of the kernel the tcgen05 GEMM reads (made once per weight version)."""
+        if not self._has_kmajor():
+            make_kmajor_kernels([[self]])
+        return self._b200_wt[1]
+
+    def _has_kmajor(self) -> bool:
         cached = self.__dict__.get("_b200_wt")
-        if cached is None or cached[0] != self._weight_key():
-            from . import engine as _engine
-            canonicalize_dense_kernel_(self)
-            wt = _engine.dense_prepare_weight(self.weight.detach().reshape(math.prod(self.in_shapes), math.prod(self.out_features)))
-            cached = self._b200_wt = (self._weight_key(), wt)
-        return cached[1]
+        return cached is not None and cached[0] == self._weight_key()
 
     def kernel_weight_half(self) -> tuple[Tensor, Tensor] | None:
         """The fp16 copy that products of many rows read (made once per weight version), or None: fp16 cannot hold these weights, or the
@@ -166,6 +166,24 @@ def _plain(*tensors: Tensor | None) -> bool:
 
 
 @torch.no_grad()
+def make_kmajor_kernels(groups: list[list["DenseGeneral"]]) -> None:
+    """K-major copies of these kernels, those of a group one behind the other (products of the same rows may then be one product).  Any stream may read a
+    copy once it is kept, so they are waited for (but for a capture, whose graph makes them)."""
+    from . import engine as _engine
+    made = []
+    for modules in groups:
+        for m in modules:
+            canonicalize_dense_kernel_(m)
+        K, sizes = math.prod(modules[0].in_shapes), [math.prod(m.out_features) for m in modules]
+        rows = torch.empty((sum(sizes), K), dtype=torch.bfloat16, device=modules[0].weight.device)
+        made += [(m, _engine.dense_prepare_weight(m.weight.detach().reshape(K, out.shape[0]), out)) for m, out in zip(modules, rows.split(sizes))]
+    if rows.is_cuda and not torch.cuda.is_current_stream_capturing():
+        torch.cuda.current_stream(rows.device).synchronize()
+    for m, wt in made:
+        m._b200_wt = (m._weight_key(), wt)
+
+
+@torch.no_grad()
 def prepare_half_kernels(modules: list["DenseGeneral"]) -> None:
     """The fp16 copies of these kernels, with one look at whether they are exact for all of them."""
     from . import engine as _engine
@@ -183,15 +201,6 @@ def prepare_half_kernels(modules: list["DenseGeneral"]) -> None:
               for i, m in enumerate(todo)]
     for m, half, inexact in zip(todo, halves, flags.tolist()):
         m._b200_half = (m._weight_key(), None if inexact else half)
-
-
-def _prepare_for_rows(module: nn.Module, probe: "DenseGeneral", M: int) -> None:
-    """The fp16 copies of those dense kernels inside ``module`` whose products of ``M`` rows read them, unless ``probe`` has its own."""
-    from . import engine as _engine
-    cached = probe.__dict__.get("_b200_half")
-    if M > 128 and (cached is None or cached[0] != probe._weight_key()) and not torch.cuda.is_current_stream_capturing():
-        prepare_half_kernels([m for m in module.modules() if isinstance(m, DenseGeneral) and m.weight.is_cuda and
-                              _engine.dense_half_rows(M, math.prod(m.out_features), math.prod(m.in_shapes), m.weight.device)])
 
 
 _ROUNDING_WARNED = False
@@ -315,18 +324,47 @@ class Attention(nn.Module):
         return self.o_proj(out.transpose(1, 2).contiguous()).to(Xq.dtype)
 
 
-def _stack_kmajor(modules: list["DenseGeneral"]) -> None:
-    """K-major copies of these kernels, one behind the other (products of the same rows may then be one product), where none of them has one yet:
-    a copy that is there may be read by another stream or a captured graph, and stays while its weights do."""
-    if any((c := m.__dict__.get("_b200_wt")) is not None and c[0] == m._weight_key() for m in modules) or len({math.prod(m.in_shapes) for m in modules}) > 1:
+def _rows_kernels(D: int, attn: Attention, mlp: MlpBlock, cross: Attention | None) -> tuple[list[DenseGeneral], tuple[tuple[int, int], ...]]:
+    """The dense kernels of a native layer call in its order, and the sizes ``(N, K)`` with which it reads them."""
+    wo = mlp.wo
+    F, Nq, Nk = wo.in_shapes[0], attn.num_query_heads * 128, attn.num_kv_heads * 128
+    modules, sizes = [attn.q_proj, attn.k_proj, attn.v_proj, attn.o_proj, mlp.wi_fused, wo], ((Nq, D), (Nk, D), (Nk, D), (D, Nq), (2 * F, D), (D, F))
+    if cross is not None:
+        Nc = cross.num_query_heads * 128
+        modules += (cross.q_proj, cross.o_proj)
+        sizes += ((Nc, D), (D, Nc))
+    return modules, sizes
+
+
+def _kmajor_groups(modules: list[DenseGeneral], missing: list[DenseGeneral]) -> list[list[DenseGeneral]]:
+    """How the missing K-major copies of a layer's kernels are made: q, k and v together, whichever of them is missing, unless one has a copy - that may be read
+    by another stream or a captured graph, and stays while its weights do."""
+    group = modules[:3] if any(m in missing for m in modules[:3]) and not any(m._has_kmajor() for m in modules[:3]) else []
+    if len({math.prod(m.in_shapes) for m in group}) > 1:
+        group = []                                                # (not products of the same rows)
+    return ([group] if group else []) + [[m] for m in missing if m not in group]
+
+
+def _prepare_for_rows(layers, M: int, D: int, device: torch.device) -> None:
+    """The copies that calls of ``M`` rows read of all of these layers, with one look at them and one wait, where the last layer has none
+    of its own yet."""
+    from . import engine as _k
+    def kernels_of(layer):
+        return _rows_kernels(D, layer.self_attention, layer.mlp, getattr(layer, "cross_attention", None))
+
+    modules, sizes = kernels_of(layers[-1])
+    probe, two = modules[5], _k.dense_half_choice(M, sizes, device)[5]
+    half = probe.__dict__.get("_b200_half")
+    if (half is not None and half[0] == probe._weight_key() if two else probe._has_kmajor()) or torch.cuda.is_current_stream_capturing():
         return
-    from . import engine as _engine
-    for m in modules:
-        canonicalize_dense_kernel_(m)
-    K, sizes = math.prod(modules[0].in_shapes), [math.prod(m.out_features) for m in modules]
-    rows = torch.empty((sum(sizes), K), dtype=torch.bfloat16, device=modules[0].weight.device)
-    for m, out in zip(modules, rows.split(sizes)):
-        m._b200_wt = (m._weight_key(), _engine.dense_prepare_weight(m.weight.detach().reshape(K, out.shape[0]), out))
+    kernels = [kernels_of(layer) for layer in layers]
+    choices = [_k.dense_half_choice(M, sizes, device) for _, sizes in kernels]
+    prepare_half_kernels([m for (modules, _), choice in zip(kernels, choices) for m, two in zip(modules, choice) if two])
+    groups = []
+    for (modules, _), choice in zip(kernels, choices):
+        groups += _kmajor_groups(modules, [m for m, two in zip(modules, choice) if not (two and m.kernel_weight_half() is not None) and not m._has_kmajor()])
+    if groups:
+        make_kmajor_kernels(groups)
 
 
 def _rows_weights(a, M: int, attn: Attention, norm: RMSNorm, mlp: MlpBlock, norm_mlp: RMSNorm, cross: Attention | None, norm_cross: RMSNorm | None,
@@ -337,16 +375,11 @@ def _rows_weights(a, M: int, attn: Attention, norm: RMSNorm, mlp: MlpBlock, norm
     arguments, us: 27 for any number of rows; kept ones 16 for the last number and 60 for another)."""
     from . import engine as _k
     D, keep = a.D, []
-    wo = mlp.wo
-    F, Nq, Nk = wo.in_shapes[0], attn.num_query_heads * 128, attn.num_kv_heads * 128
-    a.F, a.heads, a.kv_heads = F, attn.num_query_heads, attn.num_kv_heads
-    modules = [attn.q_proj, attn.k_proj, attn.v_proj, attn.o_proj, mlp.wi_fused, wo]
-    sizes = ((Nq, D), (Nk, D), (Nk, D), (D, Nq), (2 * F, D), (D, F))
+    a.F, a.heads, a.kv_heads = mlp.wo.in_shapes[0], attn.num_query_heads, attn.num_kv_heads
+    modules, sizes = _rows_kernels(D, attn, mlp, cross)
     norms = [("norm_self", norm), ("norm_mlp", norm_mlp)]
     if cross is not None:
-        Nc, a.cross_heads = cross.num_query_heads * 128, cross.num_query_heads
-        modules += (cross.q_proj, cross.o_proj)
-        sizes += ((Nc, D), (D, Nc))
+        a.cross_heads = cross.num_query_heads
         norms.append(("norm_cross", norm_cross))
     for name, n in norms:
         w = n.weight
@@ -356,12 +389,19 @@ def _rows_weights(a, M: int, attn: Attention, norm: RMSNorm, mlp: MlpBlock, norm
             w = w.detach().to(torch.float32).contiguous()
         keep.append(w)
         setattr(a, name, w.data_ptr())
-    halves = [m.kernel_weight_half() if two else None for m, two in zip(modules, _k.dense_half_choice(M, sizes, device))]      # (rows as two fp16 terms)
-    if None in halves[:3]:
-        _stack_kmajor(modules[:3])                                # (all three, whichever of them these rows read)
+    copies, missing = [], []
+    for m, two in zip(modules, _k.dense_half_choice(M, sizes, device)):
+        h = m.kernel_weight_half() if two else None               # (the product's rows go as two fp16 terms)
+        if h is None:
+            c = m.__dict__.get("_b200_wt")
+            if c is None or c[0] != m._weight_key():
+                missing.append(m)
+        copies.append(h)
+    if missing:
+        make_kmajor_kernels(_kmajor_groups(modules, missing))
     pointers = []
-    for m, size, h in zip(modules, sizes, halves):
-        wt = m.kernel_weight_kmajor() if h is None else h[0]
+    for m, size, h in zip(modules, sizes, copies):
+        wt = m._b200_wt[1] if h is None else h[0]
         if wt.shape != size:                                      # the native call takes its sizes from D, F and the heads
             raise NotImplementedError(f"a layer of width {D} on sm_100a has heads of 128 channels: dense kernel {tuple(m.kernel_shape)} where {size[::-1]} is read")
         keep.append(wt)
@@ -472,6 +512,8 @@ class Encoder(nn.Module):
             from . import engine as _k
             B, T = x_ids.shape
             x = _k.embed_rows(self.embedding.weight, x_ids.reshape(-1).to(torch.int32).contiguous()).reshape(B, T, -1)
+            if B * T and len(self.layers):
+                _prepare_for_rows(self.layers, B * T, x.shape[2], x.device)
             for layer in self.layers:
                 x = layer(x, state)
             return _k.rmsnorm_rows(x.reshape(B * T, -1), self.norm.weight,
@@ -784,8 +826,9 @@ class Decoder(nn.Module):
         if tgt_ids_BxTxC.is_cuda and not torch.is_grad_enabled():
             # own kernels end to end: embedding gather-sum, 18 x (fused-norm GEMMs, RoPE + cache scatter, fp32 attention,
             # gate, residual epilogues), final norm fused into the logits GEMM
-            _prepare_for_rows(self, self.layers[0].mlp.wi_fused, B * T)
             x = self.engine().embed_sum(tgt_ids_BxTxC.reshape(B * T, C)).reshape(B, T, -1)
+            if B * T and len(self.layers):
+                _prepare_for_rows(self.layers, B * T, x.shape[2], x.device)
             state.extras.pop("prefill_pos", None)
             for i, layer in enumerate(self.layers):
                 x = layer(x, state, self_attn_cache=state.self_attn_cache[i],

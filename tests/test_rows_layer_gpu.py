@@ -177,3 +177,31 @@ def test_decoder_layer(T, hidden):
     # (the turning angles are fp32: off by up to T 2^-24, about a tenth of that over all channels)
     assert (own.k[1, :, :T] - keys).norm() <= (2e-6 + T * 2.0 ** -27) * keys.norm() and (own.v[1, :, :T] - values).norm() <= 2e-6 * values.norm()
     assert own.current_idx == T - 1 and not own.k[:, :, T:].any() and not own.v[:, :, T:].any()
+
+
+@pytest.mark.parametrize("rows", [40, 600])
+def test_copies_are_read_on_another_stream(rows):
+    """A kernel whose copies are first made behind other work of one stream, and read on another at once"""
+    from dia_tts_prune_b200.layers import DenseGeneral
+    d = DenseGeneral((64,), (16384,), weight_dtype=torch.bfloat16, device="cuda")
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    with torch.no_grad():
+        d.weight.copy_(torch.randn((64, 16384), generator=g, device="cuda"))
+        x = torch.randn((rows, 64), generator=g, device="cuda")
+        want = x.double() @ d.weight.double()
+        one, two = torch.cuda.Stream(), torch.cuda.Stream()
+        for s in (one, two):                                      # (whatever a first call asks the device for has been asked for)
+            with torch.cuda.stream(s):
+                d(x)
+        torch.cuda.synchronize()
+        d.weight.neg_()                                           # other weights: their copies are made anew
+        want = -want
+        torch.cuda.synchronize()
+        with torch.cuda.stream(one):
+            torch.cuda._sleep(200_000_000)
+            first = d(x)
+        with torch.cuda.stream(two):
+            second = d(x)
+        torch.cuda.synchronize()
+    for y in (first, second):
+        assert (y - want).norm() <= 2e-6 * want.norm()
