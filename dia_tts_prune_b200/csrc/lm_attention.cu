@@ -60,12 +60,12 @@ __host__ __device__ inline int few_smem_floats(int HT, int kdim, int vdim, bool 
 
 template <int HT>
 __global__ void __launch_bounds__(kFewThreads)
-few_rows_attention_kernel(const __grid_constant__ FewAttention p, int cluster) {
+few_rows_attention_kernel(const __grid_constant__ FewAttention p, int cluster_bits) {
     extern __shared__ __align__(16) float sm[];
     __shared__ int s_last;
     pdl_release();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int sp = blockIdx.x, rank = sp % cluster, cl = sp / cluster, r = blockIdx.z;
+    const int cluster = 1 << cluster_bits, sp = blockIdx.x, rank = sp & (cluster - 1), cl = sp >> cluster_bits, r = blockIdx.z;
     const int rep = p.heads / p.kv_heads, chunks = (rep + HT - 1) / HT, g = blockIdx.y / chunks, h0 = g * rep + (blockIdx.y % chunks) * HT;
     const int nh = min(HT, (g + 1) * rep - h0), kdim = p.kdim, vdim = p.vdim, KS = kdim + 4, K4 = kdim >> 2;
     float* Q = sm;                                            // [HT][kdim]
@@ -80,9 +80,10 @@ few_rows_attention_kernel(const __grid_constant__ FewAttention p, int cluster) {
     pdl_wait();
     const int i = p.row_pos[r], lo = first_key(i, p.window, p.chunk), n_keep = p.window > 0 ? min(p.keep_first, lo) : 0;
     // as many clusters as the keys that are there fill (the grid has room for those that there may be)
-    const int n_keys = n_keep + (i - lo + 1), shares = min((int)gridDim.x / cluster, (n_keys + cluster * kFewLeast - 1) / (cluster * kFewLeast));
+    static_assert(kFewLeast == 32, "a shift below");
+    const int n_keys = n_keep + (i - lo + 1), shares = min((int)gridDim.x >> cluster_bits, ((n_keys - 1) >> (cluster_bits + 5)) + 1);
     if (cl >= shares) return;                                 // (all its CTAs)
-    const int S = shares * cluster, per = ((n_keys + S - 1) / S + 3) & ~3, k0 = min(n_keys, sp * per), k1 = min(n_keys, k0 + per);
+    const int per = ((((n_keys - 1) >> cluster_bits) + shares) / shares + 3) & ~3, k0 = min(n_keys, sp * per), k1 = min(n_keys, k0 + per);
     const int* pages = p.table + (size_t)p.row_slot[r] * p.max_pages;
     auto gather = [&](int t0, int buf) {                      // keys t0 .. of the share: warp w rows 4 w .. + 3
         size_t at[4];
@@ -315,7 +316,8 @@ static cudaError_t launch_few(const FewAttention& p, int M, cudaStream_t st) {
     const int rep = p.heads / p.kv_heads, groups = p.kv_heads * ((rep + HT - 1) / HT);
     long long max_keys = p.window > 0 ? (long long)p.window + p.keep_first : (long long)p.max_pages * p.page_size;
     if (p.chunk > 0) max_keys = std::min<long long>(max_keys, (long long)p.chunk + (p.window > 0 ? p.keep_first : 0));
-    const int S = few_shares(M * groups, max_keys, sms), cluster = std::min(S, kFewCluster);
+    const int S = few_shares(M * groups, max_keys, sms), cluster_bits = S >= kFewCluster ? 3 : S >= 4 ? 2 : S >= 2 ? 1 : 0;
+    static_assert(kFewCluster == 8, "its bits");
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(S, groups, M);
     cfg.blockDim = dim3(kFewThreads);
@@ -323,13 +325,13 @@ static cudaError_t launch_few(const FewAttention& p, int M, cudaStream_t st) {
     cfg.stream = st;
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = cluster;
+    attr[0].val.clusterDim.x = 1 << cluster_bits;
     attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
     attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 2;
-    return cudaLaunchKernelEx(&cfg, few_rows_attention_kernel<HT>, p, cluster);
+    return cudaLaunchKernelEx(&cfg, few_rows_attention_kernel<HT>, p, cluster_bits);
 }
 
 cudaError_t launch_few_rows_attention(const FewAttention& p, int M, cudaStream_t st) {
