@@ -103,6 +103,8 @@ _SIGNATURES = {
     "dia_b200_rows_layer_work_bytes": (C.c_size_t, [C.POINTER(RowsLayer)]),
     "dia_b200_rows_layer_forward": (_i, [C.POINTER(RowsLayer), _vp]),
     "dia_b200_attention_rows": (_i, [_fp, _fp, _fp, _fp, _i, _i, _i, _i, _i, _i, _i, C.POINTER(C.c_int32), _vp]),
+    "dia_b200_attention_rows_work_bytes": (C.c_size_t, [_i, _i, _i, _i, _i, _i, C.POINTER(C.c_int32)]),
+    "dia_b200_attention_rows_in": (_i, [_fp, _fp, _fp, _fp, _i, _i, _i, _i, _i, _i, _i, C.POINTER(C.c_int32), _vp, C.c_size_t, _vp]),
     "dia_b200_rope_rows": (_i, [_fp, _fp, _fp, _fp, _i32p, _i, _i, _i, _i, _i, _i, _i, _i, _vp]),
     "dia_b200_rmsnorm_rows": (_i, [_fp, _fp, C.c_float, _fp, _i, _i, _vp]),
     "dia_b200_silu_mul": (_i, [_fp, _fp, _i, _i, _vp]),

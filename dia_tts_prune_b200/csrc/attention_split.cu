@@ -3,15 +3,16 @@
 //
 // A CTA owns 128 (token, head) rows: up to 128 / PK consecutive tokens times PK query heads that read the same key/value head, so
 // that a tile of keys serves all of them.  It walks its keys 64 at a time:
-//   4 warps         fetch key and value rows from the pages, scale them by a power of two, split x = hi + lo into fp16 and put both
-//                   into a ring of shared-memory slots ([key / 8][channel / 8] blocks of 8 x 16 bytes: the layout is the K-major
-//                   operand of the scores and the MN-major operand of the value product)
-//   1 warp          issues tcgen05.mma: scores S = Q K^T (M = 128, N = 64; lo hi, hi lo, then hi hi, so that the small terms are
-//                   added first) per group of at most 128 channels, and the value product of the tile before (weights as the
-//                   operand in tensor memory)
-//   8 or 16 warps   two or four threads per row, 32 or 16 keys each: scores from tensor memory (the channel groups are summed here, in fp32),
-//                   cap, bias, mask, online softmax in base 2, weights split and written to tensor memory; then the value
-//                   product of the tile before is added to the row's fp32 registers
+//   3 warps   fetch key and value tiles into a ring of shared-memory slots.  A launch in front has scaled them by powers of two and split
+//             x = hi + lo into fp16 ([key / 8][channel / 8] blocks of 8 x 16 bytes: the layout is the K-major operand of the scores and the
+//             MN-major operand of the value product), so that one lane copies a tile; keys beyond the room for them are split here
+//   1 warp    issues tcgen05.mma: scores S = Q K^T (M = 128, N = 64; lo hi, hi lo, then hi hi, so that the small terms are
+//             added first) per group of at most 128 channels, and the value product of a tile before (weights as the
+//             operand in tensor memory)
+//   8 warps   two groups of four take turns: one thread weighs all 64 keys of its row of a tile - scores from tensor memory (the channel groups
+//             are summed here, in fp32), cap, bias, mask, online softmax in base 2, weights split and written to tensor memory.  All a row's two
+//             threads tell each other of a tile is the maximum (which the group that has the next tile needs when it has its scores), the
+//             weights' scale and their sum.  Both add the value product of every tile to fp32 registers, half of the channels each
 // The accumulator of a tensor-core product loses up to one unit in the last place at every step, towards zero (measured: 2e-6
 // over K = 2048).  So no accumulator lives longer than one tile and one channel group, and sums over tiles are fp32 additions
 // in registers: measured against 64 bits the output is closer than the fp32 FMA kernels' (relative 2-norm, 300 rows, two heads of 128,
@@ -22,13 +23,16 @@
 // of keys, times their values' magnitudes, are brought to the same range before they are split.  So an element down to 2^-17 of its
 // row's largest keeps its 22 bits (a smaller one is off by at most 2^-39 of the largest: a channel that is 2^17 times below the others of
 // its tokens has fewer), and nothing of a token that a row does not see, or of another row, enters its result: the bits do not depend on
-// what shares the launch.  Cost, against one scale per tile of rows, keys and values: 4096 rows, 16 heads of 128 over 4, window 1024
-// 237 -> 264 us; mixed scores, three prompts of 2048 rows, 8 heads of 128 over 2, 127 -> 146, of which the factors per key and per
-// value 5 us each; 16 keys that share a factor (scales in steps of 2^8) take as long.
+// what shares the launch.
 //
-// Bound: the instructions of the row warps and their latencies.  Per 64 keys and 128 rows 3 x 128 x 64 x (dk + dv) multiply-adds on the tensor
-// pipe (1536 cycles at 128 + 128) stand against about 8000 cycles of a tile with its share of the CTA's start and end, on 47 % of which a scheduler
-// issues (four row warps on each; with two row warps 8800 and 34 %; profiles/split_kernels_ncu.txt).
+// Bound: instructions of the row warps and where they come from.  Per 64 keys and 128 rows 3 x 128 x 64 x (dk + dv) multiply-adds on the tensor
+// pipe (128 + 128: 1150 cycles of the scores, whose operands take all of shared memory's bandwidth, and 770) stand against about 5000 cycles: a row's 64
+// scores take a thread some 1500 instructions, two warps on each scheduler, and a third of the stalls are instruction fetches (the loops below
+// are rolled where a roll is possible: the code of a tile's turn, some 35 KB with the cap, is what the caches hold just about).  With four threads per row
+// that exchanged a tile's maxima and largest weights, 16 keys each, the same took 8000 cycles.  Times (us, four or two threads per row / now): windowed
+// 4096 rows, 16 heads of 128 over 4, window 1024, capped 238 / 205; the same rows over latent rows of 256 + 32 408 / 368; mixed scores, prompts of 1500, 333
+// and 215 rows, 8 heads of 128 over 2 116 / 90; float32 model of 978 rows, four layers 216 / 191; Dia, 861 frames, 36 attentions 3024 / 1624 and 213 for the split
+// keys, which every row tile used to split for itself; 9 decoding sequences over 1134 latent rows 281 / 128.
 // Every wait is bounded: a wait that runs out makes the CTA write NaN, note it in a word that the host reads, and end; the next launch
 // on the device returns an error.
 #include <algorithm>
@@ -49,12 +53,10 @@ namespace dia {
 namespace {
 
 constexpr int kRows = 128, kKeys = 64, kGroupW = 128;        // query rows of a CTA, keys of a tile, channels of a stage
-template <int RT>
-constexpr int kSplitThreads = 32 * (4 * RT + 8);
-constexpr int kMaxSlots = 6, kMaxDepth = 5, kMaxKStages = 4;
+constexpr int kRowWarps = 8, kFetchWarps = 3, kSplitThreads = 32 * (kRowWarps + 1 + kFetchWarps);
+constexpr int kMaxSlots = 6, kMaxKStages = 4;
 constexpr int kSmemMost = 232448;                             // all of it dynamic
 constexpr float kLog2e = 1.4426950408889634f;
-constexpr int kSplitOnceRows = 512;                           // rows of a kv head (M rep) from which keys with values of up to 128 channels are split in advance
 constexpr int kSplitGrid = 148 * 16;                           // CTAs of the launch that splits them
 constexpr unsigned kSpinMost = 4000000u;
 
@@ -66,9 +68,10 @@ struct Geometry {
     int v0_layout, v_last_layout;            // widths in which the value groups lie in a slot (a latent's value group is its key group)
     int shared_kv;                           // the value is the head of the key row: value group i is key group i
     int slot_bytes, n_slots, q_bytes;
-    int o_bufs;                              // accumulators of the value product (2 where tensor memory has the columns)
+    int s_bufs, p_bufs, o_bufs;              // tiles of scores, of weights and of value products in tensor memory (1 or 2 of each)
     int k_sets;                              // scales of a key: one, with mixed scores one per kv head
     int depth;                               // tiles whose scales are in shared memory
+    int rings;                               // tiles whose rows' numbers are (2 or 4)
     // the split keys and values in SplitAttention::work: SlotTiles per slot, then inverse scales [tile][set][key], then the tiles.  A
     // tile's parts: key groups (per kv head where the launch reads one head at a time), then value groups; its sets of scales: the keys
     // of each kv head, then the values of each (shared_kv: the keys' only)
@@ -81,12 +84,14 @@ struct Geometry {
 struct SlotTiles { int base, first, end, zero; };
 
 __device__ __forceinline__ bool wait_for(uint64_t* bar, uint32_t parity) {
+#pragma unroll 1
     for (unsigned i = 0; i < kSpinMost; ++i)
         if (mbar_try_wait(bar, parity)) return true;
     return false;
 }
 // the same for a converged warp, with one answer for all lanes (so that what follows is uniform: see elect_one_sync)
 __device__ __forceinline__ bool wait_warp(uint64_t* bar, uint32_t parity) {
+#pragma unroll 1
     for (unsigned i = 0; i < kSpinMost; ++i)
         if (__any_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
     return false;
@@ -121,6 +126,7 @@ __device__ __forceinline__ void commit_to(uint64_t* bar) {
 __device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_smem_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+__device__ __forceinline__ void tmem_loaded() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tmem_load32(uint32_t addr, float (&v)[32]) {
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, "
@@ -132,12 +138,6 @@ __device__ __forceinline__ void tmem_load32(uint32_t addr, float (&v)[32]) {
         : "r"(addr)
         : "memory");
 }
-__device__ __forceinline__ void tmem_load8(uint32_t addr, float* v) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-                 : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
-                 : "r"(addr)
-                 : "memory");
-}
 __device__ __forceinline__ void tmem_load16(uint32_t addr, float* v) {
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
@@ -146,60 +146,70 @@ __device__ __forceinline__ void tmem_load16(uint32_t addr, float* v) {
         : "r"(addr)
         : "memory");
 }
+// two fp32 in one register pair, two operations in one instruction
+using f2 = unsigned long long;
+__device__ __forceinline__ f2 pack2(float lo, float hi) {
+    f2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ void unpack2(f2 v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
+__device__ __forceinline__ void tmem_load8(uint32_t addr, float (&v)[8]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
+                 : "r"(addr)
+                 : "memory");
+}
 template <int N>
-__device__ __forceinline__ void tmem_load_n(uint32_t addr, float (&v)[N]) {
-    if constexpr (N == 32) tmem_load32(addr, v);
-    else if constexpr (N == 16) tmem_load16(addr, v);
-    else tmem_load8(addr, v);
+__device__ __forceinline__ void tmem_load_pairs(uint32_t addr, f2* p) {       // 2 N columns
+    static_assert(N == 8 || N == 16, "columns of a load");
+    float v[2 * N];
+    if constexpr (N == 16) tmem_load32(addr, v);
+    else tmem_load16(addr, v);
+    tmem_loaded();
+#pragma unroll
+    for (int e = 0; e < N; ++e) p[e] = pack2(v[2 * e], v[2 * e + 1]);
 }
-// two fp32 operations in one instruction
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
-    float2 d;
-    asm("{\n\t.reg .b64 a, b, c, d;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\tmov.b64 c, {%6, %7};\n\t"
-        "fma.rn.f32x2 d, a, b, c;\n\tmov.b64 {%0, %1}, d;\n\t}"
-        : "=f"(d.x), "=f"(d.y)
-        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
+    f2 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
     return d;
 }
-__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
-    float2 d;
-    asm("{\n\t.reg .b64 a, b, d;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\tmul.rn.f32x2 d, a, b;\n\tmov.b64 {%0, %1}, d;\n\t}"
-        : "=f"(d.x), "=f"(d.y)
-        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+__device__ __forceinline__ f2 mul2(f2 a, f2 b) {
+    f2 d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
     return d;
 }
-__device__ __forceinline__ float2 add2(float2 a, float2 b) {
-    float2 d;
-    asm("{\n\t.reg .b64 a, b, d;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\tadd.rn.f32x2 d, a, b;\n\tmov.b64 {%0, %1}, d;\n\t}"
-        : "=f"(d.x), "=f"(d.y)
-        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+__device__ __forceinline__ f2 add2(f2 a, f2 b) {
+    f2 d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
     return d;
 }
+__device__ __forceinline__ f2 twice(float v) { return pack2(v, v); }
 // tanh x = x + x^3 q(x^2) for |x| <= kTanhRange: q interpolates (tanh x / x - 1) / x^2 at six Chebyshev nodes (relative error of the
 // result 3e-10 before rounding).  A tile's scores mostly lie there, and it takes a fifth of the library call's instructions
 // (a tile of capped scores: 2100 -> 800 cycles)
 constexpr float kTanhRange = 0.6f;
-__device__ __forceinline__ float2 tanh_near_zero(float2 x) {
-    const float2 u = mul2(x, x);
-    float2 q = make_float2(2.3707656405e-3f, 2.3707656405e-3f);
-    q = fma2(q, u, make_float2(-8.41007080153e-3f, -8.41007080153e-3f));
-    q = fma2(q, u, make_float2(2.17883219971e-2f, 2.17883219971e-2f));
-    q = fma2(q, u, make_float2(-5.39615517813e-2f, -5.39615517813e-2f));
-    q = fma2(q, u, make_float2(1.33333128669e-1f, 1.33333128669e-1f));
-    q = fma2(q, u, make_float2(-3.33333332312e-1f, -3.33333332312e-1f));
+__device__ __forceinline__ f2 tanh_near_zero(f2 x) {
+    const f2 u = mul2(x, x);
+    f2 q = twice(2.3707656405e-3f);
+    q = fma2(q, u, twice(-8.41007080153e-3f));
+    q = fma2(q, u, twice(2.17883219971e-2f));
+    q = fma2(q, u, twice(-5.39615517813e-2f));
+    q = fma2(q, u, twice(1.33333128669e-1f));
+    q = fma2(q, u, twice(-3.33333332312e-1f));
     return fma2(mul2(x, u), q, x);
 }
-// v[i] *= f[i] (16-byte aligned; the same addresses for all lanes)
+// v[i] *= f[i], N pairs (16-byte aligned; the same addresses for all lanes)
 template <int N>
-__device__ __forceinline__ void scale_by(float* v, const float* f) {
+__device__ __forceinline__ void scale_by(f2* v, const float* f) {
 #pragma unroll
-    for (int e = 0; e < N; e += 4) {
-        const float4 k = *reinterpret_cast<const float4*>(f + e);
-        const float2 a = mul2(make_float2(v[e], v[e + 1]), make_float2(k.x, k.y)), b = mul2(make_float2(v[e + 2], v[e + 3]), make_float2(k.z, k.w));
-        v[e] = a.x; v[e + 1] = a.y; v[e + 2] = b.x; v[e + 3] = b.y;
+    for (int e = 0; e < N; e += 2) {
+        const ulonglong2 k = *reinterpret_cast<const ulonglong2*>(f + 2 * e);
+        v[e] = mul2(v[e], k.x);
+        v[e + 1] = mul2(v[e + 1], k.y);
     }
 }
-__device__ __forceinline__ void tmem_loaded() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tmem_store8(uint32_t addr, const uint32_t (&v)[8]) {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(addr), "r"(v[0]), "r"(v[1]),
                  "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
@@ -214,6 +224,11 @@ __device__ __forceinline__ void split2(float x, float y, uint32_t& hi, uint32_t&
     hi = *reinterpret_cast<const uint32_t*>(&h);
     lo = *reinterpret_cast<const uint32_t*>(&l);
 }
+__device__ __forceinline__ void split2(f2 v, uint32_t& hi, uint32_t& lo) {
+    float x, y;
+    unpack2(v, x, y);
+    split2(x, y, hi, lo);
+}
 // the power of two that brings a largest magnitude m to [2^14, 2^15), and its inverse (m = 0: 2^114; both stay normal numbers)
 __device__ __forceinline__ float scale_of(float m, float& inverse) {
     const int e = max((int)(__float_as_uint(m) >> 23) - 127, -100);
@@ -224,6 +239,11 @@ constexpr float kFloatMost = 3.402823466e38f;
 __device__ __forceinline__ float max_nan(float a, float b) {  // (fmaxf drops a NaN)
     float m;
     asm("max.NaN.f32 %0, %1, %2;" : "=f"(m) : "f"(a), "f"(b));
+    return m;
+}
+__device__ __forceinline__ float max3_nan(float a, float b, float c) {
+    float m;
+    asm("max.NaN.f32 %0, %1, %2, %3;" : "=f"(m) : "f"(a), "f"(b), "f"(c));
     return m;
 }
 __device__ __forceinline__ float warp_max_nan(float v) {
@@ -252,6 +272,12 @@ __device__ __forceinline__ int first_key_of(int i, int window, int chunk) {
     return chunk > 0 ? max(w, i - i % chunk) : w;
 }
 
+// how many keys of a slot some row sees (rows_per_slot > 0)
+__host__ __device__ __forceinline__ int range_keys(const SplitAttention& p, int slot) {
+    const int n = p.mode == 2 && p.n_valid[slot] < p.n_keys ? p.n_valid[slot] : p.n_keys;
+    return p.mode == 0 && p.rows_per_slot < n ? p.rows_per_slot : n;
+}
+
 __device__ __forceinline__ size_t part_offset(const Geometry& geo, int part) {
     const unsigned k_head = kKeys * 4u * ((geo.n_kst - 1) * geo.wk0 + geo.wk_last), v_head = kKeys * 4u * ((geo.n_vst - 1) * geo.wv0 + geo.wv_last);
     if (part < geo.k_parts) return (size_t)(part / geo.n_kst) * k_head + (size_t)(part % geo.n_kst) * geo.wk0 * kKeys * 4;
@@ -274,6 +300,16 @@ split_keys_kernel(const __grid_constant__ SplitAttention p, const __grid_constan
         __syncthreads();                                          // (the last tile's answer has been read)
         if (tid == 0) { s_seq = -1; s_run = 0; }
         __syncthreads();
+        if (p.rows_per_slot > 0 && tid == 0) {                // every slot's keys from 0 on
+            int begin = 0;
+            for (int slot = 0; slot * p.rows_per_slot < p.M; ++slot) {
+                const int n = (range_keys(p, slot) + kKeys - 1) / kKeys;
+                if (writes_plan) plan[slot] = SlotTiles{begin, 0, min(n, geo.cap_tiles - begin), -1};
+                if (tile >= begin && tile < begin + n) s_seq = slot, s_first = tile - begin;
+                begin += n;
+            }
+        }
+        if (p.rows_per_slot > 0) __syncthreads();
         for (int s0 = 0; s0 < p.n_seq; s0 += 32) {                // warp 0: 32 sequences at a time, running sum of their tiles
             if (warp == 0) {
                 const int s = s0 + lane;
@@ -314,7 +350,9 @@ split_keys_kernel(const __grid_constant__ SplitAttention p, const __grid_constan
             __syncthreads();
         }
         if (s_seq < 0) return;                                // (nor does any later tile belong to one)
-        const int seq = s_seq, slot = p.seq_slot[seq], pos0 = p.row_pos[p.seq_row0[seq]], k_end = pos0 + p.seq_count[seq], j0 = s_first * kKeys;
+        const bool ranged = p.rows_per_slot > 0;
+        const int seq = s_seq, slot = ranged ? seq : p.seq_slot[seq], k_end = ranged ? range_keys(p, slot) : p.row_pos[p.seq_row0[seq]] + p.seq_count[seq],
+                  j0 = s_first * kKeys;
         // ---- which rows and channels? ----
         const bool is_v = part >= geo.k_parts;
         const int q = is_v ? part - geo.k_parts : part, per = is_v ? geo.n_vst : geo.n_kst, gg = q / per, st = q % per;
@@ -325,8 +363,8 @@ split_keys_kernel(const __grid_constant__ SplitAttention p, const __grid_constan
         const bool in = j < k_end;
         const float* src = is_v ? p.vcache : p.kcache;
         if (in) {
-            const int page = p.table[(size_t)slot * p.max_pages + j / p.page_size];
-            src += (((size_t)page * p.kv_heads + g) * p.page_size + j % p.page_size) * width;
+            const int page = p.table ? p.table[(size_t)slot * p.max_pages + j / p.page_size] : slot;
+            src += (((size_t)page * p.kv_heads + g) * p.page_size + (p.table ? j % p.page_size : j)) * width;
         }
         float4 v[8];
         float m = 0.f;
@@ -486,37 +524,41 @@ __device__ __noinline__ void plain_row(const SplitAttention& p, int r, int slot,
         if (lane + 32 * u < n) dst[lane + 32 * u] = o[u] * f;
 }
 
-// NVS: channel groups of a value (1: up to 128 channels, 2: up to 256).  RT: threads of a row; each takes 64 / RT keys of a tile and an equal
-// share of the output channels
-template <int NVS, int RT>
-__global__ void __launch_bounds__(kSplitThreads<RT>, 1)
+// NVS: channel groups of a value (1: up to 128 channels, 2: up to 256)
+template <int NVS>
+__global__ void __launch_bounds__(kSplitThreads, 1)
 split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_constant__ Geometry geo) {
-    constexpr int DVH = 128 * NVS / RT;                       // output channels of a thread
-    constexpr int KP = kKeys / RT, RW = 4 * RT;               // keys of a thread, row warps
-    // The block is launched with 128 registers a thread (RT = 4: 80).  (Wide values with two threads per row, 4096 rows, 16 heads over latent
-    // rows of 256 + 32, window 1024: 184 and 112 452 us, 192 and 96 443, 200 and 80 421.  What the fetching warps spill is used for
-    // keys that are not split in advance only.)
-    constexpr int kLaunchRegs = RT == 4 ? 80 : 128;
-    constexpr int kRowRegs = RT == 4 ? (NVS == 1 ? 96 : 104) : (NVS == 1 ? 176 : 200), kFetchRegs = RT == 4 ? (NVS == 1 ? 64 : 32) : (NVS == 1 ? 128 : 80);
-    static_assert(32 * RW * kRowRegs + 128 * kFetchRegs + 128 * 32 <= kLaunchRegs * kSplitThreads<RT>, "registers of the block");
+    constexpr int DVH = 64 * NVS;                             // output channels of a thread
+    // The block is launched with 168 registers a thread.  A row's thread holds 64 scores and its sums; the others' share is what the issuing warp needs
+    // for its operands (with 24 registers an instruction of the value product took 170 cycles to issue, not 77)
+    constexpr int kRowRegs = NVS == 1 ? 208 : 216, kOtherRegs = NVS == 1 ? 88 : 72;
+    static_assert(32 * kRowWarps * kRowRegs + 128 * kOtherRegs <= 168 * kSplitThreads, "registers of the block");
+    constexpr int RW = kRowWarps, LW = NVS == 1 ? 16 : 8;     // row warps, pairs of columns in flight
     extern __shared__ __align__(128) unsigned char smem[];
     unsigned char* ring = smem;
     unsigned char* qs = ring + (size_t)geo.n_slots * geo.slot_bytes;
     uint64_t* full = reinterpret_cast<uint64_t*>(qs + geo.q_bytes);
-    uint64_t* empty = full + kMaxSlots;
-    uint64_t* s_full = empty + kMaxSlots;                     // scores of a tile are there / have been read
-    uint64_t* s_empty = s_full + 1;
-    uint64_t* p_ready = s_empty + 1;                          // weights of a tile are there / its value product is done
-    uint64_t* pv_done = p_ready + 1;
-    uint64_t* q_ready = pv_done + 1;
-    uint64_t* pair = q_ready + 1;                             // [4] the warps that share rows
-    uint64_t* v_ready = pair + 4;                             // [depth] the scales of a tile's values are there
-    float* k_inv = reinterpret_cast<float*>(v_ready + kMaxDepth);      // [depth][k_sets][64] inverse scales of the keys
+    uint64_t* empty = full + geo.n_slots;
+    // of the even and of the odd tiles each: the two groups of row warps take turns, and a barrier of either's own is never two phases ahead
+    uint64_t* s_full = empty + geo.n_slots;                    // scores of a tile are there / have been read
+    uint64_t* s_empty = s_full + 2;
+    uint64_t* p_ready = s_empty + 2;                          // weights of a tile are there / its value product is done / has been added
+    uint64_t* pv_done = p_ready + 2;
+    uint64_t* o_empty = pv_done + 2;
+    uint64_t* m_ready = o_empty + 2;                          // [4] the maxima of 32 rows up to a tile are there
+    uint64_t* q_ready = m_ready + 4;
+    uint64_t* v_ready = q_ready + 1;                          // [depth] the scales of a tile's values are there
+    const int n_bars = 2 * geo.n_slots + 15 + (geo.shared_kv ? 0 : geo.depth);
+    float* m_x = reinterpret_cast<float*>(full + ((n_bars + 1) & ~1)); // [2][128] maxima up to an even and an odd tile
+    float* sum_x = m_x + 2 * kRows;                           // [rings / 2][128] sums of the weights of the odd tiles
+    float* q_inv = sum_x;                                     // [128] (the first odd tile's sums are stored when both groups have read it)
+    __nv_bfloat16* wi_x = reinterpret_cast<__nv_bfloat16*>(sum_x + geo.rings / 2 * kRows); // [rings][128] inverse scales of the weights: powers of two
+    float* k_inv = reinterpret_cast<float*>(wi_x + geo.rings * kRows); // [depth][k_sets][64] inverse scales of the keys
     float* v_inv = geo.shared_kv ? k_inv : k_inv + geo.depth * geo.k_sets * kKeys;      // [depth][64] of the values
-    float* row_x = v_inv + geo.depth * kKeys;                 // [2][RT][128] what the threads of a row tell each other
-    uint32_t* s_breaks = reinterpret_cast<uint32_t*>(row_x + 2 * RT * kRows);      // [4]
+    int4* s_tile = reinterpret_cast<int4*>(v_inv + geo.depth * kKeys); // [depth] a tile's first key, its tokens (first | end << 16), end of its keys, lo (see Walk)
+    uint32_t* s_breaks = reinterpret_cast<uint32_t*>(s_tile + geo.depth);      // [4]
     uint32_t* s_tmem = s_breaks + 4;
-    int* s_rows = reinterpret_cast<int*>(s_tmem + 1);         // [2]
+    int* s_rows = reinterpret_cast<int*>(s_tmem + 1);         // [2] the row tile; then [0]: its tiles of keys
     int* s_slot = s_rows + 3;                                 // [tokens]
     const int TT = kRows >> geo.pk_shift;
     int* s_pos = s_slot + TT;
@@ -558,17 +600,21 @@ split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_co
     }
 
     if (tid == 0) {
-        for (int i = 0; i < kMaxSlots; ++i) { mbar_init(&full[i], 4); mbar_init(&empty[i], 1); }
-        mbar_init(s_full, 1);
-        mbar_init(s_empty, RW);
-        mbar_init(p_ready, RW);
-        mbar_init(pv_done, 1);
+        for (int i = 0; i < geo.n_slots; ++i) { mbar_init(&full[i], kFetchWarps); mbar_init(&empty[i], 1); }
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(&s_full[i], 1);
+            mbar_init(&s_empty[i], 4);
+            mbar_init(&p_ready[i], 4);
+            mbar_init(&pv_done[i], 1);
+            mbar_init(&o_empty[i], RW);
+        }
+        for (int i = 0; i < 4; ++i) mbar_init(&m_ready[i], 1);
         mbar_init(q_ready, RW);
-        for (int i = 0; i < 4; ++i) mbar_init(&pair[i], RT);
-        for (int i = 0; i < kMaxDepth; ++i) mbar_init(&v_ready[i], 4);
+        if (!geo.shared_kv)
+            for (int i = 0; i < geo.depth; ++i) mbar_init(&v_ready[i], kFetchWarps);
         fence_mbar_init();
     }
-    if (warp == RW + 4) {
+    if (warp == RW) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(s_tmem)));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::);
     }
@@ -593,344 +639,369 @@ split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_co
     __syncthreads();
     fence_after();
     const uint32_t tmem = *s_tmem;
-    const uint32_t t_s = tmem, t_p = tmem + 64u * geo.n_kst, t_o = t_p + 64u;    // scores | weights (hi, lo) | value product
+    const uint32_t t_s = tmem, t_p = tmem + 64u * geo.n_kst * geo.s_bufs, t_o = t_p + 64u * geo.p_bufs;    // scores | weights (hi, lo) | value products
 
     if (warp < RW) {
-        // ================= softmax: rows 32 (warp % 4) + lane, keys KP (warp / 4) .. of a tile =================
+        // ================= softmax: rows 32 (warp % 4) + lane; warps 0 .. 3 take the even tiles, 4 .. 7 the odd ones =================
         asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kRowRegs));
         // ---- the query tile: largest magnitude, then both terms.  Row r of the tile is head h0 + r % PK of token r / PK; a warp takes
         // eight rows at a time, a lane eight channels of one.  (The first keys are on their way meanwhile: with the tile made by all
         // warps in front of the roles, its loops unrolled, a launch of one key tile took 17 us, now 14: cold instruction fetches) ----
-        const int chunks = ((geo.n_kst - 1) * geo.wk0 + geo.wk_last) >> 3, wkb = geo.wk0 >> 3;
-        auto q_values = [&](int row, int ch, float (&v)[8]) { // channels 8 ch .. of the padded row
-            const int i = row >> geo.pk_shift, h = h0 + (row & (PK - 1)), st = geo.n_kst == 1 ? 0 : ch / wkb, c = 8 * (ch - st * wkb);
-            const int width = p.talk ? p.kdim : min(kGroupW, p.kdim - st * kGroupW);
-            const bool in = i < n_tok && ch < chunks, one = in && c < width, both = in && c + 4 < width;    // (widths are multiples of 4)
-            const float* src = p.q + (size_t)(r0 + i) * p.ldq + c;
-            const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
+        constexpr int RG = kRows / (8 * RW);                  // groups of 8 RW rows
+        const int qrow = warp * 8 + (lane & 7), qch = lane >> 3;
+        auto q_load = [&](int st, float4 (&v)[RG][4][2]) {    // this lane's channels of channel group st (mixed scores: of kv head st)
+            const int width = p.talk ? p.kdim : min(kGroupW, p.kdim - st * kGroupW);      // (a multiple of 4)
+            auto add = [&](const float* src, int t, bool first) {
+#pragma unroll
+                for (int rg = 0; rg < RG; ++rg) {
+                    const int row = qrow + 8 * RW * rg, i = row >> geo.pk_shift, h = h0 + (row & (PK - 1));
+                    const float* at = src + (size_t)(r0 + i) * p.ldq + (p.talk ? 0 : (size_t)h * p.qdim);
+                    const int left = i < n_tok ? width - 8 * qch : 0;
+                    const float w = p.talk ? p.talk[h * p.heads + st * rep + t] : 1.f;
+#pragma unroll
+                    for (int k = 0; k < 4; ++k)
+#pragma unroll
+                        for (int e = 0; e < 2; ++e) {
+                            float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+                            if (32 * k + 4 * e < left) x = *reinterpret_cast<const float4*>(at + 32 * k + 4 * e);
+                            float4& y = v[rg][k][e];
+                            if (first) y = p.talk ? make_float4(w * x.x, w * x.y, w * x.z, w * x.w) : x;
+                            else y = make_float4(fmaf(w, x.x, y.x), fmaf(w, x.y, y.y), fmaf(w, x.z, y.z), fmaf(w, x.w, y.w));
+                        }
+                }
+            };
             if (!p.talk) {
-                src += (size_t)h * p.qdim + st * kGroupW;
-                const float4 a = one ? *reinterpret_cast<const float4*>(src) : z, b = both ? *reinterpret_cast<const float4*>(src + 4) : z;
-                v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
-                v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+                add(p.q + st * kGroupW + 8 * qch, 0, true);
                 return;
             }
+            // the mixed score is linear in the queries: mix those instead
+            const float* src = p.q + (size_t)st * rep * p.qdim + 8 * qch;
+            add(src, 0, true);
+#pragma unroll 1
+            for (int t = 1; t < rep; ++t) add(src + (size_t)t * p.qdim, t, false);
+        };
+        auto q_largest = [&](const float4 (&v)[RG][4][2], float (&m)[RG]) {
 #pragma unroll
-            for (int e = 0; e < 8; ++e) v[e] = 0.f;
-            if (!one) return;
-            src += (size_t)st * rep * p.qdim;
-            const float* mix = p.talk + h * p.heads + st * rep;
-#pragma unroll 4
-            for (int t = 0; t < rep; ++t) {                   // the mixed score is linear in the queries: mix those instead
-                const float w = mix[t];
-                const float4 a = *reinterpret_cast<const float4*>(src + (size_t)t * p.qdim);
-                const float4 b = both ? *reinterpret_cast<const float4*>(src + (size_t)t * p.qdim + 4) : z;
-                v[0] = fmaf(w, a.x, v[0]); v[1] = fmaf(w, a.y, v[1]); v[2] = fmaf(w, a.z, v[2]); v[3] = fmaf(w, a.w, v[3]);
-                v[4] = fmaf(w, b.x, v[4]); v[5] = fmaf(w, b.y, v[5]); v[6] = fmaf(w, b.z, v[6]); v[7] = fmaf(w, b.w, v[7]);
-            }
-        };
-        float* const q_inv = row_x + RT * kRows;              // [128] (read by a row's threads before they exchange anything there)
-        auto q_scale = [&](float m, int row, bool& bad) {     // a row's scale from the four lanes that hold it
-            float scale, inverse;
-            bad = scale_row(row_max(m), scale, inverse);
-            if (lane < 8) q_inv[row] = inverse;
-            return scale;
-        };
-        auto q_store = [&](int row, int ch, float scale, bool bad, const float (&v)[8]) {
-            if (ch >= chunks) return;
-            uint32_t hi[4], lo[4];
+            for (int rg = 0; rg < RG; ++rg)
 #pragma unroll
-            for (int e = 0; e < 4; ++e) split2(bad ? 0.f : v[2 * e] * scale, bad ? 0.f : v[2 * e + 1] * scale, hi[e], lo[e]);
-            const int st = geo.n_kst == 1 ? 0 : ch / wkb, w = st == geo.n_kst - 1 ? geo.wk_last : geo.wk0, c8 = ch - st * wkb;
-            unsigned char* dst = qs + (size_t)st * geo.wk0 * kRows * 4 + (size_t)(((row >> 3) * (w >> 3) + c8) * 128 + (row & 7) * 16);
-            *reinterpret_cast<uint4*>(dst) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-            *reinterpret_cast<uint4*>(dst + (size_t)w * kRows * 2) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+                for (int k = 0; k < 4; ++k) m[rg] = max_abs4(max_abs4(m[rg], v[rg][k][0]), v[rg][k][1]);
         };
-        constexpr int RG = 4 / RT;                            // groups of 8 RW rows
-        const int qrow = warp * 8 + (lane & 7), qch = lane >> 3;
-        if (!p.talk && geo.n_kst == 1) {                      // all of it fits the registers
-            float4 v[4 * RG][2];
+        float scale[RG], m_row[RG] = {};
+        bool bad[RG];
+        auto q_scales = [&] {                                 // from the four lanes that hold a row
 #pragma unroll
             for (int rg = 0; rg < RG; ++rg) {
-                const int row = qrow + 8 * RW * rg, i = row >> geo.pk_shift;
-                const float* src = p.q + (size_t)(r0 + i) * p.ldq + (size_t)(h0 + (row & (PK - 1))) * p.qdim + 8 * qch;
-                const int left = i < n_tok ? p.kdim - 8 * qch : 0;
-#pragma unroll
-                for (int k = 0; k < 4; ++k)
-#pragma unroll
-                    for (int e = 0; e < 2; ++e) {
-                        v[rg * 4 + k][e] = make_float4(0.f, 0.f, 0.f, 0.f);
-                        if (32 * k + 4 * e < left) v[rg * 4 + k][e] = *reinterpret_cast<const float4*>(src + 32 * k + 4 * e);
-                    }
+                float inverse;
+                bad[rg] = scale_row(row_max(m_row[rg]), scale[rg], inverse);
+                if (lane < 8) q_inv[qrow + 8 * RW * rg] = inverse;
             }
+        };
+        auto q_store = [&](int st, const float4 (&v)[RG][4][2]) {
+            const int w = st == geo.n_kst - 1 ? geo.wk_last : geo.wk0;
+            unsigned char* const group = qs + (size_t)st * geo.wk0 * kRows * 4;
 #pragma unroll
             for (int rg = 0; rg < RG; ++rg) {
-                float m = 0.f;
+                const int row = qrow + 8 * RW * rg;
 #pragma unroll
-                for (int i = 0; i < 4; ++i) m = max_abs4(max_abs4(m, v[rg * 4 + i][0]), v[rg * 4 + i][1]);
-                bool bad;
-                const float scale = q_scale(m, qrow + 8 * RW * rg, bad);
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const float4 a = v[rg * 4 + i][0], b = v[rg * 4 + i][1];
-                    const float x[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-                    q_store(qrow + 8 * RW * rg, qch + 4 * i, scale, bad, x);
+                for (int k = 0; k < 4; ++k) {
+                    const int c8 = qch + 4 * k;
+                    if (8 * c8 >= w) continue;
+                    const float f = scale[rg];
+                    const float4 z = make_float4(0.f, 0.f, 0.f, 0.f), a = bad[rg] ? z : v[rg][k][0], b = bad[rg] ? z : v[rg][k][1];
+                    uint32_t hi[4], lo[4];
+                    split2(a.x * f, a.y * f, hi[0], lo[0]);
+                    split2(a.z * f, a.w * f, hi[1], lo[1]);
+                    split2(b.x * f, b.y * f, hi[2], lo[2]);
+                    split2(b.z * f, b.w * f, hi[3], lo[3]);
+                    unsigned char* dst = group + (size_t)(((row >> 3) * (w >> 3) + c8) * 128 + (row & 7) * 16);
+                    *reinterpret_cast<uint4*>(dst) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+                    *reinterpret_cast<uint4*>(dst + (size_t)w * kRows * 2) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
                 }
             }
-        } else {
-            for (int rg = 0; rg < RG; ++rg) {
-                float m = 0.f, scale = 0.f;
-                bool bad = false;
-                for (int pass = 0; pass < 2; ++pass) {
-                    for (int ch = qch; ch < chunks; ch += 16) {
-                        float v[4][8];
-#pragma unroll
-                        for (int i = 0; i < 4; ++i) q_values(qrow + 8 * RW * rg, ch + 4 * i, v[i]);
-#pragma unroll
-                        for (int i = 0; i < 4; ++i) {
-                            if (pass == 0) {
-#pragma unroll
-                                for (int e = 0; e < 8; ++e) m = max_nan(m, fabsf(v[i][e]));
-                            } else {
-                                q_store(qrow + 8 * RW * rg, ch + 4 * i, scale, bad, v[i]);
-                            }
-                        }
-                    }
-                    if (pass == 0) scale = q_scale(m, qrow + 8 * RW * rg, bad);
-                }
-            }
+        };
+        float4 qv[RG][4][2];
+        // (one group of channels stays in registers, more are read twice)
+#pragma unroll 1
+        for (int st = 0; st < geo.n_kst; ++st) {
+            q_load(st, qv);
+            q_largest(qv, m_row);
+        }
+        q_scales();
+#pragma unroll 1
+        for (int st = 0; st < geo.n_kst; ++st) {
+            if (geo.n_kst > 1) q_load(st, qv);
+            q_store(st, qv);
         }
         fence_smem_async();
         __syncwarp();
         if (lane == 0) mbar_arrive(q_ready);
-        asm volatile("bar.sync 1, %0;" ::"n"(32 * RW) : "memory");          // (all queries are stored, and the rows' scales are there)
+        asm volatile("bar.sync 1, %0;" ::"n"(32 * RW + 32) : "memory");     // (all queries are stored, the rows' scales and the number of tiles are there)
         const int qt = warp & 3, hf = warp >> 2, row = qt * 32 + lane, tok = row >> geo.pk_shift, h = h0 + (row & (PK - 1));
         const uint32_t lanes = (uint32_t)(qt * 32) << 16;
         const int my_pos = s_pos[tok];
         const int my_lo = first_key_of(max(my_pos, 0), p.window, p.chunk), kept = p.window > 0 ? p.keep_first : 0;
         const bool ranged = p.rows_per_slot > 0 && p.mode != 0;
         // scores and maxima are in units of log 2 (a capped score from its cap on): the largest score's weight is exactly 1 at any magnitude
-        const float cap = p.cap, inv_cap = cap > 0.f ? 1.0f / cap : 0.f;
+        const float cap = p.cap;
         const float mult = q_inv[row] * p.scale * (p.temp ? p.temp[h] : 1.f) * (cap > 0.f ? 1.f : kLog2e);
         const float slope = p.slopes ? p.slopes[h] * kLog2e : 0.f;
         // channels of this thread: c0 .. + n_mine, at t_mine in tensor memory
-        const int share = NVS == 1 ? (geo.wv0 + 8 * RT - 1) / (8 * RT) * 8 : DVH, part = NVS == 1 ? hf : hf % (RT / 2), group = NVS == 1 ? 0 : hf / (RT / 2);
-        const int n_mine = max(0, min(share, (group ? geo.wv_last : geo.wv0) - part * share)), c0 = group * 128 + part * share;
+        const int share = NVS == 1 ? geo.wv0 / 2 : DVH, n_mine = NVS == 1 || hf == 0 ? min(share, geo.wv0) : geo.wv_last, c0 = hf * share;
         const uint32_t t_mine = t_o + c0 + lanes;
-        float O[DVH];
+        f2 O[DVH / 2];
 #pragma unroll
-        for (int c = 0; c < DVH; ++c) O[c] = 0.f;
-        constexpr int LP = KP / 16;                           // denominators: a sum per 16 keys of a tile, the same with any threads per row
-        float m_run = -CUDART_INF_F, l_run[LP] = {}, corr_prev = 1.f, wi_prev = 0.f;
+        for (int c = 0; c < DVH / 2; ++c) O[c] = 0;
+        float m_run = -CUDART_INF_F, l = 0.f;
+        float m_own = 0.f, wi_own = 0.f, sum_own = 0.f;       // of the tile of this group that has not been added yet
         bool ok = true;
-        constexpr int OW = NVS == 1 && RT == 2 ? 32 : 16;     // columns in flight
-        auto add_values = [&](unsigned t, float corr, float vi) {      // O <- corr O + vi * value product of tile t (which is done)
-            const bool same = __all_sync(0xffffffffu, corr == 1.f);
+        // O <- corr O + the value product of tile t, up to which the maximum is m; the denominator likewise (in the threads of the even tiles).
+        // The numbers of the other group's tile were stored in front of the weights that have been multiplied.
+        auto add_values = [&](unsigned t, float m, float wi, float sum) {
+            if (!wait_for(&pv_done[t & 1u], (t >> 1) & 1u)) return false;
+            fence_after();
+            if ((int)(t & 1u) != hf) {
+                wi = __bfloat162float(wi_x[(t & (geo.rings - 1u)) * kRows + row]);
+                if (hf == 0) sum = sum_x[((t >> 1) & (geo.rings / 2 - 1u)) * kRows + row];
+            }
+            const float corr = m_run == -CUDART_INF_F ? 0.f : ex2(m_run - m);      // (m is no less)
+            const f2 vi2 = twice(wi), c2 = twice(corr);
+            l = fmaf(l, corr, sum);
+            m_run = m;
             const uint32_t from = t_mine + (geo.o_bufs == 2 ? (t & 1u) * 128u : 0u);
-            const float2 vi2 = make_float2(vi, vi), c2 = make_float2(corr, corr);
 #pragma unroll
-            for (int c = 0; c < DVH; c += OW) {
+            for (int c = 0; c < DVH; c += 2 * LW) {
                 if (c < n_mine) {                             // (columns beyond n_mine hold whatever they held; they are not stored)
-                    float v[OW];
-                    if constexpr (OW == 32) tmem_load32(from + c, v);
-                    else { tmem_load8(from + c, v); tmem_load8(from + c + 8, v + 8); }
-                    tmem_loaded();
+                    f2 v[LW];
+                    tmem_load_pairs<LW>(from + c, v);
 #pragma unroll
-                    for (int e = 0; e < OW; e += 2) {
-                        float2 o = make_float2(O[c + e], O[c + e + 1]);
-                        if (!same) o = mul2(o, c2);
-                        o = fma2(make_float2(v[e], v[e + 1]), vi2, o);
-                        O[c + e] = o.x;
-                        O[c + e + 1] = o.y;
-                    }
+                    for (int e = 0; e < LW; ++e) O[c / 2 + e] = fma2(v[e], vi2, mul2(O[c / 2 + e], c2));
                 }
             }
+            fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&o_empty[t & 1u]);
+            return true;
         };
-        unsigned t = 0, at_t = 0, round = 0;                  // t % depth, t / depth % 2
-        Walk w(s_slot, s_pos, s_breaks, n_tok);
-        for (; w.next(p); ++t) {
-            if (!wait_for(s_full, t & 1u)) { ok = false; break; }
-            fence_after();
-            float s[KP];
-            const float* ki = k_inv + at_t * geo.k_sets * kKeys + hf * KP;
-            constexpr int SW = NVS == 1 ? KP : 8;             // scores in flight (a wide value leaves fewer registers)
-#pragma unroll
-            for (int c = 0; c < KP; c += SW) {
-                float v[SW];
-                tmem_load_n<SW>(t_s + lanes + hf * KP + c, v);
-                tmem_loaded();
-#pragma unroll
-                for (int e = 0; e < SW; ++e) s[c + e] = v[e];
-                if (geo.k_sets > 1) scale_by<SW>(s + c, ki + c);
-                for (int st = 1; st < geo.n_kst; ++st) {
-                    tmem_load_n<SW>(t_s + lanes + st * 64 + hf * KP + c, v);
-                    tmem_loaded();
-                    if (geo.k_sets > 1) scale_by<SW>(v, ki + st * kKeys + c);
-#pragma unroll
-                    for (int e = 0; e < SW; ++e) s[c + e] += v[e];
-                }
-                if (geo.k_sets == 1) scale_by<SW>(s + c, ki + c);
+        const unsigned n_tiles = (unsigned)s_rows[0];
+        unsigned my_at = hf, my_round = 0;                    // t % depth, t / depth % 2 (depth is at least 2)
+        // In turn t a group weighs tile t, if there is one.  Its own tile t - 2 it adds when it has the maximum of tile t (the product of its last
+        // weights has had the time of the loads and the maximum), the other group's tile t - 1 behind.  Wide values leave no registers for sums and
+        // scores at a time: both groups' last tiles are added in front.
+        constexpr bool MID = NVS == 1;
+        float m_other = 0.f;
+#pragma unroll 1
+        for (unsigned t = hf; ok && t < n_tiles + (MID ? 2 : 3); t += 2) {
+            ok = false;                                       // (until this turn is done)
+            if (!MID) {
+                bool added = true;
+#pragma unroll 1
+                for (unsigned u = t - 3; added && u != t - 1; ++u)         // (below zero: none)
+                    if (u < n_tiles) added = add_values(u, u == t - 2 ? m_own : m_other, wi_own, sum_own);
+                if (!added) break;
             }
-            const float2 mult2 = make_float2(mult, mult);
-#pragma unroll
-            for (int e = 0; e < KP; e += 2) {
-                const float2 x = mul2(make_float2(s[e], s[e + 1]), mult2);
-                s[e] = x.x;
-                s[e + 1] = x.y;
-            }
-            fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(s_empty);
-            // ---- cap, distance bias, visibility ----
-            const int k0 = w.j0 + hf * KP;
-            if (cap > 0.f) {
-                const float2 ic = make_float2(inv_cap, inv_cap);
-#pragma unroll
-                for (int e = 0; e < KP; e += 2) {
-                    const float2 x = mul2(make_float2(s[e], s[e + 1]), ic);
-                    s[e] = x.x;
-                    s[e + 1] = x.y;
-                }
-                float big = 0.f;
-#pragma unroll
-                for (int e = 0; e < KP; ++e) big = fmaxf(big, fabsf(s[e]));
-                // each score takes the form that its own magnitude asks for; whether all of them are near zero decides the speed only
-                const float2 cc = make_float2(cap * kLog2e, cap * kLog2e);
-                const bool near = __all_sync(0xffffffffu, big <= kTanhRange);
-                if (NVS == 1 && near) {                       // (wide values: one copy of the code, whose registers are few)
-#pragma unroll
-                    for (int e = 0; e < KP; e += 2) {
-                        const float2 r = mul2(tanh_near_zero(make_float2(s[e], s[e + 1])), cc);
-                        s[e] = r.x;
-                        s[e + 1] = r.y;
-                    }
-                } else {
-#pragma unroll
-                    for (int e = 0; e < KP; e += 2) {
-                        float2 r = tanh_near_zero(make_float2(s[e], s[e + 1]));
-                        if (NVS == 1 || !near) {
-                            if (!(fabsf(s[e]) <= kTanhRange)) r.x = tanhf(s[e]);
-                            if (!(fabsf(s[e + 1]) <= kTanhRange)) r.y = tanhf(s[e + 1]);
-                        }
-                        r = mul2(r, cc);
-                        s[e] = r.x;
-                        s[e + 1] = r.y;
-                    }
-                }
-            }
-            if (p.slopes) {
-                const float base = (float)(my_pos - k0);
-                const float2 ns = make_float2(-slope, -slope);
-#pragma unroll
-                for (int e = 0; e < KP; e += 2) {
-                    const float2 r = fma2(ns, make_float2(base - (float)e, base - (float)(e + 1)), make_float2(s[e], s[e + 1]));
-                    s[e] = r.x;
-                    s[e + 1] = r.y;
-                }
-            }
-            auto hide = [&](float x) {                        // x in the place of every key that the row does not see
-                const bool live = tok >= w.seg_a && tok < w.seg_b;
-                const int last = live ? min(w.k_end - 1, ranged ? 0x7fffffff : my_pos) : -1, first = ranged ? w.lo : my_lo;
-                if (__all_sync(0xffffffffu, k0 + KP - 1 <= last && (k0 >= first || k0 + KP - 1 < kept))) return;
-#pragma unroll
-                for (int e = 0; e < KP; ++e) {
-                    const int j = k0 + e;
-                    if (!(j <= last && (j >= first || j < kept))) s[e] = x;
-                }
-            };
-            hide(-CUDART_INF_F);
-            float mx = s[0];
-#pragma unroll
-            for (int e = 1; e < KP; ++e) mx = max_nan(mx, s[e]);
-            // (two exchanges a tile in two places: whoever writes one has seen the other threads leave the one before)
-            row_x[hf * kRows + row] = mx;
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&pair[qt]);
-            if (!wait_for(&pair[qt], 0)) { ok = false; break; }
-#pragma unroll
-            for (int i = 1; i < RT; ++i) mx = max_nan(mx, row_x[(hf ^ i) * kRows + row]);
-            const float m_new = max_nan(m_run, mx);
-            const float base = m_new == -CUDART_INF_F ? 0.f : m_new, corr = m_run == -CUDART_INF_F ? 0.f : ex2(m_run - base);
-            const float2 nb = make_float2(-base, -base);
-#pragma unroll
-            for (int c = 0; c < LP; ++c) {
-                float2 sum = make_float2(0.f, 0.f);
-#pragma unroll
-                for (int e = 16 * c; e < 16 * c + 16; e += 2) {
-                    const float2 a = add2(make_float2(s[e], s[e + 1]), nb);
-                    s[e] = ex2(a.x);
-                    s[e + 1] = ex2(a.y);
-                    sum = add2(sum, make_float2(s[e], s[e + 1]));
-                }
-                l_run[c] = fmaf(l_run[c], corr, sum.x + sum.y);
-            }
-            m_run = m_new;
-            // weight x its value's magnitude, and the largest of them that this row has in the tile
-            if (!geo.shared_kv && !wait_for(&v_ready[at_t], round)) { ok = false; break; }
-            scale_by<KP>(s, v_inv + at_t * kKeys + hf * KP);
-            auto largest = [&] {
-                float v = s[0];
-#pragma unroll
-                for (int e = 1; e < KP; ++e) v = max_nan(v, s[e]);
-                return v;
-            };
-            float wm = largest();
-            if (__any_sync(0xffffffffu, wm != wm)) {          // a value that cannot be split, 0 x NaN where it is not seen
-                hide(0.f);
-                wm = largest();
-                if (wm != wm) l_run[0] = CUDART_NAN_F;
-            }
-            row_x[(RT + hf) * kRows + row] = wm;
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&pair[qt]);
-            // (meanwhile) the value product of the tile before is done: the weights' columns are free, and its sum can be taken
-            if (t > 0) {
-                if (!wait_for(pv_done, (t - 1) & 1u)) { ok = false; break; }
+            float m_old = -CUDART_INF_F;
+            if (t < n_tiles) {
+                if (!wait_for(&s_full[hf], (t >> 1) & 1u)) break;
                 fence_after();
-            }
-            if (!wait_for(&pair[qt], 1)) { ok = false; break; }
-            float wi;
+                const int4 tile = s_tile[my_at];
+                f2 s[kKeys / 2];
+                const float* ki = k_inv + my_at * geo.k_sets * kKeys;
+                const uint32_t from = t_s + lanes + (geo.s_bufs == 2 ? (t & 1u) * 64u * geo.n_kst : 0u);
 #pragma unroll
-            for (int i = 1; i < RT; ++i) wm = fmaxf(wm, row_x[(RT + (hf ^ i)) * kRows + row]);
-            const float wscale = scale_of(wm, wi);
-            const float2 ws = make_float2(wscale, wscale);
+                for (int c = 0; c < kKeys; c += 2 * LW) {
+                    tmem_load_pairs<LW>(from + c, s + c / 2);
+                    if (geo.k_sets > 1) scale_by<LW>(s + c / 2, ki + c);
+#pragma unroll 1
+                    for (int st = 1; st < geo.n_kst; ++st) {
+                        f2 v[LW];
+                        tmem_load_pairs<LW>(from + st * 64 + c, v);
+                        if (geo.k_sets > 1) scale_by<LW>(v, ki + st * kKeys + c);
 #pragma unroll
-            for (int c = 0; c < KP / 16; ++c) {
-                uint32_t hi[8], lo[8];
-#pragma unroll
-                for (int e = 0; e < 8; ++e) {
-                    const float2 q = mul2(make_float2(s[c * 16 + 2 * e], s[c * 16 + 2 * e + 1]), ws);
-                    split2(q.x, q.y, hi[e], lo[e]);
+                        for (int e = 0; e < LW; ++e) s[c / 2 + e] = add2(s[c / 2 + e], v[e]);
+                    }
+                    if (geo.k_sets == 1) scale_by<LW>(s + c / 2, ki + c);
                 }
-                tmem_store8(t_p + lanes + hf * (KP / 2) + c * 8, hi);
-                tmem_store8(t_p + lanes + 32 + hf * (KP / 2) + c * 8, lo);
+                fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&s_empty[hf]);
+                const f2 mult2 = twice(mult);
+#pragma unroll
+                for (int e = 0; e < kKeys / 2; ++e) s[e] = mul2(s[e], mult2);
+                // ---- cap, distance bias, visibility ----
+                const int k0 = tile.x;
+                if (cap > 0.f) {
+                    const f2 ic = twice(1.0f / cap), cc = twice(cap * kLog2e);
+                    float big[2] = {0.f, 0.f};
+#pragma unroll
+                    for (int e = 0; e < kKeys / 2; ++e) {
+                        s[e] = mul2(s[e], ic);
+                        float x, y;
+                        unpack2(s[e], x, y);
+                        big[e & 1] = fmaxf(big[e & 1], fmaxf(fabsf(x), fabsf(y)));
+                    }
+                    // Each score takes the form that its own magnitude asks for; whether all of them are near zero decides the speed only.  The other
+                    // form is a rolled loop over the scores in tensor memory, where this tile's weights will be (a launch that has a cap has two
+                    // sets of them): a call or an array in local memory here made every tile's scores pass through local memory (64 capped scores
+                    // 6700 cycles, 2900 without it)
+                    if (__all_sync(0xffffffffu, fmaxf(big[0], big[1]) <= kTanhRange)) {
+#pragma unroll
+                        for (int e = 0; e < kKeys / 2; ++e) s[e] = tanh_near_zero(s[e]);
+                    } else {
+                        if (t >= 2 && !wait_for(&pv_done[hf], ((t - 2) >> 1) & 1u)) break;     // (the weights of the tile two before are read)
+                        fence_after();
+                        const uint32_t at_p = t_p + lanes + (geo.p_bufs == 2 ? (t & 1u) * 64u : 0u);
+#pragma unroll
+                        for (int c = 0; c < kKeys / 8; ++c) {
+                            uint32_t x[8];
+#pragma unroll
+                            for (int e = 0; e < 4; ++e) {
+                                x[2 * e] = (uint32_t)s[c * 4 + e];
+                                x[2 * e + 1] = (uint32_t)(s[c * 4 + e] >> 32);
+                            }
+                            tmem_store8(at_p + c * 8, x);
+                        }
+                        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+#pragma unroll 1
+                        for (int c = 0; c < kKeys; c += 8) {
+                            float x[8];
+                            uint32_t y[8];
+                            tmem_load8(at_p + c, x);
+                            tmem_loaded();
+#pragma unroll
+                            for (int e = 0; e < 8; ++e) {
+                                float near, same;
+                                unpack2(tanh_near_zero(pack2(x[e], x[e])), near, same);
+                                y[e] = __float_as_uint(fabsf(x[e]) <= kTanhRange ? near : tanhf(x[e]));
+                            }
+                            tmem_store8(at_p + c, y);
+                            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                        }
+#pragma unroll
+                        for (int c = 0; c < kKeys; c += 2 * LW) tmem_load_pairs<LW>(at_p + c, s + c / 2);
+                    }
+#pragma unroll
+                    for (int e = 0; e < kKeys / 2; ++e) s[e] = mul2(s[e], cc);
+                }
+                if (p.slopes) {
+                    const float base = (float)(my_pos - k0);
+                    const f2 ns = twice(-slope), down = twice(-2.f);
+                    f2 gap = pack2(base, base - 1.f);
+#pragma unroll
+                    for (int e = 0; e < kKeys / 2; ++e) {
+                        s[e] = fma2(ns, gap, s[e]);
+                        gap = add2(gap, down);                    // (whole numbers)
+                    }
+                }
+                // the keys that the row sees, a bit each
+                uint32_t see[2];
+                {
+                    const bool live = tok >= (tile.y & 0xffff) && tok < tile.y >> 16;
+                    const int end = live ? min(tile.z, ranged ? 0x7fffffff : my_pos + 1) - k0 : 0, from = (ranged ? tile.w : my_lo) - k0, keep = kept - k0;
+#pragma unroll
+                    for (int i = 0; i < 2; ++i) {
+                        auto below = [&](int n) { n -= 32 * i; return n >= 32 ? 0xffffffffu : n <= 0 ? 0u : (1u << n) - 1u; };
+                        see[i] = below(end) & (~below(from) | below(keep));
+                    }
+                }
+                const bool all_seen = __all_sync(0xffffffffu, (see[0] & see[1]) == 0xffffffffu);
+                auto hide = [&](float x) {                        // x in the place of every key that the row does not see
+#pragma unroll
+                    for (int e = 0; e < kKeys / 2; ++e) {
+                        float a, b;
+                        unpack2(s[e], a, b);
+                        a = see[e / 16] >> (2 * e % 32) & 1u ? a : x;
+                        b = see[e / 16] >> (2 * e % 32 + 1) & 1u ? b : x;
+                        s[e] = pack2(a, b);
+                    }
+                };
+                auto largest = [&] {                              // (four chains)
+                    float v[4];
+#pragma unroll
+                    for (int e = 0; e < kKeys / 2; ++e) {
+                        float a, b;
+                        unpack2(s[e], a, b);
+                        v[e & 3] = e < 4 ? max_nan(a, b) : max3_nan(v[e & 3], a, b);
+                    }
+                    return max_nan(max_nan(v[0], v[1]), max_nan(v[2], v[3]));
+                };
+                if (!all_seen) hide(-CUDART_INF_F);
+                const float mx = largest();
+                // the maximum up to the tile before comes from the other group, which has its scores already
+                if (t > 0) {
+                    if (!wait_for(&m_ready[qt], (t - 1) & 1u)) break;
+                    m_old = m_x[(hf ^ 1) * kRows + row];
+                }
+                const float m_new = max_nan(m_old, mx);
+                m_x[hf * kRows + row] = m_new;
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&m_ready[qt]);
+                if (MID && t >= 2 && !add_values(t - 2, m_own, wi_own, sum_own)) break;
+                m_own = m_new;
+                const float base = m_new == -CUDART_INF_F ? 0.f : m_new;
+                const f2 nb = twice(-base);
+                float sum[4];                                     // a sum per 16 keys
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    f2 a = 0;
+#pragma unroll
+                    for (int e = 8 * c; e < 8 * c + 8; ++e) {
+                        float x, y;
+                        unpack2(add2(s[e], nb), x, y);
+                        s[e] = pack2(ex2(x), ex2(y));
+                        a = add2(a, s[e]);
+                    }
+                    float x, y;
+                    unpack2(a, x, y);
+                    sum[c] = x + y;
+                }
+                sum_own = (sum[0] + sum[1]) + (sum[2] + sum[3]);
+                // weight x its value's magnitude, and the largest of them that this row has in the tile
+                if (!geo.shared_kv && !wait_for(&v_ready[my_at], my_round)) break;
+                scale_by<kKeys / 2>(s, v_inv + my_at * kKeys);
+                float wm = largest();
+                if (__any_sync(0xffffffffu, wm != wm)) {          // a value that cannot be split, 0 x NaN where it is not seen
+                    hide(0.f);
+                    wm = largest();
+                    if (wm != wm) sum_own = CUDART_NAN_F;
+                }
+                const f2 ws = twice(scale_of(wm, wi_own));
+                // the weights' columns are free once the value product that read them is done (of two sets: it has been added by now)
+                if (geo.p_bufs == 1 && t > 0) {
+                    if (!wait_for(&pv_done[(t - 1) & 1u], ((t - 1) >> 1) & 1u)) break;
+                    fence_after();
+                }
+                // (the other group has read the place: the tile `rings` before, or with one set and one product two before, has been added)
+                wi_x[(t & (geo.rings - 1u)) * kRows + row] = __float2bfloat16(wi_own);
+                if (hf == 1) sum_x[((t >> 1) & (geo.rings / 2 - 1u)) * kRows + row] = sum_own;
+                const uint32_t to = t_p + lanes + (geo.p_bufs == 2 ? (t & 1u) * 64u : 0u);
+#pragma unroll
+                for (int c = 0; c < kKeys / 16; ++c) {
+                    uint32_t hi[8], lo[8];
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) split2(mul2(s[c * 8 + e], ws), hi[e], lo[e]);
+                    tmem_store8(to + c * 8, hi);
+                    tmem_store8(to + 32 + c * 8, lo);
+                }
+                asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&p_ready[hf]);
+            } else {
+                if (MID && t >= 2 && !add_values(t - 2, m_own, wi_own, sum_own)) break;
+                if (t == n_tiles && t > 0) {                  // (the other group has the last tile)
+                    if (!wait_for(&m_ready[qt], (t - 1) & 1u)) break;
+                    m_old = m_x[(hf ^ 1) * kRows + row];
+                }
             }
-            // with two accumulators the next value product may start before the last one has been added
-            if (t > 0 && geo.o_bufs == 1) add_values(t - 1, corr_prev, wi_prev);
-            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-            fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(p_ready);
-            if (t > 0 && geo.o_bufs == 2) add_values(t - 1, corr_prev, wi_prev);
-            corr_prev = corr;
-            wi_prev = wi;
-            if (++at_t == (unsigned)geo.depth) at_t = 0, round ^= 1u;
+            m_other = m_old;
+            ok = !MID || t == 0 || t > n_tiles || add_values(t - 1, m_old, 0.f, 0.f);
+            my_at += 2;
+            if (my_at >= (unsigned)geo.depth) my_at -= geo.depth, my_round ^= 1u;
         }
-        if (ok && t > 0) {
-            ok = wait_for(pv_done, (t - 1) & 1u);
-            fence_after();
-            add_values(t - 1, corr_prev, wi_prev);
-        }
-        // ---- the threads' denominators, the sink's own term, normalise, store ----
-        // (with two threads they fill the place of the second exchange too: every thread has left it before the last value product)
-#pragma unroll
-        for (int c = 0; c < LP; ++c) row_x[(hf * LP + c) * kRows + row] = l_run[c];
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&pair[qt]);
-        ok = ok && wait_for(&pair[qt], 0);
-        float l = 0.f;
-#pragma unroll
-        for (int i = 0; i < RT * LP; ++i) l += row_x[i * kRows + row];
+        if (hf == 0) sum_x[row] = l;
+        asm volatile("bar.sync 2, %0;" ::"n"(32 * RW) : "memory");
+        l = sum_x[row];
+        // ---- the sink's own term, normalise, store ----
         if (p.sink) l += ex2(fmaf(p.sink[h], kLog2e, m_run == -CUDART_INF_F ? 0.f : -m_run));
         // through shared memory (the ring and the queries are read; 32 rows of this warp's channels): whole lines reach the output, and
         // one rolled loop serves every kind of output.  (Stored from the registers, row by row, 5500 cycles of a CTA, mostly fetching
@@ -946,7 +1017,7 @@ split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_co
         float* stage = reinterpret_cast<float*>(smem) + (size_t)warp * 32 * ldst;
 #pragma unroll
         for (int c = 0; c < DVH; c += 4)
-            if (c < n_mine) *reinterpret_cast<float4*>(stage + lane * ldst + c) = make_float4(O[c] * f, O[c + 1] * f, O[c + 2] * f, O[c + 3] * f);
+            if (c < n_mine) *reinterpret_cast<ulonglong2*>(stage + lane * ldst + c) = make_ulonglong2(mul2(O[c / 2], twice(f)), mul2(O[c / 2 + 1], twice(f)));
         __syncwarp();
         const int w4 = max(0, min(n_mine, p.vdim - c0)) >> 2; // (vdim is a multiple of 4)
         for (unsigned again = __ballot_sync(0xffffffffu, ok && tok < n_tok && l != l && w4 > 0); again; again &= again - 1) {
@@ -978,190 +1049,158 @@ split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_co
             sc += 32;
             while (sc >= w4) { sc -= w4; ++sr; }
         }
-    } else if (warp < RW + 4) {
-        // ================= keys and values: warp lw takes keys 16 lw .. + 15 of a tile, a lane one key of either eight =================
-        if constexpr (kFetchRegs < kLaunchRegs) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kFetchRegs));
-        const int lw = warp - RW, kin = lane & 7, cq = lane >> 3;
-        unsigned at = 0;                                      // ring position
-        bool ok = true;
-        size_t cur[2] = {~(size_t)0, ~(size_t)0}, prev[2];    // row of the two keys in the pages of kv head 0 (~0: none)
-        const SlotTiles* const plan = reinterpret_cast<const SlotTiles*>(p.work);
-        auto split_tile = [&](int slot, int j0) -> int {      // the tile of the room that holds these keys (-1: none)
-            if (!plan) return -1;
-            const SlotTiles s = plan[slot];
-            const int j = j0 / kKeys;
-            return j >= s.first && j < s.end ? s.base + j : j == 0 ? s.zero : -1;
-        };
-        // a part that is split already; with scales, the tile's come along: warp 1 brings its keys' and warp 2 its values' (whose tile is t)
-        auto copied = [&](int tile, int part, unsigned bytes, bool scales, unsigned t) {
-            const unsigned slot = at % geo.n_slots;
-            if (lane == 0) ok = wait_for(&empty[slot], ((at / geo.n_slots) & 1u) ^ 1u);
-            ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
-            if (!ok) return;
-            const unsigned char* work = reinterpret_cast<const unsigned char*>(p.work);
-            if (lw == 0 && lane == 0) {
-                mbar_arrive_expect_tx(&full[slot], bytes);
-                const size_t off = (size_t)tile * geo.tile_bytes + part_offset(geo, part);
-                asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                                 smem_u32(ring + (size_t)slot * geo.slot_bytes)),
-                             "l"(work + geo.tile_off + off), "r"(bytes), "r"(smem_u32(&full[slot]))
+    } else {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kOtherRegs));
+        if (warp > RW) {
+            // ================= keys and values =================
+            const int lw = warp - RW - 1, kin = lane & 7, cq = lane >> 3;
+            unsigned slot = 0, phase = 0;                         // the ring's next place, rounds % 2
+            bool ok = true;
+            const unsigned char* const work = reinterpret_cast<const unsigned char*>(p.work);
+            const size_t k_first = part_offset(geo, p.talk ? 0 : g * geo.n_kst), v_first = geo.shared_kv ? k_first : part_offset(geo, geo.k_parts + g * geo.n_vst);
+            const unsigned k_step = kKeys * 4u * geo.wk0, v_step = kKeys * 4u * (geo.shared_kv ? geo.wk0 : geo.wv0);
+            auto copy = [&](void* dst, const unsigned char* src, unsigned bytes, uint64_t* bar) {
+                asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(dst)), "l"(src), "r"(bytes),
+                             "r"(smem_u32(bar))
                              : "memory");
-            }
-            if (scales) {
-                const float* src = reinterpret_cast<const float*>(work + geo.scale_off) + (size_t)tile * geo.sets * kKeys + 2 * lane;
-                const unsigned at_t = t % geo.depth;
-                if (lw == 1)
-                    for (int i = 0; i < geo.k_sets; ++i)
-                        *reinterpret_cast<float2*>(k_inv + (at_t * geo.k_sets + i) * kKeys + 2 * lane) =
-                            *reinterpret_cast<const float2*>(src + (geo.k_sets > 1 ? i : g) * kKeys);
-                if (lw == 2 && !geo.shared_kv)
-                    *reinterpret_cast<float2*>(v_inv + at_t * kKeys + 2 * lane) = *reinterpret_cast<const float2*>(src + (p.kv_heads + g) * kKeys);
-                __syncwarp();
-                if (lane == 0 && !geo.shared_kv) mbar_arrive(&v_ready[at_t]);
-            }
-            if (lw != 0 && lane == 0) mbar_arrive(&full[slot]);
-            ++at;
-        };
-        auto row_of = [&](const float* cache, int width, int gg, size_t row) {
-            return cache + (row != ~(size_t)0 ? (row + (size_t)gg * p.page_size) * width : 0);
-        };
-        // channels [c0, c0 + w) of rows of `width` floats, of which [0, row_w) set the scale.  m_row: the rows' largest magnitudes - taken
-        // (first) or as taken by the first group; inv: where the scales go (null: they are there); ready: told when they are
-        auto stage = [&](const float* cache, int width, int row_w, int c0, int w, int wp, int gg, const size_t (&rows)[2], float (&m_row)[2],
-                         bool first, float* inv, uint64_t* ready) {
-            // groups of eight keys at a time: 16 float4 of two do not fit 64 or 80 registers (us, wide values, two / one: nine sequences over
-            // 1134 keys that the room for split keys does not hold 320 / 241, 4096 rows over latent rows of 256 + 32 440 / 405)
-            constexpr int KG = RT == 4 || NVS == 2 ? 1 : 2;
-            const unsigned slot = at % geo.n_slots;
-#pragma unroll 1
-            for (int half = 0; half < 2; half += KG) {
-                float4 v[8 * KG];
-#pragma unroll
-                for (int u = 0; u < KG; ++u) {
-                    const size_t at_row = half + u ? rows[1] : rows[0];
-                    const bool in = at_row != ~(size_t)0;
-                    const float* src = row_of(cache, width, gg, at_row) + c0;
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        const int c = 8 * (cq + 4 * i);
-                        const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
-                        v[u * 8 + 2 * i] = in && c < w ? *reinterpret_cast<const float4*>(src + c) : z;
-                        v[u * 8 + 2 * i + 1] = in && c + 4 < w ? *reinterpret_cast<const float4*>(src + c + 4) : z;
-                    }
-                }
-                float sc[KG], inverse[KG];
-#pragma unroll
-                for (int u = 0; u < KG; ++u) {
-                    float m = half + u ? m_row[1] : m_row[0];
-                    if (first) {
-                        const size_t at_row = half + u ? rows[1] : rows[0];
-                        m = 0.f;
-#pragma unroll
-                        for (int i = 0; i < 8; ++i) m = max_abs4(m, v[u * 8 + i]);
-                        if (w < row_w && at_row != ~(size_t)0)
-                            for (int c = w + 4 * cq; c < row_w; c += 16) m = max_abs4(m, *reinterpret_cast<const float4*>(row_of(cache, width, gg, at_row) + c));
-                        m = row_max(m);
-                        if (half + u) m_row[1] = m;
-                        else m_row[0] = m;
-                    }
-                    if (scale_row(m, sc[u], inverse[u])) {
-#pragma unroll
-                        for (int i = 0; i < 8; ++i) v[u * 8 + i] = make_float4(0.f, 0.f, 0.f, 0.f);
-                    }
-                }
-                auto put_scales = [&] {
-                    if (inv && lane < 8) {
-#pragma unroll
-                        for (int u = 0; u < KG; ++u) inv[lw * 16 + (half + u) * 8 + lane] = inverse[u];
-                    }
-                };
-                if (ready) {                                  // (their place is free by then: see geometry_of)
-                    put_scales();
-                    __syncwarp();
-                    if (half + KG == 2 && lane == 0) mbar_arrive(ready);
-                }
-                if (half == 0 && !wait_for(&empty[slot], ((at / geo.n_slots) & 1u) ^ 1u)) { ok = false; return; }
-                if (!ready) put_scales();
-                unsigned char* base = ring + (size_t)slot * geo.slot_bytes;
-                const int blocks = wp >> 3;
-#pragma unroll
-                for (int u = 0; u < KG; ++u)
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        const int c8 = cq + 4 * i;
-                        if (c8 < blocks) {
-                            const float4 a = v[u * 8 + 2 * i], b = v[u * 8 + 2 * i + 1];
-                            uint32_t hi[4], lo[4];
-                            split2(a.x * sc[u], a.y * sc[u], hi[0], lo[0]);
-                            split2(a.z * sc[u], a.w * sc[u], hi[1], lo[1]);
-                            split2(b.x * sc[u], b.y * sc[u], hi[2], lo[2]);
-                            split2(b.z * sc[u], b.w * sc[u], hi[3], lo[3]);
-                            unsigned char* dst = base + ((lw * 2 + half + u) * blocks + c8) * 128 + kin * 16;
-                            *reinterpret_cast<uint4*>(dst) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-                            *reinterpret_cast<uint4*>(dst + kKeys * wp * 2) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+            };
+            int4 about{};                                         // what the row warps are told of the newest tile
+            struct Tile { int split, slot, j0, k_end; };          // split: the tile of the room that holds these keys (-1: none)
+            // the ring's next part: key group `part` of the tile at place at_t of the numbers' rings, or value group `part` of it
+            auto fetch = [&](const Tile& z, unsigned at_t, bool is_v, int part) {
+                const int last = (is_v ? geo.n_vst : geo.n_kst) - 1;
+                const int wp = is_v ? (part == last ? geo.v_last_layout : geo.v0_layout) : (part == last ? geo.wk_last : geo.wk0);
+                if (z.split >= 0) {                               // split already: with its first key group a tile's scales come along
+                    if (lane == 0) {
+                        ok = wait_for(&empty[slot], phase ^ 1u);
+                        if (lw == 0) {
+                            const unsigned bytes = kKeys * wp * 4;
+                            const bool scales = !is_v && part == 0;
+                            if (scales) s_tile[at_t] = about;
+                            mbar_arrive_expect_tx(&full[slot], bytes + (scales ? kKeys * 4u * geo.k_sets : 0u));
+                            copy(ring + (size_t)slot * geo.slot_bytes, work + geo.tile_off + (size_t)z.split * geo.tile_bytes + (is_v ? v_first + part * v_step : k_first + part * k_step),
+                                 bytes, &full[slot]);
+                            if (scales) {
+                                const unsigned char* src = work + geo.scale_off + (size_t)z.split * geo.sets * kKeys * 4;
+                                copy(k_inv + at_t * geo.k_sets * kKeys, src + (geo.k_sets > 1 ? 0 : g) * kKeys * 4, kKeys * 4u * geo.k_sets, &full[slot]);
+                                if (!geo.shared_kv) {
+                                    mbar_arrive_expect_tx(&v_ready[at_t], kKeys * 4u);
+                                    copy(v_inv + at_t * kKeys, src + (p.kv_heads + g) * kKeys * 4, kKeys * 4u, &v_ready[at_t]);
+                                }
+                            }
+                        } else {
+                            if (!is_v && part == 0 && !geo.shared_kv) mbar_arrive(&v_ready[at_t]);
+                            mbar_arrive(&full[slot]);
                         }
                     }
-            }
-            fence_smem_async();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&full[slot]);
-            ++at;
-        };
-        // the value groups of tile t; a shared row's scale is its key's, m_key
-        auto values = [&](unsigned t, const size_t (&rows)[2], int tile, const float (&m_key)[2]) {
-            float m_row[2] = {m_key[0], m_key[1]};
-            for (int vs = 0; vs < NVS && ok; ++vs) {
-                const int wl = vs == geo.n_vst - 1 ? geo.v_last_layout : geo.v0_layout;
-                const bool owns = vs == 0 && !geo.shared_kv;
-                if (tile >= 0)
-                    copied(tile, geo.shared_kv ? vs : geo.k_parts + g * geo.n_vst + vs, kKeys * wl * 4, false, t);
-                else
-                    stage(p.vcache, p.vrow, p.vdim, vs * kGroupW, min(kGroupW, (geo.shared_kv ? p.kdim : p.vdim) - vs * kGroupW), wl, g, rows, m_row, owns,
-                          owns ? v_inv + (t % geo.depth) * kKeys : nullptr, owns ? &v_ready[t % geo.depth] : nullptr);
-            }
-        };
-        int tile = -1, prev_tile = -1;
-        float m_key[2] = {0.f, 0.f}, m_prev[2];
-        unsigned t = 0;
-        Walk w(s_slot, s_pos, s_breaks, n_tok);
-        for (; ok && w.next(p); ++t) {
-            const int slot = s_slot[w.seg_a];
-            prev_tile = tile;
-            tile = split_tile(slot, w.j0);
-#pragma unroll
-            for (int kg = 0; kg < 2; ++kg) {
-                const int j = w.j0 + lw * 16 + kg * 8 + kin;
-                prev[kg] = cur[kg];
-                cur[kg] = ~(size_t)0;
-                if (tile < 0 && j < w.k_end) {
-                    const int page = p.table ? p.table[(size_t)slot * p.max_pages + j / p.page_size] : slot;
-                    cur[kg] = (size_t)page * p.kv_heads * p.page_size + (p.table ? j % p.page_size : j);
+                    ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
+                    return;
+                }
+                // Beyond the room: split here, eight keys at a time, a lane a part of one.  Rolled and with few registers, since the row warps have the
+                // others: keys that are split in advance are the rule.
+                const bool shared = is_v && geo.shared_kv;        // (a shared row's scale is its key's)
+                const float* const cache = is_v ? p.vcache : p.kcache;
+                const int width = is_v ? p.vrow : p.kdim, row_w = is_v && !shared ? p.vdim : p.kdim, c0 = p.talk && !is_v ? 0 : part * kGroupW;
+                const int gg = p.talk && !is_v ? part : g, w = min(kGroupW, row_w - c0);
+                float* const inv = is_v ? (part == 0 && !shared ? v_inv + at_t * kKeys : nullptr)
+                                        : part == 0 || geo.k_sets > 1 ? k_inv + (at_t * geo.k_sets + (geo.k_sets > 1 ? part : 0)) * kKeys : nullptr;
+#pragma unroll 1
+                for (int e = lw; e < kKeys / 8; e += kFetchWarps) {
+                    const int j = z.j0 + e * 8 + kin;
+                    const bool in = j < z.k_end;
+                    const float* src = cache;
+                    if (in) {
+                        const int page = p.table ? p.table[(size_t)z.slot * p.max_pages + j / p.page_size] : z.slot;
+                        src += (((size_t)page * p.kv_heads + gg) * p.page_size + (p.table ? j % p.page_size : j)) * width;
+                    }
+                    float m = 0.f, sc, inverse;
+#pragma unroll 1
+                    for (int c = 4 * cq; in && c < row_w; c += 16) m = max_abs4(m, *reinterpret_cast<const float4*>(src + c));
+                    const bool bad = scale_row(row_max(m), sc, inverse);
+                    // (a value's scales have their place before the ring has one: see geometry_of)
+                    if (e == lw && !is_v && !wait_for(&empty[slot], phase ^ 1u)) { ok = false; return; }
+                    if (inv && lane < 8) inv[e * 8 + lane] = inverse;
+                    if (e == 0 && !is_v && part == 0 && lane == 0) s_tile[at_t] = about;
+                    if (e == lw && is_v && !wait_for(&empty[slot], phase ^ 1u)) { ok = false; return; }
+                    const int blocks = wp >> 3;
+                    unsigned char* dst = ring + (size_t)slot * geo.slot_bytes + e * blocks * 128 + kin * 16;
+#pragma unroll 1
+                    for (int c8 = cq; c8 < blocks; c8 += 4) {
+                        const float4 none = make_float4(0.f, 0.f, 0.f, 0.f);
+                        const float4 a = in && !bad && 8 * c8 < w ? *reinterpret_cast<const float4*>(src + c0 + 8 * c8) : none;
+                        const float4 b = in && !bad && 8 * c8 + 4 < w ? *reinterpret_cast<const float4*>(src + c0 + 8 * c8 + 4) : none;
+                        uint32_t hi[4], lo[4];
+                        split2(a.x * sc, a.y * sc, hi[0], lo[0]);
+                        split2(a.z * sc, a.w * sc, hi[1], lo[1]);
+                        split2(b.x * sc, b.y * sc, hi[2], lo[2]);
+                        split2(b.z * sc, b.w * sc, hi[3], lo[3]);
+                        *reinterpret_cast<uint4*>(dst + c8 * 128) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+                        *reinterpret_cast<uint4*>(dst + c8 * 128 + kKeys * wp * 2) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+                    }
+                }
+                fence_smem_async();
+                __syncwarp();
+                if (lane == 0 && is_v && inv) mbar_arrive(&v_ready[at_t]);
+                if (lane == 0) mbar_arrive(&full[slot]);
+            };
+            // the keys of a tile, then the values of the tile s_bufs before: the order in which they are multiplied
+            Tile z0{}, z1{}, z2{};                                // the newest first
+            unsigned at0 = 0, at1 = 0, at2 = 0;                   // their places
+            int known = -1, left = geo.s_bufs, n = 0;             // the sequence whose tiles in the room are known; turns that are left without keys; tiles so far
+            SlotTiles room{};
+            bool more = true;
+            Walk w(s_slot, s_pos, s_breaks, n_tok);
+#pragma unroll 1
+            while (ok) {
+                more = more && w.next(p);
+                if (!more && left-- == 0) break;                  // (the last turns have values only)
+                z2 = z1; at2 = at1;
+                z1 = z0; at1 = at0;
+                if (more) {
+                    if (n > 0 && ++at0 == (unsigned)geo.depth) at0 = 0;
+                    z0.slot = s_slot[w.seg_a];
+                    z0.j0 = w.j0;
+                    z0.k_end = w.k_end;
+                    about = make_int4(w.j0, w.seg_a | w.seg_b << 16, w.k_end, w.lo);
+                    z0.split = -1;
+                    if (work) {
+                        if (z0.slot != known) room = reinterpret_cast<const SlotTiles*>(work)[known = z0.slot];
+                        const int j = w.j0 / kKeys;
+                        z0.split = j >= room.first && j < room.end ? room.base + j : j == 0 ? room.zero : -1;
+                    }
+                }
+                ++n;
+                const bool values = n > geo.s_bufs;               // of the tile s_bufs turns before
+                const int nk = more ? geo.n_kst : 0, parts = nk + (values ? geo.n_vst : 0);
+#pragma unroll 1
+                for (int i = 0; i < parts && ok; ++i) {
+                    const bool is_v = i >= nk, two = geo.s_bufs == 2;
+                    fetch(!is_v ? z0 : two ? z2 : z1, !is_v ? at0 : two ? at2 : at1, is_v, is_v ? i - nk : i);
+                    if (++slot == (unsigned)geo.n_slots) slot = 0, phase ^= 1u;
                 }
             }
-            m_prev[0] = m_key[0];
-            m_prev[1] = m_key[1];
-            for (int st = 0; st < geo.n_kst && ok; ++st) {
-                const int wp = st == geo.n_kst - 1 ? geo.wk_last : geo.wk0;
-                const bool first = st == 0 || geo.k_sets > 1;
-                if (tile >= 0)
-                    copied(tile, p.talk ? st : g * geo.n_kst + st, kKeys * wp * 4, st == 0, t);
-                else
-                    stage(p.kcache, p.kdim, p.kdim, p.talk ? 0 : st * kGroupW, p.talk ? p.kdim : min(kGroupW, p.kdim - st * kGroupW), wp, p.talk ? st : g,
-                          cur, m_key, first, first ? k_inv + ((t % geo.depth) * geo.k_sets + (geo.k_sets > 1 ? st : 0)) * kKeys : nullptr, nullptr);
-            }
-            if (t > 0 && ok) values(t - 1, prev, prev_tile, m_prev);
-        }
-        if (t > 0 && ok) values(t - 1, cur, tile, m_key);
-    } else {
-        asm volatile("setmaxnreg.dec.sync.aligned.u32 32;");
-        if (warp == RW + 4) {
-            // ================= the MMA issuer: the whole warp walks, one elected lane issues =================
+        } else {
+            // ================= the MMA issuer: the whole warp counts tiles, one elected lane issues =================
+            // The number of tiles and the address in tensor memory are broadcast, so that everything below is known to be the same for the
+            // whole warp and the instructions' operands stay in uniform registers.  (In a loop that walked the tiles itself an instruction
+            // took 100 cycles to issue for the scores and 160 for the values: 4300 cycles of a tile.)
+            int n_tiles = 0;
+            for (Walk w(s_slot, s_pos, s_breaks, n_tok); w.next(p);) ++n_tiles;
+            n_tiles = __shfl_sync(0xffffffffu, n_tiles, 0);
+            if (lane == 0) s_rows[0] = n_tiles;
+            asm volatile("bar.arrive 1, %0;" ::"n"(32 * RW + 32) : "memory");
+            const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0);
+            const uint32_t t_s = tm, t_p = tm + 64u * geo.n_kst * geo.s_bufs, t_o = t_p + 64u * geo.p_bufs;
             const uint32_t idesc_s = (1u << 4) | ((uint32_t)(kKeys >> 3) << 17) | ((uint32_t)(kRows >> 4) << 24);
             const uint32_t q_addr = smem_u32(qs), ring_addr = smem_u32(ring);
             unsigned at = 0;
             bool ok = true;
             auto values = [&](unsigned t) {                   // value product of tile t
-                if (!wait_warp(p_ready, t & 1u)) { ok = false; return; }
+                if (!wait_warp(&p_ready[t & 1u], (t >> 1) & 1u)) { ok = false; return; }
+                const unsigned before = t - geo.o_bufs;       // the tile whose product lay there
+                if (t >= (unsigned)geo.o_bufs && !wait_warp(&o_empty[before & 1u], (before >> 1) & 1u)) { ok = false; return; }
+                const uint32_t weights = t_p + (geo.p_bufs == 2 ? (t & 1u) * 64u : 0u);
+#pragma unroll 1
                 for (int vs = 0; vs < NVS; ++vs) {
                     const unsigned slot = at % geo.n_slots;
                     if (!wait_warp(&full[slot], (at / geo.n_slots) & 1u)) { ok = false; return; }
@@ -1173,25 +1212,26 @@ split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_co
                     const uint32_t step = 2u * wp;            // 16 keys, in descriptor units of 16 bytes
                     const uint32_t d = t_o + 128u * (geo.o_bufs == 2 ? t & 1u : (unsigned)vs);
                     if (elect_one_sync()) {
+#pragma unroll 1
+                        for (uint32_t e = 0; e < 3; ++e) {        // lo hi, hi lo, hi hi
 #pragma unroll
-                        for (uint32_t k = 0; k < 4; ++k) mma_ts(d, t_p + 32u + 8u * k, vh + k * step, idesc, k != 0);
-#pragma unroll
-                        for (uint32_t k = 0; k < 4; ++k) mma_ts(d, t_p + 8u * k, vl + k * step, idesc, 1u);
-#pragma unroll
-                        for (uint32_t k = 0; k < 4; ++k) mma_ts(d, t_p + 8u * k, vh + k * step, idesc, 1u);
+                            for (uint32_t k = 0; k < 4; ++k) mma_ts(d, weights + (e == 0 ? 32u : 0u) + 8u * k, (e == 1 ? vl : vh) + k * step, idesc, (e | k) != 0);
+                        }
                         commit_to(&empty[slot]);
-                        if (vs == NVS - 1) commit_to(pv_done);
+                        if (vs == NVS - 1) commit_to(&pv_done[t & 1u]);
                     }
                     __syncwarp();
                     ++at;
                 }
             };
-            unsigned t = 0;
-            Walk w(s_slot, s_pos, s_breaks, n_tok);
             ok = wait_warp(q_ready, 0);
-            for (; ok && w.next(p); ++t) {
-                if (t > 0 && !wait_warp(s_empty, (t - 1) & 1u)) { ok = false; break; }
-                for (int st = 0; st < geo.n_kst; ++st) {
+#pragma unroll 1
+            for (unsigned t = 0; ok && t < (unsigned)(n_tiles + geo.s_bufs); ++t) {
+                const unsigned before = t - geo.s_bufs;       // the tile whose scores lay there, and whose values are next
+                const int groups = t < (unsigned)n_tiles ? geo.n_kst : 0;
+                if (groups > 0 && t >= (unsigned)geo.s_bufs && !wait_warp(&s_empty[before & 1u], (before >> 1) & 1u)) { ok = false; break; }
+#pragma unroll 1
+                for (int st = 0; st < groups; ++st) {
                     const unsigned slot = at % geo.n_slots;
                     if (!wait_warp(&full[slot], (at / geo.n_slots) & 1u)) { ok = false; break; }
                     fence_after();
@@ -1199,33 +1239,35 @@ split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_co
                     const uint32_t ka = ring_addr + slot * geo.slot_bytes, qa = q_addr + st * geo.wk0 * kRows * 4u;
                     const uint64_t kh = block_desc(ka, 128u, wp * 16u), kl = block_desc(ka + kKeys * wp * 2u, 128u, wp * 16u);
                     const uint64_t qh = block_desc(qa, 128u, wp * 16u), ql = block_desc(qa + kRows * wp * 2u, 128u, wp * 16u);
-                    const uint32_t d = t_s + 64u * st;
+                    const uint32_t d = t_s + (geo.s_bufs == 2 ? (t & 1u) * 64u * geo.n_kst : 0u) + 64u * st;
                     if (elect_one_sync()) {
                         const uint32_t n = wp >> 4;           // 16 channels per instruction: 2 blocks, 16 descriptor units
-                        for (uint32_t k = 0; k < n; ++k) mma_ss(d, ql + 16u * k, kh + 16u * k, idesc_s, k != 0);
-                        for (uint32_t k = 0; k < n; ++k) mma_ss(d, qh + 16u * k, kl + 16u * k, idesc_s, 1u);
-                        for (uint32_t k = 0; k < n; ++k) mma_ss(d, qh + 16u * k, kh + 16u * k, idesc_s, 1u);
+#pragma unroll 1
+                        for (uint32_t e = 0; e < 3; ++e) {
+                            const uint64_t qe = e == 0 ? ql : qh, ke = e == 1 ? kl : kh;
+#pragma unroll
+                            for (uint32_t k = 0; k < kGroupW / 16; ++k)
+                                if (k < n) mma_ss(d, qe + 16u * k, ke + 16u * k, idesc_s, (e | k) != 0);
+                        }
                         commit_to(&empty[slot]);
-                        if (st == geo.n_kst - 1) commit_to(s_full);
+                        if (st == geo.n_kst - 1) commit_to(&s_full[t & 1u]);
                     }
                     __syncwarp();
                     ++at;
                 }
-                if (t > 0 && ok) values(t - 1);
+                if (t >= (unsigned)geo.s_bufs && ok && before < (unsigned)n_tiles) values(before);
             }
-            if (t > 0 && ok) values(t - 1);
         }
     }
     fence_before();
     __syncthreads();
-    if (warp == RW + 4) {
+    if (warp == RW) {
         fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem));
     }
 }
 
-// with rt threads per row
-bool geometry_of(const SplitAttention& a, Geometry& g, size_t& smem, int rt) {
+bool geometry_of(const SplitAttention& a, Geometry& g, size_t& smem) {
     if (a.heads <= 0 || a.kv_heads <= 0 || a.heads % a.kv_heads || a.kdim <= 0 || a.vdim <= 0) return false;
     auto mul4 = [](int v) { return v % 4 == 0; };
     auto aligned = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
@@ -1264,47 +1306,63 @@ bool geometry_of(const SplitAttention& a, Geometry& g, size_t& smem, int rt) {
     g.sets = a.kv_heads * (g.shared_kv ? 1 : 2);
     g.tile_bytes = kKeys * 4u * (k_heads * ((g.n_kst - 1) * g.wk0 + g.wk_last) + (g.shared_kv ? 0 : a.kv_heads * ((g.n_vst - 1) * g.wv0 + g.wv_last)));
     g.cap_tiles = 0;
-    if (a.work && a.table && a.rows_per_slot <= 0 && a.n_seq > 0 && aligned(a.work)) {
+    if (a.work && aligned(a.work) && (a.rows_per_slot > 0 ? !a.table && a.n_seq == 0 : a.table && a.n_seq > 0)) {
         g.scale_off = (unsigned)a.n_slots * sizeof(SlotTiles);
         const size_t per = g.tile_bytes + 4u * kKeys * g.sets, fixed = g.scale_off + 128;
         if (a.work_bytes > fixed) g.cap_tiles = (int)std::min<size_t>((a.work_bytes - fixed) / per, 65535);
         g.tile_off = (unsigned)((g.scale_off + 4u * kKeys * g.sets * (unsigned)g.cap_tiles + 127u) & ~127u);
     }
-    g.o_bufs = g.n_vst == 1 && 64 * g.n_kst + 64 + 256 <= 512 ? 2 : 1;
+    // Two of each where tensor memory has the columns.  Two sets of weights first: the groups of row warps do not wait for each other's value
+    // product then.  (Wide values have one product of 256 columns, and keys that lie one tile ahead.)
+    static constexpr int kBufs[][3] = {{2, 2, 2}, {1, 2, 2}, {1, 1, 2}, {1, 2, 1}, {1, 1, 1}};
+    bool fits = false;
+    for (const auto& b : kBufs) {
+        if (g.n_vst == 2 && (b[0] == 2 || b[2] == 2)) continue;
+        if (a.cap > 0.f && b[1] == 1) continue;               // (capped scores pass through the weights' columns)
+        g.s_bufs = b[0]; g.p_bufs = b[1]; g.o_bufs = b[2];
+        fits = 64 * g.n_kst * b[0] + 64 * b[1] + 128 * g.n_vst * b[2] <= 512;
+        if (fits) break;
+    }
+    if (!fits) return false;
     g.slot_bytes = kKeys * std::max(g.wk0, std::max(g.wv0, g.v0_layout)) * 4;
     g.q_bytes = ((g.n_kst - 1) * g.wk0 + g.wk_last) * kRows * 4;
     // A tile's scales are written when its first key group has its slot: the stage n_slots places before is done.  They lie depth tiles
     // apart so that this stage is no earlier than the first value group of the tile whose scales were there (a value group is multiplied
-    // after the rows have used all scales of its tile).  In order, a tile is n_kst key groups and, behind those of the next, n_vst value groups.
+    // after the rows have used all scales of its tile).  In order, a tile is n_kst key groups and, behind those of the s_bufs tiles next, n_vst
+    // value groups.
     const int per_tile = g.n_kst + g.n_vst;
-    auto depth_of = [&](int slots) { return 1 + (slots + g.n_kst + per_tile - 1) / per_tile; };
+    auto depth_of = [&](int slots) { return g.s_bufs + (slots + g.n_kst + per_tile - 1) / per_tile; };
+    // A tile's numbers are stored when its weights are: with one set of weights and one product the tile before has been multiplied by then,
+    // the one before that added.
+    g.rings = g.p_bufs == 1 && g.o_bufs == 1 ? 2 : 4;
     auto control_of = [&](int slots) {
-        return (2 * kMaxSlots + 5 + 4 + kMaxDepth + 1) / 2 * 16 + (depth_of(slots) * kKeys * (g.k_sets + (g.shared_kv ? 0 : 1)) + 2 * rt * kRows + 8) * 4 + 2 * (kRows >> g.pk_shift) * 4;
+        const int depth = depth_of(slots), bars = 2 * slots + 15 + (g.shared_kv ? 0 : depth);
+        return ((bars + 1) & ~1) * 8 + kRows * (2 * 4 + g.rings * 4) + depth * (kKeys * (g.k_sets + (g.shared_kv ? 0 : 1)) * 4 + 16) + 32 + 2 * (kRows >> g.pk_shift) * 4;
     };
     for (g.n_slots = kMaxSlots; g.n_slots >= 2; --g.n_slots)
         if (g.n_slots * g.slot_bytes + g.q_bytes + control_of(g.n_slots) <= kSmemMost) break;
     if (g.n_slots < 2) return false;
     g.depth = depth_of(g.n_slots);
     const int control = control_of(g.n_slots);
-    // the output is staged in the ring and the queries: 4 rt warps of 32 rows, 4 floats between the rows
-    const int staged = kRows * rt * ((g.n_vst == 1 ? (g.wv0 + 8 * rt - 1) / (8 * rt) * 8 : 256 / rt) + 4) * 4;
+    // the output is staged in the ring and the queries: 8 warps of 32 rows, 4 floats between the rows
+    const int staged = kRows * 2 * ((g.n_vst == 1 ? g.wv0 / 2 : 128) + 4) * 4;
     g.q_bytes = std::max(g.q_bytes, staged - g.n_slots * g.slot_bytes);
     smem = (size_t)g.n_slots * g.slot_bytes + g.q_bytes + control;
     return smem <= (size_t)kSmemMost;
 }
 
-template <int NVS, int RT>
+template <int NVS>
 cudaError_t launch_inst(const SplitAttention& a, const Geometry& g, size_t smem, cudaStream_t st) {
     int device = 0;
     cudaError_t e = cudaGetDevice(&device);
-    if (e == cudaSuccess) e = ask_smem<split_attention_kernel<NVS, RT>>(device, kSmemMost);
+    if (e == cudaSuccess) e = ask_smem<split_attention_kernel<NVS>>(device, kSmemMost);
     if (e != cudaSuccess) return e;
     const int tt = kRows >> g.pk_shift, tiles = a.n_seq > 1 ? a.M / tt + a.n_seq : (a.M + tt - 1) / tt;
     if (a.work) {
         split_keys_kernel<<<dim3(std::min(g.cap_tiles, std::max(1, kSplitGrid / g.parts)), g.parts), 256, 0, st>>>(a, g);
         ++extra_launches();
     }
-    split_attention_kernel<NVS, RT><<<(a.heads >> g.pk_shift) * tiles, kSplitThreads<RT>, smem, st>>>(a, g);
+    split_attention_kernel<NVS><<<(a.heads >> g.pk_shift) * tiles, kSplitThreads, smem, st>>>(a, g);
     return cudaGetLastError();
 }
 
@@ -1341,41 +1399,31 @@ bool take_ran_out(int device, cudaStream_t st) {
 bool split_attention_ok(const SplitAttention& a) {
     Geometry g;
     size_t smem;
-    return geometry_of(a, g, smem, 2);
+    return geometry_of(a, g, smem);
 }
+
+int split_attention_keys(const SplitAttention& a, int slot) { return range_keys(a, slot); }
 
 size_t split_attention_work_bytes(const SplitAttention& a, int keys) {
     Geometry g;
     size_t smem;
-    if (!geometry_of(a, g, smem, 2)) return 0;
+    if (!geometry_of(a, g, smem)) return 0;
     return (size_t)a.n_slots * sizeof(SlotTiles) + 256 + (size_t)((keys + kKeys - 1) / kKeys) * (g.tile_bytes + 4u * kKeys * g.sets);
 }
 
 cudaError_t launch_split_attention(const SplitAttention& a, cudaStream_t st) {
     Geometry g;
     size_t smem;
-    if (a.M <= 0 || !geometry_of(a, g, smem, 2)) return cudaErrorNotSupported;
+    if (a.M <= 0 || !geometry_of(a, g, smem)) return cudaErrorNotSupported;
     int device = 0;
     const cudaError_t e = cudaGetDevice(&device);
     if (e != cudaSuccess) return e;
     g.ran_out = split_attention_ran_out(device, st);          // (mapped and unified: one address on both sides)
     if (take_ran_out(device, st)) return cudaErrorLaunchTimeout;
     SplitAttention with = a;
-    // Wide values are split in advance in every step: the fetching warps have few registers for them (9 and 24 decoding sequences over 1000
-    // cached keys, latent rows of 256 + 32, 4 layers: 1714 and 1833 us split by the row tiles, 1139 and 1250 in advance; over 100 keys 867
-    // and 863)
-    if (g.cap_tiles <= 0 || (g.n_vst == 1 && (long long)a.M * (a.heads / a.kv_heads) < kSplitOnceRows)) with.work = nullptr;
-    if (g.n_vst == 2) return launch_inst<2, 2>(with, g, smem, st);
-    // Four threads per row where the keys are split in advance (us, two / four: windowed 4096 rows, 16 heads of 128 over 4 266 / 245, mixed
-    // scores, three prompts of 2048 rows 147 / 117, 4096 rows in chunks of 2048 303 / 263, float32 model 80 / 63).  Their fetching warps have half
-    // the registers (861 rows of Dia, whose keys every row tile splits for itself, 81 / 107); wide values do not fit theirs (451 / 459).
-    Geometry g4;
-    size_t smem4;
-    if (with.work && geometry_of(a, g4, smem4, 4)) {
-        g4.ran_out = g.ran_out;
-        return launch_inst<1, 4>(with, g4, smem4, st);
-    }
-    return launch_inst<1, 2>(with, g, smem, st);
+    // Keys are split in advance wherever there is room: the fetching warps have few registers for them
+    if (g.cap_tiles <= 0) with.work = nullptr;
+    return g.n_vst == 2 ? launch_inst<2>(with, g, smem, st) : launch_inst<1>(with, g, smem, st);
 }
 
 }  // namespace dia

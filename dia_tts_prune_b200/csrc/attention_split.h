@@ -38,9 +38,9 @@ struct SplitAttention {
     const float* gate; const float* head_gate; int ldg;
     // Optional (n_seq 0: not given): the step's sequences - slot, first row and row count of each
     const int* seq_slot; const int* seq_row0; const int* seq_count; int n_seq;
-    // Optional, with the sequences: room in which a launch in front splits the keys and values that the rows see once for all row
-    // tiles (null: every row tile splits them for itself).  n_slots: slots there are.  Keys beyond the room's size are split by the
-    // row tiles.
+    // Optional, with the sequences or with rows_per_slot: room in which a launch in front splits the keys and values that the rows see once for
+    // all row tiles (null: every row tile splits them for itself, which takes several times as long).  n_slots: slots there are.  Keys beyond the
+    // room's size are split by the row tiles.
     void* work; size_t work_bytes; int n_slots;
 };
 
@@ -51,6 +51,7 @@ struct SplitAttention {
 bool split_attention_ok(const SplitAttention& a);
 // bytes of `work` for `keys` keys of this shape (0: the shape is not taken)
 size_t split_attention_work_bytes(const SplitAttention& a, int keys);
+int split_attention_keys(const SplitAttention& a, int slot);      // rows_per_slot > 0: how many keys of a slot some row sees
 // The word of `device` that a kernel sets when one of its waits has run out (its outputs are NaN then).  Made by the first call outside of a capture: engines
 // and weight copies are made with one, so that products that are captured have it.
 int* split_attention_ran_out(int device, cudaStream_t st);

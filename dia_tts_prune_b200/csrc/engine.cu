@@ -1040,24 +1040,33 @@ int dia_b200_dense_forward(const float* x, const void* wt_bf16, float* y, void* 
 
 int dia_b200_attention_rows(const float* q, const float* k, const float* v, float* out, int B, int Tq, int Tk, int Hq, int Hkv,
                             int Tk_stride, int mode, const int32_t* n_valid_host, void* stream) {
+    return dia_b200_attention_rows_in(q, k, v, out, B, Tq, Tk, Hq, Hkv, Tk_stride, mode, n_valid_host, nullptr, 0, stream);
+}
+
+size_t dia_b200_attention_rows_work_bytes(int B, int Tq, int Tk, int Hq, int Hkv, int mode, const int32_t* n_valid_host) {
+    return B > 0 && Tq > 0 && Tk >= 0 && mode >= 0 && mode <= 2 ? attention_rows_work_bytes(B, Tq, Tk, Hq, Hkv, mode, n_valid_host) : 0;
+}
+
+int dia_b200_attention_rows_in(const float* q, const float* k, const float* v, float* out, int B, int Tq, int Tk, int Hq, int Hkv,
+                               int Tk_stride, int mode, const int32_t* n_valid_host, void* work, size_t work_bytes, void* stream) {
     if (B < 0 || Tq < 0 || Tk < 0 || Hq <= 0 || Hkv <= 0 || Hq % Hkv || Tk > Tk_stride || mode < 0 || mode > 2 || B > 16)
         return DIA_B200_EINVAL;
     if (B == 0 || Tq == 0) return DIA_B200_OK;
     if (!q || !k || !v || !out) return DIA_B200_EINVAL;
     if ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v) |
-         reinterpret_cast<uintptr_t>(out)) & 15)
+         reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(work)) & 15)
         return DIA_B200_EINVAL;
     if (n_valid_host)
         for (int b = 0; b < B; ++b) if (n_valid_host[b] < 0 || n_valid_host[b] > Tk) return DIA_B200_EINVAL;
-    CK(launch_attention_rows(q, k, v, out, B, Tq, Tk, Hq, Hkv, Tk_stride, mode, n_valid_host, S(stream)));
-    g_launches++;
+    CK(launch_attention_rows(q, k, v, out, B, Tq, Tk, Hq, Hkv, Tk_stride, mode, n_valid_host, work, work_bytes, S(stream)));
+    g_launches += 1 + std::exchange(extra_launches(), 0);
     return DIA_B200_OK;
 }
 
 namespace {
 
 // What a layer of many rows keeps in its workspace: [q | k | v] rows, turned queries and attention output share the room of the gated unit's rows.
-struct RowsRoom { size_t qkv, q, att, gu, split, bytes; };
+struct RowsRoom { size_t qkv, q, att, gu, split, keys, bytes; };      // keys: bytes for the attention, at split
 RowsRoom rows_room(const dia_b200_rows_layer& a) {
     const size_t M = (size_t)a.B * a.T, most = std::max({(size_t)a.D, (size_t)a.heads * 128, (size_t)a.cross_heads * 128, (size_t)a.F});
     const size_t heads = std::max(a.heads, a.cross_heads);
@@ -1067,7 +1076,11 @@ RowsRoom rows_room(const dia_b200_rows_layer& a) {
     r.att = r.q + M * heads * 512;
     r.gu = 0;
     r.split = std::max(r.att + M * heads * 512, M * 8 * (size_t)a.F);
-    r.bytes = r.split + gemm_workspace_bytes((int)M, (int)most);
+    // the attention's split keys lie where the products' split rows lie before and after it
+    const size_t keys = std::max(attention_rows_work_bytes(a.B, a.T, a.T, a.heads, a.kv_heads, a.mode, a.n_valid),
+                                 a.cross_heads > 0 ? attention_rows_work_bytes(a.B, a.T, a.cross_slots, a.cross_heads, a.cross_kv_heads, 2, a.cross_valid) : 0);
+    r.keys = keys;
+    r.bytes = r.split + std::max(gemm_workspace_bytes((int)M, (int)most), keys);
     return r;
 }
 
@@ -1082,8 +1095,8 @@ int rows_dense(const dia_b200_dense_ref& w, const float* x, const float* norm, f
 }
 
 int rows_attention(const float* q, const float* k, const float* v, float* out, int B, int Tq, int Tk, int Hq, int Hkv, int slots, int mode,
-                   const int32_t* n_valid, cudaStream_t st) {
-    CK(launch_attention_rows(q, k, v, out, B, Tq, Tk, Hq, Hkv, slots, mode, n_valid, st));
+                   const int32_t* n_valid, void* work, size_t work_bytes, cudaStream_t st) {
+    CK(launch_attention_rows(q, k, v, out, B, Tq, Tk, Hq, Hkv, slots, mode, n_valid, work, work_bytes, st));
     g_launches += 1 + std::exchange(extra_launches(), 0);
     return DIA_B200_OK;
 }
@@ -1145,14 +1158,14 @@ int dia_b200_rows_layer_forward(const dia_b200_rows_layer* args, void* stream) {
     if (!kv && (rc = rows_dense(a.v, a.x_in, a.norm_self, a.eps, false, nullptr, v, split, M, nk, D, st))) return rc;
     CK(launch_head_rows(qkv, ldq, k, v, ldkv, q, a.k_cache, a.v_cache, a.sin_table, a.cos_table, a.positions, a.B, a.T, a.heads, a.kv_heads, a.slots, a.n_pos, st));
     g_launches++;
-    if ((rc = rows_attention(q, a.k_cache, a.v_cache, att, a.B, a.T, a.T, a.heads, a.kv_heads, a.slots, a.mode, a.n_valid, st))) return rc;
+    if ((rc = rows_attention(q, a.k_cache, a.v_cache, att, a.B, a.T, a.T, a.heads, a.kv_heads, a.slots, a.mode, a.n_valid, split, room.keys, st))) return rc;
     if ((rc = rows_dense(a.o, att, nullptr, 0.f, false, a.x_in, a.x, split, M, D, nq, st))) return rc;
     if (cross) {
         const int nc = a.cross_heads * 128;
         if ((rc = rows_dense(a.cross_q, a.x, a.norm_cross, a.eps, false, nullptr, qkv, split, M, nc, D, st))) return rc;
         CK(launch_head_rows(qkv, nc, nullptr, nullptr, 0, q, nullptr, nullptr, a.sin_table, a.cos_table, a.positions, a.B, a.T, a.cross_heads, 0, 0, a.n_pos, st));
         g_launches++;
-        if ((rc = rows_attention(q, a.cross_k, a.cross_v, att, a.B, a.T, a.cross_slots, a.cross_heads, a.cross_kv_heads, a.cross_slots, 2, a.cross_valid, st))) return rc;
+        if ((rc = rows_attention(q, a.cross_k, a.cross_v, att, a.B, a.T, a.cross_slots, a.cross_heads, a.cross_kv_heads, a.cross_slots, 2, a.cross_valid, split, room.keys, st))) return rc;
         if ((rc = rows_dense(a.cross_o, att, nullptr, 0.f, false, a.x, a.x, split, M, D, nc, st))) return rc;
     }
     if ((rc = rows_dense(a.wi, a.x, a.norm_mlp, a.eps, false, nullptr, gu, split, M, 2 * a.F, D, st))) return rc;

@@ -1023,9 +1023,10 @@ int lm_b200_engine_create(const lm_b200_model* model, const lm_b200_layer* layer
     const size_t R = (size_t)m.max_rows, D = (size_t)m.width;
     size_t qk = 0, att = 0, E = 1, top = 1, F = 1, Sf = 1, slots = 1;
     size_t n_in = 0, k_out = 0, n_rec = 0, split_dim = 0, kv_split = 0;
-    // room for the split keys and values of twice a step's rows and 4096 cached keys more (and a partly filled tile at either end of
-    // every sequence); what does not fit is split where it is used
-    const long long split_keys = std::min<long long>(2LL * m.max_rows + 4096 + 192LL * m.n_slots, 64LL * 65535);
+    // room for the split keys and values of twice a step's rows and 32768 cached keys more, as far as sequences can have them (and a partly filled
+    // tile at either end of every sequence); what does not fit is split where it is used, by few registers
+    const long long cached = std::min<long long>(32768, (long long)m.n_slots * m.max_pages * m.page_size);
+    const long long split_keys = std::min<long long>(2LL * m.max_rows + cached + 192LL * m.n_slots, 64LL * 65535);
     auto split_room = [&](int heads, int kv_heads, int kdim, int vdim, bool latent, const float* talk) {
         dia::SplitAttention s{};
         float* const some = reinterpret_cast<float*>(256);        // (only whether keys and values are one buffer, and alignment, are looked at)

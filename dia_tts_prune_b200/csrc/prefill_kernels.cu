@@ -34,10 +34,10 @@ constexpr int kAK = 64;               // keys per tile
 constexpr int kQStride = 132;         // padded row stride (floats) of the Q and K tiles: conflict-free float4 reads
 constexpr int kPStride = 68;
 constexpr int kAttnThreads = 256;
-// Queries of a batch row from which the attention runs on the tensor cores: its CTAs own 128 of them, and each splits the keys for
-// itself.  us, 16 heads of 128, this kernel / the tensor cores: one text of 64 17 / 24, 200 45 / 43, 256 47 / 44, 861 290 / 99; two texts of
-// 200 45 / 55, 256 48 / 44; two prompts with 4 key heads 400 111 / 56; cross attention over 200 bytes 200 45 / 55, 400 88 / 58.
-constexpr int kSplitRowsMin = 256;
+// Queries of a batch row from which the attention runs on the tensor cores: its CTAs own 128 (query, head) rows, and a launch in front splits
+// the keys.  us a layer, this kernel / the tensor cores, 16 heads of 128: one text of 100 17 / 21, 129 23 / 23, 200 31 / 27, 255 31 / 28; two prompts (4 key
+// heads) and their cross attention over 129 bytes 70 40 / 51, 128 42 / 50, 200 90 / 54.
+constexpr int kSplitRowsMin = 160;
 // AQ: queries per CTA, 64, or 32 where those leave SMs without a CTA (16 heads, one text of 200: 64 CTAs 42 us, 112 31)
 template <int AQ>
 constexpr int kAttnSmem = (AQ * kQStride + kAK * kQStride + kAK * kHeadDim + AQ * kPStride) * 4;
@@ -301,17 +301,35 @@ __global__ void embed_rows_kernel(const float* __restrict__ table, const int* __
 // ---- launchers ------------------------------------------------------------------------------------------------
 static int grid_for(long long n, int block) { return (int)std::min<long long>((n + block - 1) / block, 148 * 16); }
 
-cudaError_t launch_attention_rows(const float* q, const float* k, const float* v, float* out, int B, int Tq, int Tk, int Hq,
-                                  int Hkv, int Tk_stride, int mode, const int* n_valid_host, cudaStream_t st) {
+static bool on_tensor_cores(int B, int Tq) { return B <= 16 && Tq >= kSplitRowsMin; }
+static SplitAttention split_rows(const float* q, const float* k, const float* v, float* out, int B, int Tq, int Tk, int Hq, int Hkv, int Tk_stride, int mode,
+                                 const int* n_valid_host) {
     SplitAttention s{};
-    if (B <= 16 && Tq >= kSplitRowsMin) {                      // the tensor-core kernel with split fp32 operands
-        s.q = q; s.ldq = Hq * kHeadDim; s.qdim = kHeadDim;
-        s.kcache = k; s.vcache = v; s.page_size = Tk_stride;
-        s.heads = Hq; s.kv_heads = Hkv; s.kdim = s.vdim = s.vrow = kHeadDim;
-        s.scale = 0.08838834764831845f;                       // 1/sqrt(128)
-        s.M = B * Tq; s.rows_per_slot = Tq; s.mode = mode; s.n_keys = Tk;
-        for (int b = 0; b < B; ++b) s.n_valid[b] = n_valid_host ? n_valid_host[b] : Tk;
-        s.out = out; s.ldo = Hq * kHeadDim; s.out_scale = 1.f;
+    s.q = q; s.ldq = Hq * kHeadDim; s.qdim = kHeadDim;
+    s.kcache = k; s.vcache = v; s.page_size = Tk_stride;
+    s.heads = Hq; s.kv_heads = Hkv; s.kdim = s.vdim = s.vrow = kHeadDim;
+    s.scale = 0.08838834764831845f;                           // 1/sqrt(128)
+    s.M = B * Tq; s.rows_per_slot = Tq; s.mode = mode; s.n_keys = Tk; s.n_slots = B;
+    for (int b = 0; b < B; ++b) s.n_valid[b] = n_valid_host ? n_valid_host[b] : Tk;
+    s.out = out; s.ldo = Hq * kHeadDim; s.out_scale = 1.f;
+    return s;
+}
+
+// room in which launch_attention_rows splits the keys for all rows (0: it has no use for any)
+size_t attention_rows_work_bytes(int B, int Tq, int Tk, int Hq, int Hkv, int mode, const int* n_valid_host) {
+    if (!on_tensor_cores(B, Tq) || Hkv <= 0 || Hq % Hkv) return 0;
+    float* const some = reinterpret_cast<float*>(256);        // (only alignment is looked at)
+    const SplitAttention s = split_rows(some, some, some + 64, some, B, Tq, Tk, Hq, Hkv, Tk, mode, n_valid_host);
+    int keys = 0;
+    for (int b = 0; b < B; ++b) keys += (std::max(split_attention_keys(s, b), 0) + 63) & ~63;
+    return split_attention_work_bytes(s, keys);
+}
+
+cudaError_t launch_attention_rows(const float* q, const float* k, const float* v, float* out, int B, int Tq, int Tk, int Hq,
+                                  int Hkv, int Tk_stride, int mode, const int* n_valid_host, void* work, size_t work_bytes, cudaStream_t st) {
+    if (on_tensor_cores(B, Tq)) {                              // the tensor-core kernel with split fp32 operands
+        SplitAttention s = split_rows(q, k, v, out, B, Tq, Tk, Hq, Hkv, Tk_stride, mode, n_valid_host);
+        s.work = work; s.work_bytes = work ? work_bytes : 0;
         if (split_attention_ok(s)) return launch_split_attention(s, st);
     }
     DelayArg nv{};

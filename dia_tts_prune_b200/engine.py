@@ -550,15 +550,18 @@ def rows_layer_forward(args: "_lib.RowsLayer", work_bytes: int, device: torch.de
 
 
 def attention_rows(q_BTHd: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, Tk: int, mode: int,
-                   n_valid: list[int] | None) -> torch.Tensor:
-    """fp32 attention for T > 1 query rows; ``k_cache`` / ``v_cache`` are ``[B, Hkv, Tmax, 128]``."""
+                   n_valid: list[int] | None, room: bool = True) -> torch.Tensor:
+    """fp32 attention for T > 1 query rows; ``k_cache`` / ``v_cache`` are ``[B, Hkv, Tmax, 128]``.  ``room``: the keys are prepared once for all rows."""
     lib = _lib.load()
     B, Tq, Hq, d = q_BTHd.shape
     assert d == 128 and k_cache.shape[0] == B and k_cache.is_contiguous() and v_cache.is_contiguous()
     out = torch.empty_like(q_BTHd)
     nv = (C.c_int32 * B)(*[int(x) for x in n_valid]) if n_valid is not None else None
-    _lib.check(lib.dia_b200_attention_rows(_ptr(q_BTHd), _ptr(k_cache), _ptr(v_cache), _ptr(out), B, Tq, int(Tk), Hq,
-                                           k_cache.shape[1], k_cache.shape[2], int(mode), nv, _stream(q_BTHd.device)),
+    need = int(lib.dia_b200_attention_rows_work_bytes(B, Tq, int(Tk), Hq, k_cache.shape[1], int(mode), nv)) if room else 0
+    work = torch.empty((need,), dtype=torch.uint8, device=q_BTHd.device)
+    _lib.check(lib.dia_b200_attention_rows_in(_ptr(q_BTHd), _ptr(k_cache), _ptr(v_cache), _ptr(out), B, Tq, int(Tk), Hq,
+                                              k_cache.shape[1], k_cache.shape[2], int(mode), nv, work.data_ptr() if need else None, need,
+                                              _stream(q_BTHd.device)),
                "attention_rows")
     return out
 

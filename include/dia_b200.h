@@ -291,6 +291,11 @@ int dia_b200_rows_layer_forward(const dia_b200_rows_layer *a, void *stream);
  * n_valid_host: int32 [B] in HOST memory (may be NULL = Tk).  B <= 16. */
 int dia_b200_attention_rows(const float *q, const float *k, const float *v, float *out, int B, int Tq, int Tk, int Hq,
                             int Hkv, int Tk_stride, int mode, const int32_t *n_valid_host, void *stream);
+/* The same with room in device memory, where the keys and values are prepared once for all queries (without it every 128 rows prepare them for
+ * themselves, several times as long): dia_b200_attention_rows_work_bytes of these sizes, 0 where it has no use for any; 16-byte aligned. */
+size_t dia_b200_attention_rows_work_bytes(int B, int Tq, int Tk, int Hq, int Hkv, int mode, const int32_t *n_valid_host);
+int dia_b200_attention_rows_in(const float *q, const float *k, const float *v, float *out, int B, int Tq, int Tk, int Hq,
+                               int Hkv, int Tk_stride, int mode, const int32_t *n_valid_host, void *work, size_t work_bytes, void *stream);
 /* RotaryEmbedding (dia/layers.py:108-173) on projected heads src float32 [B*T][H*128] with positions pos int32 [B*T]
  * (device) looked up in host-made sin/cos tables float32 [n_pos][64] (device; the reference's CPU values, bit for bit),
  * fused with the layout change: to_cache = 0 writes dst in the source layout (may alias src), to_cache = 1 writes

@@ -131,3 +131,36 @@ def test_row_modes(mode, B, Tq, Tk, Hq, Hkv, n_valid):
         w = torch.nan_to_num(torch.softmax(s, -1), nan=0.0)
         ref = torch.einsum("hij,hjd->ihd", w, v[b].double().repeat_interleave(Hq // Hkv, 0))
         assert (got[b] - ref).abs().max() <= 2e-5 * max(1.0, ref.abs().max())
+
+
+@pytest.mark.parametrize("mode,B,Tq,Tk,Hq,Hkv,n_valid", [(0, 2, 192, 192, 4, 1, None), (1, 2, 200, 200, 2, 2, [37, 200]), (1, 1, 256, 256, 3, 3, [0]),
+                                                         (2, 3, 257, 130, 4, 2, [0, 129, 64]), (0, 1, 1000, 1000, 4, 2, None)])
+def test_row_modes_have_the_same_bits_with_keys_split_in_advance(mode, B, Tq, Tk, Hq, Hkv, n_valid):
+    """Keys that a launch in front splits, and keys that every row tile splits for itself: the same terms and scales"""
+    from dia_tts_prune_b200 import engine as E
+    g = torch.Generator().manual_seed(Tq + Tk)
+    q, k, v = (torch.randn(s, generator=g).cuda() for s in ((B, Tq, Hq, 128), (B, Hkv, Tk, 128), (B, Hkv, Tk, 128)))
+    assert torch.equal(E.attention_rows(q, k, v, Tk, mode, n_valid), E.attention_rows(q, k, v, Tk, mode, n_valid, room=False))
+
+
+@pytest.mark.parametrize("H,G,d,window", [(2, 1, 16, 0), (4, 1, 256, 400)])
+def test_keys_beyond_the_room(H, G, d, window):
+    """A sequence with more keys than the room for split keys holds (twice 64 rows, 32768 and 192 keys): the last tiles are split by the row tiles"""
+    from dia_tts_prune_b200 import synthetic as SY
+    from dia_tts_prune_b200.lm_config import PubopelConfig
+    from dia_tts_prune_b200.lm_model import CausalLM
+    past, rows, step = 33408, 40, 64
+    cfg = SY.pubopel_config(width=32, layers=1, heads=H, kv_heads=G, dim=d, experts=1, top=1, expert_ff=8, shared_ff=None, vocab=64, window=window or None,
+                            keep_first=0, softcap=None)
+    w = SY.pubopel_weights(cfg, 3)
+    model = CausalLM(PubopelConfig.model_validate(cfg), w, dtype="bfloat16", device="cuda:0", max_tokens=33600, max_sequences=1, page_size=64, max_rows=step)
+    p = {n: w[f"l0.mix.{t}"].double() for n, t in (("q", "q.norm"), ("k", "k.norm"), ("temp", "temp"), ("sink", "sink"))}
+    x = torch.randn((past + rows, (H + G) * d), generator=torch.Generator().manual_seed(5))
+    seq = model.state.open("a")
+    model.state.reserve(seq, past + rows)
+    dev = x.cuda()
+    for a in range(0, past, step):
+        model.engine.op_attention(0, dev[a:a + step].clone(), [(seq, step, a)])
+    got = model.engine.op_attention(0, dev[past:].clone(), [(seq, rows, past)])
+    ref = sink_reference(x.double(), past, H, G, d, p, window, 0, 0.0, cfg["norm"]["eps"])
+    close(got, ref, ref.abs().max().item())
