@@ -149,7 +149,7 @@ struct lm_b200_engine {
     void *catb, *outcatb;
     // the stream layer form: the streams [rows][s][width], query latents (bf16 operand), queries carried into the latent
     // space, attended latents / raw read-outs, normaliser floors, and two constants {0, 1}
-    float *xs, *qlat, *olat, *floorb, *unit;
+    float *xs, *qlat, *olat, *floorb, *unit, *delta_room;
     void* cqb;
     // records whose sublayers read the same streams: the mixer's output beside the feed-forward's, and the feed-forward's input
     float *ymix, *h2;
@@ -780,8 +780,14 @@ int stream_mixer_kernels(lm_b200_engine* e, const lm_b200_layer& l, const MixPla
         LCK(lm::launch_delta_prep(proj, ld, c.beta, d, l.conv_tail, v.rm, e->rec, ldr, M, st, c.a));
         LCK(lm::launch_conv_tail(proj, ld, v0 + nv, l.conv_taps, l.conv_tail, v.sm, n_seq, st));
         const lm::ScanInputs si{0, k0, d0, v0, b0};
-        LCK(lm::launch_column_scan(e->rec, ldr, si, lm::kScanDelta, H, l.kv_heads, l.dim, l.vdim, l.rec_state, v.sm, v.rm, n_seq, at.out, at.ldo, st,
-                                   true, M <= lm::kRowsKernelMax));
+        // long portions in chunks; a step of one sequence is either, one of several may have both kinds
+        const bool early = M <= lm::kRowsKernelMax;
+        const bool chunks = M - n_seq + 1 >= lm::kChunkTokensMin && e->delta_room && lm::delta_chunks_ok(e->rec, ldr, si, H, l.kv_heads, l.dim, l.vdim, l.rec_state);
+        if (chunks)
+            LCK(lm::launch_delta_chunks(e->rec, ldr, si, H, l.kv_heads, l.dim, l.vdim, l.rec_state, v.sm, v.rm, n_seq, M, at.out, at.ldo, e->delta_room, st, early));
+        if (!chunks || n_seq > 1)
+            LCK(lm::launch_column_scan(e->rec, ldr, si, lm::kScanDelta, H, l.kv_heads, l.dim, l.vdim, l.rec_state, v.sm, v.rm, n_seq, at.out, at.ldo, st,
+                                       true, early, nullptr, 0, 1.f, chunks));
         LCK(lm::launch_head_norm_gate(at.out, at.ldo, at.out_b, l.head_norm, gate, ld, H, l.vdim, e->m.eps, M, st, gate_act, at.scale));
     } else if (l.mixer == LM_B200_MIXER_RETENTION) {
         // q and k (adjacent in the row) turn in place, k also takes dim^-1/2; decay fixed per head, no write gate, no normaliser
@@ -1022,7 +1028,7 @@ int lm_b200_engine_create(const lm_b200_model* model, const lm_b200_layer* layer
     (void)dia::split_attention_ran_out(device, nullptr);      // (before a step is captured)
     const size_t R = (size_t)m.max_rows, D = (size_t)m.width;
     size_t qk = 0, att = 0, E = 1, top = 1, F = 1, Sf = 1, slots = 1;
-    size_t n_in = 0, k_out = 0, n_rec = 0, split_dim = 0, kv_split = 0;
+    size_t n_in = 0, k_out = 0, n_rec = 0, split_dim = 0, kv_split = 0, delta = 0;
     // room for the split keys and values of twice a step's rows and 32768 cached keys more, as far as sequences can have them (and a partly filled
     // tile at either end of every sequence); what does not fit is split where it is used, by few registers
     const long long cached = std::min<long long>(32768, (long long)m.n_slots * m.max_pages * m.page_size);
@@ -1048,6 +1054,7 @@ int lm_b200_engine_create(const lm_b200_model* model, const lm_b200_layer* layer
             for (int q = 0; q < n_parts(l); ++q) {
                 const lm_b200_layer& p = part_of(l, q);
                 n_heads = std::max(n_heads, (size_t)p.heads);
+                if (p.mixer == LM_B200_MIXER_GATED_DELTA) delta = std::max(delta, lm::delta_room_floats(R, (size_t)m.n_slots, (size_t)p.heads) * 4);
                 if (p.mixer == LM_B200_MIXER_LATENT_ATTENTION) {
                     qk = std::max(qk, (size_t)p.heads * (p.dim + p.rot_dim));
                     n_lat = std::max(n_lat, (size_t)p.heads * (p.kv_rank + p.rot_dim));
@@ -1112,7 +1119,7 @@ int lm_b200_engine_create(const lm_b200_model* model, const lm_b200_layer* layer
     const size_t o_x0 = take(pre ? R * D * 4 : 0), o_cat = take(pre ? R * 2 * D * 4 : 0), o_proj = take(R * n_in * 4),
                  o_rec = take(R * n_rec * 4), o_outcat = take(R * k_out * 4);
     const size_t o_xs = take(R * n_streams * D * 4), o_qlat = take(std::max(R * n_lat * 4, qlat_room)), o_olat = take(std::max(R * n_lat * 4, olat_room)),
-                 o_floor = take(R * n_heads * 4), o_unit = take(2 * 4);
+                 o_floor = take(R * n_heads * 4), o_unit = take(2 * 4), o_delta = take(delta);
     const size_t o_ymix = take(any_parallel ? R * D * 4 : 0), o_h2 = take(any_parallel ? R * D * 4 : 0);
     const size_t o_split = take((size_t)lm::kAttnRowsKernelMax * lm::kAttnSplitsMax * split_dim * 4);
     const size_t o_sidez = take(R * n_side * 4), o_sideg = take(R * n_side * 4);
@@ -1151,7 +1158,7 @@ int lm_b200_engine_create(const lm_b200_model* model, const lm_b200_layer* layer
     e->x0 = (float*)(b + o_x0); e->cat = (float*)(b + o_cat); e->proj = (float*)(b + o_proj); e->rec = (float*)(b + o_rec);
     e->outcat = (float*)(b + o_outcat); e->catb = b + o_catb; e->outcatb = b + o_outcatb;
     e->xs = (float*)(b + o_xs); e->qlat = (float*)(b + o_qlat); e->olat = (float*)(b + o_olat); e->floorb = (float*)(b + o_floor);
-    e->unit = (float*)(b + o_unit); e->cqb = b + o_cqb;
+    e->unit = (float*)(b + o_unit); e->delta_room = delta ? (float*)(b + o_delta) : nullptr; e->cqb = b + o_cqb;
     e->ymix = (float*)(b + o_ymix); e->h2 = (float*)(b + o_h2); e->h2b = b + o_h2b;
     e->side_z = (float*)(b + o_sidez); e->side_g = (float*)(b + o_sideg); e->side_gb = b + o_sidegb;
     e->split_ws = (float*)(b + o_split);

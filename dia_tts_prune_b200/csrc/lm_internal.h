@@ -152,7 +152,16 @@ constexpr int kScanTied = 0, kScanDelta = 1, kScanWrite = 2;
 cudaError_t launch_column_scan(const float* in, int ld, const ScanInputs& si, int rule, int H, int G, int dim, int vdim,
                                float* state, const SeqMeta& sm, const RowMeta& rm, int n_seq, float* o, int ldo,
                                cudaStream_t st, bool head_decay = false, bool early = true, const float* decay = nullptr, int ldd = 0,
-                               float q_mul = 1.f);
+                               float q_mul = 1.f, bool few = false);
+// The delta rule with one decay per head in chunks of kDeltaChunk tokens (lm_delta.cu), for the sequences of at least kChunkTokensMin tokens in a step; the
+// others are left to the scan above (few: its sequences of that many tokens are left out).  room: delta_room_floats(M, n_seq, H) floats, 16-byte aligned.
+// kChunkTokensMin: where chunks are the shorter way in any step (us of a layer of 16 heads of 128, serial / chunks: one prompt of 96 tokens 82 / 84, 160 97 / 93, 250 118 /
+// 106; beside three short prompts one of 200 82 / 87: a step with both kinds launches both).
+constexpr int kDeltaChunk = 32, kDeltaChunkFloats = 2 * kDeltaChunk * kDeltaChunk + 2 * kDeltaChunk, kChunkTokensMin = 320;
+inline size_t delta_room_floats(size_t M, size_t n_seq, size_t H) { return (M / kDeltaChunk + n_seq) * H * kDeltaChunkFloats; }
+bool delta_chunks_ok(const float* in, int ld, const ScanInputs& si, int H, int G, int dim, int vdim, const float* state);
+cudaError_t launch_delta_chunks(const float* in, int ld, const ScanInputs& si, int H, int G, int dim, int vdim, float* state, const SeqMeta& sm,
+                                const RowMeta& rm, int n_seq, int M, float* o, int ldo, float* room, cudaStream_t st, bool early, float q_mul = 1.f);
 // the same scan with scalar gates per (row, head): S <- a S + (b k) v^T and one more value column that is the constant 1
 // (the normaliser n <- a n + b k, read out as n . q), so state and read-out have vdim + 1 columns per head.  a and b are
 // columns a_off + h and beta_off + h of the input rows.  fixed_decay [H]: a = fixed_decay[h], b = 1 for every token instead.

@@ -662,6 +662,73 @@ delta_prep_kernel(const float* __restrict__ proj, int ld, int beta_off, int H, i
     for (int h = tid; h < H; h += blockDim.x) dst[b0 + h] = sigmoidf_(row[beta_off + h]);
 }
 
+// The same for kPrepRows rows of a step, four taps and one decay per head: a thread keeps its channel's weights and last three inputs while it walks the rows,
+// so that an input is read once and not by four rows.  Same operations per channel.  2275 rows of 3072 channels: 61 us by the kernel above, which reads every
+// input four times and its weights for every row, 38 here (28 MB in, 28 MB out).
+constexpr int kPrepRows = 4;
+__global__ void __launch_bounds__(256)
+delta_prep_rows_kernel(const float* __restrict__ proj, int ld, int beta_off, int H, int G, int dim, int vdim, const float* __restrict__ cw,
+                       const float* __restrict__ tail, const float* __restrict__ a_log, const float* __restrict__ dt_bias, float unit_eps,
+                       const int* __restrict__ row_slot, const int* __restrict__ row_pos, const int* __restrict__ row_start, float* __restrict__ rec,
+                       int ldr, int decay_off, int M) {
+    extern __shared__ float cbuf[];                           // [kPrepRows][2 G dim] convolved + silu queries and keys
+    pdl_release();
+    pdl_wait();
+    const int r0 = blockIdx.x * kPrepRows, n = min(kPrepRows, M - r0), tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarp = blockDim.x >> 5;
+    const int nqk = 2 * G * dim, C = nqk + H * vdim;
+    for (int c = tid; c < C; c += blockDim.x) {
+        const float4 w = *reinterpret_cast<const float4*>(cw + 4 * (size_t)c);       // (w.w: of the row's own input)
+        float u1 = 0.f, u2 = 0.f, u3 = 0.f;                   // inputs one to three positions before
+        int before = -1;                                      // the position whose inputs they are, of slot `whose`
+        int whose = -1;
+        for (int i = 0; i < n; ++i) {
+            const int r = r0 + i, slot = row_slot[r], pos = row_pos[r];
+            const float u = proj[(size_t)r * ld + c];
+            if (whose != slot || before != pos) {
+                const int start = row_start[r];
+                auto at = [&](int o) {
+                    const int p = pos - o;
+                    return p < 0 ? 0.f : p >= start ? proj[(size_t)(r - o) * ld + c] : tail[((size_t)slot * 3 + (p - (start - 3))) * C + c];
+                };
+                u1 = at(1);
+                u2 = at(2);
+                u3 = at(3);
+            }
+            float acc = fmaf(w.w, u, 0.f);
+            if (pos > 0) acc = fmaf(w.z, u1, acc);
+            if (pos > 1) acc = fmaf(w.y, u2, acc);
+            if (pos > 2) acc = fmaf(w.x, u3, acc);
+            u3 = u2;
+            u2 = u1;
+            u1 = u;
+            whose = slot;
+            before = pos + 1;
+            const float y = siluf_(acc);
+            if (c < nqk) cbuf[i * nqk + c] = y;
+            else rec[(size_t)r * ldr + c] = y;
+        }
+    }
+    __syncthreads();
+    const float qmul = 1.0f / sqrtf((float)dim);
+    for (int e = warp; e < n * 2 * G; e += nwarp) {           // q heads, then k heads of every row
+        const int i = e / (2 * G), hh = e - i * 2 * G;
+        const float* src = cbuf + i * nqk + hh * dim;
+        float* dst = rec + (size_t)(r0 + i) * ldr + hh * dim;
+        float ss = 0.f;
+        for (int c = lane; c < dim; c += 32) ss = fmaf(src[c], src[c], ss);
+        ss = warp_sum(ss);
+        const float inv = (hh < G ? qmul : 1.f) / sqrtf(ss + unit_eps);
+        for (int c = lane; c < dim; c += 32) dst[c] = src[c] * inv;
+    }
+    for (int e = tid; e < n * H; e += blockDim.x) {           // rec row: q | k | v | decay (H) | beta (H)
+        const int i = e / H, h = e - i * H;
+        const float* row = proj + (size_t)(r0 + i) * ld;
+        float* dst = rec + (size_t)(r0 + i) * ldr + C;
+        dst[h] = expf(-expf(a_log[h]) * softplusf_(row[decay_off + h] + dt_bias[h]));
+        dst[H + h] = sigmoidf_(row[beta_off + h]);
+    }
+}
+
 // tail[slot][i][c] <- projected input at position (start + count) - (taps-1) + i of every scheduled sequence: from this
 // step's rows when that position is in the step, else the old tail shifted by `count`
 __global__ void conv_tail_kernel(const float* __restrict__ proj, int ld, int C, int taps, float* __restrict__ tail,
@@ -856,6 +923,11 @@ cudaError_t launch_delta_prep(const float* proj, int ld, int beta_off, const Del
                               float* rec, int ldr, int M, cudaStream_t st, int head_decay_off) {
     if (d.taps < 1 || d.taps > kMaxTaps) return cudaErrorNotSupported;
     const int C = 2 * d.kv_heads * d.dim + d.heads * d.vdim;
+    // (from as many rows on as leave the blocks of four rows an SM each)
+    const size_t rows_smem = (size_t)kPrepRows * 2 * d.kv_heads * d.dim * 4;
+    if (head_decay_off >= 0 && d.taps == 4 && M >= kPrepRows * 148 && rows_smem <= 48 * 1024 && (reinterpret_cast<uintptr_t>(d.conv_w) & 15) == 0)
+        return launch_pdl(delta_prep_rows_kernel, dim3((M + kPrepRows - 1) / kPrepRows), dim3(256), rows_smem, st, proj, ld, beta_off, d.heads, d.kv_heads,
+                          d.dim, d.vdim, d.conv_w, tail, d.a_log, d.dt_bias, d.unit_eps, rm.slot, rm.pos, rm.start, rec, ldr, head_decay_off, M);
     const size_t smem = (size_t)C * 4;
     if (smem > 48 * 1024) {
         cudaError_t e = cudaFuncSetAttribute(delta_prep_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);

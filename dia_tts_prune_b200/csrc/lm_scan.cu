@@ -76,6 +76,7 @@ struct ScanArgs {
     const int *seq_slot, *seq_row0, *seq_count, *row_pos;
     float* o; int ldo;
     int vec_qk, vec_a;                                        // whether 16-byte pieces are aligned
+    int fewer_than;                                           // sequences with more tokens are somebody else's
 };
 
 // DP: dim padded to a multiple of 32 (a power of two); VA: one decay per key channel
@@ -92,6 +93,7 @@ state_scan_kernel(const ScanArgs p) {
     const int s = blockIdx.x, h = blockIdx.y, col0 = blockIdx.z * VC, g = h / (p.H / p.G);
     const int tid = threadIdx.x, lane = tid & 31, part = lane & (P - 1), cb = (tid >> 5) * CW + lane / P * 2;   // first column in the CTA
     const int slot = p.seq_slot[s], row0 = p.seq_row0[s], n = p.seq_count[s], start = p.row_pos[row0];
+    if (n >= p.fewer_than) return;
     const float a_fix = p.fixed_decay ? p.fixed_decay[h] : 0.f, sd = p.skip ? p.skip[h] : 0.f;
     const bool vec_state = p.dim % 4 == 0;
 
@@ -350,12 +352,12 @@ bool aligned16(const float* base, int ld, int off, int dim) {
 
 cudaError_t launch_column_scan(const float* in, int ld, const ScanInputs& si, int rule, int H, int G, int dim, int vdim, float* state,
                                const SeqMeta& sm, const RowMeta& rm, int n_seq, float* o, int ldo, cudaStream_t st, bool head_decay,
-                               bool early, const float* decay, int ldd, float q_mul) {
+                               bool early, const float* decay, int ldd, float q_mul, bool few) {
     if (G <= 0 || H <= 0) return cudaErrorInvalidValue;
     const float* a = decay ? decay : in + si.a_off;
     const int lda = decay ? ldd : ld;
     ScanArgs p{in, ld, si.q_off, si.k_off, si.v_off, rule == kScanDelta ? si.beta_off : -1, a, lda, nullptr, nullptr, q_mul, H, G, dim, vdim,
-               vdim, state, sm.slot, sm.row0, sm.count, rm.pos, o, ldo, 0, 0};
+               vdim, state, sm.slot, sm.row0, sm.count, rm.pos, o, ldo, 0, 0, few ? kChunkTokensMin : 0x7fffffff};
     p.vec_qk = aligned16(in, ld, si.q_off, dim) && (rule == kScanTied || aligned16(in, ld, si.k_off, dim));
     p.vec_a = aligned16(a, lda, 0, dim);
     switch (rule) {
@@ -372,7 +374,7 @@ cudaError_t launch_scalar_gate_scan(const float* in, int ld, const ScanInputs& s
                                     const float* fixed_decay, bool normaliser, bool early, int G, const float* skip) {
     if (G <= 0) G = H;
     ScanArgs p{in, ld, si.q_off, si.k_off, si.v_off, fixed_decay ? -1 : si.beta_off, in + si.a_off, ld, fixed_decay, skip, 1.f, H, G, dim, vdim,
-               vdim + (normaliser ? 1 : 0), state, sm.slot, sm.row0, sm.count, rm.pos, o, ldo, 0, 0};
+               vdim + (normaliser ? 1 : 0), state, sm.slot, sm.row0, sm.count, rm.pos, o, ldo, 0, 0, 0x7fffffff};
     p.vec_qk = aligned16(in, ld, si.q_off, dim) && aligned16(in, ld, si.k_off, dim);
     return launch_scan<kScanWrite, false>(p, n_seq, early, st);
 }
