@@ -315,6 +315,50 @@ linear_rows_kernel(const float* __restrict__ A, int lda, const __nv_bfloat16* __
     }
 }
 
+// The same for many rows and few outputs (router logits): a warp has two rows and eight outputs at a time, so that a row is read once and not once per
+// output.  Same order of operations.  4096 rows of 2048 channels, 8 outputs: 41 us by the kernel above, 17 here (34 MB: 5 at the copy rate).
+constexpr int kNarrowRows = 2;
+__global__ void __launch_bounds__(256)
+linear_narrow_kernel(const float* __restrict__ A, int lda, const __nv_bfloat16* __restrict__ W, float* __restrict__ Y, int ldy, int M, int N, int K) {
+    pdl_release();
+    pdl_wait();
+    const int lane = threadIdx.x & 31, r0 = (blockIdx.x * 8 + (threadIdx.x >> 5)) * kNarrowRows;
+    if (r0 >= M) return;
+    const float* row[kNarrowRows];
+#pragma unroll
+    for (int r = 0; r < kNarrowRows; ++r) row[r] = A + (size_t)min(r0 + r, M - 1) * lda;
+    for (int n0 = 0; n0 < N; n0 += 8) {
+        float acc[kNarrowRows][8] = {};
+#pragma unroll 2
+        for (int k = lane * 8; k < K; k += 256) {
+            float x[kNarrowRows][8];
+#pragma unroll
+            for (int r = 0; r < kNarrowRows; ++r) {
+                *reinterpret_cast<float4*>(x[r]) = *reinterpret_cast<const float4*>(row[r] + k);
+                *reinterpret_cast<float4*>(x[r] + 4) = *reinterpret_cast<const float4*>(row[r] + k + 4);
+            }
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const uint4 wv = *reinterpret_cast<const uint4*>(W + (size_t)min(n0 + j, N - 1) * K + k);
+                const __nv_bfloat162* p = reinterpret_cast<const __nv_bfloat162*>(&wv);
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const float lo = __low2float(p[e]), hi = __high2float(p[e]);
+#pragma unroll
+                    for (int r = 0; r < kNarrowRows; ++r) acc[r][j] = fmaf(x[r][2 * e + 1], hi, fmaf(x[r][2 * e], lo, acc[r][j]));
+                }
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < kNarrowRows; ++r)
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const float y = warp_sum(acc[r][j]);
+                if (lane == 0 && r0 + r < M && n0 + j < N) Y[(size_t)(r0 + r) * ldy + n0 + j] = y;
+            }
+    }
+}
+
 // mid[a][n] = act(A_a . Wg_e[n], A_a . Wu_e[n]) (glu_act),  W_e = [gate rows (F) | up rows
 // (F)][K].  blockIdx.y < n_assign: the
 // assignment slot a of the routed experts (row, expert and score from the maps); beyond: row blockIdx.y - n_assign through
@@ -1224,6 +1268,13 @@ cudaError_t launch_tapmix_tail(const float* x, const NormW& n, int taps, float* 
     return cudaGetLastError();
 }
 
+namespace {
+constexpr int kNarrowRowsMin = 1024;                           // rows from which two to a warp fill the SMs
+bool vectors_ok(const float* A, int lda, const void* W, int K) {
+    return K % 8 == 0 && lda % 4 == 0 && ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(W)) & 15) == 0;
+}
+}  // namespace
+
 cudaError_t launch_linear(const float* A, int lda, const void* W, long long w_expert_stride, float* Y, int ldy, int M, int N,
                           int K, const GroupMap* gm, cudaStream_t st, int act) {
     if (act == kActXielu) return cudaErrorNotSupported;       // (its two numbers are not handed in here)
@@ -1232,7 +1283,9 @@ cudaError_t launch_linear(const float* A, int lda, const void* W, long long w_ex
     const int* a_expert = gm ? gm->a_expert : nullptr;
     const int* n_slots = gm ? gm->n_slots : nullptr;
     const __nv_bfloat16* w = reinterpret_cast<const __nv_bfloat16*>(W);
-    // a few rows, or a few outputs (router logits: the same kernel for every step length, so that the choice of experts
+    if (!gm && act == kActNone && N <= kRowsKernelMaxOut && M >= kNarrowRowsMin && vectors_ok(A, lda, w, K))
+        return launch_pdl(linear_narrow_kernel, dim3((M + 8 * kNarrowRows - 1) / (8 * kNarrowRows)), dim3(256), 0, st, A, lda, w, Y, ldy, M, N, K);
+    // a few rows, or a few outputs (router logits: the same order of operations for every step length, so that the choice of experts
     // does not depend on how a prompt was cut)
     if (M <= kRowsKernelMax || (N <= kRowsKernelMaxOut && M <= 65535))
         return launch_pdl(linear_rows_kernel, dim3((N + 7) / 8, M), dim3(256), 0, st, A, lda, w, w_expert_stride, Y, ldy, M, N, K,
