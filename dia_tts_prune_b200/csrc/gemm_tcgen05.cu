@@ -497,11 +497,11 @@ dia_gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_
 // for: over Dia's widths and 130 to 3000 rows (normal, gated, positive numbers) 5.8e-7 to 9.0e-7 against 3.5e-6 to 4.0e-5, and 1.2e-6 against 3.5e-6
 // in columns that see only the other numbers of rows with one 2^20 times as large.  Chunks of 1, 2 and 4 k-blocks: 282, 215 and 162 us, 1.5e-7, 2.9e-7 and 5.8e-7 (the
 // accumulators of a chunk are read while the MMAs update the others, and the two slow each other down).
-template <bool SUMS>
+template <bool SUMS, bool GLU = false>
 struct Pair {
-    static constexpr int kFirst = SUMS ? 4 : 2, kWarps = SUMS ? 8 : 4, kThreads = 32 * (kFirst + kWarps);  // (registers go by groups of 4 warps)
+    static constexpr int kFirst = SUMS ? 4 : 2, kWarps = SUMS || GLU ? 8 : 4, kThreads = 32 * (kFirst + kWarps);  // (registers go by groups of 4 warps)
     static constexpr int kSumRegs = 208, kFewRegs = 88, kRegs = (kSumRegs * 8 + kFewRegs * 4) / 12;        // 168 a thread at launch
-    static constexpr int kSlots = SUMS ? 12 : 13;                                                          // ring, and 32 x 32 blocks to turn
+    static constexpr int kSlots = SUMS || GLU ? 12 : 13;                                                          // ring, and 32 x 32 blocks to turn
     static constexpr int kSmem = kSlots * kTileBytes + kWarps * 4096 + 1024 + 256;
 };
 constexpr int kPairStagesMost = 8, kPairChunk = 4;
@@ -516,8 +516,20 @@ struct PairProduct {
     const int* row_group; int group_rows; const int* n_rows;
     int* ran_out;
     const float* row_inv; const float* col_mag;              // SUMS: inverse scales of the rows, largest magnitudes of the columns
+    int glu; float glu_limit;                                 // GLU: the gate's form (see glu_value)
     unsigned polls;                                           // looks at a barrier until a wait has run out
 };
+
+// the activation of a gated unit on its gate g and up u products, as the kernel that runs by itself has it: 0 silu(g) u, 1 clamped, 2 gelu(g) u
+__device__ __forceinline__ float glu_value(int kind, float g, float u, float limit) {
+    if (kind == 1) {
+        g = fminf(g, limit);
+        u = fminf(fmaxf(u, -limit), limit);
+        return g * (1.0f / (1.0f + expf(-(1.702f * g)))) * (u + 1.0f);
+    }
+    if (kind == 2) return 0.5f * g * (1.0f + tanhf(0.7978845608028654f * fmaf(0.044715f * g * g, g, g))) * u;
+    return g / (1.0f + expf(-g)) * u;
+}
 
 // How often a wait of the pair kernel looks at its barrier, in products that this thread launches.  With 0 each wait runs out before anything has
 // been issued, which is how a test sees what then becomes of the outputs.
@@ -564,11 +576,13 @@ __device__ __forceinline__ void cluster_sync_all() {
 }
 
 // NaN for rows [row0, row0 + rows) and columns [c0, c1) of a product that has no result (a multiple of 4 columns)
+template <bool GLU>
 __device__ __noinline__ void pair_no_result(const PairProduct& p, int row0, int rows, int c0, int c1, int lane) {
+    const int N = GLU ? p.N >> 1 : p.N;
     const uint32_t nan = 0x7fffffffu, two = 0x7fff7fffu;      // (as fp32 and as two bf16)
     for (int r = 0; r < rows; ++r)
         for (int n = c0 + 4 * lane; n < c1; n += 128) {
-            const size_t at = (size_t)(row0 + r) * p.N + n;
+            const size_t at = (size_t)(row0 + r) * N + n;
             if (p.y_bf16) *reinterpret_cast<uint2*>(p.y_bf16 + at) = make_uint2(two, two);
             else *reinterpret_cast<uint4*>(p.y + at) = make_uint4(nan, nan, nan, nan);
         }
@@ -579,13 +593,26 @@ __device__ __forceinline__ float column_inverse(float magnitude) {
     return __uint_as_float((uint32_t)max((int)(__float_as_uint(magnitude) >> 23) - 14, 0) << 23);
 }
 
-template <int TERMS, bool SUMS>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Pair<SUMS>::kThreads, 1)
+__device__ __forceinline__ void tmem_columns16(uint32_t addr, uint32_t (&v)[16]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]),
+          "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+        : "r"(addr)
+        : "memory");
+}
+
+// GLU: the weights' rows are [gate (N / 2) | up (N / 2)], and a tile is 128 columns of either: the leader's half of the weight tile holds gate rows, the other's
+// the up rows of the same columns, so that each CTA's accumulator has both for its rows.  Eight warps take them, apply the gate and write the bf16 operand of the
+// product that follows: 268 MB of fp32 products that another kernel read again stay on the chip (4096 rows, two of eight experts of 2048 and a shared one of
+// 4096, width 2048: products and gates 397 us apart, 349 together; with four warps the exponentials and divisions took longer than a tile's MMAs).
+template <int TERMS, bool SUMS, bool GLU = false>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Pair<SUMS, GLU>::kThreads, 1)
 dia_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const __grid_constant__ PairProduct p) {
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-    unsigned char* turn = smem + Pair<SUMS>::kSlots * kTileBytes;
-    uint64_t* full = reinterpret_cast<uint64_t*>(turn + Pair<SUMS>::kWarps * 4096);      // (the leader's alone)
+    unsigned char* turn = smem + Pair<SUMS, GLU>::kSlots * kTileBytes;
+    uint64_t* full = reinterpret_cast<uint64_t*>(turn + Pair<SUMS, GLU>::kWarps * 4096);      // (the leader's alone)
     uint64_t* empty = full + kPairStagesMost;
     uint64_t* t_full = empty + kPairStagesMost;
     uint64_t* t_empty = t_full + 2;                                              // (the leader's alone)
@@ -594,15 +621,15 @@ dia_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t rank = blockIdx.x & 1;
     const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
-    const int BN = p.BN, half = BN >> 1, M = p.M, N = p.N;
+    const int BN = p.BN, half = BN >> 1, M = p.M, N = GLU ? p.N >> 1 : p.N, ON = GLU ? half : BN;       // columns of the result, of a tile of it
     const int n_kb = (p.K + BK - 1) / BK, n_stages = p.stages;
     const int m_lim = p.n_rows ? min(M, *p.n_rows) : M;
-    const int tiles_m = (M + 2 * BM - 1) / (2 * BM), n_tiles = tiles_m * ((N + BN - 1) / BN);
+    const int tiles_m = (M + 2 * BM - 1) / (2 * BM), n_tiles = tiles_m * ((N + ON - 1) / ON);
     const int stage_bytes = TERMS * kTileBytes + half * 128;
 
     if (threadIdx.x == 0) {
         for (int i = 0; i < kPairStagesMost; ++i) { mbar_init(&full[i], 1); mbar_init(&empty[i], 1); }
-        for (int i = 0; i < 2; ++i) { mbar_init(&t_full[i], 1); mbar_init(&t_empty[i], 2 * Pair<SUMS>::kWarps); }
+        for (int i = 0; i < 2; ++i) { mbar_init(&t_full[i], 1); mbar_init(&t_empty[i], 2 * Pair<SUMS, GLU>::kWarps); }
         fence_mbar_init();
     }
     if (warp == 1) {
@@ -614,15 +641,15 @@ dia_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem_base = *tmem_slot;
     bool ok = true;
-    if (warp < Pair<SUMS>::kFirst) {
-        if constexpr (SUMS) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(Pair<SUMS>::kFewRegs));
+    if (warp < Pair<SUMS, GLU>::kFirst) {
+        if constexpr (SUMS) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(Pair<SUMS, GLU>::kFewRegs));
         if (warp == 0) {
             if (lane == 0) {
                 unsigned i = 0;
                 for (int t = pair; t < n_tiles && ok; t += pairs) {
-                    const int n0 = (t / tiles_m) * BN, m0 = (t % tiles_m) * 2 * BM;
+                    const int n0 = (t / tiles_m) * ON, m0 = (t % tiles_m) * 2 * BM;
                     if (m0 >= m_lim) continue;
-                    const int a_row = m0 + (int)rank * BM, b_row = n0 + (int)rank * half + (p.row_group ? p.row_group[m0] * p.group_rows : 0);
+                    const int a_row = m0 + (int)rank * BM, b_row = n0 + (int)rank * (GLU ? N : half) + (p.row_group ? p.row_group[m0] * p.group_rows : 0);
                     for (int kb = 0; kb < n_kb; ++kb, ++i) {
                         const unsigned s = i % n_stages;
                         if (!lane_wait(&empty[s], ((i / n_stages) & 1u) ^ 1u, p.polls)) { ok = false; break; }
@@ -675,13 +702,13 @@ dia_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
             }
         }
     } else if constexpr (SUMS) {
-        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(Pair<SUMS>::kSumRegs));      // (there are as many: see pairs_of)
-        const int q = warp & 3, h0 = ((warp - Pair<SUMS>::kFirst) >> 2) * half;
-        float* const blk = reinterpret_cast<float*>(turn + (warp - Pair<SUMS>::kFirst) * 4096);
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(Pair<SUMS, GLU>::kSumRegs));      // (there are as many: see pairs_of)
+        const int q = warp & 3, h0 = ((warp - Pair<SUMS, GLU>::kFirst) >> 2) * half;
+        float* const blk = reinterpret_cast<float*>(turn + (warp - Pair<SUMS, GLU>::kFirst) * 4096);
         const int rr = lane >> 3, ch = lane & 7;
         unsigned i = 0;
         for (int t = pair; t < n_tiles; t += pairs) {
-            const int n0 = (t / tiles_m) * BN, m0 = (t % tiles_m) * 2 * BM;
+            const int n0 = (t / tiles_m) * ON, m0 = (t % tiles_m) * 2 * BM;
             float sum[128];
 #pragma unroll
             for (int c = 0; c < 128; ++c) sum[c] = 0.f;
@@ -714,7 +741,7 @@ dia_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
             }
             const int row0 = m0 + (int)rank * BM + q * 32, rows = min(32, M - row0);
             if (!ok) {                                        // the sums of this tile lack products, and no later one has any
-                pair_no_result(p, row0, rows, n0 + h0, min(n0 + h0 + half, N), lane);
+                pair_no_result<GLU>(p, row0, rows, n0 + h0, min(n0 + h0 + half, N), lane);
                 continue;
             }
             float ri[8];                                      // (loads ahead of their uses: the output of a tile took 3.2 us with one row after the other)
@@ -757,19 +784,67 @@ dia_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
                 __syncwarp();
             }
         }
-    } else {
-        const int q = warp & 3;
-        float* const blk = reinterpret_cast<float*>(turn + (warp - Pair<SUMS>::kFirst) * 4096);
-        const int rr = lane >> 3, ch = lane & 7;              // a lane's row of four and its 16-byte piece of a 32-column block
+    } else if constexpr (GLU) {
+        const int q = warp & 3, h0 = ((warp - Pair<SUMS, GLU>::kFirst) >> 2) * 64;
+        unsigned char* const blk = turn + (warp - Pair<SUMS, GLU>::kFirst) * 4096;
+        const int rr = lane >> 3, ch = lane & 7;              // a lane's row of four and its 16-byte piece of 64 columns
         unsigned it = 0;
         for (int t = pair; t < n_tiles; t += pairs) {
-            const int n0 = (t / tiles_m) * BN, m0 = (t % tiles_m) * 2 * BM;
+            const int n0 = (t / tiles_m) * ON, m0 = (t % tiles_m) * 2 * BM;
             if (m0 >= m_lim) continue;
             const int row0 = m0 + (int)rank * BM + q * 32, rows = min(32, M - row0);
             const unsigned acc = it & 1u;
             ok = ok && pair_wait(&t_full[acc], (it >> 1) & 1u, p.polls);
             if (!ok) {
-                pair_no_result(p, row0, rows, n0, min(n0 + BN, N), lane);
+                pair_no_result<GLU>(p, row0, rows, n0 + h0, n0 + h0 + 64, lane);
+                continue;
+            }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint32_t from = tmem_base + ((uint32_t)(q * 32) << 16) + acc * 256 + h0;
+#pragma unroll 1
+            for (int cb = 0; cb < 4; ++cb) {
+                uint32_t g[16], u[16];
+                tmem_columns16(from + cb * 16, g);
+                tmem_columns16(from + half + cb * 16, u);
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                uint32_t y[8];
+#pragma unroll
+                for (int e = 0; e < 8; ++e) {
+                    const __nv_bfloat162 b = __floats2bfloat162_rn(glu_value(p.glu, __uint_as_float(g[2 * e]), __uint_as_float(u[2 * e]), p.glu_limit),
+                                                                   glu_value(p.glu, __uint_as_float(g[2 * e + 1]), __uint_as_float(u[2 * e + 1]), p.glu_limit));
+                    y[e] = *reinterpret_cast<const uint32_t*>(&b);
+                }
+                // lane = row: its 16-byte piece c goes to place c ^ (row % 8) of its 128 bytes, and is read a row per eight lanes
+#pragma unroll
+                for (int c = 0; c < 2; ++c)
+                    *reinterpret_cast<uint4*>(blk + lane * 128 + (((2 * cb + c) ^ (lane & 7)) << 4)) = make_uint4(y[4 * c], y[4 * c + 1], y[4 * c + 2], y[4 * c + 3]);
+            }
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0)
+                asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(at_rank(&t_empty[acc], 0)) : "memory");
+            ++it;
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+                const int r = 4 * e + rr;
+                if (r < rows)
+                    *reinterpret_cast<uint4*>(p.y_bf16 + (size_t)(row0 + r) * N + n0 + h0 + 8 * ch) = *reinterpret_cast<const uint4*>(blk + r * 128 + ((ch ^ (r & 7)) << 4));
+            }
+            __syncwarp();
+        }
+    } else {
+        const int q = warp & 3;
+        float* const blk = reinterpret_cast<float*>(turn + (warp - Pair<SUMS, GLU>::kFirst) * 4096);
+        const int rr = lane >> 3, ch = lane & 7;              // a lane's row of four and its 16-byte piece of a 32-column block
+        unsigned it = 0;
+        for (int t = pair; t < n_tiles; t += pairs) {
+            const int n0 = (t / tiles_m) * ON, m0 = (t % tiles_m) * 2 * BM;
+            if (m0 >= m_lim) continue;
+            const int row0 = m0 + (int)rank * BM + q * 32, rows = min(32, M - row0);
+            const unsigned acc = it & 1u;
+            ok = ok && pair_wait(&t_full[acc], (it >> 1) & 1u, p.polls);
+            if (!ok) {
+                pair_no_result<GLU>(p, row0, rows, n0, min(n0 + BN, N), lane);
                 continue;
             }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -1298,27 +1373,27 @@ static bool dense_rows_f32(int terms, int M, int N, int K, int sms);
 static cudaError_t run_gemm_f32(const F32Product& p, const void* a_terms, int terms, int splits, cudaStream_t st);
 
 // clusters of two CTAs of the pair kernel that run at the same time
-template <int TERMS, bool SUMS>
+template <int TERMS, bool SUMS, bool GLU = false>
 static cudaError_t pairs_of(int dev, int* out) {
     static std::atomic<int> known[64];
     if (dev >= 0 && dev < 64 && (*out = known[dev].load(std::memory_order_relaxed)) > 0) return cudaSuccess;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(2);
-    cfg.blockDim = dim3(Pair<SUMS>::kThreads);
-    cfg.dynamicSmemBytes = Pair<SUMS>::kSmem;
+    cfg.blockDim = dim3(Pair<SUMS, GLU>::kThreads);
+    cfg.dynamicSmemBytes = Pair<SUMS, GLU>::kSmem;
     cudaLaunchAttribute attr;
     attr.id = cudaLaunchAttributeClusterDimension;
     attr.val.clusterDim.x = 2;
     attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
-    const auto kernel = dia_gemm_pair_kernel<TERMS, SUMS>;
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Pair<SUMS>::kSmem);
+    const auto kernel = dia_gemm_pair_kernel<TERMS, SUMS, GLU>;
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Pair<SUMS, GLU>::kSmem);
     cudaFuncAttributes built;
     if (e == cudaSuccess) e = cudaFuncGetAttributes(&built, kernel);
     if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(out, kernel, &cfg);
     if (e != cudaSuccess) return e;
-    if (SUMS && built.numRegs < Pair<SUMS>::kRegs) return cudaErrorNotSupported;      // (its roles would wait for registers that are not there)
+    if (SUMS && built.numRegs < Pair<SUMS, GLU>::kRegs) return cudaErrorNotSupported;      // (its roles would wait for registers that are not there)
     if (*out < 1) return cudaErrorNotSupported;
     if (dev >= 0 && dev < 64) known[dev].store(*out, std::memory_order_relaxed);
     return cudaSuccess;
@@ -1337,22 +1412,22 @@ static int pair_columns(int terms, int M, int N, int pairs) {
     }
     return best;
 }
-template <int TERMS, bool SUMS>
+template <int TERMS, bool SUMS, bool GLU = false>
 static cudaError_t run_pair(const CUtensorMap& ma, const void* wt, long long wt_rows, PairProduct& q, int dev, cudaStream_t st) {
     int pairs = 0;
-    cudaError_t e = pairs_of<TERMS, SUMS>(dev, &pairs);
-    const auto kernel = dia_gemm_pair_kernel<TERMS, SUMS>;
-    if (e == cudaSuccess) e = ask_smem<dia_gemm_pair_kernel<TERMS, SUMS>>(dev, Pair<SUMS>::kSmem);
+    cudaError_t e = pairs_of<TERMS, SUMS, GLU>(dev, &pairs);
+    const auto kernel = dia_gemm_pair_kernel<TERMS, SUMS, GLU>;
+    if (e == cudaSuccess) e = ask_smem<dia_gemm_pair_kernel<TERMS, SUMS, GLU>>(dev, Pair<SUMS, GLU>::kSmem);
     if (e != cudaSuccess) return e;
     q.polls = gemm_pair_polls();
     q.ran_out = split_attention_ran_out(dev, st);
     if (take_ran_out(dev, st)) return cudaErrorLaunchTimeout;
-    q.BN = pair_columns(TERMS, q.M, q.N, pairs);
-    q.stages = std::min(kPairStagesMost, Pair<SUMS>::kSlots * kTileBytes / (TERMS * kTileBytes + q.BN / 2 * 128));
+    q.BN = GLU ? 256 : pair_columns(TERMS, q.M, q.N, pairs);
+    q.stages = std::min(kPairStagesMost, Pair<SUMS, GLU>::kSlots * kTileBytes / (TERMS * kTileBytes + q.BN / 2 * 128));
     CUtensorMap mb;
     if (!make_map(&mb, wt, wt_rows, q.K, q.BN / 2)) return cudaErrorNotSupported;
     const int n_tiles = ((q.N + q.BN - 1) / q.BN) * ((q.M + 2 * BM - 1) / (2 * BM));
-    kernel<<<2 * std::min(n_tiles, pairs), Pair<SUMS>::kThreads, Pair<SUMS>::kSmem, st>>>(ma, mb, q);
+    kernel<<<2 * std::min(n_tiles, pairs), Pair<SUMS, GLU>::kThreads, Pair<SUMS, GLU>::kSmem, st>>>(ma, mb, q);
     return cudaGetLastError();
 }
 
@@ -1386,6 +1461,23 @@ cudaError_t launch_gemm_tcgen05_bf16(const void* a_bf16, int terms, const void* 
         reinterpret_cast<__nv_bfloat16*>(ep.y_bf16), groups ? groups->row_group : nullptr,
         groups ? groups->group_rows : 0, groups ? groups->n_rows : nullptr);
     return cudaGetLastError();
+}
+
+cudaError_t launch_gemm_glu_bf16(const void* a_bf16, const void* wt, long long wt_rows, void* y_bf16, int M, int F, int K, int kind, float limit,
+                                 const GemmGroups* groups, cudaStream_t st) {
+    if (M <= BM || F % 128 || F <= 0 || !gemm_tcgen05_shape_ok(M, 2 * F, K) || wt_rows < 2LL * F || kind < 0 || kind > 2 ||
+        (reinterpret_cast<uintptr_t>(y_bf16) & 15) || (groups && groups->tile_rows % (2 * BM)))
+        return cudaErrorNotSupported;
+    int dev = 0, sms = 0;
+    const cudaError_t e = current_sms(&dev, &sms);
+    if (e != cudaSuccess) return e;
+    if (!groups && wt_rows == 2LL * F && dense_rows_f32(1, M, 2 * F, K, sms)) return cudaErrorNotSupported;      // (fp32 sums stay: see there)
+    CUtensorMap ma;
+    if (!make_map(&ma, a_bf16, M, K, BM)) return cudaErrorNotSupported;
+    PairProduct q{};
+    q.M = M; q.N = 2 * F; q.K = K; q.y_bf16 = reinterpret_cast<__nv_bfloat16*>(y_bf16); q.glu = kind; q.glu_limit = limit;
+    if (groups) { q.row_group = groups->row_group; q.group_rows = groups->group_rows; q.n_rows = groups->n_rows; }
+    return run_pair<1, false, true>(ma, wt, wt_rows, q, dev, st);
 }
 
 bool gemm_f32_ok(const F32Product& p) {

@@ -555,6 +555,19 @@ int mixer(lm_b200_engine* e, const lm_b200_layer& l, const float* h, const void*
     return LM_B200_OK;
 }
 
+// y_bf16 [M][F] = the gated unit's activation of [gate | up] = Ab W^T, in the product where it can be, else through gu [M][2 F]
+int glu_product(const void* Ab, const void* w, long long w_rows, float* gu, void* y_bf16, int M, int F, int K, int act, float limit,
+                const dia::GemmGroups* groups, const lm::GroupMap* gm, cudaStream_t st) {
+    const cudaError_t e = dia::launch_gemm_glu_bf16(Ab, w, w_rows, y_bf16, M, F, K, act, limit, groups, st);
+    if (e != cudaErrorNotSupported) {
+        LCK(e);
+        return LM_B200_OK;
+    }
+    LCK(dia::launch_gemm_tcgen05_bf16(Ab, 1, w, w_rows, gu, M, 2 * F, K, kPlain, groups, st));
+    LCK(lm::launch_silu_mul(gu, nullptr, y_bf16, M, F, gm, st, act, limit));
+    return LM_B200_OK;
+}
+
 // x += norm(ff(h)) with a norm, x = ff(h) without.  A few rows: router + top experts + maps, gated products, and the
 // sum over the row's experts with the norm and the residual add, four launches.  Longer steps group the (row, expert)
 // assignments by expert for the tiled products.
@@ -583,9 +596,8 @@ int feed_forward(lm_b200_engine* e, const lm_b200_layer& l, const float* h, cons
     if (tc) {
         LCK(lm::launch_pack_rows_bf16(h, e->packb, bound, D, &gm, st));
         const dia::GemmGroups gu_groups{e->a_expert, 2 * F, e->n_slots, pad}, down_groups{e->a_expert, D, e->n_slots, pad};
-        LCK(dia::launch_gemm_tcgen05_bf16(e->packb, 1, l.w_gate_up, (long long)E * 2 * F, e->gu, bound, 2 * F, D, kPlain,
-                                          &gu_groups, st));
-        LCK(lm::launch_silu_mul(e->gu, nullptr, e->midb, bound, F, &gm, st));
+        const int rc = glu_product(e->packb, l.w_gate_up, (long long)E * 2 * F, e->gu, e->midb, bound, F, D, glu_kind(LM_B200_ACT_SILU_GLU), 0.f, &gu_groups, &gm, st);
+        if (rc) return rc;
         LCK(dia::launch_gemm_tcgen05_bf16(e->midb, 1, l.w_down, (long long)E * D, e->parts, bound, D, F, kPlain, &down_groups, st));
     } else {
         LCK(lm::launch_linear(h, D, l.w_gate_up, 2LL * F * D, e->gu, 2 * F, bound, 2 * F, D, &gm, st));
@@ -600,8 +612,8 @@ int feed_forward(lm_b200_engine* e, const lm_b200_layer& l, const float* h, cons
                 LCK(lm::launch_pack_rows_bf16(h, e->hb, M, D, nullptr, st));
                 hb = e->hb;
             }
-            LCK(dia::launch_gemm_tcgen05_bf16(hb, 1, l.ws_gate_up, 2 * Sf, e->sgu, M, 2 * Sf, D, kPlain, nullptr, st));
-            LCK(lm::launch_silu_mul(e->sgu, nullptr, e->smidb, M, Sf, nullptr, st));
+            const int rc = glu_product(hb, l.ws_gate_up, 2LL * Sf, e->sgu, e->smidb, M, Sf, D, glu_kind(LM_B200_ACT_SILU_GLU), 0.f, nullptr, nullptr, st);
+            if (rc) return rc;
             LCK(dia::launch_gemm_tcgen05_bf16(e->smidb, 1, l.ws_down, D, e->y, M, D, Sf, kPlain, nullptr, st));
         } else {
             LCK(linear_f32(e, h, D, l.ws_gate_up, e->sgu, 2 * Sf, M, 2 * Sf, D, st));
@@ -904,8 +916,8 @@ int gated_unit(lm_b200_engine* e, const lm_b200_layer& l, const float* h, const 
                int F, float limit, float* out, cudaStream_t st) {
     const int D = e->m.width;
     if (hb && tensor_path(e, M, 2 * F, D) && tensor_path(e, M, D, F)) {
-        LCK(dia::launch_gemm_tcgen05_bf16(hb, 1, w_gu, 2 * F, e->sgu, M, 2 * F, D, kPlain, nullptr, st));
-        LCK(lm::launch_silu_mul(e->sgu, nullptr, e->smidb, M, F, nullptr, st, glu_kind(l.act), limit));
+        const int rc = glu_product(hb, w_gu, 2LL * F, e->sgu, e->smidb, M, F, D, glu_kind(l.act), limit, nullptr, nullptr, st);
+        if (rc) return rc;
         LCK(dia::launch_gemm_tcgen05_bf16(e->smidb, 1, w_down, D, out, M, D, F, kPlain, nullptr, st));
         return LM_B200_OK;
     }
@@ -961,9 +973,8 @@ int stream_ff(lm_b200_engine* e, const lm_b200_layer& l, const float* h, const v
     if (tc) {
         LCK(lm::launch_pack_rows_bf16(h, e->packb, bound, D, &gather, st));
         const dia::GemmGroups gu_groups{e->a_expert, 2 * F, e->n_slots, pad}, down_groups{e->a_expert, D, e->n_slots, pad};
-        LCK(dia::launch_gemm_tcgen05_bf16(e->packb, 1, l.w_gate_up, (long long)E * 2 * F, e->gu, bound, 2 * F, D, kPlain,
-                                          &gu_groups, st));
-        LCK(lm::launch_silu_mul(e->gu, nullptr, e->midb, bound, F, &gm, st, act, l.act_limit));
+        const int rc = glu_product(e->packb, l.w_gate_up, (long long)E * 2 * F, e->gu, e->midb, bound, F, D, act, l.act_limit, &gu_groups, &gm, st);
+        if (rc) return rc;
         LCK(dia::launch_gemm_tcgen05_bf16(e->midb, 1, l.w_down, (long long)E * D, e->parts, bound, D, F, kPlain, &down_groups, st));
     } else {
         LCK(lm::launch_linear(h, D, l.w_gate_up, 2LL * F * D, e->gu, 2 * F, bound, 2 * F, D, &gather, st));
