@@ -126,8 +126,8 @@ __device__ __forceinline__ void fence_mbar_init() { asm volatile("fence.mbarrier
 
 // One lane of a converged warp (elect.sync).  Code that issues tcgen05 / TMA instructions for the whole CTA runs with the
 // WHOLE warp in the loop and only the issue under this predicate: the operands (descriptors, TMEM addresses) are then
-// provably warp-uniform and stay in uniform registers.  Behind a `lane == 0` branch the compiler instead wraps every
-// UTCHMMA in an ELECT / 5 x R2UR.BROADCAST / branch "waterfall" (measured: ~170 cycles per MMA instead of ~30).
+// provably the same in every lane, as these instructions need them.  Behind a `lane == 0` branch nothing proves it and an
+// issue measures ~170 cycles per MMA instead of ~30.
 __device__ __forceinline__ uint32_t elect_one_sync() {
     uint32_t pred;
     asm volatile(
