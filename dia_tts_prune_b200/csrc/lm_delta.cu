@@ -18,8 +18,8 @@
 //
 // Bound: the loads from shared memory that feed the multiply-adds (16 bytes for each lane: four cycles an instruction, and 2.7 multiply-adds for each): a
 // chunk of 32 tokens takes a block 6800 cycles by itself and 10000 beside another, where the serial scan takes 24000.  Layer of 16 heads of 128, us, serial
-// scan / chunks: 1024 tokens 323 / 242, 4096 1102 / 767, prompts of 1024, 700, 513, 37 and 1 tokens 569 / 420 (with the blocks in the sequences' order 488;
-// 32 columns a block, which read a third less, 605); 4 heads of 64, 2000 tokens 488 / 255.
+// scan / chunks: 1024 tokens 323 / 245, 4096 1102 / 737, prompts of 1024, 700, 513, 37 and 1 tokens 574 / 390 (407 with the short ones behind the long ones instead
+// of beside them; the blocks in the sequences' order took 68 more, 32 columns a block, which read a third less, 185); 4 heads of 64, 2000 tokens 488 / 256.
 // A column's order of operations depends on its sequence's portion alone.  Sequences of fewer tokens stay with the serial scan.
 #include <algorithm>
 
@@ -195,8 +195,8 @@ delta_columns_kernel(const DeltaArgs p) {
     using M = Columns<DP>;
     constexpr int LD = M::LD, ND = DP / 64, NC = kCols / 8, RP = kColThreads / (DP / 4);      // channel pairs and columns of S per thread, rows per pass of the staging
     extern __shared__ __align__(16) float sh[];
-    pdl_release();
     pdl_wait();
+    pdl_release();                                            // (behind the wait: the scan of the short sequences relies on it)
     // the longest sequences' blocks start first
     __shared__ int s_seq;
     for (int i = threadIdx.x; i < p.n_seq; i += kColThreads) {
@@ -443,7 +443,9 @@ cudaError_t launch_inst(const DeltaArgs& p, int M, bool early, cudaStream_t st) 
     if (e != cudaSuccess) return e;
     // not early: beside the kernel in front its blocks would crowd on the SMs that empty first (1024 tokens, 128 blocks: two to an SM on half of them,
     // 170 us instead of 115)
-    return launch_pdl_if(p.n_seq > 1, delta_columns_kernel<DP>, dim3((p.vdim + kCols - 1) / kCols, p.H, p.n_seq), dim3(kColThreads), (size_t)smem, st, p);
+    // (of M tokens no more than M / kChunkTokensMin sequences are long ones)
+    const int longest = std::min(p.n_seq, M / kChunkTokensMin);
+    return launch_pdl_if(p.n_seq > 1, delta_columns_kernel<DP>, dim3((p.vdim + kCols - 1) / kCols, p.H, longest), dim3(kColThreads), (size_t)smem, st, p);
 }
 
 }  // namespace

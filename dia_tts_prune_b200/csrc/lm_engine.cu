@@ -799,7 +799,7 @@ int stream_mixer_kernels(lm_b200_engine* e, const lm_b200_layer& l, const MixPla
             LCK(lm::launch_delta_chunks(e->rec, ldr, si, H, l.kv_heads, l.dim, l.vdim, l.rec_state, v.sm, v.rm, n_seq, M, at.out, at.ldo, e->delta_room, st, early));
         if (!chunks || n_seq > 1)
             LCK(lm::launch_column_scan(e->rec, ldr, si, lm::kScanDelta, H, l.kv_heads, l.dim, l.vdim, l.rec_state, v.sm, v.rm, n_seq, at.out, at.ldo, st,
-                                       true, early, nullptr, 0, 1.f, chunks));
+                                       true, early || chunks, nullptr, 0, 1.f, chunks));
         LCK(lm::launch_head_norm_gate(at.out, at.ldo, at.out_b, l.head_norm, gate, ld, H, l.vdim, e->m.eps, M, st, gate_act, at.scale));
     } else if (l.mixer == LM_B200_MIXER_RETENTION) {
         // q and k (adjacent in the row) turn in place, k also takes dim^-1/2; decay fixed per head, no write gate, no normaliser

@@ -65,6 +65,7 @@ __device__ __forceinline__ void copy4(float* dst, const float* src, bool ok) {
                  : "memory");
 }
 
+constexpr int kAllTokens = 0x7fffffff;
 struct ScanArgs {
     const float* in; int ld, q_off, k_off, v_off, b_off;      // b_off < 0: write strength 1
     const float* a_in; int lda;                               // decays: column h * dim + d, or column h (one per head)
@@ -76,7 +77,7 @@ struct ScanArgs {
     const int *seq_slot, *seq_row0, *seq_count, *row_pos;
     float* o; int ldo;
     int vec_qk, vec_a;                                        // whether 16-byte pieces are aligned
-    int fewer_than;                                           // sequences with more tokens are somebody else's
+    int fewer_than;                                           // sequences with more tokens are somebody else's: the kernel's in front, beside which this one runs
 };
 
 // DP: dim padded to a multiple of 32 (a power of two); VA: one decay per key channel
@@ -89,11 +90,17 @@ state_scan_kernel(const ScanArgs p) {
     const int VC = CW * (blockDim.x >> 5);                    // value columns of the CTA
     const int stage = kTokens * (VECS * DP + VC + 2);
     pdl_release();
-    pdl_wait();
+    // Beside the kernel in front: that one has let this one start only after its own wait, so that what both read is written, and they write different
+    // sequences.  But nobody behind may start before both have ended: one block waits for it at its end.
+    const bool beside = p.fewer_than != kAllTokens, ends_last = beside && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0;
+    if (!beside) pdl_wait();
     const int s = blockIdx.x, h = blockIdx.y, col0 = blockIdx.z * VC, g = h / (p.H / p.G);
     const int tid = threadIdx.x, lane = tid & 31, part = lane & (P - 1), cb = (tid >> 5) * CW + lane / P * 2;   // first column in the CTA
     const int slot = p.seq_slot[s], row0 = p.seq_row0[s], n = p.seq_count[s], start = p.row_pos[row0];
-    if (n >= p.fewer_than) return;
+    if (n >= p.fewer_than) {
+        if (ends_last) pdl_wait();
+        return;
+    }
     const float a_fix = p.fixed_decay ? p.fixed_decay[h] : 0.f, sd = p.skip ? p.skip[h] : 0.f;
     const bool vec_state = p.dim % 4 == 0;
 
@@ -308,6 +315,7 @@ state_scan_kernel(const ScanArgs p) {
             }
         }
     }
+    if (ends_last) pdl_wait();
 }
 
 template <int DP, int RULE, bool VA>
@@ -357,7 +365,7 @@ cudaError_t launch_column_scan(const float* in, int ld, const ScanInputs& si, in
     const float* a = decay ? decay : in + si.a_off;
     const int lda = decay ? ldd : ld;
     ScanArgs p{in, ld, si.q_off, si.k_off, si.v_off, rule == kScanDelta ? si.beta_off : -1, a, lda, nullptr, nullptr, q_mul, H, G, dim, vdim,
-               vdim, state, sm.slot, sm.row0, sm.count, rm.pos, o, ldo, 0, 0, few ? kChunkTokensMin : 0x7fffffff};
+               vdim, state, sm.slot, sm.row0, sm.count, rm.pos, o, ldo, 0, 0, few ? kChunkTokensMin : kAllTokens};
     p.vec_qk = aligned16(in, ld, si.q_off, dim) && (rule == kScanTied || aligned16(in, ld, si.k_off, dim));
     p.vec_a = aligned16(a, lda, 0, dim);
     switch (rule) {
@@ -374,7 +382,7 @@ cudaError_t launch_scalar_gate_scan(const float* in, int ld, const ScanInputs& s
                                     const float* fixed_decay, bool normaliser, bool early, int G, const float* skip) {
     if (G <= 0) G = H;
     ScanArgs p{in, ld, si.q_off, si.k_off, si.v_off, fixed_decay ? -1 : si.beta_off, in + si.a_off, ld, fixed_decay, skip, 1.f, H, G, dim, vdim,
-               vdim + (normaliser ? 1 : 0), state, sm.slot, sm.row0, sm.count, rm.pos, o, ldo, 0, 0, 0x7fffffff};
+               vdim + (normaliser ? 1 : 0), state, sm.slot, sm.row0, sm.count, rm.pos, o, ldo, 0, 0, kAllTokens};
     p.vec_qk = aligned16(in, ld, si.q_off, dim) && aligned16(in, ld, si.k_off, dim);
     return launch_scan<kScanWrite, false>(p, n_seq, early, st);
 }

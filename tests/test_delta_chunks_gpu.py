@@ -1,5 +1,5 @@
 """The delta rule with one decay per head in chunks of 32 tokens (csrc/lm_delta.cu) against the same tokens one after the other (csrc/lm_scan.cu, which
-portions of fewer than 320 tokens take): ragged last chunks, heads and columns that do not fill a block, a state that is continued, a token of NaN."""
+portions of fewer than 96 tokens take): ragged last chunks, heads and columns that do not fill a block, a state that is continued, a token of NaN."""
 
 import pytest
 import torch
@@ -35,7 +35,7 @@ def run(model, x, cuts):
     return [torch.cat(o) for o in out], state
 
 
-def portions(n, most=300):
+def portions(n, most=90):
     return [min(most, n - a) for a in range(0, n, most)]
 
 
@@ -47,10 +47,11 @@ def close(a, b):
 
 
 @pytest.mark.parametrize("heads,kv_heads,dim,vdim,rows", [
-    (2, 1, 128, 128, [320]),                                      # whole chunks
-    (4, 2, 64, 16, [321]),                                        # one token more; the smallest block of columns
+    (2, 1, 128, 128, [96]),                                       # whole chunks, the shortest portion that takes them
+    (4, 2, 64, 16, [97]),                                         # one token more; the smallest block of columns
     (3, 3, 72, 20, [351, 5, 320, 1000]),                          # channels and columns that do not fill a block; a short sequence between long ones
-    (8, 2, 128, 132, [640, 319]),                                 # the longest portion that stays with the scan
+    (8, 2, 128, 132, [640, 95]),                                  # the longest portion that stays with the scan
+    (4, 2, 64, 64, [90, 40, 95, 3]),                              # rows for chunks, but no sequence
     (4, 1, 4, 4, [330]),                                          # the narrowest heads
 ])
 def test_chunks_against_one_token_after_the_other(heads, kv_heads, dim, vdim, rows):
@@ -61,10 +62,10 @@ def test_chunks_against_one_token_after_the_other(heads, kv_heads, dim, vdim, ro
     yb, sb = run(model, x, [[n] for n in rows])
     for a, b in zip(yb + sb, ya + sa):
         close(a, b)
-    # and a state that chunks continue: a portion of 100 tokens in front
+    # and a state that chunks continue: a portion of 50 tokens in front
     x = [t for t in x if len(t) >= 420]
     if x:
-        yc, sc = run(model, x, [[100, len(t) - 100] for t in x])
+        yc, sc = run(model, x, [[50, len(t) - 50] for t in x])
         for a, b in zip(yc + sc, [y for y in ya if len(y) >= 420] + [s for s, n in zip(sa, rows) if n >= 420]):
             close(a, b)
 
