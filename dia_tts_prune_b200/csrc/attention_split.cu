@@ -72,6 +72,7 @@ struct Geometry {
     int k_sets;                              // scales of a key: one, with mixed scores one per kv head
     int depth;                               // tiles whose scales are in shared memory
     int rings;                               // tiles whose rows' numbers are (2 or 4)
+    int four;                                // a denominator per 16 keys (see split_attention_kernel)
     // the split keys and values in SplitAttention::work: SlotTiles per slot, then inverse scales [tile][set][key], then the tiles.  A
     // tile's parts: key groups (per kv head where the launch reads one head at a time), then value groups; its sets of scales: the keys
     // of each kv head, then the values of each (shared_kv: the keys' only)
@@ -524,8 +525,9 @@ __device__ __noinline__ void plain_row(const SplitAttention& p, int r, int slot,
         if (lane + 32 * u < n) dst[lane + 32 * u] = o[u] * f;
 }
 
-// NVS: channel groups of a value (1: up to 128 channels, 2: up to 256)
-template <int NVS>
+// NVS: channel groups of a value (1: up to 128 channels, 2: up to 256).  FOUR: a row has a running denominator per 16 keys of a tile (one in all where
+// the widest rows leave no shared memory for what its two threads tell each other of them)
+template <int NVS, bool FOUR>
 __global__ void __launch_bounds__(kSplitThreads, 1)
 split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_constant__ Geometry geo) {
     constexpr int DVH = 64 * NVS;                             // output channels of a thread
@@ -550,9 +552,10 @@ split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_co
     uint64_t* v_ready = q_ready + 1;                          // [depth] the scales of a tile's values are there
     const int n_bars = 2 * geo.n_slots + 15 + (geo.shared_kv ? 0 : geo.depth);
     float* m_x = reinterpret_cast<float*>(full + ((n_bars + 1) & ~1)); // [2][128] maxima up to an even and an odd tile
-    float* sum_x = m_x + 2 * kRows;                           // [rings / 2][128] sums of the weights of the odd tiles
-    float* q_inv = sum_x;                                     // [128] (the first odd tile's sums are stored when both groups have read it)
-    __nv_bfloat16* wi_x = reinterpret_cast<__nv_bfloat16*>(sum_x + geo.rings / 2 * kRows); // [rings][128] inverse scales of the weights: powers of two
+    // Denominators.  Of a row's two threads the even tiles' has those of a tile's first 32 keys, the other those of the last (not FOUR: the even tiles' has the one)
+    float* sum_x = m_x + 2 * kRows;                           // [rings][128][2] sums of a tile that the other group's thread has (not FOUR: [rings / 2][128] of the odd tiles)
+    float* q_inv = sum_x + (FOUR ? 2 * (geo.rings - 1) * kRows : 0);  // [128] (an odd tile's sums are stored there when both groups have read it)
+    __nv_bfloat16* wi_x = reinterpret_cast<__nv_bfloat16*>(sum_x + (FOUR ? 2 * geo.rings : geo.rings / 2) * kRows); // [rings][128] inverse scales of the weights: powers of two
     float* k_inv = reinterpret_cast<float*>(wi_x + geo.rings * kRows); // [depth][k_sets][64] inverse scales of the keys
     float* v_inv = geo.shared_kv ? k_inv : k_inv + geo.depth * geo.k_sets * kKeys;      // [depth][64] of the values
     int4* s_tile = reinterpret_cast<int4*>(v_inv + geo.depth * kKeys); // [depth] a tile's first key, its tokens (first | end << 16), end of its keys, lo (see Walk)
@@ -751,21 +754,25 @@ split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_co
         f2 O[DVH / 2];
 #pragma unroll
         for (int c = 0; c < DVH / 2; ++c) O[c] = 0;
-        float m_run = -CUDART_INF_F, l = 0.f;
-        float m_own = 0.f, wi_own = 0.f, sum_own = 0.f;       // of the tile of this group that has not been added yet
+        float m_run = -CUDART_INF_F;
+        float2 l2 = make_float2(0.f, 0.f);
+        float m_own = 0.f, wi_own = 0.f;                      // of the tile of this group that has not been added yet
+        float2 sum_own = make_float2(0.f, 0.f);
         bool ok = true;
-        // O <- corr O + the value product of tile t, up to which the maximum is m; the denominator likewise (in the threads of the even tiles).
+        // O <- corr O + the value product of tile t, up to which the maximum is m; this thread's denominators likewise.
         // The numbers of the other group's tile were stored in front of the weights that have been multiplied.
-        auto add_values = [&](unsigned t, float m, float wi, float sum) {
+        auto add_values = [&](unsigned t, float m, float wi, float2 sum) {
             if (!wait_for(&pv_done[t & 1u], (t >> 1) & 1u)) return false;
             fence_after();
             if ((int)(t & 1u) != hf) {
-                wi = __bfloat162float(wi_x[(t & (geo.rings - 1u)) * kRows + row]);
-                if (hf == 0) sum = sum_x[((t >> 1) & (geo.rings / 2 - 1u)) * kRows + row];
+                const unsigned at = (t & (geo.rings - 1u)) * kRows + row;
+                wi = __bfloat162float(wi_x[at]);
+                if (FOUR) sum = reinterpret_cast<const float2*>(sum_x)[at];
+                else if (hf == 0) sum.x = sum_x[((t >> 1) & (geo.rings / 2 - 1u)) * kRows + row];
             }
             const float corr = m_run == -CUDART_INF_F ? 0.f : ex2(m_run - m);      // (m is no less)
             const f2 vi2 = twice(wi), c2 = twice(corr);
-            l = fmaf(l, corr, sum);
+            l2 = make_float2(fmaf(l2.x, corr, sum.x), fmaf(l2.y, corr, sum.y));
             m_run = m;
             const uint32_t from = t_mine + (geo.o_bufs == 2 ? (t & 1u) * 128u : 0u);
 #pragma unroll
@@ -954,7 +961,6 @@ split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_co
                     unpack2(a, x, y);
                     sum[c] = x + y;
                 }
-                sum_own = (sum[0] + sum[1]) + (sum[2] + sum[3]);
                 // weight x its value's magnitude, and the largest of them that this row has in the tile
                 if (!geo.shared_kv && !wait_for(&v_ready[my_at], my_round)) break;
                 scale_by<kKeys / 2>(s, v_inv + my_at * kKeys);
@@ -962,7 +968,7 @@ split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_co
                 if (__any_sync(0xffffffffu, wm != wm)) {          // a value that cannot be split, 0 x NaN where it is not seen
                     hide(0.f);
                     wm = largest();
-                    if (wm != wm) sum_own = CUDART_NAN_F;
+                    if (wm != wm) sum[0] = CUDART_NAN_F;
                 }
                 const f2 ws = twice(scale_of(wm, wi_own));
                 // the weights' columns are free once the value product that read them is done (of two sets: it has been added by now)
@@ -971,8 +977,15 @@ split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_co
                     fence_after();
                 }
                 // (the other group has read the place: the tile `rings` before, or with one set and one product two before, has been added)
-                wi_x[(t & (geo.rings - 1u)) * kRows + row] = __float2bfloat16(wi_own);
-                if (hf == 1) sum_x[((t >> 1) & (geo.rings / 2 - 1u)) * kRows + row] = sum_own;
+                const unsigned place = (t & (geo.rings - 1u)) * kRows + row;
+                wi_x[place] = __float2bfloat16(wi_own);
+                if constexpr (FOUR) {
+                    reinterpret_cast<float2*>(sum_x)[place] = hf == 0 ? make_float2(sum[2], sum[3]) : make_float2(sum[0], sum[1]);
+                    sum_own = hf == 0 ? make_float2(sum[0], sum[1]) : make_float2(sum[2], sum[3]);
+                } else {
+                    sum_own.x = (sum[0] + sum[1]) + (sum[2] + sum[3]);
+                    if (hf == 1) sum_x[((t >> 1) & (geo.rings / 2 - 1u)) * kRows + row] = sum_own.x;
+                }
                 const uint32_t to = t_p + lanes + (geo.p_bufs == 2 ? (t & 1u) * 64u : 0u);
 #pragma unroll
                 for (int c = 0; c < kKeys / 16; ++c) {
@@ -994,13 +1007,19 @@ split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_co
                 }
             }
             m_other = m_old;
-            ok = !MID || t == 0 || t > n_tiles || add_values(t - 1, m_old, 0.f, 0.f);
+            ok = !MID || t == 0 || t > n_tiles || add_values(t - 1, m_old, 0.f, make_float2(0.f, 0.f));
             my_at += 2;
             if (my_at >= (unsigned)geo.depth) my_at -= geo.depth, my_round ^= 1u;
         }
-        if (hf == 0) sum_x[row] = l;
+        asm volatile("bar.sync 2, %0;" ::"n"(32 * RW) : "memory");           // (the last tiles' sums have been read)
+        if (FOUR) reinterpret_cast<float2*>(sum_x)[hf * kRows + row] = l2;
+        else if (hf == 0) sum_x[row] = l2.x;
         asm volatile("bar.sync 2, %0;" ::"n"(32 * RW) : "memory");
-        l = sum_x[row];
+        float l = sum_x[row];
+        if (FOUR) {
+            const float2 a = reinterpret_cast<const float2*>(sum_x)[row], b = reinterpret_cast<const float2*>(sum_x)[kRows + row];
+            l = ((a.x + a.y) + b.x) + b.y;
+        }
         // ---- the sink's own term, normalise, store ----
         if (p.sink) l += ex2(fmaf(p.sink[h], kLog2e, m_run == -CUDART_INF_F ? 0.f : -m_run));
         // through shared memory (the ring and the queries are read; 32 rows of this warp's channels): whole lines reach the output, and
@@ -1337,11 +1356,18 @@ bool geometry_of(const SplitAttention& a, Geometry& g, size_t& smem) {
     g.rings = g.p_bufs == 1 && g.o_bufs == 1 ? 2 : 4;
     auto control_of = [&](int slots) {
         const int depth = depth_of(slots), bars = 2 * slots + 15 + (g.shared_kv ? 0 : depth);
-        return ((bars + 1) & ~1) * 8 + kRows * (2 * 4 + g.rings * 4) + depth * (kKeys * (g.k_sets + (g.shared_kv ? 0 : 1)) * 4 + 16) + 32 + 2 * (kRows >> g.pk_shift) * 4;
+        return ((bars + 1) & ~1) * 8 + kRows * (2 * 4 + (g.four ? g.rings * 8 : g.rings * 2) + g.rings * 2) + depth * (kKeys * (g.k_sets + (g.shared_kv ? 0 : 1)) * 4 + 16) + 32 + 2 * (kRows >> g.pk_shift) * 4;
     };
-    for (g.n_slots = kMaxSlots; g.n_slots >= 2; --g.n_slots)
-        if (g.n_slots * g.slot_bytes + g.q_bytes + control_of(g.n_slots) <= kSmemMost) break;
-    if (g.n_slots < 2) return false;
+    g.four = 1;
+    auto most_slots = [&] {
+        for (g.n_slots = kMaxSlots; g.n_slots >= 2; --g.n_slots)
+            if (g.n_slots * g.slot_bytes + g.q_bytes + control_of(g.n_slots) <= kSmemMost) return true;
+        return false;
+    };
+    if (!most_slots()) {
+        g.four = 0;
+        if (g.n_vst == 1 || !most_slots()) return false;      // (only keys of 305 channels and more over values of 129 and more come here)
+    }
     g.depth = depth_of(g.n_slots);
     const int control = control_of(g.n_slots);
     // the output is staged in the ring and the queries: 8 warps of 32 rows, 4 floats between the rows
@@ -1351,18 +1377,18 @@ bool geometry_of(const SplitAttention& a, Geometry& g, size_t& smem) {
     return smem <= (size_t)kSmemMost;
 }
 
-template <int NVS>
+template <int NVS, bool FOUR>
 cudaError_t launch_inst(const SplitAttention& a, const Geometry& g, size_t smem, cudaStream_t st) {
     int device = 0;
     cudaError_t e = cudaGetDevice(&device);
-    if (e == cudaSuccess) e = ask_smem<split_attention_kernel<NVS>>(device, kSmemMost);
+    if (e == cudaSuccess) e = ask_smem<split_attention_kernel<NVS, FOUR>>(device, kSmemMost);
     if (e != cudaSuccess) return e;
     const int tt = kRows >> g.pk_shift, tiles = a.n_seq > 1 ? a.M / tt + a.n_seq : (a.M + tt - 1) / tt;
     if (a.work) {
         split_keys_kernel<<<dim3(std::min(g.cap_tiles, std::max(1, kSplitGrid / g.parts)), g.parts), 256, 0, st>>>(a, g);
         ++extra_launches();
     }
-    split_attention_kernel<NVS><<<(a.heads >> g.pk_shift) * tiles, kSplitThreads, smem, st>>>(a, g);
+    split_attention_kernel<NVS, FOUR><<<(a.heads >> g.pk_shift) * tiles, kSplitThreads, smem, st>>>(a, g);
     return cudaGetLastError();
 }
 
@@ -1423,7 +1449,8 @@ cudaError_t launch_split_attention(const SplitAttention& a, cudaStream_t st) {
     SplitAttention with = a;
     // Keys are split in advance wherever there is room: the fetching warps have few registers for them
     if (g.cap_tiles <= 0) with.work = nullptr;
-    return g.n_vst == 2 ? launch_inst<2>(with, g, smem, st) : launch_inst<1>(with, g, smem, st);
+    if (g.n_vst == 2) return g.four ? launch_inst<2, true>(with, g, smem, st) : launch_inst<2, false>(with, g, smem, st);
+    return launch_inst<1, true>(with, g, smem, st);
 }
 
 }  // namespace dia

@@ -1,6 +1,8 @@
 """The tensor-core attention with split fp32 operands (csrc/attention_split.cu) at the sizes where it can go wrong: edges of its
 tiles of 64 keys and 128 (token, head) rows, channel groups, segments of several sequences, windows, magnitudes far from one."""
 
+import math
+
 import pytest
 import torch
 
@@ -164,3 +166,21 @@ def test_keys_beyond_the_room(H, G, d, window):
     got = model.engine.op_attention(0, dev[past:].clone(), [(seq, rows, past)])
     ref = sink_reference(x.double(), past, H, G, d, p, window, 0, 0.0, cfg["norm"]["eps"])
     close(got, ref, ref.abs().max().item())
+
+
+@pytest.mark.parametrize("place", [3, 20, 45, 63])
+def test_denominators_are_summed_per_16_keys(place):
+    """One key of weight one and, in every tile of 64, one of 2^-25: half a unit in the last place of a sum with the first, so 64 of them are lost from a sum per
+    tile (a denominator 2^-19 too small) and none from a sum per 16 keys, unless they share those 16.  Channel 1, which has the first key's value
+    alone, is one over the denominator; four roundings of the score change a weight of 2^-25 by 2^-17 of itself at most, and the result by less than 2^-24."""
+    from dia_tts_prune_b200 import engine as E
+    tiles, light = 64, 2.0 ** -25
+    q, k, v = torch.zeros(1, 192, 1, 128), torch.zeros(1, 1, 64 * tiles, 128), torch.zeros(1, 1, 64 * tiles, 128)
+    q[..., 0] = 1.0
+    k[..., 0] = -400.0 * 128 ** 0.5                               # (exp of that is zero)
+    k[0, 0, place::64, 0] = math.log(light) * 128 ** 0.5
+    heavy = 8 if place >= 16 else 40
+    k[0, 0, heavy, 0] = 0.0
+    v[0, 0, :, 0], v[0, 0, heavy, 0], v[0, 0, heavy, 1] = 1.0, 0.0, 1.0
+    got = E.attention_rows(q.cuda(), k.cuda(), v.cuda(), 64 * tiles, 2, None)[0, :, 0, 1].double().cpu()
+    assert (got - 1.0 / (1.0 + tiles * light)).abs().max() <= 2.0 ** -22
