@@ -77,6 +77,7 @@ struct Geometry {
     // tile's parts: key groups (per kv head where the launch reads one head at a time), then value groups; its sets of scales: the keys
     // of each kv head, then the values of each (shared_kv: the keys' only)
     int parts, k_parts, sets, cap_tiles;
+    int page_shift;                          // log2 of the page size (-1: it is no power of two)
     int* ran_out;                            // the device's word (null: none)
     unsigned tile_bytes, scale_off, tile_off;
 };
@@ -89,6 +90,12 @@ __device__ __forceinline__ bool wait_for(uint64_t* bar, uint32_t parity) {
     for (unsigned i = 0; i < kSpinMost; ++i)
         if (mbar_try_wait(bar, parity)) return true;
     return false;
+}
+// one look that does not wait
+__device__ __forceinline__ bool has_passed(uint64_t* bar, uint32_t parity) {
+    uint32_t done;
+    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(done) : "r"(smem_u32(bar)), "r"(parity) : "memory");
+    return done != 0;
 }
 // the same for a converged warp, with one answer for all lanes (so that what follows is uniform: see elect_one_sync)
 __device__ __forceinline__ bool wait_warp(uint64_t* bar, uint32_t parity) {
@@ -229,6 +236,24 @@ __device__ __forceinline__ void split2(f2 v, uint32_t& hi, uint32_t& lo) {
     float x, y;
     unpack2(v, x, y);
     split2(x, y, hi, lo);
+}
+// (lo, hi) = the terms of eight values times f: the same as split2 of each, two at a time
+__device__ __forceinline__ void split8(const ulonglong2& a, const ulonglong2& b, f2 f, uint4& hi, uint4& lo) {
+    const f2 v[4] = {mul2(a.x, f), mul2(a.y, f), mul2(b.x, f), mul2(b.y, f)};
+    uint32_t h[4], l[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        float x, y;
+        unpack2(v[i], x, y);
+        const __half2 t = __floats2half2_rn(x, y);
+        const float2 u = __half22float2(t);
+        unpack2(add2(v[i], pack2(-u.x, -u.y)), x, y);
+        const __half2 r = __floats2half2_rn(x, y);
+        h[i] = *reinterpret_cast<const uint32_t*>(&t);
+        l[i] = *reinterpret_cast<const uint32_t*>(&r);
+    }
+    hi = make_uint4(h[0], h[1], h[2], h[3]);
+    lo = make_uint4(l[0], l[1], l[2], l[3]);
 }
 // the power of two that brings a largest magnitude m to [2^14, 2^15), and its inverse (m = 0: 2^114; both stay normal numbers)
 __device__ __forceinline__ float scale_of(float m, float& inverse) {
@@ -527,7 +552,8 @@ __device__ __noinline__ void plain_row(const SplitAttention& p, int r, int slot,
 
 // NVS: channel groups of a value (1: up to 128 channels, 2: up to 256).  FOUR: a row has a running denominator per 16 keys of a tile (one in all where
 // the widest rows leave no shared memory for what its two threads tell each other of them)
-template <int NVS, bool FOUR>
+// SELF: not all keys have to be split in advance.
+template <int NVS, bool FOUR, bool SELF>
 __global__ void __launch_bounds__(kSplitThreads, 1)
 split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_constant__ Geometry geo) {
     constexpr int DVH = 64 * NVS;                             // output channels of a thread
@@ -1085,10 +1111,90 @@ split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_co
             };
             int4 about{};                                         // what the row warps are told of the newest tile
             struct Tile { int split, slot, j0, k_end; };          // split: the tile of the room that holds these keys (-1: none)
+            auto part_width = [&](bool is_v, int part) {
+                const int last = (is_v ? geo.n_vst : geo.n_kst) - 1;
+                return is_v ? (part == last ? geo.v_last_layout : geo.v0_layout) : (part == last ? geo.wk_last : geo.wk0);
+            };
+            auto row_at = [&](int of, int j) -> unsigned long long {      // (in kv head 0)
+                if (!p.table) return (unsigned long long)of * p.kv_heads * p.page_size + j;
+                const unsigned at = geo.page_shift >= 0 ? (unsigned)j >> geo.page_shift : (unsigned)j / (unsigned)p.page_size;
+                const unsigned page = p.table[(size_t)of * p.max_pages + at];
+                return (unsigned long long)page * ((unsigned)p.kv_heads * (unsigned)p.page_size) + ((unsigned)j - at * (unsigned)p.page_size);
+            };
+            // SELF: a part that is not split yet comes as it is, into the bytes that its terms will have: the first four of a lane's eight channels where their high terms will be, the
+            // others where the low ones will be.  The lane that asked for them splits them there while the next part is on its way.
+            constexpr int kEights = (kKeys / 8 + kFetchWarps - 1) / kFetchWarps;      // this warp's keys: eights lw, lw + 3, lw + 6 of a tile, a lane a part of one
+            int raw = -1, raw_part = 0;                       // the place and the group of the part that is to be split (-1: none)
+            unsigned raw_at = 0;
+            bool raw_v = false;
+            float raw_more[kEights] = {};                     // largest magnitudes of the keys' channels beyond the part
+            auto split_raw = [&](bool behind) {               // behind: another part has been asked for since
+                if (behind) asm volatile("cp.async.wait_group 1;" ::: "memory");
+                else asm volatile("cp.async.wait_group 0;" ::: "memory");
+                const bool shared = raw_v && geo.shared_kv;   // (a shared row's scale is its key's)
+                const int wp = part_width(raw_v, raw_part), blocks = wp >> 3;
+                // (keys of several groups of channels have one scale, which the first group takes)
+                const bool own = raw_v ? raw_part == 0 && !shared : raw_part == 0 || geo.k_sets > 1;
+                float* const inv = raw_v && !shared ? v_inv + raw_at * kKeys : k_inv + (raw_at * geo.k_sets + (geo.k_sets > 1 ? raw_part : 0)) * kKeys;
+                __syncwarp();
+#pragma unroll 1
+                for (int e = lw; e < kKeys / 8; e += kFetchWarps) {
+                    unsigned char* const dst = ring + (size_t)raw * geo.slot_bytes + (e * blocks + cq) * 128 + kin * 16;
+                    unsigned char* const low = dst + kKeys * wp * 2;
+                    ulonglong2 v[8];
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const bool has = cq + 4 * i < blocks;
+                        v[2 * i] = has ? *reinterpret_cast<const ulonglong2*>(dst + i * 512) : make_ulonglong2(0, 0);
+                        v[2 * i + 1] = has ? *reinterpret_cast<const ulonglong2*>(low + i * 512) : make_ulonglong2(0, 0);
+                    }
+                    float sc, inverse;
+                    bool bad;
+                    if (own) {
+                        float m = e < kFetchWarps ? raw_more[0] : e < 2 * kFetchWarps ? raw_more[1] : raw_more[2], m2 = 0.f;
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) {
+                            float a, b, c, d;
+                            unpack2(v[i].x, a, b);
+                            unpack2(v[i].y, c, d);
+                            m = max3_nan(m, fabsf(a), fabsf(b));
+                            m2 = max3_nan(m2, fabsf(c), fabsf(d));
+                        }
+                        bad = scale_row(row_max(max_nan(m, m2)), sc, inverse);
+                        if (lane < 8) inv[e * 8 + lane] = inverse;
+                    } else {
+                        inverse = inv[e * 8 + kin];
+                        bad = inverse != inverse;
+                        sc = __uint_as_float((254u << 23) - __float_as_uint(inverse));      // (powers of two)
+                    }
+                    if (bad) {
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) v[i] = make_ulonglong2(0, 0);
+                        sc = 0.f;
+                    }
+                    const f2 sc2 = twice(sc);
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        uint4 hi, lo;
+                        split8(v[2 * i], v[2 * i + 1], sc2, hi, lo);
+                        if (cq + 4 * i < blocks) {
+                            *reinterpret_cast<uint4*>(dst + i * 512) = hi;
+                            *reinterpret_cast<uint4*>(low + i * 512) = lo;
+                        }
+                    }
+                }
+                fence_smem_async();
+                __syncwarp();
+                if (lane == 0 && raw_v && own) mbar_arrive(&v_ready[raw_at]);
+                if (lane == 0) mbar_arrive(&full[raw]);
+                raw = -1;
+            };
             // the ring's next part: key group `part` of the tile at place at_t of the numbers' rings, or value group `part` of it
             auto fetch = [&](const Tile& z, unsigned at_t, bool is_v, int part) {
-                const int last = (is_v ? geo.n_vst : geo.n_kst) - 1;
-                const int wp = is_v ? (part == last ? geo.v_last_layout : geo.v0_layout) : (part == last ? geo.wk_last : geo.wk0);
+                const int wp = part_width(is_v, part);
+                // (a part that is split already may bring scales to the place of those that the raw one asks for)
+                if constexpr (SELF)
+                    if (raw >= 0 && (z.split >= 0 || !__all_sync(0xffffffffu, has_passed(&empty[slot], phase ^ 1u)))) split_raw(false);
                 if (z.split >= 0) {                               // split already: with its first key group a tile's scales come along
                     if (lane == 0) {
                         ok = wait_for(&empty[slot], phase ^ 1u);
@@ -1115,52 +1221,117 @@ split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_co
                     ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
                     return;
                 }
-                // Beyond the room: split here, eight keys at a time, a lane a part of one.  Rolled and with few registers, since the row warps have the
-                // others: keys that are split in advance are the rule.
-                const bool shared = is_v && geo.shared_kv;        // (a shared row's scale is its key's)
-                const float* const cache = is_v ? p.vcache : p.kcache;
-                const int width = is_v ? p.vrow : p.kdim, row_w = is_v && !shared ? p.vdim : p.kdim, c0 = p.talk && !is_v ? 0 : part * kGroupW;
-                const int gg = p.talk && !is_v ? part : g, w = min(kGroupW, row_w - c0);
-                float* const inv = is_v ? (part == 0 && !shared ? v_inv + at_t * kKeys : nullptr)
-                                        : part == 0 || geo.k_sets > 1 ? k_inv + (at_t * geo.k_sets + (geo.k_sets > 1 ? part : 0)) * kKeys : nullptr;
-#pragma unroll 1
-                for (int e = lw; e < kKeys / 8; e += kFetchWarps) {
-                    const int j = z.j0 + e * 8 + kin;
-                    const bool in = j < z.k_end;
-                    const float* src = cache;
-                    if (in) {
-                        const int page = p.table ? p.table[(size_t)z.slot * p.max_pages + j / p.page_size] : z.slot;
-                        src += (((size_t)page * p.kv_heads + gg) * p.page_size + (p.table ? j % p.page_size : j)) * width;
-                    }
-                    float m = 0.f, sc, inverse;
-#pragma unroll 1
-                    for (int c = 4 * cq; in && c < row_w; c += 16) m = max_abs4(m, *reinterpret_cast<const float4*>(src + c));
-                    const bool bad = scale_row(row_max(m), sc, inverse);
-                    // (a value's scales have their place before the ring has one: see geometry_of)
-                    if (e == lw && !is_v && !wait_for(&empty[slot], phase ^ 1u)) { ok = false; return; }
-                    if (inv && lane < 8) inv[e * 8 + lane] = inverse;
-                    if (e == 0 && !is_v && part == 0 && lane == 0) s_tile[at_t] = about;
-                    if (e == lw && is_v && !wait_for(&empty[slot], phase ^ 1u)) { ok = false; return; }
+                if constexpr (SELF) {
                     const int blocks = wp >> 3;
-                    unsigned char* dst = ring + (size_t)slot * geo.slot_bytes + e * blocks * 128 + kin * 16;
-#pragma unroll 1
-                    for (int c8 = cq; c8 < blocks; c8 += 4) {
-                        const float4 none = make_float4(0.f, 0.f, 0.f, 0.f);
-                        const float4 a = in && !bad && 8 * c8 < w ? *reinterpret_cast<const float4*>(src + c0 + 8 * c8) : none;
-                        const float4 b = in && !bad && 8 * c8 + 4 < w ? *reinterpret_cast<const float4*>(src + c0 + 8 * c8 + 4) : none;
-                        uint32_t hi[4], lo[4];
-                        split2(a.x * sc, a.y * sc, hi[0], lo[0]);
-                        split2(a.z * sc, a.w * sc, hi[1], lo[1]);
-                        split2(b.x * sc, b.y * sc, hi[2], lo[2]);
-                        split2(b.z * sc, b.w * sc, hi[3], lo[3]);
-                        *reinterpret_cast<uint4*>(dst + c8 * 128) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-                        *reinterpret_cast<uint4*>(dst + c8 * 128 + kKeys * wp * 2) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+                    const bool shared = is_v && geo.shared_kv;
+                    const float* const cache = is_v ? p.vcache : p.kcache;
+                    const int width = is_v ? p.vrow : p.kdim, row_w = is_v && !shared ? p.vdim : p.kdim, c0 = p.talk && !is_v ? 0 : part * kGroupW;
+                    const int gg = p.talk && !is_v ? part : g, w = min(kGroupW, row_w - c0);
+                    const float* src[kEights];                    // this lane's first channels of its keys (of the cache's first row in the place of keys that are not there)
+                    bool in[kEights];
+                    const bool one_page = !p.table || geo.page_shift >= 6;      // (a tile starts at a multiple of 64 keys)
+                    const unsigned long long row0 = one_page ? row_at(z.slot, z.j0) : 0;
+                    const float* const head = cache + ((size_t)gg * p.page_size) * width + (c0 + 8 * cq);
+#pragma unroll
+                    for (int u = 0; u < kEights; ++u) {
+                        const int e = (lw + u * kFetchWarps) * 8 + kin;
+                        in[u] = lw + u * kFetchWarps < kKeys / 8 && z.j0 + e < z.k_end;
+                        src[u] = in[u] ? head + (one_page ? row0 + e : row_at(z.slot, z.j0 + e)) * (unsigned)width : cache + (c0 + 8 * cq);
                     }
+                    ok = __all_sync(0xffffffffu, wait_for(&empty[slot], phase ^ 1u));
+                    if (!ok) return;
+                    if (lw == 0 && !is_v && part == 0 && lane == 0) s_tile[at_t] = about;
+                    const uint32_t place = smem_u32(ring) + slot * geo.slot_bytes + kin * 16 + (lw * blocks + cq) * 128, low = kKeys * wp * 2;
+                    auto copy16 = [&](uint32_t dst, const float* from, int bytes) {
+                        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(from), "r"(bytes) : "memory");
+                    };
+                    const bool whole = z.j0 + kKeys <= z.k_end && w == wp;
+#pragma unroll
+                    for (int u = 0; u < kEights; ++u) {
+                        if (lw + u * kFetchWarps >= kKeys / 8) continue;
+                        const uint32_t dst = place + u * kFetchWarps * blocks * 128;
+                        if (whole) {
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) {
+                                if (cq + 4 * i >= blocks) continue;
+                                copy16(dst + i * 512, src[u] + 32 * i, 16);
+                                copy16(dst + low + i * 512, src[u] + 32 * i + 4, 16);
+                            }
+                        } else {
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) {
+                                if (cq + 4 * i >= blocks) continue;
+                                const int left = in[u] ? w - 8 * cq - 32 * i : 0;      // (no channel is read that is not there)
+                                copy16(dst + i * 512, left > 0 ? src[u] + 32 * i : cache, left > 0 ? 16 : 0);
+                                copy16(dst + low + i * 512, left > 4 ? src[u] + 32 * i + 4 : cache, left > 4 ? 16 : 0);
+                            }
+                        }
+                    }
+                    asm volatile("cp.async.commit_group;" ::: "memory");
+                    if (raw >= 0) split_raw(true);
+#pragma unroll
+                    for (int u = 0; u < kEights; ++u) raw_more[u] = 0.f;
+                    if (part == 0 && !shared && w < row_w) {
+#pragma unroll 3
+                        for (int c = w + 4 * cq; c < row_w; c += 16) {
+#pragma unroll
+                            for (int u = 0; u < kEights; ++u)
+                                if (in[u]) raw_more[u] = max_abs4(raw_more[u], *reinterpret_cast<const float4*>(src[u] + (c - 8 * cq)));
+                        }
+                    }
+                    raw = (int)slot;
+                    raw_part = part;
+                    raw_at = at_t;
+                    raw_v = is_v;
+                } else {
+                    // The launch saw to it that all keys are split in advance, or was told so.  If not, eight at a time and rolled: this instance is all about code
+                    // that is short (with the other form in it, or with neither, a latent layer of 4096 rows takes 636 us, not 620: the row warps' code is fetched
+                    // from other places)
+                    const bool shared = is_v && geo.shared_kv;        // (a shared row's scale is its key's)
+                    const float* const cache = is_v ? p.vcache : p.kcache;
+                    const int width = is_v ? p.vrow : p.kdim, row_w = is_v && !shared ? p.vdim : p.kdim, c0 = p.talk && !is_v ? 0 : part * kGroupW;
+                    const int gg = p.talk && !is_v ? part : g, w = min(kGroupW, row_w - c0);
+                    float* const inv = is_v ? (part == 0 && !shared ? v_inv + at_t * kKeys : nullptr)
+                                            : part == 0 || geo.k_sets > 1 ? k_inv + (at_t * geo.k_sets + (geo.k_sets > 1 ? part : 0)) * kKeys : nullptr;
+#pragma unroll 1
+                    for (int e = lw; e < kKeys / 8; e += kFetchWarps) {
+                        const int j = z.j0 + e * 8 + kin;
+                        const bool in = j < z.k_end;
+                        const float* src = cache;
+                        if (in) {
+                            const int page = p.table ? p.table[(size_t)z.slot * p.max_pages + j / p.page_size] : z.slot;
+                            src += (((size_t)page * p.kv_heads + gg) * p.page_size + (p.table ? j % p.page_size : j)) * width;
+                        }
+                        float m = 0.f, sc, inverse;
+#pragma unroll 1
+                        for (int c = 4 * cq; in && c < row_w; c += 16) m = max_abs4(m, *reinterpret_cast<const float4*>(src + c));
+                        const bool bad = scale_row(row_max(m), sc, inverse);
+                        // (a value's scales have their place before the ring has one: see geometry_of)
+                        if (e == lw && !is_v && !wait_for(&empty[slot], phase ^ 1u)) { ok = false; return; }
+                        if (inv && lane < 8) inv[e * 8 + lane] = inverse;
+                        if (e == 0 && !is_v && part == 0 && lane == 0) s_tile[at_t] = about;
+                        if (e == lw && is_v && !wait_for(&empty[slot], phase ^ 1u)) { ok = false; return; }
+                        const int blocks = wp >> 3;
+                        unsigned char* dst = ring + (size_t)slot * geo.slot_bytes + e * blocks * 128 + kin * 16;
+#pragma unroll 1
+                        for (int c8 = cq; c8 < blocks; c8 += 4) {
+                            const float4 none = make_float4(0.f, 0.f, 0.f, 0.f);
+                            const float4 a = in && !bad && 8 * c8 < w ? *reinterpret_cast<const float4*>(src + c0 + 8 * c8) : none;
+                            const float4 b = in && !bad && 8 * c8 + 4 < w ? *reinterpret_cast<const float4*>(src + c0 + 8 * c8 + 4) : none;
+                            uint32_t hi[4], lo[4];
+                            split2(a.x * sc, a.y * sc, hi[0], lo[0]);
+                            split2(a.z * sc, a.w * sc, hi[1], lo[1]);
+                            split2(b.x * sc, b.y * sc, hi[2], lo[2]);
+                            split2(b.z * sc, b.w * sc, hi[3], lo[3]);
+                            *reinterpret_cast<uint4*>(dst + c8 * 128) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+                            *reinterpret_cast<uint4*>(dst + c8 * 128 + kKeys * wp * 2) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+                        }
+                    }
+                    fence_smem_async();
+                    __syncwarp();
+                    if (lane == 0 && is_v && inv) mbar_arrive(&v_ready[at_t]);
+                    if (lane == 0) mbar_arrive(&full[slot]);
                 }
-                fence_smem_async();
-                __syncwarp();
-                if (lane == 0 && is_v && inv) mbar_arrive(&v_ready[at_t]);
-                if (lane == 0) mbar_arrive(&full[slot]);
             };
             // the keys of a tile, then the values of the tile s_bufs before: the order in which they are multiplied
             Tile z0{}, z1{}, z2{};                                // the newest first
@@ -1197,6 +1368,10 @@ split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_co
                     fetch(!is_v ? z0 : two ? z2 : z1, !is_v ? at0 : two ? at2 : at1, is_v, is_v ? i - nk : i);
                     if (++slot == (unsigned)geo.n_slots) slot = 0, phase ^= 1u;
                 }
+            }
+            if constexpr (SELF) {
+                if (ok && raw >= 0) split_raw(false);
+                asm volatile("cp.async.wait_group 0;" ::: "memory");  // (a wait may have run out)
             }
         } else {
             // ================= the MMA issuer: the whole warp counts tiles, one elected lane issues =================
@@ -1297,6 +1472,9 @@ bool geometry_of(const SplitAttention& a, Geometry& g, size_t& smem) {
     if (a.rows_per_slot > 0 && (long long)a.rows_per_slot * 16 < a.M) return false;
     auto pad16 = [](int v) { return (v + 15) & ~15; };
     const int rep = a.heads / a.kv_heads;
+    g.page_shift = -1;
+    if (a.page_size > 0 && (a.page_size & (a.page_size - 1)) == 0)
+        for (g.page_shift = 0; 1 << g.page_shift < a.page_size;) ++g.page_shift;
     g.pk_shift = 0;
     while (g.pk_shift < 7 && rep % (2 << g.pk_shift) == 0) ++g.pk_shift;
     if (a.talk) {
@@ -1377,19 +1555,25 @@ bool geometry_of(const SplitAttention& a, Geometry& g, size_t& smem) {
     return smem <= (size_t)kSmemMost;
 }
 
-template <int NVS, bool FOUR>
+template <int NVS, bool FOUR, bool SELF>
 cudaError_t launch_inst(const SplitAttention& a, const Geometry& g, size_t smem, cudaStream_t st) {
     int device = 0;
     cudaError_t e = cudaGetDevice(&device);
-    if (e == cudaSuccess) e = ask_smem<split_attention_kernel<NVS, FOUR>>(device, kSmemMost);
+    if (e == cudaSuccess) e = ask_smem<split_attention_kernel<NVS, FOUR, SELF>>(device, kSmemMost);
     if (e != cudaSuccess) return e;
     const int tt = kRows >> g.pk_shift, tiles = a.n_seq > 1 ? a.M / tt + a.n_seq : (a.M + tt - 1) / tt;
     if (a.work) {
         split_keys_kernel<<<dim3(std::min(g.cap_tiles, std::max(1, kSplitGrid / g.parts)), g.parts), 256, 0, st>>>(a, g);
         ++extra_launches();
     }
-    split_attention_kernel<NVS, FOUR><<<(a.heads >> g.pk_shift) * tiles, kSplitThreads, smem, st>>>(a, g);
+    split_attention_kernel<NVS, FOUR, SELF><<<(a.heads >> g.pk_shift) * tiles, kSplitThreads, smem, st>>>(a, g);
     return cudaGetLastError();
+}
+
+template <bool SELF>
+cudaError_t launch_any(const SplitAttention& a, const Geometry& g, size_t smem, cudaStream_t st) {
+    if (g.n_vst == 2) return g.four ? launch_inst<2, true, SELF>(a, g, smem, st) : launch_inst<2, false, SELF>(a, g, smem, st);
+    return launch_inst<1, true, SELF>(a, g, smem, st);
 }
 
 }  // namespace
@@ -1447,10 +1631,14 @@ cudaError_t launch_split_attention(const SplitAttention& a, cudaStream_t st) {
     g.ran_out = split_attention_ran_out(device, st);          // (mapped and unified: one address on both sides)
     if (take_ran_out(device, st)) return cudaErrorLaunchTimeout;
     SplitAttention with = a;
-    // Keys are split in advance wherever there is room: the fetching warps have few registers for them
     if (g.cap_tiles <= 0) with.work = nullptr;
-    if (g.n_vst == 2) return g.four ? launch_inst<2, true>(with, g, smem, st) : launch_inst<2, false>(with, g, smem, st);
-    return launch_inst<1, true>(with, g, smem, st);
+    // whether the room holds every key: a slot's range here, what the caller says for sequences (of kept keys in front of a window it has one tile)
+    long long tiles = a.n_tiles > 0 && (a.window <= 0 || a.keep_first <= kKeys) ? a.n_tiles : (long long)1 << 40;
+    if (a.rows_per_slot > 0) {
+        tiles = 0;
+        for (int slot = 0; slot * a.rows_per_slot < a.M; ++slot) tiles += (std::max(range_keys(a, slot), 0) + kKeys - 1) / kKeys;
+    }
+    return with.work && tiles <= g.cap_tiles ? launch_any<false>(with, g, smem, st) : launch_any<true>(with, g, smem, st);
 }
 
 }  // namespace dia

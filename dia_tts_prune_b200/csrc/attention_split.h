@@ -39,9 +39,10 @@ struct SplitAttention {
     // Optional (n_seq 0: not given): the step's sequences - slot, first row and row count of each
     const int* seq_slot; const int* seq_row0; const int* seq_count; int n_seq;
     // Optional, with the sequences or with rows_per_slot: room in which a launch in front splits the keys and values that the rows see once for
-    // all row tiles (null: every row tile splits them for itself, which takes several times as long).  n_slots: slots there are.  Keys beyond the
+    // all row tiles (null: every row tile splits them for itself, which takes about twice as long).  n_slots: slots there are.  Keys beyond the
     // room's size are split by the row tiles.
     void* work; size_t work_bytes; int n_slots;
+    long long n_tiles;                                        // with the sequences: no more tiles of 64 keys than this are seen (0: not known)
 };
 
 // Whether the kernel takes the shape; M does not matter.  Channel counts and strides that are multiples of 4 on 16-byte aligned pointers, values

@@ -254,7 +254,9 @@ StepView view(const int32_t* step, int M, int n_seq) {
 // precision of the products: its error against 64 bits is not above that of the fp32 FMA kernels (attention_split.cu).
 struct SplitUse { lm::SplitRoom room; bool use; operator const lm::SplitRoom*() const { return use ? &room : nullptr; } };
 SplitUse split_operands(const lm_b200_engine* e, const StepView& v, int M) {
-    return SplitUse{lm::SplitRoom{e->kv_split, e->kv_split_bytes, e->m.n_slots, v.sm, v.n_seq}, M > lm::kAttnRowsKernelMax};
+    // (a window that keeps the first keys has a tile of them beside its own)
+    const long long tiles = v.n_seq * (((long long)e->m.max_pages * e->m.page_size + 63) / 64 + 1);
+    return SplitUse{lm::SplitRoom{e->kv_split, e->kv_split_bytes, e->m.n_slots, v.sm, v.n_seq, tiles}, M > lm::kAttnRowsKernelMax};
 }
 
 // columns of the stacked projections of a parallel record

@@ -68,8 +68,9 @@ cudaError_t launch_router_rows(const float* h, int D, const void* Wr, int E, int
 cudaError_t launch_qk_norm_cache(float* qk, int nq, int nk, const float* qw, const float* kw, float eps, float* kcache,
                                  float* vcache, const PageMap& pm, int kv_heads, int dim, const RowMeta& rm, int M,
                                  cudaStream_t st);
-// What the tensor-core attention with split operands is given: room for keys and values split in advance, and the step's sequences
-struct SplitRoom { void* work; size_t bytes; int n_slots; SeqMeta sm; int n_seq; };
+// What the tensor-core attention with split operands is given: room for keys and values split in advance, the step's sequences, and how many tiles of 64
+// keys they can have
+struct SplitRoom { void* work; size_t bytes; int n_slots; SeqMeta sm; int n_seq; long long n_tiles; };
 // ldo: row stride of the output (0: heads * dim); out_scale multiplies it, and so does the sigmoid of gate[row * ldg + column],
 // if given.  split: steps of more than kAttnRowsKernelMax rows run on the split-operand kernel where it takes the shape
 cudaError_t launch_sink_attention(const float* qk, int q_stride, const float* kcache, const float* vcache, const PageMap& pm,

@@ -168,6 +168,39 @@ def test_keys_beyond_the_room(H, G, d, window):
     close(got, ref, ref.abs().max().item())
 
 
+@pytest.mark.parametrize("kind,window", [("latent", 0), ("latent_narrow", 0), ("latent_widest", 0), ("talk", 0), ("grouped", 0), ("grouped", 700)])
+def test_keys_beyond_the_room_have_the_same_bits(kind, window):
+    """Keys that the room holds (all, with 1024 rows a step) and keys that it does not (with 64 rows the last seven tiles of 527): split by a launch in front, or by
+    the row tiles that walk them.  The caches are filled with numbers, not by steps."""
+    from dia_tts_prune_b200 import synthetic as SY
+    from dia_tts_prune_b200.lm_config import FipadraConfig, KupelixConfig, PubopelConfig
+    from dia_tts_prune_b200.lm_model import CausalLM
+    if kind == "talk":
+        cfg = SY.kupelix_config(width=64, kinds=["attention"], heads=4, kv_heads=2, dim=72, vdim=100, ff=32, vocab=64)
+        conf, w = KupelixConfig, SY.kupelix_weights(cfg, 5)
+    elif kind == "grouped":
+        cfg = SY.pubopel_config(width=64, layers=1, heads=4, kv_heads=2, dim=64, experts=1, top=1, expert_ff=8, shared_ff=None, vocab=64, window=window or None,
+                                keep_first=4 if window else 0, softcap=30.0)
+        conf, w = PubopelConfig, SY.pubopel_weights(cfg, 5)
+    else:
+        rank, rot = {"latent": (256, 32), "latent_narrow": (64, 16), "latent_widest": (256, 64)}[kind]
+        cfg = SY.fipadra_config(width=64, kinds=["latent_attention"], heads=4, dim=32, vdim=32, vocab=64, q_rank=48, kv_rank=rank, rot_dim=rot)
+        conf, w = FipadraConfig, SY.fipadra_weights(cfg, 5)
+    past, x = (32900, 700), torch.randn(40, 64, generator=torch.Generator().manual_seed(6)).cuda()
+    got = []
+    for rows in (64, 1024):
+        model = CausalLM(conf.model_validate(cfg), w, dtype="float32", device="cuda:0", max_tokens=33800, max_sequences=2, max_sequence_tokens=33024, page_size=64, max_rows=rows)
+        seqs = [model.state.open(n) for n in "ab"]
+        for q, n in zip(seqs, past):
+            model.state.reserve(q, n + 20)
+        g = torch.Generator().manual_seed(7)
+        for t in (model.state.k_pages[0], model.state.v_pages[0], model.state.latent_pages[0]):
+            if t is not None:
+                t.copy_(torch.randn(t.shape, generator=g))
+        got.append(model.engine.op_mixer(0, x, [(q, 20, n) for q, n in zip(seqs, past)]).clone())
+    assert torch.isfinite(got[0]).all() and torch.equal(*got)
+
+
 @pytest.mark.parametrize("place", [3, 20, 45, 63])
 def test_denominators_are_summed_per_16_keys(place):
     """One key of weight one and, in every tile of 64, one of 2^-25: half a unit in the last place of a sum with the first, so 64 of them are lost from a sum per
