@@ -64,6 +64,7 @@ _SIGNATURES = {
     "dia_b200_error_string": (C.c_char_p, [_i]),
     "dia_b200_last_cuda_error": (C.c_char_p, []),
     "dia_b200_launch_count": (C.c_int64, []),
+    "dia_b200_trim": (C.c_int, []),
     "dia_b200_engine_create": (_i, [C.POINTER(Shape), _i, _i, C.POINTER(_vp)]),
     "dia_b200_engine_destroy": (_i, [_vp]),
     "dia_b200_engine_num_ctas": (_i, [_vp]),

@@ -6,6 +6,7 @@
 #include <atomic>
 #include <cstdio>
 #include <cstring>
+#include <mutex>
 #include <new>
 #include <string>
 #include <utility>
@@ -202,6 +203,62 @@ int check_sampling_supported(float temperature, int top_k) {
     if (temperature < 0.0f) return DIA_B200_EINVAL;
     (void)top_k;      // <= 0: no top-k filter (dia/model.py:43-50); 1..64: fused candidate list; wider: full-vocabulary path
     return DIA_B200_OK;
+}
+
+}  // namespace
+
+namespace {
+
+// Room for calls that bring none: from a pool per device, in the order of the call's stream.  The pool keeps at most kLentMost bytes behind a synchronisation
+// (asked of the driver anew, room takes 210 us and more) until dia_b200_trim or the end of an engine, and a stream is not made to wait for what
+// another has freed.
+constexpr size_t kLentMost = (size_t)64 << 20;
+std::mutex lent_lock;
+cudaMemPool_t lent_pools[64] = {};
+
+cudaMemPool_t lent_pool(int dev) {
+    if (dev < 0 || dev >= 64) return nullptr;
+    const std::lock_guard<std::mutex> hold(lent_lock);
+    if (!lent_pools[dev]) {
+        cudaMemPoolProps props = {};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = dev;
+        cudaMemPool_t pool = nullptr;
+        unsigned long long most = kLentMost;
+        int no = 0;
+        if (cudaMemPoolCreate(&pool, &props) != cudaSuccess || cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &most) != cudaSuccess ||
+            cudaMemPoolSetAttribute(pool, cudaMemPoolReuseAllowInternalDependencies, &no) != cudaSuccess) {
+            (void)cudaGetLastError();
+            if (pool) (void)cudaMemPoolDestroy(pool);
+            return nullptr;
+        }
+        lent_pools[dev] = pool;
+    }
+    return lent_pools[dev];
+}
+
+// (null: nothing is asked for, there is none, or the stream is being captured - a graph would own the memory)
+void* lend(size_t bytes, cudaStream_t st) {
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    int dev = 0;
+    if (bytes == 0 || cudaStreamIsCapturing(st, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone || cudaGetDevice(&dev) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return nullptr;
+    }
+    void* p = nullptr;
+    const cudaMemPool_t pool = lent_pool(dev);
+    if (pool && cudaMallocFromPoolAsync(&p, bytes, pool, st) != cudaSuccess) {
+        (void)cudaGetLastError();
+        p = nullptr;
+    }
+    return p;
+}
+
+cudaError_t give_back(int dev) {
+    if (dev < 0 || dev >= 64) return cudaSuccess;
+    const std::lock_guard<std::mutex> hold(lent_lock);
+    return lent_pools[dev] ? cudaMemPoolTrimTo(lent_pools[dev], 0) : cudaSuccess;
 }
 
 }  // namespace
@@ -444,6 +501,7 @@ int dia_b200_engine_destroy(dia_b200_engine* e) {
     if (!e) return DIA_B200_OK;
     DeviceGuard _guard(e->device);
     cudaDeviceSynchronize();
+    (void)give_back(e->device);
     void* dev[] = {e->d_wstream, e->d_tab, e->d_emb, e->d_norms, e->d_rope_sin, e->d_rope_cos, e->d_ptrs, e->d_x,
                    e->d_logits, e->d_ll, e->d_pred, e->d_tokens, e->d_gs, e->d_timing, e->d_cta_timing, e->d_bll};
     for (void* p : dev) if (p) cudaFree(p);
@@ -1038,17 +1096,9 @@ int dia_b200_dense_forward(const float* x, const void* wt_bf16, float* y, void* 
     return dia_b200_dense_forward_fused(x, nullptr, 0.f, wt_bf16, nullptr, y, workspace, M, N, K, stream);
 }
 
-int dia_b200_attention_rows(const float* q, const float* k, const float* v, float* out, int B, int Tq, int Tk, int Hq, int Hkv,
-                            int Tk_stride, int mode, const int32_t* n_valid_host, void* stream) {
-    return dia_b200_attention_rows_in(q, k, v, out, B, Tq, Tk, Hq, Hkv, Tk_stride, mode, n_valid_host, nullptr, 0, stream);
-}
-
-size_t dia_b200_attention_rows_work_bytes(int B, int Tq, int Tk, int Hq, int Hkv, int mode, const int32_t* n_valid_host) {
-    return B > 0 && Tq > 0 && Tk >= 0 && mode >= 0 && mode <= 2 ? attention_rows_work_bytes(B, Tq, Tk, Hq, Hkv, mode, n_valid_host) : 0;
-}
-
-int dia_b200_attention_rows_in(const float* q, const float* k, const float* v, float* out, int B, int Tq, int Tk, int Hq, int Hkv,
-                               int Tk_stride, int mode, const int32_t* n_valid_host, void* work, size_t work_bytes, void* stream) {
+namespace {
+int attention_rows(const float* q, const float* k, const float* v, float* out, int B, int Tq, int Tk, int Hq, int Hkv, int Tk_stride, int mode,
+                   const int32_t* n_valid_host, void* work, size_t work_bytes, bool alone, void* stream) {
     if (B < 0 || Tq < 0 || Tk < 0 || Hq <= 0 || Hkv <= 0 || Hq % Hkv || Tk > Tk_stride || mode < 0 || mode > 2 || B > 16)
         return DIA_B200_EINVAL;
     if (B == 0 || Tq == 0) return DIA_B200_OK;
@@ -1058,9 +1108,36 @@ int dia_b200_attention_rows_in(const float* q, const float* k, const float* v, f
         return DIA_B200_EINVAL;
     if (n_valid_host)
         for (int b = 0; b < B; ++b) if (n_valid_host[b] < 0 || n_valid_host[b] > Tk) return DIA_B200_EINVAL;
-    CK(launch_attention_rows(q, k, v, out, B, Tq, Tk, Hq, Hkv, Tk_stride, mode, n_valid_host, work, work_bytes, S(stream)));
+    CK(launch_attention_rows(q, k, v, out, B, Tq, Tk, Hq, Hkv, Tk_stride, mode, n_valid_host, work, work_bytes, alone, S(stream)));
     g_launches += 1 + std::exchange(extra_launches(), 0);
     return DIA_B200_OK;
+}
+}  // namespace
+
+int dia_b200_attention_rows(const float* q, const float* k, const float* v, float* out, int B, int Tq, int Tk, int Hq, int Hkv,
+                            int Tk_stride, int mode, const int32_t* n_valid_host, void* stream) {
+    const bool sizes_ok = B > 0 && B <= 16 && Tq > 0 && Tk >= 0 && Hkv > 0 && Hq > 0 && mode >= 0 && mode <= 2;
+    const size_t need = sizes_ok ? attention_rows_work_bytes(B, Tq, Tk, Hq, Hkv, mode, n_valid_host) : 0;
+    void* const work = lend(need, S(stream));
+    const int rc = attention_rows(q, k, v, out, B, Tq, Tk, Hq, Hkv, Tk_stride, mode, n_valid_host, work, work ? need : 0, !work, stream);
+    if (work) CK(cudaFreeAsync(work, S(stream)));             // (stream-ordered: behind the kernels)
+    return rc;
+}
+
+int dia_b200_trim(void) {
+    int dev = 0;
+    CK(cudaGetDevice(&dev));
+    CK(give_back(dev));
+    return DIA_B200_OK;
+}
+
+size_t dia_b200_attention_rows_work_bytes(int B, int Tq, int Tk, int Hq, int Hkv, int mode, const int32_t* n_valid_host) {
+    return B > 0 && Tq > 0 && Tk >= 0 && mode >= 0 && mode <= 2 ? attention_rows_work_bytes(B, Tq, Tk, Hq, Hkv, mode, n_valid_host) : 0;
+}
+
+int dia_b200_attention_rows_in(const float* q, const float* k, const float* v, float* out, int B, int Tq, int Tk, int Hq, int Hkv,
+                               int Tk_stride, int mode, const int32_t* n_valid_host, void* work, size_t work_bytes, void* stream) {
+    return attention_rows(q, k, v, out, B, Tq, Tk, Hq, Hkv, Tk_stride, mode, n_valid_host, work, work_bytes, false, stream);
 }
 
 namespace {
@@ -1096,7 +1173,7 @@ int rows_dense(const dia_b200_dense_ref& w, const float* x, const float* norm, f
 
 int rows_attention(const float* q, const float* k, const float* v, float* out, int B, int Tq, int Tk, int Hq, int Hkv, int slots, int mode,
                    const int32_t* n_valid, void* work, size_t work_bytes, cudaStream_t st) {
-    CK(launch_attention_rows(q, k, v, out, B, Tq, Tk, Hq, Hkv, slots, mode, n_valid, work, work_bytes, st));
+    CK(launch_attention_rows(q, k, v, out, B, Tq, Tk, Hq, Hkv, slots, mode, n_valid, work, work_bytes, false, st));
     g_launches += 1 + std::exchange(extra_launches(), 0);
     return DIA_B200_OK;
 }

@@ -294,9 +294,9 @@ cudaError_t launch_gemm_tcgen05(const float* x, const float* norm_w, float eps, 
 
 // the rest of the T > 1 passes (prefill_kernels.cu)
 size_t attention_rows_work_bytes(int B, int Tq, int Tk, int Hq, int Hkv, int mode, const int* n_valid_host);
-// (work: null, or that many bytes)
+// (work: null, or that many bytes; alone: there was none to be had, and the tensor cores are worth it from more rows on)
 cudaError_t launch_attention_rows(const float* q, const float* k, const float* v, float* out, int B, int Tq, int Tk, int Hq,
-                                  int Hkv, int Tk_stride, int mode, const int* n_valid_host, void* work, size_t work_bytes, cudaStream_t st);
+                                  int Hkv, int Tk_stride, int mode, const int* n_valid_host, void* work, size_t work_bytes, bool alone, cudaStream_t st);
 cudaError_t launch_rope_rows(const float* src, float* dst, const float* sin_tab, const float* cos_tab, const int* pos, int B,
                              int T, int H, int rotate, int to_cache, int dst_T, int dst_t0, int n_pos, cudaStream_t st);
 cudaError_t launch_head_rows(const float* q, int ldq, const float* k, const float* v, int ldkv, float* q_out, float* k_cache, float* v_cache,

@@ -37,7 +37,9 @@ constexpr int kAttnThreads = 256;
 // Queries of a batch row from which the attention runs on the tensor cores: its CTAs own 128 (query, head) rows, and a launch in front splits
 // the keys.  us a layer, this kernel / the tensor cores, 16 heads of 128: one text of 100 17 / 21, 129 23 / 23, 200 31 / 27, 255 31 / 28; two prompts (4 key
 // heads) and their cross attention over 129 bytes 70 40 / 51, 128 42 / 50, 200 90 / 54.
-constexpr int kSplitRowsMin = 160;
+// Without room (the stream is captured) each CTA splits the keys it walks: one text of 160 25 / 35, 200 31 / 41, 256 32 / 42, two prompts' cross attention over 129
+// bytes 200 41 / 54, their self attention 200 52 / 47, 250 54 / 48 and 400 108 / 68, 861 304 / 120.
+constexpr int kSplitRowsMin = 160, kSplitRowsAloneMin = 256;
 // AQ: queries per CTA, 64, or 32 where those leave SMs without a CTA (16 heads, one text of 200: 64 CTAs 42 us, 112 31)
 template <int AQ>
 constexpr int kAttnSmem = (AQ * kQStride + kAK * kQStride + kAK * kHeadDim + AQ * kPStride) * 4;
@@ -301,7 +303,7 @@ __global__ void embed_rows_kernel(const float* __restrict__ table, const int* __
 // ---- launchers ------------------------------------------------------------------------------------------------
 static int grid_for(long long n, int block) { return (int)std::min<long long>((n + block - 1) / block, 148 * 16); }
 
-static bool on_tensor_cores(int B, int Tq) { return B <= 16 && Tq >= kSplitRowsMin; }
+static bool on_tensor_cores(int B, int Tq, int rows_min) { return B <= 16 && Tq >= rows_min; }
 static SplitAttention split_rows(const float* q, const float* k, const float* v, float* out, int B, int Tq, int Tk, int Hq, int Hkv, int Tk_stride, int mode,
                                  const int* n_valid_host) {
     SplitAttention s{};
@@ -317,7 +319,7 @@ static SplitAttention split_rows(const float* q, const float* k, const float* v,
 
 // room in which launch_attention_rows splits the keys for all rows (0: it has no use for any)
 size_t attention_rows_work_bytes(int B, int Tq, int Tk, int Hq, int Hkv, int mode, const int* n_valid_host) {
-    if (!on_tensor_cores(B, Tq) || Hkv <= 0 || Hq % Hkv) return 0;
+    if (!on_tensor_cores(B, Tq, kSplitRowsMin) || Hkv <= 0 || Hq % Hkv) return 0;
     float* const some = reinterpret_cast<float*>(256);        // (only alignment is looked at)
     const SplitAttention s = split_rows(some, some, some + 64, some, B, Tq, Tk, Hq, Hkv, Tk, mode, n_valid_host);
     int keys = 0;
@@ -326,8 +328,8 @@ size_t attention_rows_work_bytes(int B, int Tq, int Tk, int Hq, int Hkv, int mod
 }
 
 cudaError_t launch_attention_rows(const float* q, const float* k, const float* v, float* out, int B, int Tq, int Tk, int Hq,
-                                  int Hkv, int Tk_stride, int mode, const int* n_valid_host, void* work, size_t work_bytes, cudaStream_t st) {
-    if (on_tensor_cores(B, Tq)) {                              // the tensor-core kernel with split fp32 operands
+                                  int Hkv, int Tk_stride, int mode, const int* n_valid_host, void* work, size_t work_bytes, bool alone, cudaStream_t st) {
+    if (on_tensor_cores(B, Tq, alone ? kSplitRowsAloneMin : kSplitRowsMin)) {                              // the tensor-core kernel with split fp32 operands
         SplitAttention s = split_rows(q, k, v, out, B, Tq, Tk, Hq, Hkv, Tk_stride, mode, n_valid_host);
         s.work = work; s.work_bytes = work ? work_bytes : 0;
         if (split_attention_ok(s)) return launch_split_attention(s, st);

@@ -291,8 +291,10 @@ int dia_b200_rows_layer_forward(const dia_b200_rows_layer *a, void *stream);
  * n_valid_host: int32 [B] in HOST memory (may be NULL = Tk).  B <= 16. */
 int dia_b200_attention_rows(const float *q, const float *k, const float *v, float *out, int B, int Tq, int Tk, int Hq,
                             int Hkv, int Tk_stride, int mode, const int32_t *n_valid_host, void *stream);
-/* The same with room in device memory, where the keys and values are prepared once for all queries (without it every 128 rows prepare them for
- * themselves, several times as long): dia_b200_attention_rows_work_bytes of these sizes, 0 where it has no use for any; 16-byte aligned. */
+/* The same with the caller's room in device memory, where the keys and values are prepared once for all queries: dia_b200_attention_rows_work_bytes of these
+ * sizes, 0 where it has no use for any; 16-byte aligned.  Less room, or NULL, is taken as far as it goes: every 128 rows prepare the other keys for
+ * themselves, about twice as long from 256 rows on.  (dia_b200_attention_rows borrows the room for the call, in the order of its stream, from a pool that
+ * keeps at most 64 MB per device; while the stream is captured it goes without.) */
 size_t dia_b200_attention_rows_work_bytes(int B, int Tq, int Tk, int Hq, int Hkv, int mode, const int32_t *n_valid_host);
 int dia_b200_attention_rows_in(const float *q, const float *k, const float *v, float *out, int B, int Tq, int Tk, int Hq,
                                int Hkv, int Tk_stride, int mode, const int32_t *n_valid_host, void *work, size_t work_bytes, void *stream);
@@ -334,6 +336,8 @@ int dia_b200_debug_last_device_error(dia_b200_engine *e, int32_t *out, int n_wor
 /* words [4..7]: site-specific detail; [16 + 2*(block*10 + warp)]: (site, info) of every warp that was waiting */
 /* number of kernels this library has launched since load (for bench.py's gpu_launches) */
 int64_t dia_b200_launch_count(void);
+/* Gives back the memory that calls without room of their own have left in the current device's pool (so does dia_b200_engine_destroy). */
+int dia_b200_trim(void);
 
 #ifdef __cplusplus
 }

@@ -201,6 +201,31 @@ def test_keys_beyond_the_room_have_the_same_bits(kind, window):
     assert torch.isfinite(got[0]).all() and torch.equal(*got)
 
 
+@pytest.mark.parametrize("B,Tq,Hq,Hkv", [(1, 200, 16, 16), (2, 300, 4, 1)])
+def test_calls_without_room_borrow_it(B, Tq, Hq, Hkv):
+    """Their keys are split by a launch in front like those of calls that bring room; during a capture they go without"""
+    from dia_tts_prune_b200 import _lib, engine as E
+    lib = _lib.load()
+    g = torch.Generator().manual_seed(Tq)
+    q, k, v = (torch.randn(s, generator=g).cuda() for s in ((B, Tq, Hq, 128), (B, Hkv, 300, 128), (B, Hkv, 300, 128)))
+
+    def call(out):
+        before = lib.dia_b200_launch_count()
+        _lib.check(lib.dia_b200_attention_rows(*[t.data_ptr() for t in (q, k, v, out)], B, Tq, 300, Hq, Hkv, 300, 2, None, torch.cuda.current_stream().cuda_stream),
+                   "attention_rows")
+        return lib.dia_b200_launch_count() - before
+
+    want, out = E.attention_rows(q, k, v, 300, 2, None), torch.zeros_like(q)
+    assert call(out) == 2 and torch.equal(out, want)
+    side, graph, again = torch.cuda.Stream(), torch.cuda.CUDAGraph(), torch.zeros_like(q)
+    with torch.cuda.graph(graph, stream=side):
+        assert call(again) == 1
+    graph.replay()
+    torch.cuda.synchronize()
+    assert (again - want).abs().max() <= 2e-5 * want.abs().max()      # (200 rows: the fp32 kernel)
+    assert lib.dia_b200_trim() == 0 and call(out) == 2 and torch.equal(out, want)
+
+
 @pytest.mark.parametrize("place", [3, 20, 45, 63])
 def test_denominators_are_summed_per_16_keys(place):
     """One key of weight one and, in every tile of 64, one of 2^-25: half a unit in the last place of a sum with the first, so 64 of them are lost from a sum per
