@@ -82,6 +82,7 @@ _SIGNATURES = {
     "lm_b200_op_mixer": (_ci, [_vp, _ci, _vp, _vp, _ci, _ci, _vp, _vp]),
     "lm_b200_op_attention": (_ci, [_vp, _ci, _vp, _vp, _ci, _ci, _vp, _vp]),
     "lm_b200_op_mixer_kernels": (_ci, [_vp, _ci, _vp, _vp, _ci, _ci, _vp, _vp]),
+    "lm_b200_step_sizes": (_ci, [_vp, _vp, _vp, _ci]),
     "lm_b200_op_ff": (_ci, [_vp, _ci, _vp, _ci, _vp, _vp]),
     "lm_b200_op_token_input": (_ci, [_vp, _ci, _vp, _vp, _ci, _vp, _vp]),
     "lm_b200_op_linear": (_ci, [_vp, _vp, _vp, _ci, _ci, _ci, _vp]),

@@ -165,6 +165,14 @@ struct lm_b200_engine {
     size_t a_split_bytes;
     void* kv_split;                              // keys and values of a long step's attention, split for the tensor cores
     size_t kv_split_bytes;
+    // what lm_b200_step_sizes said of the next step; the shapes whose keys have to fit the room, and the rooms that have been made for larger steps since
+    // the engine's own (the last one is in use, the others may still be read)
+    std::vector<int> said_rows, said_first;
+    bool said = false;
+    struct KeyShape { dia::SplitAttention shape; int window, chunk, keep_first; };
+    std::vector<KeyShape> key_shapes;
+    std::vector<void*> rooms;
+    size_t room_refused = (size_t)-1;            // bytes that the device did not have
     // steps of a few rows are captured once per (rows, sequences, wanted) into a CUDA graph over these fixed buffers
     int32_t* step_static = nullptr;
     float* logits_static = nullptr;
@@ -238,9 +246,52 @@ struct StepView {
     lm::RowMeta rm;
     lm::SeqMeta sm;
     int n_seq;
+    lm::StepSizes sizes;
 };
-StepView view(const int32_t* step, int M, int n_seq) {
+
+// A larger room for the split keys of this step.  What it replaces is freed behind all that reads it, or with the engine
+void grow_room(lm_b200_engine* e, size_t bytes, cudaStream_t st) {
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (bytes >= e->room_refused || cudaStreamIsCapturing(st, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) {
+        (void)cudaGetLastError();
+        return;
+    }
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;       // (another thread may be capturing: this one's memory is its own)
+    (void)cudaThreadExchangeStreamCaptureMode(&mode);
+    void* room = nullptr;
+    if (cudaMalloc(&room, bytes) != cudaSuccess) {
+        (void)cudaGetLastError();
+        e->room_refused = bytes;
+    } else {
+        if (!e->rooms.empty() && cudaDeviceSynchronize() == cudaSuccess) {
+            (void)cudaFree(e->rooms.back());
+            e->rooms.pop_back();
+        }
+        (void)cudaGetLastError();
+        e->rooms.push_back(room);
+        e->kv_split = room;
+        e->kv_split_bytes = bytes;
+    }
+    (void)cudaThreadExchangeStreamCaptureMode(&mode);
+}
+
+// The step's arrays, and what the host has said of it.  A long step whose keys are known not to fit gets room for them, a quarter more than they need
+StepView view(lm_b200_engine* e, const int32_t* step, int M, int n_seq, cudaStream_t st) {
     StepView v;
+    v.sizes = lm::StepSizes{nullptr, nullptr, 0};
+    if (e->said && (int)e->said_rows.size() == n_seq) {
+        long long rows = 0;
+        for (int n : e->said_rows) rows += n;
+        if (rows == M) v.sizes = lm::StepSizes{e->said_rows.data(), e->said_first.data(), n_seq};
+    }
+    e->said = false;
+    if (M > lm::kAttnRowsKernelMax && v.sizes.n > 0) {
+        size_t need = 0;
+        for (const auto& k : e->key_shapes)
+            need = std::max(need, dia::split_attention_work_bytes(k.shape, 64 * (int)std::min<long long>(lm::step_tiles(v.sizes, k.window, k.chunk, k.keep_first), 65535)));
+        if (need > e->kv_split_bytes) grow_room(e, need + need / 4, st);
+        if (need > e->kv_split_bytes) grow_room(e, need, st);
+    }
     v.token = step;
     v.rm = lm::RowMeta{step + M, step + 2 * (size_t)M, step + 3 * (size_t)M};
     const int32_t* s = step + 4 * (size_t)M;
@@ -255,8 +306,8 @@ StepView view(const int32_t* step, int M, int n_seq) {
 struct SplitUse { lm::SplitRoom room; bool use; operator const lm::SplitRoom*() const { return use ? &room : nullptr; } };
 SplitUse split_operands(const lm_b200_engine* e, const StepView& v, int M) {
     // (a window that keeps the first keys has a tile of them beside its own)
-    const long long tiles = v.n_seq * (((long long)e->m.max_pages * e->m.page_size + 63) / 64 + 1);
-    return SplitUse{lm::SplitRoom{e->kv_split, e->kv_split_bytes, e->m.n_slots, v.sm, v.n_seq, tiles}, M > lm::kAttnRowsKernelMax};
+    const long long most = v.n_seq * (((long long)e->m.max_pages * e->m.page_size + 63) / 64 + 1);
+    return SplitUse{lm::SplitRoom{e->kv_split, e->kv_split_bytes, e->m.n_slots, v.sm, v.n_seq, v.sizes, most}, M > lm::kAttnRowsKernelMax};
 }
 
 // columns of the stacked projections of a parallel record
@@ -1042,11 +1093,12 @@ int lm_b200_engine_create(const lm_b200_model* model, const lm_b200_layer* layer
     const size_t R = (size_t)m.max_rows, D = (size_t)m.width;
     size_t qk = 0, att = 0, E = 1, top = 1, F = 1, Sf = 1, slots = 1;
     size_t n_in = 0, k_out = 0, n_rec = 0, split_dim = 0, kv_split = 0, delta = 0;
-    // room for the split keys and values of twice a step's rows and 32768 cached keys more, as far as sequences can have them (and a partly filled
-    // tile at either end of every sequence); what does not fit is split where it is used, by few registers
+    // Room for the split keys and values of twice a step's rows and 32768 cached keys more, as far as sequences can have them (and a partly filled
+    // tile at either end of every sequence).  A step that is known to need more gets it (see grow_room); else what does not fit is split where it is used, in
+    // up to four times the time (us, 12 sequences over 4096 keys, row tiles / room: 4 heads 597 / 279, latent rows 1950 / 520; 64 over 1500 407 / 358 and 886 / 398)
     const long long cached = std::min<long long>(32768, (long long)m.n_slots * m.max_pages * m.page_size);
     const long long split_keys = std::min<long long>(2LL * m.max_rows + cached + 192LL * m.n_slots, 64LL * 65535);
-    auto split_room = [&](int heads, int kv_heads, int kdim, int vdim, bool latent, const float* talk) {
+    auto split_room = [&](int heads, int kv_heads, int kdim, int vdim, bool latent, const float* talk, int window, int chunk, int keep_first) {
         dia::SplitAttention s{};
         float* const some = reinterpret_cast<float*>(256);        // (only whether keys and values are one buffer, and alignment, are looked at)
         s.q = s.out = some;
@@ -1054,7 +1106,13 @@ int lm_b200_engine_create(const lm_b200_model* model, const lm_b200_layer* layer
         s.vcache = latent ? some : some + 64;
         s.heads = heads; s.kv_heads = kv_heads; s.qdim = s.kdim = kdim; s.vdim = vdim; s.vrow = latent ? kdim : vdim; s.talk = talk;
         s.n_slots = m.n_slots;
-        kv_split = std::max(kv_split, dia::split_attention_work_bytes(s, (int)split_keys));
+        const size_t bytes = dia::split_attention_work_bytes(s, (int)split_keys);
+        kv_split = std::max(kv_split, bytes);
+        auto same = [&](const lm_b200_engine::KeyShape& k) {
+            return k.shape.heads == heads && k.shape.kv_heads == kv_heads && k.shape.kdim == kdim && k.shape.vdim == vdim && k.shape.vcache == s.vcache &&
+                   k.window == window && k.chunk == chunk && k.keep_first == keep_first;
+        };
+        if (bytes > 0 && std::none_of(e->key_shapes.begin(), e->key_shapes.end(), same)) e->key_shapes.push_back({s, window, chunk, keep_first});
     };
     size_t n_streams = 0, n_lat = 0, q_rank = 0, n_heads = 0, n_side = 0, n_second = 0, olat_room = 0, qlat_room = 0;
     bool pre = false, any_parallel = false;
@@ -1076,12 +1134,12 @@ int lm_b200_engine_create(const lm_b200_model* model, const lm_b200_layer* layer
                     olat_room = std::max(olat_room, dia::gemm_f32_work_bytes(R, (size_t)p.heads * p.dim));
                     qlat_room = std::max(qlat_room, dia::gemm_f32_work_bytes(R, (size_t)p.heads * p.kv_rank));
                     if (lm::talk_attention_supported(latent_shape(p))) split_dim = std::max(split_dim, (size_t)p.heads * (p.kv_rank + 2));
-                    split_room(p.heads, 1, p.kv_rank + p.rot_dim, p.kv_rank, true, nullptr);
+                    split_room(p.heads, 1, p.kv_rank + p.rot_dim, p.kv_rank, true, nullptr, p.window, 0, 0);
                 } else if (p.mixer == LM_B200_MIXER_MLSTM) {
                     n_lat = std::max(n_lat, (size_t)p.heads * (p.vdim + 1));
                 } else if (p.mixer == LM_B200_MIXER_ROTARY_ATTENTION) {
                     split_dim = std::max(split_dim, (size_t)p.heads * (p.dim + 2));
-                    split_room(p.heads, p.kv_heads, p.dim, p.dim, false, nullptr);
+                    split_room(p.heads, p.kv_heads, p.dim, p.dim, false, nullptr, p.window, p.chunk, 0);
                 }
                 n_rec = std::max(n_rec, (size_t)stream_rec_cols(p));
             }
@@ -1105,14 +1163,14 @@ int lm_b200_engine_create(const lm_b200_model* model, const lm_b200_layer* layer
             pre = pre || l.w_pre;
             if (l.mixer == LM_B200_MIXER_TALK_ATTENTION) {
                 split_dim = std::max(split_dim, (size_t)l.heads * (l.vdim + 2));
-                split_room(l.heads, l.kv_heads, l.dim, l.vdim, false, l.talk);
+                split_room(l.heads, l.kv_heads, l.dim, l.vdim, false, l.talk, 0, 0, 0);
             }
             continue;
         }
         qk = std::max(qk, (size_t)(l.heads + l.kv_heads) * l.dim);
         att = std::max(att, (size_t)l.heads * l.dim);
         split_dim = std::max(split_dim, (size_t)l.heads * (l.dim + 2));
-        split_room(l.heads, l.kv_heads, l.dim, l.dim, false, nullptr);
+        split_room(l.heads, l.kv_heads, l.dim, l.dim, false, nullptr, l.window, 0, l.keep_first);
         if (l.ff == LM_B200_FF_ROUTED_EXPERTS) {
             E = std::max(E, (size_t)l.experts);
             top = std::max(top, (size_t)l.top);
@@ -1200,11 +1258,24 @@ int lm_b200_engine_destroy(lm_b200_engine* e) {
     for (auto& kv : e->graphs) cudaGraphExecDestroy(kv.second.exec);
     if (e->capture_stream) cudaStreamDestroy(e->capture_stream);
     if (e->arena) cudaFree(e->arena);
+    for (void* room : e->rooms) cudaFree(room);
     delete e;
     return LM_B200_OK;
 }
 
-size_t lm_b200_engine_workspace_bytes(const lm_b200_engine* e) { return e ? e->arena_bytes : 0; }
+size_t lm_b200_engine_workspace_bytes(const lm_b200_engine* e) { return e ? e->arena_bytes + (e->rooms.empty() ? 0 : e->kv_split_bytes) : 0; }
+
+int lm_b200_step_sizes(lm_b200_engine* e, const int32_t* rows, const int32_t* first, int n_seq) {
+    if (!e) return LM_B200_EINVAL;
+    e->said = false;
+    if (!rows || !first || n_seq <= 0) return LM_B200_EINVAL;
+    for (int s = 0; s < n_seq; ++s)
+        if (rows[s] <= 0 || first[s] < 0 || rows[s] > e->m.max_rows || (long long)first[s] + rows[s] > (long long)e->m.max_pages * e->m.page_size) return LM_B200_EINVAL;
+    e->said_rows.assign(rows, rows + n_seq);
+    e->said_first.assign(first, first + n_seq);
+    e->said = true;
+    return LM_B200_OK;
+}
 
 }  // extern "C"
 
@@ -1332,7 +1403,7 @@ int run_stream_layers(lm_b200_engine* e, const StepView& v, int M, int n_seq, fl
 // the launch sequence of one step
 int run_step(lm_b200_engine* e, const int32_t* step, int M, int n_seq, int n_want, float* logits_out, float* layers_out,
              cudaStream_t st) {
-    const StepView v = view(step, M, n_seq);
+    const StepView v = view(e, step, M, n_seq, st);
     const int D = e->m.width;
     if (e->stream_form) {
         const int rc = run_stream_layers(e, v, M, n_seq, layers_out, st);
@@ -1443,6 +1514,7 @@ int lm_b200_forward(lm_b200_engine* e, const int32_t* step, int M, int n_seq, in
     Guard g(e->device);
     if (!g.ok) return LM_B200_ECUDA;
     if (dia::take_ran_out(e->device, S(stream))) return cuda_fail(cudaErrorLaunchTimeout);
+    if (M <= lm::kRowsKernelMax) e->said = false;             // (nothing there depends on it, and a captured step reads another one's rows)
     if (e->m.step_graphs && M <= lm::kRowsKernelMax && !layers_out)
         return run_step_graph(e, step, M, n_seq, n_want, logits_out, S(stream));
     return run_step(e, step, M, n_seq, n_want, logits_out, layers_out, S(stream));
@@ -1456,7 +1528,7 @@ int lm_b200_op_norm_tapmix(lm_b200_engine* e, int layer, int sub, const float* x
     Guard g(e->device);
     if (!g.ok) return LM_B200_ECUDA;
     if (e->layers[layer].form != LM_B200_FORM_SEQUENTIAL) return LM_B200_EUNSUPPORTED;
-    return norm_tapmix(e, e->layers[layer], sub, x, view(step, M, n_seq), M, n_seq, out, S(stream));
+    return norm_tapmix(e, e->layers[layer], sub, x, view(e, step, M, n_seq, S(stream)), M, n_seq, out, S(stream));
 }
 
 int lm_b200_op_mixer(lm_b200_engine* e, int layer, const float* h, const int32_t* step, int M, int n_seq, float* y,
@@ -1466,16 +1538,16 @@ int lm_b200_op_mixer(lm_b200_engine* e, int layer, const float* h, const int32_t
     Guard g(e->device);
     if (!g.ok) return LM_B200_ECUDA;
     if (e->layers[layer].form == LM_B200_FORM_PARALLEL)
-        return parallel_layer(e, e->layers[layer], view(step, M, n_seq), M, n_seq, 1, h, y, S(stream));
+        return parallel_layer(e, e->layers[layer], view(e, step, M, n_seq, S(stream)), M, n_seq, 1, h, y, S(stream));
     if (e->layers[layer].form == LM_B200_FORM_STREAMS) {
         const void* hb = nullptr;
         if (e->m.precision == LM_B200_PRECISION_BF16 && M >= kTensorRowsMin) {
             LCK(lm::launch_pack_rows_bf16(h, e->hb, M, e->m.width, nullptr, S(stream)));
             hb = e->hb;
         }
-        return stream_mixer(e, e->layers[layer], h, hb, view(step, M, n_seq), M, n_seq, y, S(stream));
+        return stream_mixer(e, e->layers[layer], h, hb, view(e, step, M, n_seq, S(stream)), M, n_seq, y, S(stream));
     }
-    return mixer(e, e->layers[layer], h, nullptr, view(step, M, n_seq), M, y, nullptr, lm::TapOut{}, S(stream));
+    return mixer(e, e->layers[layer], h, nullptr, view(e, step, M, n_seq, S(stream)), M, y, nullptr, lm::TapOut{}, S(stream));
 }
 
 int lm_b200_op_attention(lm_b200_engine* e, int layer, float* qk, const int32_t* step, int M, int n_seq, float* out,
@@ -1486,7 +1558,7 @@ int lm_b200_op_attention(lm_b200_engine* e, int layer, float* qk, const int32_t*
     if (!g.ok) return LM_B200_ECUDA;
     const lm_b200_layer& l = e->layers[layer];
     if (l.form != LM_B200_FORM_SEQUENTIAL) return LM_B200_EUNSUPPORTED;
-    const StepView v = view(step, M, n_seq);
+    const StepView v = view(e, step, M, n_seq, S(stream));
     const int nq = l.heads * l.dim, nk = l.kv_heads * l.dim;
     const lm::PageMap pm{e->m.page_table, e->m.max_pages, e->m.page_size};
     LCK(lm::launch_qk_norm_cache(qk, nq, nk, l.q_norm, l.k_norm, e->m.eps, l.k_pages, l.v_pages, pm, l.kv_heads, l.dim, v.rm, M,
@@ -1506,13 +1578,13 @@ int lm_b200_op_mixer_kernels(lm_b200_engine* e, int layer, float* proj, const in
     Guard g(e->device);
     if (!g.ok) return LM_B200_ECUDA;
     if (l.form == LM_B200_FORM_STREAMS) {
-        const int rc = stream_mixers(e, l, proj, view(step, M, n_seq), M, n_seq, S(stream));
+        const int rc = stream_mixers(e, l, proj, view(e, step, M, n_seq, S(stream)), M, n_seq, S(stream));
         if (rc) return rc;
         if (cudaMemcpyAsync(out, e->att, (size_t)M * mix_out_cols(l) * 4, cudaMemcpyDeviceToDevice, S(stream)) != cudaSuccess)
             return cuda_fail(cudaGetLastError());
         return LM_B200_OK;
     }
-    const int rc = mixer_kernels(e, l, in_cols(l), proj, view(step, M, n_seq), M, n_seq, nullptr, S(stream));
+    const int rc = mixer_kernels(e, l, in_cols(l), proj, view(e, step, M, n_seq, S(stream)), M, n_seq, nullptr, S(stream));
     if (rc) return rc;
     const size_t w = (size_t)l.heads * l.vdim * 4;
     if (cudaMemcpy2DAsync(out, w, e->outcat, (size_t)l.k_out * 4, w, M, cudaMemcpyDeviceToDevice, S(stream)) != cudaSuccess)
@@ -1567,7 +1639,7 @@ int lm_b200_op_token_input(lm_b200_engine* e, int layer, const float* x, const i
         LCK(lm::launch_pack_rows_bf16(x, e->hb, M, e->m.width, nullptr, st));
         xb = e->hb;
     }
-    const int rc = token_input(e, l, x, xb, view(step, M, 1).token, M, e->y, st);
+    const int rc = token_input(e, l, x, xb, view(e, step, M, 1, st).token, M, e->y, st);
     if (rc) return rc;
     if (cudaMemcpyAsync(out, x, (size_t)M * e->m.width * 4, cudaMemcpyDeviceToDevice, st) != cudaSuccess) return cuda_fail(cudaGetLastError());
     const lm::StreamWrite wr{e->unit + 1, e->unit + 1, e->y, nullptr, nullptr, nullptr, 0};

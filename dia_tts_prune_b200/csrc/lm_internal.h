@@ -68,9 +68,23 @@ cudaError_t launch_router_rows(const float* h, int D, const void* Wr, int E, int
 cudaError_t launch_qk_norm_cache(float* qk, int nq, int nk, const float* qw, const float* kw, float eps, float* kcache,
                                  float* vcache, const PageMap& pm, int kv_heads, int dim, const RowMeta& rm, int M,
                                  cudaStream_t st);
-// What the tensor-core attention with split operands is given: room for keys and values split in advance, the step's sequences, and how many tiles of 64
-// keys they can have
-struct SplitRoom { void* work; size_t bytes; int n_slots; SeqMeta sm; int n_seq; long long n_tiles; };
+// What the host knows of a step's sequences (n 0: nothing): rows and first position of each
+struct StepSizes { const int *rows, *first; int n; };
+// tiles of 64 keys that their rows see under a mask (see SplitAttention), as the launch that splits them counts them
+inline long long step_tiles(const StepSizes& z, int window, int chunk, int keep_first) {
+    long long tiles = 0;
+    for (int s = 0; s < z.n; ++s) {
+        const int pos = z.first[s], from = std::max(window > 0 ? std::max(0, pos - window + 1) : 0, chunk > 0 ? pos - pos % chunk : 0) / 64;
+        tiles += (pos + z.rows[s] + 63) / 64 - from + (window > 0 && keep_first > 0 && from > 0 ? 1 : 0);
+    }
+    return tiles;
+}
+// What the tensor-core attention with split operands is given: room for keys and values split in advance, the step's sequences, what the host knows of
+// them, and how many tiles they can have where it knows nothing
+struct SplitRoom {
+    void* work; size_t bytes; int n_slots; SeqMeta sm; int n_seq; StepSizes sizes; long long most_tiles;
+    long long tiles(int window, int chunk, int keep_first) const { return sizes.n > 0 ? step_tiles(sizes, window, chunk, keep_first) : most_tiles; }
+};
 // ldo: row stride of the output (0: heads * dim); out_scale multiplies it, and so does the sigmoid of gate[row * ldg + column],
 // if given.  split: steps of more than kAttnRowsKernelMax rows run on the split-operand kernel where it takes the shape
 cudaError_t launch_sink_attention(const float* qk, int q_stride, const float* kcache, const float* vcache, const PageMap& pm,

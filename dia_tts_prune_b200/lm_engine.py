@@ -92,7 +92,7 @@ class LMEngine:
         n_rows = sum(len(t) for _, t, _, _ in parts)
         S = len(parts)
         want = [k for _, _, _, w in parts for k in w]
-        buf = np.empty(4 * n_rows + 3 * S + len(want), dtype=np.int32)
+        buf = np.empty(4 * n_rows + 3 * S + len(want) + S, dtype=np.int32)      # (the last S: the sequences' first positions, for the host alone)
         tok, slot, pos, start = (buf[i * n_rows:(i + 1) * n_rows] for i in range(4))
         meta, r0, at = buf[4 * n_rows:], 0, 0
         for s, (seq, tokens, p0, w) in enumerate(parts):
@@ -101,15 +101,23 @@ class LMEngine:
             slot[r0:r0 + n] = seq.slot
             pos[r0:r0 + n] = np.arange(p0, p0 + n, dtype=np.int32)
             start[r0:r0 + n] = p0
-            meta[s], meta[S + s], meta[2 * S + s] = seq.slot, r0, n
+            meta[s], meta[S + s], meta[2 * S + s], meta[s - S] = seq.slot, r0, n, p0
             for k in w:
                 meta[3 * S + at] = r0 + k
                 at += 1
             r0 += n
+        if n_rows > 8:                                          # (shorter steps have no use for it)
+            at = buf.__array_interface__["data"][0]
+            self._say(at + 4 * (4 * n_rows + 2 * S), at + 4 * (buf.size - S), S)
         t = torch.from_numpy(buf)
         if buf.size > 4096:                                     # a long step: asynchronous copy from pinned memory
             t = t.pin_memory()
         return t.to(self.device, non_blocking=True), n_rows, S, len(want)
+
+    def _say(self, rows: int, first: int, n: int) -> None:
+        """Tells the engine the sizes of the step that is packed, ``n`` int32 at either address (it takes them with the call that follows; what it
+        refuses it does not know)."""
+        self.lib.lm_b200_step_sizes(self._h, rows, first, n)
 
     def check(self) -> None:
         """Behind a synchronisation: raises if a wait of a kernel ran out since the last look (what it wrote is NaN)."""

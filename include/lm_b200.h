@@ -249,6 +249,11 @@ int lm_b200_engine_create(const lm_b200_model *model, const lm_b200_layer *layer
 int lm_b200_engine_destroy(lm_b200_engine *e);
 size_t lm_b200_engine_workspace_bytes(const lm_b200_engine *e);
 
+/* Optional, in front of a call with a step: what the host knows of it, rows and first position of each of its n_seq sequences (int32 in HOST memory, copied;
+ * the call that follows takes it, and none else).  It has to be that step's.  With it the call gets the room and the launches that the step needs: keys of more
+ * than max_rows rows and 32768 cached ones have no room in the engine's workspace until a step asks for it (lm_b200_engine_workspace_bytes counts it). */
+int lm_b200_step_sizes(lm_b200_engine *e, const int32_t *rows, const int32_t *first, int n_seq);
+
 /* Behind a synchronisation: LM_B200_ECUDA if a wait of a kernel ran out on the engine's device since the last look (its outputs are NaN). */
 int lm_b200_check(lm_b200_engine *e, void *stream);
 

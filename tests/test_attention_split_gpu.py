@@ -171,7 +171,7 @@ def test_keys_beyond_the_room(H, G, d, window):
 @pytest.mark.parametrize("kind,window", [("latent", 0), ("latent_narrow", 0), ("latent_widest", 0), ("talk", 0), ("grouped", 0), ("grouped", 700)])
 def test_keys_beyond_the_room_have_the_same_bits(kind, window):
     """Keys that the room holds (all, with 1024 rows a step) and keys that it does not (with 64 rows the last seven tiles of 527): split by a launch in front, or by
-    the row tiles that walk them.  The caches are filled with numbers, not by steps."""
+    the row tiles that walk them; an engine that is told the step's sizes gets room for them.  The caches are filled with numbers, not by steps."""
     from dia_tts_prune_b200 import synthetic as SY
     from dia_tts_prune_b200.lm_config import FipadraConfig, KupelixConfig, PubopelConfig
     from dia_tts_prune_b200.lm_model import CausalLM
@@ -187,8 +187,8 @@ def test_keys_beyond_the_room_have_the_same_bits(kind, window):
         cfg = SY.fipadra_config(width=64, kinds=["latent_attention"], heads=4, dim=32, vdim=32, vocab=64, q_rank=48, kv_rank=rank, rot_dim=rot)
         conf, w = FipadraConfig, SY.fipadra_weights(cfg, 5)
     past, x = (32900, 700), torch.randn(40, 64, generator=torch.Generator().manual_seed(6)).cuda()
-    got = []
-    for rows in (64, 1024):
+    got, more = [], []
+    for rows, told in ((64, False), (64, True), (1024, True)):
         model = CausalLM(conf.model_validate(cfg), w, dtype="float32", device="cuda:0", max_tokens=33800, max_sequences=2, max_sequence_tokens=33024, page_size=64, max_rows=rows)
         seqs = [model.state.open(n) for n in "ab"]
         for q, n in zip(seqs, past):
@@ -197,8 +197,14 @@ def test_keys_beyond_the_room_have_the_same_bits(kind, window):
         for t in (model.state.k_pages[0], model.state.v_pages[0], model.state.latent_pages[0]):
             if t is not None:
                 t.copy_(torch.randn(t.shape, generator=g))
+        if not told:
+            model.engine._say = lambda *sizes: None
+        bytes_of = lambda: model.engine.lib.lm_b200_engine_workspace_bytes(model.engine._h)
+        before = bytes_of()
         got.append(model.engine.op_mixer(0, x, [(q, 20, n) for q, n in zip(seqs, past)]).clone())
-    assert torch.isfinite(got[0]).all() and torch.equal(*got)
+        more.append(bytes_of() - before)
+    assert torch.isfinite(got[0]).all() and torch.equal(got[0], got[1]) and torch.equal(got[0], got[2])
+    assert more[0] == 0 and (more[1] > 0) == (window == 0) and more[2] == 0      # (a window's keys fit in any case)
 
 
 @pytest.mark.parametrize("B,Tq,Hq,Hkv", [(1, 200, 16, 16), (2, 300, 4, 1)])
