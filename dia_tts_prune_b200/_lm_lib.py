@@ -69,6 +69,7 @@ class Model(C.Structure):
 
 
 _ci = C.c_int
+_cf = C.c_float
 _SIGNATURES = {
     "lm_b200_abi_version": (_ci, []),
     "lm_b200_last_cuda_error": (C.c_char_p, []),
@@ -87,6 +88,7 @@ _SIGNATURES = {
     "lm_b200_op_token_input": (_ci, [_vp, _ci, _vp, _vp, _ci, _vp, _vp]),
     "lm_b200_op_linear": (_ci, [_vp, _vp, _vp, _ci, _ci, _ci, _vp]),
     "lm_b200_op_linear_tc": (_ci, [_vp, _vp, _vp, _vp, _ci, _ci, _ci, _vp]),
+    "lm_b200_op_gated_tc": (_ci, [_vp, _vp, _vp, _vp, _vp, _ci, _ci, _ci, _ci, _cf, _ci, _vp, _ci, _vp, _vp]),
     "lm_b200_argmax_rows": (_ci, [_vp, _ci, _ci, _vp, _vp]),
 }
 

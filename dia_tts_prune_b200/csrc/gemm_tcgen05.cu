@@ -528,7 +528,12 @@ __device__ __forceinline__ float glu_value(int kind, float g, float u, float lim
         return g * (1.0f / (1.0f + expf(-(1.702f * g)))) * (u + 1.0f);
     }
     if (kind == 2) return 0.5f * g * (1.0f + tanhf(0.7978845608028654f * fmaf(0.044715f * g * g, g, g))) * u;
-    return g / (1.0f + expf(-g)) * u;
+    // Zero divided by two is zero; the division's short way does not take it, and rows that are not there made the gate of their tile take 7 us more.  (The
+    // numerator is hidden, or the two selections become one again.)
+    float n = g == 0.f ? 1.f : g;
+    asm("" : "+f"(n));
+    const float q = n / (1.0f + expf(-g));
+    return (g == 0.f ? g : q) * u;
 }
 
 // How often a wait of the pair kernel looks at its barrier, in products that this thread launches.  With 0 each wait runs out before anything has
@@ -1463,8 +1468,23 @@ cudaError_t launch_gemm_tcgen05_bf16(const void* a_bf16, int terms, const void* 
     return cudaGetLastError();
 }
 
+// Whether product and gate are shorter one after the other: the gate of a tile takes eight warps 8 us, which a short k loop or a single round does not hide, and
+// its tiles are 256 columns wide, which leaves more pairs idle.  Estimates in us, fitted to 150 to 4096 rows of widths 512 to 2048 and hidden widths of 256 to 4096,
+// dense and grouped (within 2 us).  Measured, together / apart: 1030 rows, 512 -> 2048 26.9 / 24.8, 1024 -> 4096 39.2 / 37.2, 2048 -> 2048 37.2 / 39.2; 600 rows,
+// 2048 -> 1024 26.9 / 25.5; 3000 rows, 512 -> 1024 28.0 / 26.9, 2048 -> 2048 51.1 / 62.6; four experts of 256, width 2048, 260 rows 26.9 / 24.9, 2800 29.0 / 29.7
+static bool gate_apart(int M, int F, int K, int pairs) {
+    const int tiles_m = (M + 2 * BM - 1) / (2 * BM), bn = pair_columns(1, M, 2 * F, pairs);
+    const auto rounds = [&](int per_row) { return (int)(((long long)tiles_m * per_row + pairs - 1) / pairs); };
+    const double k_blocks = (K + BK - 1) / BK, wide = bn / 256.0, outputs = (double)M * F;
+    const double together = 12.0 + 0.3 * k_blocks + (rounds(F / 128) - 1) * std::max(0.34 * k_blocks, 8.3);
+    const double of_round = 0.3 * k_blocks * (700 + bn) / 956.0;
+    const double apart = 4.5 + 3.0 * wide + of_round + (rounds((2 * F + bn - 1) / bn) - 1) * std::max(of_round, 5.0 * wide) + 4.0 +
+                         outputs * (outputs > 7.5e6 ? 2.4e-6 : 1.5e-6);      // (the gate's pass; above, the products leave L2)
+    return apart + 0.6 < together;
+}
+
 cudaError_t launch_gemm_glu_bf16(const void* a_bf16, const void* wt, long long wt_rows, void* y_bf16, int M, int F, int K, int kind, float limit,
-                                 const GemmGroups* groups, cudaStream_t st) {
+                                 const GemmGroups* groups, cudaStream_t st, bool in_any_case) {
     if (M <= BM || F % 128 || F <= 0 || !gemm_tcgen05_shape_ok(M, 2 * F, K) || wt_rows < 2LL * F || kind < 0 || kind > 2 ||
         (reinterpret_cast<uintptr_t>(y_bf16) & 15) || (groups && groups->tile_rows % (2 * BM)))
         return cudaErrorNotSupported;
@@ -1472,6 +1492,10 @@ cudaError_t launch_gemm_glu_bf16(const void* a_bf16, const void* wt, long long w
     const cudaError_t e = current_sms(&dev, &sms);
     if (e != cudaSuccess) return e;
     if (!groups && wt_rows == 2LL * F && dense_rows_f32(1, M, 2 * F, K, sms)) return cudaErrorNotSupported;      // (fp32 sums stay: see there)
+    int pairs = 0;
+    const cudaError_t known = pairs_of<1, false, true>(dev, &pairs);
+    if (known != cudaSuccess) return known;
+    if (!in_any_case && gate_apart(M, F, K, pairs)) return cudaErrorNotSupported;
     CUtensorMap ma;
     if (!make_map(&ma, a_bf16, M, K, BM)) return cudaErrorNotSupported;
     PairProduct q{};

@@ -65,10 +65,10 @@ inline bool gemm_tcgen05_shape_ok(int M, int N, int K) { return M > 0 && N > 0 &
 cudaError_t launch_gemm_tcgen05_bf16(const void* a_bf16, int terms, const void* wt, long long wt_rows, float* y, int M, int N,
                                      int K, const GemmEpilogue& ep, const GemmGroups* groups, cudaStream_t st);
 // Yb[M][F] = bf16(glu(gate, up)) of [gate | up] = A[M][K] (bf16) . Wt[2 F][K]^T: the products of launch_gemm_tcgen05_bf16 with the gate in front of the bf16
-// rounding (kind: kGlu* of the language models).  cudaErrorNotSupported where that product would not run on pairs of SMs or F is no multiple of 128: the caller
-// then runs the product and the gate one after the other, to the same bits.
+// rounding (kind: kGlu* of the language models).  cudaErrorNotSupported where that product would not run on pairs of SMs, F is no multiple of 128 or (but for
+// in_any_case) the two are the shorter way: the caller then runs the product and the gate one after the other, to the same bits.
 cudaError_t launch_gemm_glu_bf16(const void* a_bf16, const void* wt, long long wt_rows, void* y_bf16, int M, int F, int K, int kind, float limit,
-                                 const GemmGroups* groups, cudaStream_t st);
+                                 const GemmGroups* groups, cudaStream_t st, bool in_any_case = false);
 
 // Per head h < heads: Y[m][h y_hs + n] = act(alpha sum_k A[m][h a_hs + k] W[h][n][k]) [* sigmoid of a gate column], as fp32 FMA
 // arithmetic gives it: A (fp32, row stride lda) is split into three bf16 terms (24 bits) in `work` (gemm_f32_work_bytes), every 64

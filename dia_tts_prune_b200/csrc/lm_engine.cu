@@ -1663,6 +1663,25 @@ int lm_b200_op_linear_tc(const float* A, const void* W_bf16, float* Y, void* a_b
     return LM_B200_OK;
 }
 
+int lm_b200_op_gated_tc(const float* A, const void* W_bf16, void* a_bf16, float* gate_up, void* y_bf16, int M, int F, int K, int act, float limit, int fused,
+                        const int32_t* row_group, int groups, const int32_t* n_rows, void* stream) {
+    if (!A || !W_bf16 || !a_bf16 || !y_bf16 || (!fused && !gate_up) || M <= 0 || F <= 0 || K <= 0 || (row_group && groups <= 0) ||
+        (act != LM_B200_ACT_SILU_GLU && act != LM_B200_ACT_CLAMPED_GLU && act != LM_B200_ACT_GELU_GLU))
+        return LM_B200_EINVAL;
+    if (!dia::gemm_tcgen05_shape_ok(M, 2 * F, K)) return LM_B200_EUNSUPPORTED;
+    const dia::GemmGroups g{row_group, 2 * F, n_rows, dia::kGemmPairRows};
+    const dia::GemmGroups* const gp = row_group ? &g : nullptr;
+    const long long w_rows = 2LL * F * (row_group ? groups : 1);
+    LCK(lm::launch_pack_rows_bf16(A, a_bf16, M, K, nullptr, S(stream)));
+    if (fused) {
+        LCK(dia::launch_gemm_glu_bf16(a_bf16, W_bf16, w_rows, y_bf16, M, F, K, glu_kind(act), limit, gp, S(stream), true));
+    } else {
+        LCK(dia::launch_gemm_tcgen05_bf16(a_bf16, 1, W_bf16, w_rows, gate_up, M, 2 * F, K, kPlain, gp, S(stream)));
+        LCK(lm::launch_silu_mul(gate_up, nullptr, y_bf16, M, F, nullptr, S(stream), glu_kind(act), limit));
+    }
+    return LM_B200_OK;
+}
+
 int lm_b200_argmax_rows(const float* logits, int M, int V, int32_t* out, void* stream) {
     if (!logits || !out || M <= 0 || V <= 0) return LM_B200_EINVAL;
     LCK(lm::launch_argmax_rows(logits, M, V, out, S(stream)));

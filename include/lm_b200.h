@@ -287,6 +287,12 @@ int lm_b200_op_linear(const float *A, const void *W_bf16, float *Y, int M, int N
 /* the same on the tensor cores: A is rounded to bf16 into a_bf16 [M][K] first.  K a multiple of 8, N of 4, else
  * LM_B200_EUNSUPPORTED */
 int lm_b200_op_linear_tc(const float *A, const void *W_bf16, float *Y, void *a_bf16, int M, int N, int K, void *stream);
+/* y_bf16[M][F] = the gated unit's activation (lm_b200_act: SILU_GLU, CLAMPED_GLU with `limit`, GELU_GLU) of [gate | up] = A . W[2 F][K]^T, A rounded to bf16 into
+ * a_bf16 [M][K] first.  fused != 0: the gate behind the product's accumulators (LM_B200_EUNSUPPORTED where the kernel does not take the sizes), else product (into
+ * gate_up [M][2 F]) and gate one after the other; to the same bits where both are of one kind of sums (see csrc/gemm_tcgen05.h).  Groups (row_group NULL: none):
+ * rows in groups of 256, row r of group row_group[r], whose weights are rows row_group[r] * 2 F .. of W [groups * 2 F][K]; n_rows: device, rows in use. */
+int lm_b200_op_gated_tc(const float *A, const void *W_bf16, void *a_bf16, float *gate_up, void *y_bf16, int M, int F, int K, int act, float limit, int fused,
+                        const int32_t *row_group, int groups, const int32_t *n_rows, void *stream);
 /* greedy sampling: out[r] = index of the largest of logits[r][0 .. V) (ties: the lowest index) */
 int lm_b200_argmax_rows(const float *logits, int M, int V, int32_t *out, void *stream);
 
