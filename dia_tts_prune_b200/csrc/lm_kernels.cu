@@ -1269,7 +1269,10 @@ cudaError_t launch_tapmix_tail(const float* x, const NormW& n, int taps, float* 
 }
 
 namespace {
-constexpr int kNarrowRowsMin = 1024;                           // rows from which two to a warp fill the SMs
+// Rows times outputs (at most eight of them: the other kernel has a warp for each) from which a row is read once.  Below, that kernel's many short blocks end
+// sooner than these few long ones (us, other kernel / this one, 2048 channels: 8 outputs of 1024 rows 7.4 / 8.1, 1500 10.8 / 8.4, 4096 24.5 / 8.8; 4 of 1500
+// 6.2 / 8.2, 2048 8.5 / 8.4, 4096 14.6 / 8.7; 64 of 1024 48 / 53, 1500 70 / 55, 4096 187 / 57; 512 channels: 8 of 2048 6.7 / 5.0, 64 41 / 21)
+constexpr int kNarrowWorkMin = 10240;
 bool vectors_ok(const float* A, int lda, const void* W, int K) {
     return K % 8 == 0 && lda % 4 == 0 && ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(W)) & 15) == 0;
 }
@@ -1283,7 +1286,7 @@ cudaError_t launch_linear(const float* A, int lda, const void* W, long long w_ex
     const int* a_expert = gm ? gm->a_expert : nullptr;
     const int* n_slots = gm ? gm->n_slots : nullptr;
     const __nv_bfloat16* w = reinterpret_cast<const __nv_bfloat16*>(W);
-    if (!gm && act == kActNone && N <= kRowsKernelMaxOut && M >= kNarrowRowsMin && vectors_ok(A, lda, w, K))
+    if (!gm && act == kActNone && N <= kRowsKernelMaxOut && (long long)M * std::min(N, 8) >= kNarrowWorkMin && vectors_ok(A, lda, w, K))
         return launch_pdl(linear_narrow_kernel, dim3((M + 8 * kNarrowRows - 1) / (8 * kNarrowRows)), dim3(256), 0, st, A, lda, w, Y, ldy, M, N, K);
     // a few rows, or a few outputs (router logits: the same order of operations for every step length, so that the choice of experts
     // does not depend on how a prompt was cut)

@@ -620,3 +620,22 @@ def test_registry_loads_a_model_folder_and_the_cli_entry(tmp_path):
     model = load_model(tmp_path, dtype="float32", max_tokens=128)
     toks = tokens(cfg, 40, 31)
     close(whole(model, "r", toks), O.forward(cfg, w, toks, dtype=torch.float64))
+
+
+@pytest.mark.parametrize("K", [24, 2048])
+@pytest.mark.parametrize("M,N", [(1281, 8), (1281, 33), (2561, 4), (1301, 64), (10241, 1)])
+def test_few_outputs_of_many_rows_have_the_bits_of_few_rows(M, N, K):
+    """A row read once for eight outputs, and a warp per output (portions of 250 rows): the same order of operations, so that a router's choice does not depend on
+    how a prompt was cut"""
+    from dia_tts_prune_b200 import _lm_lib
+    lib, st = _lm_lib.load(), torch.cuda.current_stream().cuda_stream
+    g = torch.Generator(device="cuda").manual_seed(M + K)
+    x, w = torch.randn((M, K), generator=g, device="cuda"), torch.randn((N, K), generator=g, device="cuda").bfloat16()
+
+    def product(rows):
+        y = torch.full((rows.shape[0], N), float("nan"), device="cuda")
+        assert lib.lm_b200_op_linear(rows.data_ptr(), w.data_ptr(), y.data_ptr(), rows.shape[0], N, K, st) == 0
+        return y
+
+    whole = product(x)
+    assert torch.isfinite(whole).all() and torch.equal(whole, torch.cat([product(part.contiguous()) for part in x.split(250)]))
