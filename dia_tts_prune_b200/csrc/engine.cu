@@ -1153,9 +1153,10 @@ RowsRoom rows_room(const dia_b200_rows_layer& a) {
     r.att = r.q + M * heads * 512;
     r.gu = 0;
     r.split = std::max(r.att + M * heads * 512, M * 8 * (size_t)a.F);
-    // the attention's split keys lie where the products' split rows lie before and after it
-    const size_t keys = std::max(attention_rows_work_bytes(a.B, a.T, a.T, a.heads, a.kv_heads, a.mode, a.n_valid),
-                                 a.cross_heads > 0 ? attention_rows_work_bytes(a.B, a.T, a.cross_slots, a.cross_heads, a.cross_kv_heads, 2, a.cross_valid) : 0);
+    // The attention's split keys lie where the products' split rows lie before and after it.  (As many as there can be: the room may be taken once for calls
+    // whose numbers of valid keys differ.)
+    const size_t keys = std::max(attention_rows_work_bytes(a.B, a.T, a.T, a.heads, a.kv_heads, a.mode, nullptr),
+                                 a.cross_heads > 0 ? attention_rows_work_bytes(a.B, a.T, a.cross_slots, a.cross_heads, a.cross_kv_heads, 2, nullptr) : 0);
     r.keys = keys;
     r.bytes = r.split + std::max(gemm_workspace_bytes((int)M, (int)most), keys);
     return r;

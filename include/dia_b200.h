@@ -275,7 +275,7 @@ typedef struct dia_b200_rows_layer {
     dia_b200_dense_ref q, k, v, o, wi, wo, cross_q, cross_o;
     float *k_cache, *v_cache;
     const float *cross_k, *cross_v;
-    void *work;                              /* dia_b200_rows_layer_work_bytes(a) bytes of device memory */
+    void *work;                              /* dia_b200_rows_layer_work_bytes(a) bytes of device memory (of the sizes alone: the same for any n_valid) */
 } dia_b200_rows_layer;
 size_t dia_b200_rows_layer_work_bytes(const dia_b200_rows_layer *a);
 int dia_b200_rows_layer_forward(const dia_b200_rows_layer *a, void *stream);

@@ -189,3 +189,16 @@ def test_numbers_of_valid_keys(calls):
     with pytest.raises(ValueError):
         run(layer, 5, B=17)
     assert len(calls) == 1
+
+
+@pytest.mark.parametrize("T,mode", [(200, 2), (300, 1), (300, 0)])
+def test_the_workspace_does_not_depend_on_the_valid_keys(T, mode):
+    """A caller may take it before the numbers of valid keys are set, or once for several calls"""
+    from dia_tts_prune_b200 import _lib
+    lib, bytes_of = _lib.load(), []
+    for valid in (0, 1, T):
+        a = _lib.RowsLayer(B=2, T=T, D=1024, F=4096, heads=16, kv_heads=16, slots=T, mode=mode, cross_heads=16, cross_kv_heads=16, cross_slots=1024, n_pos=2048)
+        for b in range(2):
+            a.n_valid[b], a.cross_valid[b] = valid, 3 * valid
+        bytes_of.append(lib.dia_b200_rows_layer_work_bytes(C.byref(a)))
+    assert bytes_of[0] == bytes_of[1] == bytes_of[2] > 0
