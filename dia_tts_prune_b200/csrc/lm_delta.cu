@@ -22,10 +22,12 @@
 // of beside them; the blocks in the sequences' order took 68 more, 32 columns a block, which read a third less, 185); 4 heads of 64, 2000 tokens 488 / 256.
 // A column's order of operations depends on its sequence's portion alone.  Sequences of fewer tokens stay with the serial scan.
 #include <algorithm>
+#include <atomic>
 
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "gemm_tcgen05.h"
 #include "lm_device.cuh"
 #include "lm_internal.h"
 
@@ -71,7 +73,6 @@ __device__ __forceinline__ void copies_done_but() { asm volatile("cp.async.wait_
 
 struct DeltaArgs {
     const float* in; int ld, q_off, k_off, v_off, b_off, a_off;
-    float q_mul;
     int H, G, dim, vdim, n_seq;
     float* state;
     const int *seq_slot, *seq_row0, *seq_count, *row_pos;
@@ -380,7 +381,7 @@ delta_columns_kernel(const DeltaArgs p) {
                 float* o = p.o + (size_t)(row0 + t0 + tok) * p.ldo + h * p.vdim + col0 + c0;
 #pragma unroll
                 for (int e = 0; e < NC; ++e)
-                    if (col0 + c0 + e < p.vdim) o[e] = fmaf(a_tok, qs[e], y[e]) * p.q_mul;
+                    if (col0 + c0 + e < p.vdim) o[e] = fmaf(a_tok, qs[e], y[e]);
             }
         }
         // ---- S = A_32 S + (D_32 K)^T U ----
@@ -429,23 +430,29 @@ delta_columns_kernel(const DeltaArgs p) {
 }
 
 template <int DP>
-cudaError_t launch_inst(const DeltaArgs& p, int M, bool early, cudaStream_t st) {
-    cudaError_t e = launch_pdl_if(early, delta_chunk_kernel<DP>, dim3(M / kC + p.n_seq, p.H), dim3(kThreads), 0, st, p);
+cudaError_t launch_inst(const DeltaArgs& p, int M, int n_long, int longest_tokens, cudaStream_t st) {
+    cudaError_t e = launch_pdl_if(false, delta_chunk_kernel<DP>, dim3(M / kC + p.n_seq, p.H), dim3(kThreads), 0, st, p);
     if (e != cudaSuccess) return e;
+    ++dia::extra_launches();
     constexpr int smem = Columns<DP>::floats * 4;
     int dev = 0;
     e = cudaGetDevice(&dev);
-    static bool asked[64] = {};
-    if (e == cudaSuccess && (dev < 0 || dev >= 64 || !asked[dev])) {
+    static std::atomic<bool> asked[64];
+    if (e == cudaSuccess && (dev < 0 || dev >= 64 || !asked[dev].load(std::memory_order_relaxed))) {
         e = cudaFuncSetAttribute(delta_columns_kernel<DP>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        if (e == cudaSuccess && dev >= 0 && dev < 64) asked[dev] = true;
+        if (e == cudaSuccess && dev >= 0 && dev < 64) asked[dev].store(true, std::memory_order_relaxed);
     }
     if (e != cudaSuccess) return e;
-    // not early: beside the kernel in front its blocks would crowd on the SMs that empty first (1024 tokens, 128 blocks: two to an SM on half of them,
-    // 170 us instead of 115)
     // (of M tokens no more than M / kChunkTokensMin sequences are long ones)
-    const int longest = std::min(p.n_seq, M / kChunkTokensMin);
-    return launch_pdl_if(p.n_seq > 1, delta_columns_kernel<DP>, dim3((p.vdim + kCols - 1) / kCols, p.H, longest), dim3(kColThreads), (size_t)smem, st, p);
+    const int columns = (p.vdim + kCols - 1) / kCols, longest = std::min(n_long > 0 ? n_long : p.n_seq, M / kChunkTokensMin);
+    int sms = 0;
+    e = dia::current_sms(&dev, &sms);
+    if (e != cudaSuccess) return e;
+    // Beside the kernel in front the blocks crowd on the SMs that empty first.  Where there is one of the larger kind for each SM at most and a walk is long, that
+    // costs more than the early start gives (us, 2048 tokens and 1, 128 blocks: 548 early, 400 behind it; 900 and five of 40 300 / 253; 96 and three of 10, 32
+    // blocks 58 / 63; four of 300, 512 blocks 257 / 262); a step of one sequence has nothing that starts beside
+    const bool spread = DP > 64 && (long long)columns * p.H * longest <= sms && longest_tokens >= 8 * kC;
+    return launch_pdl_if(p.n_seq > 1 && !spread, delta_columns_kernel<DP>, dim3(columns, p.H, longest), dim3(kColThreads), (size_t)smem, st, p);
 }
 
 }  // namespace
@@ -457,9 +464,9 @@ bool delta_chunks_ok(const float* in, int ld, const ScanInputs& si, int H, int G
 }
 
 cudaError_t launch_delta_chunks(const float* in, int ld, const ScanInputs& si, int H, int G, int dim, int vdim, float* state, const SeqMeta& sm,
-                                const RowMeta& rm, int n_seq, int M, float* o, int ldo, float* room, cudaStream_t st, bool early, float q_mul) {
-    const DeltaArgs p{in, ld, si.q_off, si.k_off, si.v_off, si.beta_off, si.a_off, q_mul, H, G, dim, vdim, n_seq, state, sm.slot, sm.row0, sm.count, rm.pos, o, ldo, room};
-    return dim <= 64 ? launch_inst<64>(p, M, early, st) : launch_inst<128>(p, M, early, st);
+                                const RowMeta& rm, int n_seq, int M, float* o, int ldo, float* room, int n_long, int longest_tokens, cudaStream_t st) {
+    const DeltaArgs p{in, ld, si.q_off, si.k_off, si.v_off, si.beta_off, si.a_off, H, G, dim, vdim, n_seq, state, sm.slot, sm.row0, sm.count, rm.pos, o, ldo, room};
+    return dim <= 64 ? launch_inst<64>(p, M, n_long, longest_tokens, st) : launch_inst<128>(p, M, n_long, longest_tokens, st);
 }
 
 }  // namespace lm

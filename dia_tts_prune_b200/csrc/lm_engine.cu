@@ -845,14 +845,22 @@ int stream_mixer_kernels(lm_b200_engine* e, const lm_b200_layer& l, const MixPla
         LCK(lm::launch_delta_prep(proj, ld, c.beta, d, l.conv_tail, v.rm, e->rec, ldr, M, st, c.a));
         LCK(lm::launch_conv_tail(proj, ld, v0 + nv, l.conv_taps, l.conv_tail, v.sm, n_seq, st));
         const lm::ScanInputs si{0, k0, d0, v0, b0};
-        // long portions in chunks; a step of one sequence is either, one of several may have both kinds
-        const bool early = M <= lm::kRowsKernelMax;
-        const bool chunks = M - n_seq + 1 >= lm::kChunkTokensMin && e->delta_room && lm::delta_chunks_ok(e->rec, ldr, si, H, l.kv_heads, l.dim, l.vdim, l.rec_state);
+        // Long portions in chunks, short ones one token after the other.  A step of one sequence has one kind; one of several may have both, unless the host has
+        // said which
+        bool any_long = M - n_seq + 1 >= lm::kChunkTokensMin, any_short = n_seq > 1 || !any_long;
+        int n_long = 0, longest = M;
+        if (v.sizes.n > 0) {
+            n_long = (int)std::count_if(v.sizes.rows, v.sizes.rows + n_seq, [](int n) { return n >= lm::kChunkTokensMin; });
+            any_long = n_long > 0;
+            longest = *std::max_element(v.sizes.rows, v.sizes.rows + n_seq);
+            any_short = n_long < n_seq;
+        }
+        const bool chunks = any_long && e->delta_room && lm::delta_chunks_ok(e->rec, ldr, si, H, l.kv_heads, l.dim, l.vdim, l.rec_state);
         if (chunks)
-            LCK(lm::launch_delta_chunks(e->rec, ldr, si, H, l.kv_heads, l.dim, l.vdim, l.rec_state, v.sm, v.rm, n_seq, M, at.out, at.ldo, e->delta_room, st, early));
-        if (!chunks || n_seq > 1)
+            LCK(lm::launch_delta_chunks(e->rec, ldr, si, H, l.kv_heads, l.dim, l.vdim, l.rec_state, v.sm, v.rm, n_seq, M, at.out, at.ldo, e->delta_room, n_long, longest, st));
+        if (!chunks || any_short)
             LCK(lm::launch_column_scan(e->rec, ldr, si, lm::kScanDelta, H, l.kv_heads, l.dim, l.vdim, l.rec_state, v.sm, v.rm, n_seq, at.out, at.ldo, st,
-                                       true, early || chunks, nullptr, 0, 1.f, chunks));
+                                       true, M <= lm::kRowsKernelMax || chunks, nullptr, 0, 1.f, chunks));
         LCK(lm::launch_head_norm_gate(at.out, at.ldo, at.out_b, l.head_norm, gate, ld, H, l.vdim, e->m.eps, M, st, gate_act, at.scale));
     } else if (l.mixer == LM_B200_MIXER_RETENTION) {
         // q and k (adjacent in the row) turn in place, k also takes dim^-1/2; decay fixed per head, no write gate, no normaliser

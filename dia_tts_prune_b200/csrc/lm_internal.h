@@ -177,7 +177,8 @@ cudaError_t launch_column_scan(const float* in, int ld, const ScanInputs& si, in
                                cudaStream_t st, bool head_decay = false, bool early = true, const float* decay = nullptr, int ldd = 0,
                                float q_mul = 1.f, bool few = false);
 // The delta rule with one decay per head in chunks of kDeltaChunk tokens (lm_delta.cu), for the sequences of at least kChunkTokensMin tokens in a step; the
-// others are left to the scan above (few: its sequences of that many tokens are left out; launched early, directly behind launch_delta_chunks, it runs beside that).  room: delta_room_floats(M, n_seq, H) floats, 16-byte aligned.
+// others are left to the scan above (few: its sequences of that many tokens are left out; launched early, directly behind launch_delta_chunks, it runs beside
+// that).  n_long: how many there are (0: not known), of at most longest_tokens.  room: delta_room_floats(M, n_seq, H) floats, 16-byte aligned.
 // kChunkTokensMin: from where chunks are the shorter way beside other sequences (us of a layer of 16 heads of 128, serial / chunks from 96, 128 and 160 tokens on: one prompt
 // of 128 tokens 88 / 87 82 82, prompts of 200, 150, 100, 50, 200 and 150 224 / 204 216 227, four of 300 264 / 255 255 255, eight of 250 412 / 338 340 338).  The longest sequences
 // below it wait for more SMs where others are just above: three of 95, 95 and 96 tokens 104 / 125 106 106, of 127, 127 and 128 115 / 123 139 117.
@@ -185,7 +186,7 @@ constexpr int kDeltaChunk = 32, kDeltaChunkFloats = 2 * kDeltaChunk * kDeltaChun
 inline size_t delta_room_floats(size_t M, size_t n_seq, size_t H) { return (M / kDeltaChunk + n_seq) * H * kDeltaChunkFloats; }
 bool delta_chunks_ok(const float* in, int ld, const ScanInputs& si, int H, int G, int dim, int vdim, const float* state);
 cudaError_t launch_delta_chunks(const float* in, int ld, const ScanInputs& si, int H, int G, int dim, int vdim, float* state, const SeqMeta& sm,
-                                const RowMeta& rm, int n_seq, int M, float* o, int ldo, float* room, cudaStream_t st, bool early, float q_mul = 1.f);
+                                const RowMeta& rm, int n_seq, int M, float* o, int ldo, float* room, int n_long, int longest_tokens, cudaStream_t st);
 // the same scan with scalar gates per (row, head): S <- a S + (b k) v^T and one more value column that is the constant 1
 // (the normaliser n <- a n + b k, read out as n . q), so state and read-out have vdim + 1 columns per head.  a and b are
 // columns a_off + h and beta_off + h of the input rows.  fixed_decay [H]: a = fixed_decay[h], b = 1 for every token instead.

@@ -102,3 +102,29 @@ def test_short_sequences_of_a_long_step():
             y, s = run(model, [x[i]], [cuts[i]])
             close(together[i], y[0])
             close(states[i], s[0])
+
+
+def test_steps_of_long_and_short_portions_repeat_their_bits():
+    """The scan of the short ones runs beside the chunks of the long ones: thirty times the same outputs and states"""
+    model = delta_model(4, 2, 128, 128)
+    g = torch.Generator().manual_seed(11)
+    x = [torch.randn(n, 64, generator=g).cuda() for n in (700, 37, 96, 95)]
+    first = None
+    for _ in range(30):
+        got = run(model, x, [[len(t)] for t in x])
+        first = first or got
+        for a, b in zip(got[0] + got[1], first[0] + first[1]):
+            assert torch.equal(a, b)
+
+
+def test_only_kernels_with_sequences_are_launched():
+    """The same 288 rows: short portions by the scan, long ones by the two kernels of the chunks, both by all three"""
+    model = delta_model(2, 2, 64, 64)
+    count = model.engine.lib.lm_b200_launch_count
+    launches = []
+    for rows in ([95, 95, 95, 3], [96, 96, 96], [100, 92, 93, 3]):
+        x = [torch.randn(n, 64, generator=torch.Generator().manual_seed(n)).cuda() for n in rows]
+        before = count()
+        run(model, x, [[n] for n in rows])
+        launches.append(count() - before)
+    assert launches[1] - launches[0] == 1 and launches[2] - launches[0] == 2
