@@ -46,6 +46,7 @@ class LMEngine:
         self.head = head.detach().to(device=self.device, dtype=torch.bfloat16).contiguous()
         self.final_norm = final_norm
         self.width, self.vocab, self.max_rows = int(width), int(vocab), int(max_rows)
+        self._zeros = np.zeros(64, dtype=np.int32)
         m = _lm_lib.Model()
         m.n_layer, m.width, m.vocab, m.taps = len(layers), self.width, self.vocab, int(taps)
         m.page_size, m.max_pages, m.n_slots, m.max_rows = state.page_size, state.max_pages, state.n_slots, self.max_rows
@@ -89,30 +90,38 @@ class LMEngine:
     # ---- one launch sequence over <= max_rows rows -----------------------------------------------------------
     def _pack(self, parts: list[tuple[Sequence, list[int], int, list[int]]]) -> tuple[torch.Tensor, int, int, int]:
         """parts: (sequence, tokens, position of the first token, wanted indexes into tokens) -> the step buffer."""
-        n_rows = sum(len(t) for _, t, _, _ in parts)
         S = len(parts)
-        want = [k for _, _, _, w in parts for k in w]
-        buf = np.empty(4 * n_rows + 3 * S + len(want) + S, dtype=np.int32)      # (the last S: the sequences' first positions, for the host alone)
-        tok, slot, pos, start = (buf[i * n_rows:(i + 1) * n_rows] for i in range(4))
-        meta, r0, at = buf[4 * n_rows:], 0, 0
-        for s, (seq, tokens, p0, w) in enumerate(parts):
-            n = len(tokens)
-            tok[r0:r0 + n] = tokens
-            slot[r0:r0 + n] = seq.slot
-            pos[r0:r0 + n] = np.arange(p0, p0 + n, dtype=np.int32)
-            start[r0:r0 + n] = p0
-            meta[s], meta[S + s], meta[2 * S + s], meta[s - S] = seq.slot, r0, n, p0
-            for k in w:
-                meta[3 * S + at] = r0 + k
-                at += 1
-            r0 += n
-        if n_rows > 8:                                          # (shorter steps have no use for it)
-            at = buf.__array_interface__["data"][0]
-            self._say(at + 4 * (4 * n_rows + 2 * S), at + 4 * (buf.size - S), S)
+        counts = [len(t) for _, t, _, _ in parts]
+        n_rows = sum(counts)
+        # token, slot, position, start of every row; slot, first row, rows of every sequence; wanted rows; and, for the host alone, first positions
+        n_want = sum([len(p[3]) for p in parts])
+        buf = np.empty(4 * n_rows + 4 * S + n_want, dtype=np.int32)
+        want, row0, a = [], [], 0
+        for n, (seq, tokens, p0, w) in zip(counts, parts):
+            b = a + n
+            buf[a:b] = tokens
+            buf[n_rows + a:n_rows + b] = seq.slot
+            buf[2 * n_rows + a:2 * n_rows + b] = np.arange(p0, p0 + n, dtype=np.int32)
+            buf[3 * n_rows + a:3 * n_rows + b] = p0
+            if w:
+                want += [a + k for k in w]
+            row0.append(a)
+            a = b
+        buf[4 * n_rows:] = [p[0].slot for p in parts] + row0 + counts + want + [p[2] for p in parts]
         t = torch.from_numpy(buf)
+        if n_rows > 8:                                          # (shorter steps have no use for it)
+            at = t.data_ptr()
+            self._say(at + 4 * (4 * n_rows + 2 * S), at + 4 * (buf.size - S), S)
         if buf.size > 4096:                                     # a long step: asynchronous copy from pinned memory
             t = t.pin_memory()
-        return t.to(self.device, non_blocking=True), n_rows, S, len(want)
+        return t.to(self.device, non_blocking=True), n_rows, S, n_want
+
+    def _pack_rows(self, parts) -> tuple[torch.Tensor, int, int, int]:
+        """The step buffer of rows without tokens; parts: (sequence, rows, first position)"""
+        most = max([n for _, n, _ in parts], default=0)
+        if self._zeros.size < most:
+            self._zeros = np.zeros(most, dtype=np.int32)
+        return self._pack([(s, self._zeros[:n], p0, ()) for s, n, p0 in parts])
 
     def _say(self, rows: int, first: int, n: int) -> None:
         """Tells the engine the sizes of the step that is packed, ``n`` int32 at either address (it takes them with the call that follows; what it
@@ -187,7 +196,7 @@ class LMEngine:
 
     # ---- operator boundaries (one mechanism at a time; used by the parity tests) ----------------------------------
     def op_norm_tapmix(self, layer: int, sub: int, x: torch.Tensor, parts) -> torch.Tensor:
-        buf, M, S, _ = self._pack([(s, [0] * n, p0, []) for s, n, p0 in parts])
+        buf, M, S, _ = self._pack_rows(parts)
         x = x.to(device=self.device, dtype=torch.float32).contiguous()
         out = torch.empty_like(x)
         _lm_lib.check(self.lib.lm_b200_op_norm_tapmix(self._h, layer, sub, x.data_ptr(), buf.data_ptr(), M, S, out.data_ptr(),
@@ -195,7 +204,7 @@ class LMEngine:
         return out
 
     def op_mixer(self, layer: int, h: torch.Tensor, parts) -> torch.Tensor:
-        buf, M, S, _ = self._pack([(s, [0] * n, p0, []) for s, n, p0 in parts])
+        buf, M, S, _ = self._pack_rows(parts)
         self.state.sync_table()
         h = h.to(device=self.device, dtype=torch.float32).contiguous()
         y = torch.empty((M, self.width), dtype=torch.float32, device=self.device)
@@ -206,7 +215,7 @@ class LMEngine:
     def op_attention(self, layer: int, qk: torch.Tensor, parts) -> torch.Tensor:
         """Attention of ``layer`` alone on projected rows ``qk [M, (heads + kv_heads) * dim]`` (queries, then keys), which
         are appended to the pages of their sequences; ``parts``: (sequence, rows, first position) like ``op_mixer``."""
-        buf, M, S, _ = self._pack([(s, [0] * n, p0, []) for s, n, p0 in parts])
+        buf, M, S, _ = self._pack_rows(parts)
         self.state.sync_table()
         a = self.layers[layer].mixer
         qk = qk.to(device=self.device, dtype=torch.float32).contiguous().clone()
@@ -218,7 +227,7 @@ class LMEngine:
     def op_mixer_kernels(self, layer: int, proj: torch.Tensor, parts) -> torch.Tensor:
         """The mixer kernels of a parallel- or stream-form record alone on stacked projections ``proj [M, n_in]`` (its attention
         or recurrence without the products around it); the state of the sequences in ``parts`` is appended to."""
-        buf, M, S, _ = self._pack([(s, [0] * n, p0, []) for s, n, p0 in parts])
+        buf, M, S, _ = self._pack_rows(parts)
         self.state.sync_table()
         m = self.layers[layer].mixer
         proj = proj.to(device=self.device, dtype=torch.float32).contiguous().clone()

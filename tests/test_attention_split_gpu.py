@@ -218,7 +218,7 @@ def test_steps_of_one_tile_of_keys_split_it_themselves(rows, past, launches):
     g = torch.Generator().manual_seed(8)
     seqs = [model.state.open(str(i)) for i in range(len(rows))]
     for q in seqs:
-        model.state.reserve(q, past + 64)
+        model.state.reserve(q, past + 80)
         if past:
             model.engine.op_attention(0, torch.randn(past, 6 * 64, generator=g), [(q, past, 0)])
     x, parts = torch.randn(sum(rows), 6 * 64, generator=g), [(q, n, past) for q, n in zip(seqs, rows)]
