@@ -15,11 +15,11 @@ CSRC = PKG / "csrc"
 INCLUDE = PKG.parent / "include"
 LIB = CSRC / "libdia_b200.so"
 SOURCES = ["step_kernel.cu", "aux_kernels.cu", "gemm_tcgen05.cu", "prefill_kernels.cu", "batch_kernel.cu", "engine.cu", "attention_split.cu"]
-HEADERS = ["common.cuh", "engine_internal.h", "sampler.cuh", "gemm_tcgen05.h", "attention_split.h"]
+HEADERS = ["common.cuh", "engine_internal.h", "sampler.cuh", "gemm_tcgen05.h", "attention_split.h", "fp32_pairs.cuh"]
 LM_LIB = CSRC / "liblm_b200.so"
 LM_SOURCES = ["lm_kernels.cu", "lm_mixers.cu", "lm_streams.cu", "lm_linear.cu", "lm_scan.cu", "lm_delta.cu", "lm_attention.cu", "lm_engine.cu", "gemm_tcgen05.cu",
               "attention_split.cu"]                                # the tensor-core GEMM is shared with Dia
-LM_HEADERS = ["lm_internal.h", "lm_device.cuh", "gemm_tcgen05.h", "attention_split.h", "common.cuh", "engine_internal.h"]
+LM_HEADERS = ["lm_internal.h", "lm_device.cuh", "gemm_tcgen05.h", "attention_split.h", "common.cuh", "engine_internal.h", "fp32_pairs.cuh"]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-lineinfo", "-std=c++17",
               "-Xcompiler", "-fPIC", "-shared"]
 

@@ -154,14 +154,6 @@ __device__ __forceinline__ void tmem_load16(uint32_t addr, float* v) {
         : "r"(addr)
         : "memory");
 }
-// two fp32 in one register pair, two operations in one instruction
-using f2 = unsigned long long;
-__device__ __forceinline__ f2 pack2(float lo, float hi) {
-    f2 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-    return r;
-}
-__device__ __forceinline__ void unpack2(f2 v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
 __device__ __forceinline__ void tmem_load8(uint32_t addr, float (&v)[8]) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
                  : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
@@ -178,22 +170,6 @@ __device__ __forceinline__ void tmem_load_pairs(uint32_t addr, f2* p) {       //
 #pragma unroll
     for (int e = 0; e < N; ++e) p[e] = pack2(v[2 * e], v[2 * e + 1]);
 }
-__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
-    f2 d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-    return d;
-}
-__device__ __forceinline__ f2 mul2(f2 a, f2 b) {
-    f2 d;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-__device__ __forceinline__ f2 add2(f2 a, f2 b) {
-    f2 d;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-__device__ __forceinline__ f2 twice(float v) { return pack2(v, v); }
 // tanh x = x + x^3 q(x^2) for |x| <= kTanhRange: q interpolates (tanh x / x - 1) / x^2 at six Chebyshev nodes (relative error of the
 // result 3e-10 before rounding).  A tile's scores mostly lie there, and it takes a fifth of the library call's instructions
 // (a tile of capped scores: 2100 -> 800 cycles)

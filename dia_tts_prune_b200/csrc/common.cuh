@@ -10,6 +10,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "fp32_pairs.cuh"
+
 namespace dia {
 
 constexpr int kHeadDim = 128;
@@ -244,21 +246,8 @@ __device__ __forceinline__ uint32_t ll_wait32(const unsigned long long* p, uint3
 __host__ __device__ inline int sp_meta_word(int n, int gq) { return (n & 7) * 2 + (gq >> 2); }
 __host__ __device__ inline int sp_meta_shift(int n, int gq) { return 4 * ((n >> 3) * 4 + (gq & 3)); }
 
-// ---- packed fp32x2 math (Blackwell FFMA2) -------------------------------------------------------
-typedef unsigned long long f32x2;   // two packed floats in a 64-bit register
-__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
-    f32x2 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-    return r;
-}
-__device__ __forceinline__ void unpack2(f32x2 v, float& lo, float& hi) {
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
-}
-__device__ __forceinline__ f32x2 ffma2(f32x2 a, f32x2 b, f32x2 c) {
-    f32x2 d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-    return d;
-}
+using f32x2 = f2;                    // (see fp32_pairs.cuh)
+__device__ __forceinline__ f32x2 ffma2(f32x2 a, f32x2 b, f32x2 c) { return fma2(a, b, c); }
 // two bf16 packed in a u32 -> (lo element, hi element) as exact fp32
 __device__ __forceinline__ f32x2 bf16x2_to_f32x2(uint32_t w) {
     return pack2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u));

@@ -27,6 +27,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "fp32_pairs.cuh"
 #include "gemm_tcgen05.h"
 #include "lm_device.cuh"
 #include "lm_internal.h"
@@ -38,26 +39,11 @@ namespace {
 constexpr int kC = kDeltaChunk, kCols = 16, kThreads = 128, kColThreads = 256, kTS = kC + 4;      // kTS: row stride of the triangles in shared memory
 static_assert(kC == 32, "a lane per column of the triangle");
 
-using f2 = unsigned long long;                                // two packed fp32
-__device__ __forceinline__ f2 pack2(float lo, float hi) {
-    f2 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-    return r;
-}
+using dia::f2; using dia::pack2; using dia::fma2;
 __device__ __forceinline__ float sum2(f2 v) {
     float x, y;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(v));
+    dia::unpack2(v, x, y);
     return x + y;
-}
-__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
-    f2 r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-__device__ __forceinline__ f2 mul2(f2 a, f2 b) {
-    f2 r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
 }
 __device__ __forceinline__ void copy16(float* dst, const float* src, bool ok) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src), "r"(ok ? 16 : 0)

@@ -19,6 +19,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "fp32_pairs.cuh"
 #include "lm_device.cuh"
 #include "lm_internal.h"
 
@@ -32,23 +33,7 @@ constexpr int kMaxWarps = 8;
 // lanes that share a pair of columns
 template <int DP> constexpr int kParts = DP > 64 ? DP / 8 : 8;
 
-using f2 = unsigned long long;                                // two packed fp32
-__device__ __forceinline__ f2 pack2(float lo, float hi) {
-    f2 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-    return r;
-}
-__device__ __forceinline__ void unpack2(f2 v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
-__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
-    f2 r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-__device__ __forceinline__ f2 mul2(f2 a, f2 b) {
-    f2 r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
+using dia::f2; using dia::pack2; using dia::unpack2; using dia::fma2; using dia::mul2;
 __device__ __forceinline__ float sum2(f2 a, f2 b) {
     float x, y, z, w;
     unpack2(a, x, y);
