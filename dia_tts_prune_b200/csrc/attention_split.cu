@@ -5,14 +5,14 @@
 // that a tile of keys serves all of them.  It walks its keys 64 at a time:
 //   3 warps   fetch key and value tiles into a ring of shared-memory slots.  A launch in front has scaled them by powers of two and split
 //             x = hi + lo into fp16 ([key / 8][channel / 8] blocks of 8 x 16 bytes: the layout is the K-major operand of the scores and the
-//             MN-major operand of the value product), so that one lane copies a tile; keys beyond the room for them are split here
+//             MN-major operand of the value product), so that one lane copies a tile.  Keys beyond the room for them are split here, in an instance of its own
 //   1 warp    issues tcgen05.mma: scores S = Q K^T (M = 128, N = 64; lo hi, hi lo, then hi hi, so that the small terms are
 //             added first) per group of at most 128 channels, and the value product of a tile before (weights as the
 //             operand in tensor memory)
 //   8 warps   two groups of four take turns: one thread weighs all 64 keys of its row of a tile - scores from tensor memory (the channel groups
 //             are summed here, in fp32), cap, bias, mask, online softmax in base 2, weights split and written to tensor memory.  All a row's two
 //             threads tell each other of a tile is the maximum (which the group that has the next tile needs when it has its scores), the
-//             weights' scale and their sum.  Both add the value product of every tile to fp32 registers, half of the channels each
+//             weights' scale and two of their four sums.  Both add the value product of every tile to fp32 registers, half of the channels each
 // The accumulator of a tensor-core product loses up to one unit in the last place at every step, towards zero (measured: 2e-6
 // over K = 2048).  So no accumulator lives longer than one tile and one channel group, and sums over tiles are fp32 additions
 // in registers: measured against 64 bits the output is closer than the fp32 FMA kernels' (relative 2-norm, 300 rows, two heads of 128,
@@ -25,14 +25,15 @@
 // its tokens has fewer), and nothing of a token that a row does not see, or of another row, enters its result: the bits do not depend on
 // what shares the launch.
 //
-// Bound: instructions of the row warps and where they come from.  Per 64 keys and 128 rows 3 x 128 x 64 x (dk + dv) multiply-adds on the tensor
-// pipe (128 + 128: 1150 cycles of the scores, whose operands take all of shared memory's bandwidth, and 770) stand against about 5000 cycles: a row's 64
-// scores take a thread some 1500 instructions, two warps on each scheduler, and a third of the stalls are instruction fetches (the loops below
-// are rolled where a roll is possible: the code of a tile's turn, some 35 KB with the cap, is what the caches hold just about).  With four threads per row
-// that exchanged a tile's maxima and largest weights, 16 keys each, the same took 8000 cycles.  Times (us, four or two threads per row / now): windowed
-// 4096 rows, 16 heads of 128 over 4, window 1024, capped 238 / 205; the same rows over latent rows of 256 + 32 408 / 368; mixed scores, prompts of 1500, 333
-// and 215 rows, 8 heads of 128 over 2 116 / 90; float32 model of 978 rows, four layers 216 / 191; Dia, 861 frames, 36 attentions 3024 / 1624 and 213 for the split
-// keys, which every row tile used to split for itself; 9 decoding sequences over 1134 latent rows 281 / 128.
+// Bound: the latencies of the row warps' chains.  Per 64 keys and 128 rows 3 x 128 x 64 x (dk + dv) multiply-adds on the tensor pipe (128 + 128: 1150 cycles of
+// the scores, whose operands take all of shared memory's bandwidth, and 770) stand against about 5000 cycles.  A row's 64 scores take a thread some 1500
+// instructions; with two such warps a scheduler issues on 40 % of the cycles (windowed rows; 31 % over latent rows and for Dia's prompts), and the tensor pipe is
+// busy for 24 % (27, 20).  What warps wait for instead, in the same order: instruction fetches 29, 8 and 27 % of their stalls (the code of a tile's turn is some
+// 35 KB with the cap; loops are rolled where a roll is possible), loads from tensor memory and of spilled registers 18, 49 and 25 %, fixed latencies 24, 20 and
+// 20 %.  Four threads per row that exchanged a tile's maxima and largest weights, 16 keys each, took 8000 cycles.  Times (us, four or two threads per row / now):
+// windowed 4096 rows, 16 heads of 128 over 4, window 1024, capped 238 / 205; the same rows over latent rows of 256 + 32 408 / 368; mixed scores, prompts of 1500,
+// 333 and 215 rows, 8 heads of 128 over 2 116 / 90; float32 model of 978 rows, four layers 216 / 191; Dia, 861 frames, 36 attentions 3024 / 1624 and 213 for the
+// split keys, which every row tile used to split for itself; 9 decoding sequences over 1134 latent rows 281 / 128.
 // Every wait is bounded: a wait that runs out makes the CTA write NaN, note it in a word that the host reads, and end; the next launch
 // on the device returns an error.
 #include <algorithm>
@@ -289,8 +290,8 @@ __device__ __forceinline__ size_t part_offset(const Geometry& geo, int part) {
 
 // Splits the keys and values that the step's rows see, once for all row tiles: without it each of the M rep / 128 row tiles of a
 // key/value head converts every tile it walks, and that conversion (two thirds of the instructions) bounds the kernel below.
-// A CTA per (tile of the room, part), and two rounds of them at most: a room for many sequences has far more tiles than a short step
-// fills.  Tiles are dealt to the sequences in order.  Warp w takes keys 8 w .. of the tile.
+// A CTA per (tile of the room, part), but kSplitGrid of them at most, which take further tiles in turn and look up whose they are each time: a room for
+// many sequences has far more tiles than a short step fills.  Tiles are dealt to the sequences in order.  Warp w takes keys 8 w .. of the tile.
 __global__ void __launch_bounds__(256)
 split_keys_kernel(const __grid_constant__ SplitAttention p, const __grid_constant__ Geometry geo) {
     __shared__ int s_first, s_seq, s_run;
@@ -534,7 +535,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1)
 split_attention_kernel(const __grid_constant__ SplitAttention p, const __grid_constant__ Geometry geo) {
     constexpr int DVH = 64 * NVS;                             // output channels of a thread
     // The block is launched with 168 registers a thread.  A row's thread holds 64 scores and its sums; the others' share is what the issuing warp needs
-    // for its operands (with 24 registers an instruction of the value product took 170 cycles to issue, not 77)
+    // for its operands (with 24 registers an instruction of the value product took 170 cycles to issue, 77 with these)
     constexpr int kRowRegs = NVS == 1 ? 208 : 216, kOtherRegs = NVS == 1 ? 88 : 72;
     static_assert(32 * kRowWarps * kRowRegs + 128 * kOtherRegs <= 168 * kSplitThreads, "registers of the block");
     constexpr int RW = kRowWarps, LW = NVS == 1 ? 16 : 8;     // row warps, pairs of columns in flight

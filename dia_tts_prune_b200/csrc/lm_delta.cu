@@ -18,8 +18,8 @@
 //
 // Bound: the loads from shared memory that feed the multiply-adds (16 bytes for each lane: four cycles an instruction, and 2.7 multiply-adds for each): a
 // chunk of 32 tokens takes a block 6800 cycles by itself and 10000 beside another, where the serial scan takes 24000.  Layer of 16 heads of 128, us, serial
-// scan / chunks: 1024 tokens 323 / 245, 4096 1102 / 737, prompts of 1024, 700, 513, 37 and 1 tokens 574 / 390 (407 with the short ones behind the long ones instead
-// of beside them; the blocks in the sequences' order took 68 more, 32 columns a block, which read a third less, 185); 4 heads of 64, 2000 tokens 488 / 256.
+// scan / chunks: 1024 tokens 323 / 243, 4096 1102 / 729, 2048 beside 1 684 / 399, prompts of 1024, 700, 513, 37 and 1 tokens 574 / 390 (407 with the short ones behind
+// the long ones instead of beside them; the blocks in the sequences' order took 68 more, 32 columns a block, which read a third less, 185); 4 heads of 64, 2000 tokens 488 / 256.
 // A column's order of operations depends on its sequence's portion alone.  Sequences of fewer tokens stay with the serial scan.
 #include <algorithm>
 #include <atomic>

@@ -172,6 +172,7 @@ struct lm_b200_engine {
     struct KeyShape { dia::SplitAttention shape; int window, chunk, keep_first; };
     std::vector<KeyShape> key_shapes;
     std::vector<void*> rooms;
+    bool room_kept = false;                      // the last one is in a graph of the caller's: it stays as long as the engine
     size_t room_refused = (size_t)-1;            // bytes that the device did not have
     // steps of a few rows are captured once per (rows, sequences, wanted) into a CUDA graph over these fixed buffers
     int32_t* step_static = nullptr;
@@ -249,6 +250,12 @@ struct StepView {
     lm::StepSizes sizes;
 };
 
+// What the host has said of a step's sizes is for one call, whatever becomes of it
+struct TakesSizes {
+    lm_b200_engine* e;
+    ~TakesSizes() { if (e) e->said = false; }
+};
+
 // A larger room for the split keys of this step.  What it replaces is freed behind all that reads it, or with the engine
 void grow_room(lm_b200_engine* e, size_t bytes, cudaStream_t st) {
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
@@ -263,12 +270,13 @@ void grow_room(lm_b200_engine* e, size_t bytes, cudaStream_t st) {
         (void)cudaGetLastError();
         e->room_refused = bytes;
     } else {
-        if (!e->rooms.empty() && cudaDeviceSynchronize() == cudaSuccess) {
+        if (!e->rooms.empty() && !e->room_kept && cudaDeviceSynchronize() == cudaSuccess) {
             (void)cudaFree(e->rooms.back());
             e->rooms.pop_back();
         }
         (void)cudaGetLastError();
         e->rooms.push_back(room);
+        e->room_kept = false;
         e->kv_split = room;
         e->kv_split_bytes = bytes;
     }
@@ -279,12 +287,17 @@ void grow_room(lm_b200_engine* e, size_t bytes, cudaStream_t st) {
 StepView view(lm_b200_engine* e, const int32_t* step, int M, int n_seq, cudaStream_t st) {
     StepView v;
     v.sizes = lm::StepSizes{nullptr, nullptr, 0};
-    if (e->said && (int)e->said_rows.size() == n_seq) {
+    // (nothing in a step of a few rows depends on them, and its graph is replayed for other sizes)
+    if (M > lm::kRowsKernelMax && e->said && (int)e->said_rows.size() == n_seq) {
         long long rows = 0;
         for (int n : e->said_rows) rows += n;
         if (rows == M) v.sizes = lm::StepSizes{e->said_rows.data(), e->said_first.data(), n_seq};
     }
-    e->said = false;
+    if (M > lm::kAttnRowsKernelMax && !e->rooms.empty() && !e->room_kept) {
+        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(st, &capture) != cudaSuccess) (void)cudaGetLastError();
+        e->room_kept = capture != cudaStreamCaptureStatusNone;
+    }
     if (M > lm::kAttnRowsKernelMax && v.sizes.n > 0) {
         size_t need = 0;
         for (const auto& k : e->key_shapes)
@@ -1516,13 +1529,13 @@ int lm_b200_check(lm_b200_engine* e, void* stream) {
 
 int lm_b200_forward(lm_b200_engine* e, const int32_t* step, int M, int n_seq, int n_want, float* logits_out, float* layers_out,
                     void* stream) {
+    const TakesSizes once{e};
     if (!e || !step || M <= 0 || M > e->m.max_rows || n_seq <= 0 || n_seq > M || n_want < 0 || n_want > M ||
         (n_want > 0 && !logits_out))
         return LM_B200_EINVAL;
     Guard g(e->device);
     if (!g.ok) return LM_B200_ECUDA;
     if (dia::take_ran_out(e->device, S(stream))) return cuda_fail(cudaErrorLaunchTimeout);
-    if (M <= lm::kRowsKernelMax) e->said = false;             // (nothing there depends on it, and a captured step reads another one's rows)
     if (e->m.step_graphs && M <= lm::kRowsKernelMax && !layers_out)
         return run_step_graph(e, step, M, n_seq, n_want, logits_out, S(stream));
     return run_step(e, step, M, n_seq, n_want, logits_out, layers_out, S(stream));
@@ -1530,6 +1543,7 @@ int lm_b200_forward(lm_b200_engine* e, const int32_t* step, int M, int n_seq, in
 
 int lm_b200_op_norm_tapmix(lm_b200_engine* e, int layer, int sub, const float* x, const int32_t* step, int M, int n_seq,
                            float* out, void* stream) {
+    const TakesSizes once{e};
     if (!e || layer < 0 || layer >= e->m.n_layer || (sub != 0 && sub != 1) || !x || !step || !out || M <= 0 ||
         M > e->m.max_rows || n_seq <= 0)
         return LM_B200_EINVAL;
@@ -1541,6 +1555,7 @@ int lm_b200_op_norm_tapmix(lm_b200_engine* e, int layer, int sub, const float* x
 
 int lm_b200_op_mixer(lm_b200_engine* e, int layer, const float* h, const int32_t* step, int M, int n_seq, float* y,
                      void* stream) {
+    const TakesSizes once{e};
     if (!e || layer < 0 || layer >= e->m.n_layer || !h || !step || !y || M <= 0 || M > e->m.max_rows || n_seq <= 0)
         return LM_B200_EINVAL;
     Guard g(e->device);
@@ -1560,6 +1575,7 @@ int lm_b200_op_mixer(lm_b200_engine* e, int layer, const float* h, const int32_t
 
 int lm_b200_op_attention(lm_b200_engine* e, int layer, float* qk, const int32_t* step, int M, int n_seq, float* out,
                          void* stream) {
+    const TakesSizes once{e};
     if (!e || layer < 0 || layer >= e->m.n_layer || !qk || !step || !out || M <= 0 || M > e->m.max_rows || n_seq <= 0)
         return LM_B200_EINVAL;
     Guard g(e->device);
@@ -1579,6 +1595,7 @@ int lm_b200_op_attention(lm_b200_engine* e, int layer, float* qk, const int32_t*
 
 int lm_b200_op_mixer_kernels(lm_b200_engine* e, int layer, float* proj, const int32_t* step, int M, int n_seq, float* out,
                              void* stream) {
+    const TakesSizes once{e};
     if (!e || layer < 0 || layer >= e->m.n_layer || !proj || !step || !out || M <= 0 || M > e->m.max_rows || n_seq <= 0)
         return LM_B200_EINVAL;
     const lm_b200_layer& l = e->layers[layer];
@@ -1636,6 +1653,7 @@ int lm_b200_op_ff(lm_b200_engine* e, int layer, const float* h, int M, float* y,
 }
 
 int lm_b200_op_token_input(lm_b200_engine* e, int layer, const float* x, const int32_t* step, int M, float* out, void* stream) {
+    const TakesSizes once{e};
     if (!e || layer < 0 || layer >= e->m.n_layer || !x || !step || !out || M <= 0 || M > e->m.max_rows) return LM_B200_EINVAL;
     const lm_b200_layer& l = e->layers[layer];
     if (l.form != LM_B200_FORM_STREAMS || l.side_dim <= 0) return LM_B200_EINVAL;

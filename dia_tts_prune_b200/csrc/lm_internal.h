@@ -181,7 +181,8 @@ cudaError_t launch_column_scan(const float* in, int ld, const ScanInputs& si, in
 // that).  n_long: how many there are (0: not known), of at most longest_tokens.  room: delta_room_floats(M, n_seq, H) floats, 16-byte aligned.
 // kChunkTokensMin: from where chunks are the shorter way beside other sequences (us of a layer of 16 heads of 128, serial / chunks from 96, 128 and 160 tokens on: one prompt
 // of 128 tokens 88 / 87 82 82, prompts of 200, 150, 100, 50, 200 and 150 224 / 204 216 227, four of 300 264 / 255 255 255, eight of 250 412 / 338 340 338).  The longest sequences
-// below it wait for more SMs where others are just above: three of 95, 95 and 96 tokens 104 / 125 106 106, of 127, 127 and 128 115 / 123 139 117.
+// below it wait for the chunks' first kernel, and for registers beside the second, where others are just above: three of 95, 95 and 96 tokens 104 / 125 106 106, of
+// 127, 127 and 128 115 / 121 139 117.  (On a stream of their own they start at once, 115 for the former, but 900 and five of 40 take 321 instead of 254.)
 constexpr int kDeltaChunk = 32, kDeltaChunkFloats = 2 * kDeltaChunk * kDeltaChunk + 2 * kDeltaChunk, kChunkTokensMin = 96;
 inline size_t delta_room_floats(size_t M, size_t n_seq, size_t H) { return (M / kDeltaChunk + n_seq) * H * kDeltaChunkFloats; }
 bool delta_chunks_ok(const float* in, int ld, const ScanInputs& si, int H, int G, int dim, int vdim, const float* state);

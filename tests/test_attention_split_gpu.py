@@ -270,3 +270,35 @@ def test_denominators_are_summed_per_16_keys(place):
     v[0, 0, :, 0], v[0, 0, heavy, 0], v[0, 0, heavy, 1] = 1.0, 0.0, 1.0
     got = E.attention_rows(q.cuda(), k.cuda(), v.cuda(), 64 * tiles, 2, None)[0, :, 0, 1].double().cpu()
     assert (got - 1.0 / (1.0 + tiles * light)).abs().max() <= 2.0 ** -22
+
+
+def test_sizes_are_for_one_call():
+    """Sizes said for a call that is refused are gone with it: the call that follows, with as many sequences and rows, is another step"""
+    import ctypes as C
+
+    import numpy as np
+
+    from dia_tts_prune_b200 import synthetic as SY
+    from dia_tts_prune_b200.lm_config import FipadraConfig
+    from dia_tts_prune_b200.lm_model import CausalLM
+    cfg = SY.fipadra_config(width=64, kinds=["delta"], heads=2, kv_heads=2, dim=64, vdim=64, vocab=64)
+    model = CausalLM(FipadraConfig.model_validate(cfg), SY.fipadra_weights(cfg, 5), dtype="float32", device="cuda:0", max_tokens=1024, max_sequences=2, max_rows=256)
+    x = torch.randn(200, 64, generator=torch.Generator().manual_seed(3)).cuda()
+
+    def run(rows):
+        seqs = [model.state.open(n) for n in "ab"]
+        for q, n in zip(seqs, rows):
+            model.state.reserve(q, n)
+        y = model.engine.op_mixer(0, x, [(q, n, 0) for q, n in zip(seqs, rows)]).clone()
+        for n in "ab":
+            model.state.close(n)
+        return y
+
+    want = run((190, 10))
+    model.engine._say = lambda *sizes: None
+    sizes = np.array([100, 100, 0, 0], dtype=np.int32)            # (both long: with these the short one would have no kernel)
+    lib, h = model.engine.lib, model.engine._h
+    assert lib.lm_b200_step_sizes(h, sizes.ctypes.data, sizes.ctypes.data + 8, 2) == 0
+    assert lib.lm_b200_op_mixer(h, 0, None, None, 200, 2, None, C.c_void_p(0)) != 0
+    assert torch.equal(run((190, 10)), want)
+    assert lib.lm_b200_step_sizes(h, sizes.ctypes.data, sizes.ctypes.data + 8, 0) != 0
