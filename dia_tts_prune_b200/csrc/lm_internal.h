@@ -84,14 +84,6 @@ inline long long step_tiles(const StepSizes& z, int window, int chunk, int keep_
 struct SplitRoom {
     void* work; size_t bytes; int n_slots; SeqMeta sm; int n_seq; StepSizes sizes; long long most_tiles;
     long long tiles(int window, int chunk, int keep_first) const { return sizes.n > 0 ? step_tiles(sizes, window, chunk, keep_first) : most_tiles; }
-    // Whether no row sees more than one tile, of keys and values of one group of channels each: the row tiles split it for themselves, no launch goes in front
-    // (us, launch / none: 12 rows of 8 heads of 64 46.0 / 44.2, mixed scores of 8 heads of 128 56.6 / 55.0; rows of several groups are slower without,
-    // 160 latent channels 85.0 / 87.0, 288 96 / 103)
-    bool one_tile(int kdim, int vdim) const {
-        for (int s = 0; s < sizes.n; ++s)
-            if (sizes.first[s] + sizes.rows[s] > 64) return false;
-        return sizes.n > 0 && kdim <= 128 && vdim <= 128;
-    }
 };
 // ldo: row stride of the output (0: heads * dim); out_scale multiplies it, and so does the sigmoid of gate[row * ldg + column],
 // if given.  split: steps of more than kAttnRowsKernelMax rows run on the split-operand kernel where it takes the shape

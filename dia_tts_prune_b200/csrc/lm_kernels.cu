@@ -1408,7 +1408,7 @@ cudaError_t launch_sink_attention(const float* qk, int q_stride, const float* kc
             s.row_slot = rm.slot; s.row_pos = rm.pos; s.M = M;
             s.window = a.window; s.keep_first = a.keep_first; s.chunk = a.chunk;
             s.out = out; s.ldo = ldo; s.out_bf16 = out_bf16; s.out_scale = out_scale; s.gate = gate; s.ldg = ldg;
-            s.work = split->one_tile(a.dim, a.dim) ? nullptr : split->work; s.work_bytes = split->bytes; s.n_slots = split->n_slots;
+            s.work = split->work; s.work_bytes = split->bytes; s.n_slots = split->n_slots;
             s.seq_slot = split->sm.slot; s.seq_row0 = split->sm.row0; s.seq_count = split->sm.count; s.n_seq = split->n_seq;
             s.n_tiles = split->tiles(a.window, a.chunk, a.keep_first);
             if (dia::split_attention_ok(s)) return dia::launch_split_attention(s, st);

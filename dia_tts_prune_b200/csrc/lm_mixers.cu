@@ -882,7 +882,7 @@ cudaError_t launch_talk_attention(const float* proj, int ld, int q_off, int gate
         s.row_slot = rm.slot; s.row_pos = rm.pos; s.M = M; s.window = a.window;
         s.out = out; s.ldo = ldo; s.out_bf16 = out_bf16; s.out_scale = 1.f;
         if (gate_off >= 0) { s.head_gate = proj + gate_off; s.ldg = ld; }
-        s.work = split->one_tile(a.dim, a.vdim) ? nullptr : split->work; s.work_bytes = split->bytes; s.n_slots = split->n_slots;
+        s.work = split->work; s.work_bytes = split->bytes; s.n_slots = split->n_slots;
         s.seq_slot = split->sm.slot; s.seq_row0 = split->sm.row0; s.seq_count = split->sm.count; s.n_seq = split->n_seq;
         s.n_tiles = split->tiles(a.window, 0, 0);
         if (dia::split_attention_ok(s)) return dia::launch_split_attention(s, st);

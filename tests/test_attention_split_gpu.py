@@ -207,28 +207,6 @@ def test_keys_beyond_the_room_have_the_same_bits(kind, window):
     assert more[0] == 0 and (more[1] > 0) == (window == 0) and more[2] == 0      # (a window's keys fit in any case)
 
 
-@pytest.mark.parametrize("rows,past,launches", [([12], 0, 2), ([64], 0, 2), ([9, 20, 10], 44, 2), ([65], 0, 3), ([20, 20], 45, 3)])
-def test_steps_of_one_tile_of_keys_split_it_themselves(rows, past, launches):
-    """Norm and append, then the attention alone where no sequence has more than 64 keys; the same bits as with a launch in front"""
-    from dia_tts_prune_b200 import synthetic as SY
-    from dia_tts_prune_b200.lm_config import PubopelConfig
-    from dia_tts_prune_b200.lm_model import CausalLM
-    cfg = SY.pubopel_config(width=32, layers=1, heads=4, kv_heads=2, dim=64, experts=1, top=1, expert_ff=8, shared_ff=None, vocab=64, window=None, keep_first=0, softcap=30.0)
-    model = CausalLM(PubopelConfig.model_validate(cfg), SY.pubopel_weights(cfg, 3), dtype="bfloat16", device="cuda:0", max_tokens=512, max_sequences=4, page_size=16, max_rows=128)
-    g = torch.Generator().manual_seed(8)
-    seqs = [model.state.open(str(i)) for i in range(len(rows))]
-    for q in seqs:
-        model.state.reserve(q, past + 80)
-        if past:
-            model.engine.op_attention(0, torch.randn(past, 6 * 64, generator=g), [(q, past, 0)])
-    x, parts = torch.randn(sum(rows), 6 * 64, generator=g), [(q, n, past) for q, n in zip(seqs, rows)]
-    before = model.engine.lib.lm_b200_launch_count()
-    got = model.engine.op_attention(0, x, parts)
-    assert model.engine.lib.lm_b200_launch_count() - before == launches
-    model.engine._say = lambda *sizes: None
-    assert torch.equal(got, model.engine.op_attention(0, x, parts))
-
-
 @pytest.mark.parametrize("B,Tq,Hq,Hkv", [(1, 200, 16, 16), (2, 300, 4, 1)])
 def test_calls_without_room_borrow_it(B, Tq, Hq, Hkv):
     """Their keys are split by a launch in front like those of calls that bring room; during a capture they go without"""
