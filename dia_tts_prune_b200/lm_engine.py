@@ -47,6 +47,10 @@ class LMEngine:
         self.final_norm = final_norm
         self.width, self.vocab, self.max_rows = int(width), int(vocab), int(max_rows)
         self._zeros = np.zeros(64, dtype=np.int32)
+        # Steps whose sizes decide something: their keys may not fit the room that the engine starts with, or recurrences may go in chunks of many tokens
+        # (telling takes the host a microsecond)
+        recurrent = any(r is not None for r in state.rec_states) or any(r.parts for r in state.records)
+        self._say_from = 9 if state.n_slots * state.max_pages * state.page_size > 32768 else 96 if recurrent else 1 << 62
         m = _lm_lib.Model()
         m.n_layer, m.width, m.vocab, m.taps = len(layers), self.width, self.vocab, int(taps)
         m.page_size, m.max_pages, m.n_slots, m.max_rows = state.page_size, state.max_pages, state.n_slots, self.max_rows
@@ -109,7 +113,7 @@ class LMEngine:
             a = b
         buf[4 * n_rows:] = [p[0].slot for p in parts] + row0 + counts + want + [p[2] for p in parts]
         t = torch.from_numpy(buf)
-        if n_rows > 8:                                          # (shorter steps have no use for it)
+        if n_rows >= self._say_from:
             at = t.data_ptr()
             self._say(at + 4 * (4 * n_rows + 2 * S), at + 4 * (buf.size - S), S)
         if buf.size > 4096:                                     # a long step: asynchronous copy from pinned memory
