@@ -97,9 +97,9 @@ class LMEngine:
         S = len(parts)
         counts = [len(t) for _, t, _, _ in parts]
         n_rows = sum(counts)
-        # token, slot, position, start of every row; slot, first row, rows of every sequence; wanted rows; and, for the host alone, first positions
+        # token, slot, position, start of every row; slot, first row, rows of every sequence; wanted rows
         n_want = sum([len(p[3]) for p in parts])
-        buf = np.empty(4 * n_rows + 4 * S + n_want, dtype=np.int32)
+        buf = np.empty(4 * n_rows + 3 * S + n_want, dtype=np.int32)
         want, row0, a = [], [], 0
         for n, (seq, tokens, p0, w) in zip(counts, parts):
             b = a + n
@@ -111,11 +111,11 @@ class LMEngine:
                 want += [a + k for k in w]
             row0.append(a)
             a = b
-        buf[4 * n_rows:] = [p[0].slot for p in parts] + row0 + counts + want + [p[2] for p in parts]
+        buf[4 * n_rows:] = [p[0].slot for p in parts] + row0 + counts + want
         t = torch.from_numpy(buf)
         if n_rows >= self._say_from:
-            at = t.data_ptr()
-            self._say(at + 4 * (4 * n_rows + 2 * S), at + 4 * (buf.size - S), S)
+            first = np.array([p[2] for p in parts], dtype=np.int32)
+            self._say(t.data_ptr() + 4 * (4 * n_rows + 2 * S), first.__array_interface__["data"][0], S)
         if buf.size > 4096:                                     # a long step: asynchronous copy from pinned memory
             t = t.pin_memory()
         return t.to(self.device, non_blocking=True), n_rows, S, n_want
