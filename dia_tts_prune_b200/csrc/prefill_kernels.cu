@@ -322,9 +322,9 @@ size_t attention_rows_work_bytes(int B, int Tq, int Tk, int Hq, int Hkv, int mod
     if (!on_tensor_cores(B, Tq, kSplitRowsMin) || Hkv <= 0 || Hq % Hkv) return 0;
     float* const some = reinterpret_cast<float*>(256);        // (only alignment is looked at)
     const SplitAttention s = split_rows(some, some, some + 64, some, B, Tq, Tk, Hq, Hkv, Tk, mode, n_valid_host);
-    int keys = 0;
-    for (int b = 0; b < B; ++b) keys += (std::max(split_attention_keys(s, b), 0) + 63) & ~63;
-    return split_attention_work_bytes(s, keys);
+    long long tiles = 0;                                      // (a room has 65535 at most; the sizes may be any numbers here)
+    for (int b = 0; b < B; ++b) tiles += (std::max(split_attention_keys(s, b), 0) + 63LL) / 64;
+    return split_attention_work_bytes(s, 64 * (int)std::min(tiles, 65535LL));
 }
 
 cudaError_t launch_attention_rows(const float* q, const float* k, const float* v, float* out, int B, int Tq, int Tk, int Hq,

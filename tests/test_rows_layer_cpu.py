@@ -202,3 +202,12 @@ def test_the_workspace_does_not_depend_on_the_valid_keys(T, mode):
             a.n_valid[b], a.cross_valid[b] = valid, 3 * valid
         bytes_of.append(lib.dia_b200_rows_layer_work_bytes(C.byref(a)))
     assert bytes_of[0] == bytes_of[1] == bytes_of[2] > 0
+
+
+@pytest.mark.parametrize("Tk", [0, 1, 64, 2 ** 31 - 1])
+def test_the_room_of_any_number_of_keys(Tk):
+    """Whole tiles of 64 keys, 65535 of them at most: what a caller asks for is not yet checked against what there is"""
+    from dia_tts_prune_b200 import _lib
+    need = _lib.load().dia_b200_attention_rows_work_bytes(16, 200, Tk, 16, 16, 2, None)
+    tiles = min(16 * (-(-Tk // 64)), 65535)
+    assert need >= tiles * 64 * 16 * 2 * 512 and need <= tiles * 64 * 16 * (2 * 512 + 8) + 1024
